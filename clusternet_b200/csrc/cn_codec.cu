@@ -36,11 +36,6 @@
 #define LUT_SHIFT 16
 #define LUT_MAX 2816
 
-// Programmatic dependent launch: "my successor in the stream may start" / "my predecessor has finished and its writes are
-// visible".  Without the launch attribute both are no-ops.
-__device__ __forceinline__ void cdc_pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void cdc_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // The small per-codebook tables travel as kernel parameters (constant bank): read from global memory they would be a
 // cold DRAM miss on the critical path of every launch's table build.
 struct CodecConst {
@@ -132,8 +127,8 @@ cn_compress_kernel(const float *__restrict__ A, float precision_arg, const float
 {
     __shared__ CodecTables t;
     const int tid = threadIdx.x;
-    cdc_pdl_launch_dependents();
-    cdc_pdl_wait();
+    cn_pdl_launch_dependents();
+    cn_pdl_wait();
     const float p = PRECISION_ON_DEVICE ? *d_precision : precision_arg;
     const uint32_t pb = __float_as_uint(p);
     const uint32_t psign4 = (pb >> 31) * 0x80808080u;
@@ -512,7 +507,7 @@ cn_compress_ring_kernel(const float *__restrict__ A, float precision_arg, float 
         for (int s = 0; s < RING_STAGES; ++s) { cdc_mbar_init(full_bar(s), 1); cdc_mbar_init(empty_bar(s), RING_THREADS / 32); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    cdc_pdl_launch_dependents();
+    cn_pdl_launch_dependents();
     if (tid < 128) {
         t.T[tid] = rc.thr[tid];
         t.lc[tid] = rc.lc[tid];
@@ -549,7 +544,7 @@ cn_compress_ring_kernel(const float *__restrict__ A, float precision_arg, float 
     };
     if (SCALE == RING_SCALE_DEVICE && input_ready_before_predecessor && tid == 0) fill_ring();
     // ---- everything below may touch global memory: the predecessor in the stream must have finished
-    cdc_pdl_wait();
+    cn_pdl_wait();
     float p = precision_arg;
     if (SCALE == RING_SCALE_ABSMAX) {
         // pass 1: maximum of |A| over this CTA's tiles (and, in CTA 0, the last n % 4 elements)
@@ -877,8 +872,8 @@ cn_decompress_kernel(const uint8_t *__restrict__ codes, float precision_arg, con
 {
     __shared__ float lut[256];
     const int tid = threadIdx.x;
-    cdc_pdl_launch_dependents();
-    if (PRECISION_ON_DEVICE) cdc_pdl_wait();   // the scale is in global memory; a host scale lets the table precede the wait
+    cn_pdl_launch_dependents();
+    if (PRECISION_ON_DEVICE) cn_pdl_wait();   // the scale is in global memory; a host scale lets the table precede the wait
     const float p = PRECISION_ON_DEVICE ? *d_precision : precision_arg;
     if (tid < 256) {
         float v = 0.0f;
@@ -891,7 +886,7 @@ cn_decompress_kernel(const uint8_t *__restrict__ codes, float precision_arg, con
         }
         lut[tid] = v;
     }
-    if (!PRECISION_ON_DEVICE) cdc_pdl_wait();
+    if (!PRECISION_ON_DEVICE) cn_pdl_wait();
     __syncthreads();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     float4 *out4 = reinterpret_cast<float4 *>(out);
@@ -943,8 +938,8 @@ cn_decompress16_kernel(const uint8_t *__restrict__ codes, float precision_arg, c
 {
     __shared__ float lut[256];
     const int tid = threadIdx.x;
-    cdc_pdl_launch_dependents();
-    if (PRECISION_ON_DEVICE) cdc_pdl_wait();   // the scale is in global memory; a host scale lets the table precede the wait
+    cn_pdl_launch_dependents();
+    if (PRECISION_ON_DEVICE) cn_pdl_wait();   // the scale is in global memory; a host scale lets the table precede the wait
     const float p = PRECISION_ON_DEVICE ? *d_precision : precision_arg;
     if (tid < 256) {
         float v = 0.0f;
@@ -957,7 +952,7 @@ cn_decompress16_kernel(const uint8_t *__restrict__ codes, float precision_arg, c
         }
         lut[tid] = v;
     }
-    if (!PRECISION_ON_DEVICE) cdc_pdl_wait();
+    if (!PRECISION_ON_DEVICE) cn_pdl_wait();
     __syncthreads();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     float4 *out4 = reinterpret_cast<float4 *>(out);
@@ -996,8 +991,8 @@ cn_absmax_kernel(const float *__restrict__ A, int64_t n, float *__restrict__ out
     const int tid = threadIdx.x;
     // wait first, then release the successor: a kernel that follows absmax in the stream may then rely on everything
     // before absmax having finished (cn_absmax_compress_8bit's compressor starts loading A before its own wait)
-    cdc_pdl_wait();
-    cdc_pdl_launch_dependents();
+    cn_pdl_wait();
+    cn_pdl_launch_dependents();
     float m = -1.0f;   // the reference seeds thrust::reduce with -1.0f (source/basicOps.cu:1079)
     const int64_t nvec = vector_ok ? (n >> 2) : 0;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -1087,8 +1082,8 @@ cn_absmax_ring_kernel(const float *__restrict__ A, int64_t n, float *__restrict_
         return (int)(left < tile_groups ? left : tile_groups);
     };
     __syncthreads();
-    cdc_pdl_wait();
-    cdc_pdl_launch_dependents();   // after the wait: see cn_absmax_kernel
+    cn_pdl_wait();
+    cn_pdl_launch_dependents();   // after the wait: see cn_absmax_kernel
     if (tid == 0) {
         for (int i = 0; i < RING_STAGES && i < my_tiles; ++i) {
             const int64_t j = blockIdx.x + (int64_t)i * gridDim.x;
@@ -1174,24 +1169,6 @@ static int codec_grid(const cn_context *ctx, int64_t n, int threads, int per_thr
     int64_t cap = (int64_t)ctx->sm_count * ctas_per_sm;
     if (need < 1) need = 1;
     return (int)(need < cap ? need : cap);
-}
-
-// Launch with programmatic stream serialisation: the kernel may become resident while its predecessor in the stream is
-// still running; it synchronises with it through griddepcontrol.wait.
-template <typename... KArgs, typename... Args>
-static cudaError_t launch_pdl(void (*kernel)(KArgs...), int grid, int block, size_t smem, cudaStream_t s, Args... args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 // The 127 boundaries in |x| space for a host-side scale: the smallest fp32 |x| with fl(|x| / |p|) >= T_j, found with the
@@ -1311,10 +1288,10 @@ static int compress_impl(cn_context *ctx, const float *d_A, float precision, flo
             CN_CUDA(cudaLaunchKernelEx(&cfg, cn_compress_ring_kernel<RING_SCALE_ABSMAX>, d_A, 0.f, d_precision, n, d_codes, rc, d_status, tile_groups,
                                        tiles_per_cta, ctx->d_partials, barrier_words, 0));
         } else if (scale_mode == RING_SCALE_DEVICE) {
-            CN_CUDA(launch_pdl(cn_compress_ring_kernel<RING_SCALE_DEVICE>, grid, RING_THREADS, smem, s, d_A, 0.f, d_precision, n, d_codes, rc, d_status,
+            CN_CUDA(cn_launch_pdl(cn_compress_ring_kernel<RING_SCALE_DEVICE>, grid, RING_THREADS, smem, s, d_A, 0.f, d_precision, n, d_codes, rc, d_status,
                                tile_groups, tiles_per_cta, (float *)nullptr, (unsigned int *)nullptr, after_own_absmax));
         } else {
-            CN_CUDA(launch_pdl(cn_compress_ring_kernel<RING_SCALE_HOST>, grid, RING_THREADS, smem, s, d_A, precision, (float *)nullptr, n, d_codes, rc,
+            CN_CUDA(cn_launch_pdl(cn_compress_ring_kernel<RING_SCALE_HOST>, grid, RING_THREADS, smem, s, d_A, precision, (float *)nullptr, n, d_codes, rc,
                                d_status, tile_groups, tiles_per_cta, (float *)nullptr, (unsigned int *)nullptr, 0));
         }
         cn_count_launch();
@@ -1324,9 +1301,9 @@ static int compress_impl(cn_context *ctx, const float *d_A, float precision, flo
     CodecConst cc;
     for (int i = 0; i < 128; ++i) { cc.thr[i] = ctx->h_thr[i]; cc.lc[i] = ctx->h_level_codes[i]; }
     if (scale_mode == RING_SCALE_DEVICE)
-        CN_CUDA(launch_pdl(cn_compress_kernel<true>, grid, CODEC_THREADS, 0, s, d_A, 0.f, (const float *)d_precision, n, d_codes, cc, 0));
+        CN_CUDA(cn_launch_pdl(cn_compress_kernel<true>, grid, CODEC_THREADS, 0, s, d_A, 0.f, (const float *)d_precision, n, d_codes, cc, 0));
     else
-        CN_CUDA(launch_pdl(cn_compress_kernel<false>, grid, CODEC_THREADS, 0, s, d_A, precision, (const float *)nullptr, n, d_codes, cc, 0));
+        CN_CUDA(cn_launch_pdl(cn_compress_kernel<false>, grid, CODEC_THREADS, 0, s, d_A, precision, (const float *)nullptr, n, d_codes, cc, 0));
     cn_count_launch();
     return CN_OK;
 }
@@ -1413,16 +1390,16 @@ static int decompress_impl(cn_context *ctx, const uint8_t *d_codes, float precis
     for (int i = 0; i < 128; ++i) dc.tbl[i] = ctx->h_tbl[i];
     if (vector_ok == 2) {
         if (d_precision)
-            CN_CUDA(launch_pdl(cn_decompress16_kernel<true>, grid, CODEC_THREADS, 0, cn_stream(stream), d_codes, 0.f, d_precision, n, d_out, dc));
+            CN_CUDA(cn_launch_pdl(cn_decompress16_kernel<true>, grid, CODEC_THREADS, 0, cn_stream(stream), d_codes, 0.f, d_precision, n, d_out, dc));
         else
-            CN_CUDA(launch_pdl(cn_decompress16_kernel<false>, grid, CODEC_THREADS, 0, cn_stream(stream), d_codes, precision, (const float *)nullptr, n, d_out, dc));
+            CN_CUDA(cn_launch_pdl(cn_decompress16_kernel<false>, grid, CODEC_THREADS, 0, cn_stream(stream), d_codes, precision, (const float *)nullptr, n, d_out, dc));
         cn_count_launch();
         return CN_OK;
     }
     if (d_precision)
-        CN_CUDA(launch_pdl(cn_decompress_kernel<true>, grid, CODEC_THREADS, 0, cn_stream(stream), d_codes, 0.f, d_precision, n, d_out, dc, vector_ok));
+        CN_CUDA(cn_launch_pdl(cn_decompress_kernel<true>, grid, CODEC_THREADS, 0, cn_stream(stream), d_codes, 0.f, d_precision, n, d_out, dc, vector_ok));
     else
-        CN_CUDA(launch_pdl(cn_decompress_kernel<false>, grid, CODEC_THREADS, 0, cn_stream(stream), d_codes, precision, (const float *)nullptr, n, d_out, dc, vector_ok));
+        CN_CUDA(cn_launch_pdl(cn_decompress_kernel<false>, grid, CODEC_THREADS, 0, cn_stream(stream), d_codes, precision, (const float *)nullptr, n, d_out, dc, vector_ok));
     cn_count_launch();
     return CN_OK;
 }
@@ -1460,7 +1437,7 @@ extern "C" int cn_absmax_f32(cn_context *ctx, const float *d_A, int64_t n, float
         const int tiles_per_cta = (int)((min_tiles + grid - 1) / grid);
         int tile_groups = (int)((groups + (int64_t)grid * tiles_per_cta - 1) / ((int64_t)grid * tiles_per_cta));
         if (max_groups * 100 <= (int64_t)tile_groups * 102) tile_groups = (int)max_groups;   // whole tiles when nearly balanced anyway
-        CN_CUDA(launch_pdl(cn_absmax_ring_kernel, grid, RING_THREADS, smem, cn_stream(stream), d_A, n, d_out, ctx->d_partials, ctx->d_ticket,
+        CN_CUDA(cn_launch_pdl(cn_absmax_ring_kernel, grid, RING_THREADS, smem, cn_stream(stream), d_A, n, d_out, ctx->d_partials, ctx->d_ticket,
                            d_status, tile_groups, tiles_per_cta));
         cn_count_launch();
         return CN_OK;
@@ -1469,7 +1446,7 @@ extern "C" int cn_absmax_f32(cn_context *ctx, const float *d_A, int64_t n, float
     // four), eight per SM stream best on large ones (1 GiB: 6737 GB/s vs 6332)
     int grid = codec_grid(ctx, n, ABSMAX_THREADS, 16, n < (1LL << 27) ? 2 : 8);
     if (grid > CN_MAX_PARTIALS) grid = CN_MAX_PARTIALS;
-    CN_CUDA(launch_pdl(cn_absmax_kernel<true>, grid, ABSMAX_THREADS, 0, cn_stream(stream), d_A, n, d_out, ctx->d_partials, ctx->d_ticket, vector_ok));
+    CN_CUDA(cn_launch_pdl(cn_absmax_kernel<true>, grid, ABSMAX_THREADS, 0, cn_stream(stream), d_A, n, d_out, ctx->d_partials, ctx->d_ticket, vector_ok));
     cn_count_launch();
     return CN_OK;
 }

@@ -3,14 +3,24 @@
 // maxout (source/basicOps.cu:1287-1299; kMaxout source/clusterKernels.cu:1432-1458).
 #include "cn_epilogue.cuh"
 
-__global__ void cn_bias_act_kernel(const float *__restrict__ A, const float *__restrict__ bias, int act,
-                                   float *__restrict__ out, int64_t rows, int64_t n)
+// Blocks of rows of one column: the column's bias is read once and no element needs a division to find its column.
+__global__ void __launch_bounds__(256)
+cn_bias_act_kernel(const float *A, const float *bias, int act, float *out, int64_t rows, int64_t cols, int64_t row_blocks)
 {
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        float v = A[i];
-        if (bias) v += bias[i / rows];   // kAddMatrixVector: one bias value per column
-        out[i] = cn_apply_activation(v, act);
+    cn_pdl_launch_dependents();
+    cn_pdl_wait();
+    for (int64_t b = blockIdx.x; b < row_blocks * cols; b += gridDim.x) {
+        const int64_t col = b / row_blocks, r0 = (b - col * row_blocks) * 1024;
+        const float bj = bias ? bias[col] : 0.0f;   // kAddMatrixVector: one bias value per column
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int64_t r = r0 + u * 256 + threadIdx.x;
+            if (r < rows) {
+                float v = A[col * rows + r];
+                if (bias) v += bj;
+                out[col * rows + r] = cn_apply_activation(v, act);
+            }
+        }
     }
 }
 
@@ -19,9 +29,10 @@ __global__ void cn_bias_act_kernel(const float *__restrict__ A, const float *__r
 // takes slot t+offset when its own value is strictly smaller (reduceToMaxAndArgMax,
 // source/clusterKernels.cu:563-604).  The same tree is walked here with shuffles so that ties resolve
 // to the same column.
-__global__ void cn_maxout_kernel(const float *__restrict__ A, float *__restrict__ out, float *__restrict__ argmax,
-                                 int64_t rows, int64_t out_cols, int L)
+__global__ void cn_maxout_kernel(const float *A, float *out, float *argmax, int64_t rows, int64_t out_cols, int L)
 {
+    cn_pdl_launch_dependents();
+    cn_pdl_wait();
     const int lane = threadIdx.x & 31;
     const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     const int64_t total = rows * out_cols;
@@ -53,9 +64,10 @@ extern "C" int cn_bias_activation(cn_context *ctx, const float *d_A, const float
     if (n == 0) return CN_OK;
     CN_REQUIRE(d_A && d_out, CN_ERR_ARG, "cn_bias_activation: null buffer");
     CN_REQUIRE(activation >= CN_ACT_LINEAR && activation <= CN_ACT_DOUBLE_RELU, CN_ERR_ARG, "cn_bias_activation: unknown activation %d", activation);
-    int64_t blocks = (n + 255) / 256, cap = (int64_t)ctx->sm_count * 8;
-    cn_bias_act_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, cn_stream(stream)>>>(d_A, d_bias, activation, d_out, rows, n);
-    CN_CUDA(cudaGetLastError());
+    const int64_t row_blocks = (rows + 1023) / 1024;
+    int64_t blocks = row_blocks * cols, cap = (int64_t)ctx->sm_count * 8;
+    CN_CUDA(cn_launch_pdl(cn_bias_act_kernel, dim3((unsigned)(blocks < cap ? blocks : cap)), 256, 0, cn_stream(stream), d_A, d_bias, activation, d_out,
+                          rows, cols, row_blocks));
     cn_count_launch();
     return CN_OK;
 }
@@ -71,8 +83,8 @@ extern "C" int cn_maxout(cn_context *ctx, const float *d_A, float *d_out, float 
     if (total == 0) return CN_OK;
     CN_REQUIRE(d_A && d_out, CN_ERR_ARG, "cn_maxout: null buffer");
     int64_t blocks = (total + 7) / 8, cap = (int64_t)ctx->sm_count * 8;
-    cn_maxout_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, cn_stream(stream)>>>(d_A, d_out, d_argmax, rows, out_cols, maxout_level);
-    CN_CUDA(cudaGetLastError());
+    CN_CUDA(cn_launch_pdl(cn_maxout_kernel, dim3((unsigned)(blocks < cap ? blocks : cap)), 256, 0, cn_stream(stream), d_A, d_out, d_argmax, rows, out_cols,
+                          maxout_level));
     cn_count_launch();
     return CN_OK;
 }

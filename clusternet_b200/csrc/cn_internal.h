@@ -81,6 +81,32 @@ int cn_comm_flag_barrier(cn_context *ctx, int slot, unsigned int epoch, cudaStre
 
 static inline cudaStream_t cn_stream(void *s) { return reinterpret_cast<cudaStream_t>(s); }
 
+#ifdef __CUDACC__
+// Programmatic dependent launch.  A kernel launched with cn_launch_pdl may become resident while its predecessor in the
+// stream still runs; it calls cn_pdl_launch_dependents() ("my successor may start too") and, before its first access to
+// global memory, cn_pdl_wait() ("my predecessor has finished and its writes are visible").  Every thread of every such kernel
+// waits, so that a kernel's end implies the end of everything before it.  Launch latency and CTA start-up then overlap the
+// predecessor's tail: about 1 us per launch in a chain of small kernels.
+__device__ __forceinline__ void cn_pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void cn_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... KArgs, typename... Args>
+static inline cudaError_t cn_launch_pdl(void (*kernel)(KArgs...), dim3 grid, int block, size_t smem, cudaStream_t s, Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+#endif
+
 // Pushed block exchange, seen from the codec: where this rank's codes and scale go in every peer's area, and the flags
 // that frame the stores ("your area may be written" = slot, "my block has arrived" = slot + 1; see cn_push_exchange_kernel).
 struct cn_codec_push {

@@ -9,9 +9,11 @@
 
 // out (C x R, row-major) = transpose of in (R x C, row-major).  One CTA per 32x32 tile, linear tile index.
 __global__ void __launch_bounds__(TP_TILE *TP_ROWS)
-cn_transpose_kernel(const float *__restrict__ in, float *__restrict__ out, int64_t R, int64_t C, int64_t tiles_c)
+cn_transpose_kernel(const float *in, float *out, int64_t R, int64_t C, int64_t tiles_c)
 {
     __shared__ float tile[TP_TILE][TP_TILE + 1];
+    cn_pdl_launch_dependents();
+    cn_pdl_wait();
     const int64_t tile_id = blockIdx.x;
     const int64_t tr = tile_id / tiles_c, tc = tile_id % tiles_c;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -30,8 +32,10 @@ cn_transpose_kernel(const float *__restrict__ in, float *__restrict__ out, int64
     }
 }
 
-__global__ void cn_fill_kernel(float *__restrict__ A, int64_t n, float v)
+__global__ void cn_fill_kernel(float *A, int64_t n, float v)
 {
+    cn_pdl_launch_dependents();
+    cn_pdl_wait();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) A[i] = v;
 }
@@ -42,8 +46,7 @@ static int transpose_launch(const float *in, float *out, int64_t R, int64_t C, c
     const int64_t tiles_r = (R + TP_TILE - 1) / TP_TILE, tiles_c = (C + TP_TILE - 1) / TP_TILE;
     const int64_t tiles = tiles_r * tiles_c;
     CN_REQUIRE(tiles < (1LL << 31), CN_ERR_UNSUPPORTED, "transpose: %lld tiles exceed the grid limit", (long long)tiles);
-    cn_transpose_kernel<<<(unsigned)tiles, TP_TILE * TP_ROWS, 0, s>>>(in, out, R, C, tiles_c);
-    CN_CUDA(cudaGetLastError());
+    CN_CUDA(cn_launch_pdl(cn_transpose_kernel, dim3((unsigned)tiles), TP_TILE * TP_ROWS, 0, s, in, out, R, C, tiles_c));
     cn_count_launch();
     return CN_OK;
 }
@@ -80,8 +83,10 @@ extern "C" int cn_download_row_major(cn_context *ctx, const float *d_src, float 
 }
 
 // kArange (source/clusterKernels.cu:925-937): the column-major image of the row-major counter start, start+1, ...
-__global__ void cn_arange_kernel(float *__restrict__ out, int64_t start, int64_t rows, int64_t cols, int64_t n)
+__global__ void cn_arange_kernel(float *out, int64_t start, int64_t rows, int64_t cols, int64_t n)
 {
+    cn_pdl_launch_dependents();
+    cn_pdl_wait();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
         out[i] = (float)((i % rows) * cols + (i / rows) + start);
@@ -94,8 +99,7 @@ extern "C" int cn_arange_f32(cn_context *ctx, float *d_A, int64_t start, int64_t
     if (n == 0) return CN_OK;
     int64_t blocks = (n + 1023) / 1024;
     int64_t cap = (int64_t)ctx->sm_count * 8;
-    cn_arange_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, cn_stream(stream)>>>(d_A, start, rows, cols, n);
-    CN_CUDA(cudaGetLastError());
+    CN_CUDA(cn_launch_pdl(cn_arange_kernel, dim3((unsigned)(blocks < cap ? blocks : cap)), 256, 0, cn_stream(stream), d_A, start, rows, cols, n));
     cn_count_launch();
     return CN_OK;
 }
@@ -106,8 +110,7 @@ extern "C" int cn_fill_f32(cn_context *ctx, float *d_A, int64_t n, float value, 
     if (n == 0) return CN_OK;
     int64_t blocks = (n + 1023) / 1024;
     int64_t cap = (int64_t)ctx->sm_count * 8;
-    cn_fill_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, cn_stream(stream)>>>(d_A, n, value);
-    CN_CUDA(cudaGetLastError());
+    CN_CUDA(cn_launch_pdl(cn_fill_kernel, dim3((unsigned)(blocks < cap ? blocks : cap)), 256, 0, cn_stream(stream), d_A, n, value));
     cn_count_launch();
     return CN_OK;
 }

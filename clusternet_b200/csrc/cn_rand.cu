@@ -31,14 +31,32 @@ __device__ __forceinline__ float u01(uint32_t x) { return fmaf((float)x, 2.32830
 
 enum { RAND_UNIFORM = 0, RAND_NORMAL = 1, RAND_SQRT_WEIGHT = 2, RAND_DROPOUT = 3, RAND_INT = 4 };
 
+// One Philox block per thread and step: four elements, stored (and for dropout read) with one 16-byte access where the buffers
+// are 16-byte aligned (vec_ok).  Bound by launch latency at a layer's size (128 x 1200: 2.4 us) and by the generator's integer
+// multiplies on large matrices.
 template <int KIND>
-__global__ void cn_rand_kernel(const float *__restrict__ A, float *__restrict__ out, int64_t n, uint64_t seed_arg, uint64_t offset,
-                               float p0, float p1, const uint64_t *__restrict__ d_seed)
+__global__ void __launch_bounds__(256)
+cn_rand_kernel(const float *A, float *out, int64_t n, uint64_t seed_arg, uint64_t offset, float p0, float p1, const uint64_t *d_seed, int vec_ok)
 {
+    cn_pdl_launch_dependents();
+    cn_pdl_wait();
     const uint64_t seed = d_seed ? *d_seed : seed_arg;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int64_t ngroups = (n + 3) >> 2;
     for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < ngroups; g += stride) {
+        const int64_t i0 = g << 2;
+        const bool whole = vec_ok && i0 + 4 <= n;
+        float a[4] = {0.f, 0.f, 0.f, 0.f};
+        if (KIND == RAND_DROPOUT) {   // the loads first: the generator hides their latency
+            if (whole) {
+                const float4 q = *reinterpret_cast<const float4 *>(A + i0);
+                a[0] = q.x; a[1] = q.y; a[2] = q.z; a[3] = q.w;
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    if (i0 + k < n) a[k] = A[i0 + k];
+            }
+        }
         const uint4 r = philox4x32_10(offset + (uint64_t)g, seed);
         float v[4] = {u01(r.x), u01(r.y), u01(r.z), u01(r.w)};
         if (KIND == RAND_NORMAL) {
@@ -50,15 +68,18 @@ __global__ void cn_rand_kernel(const float *__restrict__ A, float *__restrict__ 
             v[0] = fmaf(r0 * c0, p1, p0); v[1] = fmaf(r0 * s0, p1, p0);
             v[2] = fmaf(r1 * c1, p1, p0); v[3] = fmaf(r1 * s1, p1, p0);
         }
-        const int64_t i0 = g << 2;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const int64_t i = i0 + k;
-            if (i >= n) break;
-            if (KIND == RAND_SQRT_WEIGHT) out[i] = p0 + v[k] * p1;            // lower + u * range, as the reference kernel
-            else if (KIND == RAND_DROPOUT) out[i] = v[k] > p0 ? A[i] : 0.0f;  // kDropout: keep where u > rate, no rescale
-            else if (KIND == RAND_INT) out[i] = fminf((float)((int)(v[k] * p1)) + p0, p0 + p1 - 1.0f);   // kRandInt; u == 1 stays in range
-            else out[i] = v[k];
+            if (KIND == RAND_SQRT_WEIGHT) v[k] = p0 + v[k] * p1;            // lower + u * range, as the reference kernel
+            else if (KIND == RAND_DROPOUT) v[k] = v[k] > p0 ? a[k] : 0.0f;  // kDropout: keep where u > rate, no rescale
+            else if (KIND == RAND_INT) v[k] = fminf((float)((int)(v[k] * p1)) + p0, p0 + p1 - 1.0f);   // kRandInt; u == 1 stays in range
+        }
+        if (whole) {
+            *reinterpret_cast<float4 *>(out + i0) = make_float4(v[0], v[1], v[2], v[3]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (i0 + k < n) out[i0 + k] = v[k];
         }
     }
 }
@@ -71,8 +92,9 @@ static int rand_launch(cn_context *ctx, const float *A, float *out, int64_t n, u
     if (n == 0) return CN_OK;
     int64_t blocks = ((n + 3) / 4 + 255) / 256;
     int64_t cap = (int64_t)ctx->sm_count * 8;
-    cn_rand_kernel<KIND><<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, cn_stream(stream)>>>(A, out, n, seed, offset, p0, p1, d_seed);
-    CN_CUDA(cudaGetLastError());
+    const int vec_ok = ((uintptr_t)out % 16 == 0) && ((uintptr_t)A % 16 == 0);
+    CN_CUDA(cn_launch_pdl(cn_rand_kernel<KIND>, dim3((unsigned)(blocks < cap ? blocks : cap)), 256, 0, cn_stream(stream), A, out, n, seed, offset, p0,
+                          p1, d_seed, vec_ok));
     cn_count_launch();
     return CN_OK;
 }
@@ -120,13 +142,17 @@ extern "C" int cn_dropout_dp(cn_context *ctx, const float *d_A, float *d_out, in
     return rand_launch<RAND_DROPOUT>(ctx, d_A, d_out, n, 0, offset, rate, 0.f, stream, d_seed);
 }
 
-__global__ void cn_seed_advance_kernel(uint64_t *seed) { *seed += 0x9E3779B97F4A7C15ull; }
+__global__ void cn_seed_advance_kernel(uint64_t *seed)
+{
+    cn_pdl_launch_dependents();
+    cn_pdl_wait();
+    *seed += 0x9E3779B97F4A7C15ull;
+}
 
 extern "C" int cn_seed_advance(cn_context *ctx, uint64_t *d_seed, void *stream)
 {
     CN_REQUIRE(ctx && d_seed, CN_ERR_ARG, "cn_seed_advance: null argument");
-    cn_seed_advance_kernel<<<1, 1, 0, cn_stream(stream)>>>(d_seed);
-    CN_CUDA(cudaGetLastError());
+    CN_CUDA(cn_launch_pdl(cn_seed_advance_kernel, dim3(1), 1, 0, cn_stream(stream), d_seed));
     cn_count_launch();
     return CN_OK;
 }

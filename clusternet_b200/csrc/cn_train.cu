@@ -9,66 +9,94 @@
 #include "cn_gemm.h"
 
 // ---- softmax over the columns of a column-major rows x cols matrix: one thread per row, the row's maximum, sum and
-// quotient taken in the reference's order with the same fast exponential, so results match it bit for bit.
-__global__ void cn_softmax_kernel(const float *__restrict__ A, float *__restrict__ out, int64_t rows, int64_t cols)
-{
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; row < rows; row += stride) {
-        float mx = -FLT_MAX;
-        for (int64_t i = 0; i < cols; ++i) {
-            const float v = A[i * rows + row];
-            if (v > mx) mx = v;
-        }
-        float sum = 0.0f;
-        for (int64_t i = 0; i < cols; ++i) sum += __expf(A[i * rows + row] - mx);
-        for (int64_t i = 0; i < cols; ++i) out[i * rows + row] = __expf(A[i * rows + row] - mx) / sum;
-    }
-}
+// quotient taken in the reference's order with the same fast exponential, so results match it bit for bit.  Up to
+// SOFTMAX_REGS columns the row lives in registers: its loads are all in flight at once and each exponential is taken once
+// (bound by latency: 128 x 10 took 3.3 us with three passes over memory).
+#define SOFTMAX_REGS 32
+#define SOFTMAX_THREADS 64
 
-// softmax of each row (as cn_softmax_kernel) and, in the same pass, the output layer's error softmax - onehot(label):
-// the three launches softmax / create_t_matrix / sub of the reference's step (source/Layer.cpp:163-165,318-322) in one.
-__global__ void cn_softmax_error_kernel(const float *__restrict__ A, const float *__restrict__ labels, float *__restrict__ prob,
-                                        float *__restrict__ err, int64_t rows, int64_t cols)
+// ERROR: the output layer's error softmax - onehot(label) in the same pass (the three launches softmax / create_t_matrix / sub
+// of the reference's step, source/Layer.cpp:163-165,318-322).  A and prob may be the same matrix.
+template <bool ERROR, bool SHORT_ROWS>
+__global__ void __launch_bounds__(SOFTMAX_THREADS)
+cn_softmax_kernel(const float *A, const float *labels, float *prob, float *err, int64_t rows, int64_t cols)
 {
+    cn_pdl_launch_dependents();
+    cn_pdl_wait();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; row < rows; row += stride) {
-        float mx = -FLT_MAX;
-        for (int64_t i = 0; i < cols; ++i) {
-            const float v = A[i * rows + row];
-            if (v > mx) mx = v;
-        }
-        float sum = 0.0f;
-        for (int64_t i = 0; i < cols; ++i) sum += __expf(A[i * rows + row] - mx);
-        const int64_t hot = (int64_t)(int)labels[row];
-        for (int64_t i = 0; i < cols; ++i) {
-            const float pr = __expf(A[i * rows + row] - mx) / sum;
-            prob[i * rows + row] = pr;
-            err[i * rows + row] = pr - (i == hot ? 1.0f : 0.0f);
+        const int64_t hot = ERROR ? (int64_t)(int)labels[row] : -1;
+        float mx = -FLT_MAX, sum = 0.0f;
+        if (SHORT_ROWS) {
+            float v[SOFTMAX_REGS];
+#pragma unroll
+            for (int i = 0; i < SOFTMAX_REGS; ++i) v[i] = i < cols ? A[i * rows + row] : -FLT_MAX;
+#pragma unroll
+            for (int i = 0; i < SOFTMAX_REGS; ++i)
+                if (v[i] > mx) mx = v[i];
+#pragma unroll
+            for (int i = 0; i < SOFTMAX_REGS; ++i)
+                if (i < cols) { v[i] = __expf(v[i] - mx); sum += v[i]; }
+#pragma unroll
+            for (int i = 0; i < SOFTMAX_REGS; ++i)
+                if (i < cols) {
+                    const float pr = v[i] / sum;
+                    prob[i * rows + row] = pr;
+                    if (ERROR) err[i * rows + row] = pr - (i == hot ? 1.0f : 0.0f);
+                }
+        } else {
+            for (int64_t i = 0; i < cols; ++i) {
+                const float v = A[i * rows + row];
+                if (v > mx) mx = v;
+            }
+            for (int64_t i = 0; i < cols; ++i) sum += __expf(A[i * rows + row] - mx);
+            for (int64_t i = 0; i < cols; ++i) {
+                const float pr = __expf(A[i * rows + row] - mx) / sum;
+                prob[i * rows + row] = pr;
+                if (ERROR) err[i * rows + row] = pr - (i == hot ? 1.0f : 0.0f);
+            }
         }
     }
 }
 
 // err_out = err_in * f'(activation), and optionally grad_out = f'(activation) (the reference writes the derivative into
 // the layer's `out` matrix and multiplies in a second kernel, source/Layer.cpp:323-329)
+//
+// Elementwise kernels below: bound by HBM on large matrices and by launch latency on a layer's activations.  Four elements per
+// thread with 16-byte accesses where every buffer is 16-byte aligned (n4 > 0), the rest one by one.
 template <int ACT>
-__global__ void cn_mul_grad_kernel(const float *__restrict__ err_in, const float *__restrict__ act, float *__restrict__ grad_out,
-                                   float *__restrict__ err_out, int64_t n)
+__device__ __forceinline__ float act_derivative(float a)
 {
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const float a = act[i];
-        float g;
-        if (ACT == CN_ACT_RELU) g = a > 0.0f ? 1.0f : 0.0f;
-        else if (ACT == CN_ACT_LOGISTIC) g = a * (1.0f - a);
-        else g = (a > 0.0f && a < 1.0f) ? 1.0f : 0.0f;
+    if (ACT == CN_ACT_RELU) return a > 0.0f ? 1.0f : 0.0f;
+    if (ACT == CN_ACT_LOGISTIC) return a * (1.0f - a);
+    return (a > 0.0f && a < 1.0f) ? 1.0f : 0.0f;
+}
+
+template <int ACT>
+__global__ void __launch_bounds__(256)
+cn_mul_grad_kernel(const float *err_in, const float *act, float *grad_out, float *err_out, int64_t n, int64_t n4)
+{
+    cn_pdl_launch_dependents();
+    cn_pdl_wait();
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x, t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (int64_t v = t0; v < n4; v += stride) {
+        const float4 a = reinterpret_cast<const float4 *>(act)[v], e = reinterpret_cast<const float4 *>(err_in)[v];
+        const float4 g = make_float4(act_derivative<ACT>(a.x), act_derivative<ACT>(a.y), act_derivative<ACT>(a.z), act_derivative<ACT>(a.w));
+        if (grad_out) reinterpret_cast<float4 *>(grad_out)[v] = g;
+        reinterpret_cast<float4 *>(err_out)[v] = make_float4(e.x * g.x, e.y * g.y, e.z * g.z, e.w * g.w);
+    }
+    for (int64_t i = (n4 << 2) + t0; i < n; i += stride) {
+        const float g = act_derivative<ACT>(act[i]);
         if (grad_out) grad_out[i] = g;
         err_out[i] = err_in[i] * g;
     }
 }
 
 // out = one-hot(labels): zero fill and scatter in one pass over the output
-__global__ void cn_t_matrix_kernel(const float *__restrict__ labels, float *__restrict__ out, int64_t rows, int64_t n)
+__global__ void cn_t_matrix_kernel(const float *labels, float *out, int64_t rows, int64_t n)
 {
+    cn_pdl_launch_dependents();
+    cn_pdl_wait();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         const int64_t row = i % rows, col = i / rows;
@@ -80,53 +108,99 @@ enum { EW_ADD = 0, EW_SUB = 1, EW_MUL = 2, EW_SCALAR_MUL = 3, EW_GRAD_RELU = 4, 
        EW_ABS = 7, EW_DIV = 8, EW_SCALAR_ADD = 9, EW_SQUARE = 10 };
 
 template <int OP>
-__global__ void cn_ew_kernel(const float *__restrict__ A, const float *__restrict__ B, float s, float *__restrict__ out, int64_t n)
+__device__ __forceinline__ float ew_op(float a, float b, float s)
 {
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const float a = A[i];
-        float r;
-        if (OP == EW_ADD) r = a + B[i];
-        else if (OP == EW_SUB) r = a - B[i];
-        else if (OP == EW_MUL) r = a * B[i];
-        else if (OP == EW_SCALAR_MUL) r = a * s;
-        else if (OP == EW_GRAD_RELU) r = a > 0.0f ? 1.0f : 0.0f;
-        else if (OP == EW_GRAD_LOGISTIC) r = a * (1.0f - a);
-        else if (OP == EW_ABS) r = fabsf(a);
-        else if (OP == EW_DIV) r = fdividef(a, B[i]);   // kDiv divides with fdividef (source/clusterKernels.cu:341-348)
-        else if (OP == EW_SCALAR_ADD) r = a + s;
-        else if (OP == EW_SQUARE) r = powf(a, 2.0f);    // kSquare (source/clusterKernels.cu:420-427)
-        else r = (a > 0.0f && a < 1.0f) ? 1.0f : 0.0f;
-        out[i] = r;
+    if (OP == EW_ADD) return a + b;
+    if (OP == EW_SUB) return a - b;
+    if (OP == EW_MUL) return a * b;
+    if (OP == EW_SCALAR_MUL) return a * s;
+    if (OP == EW_GRAD_RELU) return act_derivative<CN_ACT_RELU>(a);
+    if (OP == EW_GRAD_LOGISTIC) return act_derivative<CN_ACT_LOGISTIC>(a);
+    if (OP == EW_ABS) return fabsf(a);
+    if (OP == EW_DIV) return fdividef(a, b);   // kDiv divides with fdividef (source/clusterKernels.cu:341-348)
+    if (OP == EW_SCALAR_ADD) return a + s;
+    if (OP == EW_SQUARE) return a * a;         // kSquare calls powf(a, 2) (source/clusterKernels.cu:420-427): the product is its correctly rounded value
+    return act_derivative<CN_ACT_DOUBLE_RELU>(a);
+}
+
+template <int OP>
+__global__ void __launch_bounds__(256)
+cn_ew_kernel(const float *A, const float *B, float s, float *out, int64_t n, int64_t n4)
+{
+    constexpr bool TWO = OP == EW_ADD || OP == EW_SUB || OP == EW_MUL || OP == EW_DIV;
+    cn_pdl_launch_dependents();
+    cn_pdl_wait();
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x, t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (int64_t v = t0; v < n4; v += stride) {
+        const float4 a = reinterpret_cast<const float4 *>(A)[v];
+        float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (TWO) b = reinterpret_cast<const float4 *>(B)[v];
+        reinterpret_cast<float4 *>(out)[v] = make_float4(ew_op<OP>(a.x, b.x, s), ew_op<OP>(a.y, b.y, s), ew_op<OP>(a.z, b.z, s), ew_op<OP>(a.w, b.w, s));
     }
+    for (int64_t i = (n4 << 2) + t0; i < n; i += stride) out[i] = ew_op<OP>(A[i], TWO ? B[i] : 0.f, s);
 }
 
 // kNesterov_weight_update (source/clusterKernels.cu:1064-1077): g = lr * grad / batch_size; m = momentum * m - g; w -= g
-__global__ void cn_nesterov_kernel(const float *__restrict__ grad, float *__restrict__ w, float *__restrict__ m, float lr, float batch_size,
-                                   float momentum, int64_t n)
+__device__ __forceinline__ void nesterov_step(float grad, float &w, float &m, float lr, float batch_size, float momentum)
 {
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const float g = lr * fdividef(grad[i], batch_size);
-        m[i] = (momentum * m[i]) - g;
-        w[i] -= g;
+    const float g = lr * fdividef(grad, batch_size);
+    m = (momentum * m) - g;
+    w -= g;
+}
+
+__global__ void __launch_bounds__(256)
+cn_nesterov_kernel(const float *grad, float *w, float *m, float lr, float batch_size, float momentum, int64_t n, int64_t n4)
+{
+    cn_pdl_launch_dependents();
+    cn_pdl_wait();
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x, t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (int64_t v = t0; v < n4; v += stride) {
+        const float4 g = reinterpret_cast<const float4 *>(grad)[v];
+        float4 x = reinterpret_cast<const float4 *>(w)[v], q = reinterpret_cast<const float4 *>(m)[v];
+        nesterov_step(g.x, x.x, q.x, lr, batch_size, momentum);
+        nesterov_step(g.y, x.y, q.y, lr, batch_size, momentum);
+        nesterov_step(g.z, x.z, q.z, lr, batch_size, momentum);
+        nesterov_step(g.w, x.w, q.w, lr, batch_size, momentum);
+        reinterpret_cast<float4 *>(m)[v] = q;
+        reinterpret_cast<float4 *>(w)[v] = x;
+    }
+    for (int64_t i = (n4 << 2) + t0; i < n; i += stride) {
+        float x = w[i], q = m[i];
+        nesterov_step(grad[i], x, q, lr, batch_size, momentum);
+        m[i] = q;
+        w[i] = x;
     }
 }
 
-// kRMSprop_with_weight_update: RMS = m*RMS + (1-m)*g^2 ; w -= lr * g / (sqrt(RMS) + 1e-8).  The reference divides with
-// fdividef and squares with powf(g, 2.0f); both are reproduced as written.
+// kRMSprop_with_weight_update: RMS = m*RMS + (1-m)*g^2 ; w -= lr * g / (sqrt(RMS) + 1e-8).  The reference divides with fdividef,
+// reproduced as written, and squares with powf(g, 2.0f), whose correctly rounded value is the product.
 __device__ __forceinline__ void rmsprop_step(float g, float &rms, float &w, float rms_mult, float rec, float lr)
 {
-    const float r = (rms_mult * rms) + (powf(g, 2.0f) * rec);
+    const float r = (rms_mult * rms) + ((g * g) * rec);
     rms = r;
     w -= lr * fdividef(g, sqrtf(r) + 1.0e-08f);
 }
 
-__global__ void cn_rmsprop_kernel(float *__restrict__ RMS, const float *__restrict__ grad, float *__restrict__ w, float rms_mult, float lr, int64_t n)
+// 20 bytes per element.  With one element per thread and powf it took 77 us on 4096 x 4096, against 51 us for the bytes at the
+// measured copy rate.
+__global__ void __launch_bounds__(256)
+cn_rmsprop_kernel(float *RMS, const float *grad, float *w, float rms_mult, float lr, int64_t n, int64_t n4)
 {
+    cn_pdl_launch_dependents();
+    cn_pdl_wait();
     const float rec = 1.0f - rms_mult;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x, t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    for (int64_t v = t0; v < n4; v += stride) {
+        const float4 g = reinterpret_cast<const float4 *>(grad)[v];
+        float4 q = reinterpret_cast<const float4 *>(RMS)[v], x = reinterpret_cast<const float4 *>(w)[v];
+        rmsprop_step(g.x, q.x, x.x, rms_mult, rec, lr);
+        rmsprop_step(g.y, q.y, x.y, rms_mult, rec, lr);
+        rmsprop_step(g.z, q.z, x.z, rms_mult, rec, lr);
+        rmsprop_step(g.w, q.w, x.w, rms_mult, rec, lr);
+        reinterpret_cast<float4 *>(RMS)[v] = q;
+        reinterpret_cast<float4 *>(w)[v] = x;
+    }
+    for (int64_t i = (n4 << 2) + t0; i < n; i += stride) {
         float r = RMS[i], x = w[i];
         rmsprop_step(grad[i], r, x, rms_mult, rec, lr);
         RMS[i] = r;
@@ -153,6 +227,8 @@ cn_decode_sum_multi_kernel(float *__restrict__ grad, const uint8_t *__restrict__
                            float *__restrict__ RMS, float *__restrict__ w, float rms_mult, float lr, int vec_ok)
 {
     extern __shared__ float lut[];   // (segment, rank) x 256
+    cn_pdl_launch_dependents();
+    cn_pdl_wait();
     for (int e = threadIdx.x; e < sp.nseg * nranks * 256; e += blockDim.x) {
         const int sr = e >> 8, c = e & 255, i = c & 127;
         const int seg = sr / nranks, r = sr - seg * nranks;
@@ -218,21 +294,38 @@ cn_decode_sum_multi_kernel(float *__restrict__ grad, const uint8_t *__restrict__
     for (int64_t i = (n4 << 2) + tid0; i < n; i += stride) one(i);
 }
 
-static int ew_grid(const cn_context *ctx, int64_t n)
+// blocks of 256 threads, `per_thread` elements each, at most eight per SM
+static dim3 ew_grid(const cn_context *ctx, int64_t n, int per_thread)
 {
-    int64_t blocks = (n + 255) / 256, cap = (int64_t)ctx->sm_count * 8;
+    const int64_t cap = (int64_t)ctx->sm_count * 8;
+    int64_t blocks = (n + 256 * per_thread - 1) / (256 * per_thread);
     if (blocks < 1) blocks = 1;
-    return (int)(blocks < cap ? blocks : cap);
+    return dim3((unsigned)(blocks < cap ? blocks : cap));
+}
+
+static bool aligned16(const void *a, const void *b = nullptr, const void *c = nullptr, const void *d = nullptr)
+{
+    return (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c | (uintptr_t)d) & 15u) == 0;
+}
+
+template <bool ERROR>
+static int softmax_launch(cn_context *ctx, const float *A, const float *labels, float *prob, float *err, int64_t rows, int64_t cols, void *stream)
+{
+    const int64_t blocks = (rows + SOFTMAX_THREADS - 1) / SOFTMAX_THREADS;
+    const dim3 grid((unsigned)(blocks < 4096 ? blocks : 4096));
+    if (cols <= SOFTMAX_REGS)
+        CN_CUDA(cn_launch_pdl(cn_softmax_kernel<ERROR, true>, grid, SOFTMAX_THREADS, 0, cn_stream(stream), A, labels, prob, err, rows, cols));
+    else
+        CN_CUDA(cn_launch_pdl(cn_softmax_kernel<ERROR, false>, grid, SOFTMAX_THREADS, 0, cn_stream(stream), A, labels, prob, err, rows, cols));
+    cn_count_launch();
+    return CN_OK;
 }
 
 extern "C" int cn_softmax(cn_context *ctx, const float *d_A, float *d_out, int64_t rows, int64_t cols, void *stream)
 {
     CN_REQUIRE(ctx && rows >= 0 && cols >= 0 && (rows * cols == 0 || (d_A && d_out)), CN_ERR_ARG, "cn_softmax: bad argument");
     if (rows * cols == 0) return CN_OK;
-    cn_softmax_kernel<<<(unsigned)((rows + 127) / 128 < 1024 ? (rows + 127) / 128 : 1024), 128, 0, cn_stream(stream)>>>(d_A, d_out, rows, cols);
-    CN_CUDA(cudaGetLastError());
-    cn_count_launch();
-    return CN_OK;
+    return softmax_launch<false>(ctx, d_A, nullptr, d_out, nullptr, rows, cols, stream);
 }
 
 extern "C" int cn_softmax_error(cn_context *ctx, const float *d_A, const float *d_labels, float *d_softmax_out, float *d_error_out,
@@ -241,19 +334,14 @@ extern "C" int cn_softmax_error(cn_context *ctx, const float *d_A, const float *
     CN_REQUIRE(ctx && rows >= 0 && cols >= 0 && (rows * cols == 0 || (d_A && d_labels && d_softmax_out && d_error_out)), CN_ERR_ARG,
                "cn_softmax_error: bad argument");
     if (rows * cols == 0) return CN_OK;
-    cn_softmax_error_kernel<<<(unsigned)((rows + 127) / 128 < 1024 ? (rows + 127) / 128 : 1024), 128, 0, cn_stream(stream)>>>(
-        d_A, d_labels, d_softmax_out, d_error_out, rows, cols);
-    CN_CUDA(cudaGetLastError());
-    cn_count_launch();
-    return CN_OK;
+    return softmax_launch<true>(ctx, d_A, d_labels, d_softmax_out, d_error_out, rows, cols, stream);
 }
 
 extern "C" int cn_create_t_matrix(cn_context *ctx, const float *d_labels, float *d_out, int64_t rows, int64_t cols, void *stream)
 {
     CN_REQUIRE(ctx && rows >= 0 && cols >= 0 && (rows * cols == 0 || (d_labels && d_out)), CN_ERR_ARG, "cn_create_t_matrix: bad argument");
     if (rows * cols == 0) return CN_OK;
-    cn_t_matrix_kernel<<<ew_grid(ctx, rows * cols), 256, 0, cn_stream(stream)>>>(d_labels, d_out, rows, rows * cols);
-    CN_CUDA(cudaGetLastError());
+    CN_CUDA(cn_launch_pdl(cn_t_matrix_kernel, ew_grid(ctx, rows * cols, 1), 256, 0, cn_stream(stream), d_labels, d_out, rows, rows * cols));
     cn_count_launch();
     return CN_OK;
 }
@@ -263,8 +351,8 @@ static int ew_launch(cn_context *ctx, const float *A, const float *B, float s, f
 {
     CN_REQUIRE(ctx && n >= 0 && (n == 0 || (A && out && (!needs_b || B))), CN_ERR_ARG, "elementwise op: bad argument");
     if (n == 0) return CN_OK;
-    cn_ew_kernel<OP><<<ew_grid(ctx, n), 256, 0, cn_stream(stream)>>>(A, B, s, out, n);
-    CN_CUDA(cudaGetLastError());
+    const int64_t n4 = aligned16(A, needs_b ? B : nullptr, out) ? n >> 2 : 0;
+    CN_CUDA(cn_launch_pdl(cn_ew_kernel<OP>, ew_grid(ctx, n, n4 ? 4 : 1), 256, 0, cn_stream(stream), A, B, s, out, n, n4));
     cn_count_launch();
     return CN_OK;
 }
@@ -284,8 +372,9 @@ extern "C" int cn_nesterov_update(cn_context *ctx, const float *d_grad, float *d
 {
     CN_REQUIRE(ctx && n >= 0 && batch_size > 0 && (n == 0 || (d_grad && d_w && d_m)), CN_ERR_ARG, "cn_nesterov_update: bad argument");
     if (n == 0) return CN_OK;
-    cn_nesterov_kernel<<<ew_grid(ctx, n), 256, 0, cn_stream(stream)>>>(d_grad, d_w, d_m, learning_rate, (float)batch_size, momentum, n);
-    CN_CUDA(cudaGetLastError());
+    const int64_t n4 = aligned16(d_grad, d_w, d_m) ? n >> 2 : 0;
+    CN_CUDA(cn_launch_pdl(cn_nesterov_kernel, ew_grid(ctx, n, n4 ? 4 : 1), 256, 0, cn_stream(stream), d_grad, d_w, d_m, learning_rate, (float)batch_size,
+                          momentum, n, n4));
     cn_count_launch();
     return CN_OK;
 }
@@ -306,16 +395,19 @@ extern "C" int cn_mul_activation_gradient(cn_context *ctx, const float *d_error_
 {
     CN_REQUIRE(ctx && n >= 0 && (n == 0 || (d_error_in && d_activation && d_error_out)), CN_ERR_ARG, "cn_mul_activation_gradient: bad argument");
     if (n == 0) return CN_OK;
-    const int grid = ew_grid(ctx, n);
+    const int64_t n4 = aligned16(d_error_in, d_activation, d_gradient_out, d_error_out) ? n >> 2 : 0;
+    const dim3 grid = ew_grid(ctx, n, n4 ? 4 : 1);
+#define CN_MUL_GRAD(ACT) \
+    CN_CUDA(cn_launch_pdl(cn_mul_grad_kernel<ACT>, grid, 256, 0, cn_stream(stream), d_error_in, d_activation, d_gradient_out, d_error_out, n, n4))
     switch (activation) {
-        case CN_ACT_RELU: cn_mul_grad_kernel<CN_ACT_RELU><<<grid, 256, 0, cn_stream(stream)>>>(d_error_in, d_activation, d_gradient_out, d_error_out, n); break;
-        case CN_ACT_LOGISTIC: cn_mul_grad_kernel<CN_ACT_LOGISTIC><<<grid, 256, 0, cn_stream(stream)>>>(d_error_in, d_activation, d_gradient_out, d_error_out, n); break;
-        case CN_ACT_DOUBLE_RELU: cn_mul_grad_kernel<CN_ACT_DOUBLE_RELU><<<grid, 256, 0, cn_stream(stream)>>>(d_error_in, d_activation, d_gradient_out, d_error_out, n); break;
+        case CN_ACT_RELU: CN_MUL_GRAD(CN_ACT_RELU); break;
+        case CN_ACT_LOGISTIC: CN_MUL_GRAD(CN_ACT_LOGISTIC); break;
+        case CN_ACT_DOUBLE_RELU: CN_MUL_GRAD(CN_ACT_DOUBLE_RELU); break;
         default:
             cn_set_error("cn_mul_activation_gradient: no derivative for activation %d (the reference throws 'Unknown unit')", activation);
             return CN_ERR_ARG;
     }
-    CN_CUDA(cudaGetLastError());
+#undef CN_MUL_GRAD
     cn_count_launch();
     return CN_OK;
 }
@@ -325,8 +417,9 @@ extern "C" int cn_rmsprop_update(cn_context *ctx, float *d_rms, const float *d_g
 {
     CN_REQUIRE(ctx && n >= 0 && (n == 0 || (d_rms && d_grad && d_w)), CN_ERR_ARG, "cn_rmsprop_update: bad argument");
     if (n == 0) return CN_OK;
-    cn_rmsprop_kernel<<<ew_grid(ctx, n), 256, 0, cn_stream(stream)>>>(d_rms, d_grad, d_w, rms_multiplier, learning_rate, n);
-    CN_CUDA(cudaGetLastError());
+    const int64_t n4 = aligned16(d_rms, d_grad, d_w) ? n >> 2 : 0;
+    CN_CUDA(cn_launch_pdl(cn_rmsprop_kernel, ew_grid(ctx, n, n4 ? 4 : 1), 256, 0, cn_stream(stream), d_rms, d_grad, d_w, rms_multiplier, learning_rate, n,
+                          n4));
     cn_count_launch();
     return CN_OK;
 }
