@@ -958,15 +958,14 @@ extern "C" int cn_gemm_prepare_create(cn_context *ctx, int64_t M, int64_t K, int
     p->ctx = ctx;
     p->M = M;
     p->K = K;
-    p->Kpad = (K + 31) / 32 * 32;
     p->mode = mode;
-    const size_t plane = (size_t)M * p->Kpad;
-    cudaError_t e = cudaMalloc(&p->hi, plane * sizeof(float) * (mode == CN_GEMM_3XTF32 ? 2 : 1));
+    cn_planes pl;
+    cn_plane_layout(M, K, mode, &pl);
+    cudaError_t e = cudaMalloc(&p->planes, pl.bytes);
     if (e != cudaSuccess) {
         delete p;
         return cn_cuda_fail(e, "cn_gemm_prepare_create");
     }
-    p->lo = mode == CN_GEMM_3XTF32 ? p->hi + plane : nullptr;
     *out = p;
     return CN_OK;
 }
@@ -974,7 +973,7 @@ extern "C" int cn_gemm_prepare_create(cn_context *ctx, int64_t M, int64_t K, int
 extern "C" int cn_gemm_prepare_destroy(cn_prepared *p)
 {
     if (!p) return CN_OK;
-    cudaFree(p->hi);
+    cudaFree(p->planes);
     delete p;
     return CN_OK;
 }
@@ -984,7 +983,7 @@ extern "C" int cn_gemm_prepare(cn_context *ctx, cn_prepared *p, int transA, cons
     CN_REQUIRE(ctx && p && d_A && p->ctx == ctx, CN_ERR_ARG, "cn_gemm_prepare: null argument or a handle of another context");
     CN_REQUIRE(lda >= (transA ? p->K : p->M), CN_ERR_SHAPE, "cn_gemm_prepare: leading dimension smaller than the stored rows");
     if (!ctx->gemm) ctx->gemm = cn_gemm_workspace_new();
-    int st = cn_gemm_tc_split_activations(ctx, transA, p->M, p->K, d_A, lda, p->hi, p->lo, cn_stream(stream));
+    int st = cn_gemm_tc_split_activations(ctx, transA, p->M, p->K, d_A, lda, p->mode, p->planes, cn_stream(stream));
     if (st == CN_OK) p->filled = true;
     return st;
 }
@@ -1000,11 +999,11 @@ extern "C" int cn_dotmpi_prepared_f32(cn_context *ctx, const cn_prepared *p, int
     cn_shard_cols(n_total, rank, G, &start, &cnt);
     // the planes only feed the tensor-core kernel; every rank must be able to take it (the decision is made from the
     // shapes and this rank's W pointer, like the fused gather's)
-    CN_REQUIRE(cnt > 0 && cn_gemm_tc_supported(ctx, 0, 0, p->M, cnt, p->K, p->hi, p->M, d_Wshard, p->K, d_C, p->M), CN_ERR_UNSUPPORTED,
+    CN_REQUIRE(cnt > 0 && cn_gemm_tc_supported(ctx, 0, 0, p->M, cnt, p->K, nullptr, p->M, d_Wshard, p->K, d_C, p->M), CN_ERR_UNSUPPORTED,
                "cn_dotmpi_prepared_f32: this shard is no shape for the tensor-core kernel (empty, or W not 16-byte aligned)");
     if (!ctx->gemm) ctx->gemm = cn_gemm_workspace_new();
     ctx->gemm->prepared = p;   // consumed by the launch inside the call below; the fp32 pointer handed down is a placeholder
-    int st = dotmpi_impl(ctx, 0, p->M, p->K, n_total, p->hi, p->M, d_Wshard, d_C, epi, p->mode, exchange, stream);
+    int st = dotmpi_impl(ctx, 0, p->M, p->K, n_total, reinterpret_cast<const float *>(p->planes), p->M, d_Wshard, d_C, epi, p->mode, exchange, stream);
     ctx->gemm->prepared = nullptr;
     return st;
 }

@@ -4,8 +4,8 @@
 
 enum {
     CN_GEMM_SLOT_MAXOUT = 0,   // full product ahead of an un-fused maxout
-    CN_GEMM_SLOT_ASPLIT = 1,   // activations re-laid K-major as TF32 hi / lo planes
-    CN_GEMM_SLOT_SPLITK = 2,   // per-split partial tiles of a split-K launch
+    CN_GEMM_SLOT_ASPLIT = 1,   // activations re-laid K-major as hi / lo planes with their scales
+    CN_GEMM_SLOT_SPLITK = 2,   // partial tiles of the runs of K blocks of a launch
     CN_GEMM_SLOT_EXCHANGE = 3, // codes + scales of the 8-bit exchange in dotMPI
     CN_GEMM_SLOTS = 4
 };
@@ -22,12 +22,21 @@ struct cn_coded_src {
     int nranks = 1, own_rank = 0;
 };
 
-// The K-major TF32 hi / lo planes of an activation operand, made ahead of the product that consumes them
-// (cn_gemm_prepare): the product's own pre-pass is then skipped.  `hi` holds both planes back to back.
+// Planes of an M x K activation operand, in one allocation: fp16 hi [M][Kp], fp16 lo [M][Kp] (only in the 3x mode), inverse
+// scales [groups of CN_PLANE_GROUP_K k][m_pad] (see cn_gemm_tc.cu).
+#define CN_PLANE_GROUP_K 512
+struct cn_planes {
+    int64_t Kp, m_pad, groups;
+    size_t lo_off, inv_off, bytes;   // lo_off = 0: no low plane
+};
+void cn_plane_layout(int64_t M, int64_t K, int mode, cn_planes *pl);
+
+// The planes of an activation operand made ahead of the product that consumes them (cn_gemm_prepare): the product's own
+// pre-pass is then skipped.
 struct cn_prepared {
     cn_context *ctx = nullptr;
-    float *hi = nullptr, *lo = nullptr;
-    int64_t M = 0, K = 0, Kpad = 0;
+    void *planes = nullptr;
+    int64_t M = 0, K = 0;
     int mode = 0;
     bool filled = false;
 };
@@ -69,8 +78,8 @@ struct cn_peer_out {
 bool cn_gemm_tc_supported(cn_context *ctx, int transA, int transB, int64_t M, int64_t N, int64_t K,
                           const float *A, int64_t lda, const float *B, int64_t ldb, const float *C, int64_t ldc);
 bool cn_gemm_tc_can_fuse_maxout(int level);
-// the activation pre-pass alone, into caller-owned planes (lo == nullptr in the single-pass mode)
-int cn_gemm_tc_split_activations(cn_context *ctx, int transA, int64_t M, int64_t K, const float *A, int64_t lda, float *hi, float *lo,
+// the activation pre-pass alone, into caller-owned planes of cn_plane_layout's size
+int cn_gemm_tc_split_activations(cn_context *ctx, int transA, int64_t M, int64_t K, const float *A, int64_t lda, int mode, void *planes,
                                  cudaStream_t s);
 int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda,
                       const float *B, int64_t ldb, float *C, int64_t ldc, const cn_epilogue *epi, int mode, cudaStream_t s,

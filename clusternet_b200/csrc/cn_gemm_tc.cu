@@ -4,26 +4,36 @@
 // Problem: C (M x N) = A (M x K) . W (K x N), everything fp32 column-major (the reference's device layout),
 // which is the product ClusterNet::dot hands to cublasSgemm (source/clusterNet.cpp:459-461).
 //
+// Operands.  Every fp32 value is split into a high and a low part of 11 significand bits each (the TF32 split), and three
+// products per k-step give fp32-level accuracy: D += Whi.Ahi + Wlo.Ahi + Whi.Alo.  CN_GEMM_TF32 issues only the first.
+// TF32 and fp16 carry the same 11 significand bits, but the tensor cores multiply fp16 at twice the rate and its operands
+// take half the room, so the parts are kept as fp16.  What fp16 lacks is exponent range; that is supplied by a power-of-two
+// scale per row of the operand and segment of at most TC_GROUP_K = 512 k, exact to apply and to remove:
+//   * activations: row m, segment of 512 k: the largest magnitude is brought into [2^14, 2^15);
+//   * weights: column n, accumulation chain (below): the first K block that is not all zero brings its largest magnitude
+//     into [2^13, 2^14); a later block that would leave fp16's range ends the chain early and starts a new one with a new scale.
+// hi = fp16(s x) is exact to 2^-12 |s x|, lo = fp16(s x - hi) to 2^-24 |s x| or 2^-25, whichever is larger.  So every
+// element within a factor 2^-15 of the largest of its segment keeps all 22 bits of the split, and a smaller one has an absolute
+// error below 2^-38 of that largest element: 2^-14 of the last bit the largest element itself has in fp32.
+//
 // Mapping.  A column-major W has its K index contiguous for a fixed column n, i.e. it is a K-major operand with
 // N "rows".  The kernel therefore computes the transposed tile D[n, m] = sum_k W[k, n] * A[m, k]:
 //   * the tcgen05 "A" operand (128 rows = 128 columns n of W) is read from TENSOR MEMORY.  W is streamed from
-//     HBM exactly once as raw fp32 by TMA; four converter warps read each 128 x 32 tile from shared memory,
-//     split every value into TF32 hi = rna(x) and lo = rna(x - hi) in registers and write both planes to TMEM
-//     with tcgen05.st.  No shared-memory traffic is spent on the split and the raw weights never need a
-//     second copy in HBM;
+//     HBM exactly once as raw fp32 by TMA; four converter warps read each 128 x 32 tile from shared memory, scale and split
+//     every value in registers and write both parts to TMEM with tcgen05.st.  No shared-memory traffic is spent on the split
+//     and the raw weights never need a second copy in HBM;
 //   * the tcgen05 "B" operand (UMMA N = 128 rows m of the activations) is read from shared memory.  The
 //     activations are small next to W (M = 128 in the reference's layers), so a pre-pass re-lays them K-major
-//     and pre-split into hi / lo planes once per call; every CTA then pulls 128 x 32 tiles of both planes by TMA;
-//   * three products per k-step give fp32-level accuracy: D += Whi.Ahi + Wlo.Ahi + Whi.Alo ("3xTF32").
-//     CN_GEMM_TF32 issues only the first.
+//     and pre-split into hi / lo planes once per call; every CTA then pulls 128 x 64 tiles of both planes by TMA;
 //   * the accumulator tile lives in TMEM with lane = n and column = m, so in the epilogue one thread owns one
-//     output column n and 32 consecutive rows m: the bias is a per-thread scalar, the stores are contiguous
-//     128-byte runs of the column-major C, and maxout over L consecutive columns is a shuffle across L lanes.
+//     output column n and 128 consecutive rows m: the bias is a per-thread scalar, and maxout over L consecutive columns is a
+//     shuffle across L lanes.
 //
-// Work decomposition.  One CTA per (m tile of 128, group of NT n tiles of 128, K split).  Skinny products have
-// few tiles, so K is split across CTAs; each split leaves its partial tile in scratch and a second, grid-wide
-// kernel adds the partials in split order (a fixed order, so results are reproducible) and runs the epilogue.  Launch order is split-major, which makes the CTAs resident at one time walk the same K
-// range of the activations and share it through L2.
+// Work decomposition.  One persistent CTA per SM; a tile is 128 rows m by NT * 128 columns n.  As many whole tiles as there
+// are full rounds over the SMs are multiplied over all of K by one CTA each (in lockstep along K, so that the activation tiles
+// are shared through L2); the tiles that are left are cut into equal runs of K blocks over all SMs.  A run leaves its partial
+// tile in scratch and a second, grid-wide kernel adds the partial tiles in K order (a fixed order, so results are
+// reproducible) and runs the epilogue.
 //
 // Every wait on an mbarrier is bounded by a clock limit; a wait that runs out sets a status word that the host
 // reads back as CN_ERR_TIMEOUT, lets the other roles drain, frees the tensor memory and returns.
@@ -34,60 +44,124 @@
 
 #define TC_BM 128          // activation rows per CTA = UMMA N
 #define TC_BN 128          // W columns per tile       = UMMA M
-#define TC_BK 32           // fp32 per 128-byte swizzle row
-#define TC_TILE_BYTES (128 * 128)
-#define TC_CHAIN_DEFAULT 16   // K blocks (of 32) accumulated in TMEM before the sum is drained to registers
-#define TC_DRAIN_SLEEP_NS 200   // poll interval of the drain warps while a chain accumulates
+#define TC_WK 32           // k per W block: one 128-byte swizzle row of fp32
+#define TC_AK 64           // k per activation stage: one 128-byte swizzle row of fp16
+#define TC_W_TILE_BYTES (TC_BN * TC_WK * 4)
+#define TC_A_TILE_BYTES (TC_BM * TC_AK * 2)
+#define TC_GROUP_K CN_PLANE_GROUP_K
+#define TC_GROUP_KB (TC_GROUP_K / TC_WK)
+#define TC_DRAIN_SLEEP_NS 100   // poll interval of the drain warps while a chain accumulates
 #define TC_WAIT_LIMIT (6000000000LL)   // clock cycles (~3 s)
 
 template <int NT>
 struct TcCfg {
-    static constexpr int THREADS = 256 + 128 * NT;    // WG0 (producers, MMA), WG1 (converters), NT drain warpgroups
-    // Two shared-memory rings with their own depth: raw W tiles (released by the converters as soon as they have
+    static constexpr int THREADS = 128 + 256 * NT;    // WG0 (producers, MMA), per W tile one converter and one drain warpgroup
+    // Two shared-memory rings with their own depth: raw W blocks (released by the converters as soon as they have
     // been read) and activation hi / lo tiles (released when the MMAs that read them retire).
-    static constexpr int W_STAGES = NT == 1 ? 4 : 3;
-    static constexpr int A_STAGES = NT == 1 ? 4 : 3;
-    static constexpr int W_STAGE_BYTES = NT * TC_TILE_BYTES;
-    static constexpr int A_STAGE_BYTES = 2 * TC_TILE_BYTES;
+    static constexpr int W_STAGES = NT == 1 ? 6 : 3;
+    static constexpr int A_STAGES = 3;
+    static constexpr int W_STAGE_BYTES = NT * TC_W_TILE_BYTES;
+    static constexpr int A_STAGE_BYTES = 2 * TC_A_TILE_BYTES;
     static constexpr int W_RING = 0;
     static constexpr int A_RING = W_STAGES * W_STAGE_BYTES;
     static constexpr int RING_BYTES = A_RING + A_STAGES * A_STAGE_BYTES;
-    static constexpr int TMEM_STAGES = NT == 1 ? 4 : 2;
+    static constexpr int TMEM_STAGES = 4;
     static constexpr int ACC_BUFS = NT == 1 ? 2 : 1;  // accumulators per W tile
     static constexpr int ACC_COL = 0;                 // NT * ACC_BUFS accumulators of 128 columns
-    static constexpr int A_COL = NT * ACC_BUFS * TC_BM;   // then TMEM_STAGES x NT x (32 hi + 32 lo) columns
-    static constexpr int A_STAGE_COLS = NT * 64;
-    static constexpr int SMEM_BYTES = RING_BYTES + 1024 /*align*/ + 512 /*barriers*/;
-    // register budgets after the warpgroups re-balance (multiples of 8); launch value is 65536 / THREADS
-    static constexpr int REGS_WG0 = 88;
-    static constexpr int REGS_CONV = 72;
-    static constexpr int REGS_DRAIN = NT == 1 ? 232 : 176;
+    static constexpr int OP_COL = NT * ACC_BUFS * TC_BM;   // then TMEM_STAGES x NT x 2 k-steps x (8 hi + 8 lo) columns
+    static constexpr int OP_STAGE_COLS = NT * 32;
+    static_assert(OP_COL + TMEM_STAGES * OP_STAGE_COLS <= 512, "tensor memory");
+    // Scales of the W rows, one slot per W block: the drain warps read the slot of a chain's last block.  The converters
+    // run at most TMEM_STAGES blocks ahead of the MMAs, and the MMAs at most ACC_BUFS - 1 chains ahead of the drain.
+    static constexpr int WS_SLOTS = NT == 1 ? 32 : 8;
+    static_assert(WS_SLOTS > TMEM_STAGES + (ACC_BUFS - 1) * TC_GROUP_KB, "a scale must outlive its chain");
+    static constexpr int WS_OFF = RING_BYTES;                              // [WS_SLOTS][NT][128] floats
+    static constexpr int AS_OFF = WS_OFF + WS_SLOTS * NT * TC_BN * 4;      // [2][NT][128] floats
+    static constexpr int BRK_OFF = AS_OFF + 2 * NT * TC_BM * 4;            // [TMEM_STAGES][NT] words of four bytes, one per converter warp
+    static constexpr int INFO_OFF = BRK_OFF + TMEM_STAGES * NT * 4;        // [NT][ACC_BUFS] pairs of words
+    static constexpr int BAR_OFF = (INFO_OFF + NT * ACC_BUFS * 8 + 7) & ~7;
+    static constexpr int BARS = 2 * (W_STAGES + A_STAGES + NT * TMEM_STAGES + NT * ACC_BUFS);
+    static constexpr int HOLD_OFF = BAR_OFF + BARS * 8;                    // tensor-memory base, abort flag
+    static constexpr int SMEM_BYTES = HOLD_OFF + 16 + 1024 /*align*/;
+    static_assert(SMEM_BYTES <= 232448, "shared memory");
+    // register budgets after the warpgroups re-balance: multiples of 8, their sum over the warpgroups at most what the launch has
+    // (NT = 2: 5 x 96, NT = 1: 3 x 168)
+    static constexpr int REGS_WG0 = NT == 1 ? 88 : 48;
+    static constexpr int REGS_CONV = NT == 1 ? 104 : 48;
+    static constexpr int REGS_DRAIN = NT == 1 ? 232 : 168;
+    static_assert(REGS_WG0 + NT * (REGS_CONV + REGS_DRAIN) <= (1 + 2 * NT) * (65536 / THREADS / 8 * 8), "registers");
 };
 
 struct TcParams {
-    int64_t M, N, K;
+    int64_t M, N;
     float *C;
     int64_t ldc;
     const float *bias;
     int act;
     int maxout_level;
     float *argmax;
-    int64_t tiles_n;        // groups of NT*128 columns
-    int64_t tiles_m;
-    int splits;
-    int kb_per_split;       // K blocks (of 32) per split
-    int kb_total;
-    int chain_kb;           // K blocks accumulated in TMEM before the sum is drained to registers
-    float *partials;        // [tile * NT + w][split][128 n][128 m]: every partial tile laid out like C
+    int tiles_n;            // groups of NT*128 columns
+    int tiles_m;
+    int full_tiles;         // tiles [0, full_tiles): all of K by one CTA; the others are cut into runs over tail_ctas CTAs
+    int tail_ctas;
+    int kb_total;           // K blocks of 32
+    int chain_mask;         // K blocks per accumulation chain - 1 (a power of two, at most TC_GROUP_KB)
+    const float *a_inv;     // [group of 512 k][m_pad] inverse scales of the activation rows
+    int64_t m_pad;
+    float *partials;        // [slot][w][32 quads of m][128 n] float4: slot = CTA + tile - full_tiles
     unsigned int *status;
-    // fused all-gather: peer copies of the C window (same leading dimension), flags the peers raise when ready
+    int w_ready;            // nothing before the pre-pass still writes W: it may be loaded before the pre-pass has finished
+    // fused all-gather: the peers are told that this rank's C may be overwritten; the tiles go to them in the reduction
     int npeers;
-    float *peerC[CN_MAX_PEERS];
-    const unsigned int *ready;
     unsigned int *const *peer_flags;
     int nranks;
     int my_rank;
     unsigned int epoch;
+};
+
+// One run of K blocks of one tile.
+struct TcSeg {
+    int tile, k0, k1;
+    int slot;       // where the partial tile goes; -1: the run is the whole tile and is finished in place
+};
+
+// The runs of CTA `cta`, in order.  All roles of a CTA walk the same list.
+struct TcWalk {
+    int t;
+    int64_t pos, end;
+    __device__ __forceinline__ explicit TcWalk(const TcParams &p)
+    {
+        t = blockIdx.x;
+        pos = end = 0;
+        if ((int)blockIdx.x < p.tail_ctas) {
+            const int64_t total = (int64_t)(p.tiles_n * p.tiles_m - p.full_tiles) * p.kb_total;
+            pos = total * blockIdx.x / p.tail_ctas;
+            end = total * (blockIdx.x + 1) / p.tail_ctas;
+        }
+    }
+    __device__ __forceinline__ bool next(const TcParams &p, TcSeg &s)
+    {
+        if (t < p.full_tiles) {
+            s.tile = t;
+            s.k0 = 0;
+            s.k1 = p.kb_total;
+            s.slot = -1;
+            t += gridDim.x;
+            return true;
+        }
+        if (pos < end) {
+            const int r = (int)(pos / p.kb_total);
+            s.k0 = (int)(pos - (int64_t)r * p.kb_total);
+            const int64_t left = end - pos;
+            const int room = p.kb_total - s.k0;
+            s.k1 = s.k0 + (left < room ? (int)left : room);
+            s.tile = p.full_tiles + r;
+            s.slot = blockIdx.x + r;
+            pos += s.k1 - s.k0;
+            return true;
+        }
+        return false;
+    }
 };
 
 // ---------------------------------------------------------------------------------------------- PTX wrappers
@@ -115,11 +189,34 @@ __device__ __forceinline__ uint32_t mbar_try(uint32_t bar, uint32_t parity)
         : "=r"(done) : "r"(bar), "r"(parity) : "memory");
     return done;
 }
+// Shared-memory accesses by 32-bit address (half the registers of generic pointers).
+__device__ __forceinline__ float4 lds4(uint32_t a)
+{
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ float lds1(uint32_t a)
+{
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint32_t lds1u(uint32_t a)
+{
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void sts1(uint32_t a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory"); }
+__device__ __forceinline__ void sts1u(uint32_t a, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+__device__ __forceinline__ void sts1b(uint32_t a, uint32_t v) { asm volatile("st.shared.u8 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
+
 // Bounded wait.  Returns false when the limit ran out or another role already gave up.
 // SLEEP_NS > 0 parks the warp between polls: used by roles that wait for a long time (the drain warps sit out a
 // whole accumulation chain) so that their polling does not take issue slots from the converter and MMA warps.
 template <int SLEEP_NS = 0>
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int *abort_flag, unsigned int *status, unsigned int code)
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t abort_flag, unsigned int *status, unsigned int code)
 {
     if (mbar_try(bar, parity)) return true;
     const long long t0 = clock64();
@@ -127,9 +224,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
         if (SLEEP_NS > 0) __nanosleep(SLEEP_NS);
         if (mbar_try(bar, parity)) return true;
         if ((it & 63u) == 0u) {
-            if (*abort_flag) return false;
+            if (lds1u(abort_flag) != 0u) return false;
             if (clock64() - t0 > TC_WAIT_LIMIT) {
-                *abort_flag = 1;
+                sts1u(abort_flag, 1u);
                 atomicMax(status, code);
                 return false;
             }
@@ -152,7 +249,7 @@ __device__ __forceinline__ void tc_commit(uint32_t bar)
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
-// D[tmem] (+)= A[tmem] * B[smem desc]; A: 128 lanes x 8 columns of TF32, B: 128 x 8 K-major TF32 tile.
+// D[tmem] (+)= A[tmem] * B[smem desc]; A: 128 lanes x 16 fp16 (two per column: 8 columns), B: 128 x 16 K-major fp16 tile.
 // The descriptor travels as two 32-bit halves so that stepping along K is a 32-bit add on the low half.
 __device__ __forceinline__ void tc_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_desc_lo, uint32_t b_desc_hi, uint32_t idesc, uint32_t accumulate)
 {
@@ -160,38 +257,25 @@ __device__ __forceinline__ void tc_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint
         "{\n\t.reg .pred p;\n\t.reg .b64 bd;\n\t"
         "setp.ne.b32 p, %5, 0;\n\t"
         "mov.b64 bd, {%2, %3};\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], bd, %4, p;\n\t}"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], bd, %4, p;\n\t}"
         ::"r"(d_tmem), "r"(a_tmem), "r"(b_desc_lo), "r"(b_desc_hi), "r"(idesc), "r"(accumulate) : "memory");
 }
 
-#define TC_R32(a) \
-    a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], a[8], a[9], a[10], a[11], a[12], a[13], a[14], a[15], a[16], a[17], \
-    a[18], a[19], a[20], a[21], a[22], a[23], a[24], a[25], a[26], a[27], a[28], a[29], a[30], a[31]
-
-__device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&r)[32])
+__device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16])
 {
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, "
-        "%24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr) : "memory");
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-__device__ __forceinline__ void tc_st32(uint32_t taddr, const uint32_t (&r)[32])
+__device__ __forceinline__ void tc_st8(uint32_t taddr, const uint32_t (&r)[16])
 {
     asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, "
-        "%25, %26, %27, %28, %29, %30, %31, %32};"
-        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-          "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]),
-          "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]),
-          "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+        "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
         : "memory");
 }
 __device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t (&r)[16])
@@ -204,15 +288,7 @@ __device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t (&r)[16])
 }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// fp32 -> TF32 (10 mantissa bits kept, low 13 bits zero), round to nearest with ties away from zero: add half a
-// TF32 ulp to the magnitude bits and truncate.  Same result as cvt.rna.tf32.f32 for finite inputs, but two full-rate
-// integer operations; the cvt form issues at a fraction of that rate and made the converter warps the bottleneck.
-__device__ __forceinline__ uint32_t to_tf32(float x)
-{
-    return (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-}
-
-// Shared-memory matrix descriptor of a K-major tile whose rows are 128 bytes (32 fp32) with the 128-byte
+// Shared-memory matrix descriptor of a K-major tile whose rows are 128 bytes (64 fp16) with the 128-byte
 // swizzle TMA applies: 8-row groups are 1024 bytes apart (stride byte offset), the leading byte offset is
 // unused for swizzled K-major layouts, version field 1 (sm_100), layout type 2 (128-byte swizzle).
 __device__ __forceinline__ uint64_t make_kmajor_sw128_desc(uint32_t smem_addr)
@@ -226,529 +302,646 @@ __device__ __forceinline__ uint64_t make_kmajor_sw128_desc(uint32_t smem_addr)
     return d;
 }
 
-// kind::tf32 instruction descriptor: D fp32 (bits 4-5 = 1), A and B TF32 (format 2 at bits 7-9 and 10-12),
+// kind::f16 instruction descriptor: D fp32 (bits 4-5 = 1), A and B fp16 (format 0 at bits 7-9 and 10-12),
 // both operands K-major (bits 15, 16 = 0), N >> 3 at bits 17-22, M >> 4 at bits 24-28.
-__host__ __device__ constexpr uint32_t make_idesc_tf32(int m, int n)
+__host__ __device__ constexpr uint32_t make_idesc_f16(int m, int n)
 {
-    return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+    return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
+
+// ------------------------------------------------------------------------------------------------------- split
+// Power of two that brings a magnitude with these bits into [2^EXP, 2^(EXP+1)), and its inverse; both are normal numbers.
+// Zero and non-finite magnitudes keep the scale 1 (a non-finite element makes every sum it enters non-finite anyway).
+template <int EXP>
+__device__ __forceinline__ void tc_scale(uint32_t amax_bits, float &sc, float &inv)
+{
+    const int e = (int)(amax_bits >> 23);
+    int b = 254 + EXP - e;
+    if (b > 253) b = 253;
+    if (amax_bits == 0u || e == 255) b = 127;
+    sc = __uint_as_float((uint32_t)b << 23);
+    inv = __uint_as_float((uint32_t)(254 - b) << 23);
+}
+#define TC_A_EXP 14
+#define TC_W_EXP 13
+
+// Two floats in one 64-bit register pair, as the packed fp32 instructions take them.
+__device__ __forceinline__ uint64_t tc_pack2(float a, float b)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void tc_unpack2(uint64_t r, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r)); }
+__device__ __forceinline__ uint64_t tc_mul2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t tc_fma2(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// Two scaled values -> packed fp16 high parts, and (LO) packed fp16 low parts: lo = fp16(y - hi), the difference being exact.
+// Measured on registers with two warps per scheduler: 10 issue cycles per pair, 12 with the mixed-precision subtraction
+// (sub.f32.f16) in place of the two conversions back and the packed one.
+template <bool LO>
+__device__ __forceinline__ void tc_split2(uint64_t y, uint32_t &hi, uint32_t &lo)
+{
+    float y0, y1;
+    tc_unpack2(y, y0, y1);
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(y1), "f"(y0));
+    if (LO) {
+        float h0, h1;
+        asm("{\n\t.reg .b16 a, b;\n\t"
+            "mov.b32 {a, b}, %2;\n\t"
+            "cvt.f32.f16 %0, a;\n\t"
+            "cvt.f32.f16 %1, b;\n\t}"
+            : "=f"(h0), "=f"(h1) : "r"(hi));
+        uint64_t d;
+        asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(y), "l"(tc_pack2(-h0, -h1)));
+        float d0, d1;
+        tc_unpack2(d, d0, d1);
+        asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(d1), "f"(d0));
+    }
 }
 
 // ------------------------------------------------------------------------------------------ activation pre-pass
-// A (M x K, column-major, lda) -> planes hi, lo : [M][Kpad] with k contiguous; k in [K, Kpad) is zero.
-__global__ void __launch_bounds__(256)
-cn_act_split_kernel(const float *__restrict__ A, int64_t lda, int64_t M, int64_t K, int64_t Kpad,
-                    float *__restrict__ hi, float *__restrict__ lo, int64_t tiles_k)
-{
-    __shared__ float tile[32][33];
-    const int64_t tm = blockIdx.x / tiles_k, tk = blockIdx.x % tiles_k;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int64_t m_in = tm * 32 + tx;
-#pragma unroll
-    for (int j = ty; j < 32; j += 8) {
-        const int64_t k = tk * 32 + j;
-        tile[j][tx] = (m_in < M && k < K) ? A[m_in + k * lda] : 0.0f;
-    }
-    __syncthreads();
-    const int64_t k_out = tk * 32 + tx;
-#pragma unroll
-    for (int j = ty; j < 32; j += 8) {
-        const int64_t m = tm * 32 + j;
-        if (m < M && k_out < Kpad) {
-            const float x = tile[tx][j];
-            const uint32_t h = to_tf32(x);
-            hi[m * Kpad + k_out] = __uint_as_float(h);
-            if (lo) lo[m * Kpad + k_out] = __uint_as_float(to_tf32(x - __uint_as_float(h)));
-        }
-    }
-}
+// A (M x K) -> planes hi, lo: [M][Kp] fp16 with k contiguous, k in [K, Kp) zero, and the inverse scales a_inv[group][m_pad].
+// One CTA per 16 rows and group of 512 k.  Bound by latency for a layer's activations and by memory otherwise: 4 bytes read
+// and 4 written per element.  CODED: the consumer-side half of the 8-bit exchange.  The activations arrive as gathered codes
+// (column-major like the fp32 matrix; column block r was coded by rank r with scale scales[r]) and are decoded here, inside
+// the pre-pass of the GEMM that consumes them, instead of being written out as fp32 first.  This rank's own block is taken
+// from its exact fp32 values.  Decode table as kDecompression_8bit builds it (source/clusterKernels.cu:1141-1152).
+struct ActCoded {
+    const uint8_t *codes;
+    const float *scales, *tbl, *own_fp32;
+    int own_rank, nranks;
+};
+#define ACT_ROWS 16
+#define ACT_PITCH (ACT_ROWS + 1)
 
-// The consumer-side half of the 8-bit exchange: the activations arrive as gathered codes (column-major like the fp32
-// matrix; column block r was coded by rank r with scale scales[r]) and are decoded here, inside the pre-pass of the GEMM
-// that consumes them, instead of being written out as fp32 first.  This rank's own block is taken from its exact fp32
-// values.  Decode table as kDecompression_8bit builds it (source/clusterKernels.cu:1141-1152).
+template <bool CODED>
 __global__ void __launch_bounds__(256)
-cn_act_split_coded_kernel(const uint8_t *__restrict__ codes, const float *__restrict__ scales, const float *__restrict__ g_tbl,
-                          const float *__restrict__ own_fp32, int own_rank, int nranks, int64_t M, int64_t K, int64_t Kpad,
-                          float *__restrict__ hi, float *__restrict__ lo, int64_t tiles_k)
+cn_act_planes_kernel(const float *A, int64_t lda, int64_t M, int64_t K, int64_t Kp, uint16_t *hi, uint16_t *lo, float *a_inv, int64_t m_pad,
+                     const ActCoded cd)
 {
-    __shared__ float tile[32][33];
-    extern __shared__ float lut[];   // nranks x 256
-    for (int e = threadIdx.x; e < nranks * 256; e += blockDim.x) {
-        const int r = e >> 8, c = e & 255, i = c & 127;
-        const float p = scales[r];
-        float v;
-        if (i < CN_CODEBOOK_N) {
-            v = __fmul_rn(g_tbl[i], p);
-            if (c >= 128) v = -v;
-        } else {
-            v = (c == 255) ? -p : p;
+    __shared__ float tile[TC_GROUP_K * ACT_PITCH];
+    __shared__ uint32_t red[16][ACT_ROWS];
+    __shared__ float s_sc[ACT_ROWS];
+    extern __shared__ float lut[];   // CODED: nranks x 256
+    const int tid = threadIdx.x;
+    // wait first, then release the product: it may then rely on everything before this pass having finished, and start on W
+    cn_pdl_wait();
+    cn_pdl_launch_dependents();
+    if (CODED) {
+        for (int e = tid; e < cd.nranks * 256; e += 256) {
+            const int r = e >> 8, c = e & 255, i = c & 127;
+            const float p = cd.scales[r];
+            float v;
+            if (i < CN_CODEBOOK_N) {
+                v = __fmul_rn(cd.tbl[i], p);
+                if (c >= 128) v = -v;
+            } else {
+                v = (c == 255) ? -p : p;
+            }
+            lut[e] = v;
         }
-        lut[e] = v;
+        __syncthreads();
+    }
+    const int64_t split = CODED ? K / cd.nranks : 0;
+    const int64_t m_blocks = m_pad / ACT_ROWS;
+    const int64_t g = blockIdx.x / m_blocks, m0 = (blockIdx.x - g * m_blocks) * ACT_ROWS, k0 = g * TC_GROUP_K;
+    {
+        const int ml = tid & 15, kl = tid >> 4;
+        const int64_t m = m0 + ml;
+        uint32_t amax = 0u;
+#pragma unroll 8
+        for (int j = 0; j < TC_GROUP_K / 16; ++j) {
+            const int kk = j * 16 + kl;
+            const int64_t k = k0 + kk;
+            float x = 0.0f;
+            if (m < M && k < K) {
+                if (CODED) {
+                    int r = split > 0 ? (int)(k / split) : cd.nranks - 1;
+                    if (r > cd.nranks - 1) r = cd.nranks - 1;
+                    if (r == cd.own_rank && cd.own_fp32) x = cd.own_fp32[m + (k - split * cd.own_rank) * M];
+                    else x = lut[(r << 8) + cd.codes[m + k * M]];
+                } else {
+                    x = A[m + k * lda];
+                }
+            }
+            tile[kk * ACT_PITCH + ml] = x;
+            amax = max(amax, __float_as_uint(x) & 0x7fffffffu);
+        }
+        red[kl][ml] = amax;
     }
     __syncthreads();
-    const int64_t split = K / nranks;
-    const int64_t tm = blockIdx.x / tiles_k, tk = blockIdx.x % tiles_k;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int64_t m_in = tm * 32 + tx;
+    if (tid < ACT_ROWS) {
+        uint32_t amax = 0u;
 #pragma unroll
-    for (int j = ty; j < 32; j += 8) {
-        const int64_t k = tk * 32 + j;
-        float x = 0.0f;
-        if (m_in < M && k < K) {
-            int r = split > 0 ? (int)(k / split) : nranks - 1;
-            if (r > nranks - 1) r = nranks - 1;
-            if (r == own_rank && own_fp32) x = own_fp32[m_in + (k - split * own_rank) * M];
-            else x = lut[(r << 8) + codes[m_in + k * M]];
-        }
-        tile[j][tx] = x;
+        for (int j = 0; j < 16; ++j) amax = max(amax, red[j][tid]);
+        float sc, inv;
+        tc_scale<TC_A_EXP>(amax, sc, inv);
+        s_sc[tid] = sc;
+        a_inv[g * m_pad + m0 + tid] = inv;
     }
     __syncthreads();
-    const int64_t k_out = tk * 32 + tx;
+    // eight consecutive k per item; a warp covers 8 rows x 32 k (conflict-free reads, 64 contiguous bytes per row)
+    const int lane = tid & 31, warp = tid >> 5;
 #pragma unroll
-    for (int j = ty; j < 32; j += 8) {
-        const int64_t m = tm * 32 + j;
-        if (m < M && k_out < Kpad) {
-            const float x = tile[tx][j];
-            const uint32_t h = to_tf32(x);
-            hi[m * Kpad + k_out] = __uint_as_float(h);
-            if (lo) lo[m * Kpad + k_out] = __uint_as_float(to_tf32(x - __uint_as_float(h)));
+    for (int it = 0; it < 4; ++it) {
+        const int ml = (it & 1) * 8 + (lane & 7), kk = ((warp + 8 * (it >> 1)) * 4 + (lane >> 3)) * 8;
+        const int64_t m = m0 + ml, k = k0 + kk;
+        if (m < M && k < Kp) {
+            const float sc = s_sc[ml];
+            uint32_t h[4], l[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const float y0 = tile[(kk + 2 * e) * ACT_PITCH + ml] * sc, y1 = tile[(kk + 2 * e + 1) * ACT_PITCH + ml] * sc;
+                if (lo) tc_split2<true>(tc_pack2(y0, y1), h[e], l[e]);
+                else tc_split2<false>(tc_pack2(y0, y1), h[e], l[e]);
+            }
+            *reinterpret_cast<uint4 *>(hi + m * Kp + k) = make_uint4(h[0], h[1], h[2], h[3]);
+            if (lo) *reinterpret_cast<uint4 *>(lo + m * Kp + k) = make_uint4(l[0], l[1], l[2], l[3]);
         }
     }
 }
 
 // Same planes for a transposed activation operand: op(A)(m, k) = A[k + m * lda] is already K-major (this is also what
-// a row-major M x K batch looks like), so this is a copy-and-split: four consecutive k per thread, 16-byte loads and
-// stores when the row pitch and the base allow, one block row per m.
+// a row-major M x K batch looks like): one warp per row and group, sixteen k per lane, 16-byte loads when the row pitch and
+// the base allow.
 __global__ void __launch_bounds__(256)
-cn_act_split_t_kernel(const float *__restrict__ A, int64_t lda, int64_t M, int64_t K, int64_t Kpad,
-                      float *__restrict__ hi, float *__restrict__ lo, int vec_ok)
+cn_act_planes_t_kernel(const float *A, int64_t lda, int64_t M, int64_t K, int64_t Kp, uint16_t *hi, uint16_t *lo, float *a_inv, int64_t m_pad,
+                       int vec_ok)
 {
-    const int64_t k4 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
-    if (k4 >= Kpad) return;
-    for (int64_t m = blockIdx.y; m < M; m += gridDim.y) {
-        const float *src = A + m * lda + k4;
-        float x[4];
-        if (vec_ok && k4 + 3 < K) {
-            const float4 v = __ldg(reinterpret_cast<const float4 *>(src));
-            x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+    const int lane = threadIdx.x & 31;
+    const int64_t m_blocks = m_pad / 8;
+    const int64_t g = blockIdx.x / m_blocks, m = (blockIdx.x - g * m_blocks) * 8 + (threadIdx.x >> 5);
+    cn_pdl_wait();
+    cn_pdl_launch_dependents();   // after the wait: see cn_act_planes_kernel
+    if (m >= M) return;
+    const float *src = A + m * lda;
+    float x[16];
+    uint32_t amax = 0u;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int64_t k = g * TC_GROUP_K + 128 * j + 4 * lane;
+        if (vec_ok && k + 3 < K) {
+            const float4 v = *reinterpret_cast<const float4 *>(src + k);
+            x[4 * j] = v.x; x[4 * j + 1] = v.y; x[4 * j + 2] = v.z; x[4 * j + 3] = v.w;
         } else {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) x[e] = (k4 + e < K) ? src[e] : 0.0f;
+            for (int e = 0; e < 4; ++e) x[4 * j + e] = (k + e < K) ? src[k + e] : 0.0f;
         }
-        uint32_t h[4], l[4];
+    }
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            h[e] = to_tf32(x[e]);
-            l[e] = to_tf32(x[e] - __uint_as_float(h[e]));
+    for (int e = 0; e < 16; ++e) amax = max(amax, __float_as_uint(x[e]) & 0x7fffffffu);
+    amax = __reduce_max_sync(0xffffffffu, amax);
+    float sc, inv;
+    tc_scale<TC_A_EXP>(amax, sc, inv);
+    if (lane == 0) a_inv[g * m_pad + m] = inv;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int64_t k = g * TC_GROUP_K + 128 * j + 4 * lane;
+        if (k >= Kp) continue;   // Kp is a multiple of 64
+        uint32_t h0, h1, l0 = 0u, l1 = 0u;
+        if (lo) {
+            tc_split2<true>(tc_pack2(x[4 * j] * sc, x[4 * j + 1] * sc), h0, l0);
+            tc_split2<true>(tc_pack2(x[4 * j + 2] * sc, x[4 * j + 3] * sc), h1, l1);
+            *reinterpret_cast<uint2 *>(lo + m * Kp + k) = make_uint2(l0, l1);
+        } else {
+            tc_split2<false>(tc_pack2(x[4 * j] * sc, x[4 * j + 1] * sc), h0, l0);
+            tc_split2<false>(tc_pack2(x[4 * j + 2] * sc, x[4 * j + 3] * sc), h1, l1);
         }
-        const int64_t o = m * Kpad + k4;   // Kpad is a multiple of 32 and the planes are 256-byte aligned
-        *reinterpret_cast<uint4 *>(hi + o) = make_uint4(h[0], h[1], h[2], h[3]);
-        if (lo) *reinterpret_cast<uint4 *>(lo + o) = make_uint4(l[0], l[1], l[2], l[3]);
+        *reinterpret_cast<uint2 *>(hi + m * Kp + k) = make_uint2(h0, h1);
     }
 }
 
 // -------------------------------------------------------------------------------------------------- main kernel
+// Four consecutive k of one row of a 128 x 32 W tile (chunk c of 8).
+// TRANSB: the weight operand is stored transposed (N x K column-major, n contiguous).  Its tiles arrive in shared
+// memory as [32 k][128 n] without swizzle and are read column-wise (conflict-free: consecutive lanes read consecutive n).
+// `base` is the address tc_row_base gives.
+template <bool TRANSB>
+__device__ __forceinline__ uint32_t tc_row_base(uint32_t tile, int row)
+{
+    // 16-byte chunk c of row r sits at chunk position c ^ (r & 7) under the 128-byte swizzle (tiles are 1024-byte aligned)
+    return TRANSB ? tile + row * 4 : tile + row * 128 + ((row & 7) << 4);
+}
+template <bool TRANSB>
+__device__ __forceinline__ float4 tc_read4(uint32_t base, int c)
+{
+    if (TRANSB)
+        return make_float4(lds1(base + (4 * c) * (TC_BN * 4)), lds1(base + (4 * c + 1) * (TC_BN * 4)), lds1(base + (4 * c + 2) * (TC_BN * 4)),
+                           lds1(base + (4 * c + 3) * (TC_BN * 4)));
+    return lds4(base ^ (c << 4));
+}
+
+// One k-step (16 consecutive k of column n) of one row, scaled by sc -> hl[0..7] packed high parts, hl[8..15] packed low parts.
+// Returns the running packed largest |high part|: a half equal to 0x7c00 means that a value left fp16's range.
+template <bool MODE3X, bool TRANSB>
+__device__ __forceinline__ void tc_convert_step(uint32_t base, int step, uint64_t sc2, uint32_t (&hl)[16], uint32_t &top)
+{
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const float4 v = tc_read4<TRANSB>(base, step * 4 + c);
+        tc_split2<MODE3X>(tc_mul2(tc_pack2(v.x, v.y), sc2), hl[2 * c], hl[8 + 2 * c]);
+        tc_split2<MODE3X>(tc_mul2(tc_pack2(v.z, v.w), sc2), hl[2 * c + 1], hl[8 + 2 * c + 1]);
+        asm("max.xorsign.abs.f16x2 %0, %0, %1;" : "+r"(top) : "r"(hl[2 * c]));
+        asm("max.xorsign.abs.f16x2 %0, %0, %1;" : "+r"(top) : "r"(hl[2 * c + 1]));
+    }
+}
+
+template <bool TRANSB>
+__device__ __forceinline__ uint32_t tc_row_amax(uint32_t base)
+{
+    uint32_t amax = 0u;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        const float4 v = tc_read4<TRANSB>(base, c);
+        amax = max(max(amax, __float_as_uint(v.x) & 0x7fffffffu), max(__float_as_uint(v.y) & 0x7fffffffu, __float_as_uint(v.z) & 0x7fffffffu));
+        amax = max(amax, __float_as_uint(v.w) & 0x7fffffffu);
+    }
+    return amax;
+}
+
 // Warp roles (warpgroups of 4 warps so that register budgets can be moved between them):
 //   WG0  warp 0: TMA producer for W, warp 1: MMA issuer of W tile 0 + TMEM owner, warp 2: TMA producer for the
 //        activations, warp 3: MMA issuer of W tile 1 (NT == 2)
-//   WG1  warps 4-7:  converters (raw W tile in shared memory -> TF32 hi / lo planes in TMEM)
-//   WG2  warps 8-11: accumulator drain + epilogue of W tile 0
-//   WG3  warps 12-15 (NT == 2 only): the same for W tile 1
+//   then one warpgroup of converters per W tile (raw W block in shared memory -> scaled fp16 hi / lo parts in TMEM)
+//   and one warpgroup for accumulator drain + epilogue per W tile.
+// The two W tiles of a CTA share the W and activation rings and are otherwise independent of each other.  One converter
+// warpgroup for both tiles was short of registers (their spills went through the shared-memory pipe) and of warps to hide
+// the latency of its conversions: 3.8 ms for 128 x 100000 x 40000 against 3.2 ms with the conversion left out.
 //
 // Accumulation chains.  The tensor core adds into its fp32 accumulator with truncation, so a long chain of
 // accumulating MMAs drifts (about 6e-8 of the running sum per step, all in one direction).  The K loop is therefore
-// cut into chains of a few hundred k (TC_CHAIN_DEFAULT K blocks): each chain starts a fresh TMEM accumulator, and when it ends the drain warps
-// read it with tcgen05.ld and add it, in round-to-nearest fp32, to running sums that they keep in registers
-// (one thread = one output column n, 128 sums = 128 rows m).  With two W tiles per CTA the drain of one tile runs
-// while the MMAs of the other tile execute; with one tile the accumulator is double-buffered in TMEM instead.
-// TRANSB: the weight operand is stored transposed (N x K column-major, n contiguous).  Its tiles then arrive in shared
-// memory as [32 k][128 n] without swizzle and the converters read them column-wise (conflict-free: consecutive lanes
-// read consecutive n); everything downstream of TMEM is unchanged.
+// cut into chains of at most 512 k, which end where the activations' scale groups end: each chain starts a fresh TMEM
+// accumulator, and when it ends the drain warps read it with tcgen05.ld, remove both scales and add it, in round-to-nearest
+// fp32, to running sums that they keep in registers (one thread = one output column n, 128 sums = 128 rows m).
 template <int NT, bool MODE3X, bool TRANSB>
 __global__ void __launch_bounds__(TcCfg<NT>::THREADS, 1)
 cn_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_ahi,
-                  const __grid_constant__ CUtensorMap tm_alo, const TcParams p)
+                  const __grid_constant__ CUtensorMap tm_alo, const __grid_constant__ TcParams p)
 {
     using Cfg = TcCfg<NT>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    uint8_t *smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-    // barriers and small words sit after the rings
-    const uint32_t bar_base = smem_base + Cfg::RING_BYTES;
-    uint8_t *bar_gen = smem_gen + Cfg::RING_BYTES;
     constexpr int B_WFULL = 0, B_WEMPTY = B_WFULL + Cfg::W_STAGES, B_AFULL = B_WEMPTY + Cfg::W_STAGES,
-                  B_AEMPTY = B_AFULL + Cfg::A_STAGES, B_TFULL = B_AEMPTY + Cfg::A_STAGES, B_TEMPTY = B_TFULL + Cfg::TMEM_STAGES,
-                  B_ACCFULL = B_TEMPTY + Cfg::TMEM_STAGES, B_ACCEMPTY = B_ACCFULL + NT * Cfg::ACC_BUFS,
-                  B_COUNT = B_ACCEMPTY + NT * Cfg::ACC_BUFS;
-    static_assert(B_COUNT * 8 <= 448, "barrier area");
-    auto bar = [&](int idx) { return bar_base + 8u * idx; };
+                  B_AEMPTY = B_AFULL + Cfg::A_STAGES, B_TFULL = B_AEMPTY + Cfg::A_STAGES, B_TEMPTY = B_TFULL + NT * Cfg::TMEM_STAGES,
+                  B_ACCFULL = B_TEMPTY + NT * Cfg::TMEM_STAGES, B_ACCEMPTY = B_ACCFULL + NT * Cfg::ACC_BUFS;
+    static_assert(B_ACCEMPTY + NT * Cfg::ACC_BUFS == Cfg::BARS, "barrier count");
+    auto bar = [&](int idx) { return smem_base + Cfg::BAR_OFF + 8u * idx; };
     auto wfull_bar = [&](int s) { return bar(B_WFULL + s); };
     auto wempty_bar = [&](int s) { return bar(B_WEMPTY + s); };
     auto afull_bar = [&](int s) { return bar(B_AFULL + s); };
     auto aempty_bar = [&](int s) { return bar(B_AEMPTY + s); };
-    auto tfull_bar = [&](int t) { return bar(B_TFULL + t); };
-    auto tempty_bar = [&](int t) { return bar(B_TEMPTY + t); };
+    auto tfull_bar = [&](int w, int t) { return bar(B_TFULL + w * Cfg::TMEM_STAGES + t); };
+    auto tempty_bar = [&](int w, int t) { return bar(B_TEMPTY + w * Cfg::TMEM_STAGES + t); };
     auto accfull_bar = [&](int w, int b) { return bar(B_ACCFULL + w * Cfg::ACC_BUFS + b); };
     auto accempty_bar = [&](int w, int b) { return bar(B_ACCEMPTY + w * Cfg::ACC_BUFS + b); };
-    volatile uint32_t *tmem_holder = reinterpret_cast<volatile uint32_t *>(bar_gen + 448);
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(bar_gen + 452);
+    const uint32_t tmem_holder = smem_base + Cfg::HOLD_OFF, abort_flag = tmem_holder + 4;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    cn_pdl_launch_dependents();
 
-    // Fused all-gather: the start of this kernel means everything queued earlier on this GPU's stream has finished, so
-    // this rank's copy of C may now be overwritten by its peers: tell them (slot 0 of their flag block).
+    // Fused all-gather: everything queued earlier on this GPU's stream has finished, so this rank's copy of C may now be
+    // overwritten by its peers: tell them (slot 0 of their flag block).
     if (p.npeers > 0 && blockIdx.x == 0 && threadIdx.x < p.nranks && (int)threadIdx.x != p.my_rank) {
+        cn_pdl_wait();
         __threadfence_system();
         volatile unsigned int *f = p.peer_flags[threadIdx.x] + p.my_rank;
         *f = p.epoch;
     }
 
-    // unit decode: split-major launch order
-    const int64_t tiles = p.tiles_n * p.tiles_m;
-    const int split = (int)(blockIdx.x / tiles);
-    const int64_t tile_id = blockIdx.x % tiles;
-    const int64_t tile_n = tile_id % p.tiles_n, tile_m = tile_id / p.tiles_n;
-    const int64_t n0 = tile_n * (NT * TC_BN), m0 = tile_m * TC_BM;
-    const int kb_begin = split * p.kb_per_split;
-    int kb_end = kb_begin + p.kb_per_split;
-    if (kb_end > p.kb_total) kb_end = p.kb_total;
-    const int num_kb = kb_end - kb_begin;   // >= 1 by construction on the host
-    const int chain_kb = p.chain_kb;
-
     if (threadIdx.x == 0) {
-        for (int s = 0; s < Cfg::W_STAGES; ++s) { mbar_init(wfull_bar(s), 1); mbar_init(wempty_bar(s), 128); }
+        for (int s = 0; s < Cfg::W_STAGES; ++s) { mbar_init(wfull_bar(s), 1); mbar_init(wempty_bar(s), 4 * NT); }
         for (int s = 0; s < Cfg::A_STAGES; ++s) { mbar_init(afull_bar(s), 1); mbar_init(aempty_bar(s), NT); }
-        for (int t = 0; t < Cfg::TMEM_STAGES; ++t) { mbar_init(tfull_bar(t), 128); mbar_init(tempty_bar(t), NT); }
-        for (int w = 0; w < NT; ++w)
-            for (int b = 0; b < Cfg::ACC_BUFS; ++b) { mbar_init(accfull_bar(w, b), 1); mbar_init(accempty_bar(w, b), 128); }
-        *abort_flag = 0;
+        for (int w = 0; w < NT; ++w) {
+            for (int t = 0; t < Cfg::TMEM_STAGES; ++t) { mbar_init(tfull_bar(w, t), 4); mbar_init(tempty_bar(w, t), 1); }
+            for (int b = 0; b < Cfg::ACC_BUFS; ++b) { mbar_init(accfull_bar(w, b), 2); mbar_init(accempty_bar(w, b), 4); }
+        }
+        sts1u(abort_flag, 0u);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {   // this warp owns the tensor-memory allocation
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void *)tmem_holder)), "r"(512u) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_holder), "r"(512u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_base = *tmem_holder;
+    const uint32_t tmem_base = lds1u(tmem_holder);
 
     if (warp < 4) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::REGS_WG0));
-        if (warp == 0 || warp == 2) {
-            // ------------------------------------------------------------ TMA producers: warp 0 streams W, warp 2 the activations
+        if (warp == 0) {
+            // ------------------------------------------------------------ TMA producer of W
             if (lane == 0) {
-                const bool is_w = warp == 0;
-                const int depth = is_w ? Cfg::W_STAGES : Cfg::A_STAGES;
-                int issued = 0;
-                for (int i = 0; i < num_kb; ++i) {
-                    const int s = i % depth;
-                    const uint32_t ph = (uint32_t)(i / depth) & 1u;
-                    const int32_t kx = (kb_begin + i) * TC_BK;
-                    if (is_w) {
-                        if (!mbar_wait(wempty_bar(s), ph ^ 1u, abort_flag, p.status, 1u)) break;
+                TcWalk walk(p);
+                TcSeg seg;
+                if (!p.w_ready) cn_pdl_wait();
+                uint32_t it = 0;
+                bool ok = true;
+                while (ok && walk.next(p, seg)) {
+                    const int32_t n0 = (seg.tile / p.tiles_m) * (NT * TC_BN);
+                    for (int kb = seg.k0; kb < seg.k1; ++kb, ++it) {
+                        const int s = it % Cfg::W_STAGES;
+                        ok = mbar_wait(wempty_bar(s), ((it / Cfg::W_STAGES) & 1u) ^ 1u, abort_flag, p.status, 1u);
+                        if (!ok) break;
                         const uint32_t stage = smem_base + Cfg::W_RING + s * Cfg::W_STAGE_BYTES;
                         mbar_expect_tx(wfull_bar(s), (uint32_t)Cfg::W_STAGE_BYTES);
 #pragma unroll
                         for (int t = 0; t < NT; ++t) {
-                            if (TRANSB) tma_load_2d(stage + t * TC_TILE_BYTES, &tm_w, wfull_bar(s), (int32_t)(n0 + t * TC_BN), kx);
-                            else        tma_load_2d(stage + t * TC_TILE_BYTES, &tm_w, wfull_bar(s), kx, (int32_t)(n0 + t * TC_BN));
+                            if (TRANSB) tma_load_2d(stage + t * TC_W_TILE_BYTES, &tm_w, wfull_bar(s), n0 + t * TC_BN, kb * TC_WK);
+                            else        tma_load_2d(stage + t * TC_W_TILE_BYTES, &tm_w, wfull_bar(s), kb * TC_WK, n0 + t * TC_BN);
                         }
-                    } else {
-                        if (!mbar_wait(aempty_bar(s), ph ^ 1u, abort_flag, p.status, 8u)) break;
-                        const uint32_t stage = smem_base + Cfg::A_RING + s * Cfg::A_STAGE_BYTES;
-                        mbar_expect_tx(afull_bar(s), (uint32_t)((MODE3X ? 2 : 1) * TC_TILE_BYTES));
-                        tma_load_2d(stage, &tm_ahi, afull_bar(s), kx, (int32_t)m0);
-                        if (MODE3X) tma_load_2d(stage + TC_TILE_BYTES, &tm_alo, afull_bar(s), kx, (int32_t)m0);
                     }
-                    issued = i + 1;
                 }
-                if (*abort_flag) {
+                if (lds1u(abort_flag) != 0u) {
                     // give copies that are still in flight a bounded chance to land before the CTA exits
-                    for (int i = issued > depth ? issued - depth : 0; i < issued; ++i) {
-                        const int s = i % depth;
-                        const uint32_t ph = (uint32_t)(i / depth) & 1u;
+                    for (uint32_t i = it > Cfg::W_STAGES ? it - Cfg::W_STAGES : 0; i < it; ++i) {
                         const long long t0 = clock64();
-                        while (!mbar_try(is_w ? wfull_bar(s) : afull_bar(s), ph) && clock64() - t0 < 20000000LL) {}
+                        while (!mbar_try(wfull_bar(i % Cfg::W_STAGES), (i / Cfg::W_STAGES) & 1u) && clock64() - t0 < 20000000LL) {}
+                    }
+                }
+            }
+            __syncwarp();
+        } else if (warp == 2) {
+            // ------------------------------------------------------------ TMA producer of the activations
+            if (lane == 0) {
+                TcWalk walk(p);
+                TcSeg seg;
+                cn_pdl_wait();
+                uint32_t it = 0;
+                bool ok = true;
+                while (ok && walk.next(p, seg)) {
+                    const int32_t m0 = (seg.tile % p.tiles_m) * TC_BM;
+                    for (int kb = seg.k0 & ~1; kb < seg.k1; kb += 2, ++it) {
+                        const int s = it % Cfg::A_STAGES;
+                        ok = mbar_wait(aempty_bar(s), ((it / Cfg::A_STAGES) & 1u) ^ 1u, abort_flag, p.status, 8u);
+                        if (!ok) break;
+                        const uint32_t stage = smem_base + Cfg::A_RING + s * Cfg::A_STAGE_BYTES;
+                        mbar_expect_tx(afull_bar(s), (uint32_t)((MODE3X ? 2 : 1) * TC_A_TILE_BYTES));
+                        tma_load_2d(stage, &tm_ahi, afull_bar(s), kb * TC_WK, m0);
+                        if (MODE3X) tma_load_2d(stage + TC_A_TILE_BYTES, &tm_alo, afull_bar(s), kb * TC_WK, m0);
+                    }
+                }
+                // the last stages' releases (commits of the MMA issuers) must have arrived before the CTA may exit; on the way out
+                // after a wait that ran out, copies in flight get a bounded chance to land
+                const bool aborted = lds1u(abort_flag) != 0u;
+                for (uint32_t i = it > Cfg::A_STAGES ? it - Cfg::A_STAGES : 0; i < it; ++i) {
+                    const int s = i % Cfg::A_STAGES;
+                    const uint32_t ph = (i / Cfg::A_STAGES) & 1u;
+                    if (!aborted) {
+                        if (!mbar_wait(aempty_bar(s), ph, abort_flag, p.status, 11u)) break;
+                    } else {
+                        const long long t0 = clock64();
+                        while (!mbar_try(afull_bar(s), ph) && clock64() - t0 < 20000000LL) {}
                     }
                 }
             }
             __syncwarp();
         } else if (warp == 1 || (NT == 2 && warp == 3)) {
-            // ------------------------------------------------------------ MMA issuers: one thread per W tile (a single thread
-            // cannot issue the 64-cycle TF32 MMAs of two tiles fast enough to keep the tensor pipe busy)
+            // ------------------------------------------------------------ MMA issuers: one thread per W tile
             if (lane == 0) {
+                TcWalk walk(p);
+                TcSeg seg;
                 const int w = warp == 1 ? 0 : 1;
-                constexpr uint32_t idesc = make_idesc_tf32(TC_BN, TC_BM);
-                bool ok = true;
-                // chain bookkeeping without divisions: position inside the chain, accumulator buffer and its phase
-                // W tile 1 starts half a chain into its schedule, so that the two tiles never reach a chain end (and the
-                // wait for their drain warps) on the same K block: while one tile's accumulator is read out, the MMAs of
-                // the other keep the tensor pipe busy
-                int chain_pos = (NT == 2 && w == 1) ? chain_kb / 2 : 0, ab = 0;
-                bool chain_first = true;   // the next K block opens a chain: it overwrites the accumulator
+                constexpr uint32_t idesc = make_idesc_f16(TC_BN, TC_BM);
+                uint32_t it = 0, a_it = 0;       // W blocks and activation stages so far
+                int ab = 0;                      // accumulator buffer and its phase
                 uint32_t aph = 0;
-                // operands of the first K block
-                ok = mbar_wait(afull_bar(0), 0u, abort_flag, p.status, 2u) && mbar_wait(tfull_bar(0), 0u, abort_flag, p.status, 3u);
-                for (int i = 0; i < num_kb && ok; ++i) {
-                    const int s = i % Cfg::A_STAGES, t = i % Cfg::TMEM_STAGES;
-                    const bool chain_last = chain_pos == chain_kb - 1 || i == num_kb - 1;
-                    tc_fence_after();
-                    const uint32_t stage = smem_base + Cfg::A_RING + s * Cfg::A_STAGE_BYTES;
-                    const uint64_t bhi = make_kmajor_sw128_desc(stage);
-                    const uint64_t blo = make_kmajor_sw128_desc(stage + TC_TILE_BYTES);
-                    const uint32_t bhi_lo = (uint32_t)bhi, bhi_hi = (uint32_t)(bhi >> 32), blo_lo = (uint32_t)blo, blo_hi = (uint32_t)(blo >> 32);
-                    if (chain_first) {   // the drain warps must have emptied this accumulator
-                        ok = mbar_wait(accempty_bar(w, ab), aph ^ 1u, abort_flag, p.status, 7u);
-                        if (!ok) break;
+                bool open = false, ok = true;    // a chain is accumulating
+                // Ends the open chain: the drain warps learn where its scales are, and that it is complete when its MMAs retire
+                auto close_chain = [&](uint32_t last_it, int last_kb, bool last_of_run) {
+                    const uint32_t q = smem_base + Cfg::INFO_OFF + (w * Cfg::ACC_BUFS + ab) * 8;
+                    sts1u(q, (last_it % Cfg::WS_SLOTS) | (last_of_run ? 0x100u : 0u));
+                    sts1u(q + 4, (uint32_t)(last_kb / TC_GROUP_KB));
+                    mbar_arrive(accfull_bar(w, ab));
+                    tc_commit(accfull_bar(w, ab));
+                    if (++ab == Cfg::ACC_BUFS) { ab = 0; aph ^= 1u; }
+                    open = false;
+                };
+                // operands of one W block: the activation stage where it opens one, and the converted W rows
+                auto wait_block = [&](uint32_t i, uint32_t a, bool opens_stage) {
+                    if (opens_stage && !mbar_wait(afull_bar(a % Cfg::A_STAGES), (a / Cfg::A_STAGES) & 1u, abort_flag, p.status, 2u)) return false;
+                    return mbar_wait(tfull_bar(w, i % Cfg::TMEM_STAGES), (i / Cfg::TMEM_STAGES) & 1u, abort_flag, p.status, 3u);
+                };
+                while (ok && walk.next(p, seg)) {
+                    ok = wait_block(it, a_it, true);
+                    for (int kb = seg.k0; kb < seg.k1 && ok; ++kb, ++it) {
+                        const int t = it % Cfg::TMEM_STAGES;
                         tc_fence_after();
-                    }
-                    const uint32_t acc = tmem_base + Cfg::ACC_COL + (w * Cfg::ACC_BUFS + ab) * TC_BM;
-                    const uint32_t a_hi = tmem_base + Cfg::A_COL + t * Cfg::A_STAGE_COLS + w * 64;
-                    const uint32_t a_lo = a_hi + 32;
-#pragma unroll
-                    for (int j = 0; j < TC_BK / 8; ++j) {
-                        if (j == TC_BK / 8 - 1 && i + 1 < num_kb) {
-                            // Look ahead: make sure the operands of the next K block are there BEFORE the last MMAs of
-                            // this one are issued.  Issue is back-pressured by the tensor pipe, so once those are in,
-                            // only the commits stand between them and the next block's first MMA.
-                            const int s1 = (i + 1) % Cfg::A_STAGES, t1 = (i + 1) % Cfg::TMEM_STAGES;
-                            const uint32_t ph1 = (uint32_t)((i + 1) / Cfg::A_STAGES) & 1u, tph1 = (uint32_t)((i + 1) / Cfg::TMEM_STAGES) & 1u;
-                            ok = mbar_wait(afull_bar(s1), ph1, abort_flag, p.status, 2u) && mbar_wait(tfull_bar(t1), tph1, abort_flag, p.status, 3u);
+                        // a row whose scale had to change (see the converters) ends the chain before this block
+                        if (open && lds1u(smem_base + Cfg::BRK_OFF + (t * NT + w) * 4) != 0u) close_chain(it - 1, kb - 1, false);
+                        bool first = false;
+                        if (!open) {   // the drain warps must have emptied this accumulator
+                            ok = mbar_wait(accempty_bar(w, ab), aph ^ 1u, abort_flag, p.status, 7u);
+                            if (!ok) break;
+                            tc_fence_after();
+                            open = first = true;
                         }
-                        // 8 TF32 per k-step: 8 TMEM columns of A, 32 bytes (descriptor units of 16 B) of B
-                        tc_mma_ts(acc, a_hi + j * 8, bhi_lo + j * 2, bhi_hi, idesc, (!chain_first || j > 0) ? 1u : 0u);
+                        const int s = a_it % Cfg::A_STAGES;
+                        const uint32_t stage = smem_base + Cfg::A_RING + s * Cfg::A_STAGE_BYTES + (uint32_t)(kb & 1) * (TC_WK * 2);
+                        const uint64_t bhi = make_kmajor_sw128_desc(stage), blo = make_kmajor_sw128_desc(stage + TC_A_TILE_BYTES);
+                        const uint32_t bhi_lo = (uint32_t)bhi, bhi_hi = (uint32_t)(bhi >> 32), blo_lo = (uint32_t)blo, blo_hi = (uint32_t)(blo >> 32);
+                        const uint32_t acc = tmem_base + Cfg::ACC_COL + (w * Cfg::ACC_BUFS + ab) * TC_BM;
+                        const uint32_t w_hi = tmem_base + Cfg::OP_COL + t * Cfg::OP_STAGE_COLS + w * 32;
+                        const bool last_of_run = kb == seg.k1 - 1, ends_stage = (kb & 1) || last_of_run;
+                        // 16 fp16 per k-step: 8 TMEM columns of W, 32 bytes (descriptor units of 16 B) of the activations
+                        tc_mma_ts(acc, w_hi, bhi_lo, bhi_hi, idesc, first ? 0u : 1u);
                         if (MODE3X) {
-                            tc_mma_ts(acc, a_lo + j * 8, bhi_lo + j * 2, bhi_hi, idesc, 1u);
-                            tc_mma_ts(acc, a_hi + j * 8, blo_lo + j * 2, blo_hi, idesc, 1u);
+                            tc_mma_ts(acc, w_hi + 8, bhi_lo, bhi_hi, idesc, 1u);
+                            tc_mma_ts(acc, w_hi, blo_lo, blo_hi, idesc, 1u);
                         }
+                        // Look ahead: make sure the operands of the next block are there BEFORE the last MMAs of this one are
+                        // issued.  Issue is back-pressured by the tensor pipe, so once those are in, only the commits stand
+                        // between them and the next block's first MMA.
+                        if (!last_of_run) ok = wait_block(it + 1, a_it + 1, ends_stage);
+                        tc_mma_ts(acc, w_hi + 16, bhi_lo + 2, bhi_hi, idesc, 1u);
+                        if (MODE3X) {
+                            tc_mma_ts(acc, w_hi + 24, bhi_lo + 2, bhi_hi, idesc, 1u);
+                            tc_mma_ts(acc, w_hi + 16, blo_lo + 2, blo_hi, idesc, 1u);
+                        }
+                        if (last_of_run || ((kb + 1) & p.chain_mask) == 0) close_chain(it, kb, last_of_run);
+                        if (ends_stage) {   // the activation stage may be refilled once these MMAs retire
+                            tc_commit(aempty_bar(s));
+                            ++a_it;
+                        }
+                        tc_commit(tempty_bar(w, t));   // and the TMEM operand stage rewritten
                     }
-                    if (chain_last) {
-                        tc_commit(accfull_bar(w, ab));
-                        chain_pos = 0;
-                        chain_first = true;
-                        if (++ab == Cfg::ACC_BUFS) { ab = 0; aph ^= 1u; }
-                    } else {
-                        ++chain_pos;
-                        chain_first = false;
-                    }
-                    tc_commit(aempty_bar(s));   // activation stage may be refilled once these MMAs retire
-                    tc_commit(tempty_bar(t));   // and the TMEM operand stage rewritten
                 }
             }
             __syncwarp();
         }
-    } else if (warp < 8) {
-        // ---------------------------------------------------------------- converter warps
+    } else if (warp < 4 + 4 * NT) {
+        // ---------------------------------------------------------------- converter warps, one warpgroup per W tile
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::REGS_CONV));
+        const int w = (warp - 4) >> 2;                // W tile of this warpgroup
         const int q = warp & 3;                       // TMEM lane quarter this warp may touch
         const int row = q * 32 + lane;                // row of the W tile = TMEM lane
-        const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
+        const uint32_t dst0 = tmem_base + ((uint32_t)(q * 32) << 16) + Cfg::OP_COL + w * 32;
+        TcWalk walk(p);
+        TcSeg seg;
+        float sc = 1.0f, inv = 1.0f;                  // this row's scale in the open chain
+        bool set = false;                             // ... is fixed: the row has had a nonzero element
+        uint32_t it = 0;
         bool ok = true;
-        for (int i = 0; i < num_kb && ok; ++i) {
-            const int s = i % Cfg::W_STAGES, t = i % Cfg::TMEM_STAGES;
-            const uint32_t ph = (uint32_t)(i / Cfg::W_STAGES) & 1u, tph = (uint32_t)(i / Cfg::TMEM_STAGES) & 1u;
-            ok = mbar_wait(wfull_bar(s), ph, abort_flag, p.status, 4u) && mbar_wait(tempty_bar(t), tph ^ 1u, abort_flag, p.status, 5u);
-            ok = __all_sync(0xffffffffu, ok);   // the tcgen05 stores below need the whole warp
-            if (!ok) break;
-            tc_fence_after();
-            const uint8_t *stage = smem_gen + Cfg::W_RING + s * Cfg::W_STAGE_BYTES;
-#pragma unroll 1
-            for (int w = 0; w < NT; ++w) {
-                const uint8_t *tilep = stage + w * TC_TILE_BYTES;
-                const uint32_t a_hi = tmem_base + lane_addr + Cfg::A_COL + t * Cfg::A_STAGE_COLS + w * 64;
-                uint32_t hi[32], lo[32];
-                if (TRANSB) {
-#pragma unroll
-                    for (int k = 0; k < 32; ++k) {
-                        const float x = *reinterpret_cast<const float *>(tilep + k * (TC_BN * 4) + row * 4);
-                        const uint32_t h = to_tf32(x);
-                        hi[k] = h;
-                        if (MODE3X) lo[k] = to_tf32(x - __uint_as_float(h));
-                    }
-                } else {
-                    const uint8_t *rowp = tilep + row * 128;
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        // 16-byte chunk c of row r sits at chunk position c ^ (r & 7) under the 128-byte swizzle
-                        const float4 v = *reinterpret_cast<const float4 *>(rowp + ((c ^ (row & 7)) << 4));
-                        const float x[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const uint32_t h = to_tf32(x[e]);
-                            hi[c * 4 + e] = h;
-                            if (MODE3X) lo[c * 4 + e] = to_tf32(x[e] - __uint_as_float(h));
-                        }
-                    }
+        while (ok && walk.next(p, seg)) {
+            for (int kb = seg.k0; kb < seg.k1; ++kb, ++it) {
+                const int s = it % Cfg::W_STAGES, t = it % Cfg::TMEM_STAGES;
+                ok = mbar_wait(wfull_bar(s), (it / Cfg::W_STAGES) & 1u, abort_flag, p.status, 4u) &&
+                     mbar_wait(tempty_bar(w, t), ((it / Cfg::TMEM_STAGES) & 1u) ^ 1u, abort_flag, p.status, 5u);
+                ok = __all_sync(0xffffffffu, ok);   // the tcgen05 stores below need the whole warp
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t rowp = tc_row_base<TRANSB>(smem_base + Cfg::W_RING + s * Cfg::W_STAGE_BYTES + w * TC_W_TILE_BYTES, row);
+                const bool chain_start = kb == seg.k0 || (kb & p.chain_mask) == 0;
+                if (chain_start) set = false;
+                if (!set) {
+                    // nothing but zeros of this row is in the accumulator: any scale is right for what is there
+                    const uint32_t amax = tc_row_amax<TRANSB>(rowp);
+                    tc_scale<TC_W_EXP>(amax, sc, inv);
+                    set = amax != 0u;
                 }
-                tc_st32(a_hi, hi);
-                if (MODE3X) tc_st32(a_hi + 32, lo);
+                __syncwarp();
+                const uint32_t dst = dst0 + t * Cfg::OP_STAGE_COLS;
+                bool grew = false;
+                for (;;) {
+                    uint32_t top = 0u;
+                    const uint64_t sc2 = tc_pack2(sc, sc);
+#pragma unroll 1
+                    for (int step = 0; step < 2; ++step) {
+                        uint32_t hl[16];
+                        tc_convert_step<MODE3X, TRANSB>(rowp, step, sc2, hl, top);
+                        if (MODE3X) tc_st16(dst + step * 16, hl);
+                        else        tc_st8(dst + step * 16, hl);
+                    }
+                    top &= 0x7fff7fffu;
+                    const bool over = (top >> 16) >= 0x7c00u || (top & 0xffffu) >= 0x7c00u;
+                    if (grew || !__any_sync(0xffffffffu, over)) break;
+                    // rare: a row's magnitudes grew more than fourfold since its chain began: new scale, and once more
+                    grew = true;
+                    if (over) tc_scale<TC_W_EXP>(tc_row_amax<TRANSB>(rowp), sc, inv);
+                    tc_wait_st();
+                    __syncwarp();
+                }
+                sts1(smem_base + Cfg::WS_OFF + (((it % Cfg::WS_SLOTS) * NT + w) * TC_BN + row) * 4, inv);
+                if (lane == 0) sts1b(smem_base + Cfg::BRK_OFF + (t * NT + w) * 4 + q, grew && !chain_start ? 1u : 0u);
+                tc_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive(wempty_bar(s));   // the raw block now lives in TMEM: its ring slot may be refilled
+                    mbar_arrive(tfull_bar(w, t));
+                }
             }
-            mbar_arrive(wempty_bar(s));   // the raw tile now lives in registers / TMEM: its ring slot may be refilled
-            tc_wait_st();
-            tc_fence_before();
-            mbar_arrive(tfull_bar(t));
         }
+        // the last operand stages' releases must have arrived before the CTA may exit
+        for (uint32_t i = it > Cfg::TMEM_STAGES ? it - Cfg::TMEM_STAGES : 0; i < it && ok; ++i)
+            ok = mbar_wait(tempty_bar(w, i % Cfg::TMEM_STAGES), (i / Cfg::TMEM_STAGES) & 1u, abort_flag, p.status, 13u);
     } else {
         // ---------------------------------------------------------------- drain + epilogue warps, one warpgroup per W tile
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Cfg::REGS_DRAIN));
-        const int w = (warp - 8) >> 2;                // W tile of this warpgroup
+        const int w = (warp - 4 - 4 * NT) >> 2;       // W tile of this warpgroup
         const int q = warp & 3;
         const int row = q * 32 + lane;
         const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
-        const int et = threadIdx.x & 127;
-        float acc[TC_BM];
-#pragma unroll
-        for (int i = 0; i < TC_BM; ++i) acc[i] = 0.0f;
+        TcWalk walk(p);
+        TcSeg seg;
+        cn_pdl_wait();
+        uint32_t chains = 0;
         bool ok = true;
-        // chains of this W tile: tile 1's first chain is the short one (see the MMA issuer)
-        const int my_chains = (num_kb + ((NT == 2 && w == 1) ? chain_kb / 2 : 0) + chain_kb - 1) / chain_kb;
-        for (int c = 0; c < my_chains && ok; ++c) {
-            const int ab = c % Cfg::ACC_BUFS;
-            const uint32_t aph = (uint32_t)(c / Cfg::ACC_BUFS) & 1u;
-            ok = mbar_wait<TC_DRAIN_SLEEP_NS>(accfull_bar(w, ab), aph, abort_flag, p.status, 6u);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
-            tc_fence_after();
-            const uint32_t src = tmem_base + lane_addr + Cfg::ACC_COL + (w * Cfg::ACC_BUFS + ab) * TC_BM;
+        while (ok && walk.next(p, seg)) {
+            const int64_t m0 = (int64_t)(seg.tile % p.tiles_m) * TC_BM, n0 = (int64_t)(seg.tile / p.tiles_m) * (NT * TC_BN) + w * TC_BN;
+            uint64_t sum[TC_BM / 2];   // pairs of rows
 #pragma unroll
-            for (int cc = 0; cc < TC_BM / 32; ++cc) {
-                uint32_t r[32];
-                tc_ld32(src + cc * 32, r);
-#pragma unroll
-                for (int i = 0; i < 32; ++i) acc[cc * 32 + i] += __uint_as_float(r[i]);
-            }
-            tc_fence_before();
-            mbar_arrive(accempty_bar(w, ab));
-        }
-        {   // all 128 threads of the warpgroup go on together or not at all
-            uint32_t all_ok;
-            asm volatile(
-                "{\n\t.reg .pred pi, po;\n\t"
-                "setp.ne.u32 pi, %1, 0;\n\t"
-                "bar.red.and.pred po, %2, 128, pi;\n\t"
-                "selp.u32 %0, 1, 0, po;\n\t}"
-                : "=r"(all_ok) : "r"((uint32_t)ok), "r"(1 + w) : "memory");
-            ok = all_ok != 0;
-        }
-        if (ok && NT == 2 && w == 1) {
-            // This warpgroup stages its output tile in the activation ring.  Its own accumulator being complete says
-            // nothing about the other tile's MMAs, which read the same ring stages: wait until the last K block's stage
-            // has been released by both issuers (their commits arrive in issue order, so every earlier stage is free too).
-            const int last = num_kb - 1;
-            ok = mbar_wait(aempty_bar(last % Cfg::A_STAGES), (uint32_t)(last / Cfg::A_STAGES) & 1u, abort_flag, p.status, 11u);
-            uint32_t all_ok;
-            asm volatile(
-                "{\n\t.reg .pred pi, po;\n\t"
-                "setp.ne.u32 pi, %1, 0;\n\t"
-                "bar.red.and.pred po, %2, 128, pi;\n\t"
-                "selp.u32 %0, 1, 0, po;\n\t}"
-                : "=r"(all_ok) : "r"((uint32_t)ok), "r"(1 + w) : "memory");
-            ok = all_ok != 0;
-            tc_fence_after();
-        }
-        if (ok) {
-            const int64_t ticket_id = tile_id * NT + w;
-            const size_t tile_elems = (size_t)TC_BM * TC_BN;
-            bool do_final = true;
-            if (p.splits > 1) {
-                // Split-K: this CTA's partial tile goes to scratch as one contiguous 64 KB block laid out like C (column n =
-                // 512 bytes), staged through the idle rings and written with a single bulk copy; cn_splitk_reduce_kernel adds
-                // the partials of all splits in split order and applies the epilogue, spread over the whole GPU.
-                float *stg = reinterpret_cast<float *>(smem_gen + (w == 0 ? Cfg::W_RING : Cfg::A_RING));
-#pragma unroll
-                for (int i = 0; i < TC_BM; i += 4)
-                    *reinterpret_cast<float4 *>(stg + row * TC_BM + i) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                asm volatile("bar.sync %0, 128;" ::"r"(1 + w) : "memory");
-                if (et == 0) {
-                    float *P = p.partials + ((size_t)ticket_id * p.splits + split) * tile_elems;
-                    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
-                                 ::"l"(P), "r"(smem_u32(stg)), "r"((uint32_t)(tile_elems * sizeof(float))) : "memory");
-                    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+            for (int i = 0; i < TC_BM / 2; ++i) sum[i] = 0ull;
+            // the inverse scales of the activation rows: thread `row` fetches row m0 + row of the group it expects next
+            int have_group = seg.k0 / TC_GROUP_KB;
+            float my_inv = p.a_inv[(int64_t)have_group * p.m_pad + m0 + row];
+            for (bool last = false; !last; ++chains) {
+                const int ab = chains % Cfg::ACC_BUFS;
+                ok = mbar_wait<TC_DRAIN_SLEEP_NS>(accfull_bar(w, ab), (chains / Cfg::ACC_BUFS) & 1u, abort_flag, p.status, 6u);
+                {   // all 128 threads of the warpgroup go on together or not at all
+                    uint32_t all_ok;
+                    asm volatile(
+                        "{\n\t.reg .pred pi, po;\n\t"
+                        "setp.ne.u32 pi, %1, 0;\n\t"
+                        "bar.red.and.pred po, %2, 128, pi;\n\t"
+                        "selp.u32 %0, 1, 0, po;\n\t}"
+                        : "=r"(all_ok) : "r"((uint32_t)ok), "r"(1 + w) : "memory");
+                    ok = all_ok != 0;
                 }
-                do_final = false;
-            }
-            if (do_final) {
-                const int L = p.maxout_level;
-                const int64_t n = n0 + w * TC_BN + row;
-                const float bias = (p.bias && n < p.N) ? p.bias[n] : 0.0f;
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t what = lds1u(smem_base + Cfg::INFO_OFF + (w * Cfg::ACC_BUFS + ab) * 8);
+                const int group = (int)lds1u(smem_base + Cfg::INFO_OFF + (w * Cfg::ACC_BUFS + ab) * 8 + 4);
+                last = (what & 0x100u) != 0u;
+                if (group != have_group) my_inv = p.a_inv[(int64_t)group * p.m_pad + m0 + row];
+                const uint32_t as = smem_base + Cfg::AS_OFF + ((chains & 1u) * NT + w) * (TC_BM * 4);
+                sts1(as + row * 4, my_inv);
+                const float wi = lds1(smem_base + Cfg::WS_OFF + (((what & 0xffu) * NT + w) * TC_BN + row) * 4);
+                asm volatile("bar.sync %0, 128;" ::"r"(1 + w) : "memory");
+                have_group = group;
+                if (!last && group < (seg.k1 - 1) / TC_GROUP_KB) {   // most likely the next chain's group
+                    have_group = group + 1;
+                    my_inv = p.a_inv[(int64_t)have_group * p.m_pad + m0 + row];
+                }
+                const uint32_t src = tmem_base + lane_addr + Cfg::ACC_COL + (w * Cfg::ACC_BUFS + ab) * TC_BM;
+                // Remove both scales and add.  (The product of the two inverse scales is finite unless the product of the segment's
+                // largest magnitudes is beyond fp32's range by 2^27.)
+                const uint64_t wi2 = tc_pack2(wi, wi);
 #pragma unroll
-                for (int i = 0; i < TC_BM; ++i) acc[i] = cn_apply_activation(p.bias ? acc[i] + bias : acc[i], p.act);
-                if (L <= 1) {
-                    if (p.npeers > 0) {
-                        // the peers must have announced that their copy of C may be overwritten (bounded wait)
-                        if (et == 0) {
-                            const long long t0 = clock64();
-                            for (int r = 0; r < p.nranks; ++r) {
-                                if (r == p.my_rank) continue;
-                                const volatile unsigned int *f = p.ready + r;
-                                while ((int)(*f - p.epoch) < 0) {
-                                    if (clock64() - t0 > TC_WAIT_LIMIT) { atomicMax(p.status, 9u); break; }
-                                    __nanosleep(100);
-                                }
-                            }
-                        }
-                        asm volatile("bar.sync %0, 128;" ::"r"(1 + w) : "memory");
+                for (int cc = 0; cc < TC_BM / 16; ++cc) {
+                    uint32_t r[16];
+                    tc_ld16(src + cc * 16, r);
+#pragma unroll
+                    for (int i = 0; i < 16; i += 4) {
+                        const float4 f = lds4(as + (cc * 16 + i) * 4);
+                        uint64_t &s0 = sum[(cc * 16 + i) / 2], &s1 = sum[(cc * 16 + i) / 2 + 1];
+                        s0 = tc_fma2(tc_pack2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), tc_mul2(tc_pack2(f.x, f.y), wi2), s0);
+                        s1 = tc_fma2(tc_pack2(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])), tc_mul2(tc_pack2(f.z, f.w), wi2), s1);
                     }
-                    const int64_t rows_valid = (p.M - m0) < TC_BM ? (p.M - m0) : TC_BM;
-                    if (p.npeers > 0 && (rows_valid & 3) == 0 && (p.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15u) == 0) {
-                        // Fused all-gather.  Scattered 16-byte stores from registers are a poor fit for NVLink, so the tile is
-                        // first laid out in shared memory exactly as it lies in C (column n = 512 contiguous bytes; the rings
-                        // are idle by now: tile 0 borrows the W ring, tile 1 the activation ring) and then written to the
-                        // local C and to every peer's C with bulk asynchronous copies.
-                        float *stg = reinterpret_cast<float *>(smem_gen + (w == 0 ? Cfg::W_RING : Cfg::A_RING));
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(accempty_bar(w, ab));
+            }
+            if (!ok) break;
+            const int64_t n = n0 + row;
+            if (seg.slot >= 0) {
+                // partial tile: float4 number i of 32 for all 128 columns, then the next, so that a warp writes 512 contiguous bytes
+                ulonglong2 *P = reinterpret_cast<ulonglong2 *>(p.partials) + ((int64_t)seg.slot * NT + w) * (TC_BM * TC_BN / 4) + row;
 #pragma unroll
-                        for (int i = 0; i < TC_BM; i += 4)
-                            *reinterpret_cast<float4 *>(stg + row * TC_BM + i) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
-                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                        asm volatile("bar.sync %0, 128;" ::"r"(1 + w) : "memory");
-                        const int64_t col0 = n0 + w * TC_BN;
-                        const int64_t cols_valid = (p.N - col0) < TC_BN ? (p.N - col0) : TC_BN;
-                        if (rows_valid == TC_BM && p.ldc == TC_BM) {
-                            // the tile is one contiguous block of C: one copy per destination
-                            if (et == 0 && cols_valid > 0) {
-                                const uint32_t bytes = (uint32_t)(cols_valid * TC_BM * sizeof(float));
-                                const int64_t off = col0 * p.ldc + m0;
-                                for (int d = 0; d <= p.npeers; ++d) {
-                                    float *dst = (d == 0 ? p.C : p.peerC[d - 1]) + off;
-                                    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
-                                                 ::"l"(dst), "r"(smem_u32(stg)), "r"(bytes) : "memory");
-                                }
-                                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                                asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-                            }
-                        } else if (n < p.N) {
-                            // one copy per column and destination
-                            const uint32_t bytes = (uint32_t)(rows_valid * sizeof(float));
-                            const int64_t off = n * p.ldc + m0;
-                            for (int d = 0; d <= p.npeers; ++d) {
-                                float *dst = (d == 0 ? p.C : p.peerC[d - 1]) + off;
-                                asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;"
-                                             ::"l"(dst), "r"(smem_u32(stg + row * TC_BM)), "r"(bytes) : "memory");
-                            }
-                            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                            asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-                        }
-                    } else if (n < p.N) {
-                        const int64_t off = n * p.ldc + m0;
-                        float *dst = p.C + off;
-                        if (m0 + TC_BM <= p.M && ((reinterpret_cast<uintptr_t>(dst) & 15u) == 0)) {
+                for (int i = 0; i < TC_BM / 4; ++i) P[i * TC_BN] = make_ulonglong2(sum[2 * i], sum[2 * i + 1]);
+                continue;
+            }
+            const int L = p.maxout_level;
+            const float bias = (p.bias && n < p.N) ? p.bias[n] : 0.0f;
+            float *dst = p.C + n * p.ldc + m0;
+            const bool vec = m0 + TC_BM <= p.M && ((reinterpret_cast<uintptr_t>(dst) & 15u) == 0);
+            if (L <= 1 && n >= p.N) continue;
 #pragma unroll
-                            for (int i = 0; i < TC_BM; i += 4)
-                                *reinterpret_cast<float4 *>(dst + i) = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
-                        } else {
+            for (int i = 0; i < TC_BM; i += 4) {
+                float v[4];
+                tc_unpack2(sum[i / 2], v[0], v[1]);
+                tc_unpack2(sum[i / 2 + 1], v[2], v[3]);
 #pragma unroll
-                            for (int i = 0; i < TC_BM; ++i)
-                                if (m0 + i < p.M) dst[i] = acc[i];
-                        }
-                        for (int pr = 0; pr < p.npeers; ++pr) {   // rare shapes only: rows not a multiple of four
-                            float *pd = p.peerC[pr] + off;
+                for (int e = 0; e < 4; ++e) v[e] = cn_apply_activation(p.bias ? v[e] + bias : v[e], p.act);
+                if (L <= 1) {
+                    if (vec) {
+                        *reinterpret_cast<float4 *>(dst + i) = make_float4(v[0], v[1], v[2], v[3]);
+                    } else {
 #pragma unroll
-                            for (int i = 0; i < TC_BM; ++i)
-                                if (m0 + i < p.M) pd[i] = acc[i];
-                        }
+                        for (int e = 0; e < 4; ++e)
+                            if (m0 + i + e < p.M) dst[i + e] = v[e];
                     }
                 } else {
                     // maxout over L consecutive columns = L adjacent lanes (L is a power of two <= 32).
@@ -756,17 +949,17 @@ cn_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
                     // takes slot t+offset when strictly smaller; larger offsets only meet -FLT_MAX padding.
                     const int tl = lane & (L - 1);
 #pragma unroll
-                    for (int i = 0; i < TC_BM; ++i) {
-                        float val = acc[i], idx = (float)n;
+                    for (int e = 0; e < 4; ++e) {
+                        float val = v[e], idx = (float)n;
                         for (int off = L >> 1; off > 0; off >>= 1) {
                             const float ov = __shfl_down_sync(0xffffffffu, val, off, L);
                             const float oi = __shfl_down_sync(0xffffffffu, idx, off, L);
                             if (tl < off && val < ov) { val = ov; idx = oi; }
                         }
-                        if (tl == 0 && n < p.N && m0 + i < p.M) {
+                        if (tl == 0 && n < p.N && m0 + i + e < p.M) {
                             const int64_t g = n / L;
-                            p.C[g * p.ldc + m0 + i] = val;
-                            if (p.argmax) p.argmax[g * p.ldc + m0 + i] = idx;
+                            p.C[g * p.ldc + m0 + i + e] = val;
+                            if (p.argmax) p.argmax[g * p.ldc + m0 + i + e] = idx;
                         }
                     }
                 }
@@ -782,14 +975,16 @@ cn_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
     }
 }
 
-// ------------------------------------------------------------------------------------------- split-K reduction
-// One thread = four consecutive rows m of one output column n: adds the partial tiles of all splits in split order (a
-// fixed order, so the result does not depend on scheduling), applies bias and activation, stores to C and, for the
-// fused all-gather, to every peer's C (a warp writes 512 contiguous bytes of a column: full NVLink packets).
+// ------------------------------------------------------------------------------------------ reduction of the runs
+// One CTA per 32 columns of one W tile: adds the partial tiles of all runs in K order (a fixed order, so the result does not
+// depend on scheduling), applies bias and activation, turns the block through shared memory so that a warp stores 512
+// contiguous bytes of a column, and stores to C and, for the fused all-gather, to every peer's C (full NVLink packets).
 struct ReduceParams {
     const float *partials;
-    int splits, nt;
-    int64_t tiles_n, tiles_m, M, N;
+    int nt, tail_ctas, kb_total;
+    int tail_tiles;              // tiles cut into runs, [full_tiles, full_tiles + tail_tiles)
+    int full_tiles, tiles_m;
+    int64_t M, N;
     float *C;
     int64_t ldc;
     const float *bias;
@@ -803,8 +998,11 @@ struct ReduceParams {
 };
 
 __global__ void __launch_bounds__(256)
-cn_splitk_reduce_kernel(const ReduceParams p)
+cn_splitk_reduce_kernel(const __grid_constant__ ReduceParams p)
 {
+    __shared__ float turn[32][TC_BM + 4];
+    cn_pdl_launch_dependents();
+    cn_pdl_wait();
     if (p.npeers > 0) {   // peers must have announced that their copy of C may be overwritten (bounded wait)
         if (threadIdx.x == 0) {
             const long long t0 = clock64();
@@ -819,48 +1017,71 @@ cn_splitk_reduce_kernel(const ReduceParams p)
         }
         __syncthreads();
     }
-    const size_t tile_elems = (size_t)TC_BM * TC_BN;
-    const int64_t quads_per_tile = tile_elems / 4;
-    const int64_t total = p.tiles_n * p.tiles_m * p.nt * quads_per_tile;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += stride) {
-        const int64_t ticket = q / quads_per_tile;          // (tile_id * nt + w)
-        const int64_t inner = q - ticket * quads_per_tile;  // n_local * 32 + m4
-        const int n_local = (int)(inner >> 5), m_local = (int)(inner & 31) * 4;
-        const int64_t tile_id = ticket / p.nt;
-        const int w = (int)(ticket - tile_id * p.nt);
-        const int64_t tile_n = tile_id % p.tiles_n, tile_m = tile_id / p.tiles_n;
-        const int64_t n = tile_n * (p.nt * TC_BN) + w * TC_BN + n_local, m = tile_m * TC_BM + m_local;
+    const int chunk = blockIdx.x & 3;
+    const int tw = blockIdx.x >> 2, r = tw / p.nt, w = tw - r * p.nt, tile = p.full_tiles + r;
+    const int64_t m0 = (int64_t)(tile % p.tiles_m) * TC_BM, n0 = ((int64_t)(tile / p.tiles_m) * p.nt + w) * TC_BN + chunk * 32;
+    if (n0 >= p.N) return;
+    // the CTAs whose runs hold K blocks of this tile: run c is [total c / ctas, total (c + 1) / ctas)
+    const int64_t total = (int64_t)p.tail_tiles * p.kb_total, first = (int64_t)r * p.kb_total, last = first + p.kb_total - 1;
+    auto owner = [&](int64_t x) {
+        int64_t c = x * p.tail_ctas / total;
+        while (total * (c + 1) / p.tail_ctas <= x) ++c;
+        while (total * c / p.tail_ctas > x) --c;
+        return c;
+    };
+    const int64_t c0 = owner(first), c1 = owner(last);
+    const int row = threadIdx.x & 31, quad = threadIdx.x >> 5;   // column of the chunk; quads of m: quad + 8 j
+    constexpr int64_t TILE4 = TC_BM * TC_BN / 4;
+    const float4 *src = reinterpret_cast<const float4 *>(p.partials) + ((c0 + r) * p.nt + w) * TILE4 + quad * TC_BN + chunk * 32 + row;
+    const int64_t step = p.nt * TILE4;
+    float4 acc[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    int64_t left = c1 - c0 + 1;
+    // two partial tiles in flight at a time; the additions stay in K order, so the sum does not depend on the grouping
+    for (; left >= 2; left -= 2, src += 2 * step) {
+        float4 v[2][4];
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[u][j] = __ldcs(src + u * step + j * 8 * TC_BN);
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) { acc[j].x += v[u][j].x; acc[j].y += v[u][j].y; acc[j].z += v[u][j].z; acc[j].w += v[u][j].w; }
+    }
+    if (left > 0) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float4 v = __ldcs(src + j * 8 * TC_BN);
+            acc[j].x += v.x; acc[j].y += v.y; acc[j].z += v.z; acc[j].w += v.w;
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) *reinterpret_cast<float4 *>(&turn[row][(quad + 8 * j) * 4]) = acc[j];
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const int64_t m = m0 + lane * 4;
+    const bool vec = (m + 4 <= p.M) && ((p.ldc & 3) == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15u) == 0);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int nl = (threadIdx.x >> 5) + 8 * j;
+        const int64_t n = n0 + nl;
         if (n >= p.N || m >= p.M) continue;
-        const float *src = p.partials + (size_t)ticket * p.splits * tile_elems + (size_t)n_local * TC_BM + m_local;
-        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        int sp = 0;
-        // four loads in flight at a time; the additions stay in split order, so the sum does not depend on the grouping
-        for (; sp + 4 <= p.splits; sp += 4) {
-            float4 v[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) v[u] = __ldcg(reinterpret_cast<const float4 *>(src + (size_t)(sp + u) * tile_elems));
-#pragma unroll
-            for (int u = 0; u < 4; ++u) { acc.x += v[u].x; acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w; }
-        }
-        for (; sp < p.splits; ++sp) {
-            const float4 v = __ldcg(reinterpret_cast<const float4 *>(src + (size_t)sp * tile_elems));
-            acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
-        }
         const float b = p.bias ? p.bias[n] : 0.0f;
-        float r[4] = {acc.x, acc.y, acc.z, acc.w};
+        const float4 a = *reinterpret_cast<const float4 *>(&turn[nl][lane * 4]);
+        float v[4] = {a.x, a.y, a.z, a.w};
 #pragma unroll
-        for (int i = 0; i < 4; ++i) r[i] = cn_apply_activation(p.bias ? r[i] + b : r[i], p.act);
+        for (int i = 0; i < 4; ++i) v[i] = cn_apply_activation(p.bias ? v[i] + b : v[i], p.act);
         const int64_t off = n * p.ldc + m;
-        const bool vec = (m + 4 <= p.M) && ((p.ldc & 3) == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15u) == 0);
         for (int d = 0; d <= p.npeers; ++d) {
             float *dst = (d == 0 ? p.C : p.peerC[d - 1]) + off;
             if (vec) {
-                *reinterpret_cast<float4 *>(dst) = make_float4(r[0], r[1], r[2], r[3]);
+                *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
             } else {
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
-                    if (m + i < p.M) dst[i] = r[i];
+                    if (m + i < p.M) dst[i] = v[i];
             }
         }
     }
@@ -885,20 +1106,32 @@ static int get_encode_fn(cn_context *ctx, EncodeTiledFn *out)
     return CN_OK;
 }
 
-// 2-D fp32 map over a K-major array: inner extent `inner` (k), outer extent `outer` (rows), row pitch in elements.
-// transposed = false: box 32 (k, inner) x 128 rows with the 128-byte swizzle; transposed = true (weight stored with n
-// contiguous): box 128 (n, inner) x 32 k-rows, no swizzle.
-static int make_map(EncodeTiledFn enc, CUtensorMap *map, const float *base, int64_t inner, int64_t outer, int64_t pitch, bool transposed = false)
+// Weight map: fp32, inner extent `inner`, outer extent `outer`, row pitch in elements.  K-major: box 32 (k) x 128 rows with the
+// 128-byte swizzle; transposed (n contiguous): box 128 (n) x 32 k-rows, no swizzle.
+static int make_w_map(EncodeTiledFn enc, CUtensorMap *map, const float *base, int64_t inner, int64_t outer, int64_t pitch, bool transposed)
 {
     cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)outer};
     cuuint64_t strides[1] = {(cuuint64_t)pitch * sizeof(float)};
-    cuuint32_t box[2] = {transposed ? 128u : (cuuint32_t)TC_BK, transposed ? (cuuint32_t)TC_BK : 128u};
+    cuuint32_t box[2] = {transposed ? (cuuint32_t)TC_BN : (cuuint32_t)TC_WK, transposed ? (cuuint32_t)TC_WK : (cuuint32_t)TC_BN};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(base), dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, transposed ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     CN_REQUIRE(r == CUDA_SUCCESS, CN_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d (inner %lld outer %lld pitch %lld)", (int)r,
                (long long)inner, (long long)outer, (long long)pitch);
+    return CN_OK;
+}
+
+// Activation plane: fp16, k contiguous with pitch Kp, box 64 k x 128 rows, 128-byte swizzle.
+static int make_a_map(EncodeTiledFn enc, CUtensorMap *map, const uint16_t *base, int64_t Kp, int64_t M)
+{
+    cuuint64_t dims[2] = {(cuuint64_t)Kp, (cuuint64_t)M};
+    cuuint64_t strides[1] = {(cuuint64_t)Kp * sizeof(uint16_t)};
+    cuuint32_t box[2] = {(cuuint32_t)TC_AK, (cuuint32_t)TC_BM};
+    cuuint32_t estr[2] = {1, 1};
+    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<uint16_t *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    CN_REQUIRE(r == CUDA_SUCCESS, CN_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d (activation planes %lld x %lld)", (int)r, (long long)M, (long long)Kp);
     return CN_OK;
 }
 
@@ -915,55 +1148,60 @@ bool cn_gemm_tc_supported(cn_context *, int transA, int transB, int64_t M, int64
     return true;
 }
 
-static int pick_splits(int64_t tiles, int kb_total, int sm_count)
-{
-    if (tiles >= 2 * (int64_t)sm_count) return 1;
-    int best = 1;
-    double best_score = -1.0;
-    for (int s = 1; s <= 32; ++s) {
-        if (kb_total / s < 8) break;   // keep at least 8 K blocks (256 k) per split
-        const int64_t units = tiles * s;
-        const int64_t waves = (units + sm_count - 1) / sm_count;
-        const double eff = (double)units / (double)(waves * sm_count);
-        const double score = eff - 0.004 * s;   // prefer fewer splits when the fill is about equal
-        if (score > best_score) { best_score = score; best = s; }
-    }
-    return best;
-}
-
 template <int NT, bool MODE3X, bool TRANSB>
-static int launch_cfg(const CUtensorMap &mw, const CUtensorMap &mhi, const CUtensorMap &mlo, const TcParams &prm, int64_t grid, cudaStream_t s)
+static int launch_cfg(const CUtensorMap &mw, const CUtensorMap &mhi, const CUtensorMap &mlo, const TcParams &prm, int64_t grid, int dev, cudaStream_t s)
 {
     static bool attr_set[64] = {};   // per device: the attribute belongs to the device's copy of the function
-    int dev = 0;
-    CN_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
         CN_CUDA(cudaFuncSetAttribute(cn_gemm_tc_kernel<NT, MODE3X, TRANSB>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<NT>::SMEM_BYTES));
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
-    cn_gemm_tc_kernel<NT, MODE3X, TRANSB><<<(unsigned)grid, TcCfg<NT>::THREADS, TcCfg<NT>::SMEM_BYTES, s>>>(mw, mhi, mlo, prm);
-    CN_CUDA(cudaGetLastError());
+    CN_CUDA(cn_launch_pdl(cn_gemm_tc_kernel<NT, MODE3X, TRANSB>, dim3((unsigned)grid), TcCfg<NT>::THREADS, TcCfg<NT>::SMEM_BYTES, s, mw, mhi, mlo, prm));
     cn_count_launch();
     return CN_OK;
 }
 
-int cn_gemm_tc_split_activations(cn_context *ctx, int transA, int64_t M, int64_t K, const float *A, int64_t lda, float *hi, float *lo,
-                                 cudaStream_t s)
+// Geometry of the planes of an M x K operand in one allocation: hi, lo (only in the 3x mode), inverse scales.
+void cn_plane_layout(int64_t M, int64_t K, int mode, cn_planes *pl)
 {
-    (void)ctx;
-    const int64_t Kpad = (K + TC_BK - 1) / TC_BK * TC_BK;
-    const int64_t tiles_k = Kpad / 32, tiles_mm = (M + 31) / 32;
-    CN_REQUIRE(tiles_k * tiles_mm < (1LL << 31), CN_ERR_UNSUPPORTED, "cn_gemm_f32: activation matrix too large for the split pre-pass");
-    if (transA) {
+    pl->Kp = (K + TC_AK - 1) / TC_AK * TC_AK;
+    pl->m_pad = (M + TC_BM - 1) / TC_BM * TC_BM;
+    pl->groups = (K + TC_GROUP_K - 1) / TC_GROUP_K;
+    const size_t plane = ((size_t)M * pl->Kp * sizeof(uint16_t) + 255) & ~(size_t)255;
+    pl->lo_off = mode == CN_GEMM_3XTF32 ? plane : 0;
+    pl->inv_off = plane * (mode == CN_GEMM_3XTF32 ? 2 : 1);
+    pl->bytes = pl->inv_off + (size_t)pl->groups * pl->m_pad * sizeof(float);
+}
+
+static int act_planes(cn_context *ctx, int transA, int64_t M, int64_t K, const float *A, int64_t lda, const cn_coded_src *cs, const cn_planes &pl,
+                      uint8_t *base, cudaStream_t s)
+{
+    uint16_t *hi = reinterpret_cast<uint16_t *>(base), *lo = pl.lo_off ? reinterpret_cast<uint16_t *>(base + pl.lo_off) : nullptr;
+    float *inv = reinterpret_cast<float *>(base + pl.inv_off);
+    CN_REQUIRE(pl.groups * (pl.m_pad / 8) < (1LL << 31), CN_ERR_UNSUPPORTED, "cn_gemm_f32: activation matrix too large for the split pre-pass");
+    if (cs) {
+        ActCoded cd;
+        cd.codes = cs->codes; cd.scales = cs->scales; cd.tbl = ctx->d_tbl; cd.own_fp32 = cs->own_fp32;
+        cd.own_rank = cs->own_rank; cd.nranks = cs->nranks;
+        CN_CUDA(cn_launch_pdl(cn_act_planes_kernel<true>, dim3((unsigned)(pl.groups * (pl.m_pad / ACT_ROWS))), 256, (size_t)cs->nranks * 256 * sizeof(float), s,
+                              A, lda, M, K, pl.Kp, hi, lo, inv, pl.m_pad, cd));
+    } else if (transA) {
         const int vec_ok = ((lda & 3) == 0) && ((reinterpret_cast<uintptr_t>(A) & 15u) == 0);
-        dim3 grid((unsigned)((Kpad / 4 + 255) / 256), (unsigned)(M < 65535 ? M : 65535));
-        cn_act_split_t_kernel<<<grid, 256, 0, s>>>(A, lda, M, K, Kpad, hi, lo, vec_ok);
+        CN_CUDA(cn_launch_pdl(cn_act_planes_t_kernel, dim3((unsigned)(pl.groups * (pl.m_pad / 8))), 256, 0, s, A, lda, M, K, pl.Kp, hi, lo, inv, pl.m_pad,
+                              vec_ok));
     } else {
-        cn_act_split_kernel<<<(unsigned)(tiles_k * tiles_mm), 256, 0, s>>>(A, lda, M, K, Kpad, hi, lo, tiles_k);
+        CN_CUDA(cn_launch_pdl(cn_act_planes_kernel<false>, dim3((unsigned)(pl.groups * (pl.m_pad / ACT_ROWS))), 256, 0, s, A, lda, M, K, pl.Kp, hi, lo, inv,
+                              pl.m_pad, ActCoded()));
     }
-    CN_CUDA(cudaGetLastError());
     cn_count_launch();
     return CN_OK;
+}
+
+int cn_gemm_tc_split_activations(cn_context *ctx, int transA, int64_t M, int64_t K, const float *A, int64_t lda, int mode, void *planes, cudaStream_t s)
+{
+    cn_planes pl;
+    cn_plane_layout(M, K, mode, &pl);
+    return act_planes(ctx, transA, M, K, A, lda, nullptr, pl, (uint8_t *)planes, s);
 }
 
 int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, const float *B,
@@ -979,81 +1217,89 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
         if ((st = cn_status_block(ctx, &d_status)) != CN_OK) return st;
     }
     const bool mode3x = mode == CN_GEMM_3XTF32;
-    const int64_t Kpad = (K + TC_BK - 1) / TC_BK * TC_BK;
 
     // 1. activations -> K-major hi / lo planes (made here, or ahead of the call by cn_gemm_prepare)
-    const size_t plane_elems = (size_t)M * Kpad;
-    float *hi = nullptr, *lo = nullptr;
-    if (ws->prepared) {
+    cn_planes pl;
+    cn_plane_layout(M, K, mode, &pl);
+    uint8_t *planes = nullptr;
+    const bool ahead = ws->prepared != nullptr;
+    if (ahead) {
         const cn_prepared *pr = ws->prepared;
         ws->prepared = nullptr;
-        CN_REQUIRE(pr->filled && pr->M == M && pr->K == K && pr->Kpad == Kpad && pr->mode == mode, CN_ERR_SHAPE,
+        CN_REQUIRE(pr->filled && pr->M == M && pr->K == K && pr->mode == mode, CN_ERR_SHAPE,
                    "prepared activations are %lld x %lld for mode %d, the product wants %lld x %lld for mode %d", (long long)pr->M,
                    (long long)pr->K, pr->mode, (long long)M, (long long)K, mode);
-        hi = pr->hi;
-        lo = mode3x ? pr->lo : nullptr;
+        planes = (uint8_t *)pr->planes;
     } else {
-        void *planes = nullptr;
-        st = cn_gemm_scratch(ctx, CN_GEMM_SLOT_ASPLIT, plane_elems * sizeof(float) * (mode3x ? 2 : 1), &planes);
-        if (st != CN_OK) return st;
-        hi = (float *)planes;
-        lo = mode3x ? hi + plane_elems : nullptr;
-        if (ws->coded_src) {
-            const int64_t tiles_k = Kpad / 32, tiles_mm = (M + 31) / 32;
-            CN_REQUIRE(tiles_k * tiles_mm < (1LL << 31), CN_ERR_UNSUPPORTED, "cn_gemm_f32: activation matrix too large for the split pre-pass");
-            const cn_coded_src *cs = ws->coded_src;
-            ws->coded_src = nullptr;
-            CN_REQUIRE(!transA && lda == M, CN_ERR_UNSUPPORTED, "coded activations must be untransposed with ld = rows");
-            cn_act_split_coded_kernel<<<(unsigned)(tiles_k * tiles_mm), 256, (size_t)cs->nranks * 256 * sizeof(float), s>>>(
-                cs->codes, cs->scales, ctx->d_tbl, cs->own_fp32, cs->own_rank, cs->nranks, M, K, Kpad, hi, lo, tiles_k);
-            CN_CUDA(cudaGetLastError());
-            cn_count_launch();
-        } else if ((st = cn_gemm_tc_split_activations(ctx, transA, M, K, A, lda, hi, lo, s)) != CN_OK) {
-            return st;
-        }
+        void *buf = nullptr;
+        if ((st = cn_gemm_scratch(ctx, CN_GEMM_SLOT_ASPLIT, pl.bytes, &buf)) != CN_OK) return st;
+        planes = (uint8_t *)buf;
+        const cn_coded_src *cs = ws->coded_src;
+        ws->coded_src = nullptr;
+        CN_REQUIRE(!cs || (!transA && lda == M), CN_ERR_UNSUPPORTED, "coded activations must be untransposed with ld = rows");
+        if ((st = act_planes(ctx, transA, M, K, A, lda, cs, pl, planes, s)) != CN_OK) return st;
     }
 
-    // 2. tiling
-    const int prm_maxout = epi ? epi->maxout_level : 1;
-    int nt = (N >= 2048) ? 2 : 1;
+    // 2. work decomposition
+    const int maxout = epi ? epi->maxout_level : 1;
+    int nt = N > TC_BN ? 2 : 1;
     if (ws->force_nt == 1 || ws->force_nt == 2) nt = ws->force_nt;
-    const int64_t tiles_n = (N + nt * TC_BN - 1) / (nt * TC_BN), tiles_m = (M + TC_BM - 1) / TC_BM;
-    const int64_t tiles = tiles_n * tiles_m;
-    const int kb_total = (int)(Kpad / TC_BK);
-    int splits = pick_splits(tiles, kb_total, ctx->sm_count);
-    if (ws->force_splits >= 1 && ws->force_splits <= kb_total) splits = ws->force_splits;
-    if (prm_maxout > 1) splits = 1;   // the split-K reduction kernel has no maxout; such layers are small
-    int kb_per_split = (kb_total + splits - 1) / splits;
-    splits = (kb_total + kb_per_split - 1) / kb_per_split;   // no empty split
-    CN_REQUIRE(tiles * splits < (1LL << 31), CN_ERR_UNSUPPORTED, "cn_gemm_f32: too many work units");
+    const int64_t tiles_n = (N + nt * TC_BN - 1) / (nt * TC_BN), tiles_m = (M + TC_BM - 1) / TC_BM, tiles = tiles_n * tiles_m;
+    const int kb_total = (int)((K + TC_WK - 1) / TC_WK);
+    const int64_t sms = ctx->sm_count;
+    int64_t full = 0, tail_ctas = 0;
+    if (maxout > 1) {
+        full = tiles;   // the reduction kernel has no maxout; such layers are small
+    } else if (ws->force_splits >= 1) {
+        const int64_t splits = ws->force_splits <= kb_total ? ws->force_splits : kb_total;
+        if (splits == 1 && !(peers && peers->npeers > 0)) full = tiles; else tail_ctas = tiles * splits;
+    } else {
+        // Whole tiles only, where the last round over the SMs is nearly full or cutting it would cost more than it saves: the
+        // reduction of a cut tail takes as long as about 12 K blocks of a CTA (8 us).  Peers take their tiles from the reduction.
+        const int64_t rounds = (tiles + sms - 1) / sms;
+        const bool push = peers && peers->npeers > 0;
+        if (!push && rounds * kb_total <= tiles * kb_total / sms + 12) {
+            full = tiles;
+        } else {
+            full = push ? 0 : tiles / sms * sms;
+            const int64_t rest = tiles - full;
+            tail_ctas = rest * kb_total / 6;   // at least six K blocks per CTA: shorter runs cost more in partial tiles than they save
+            if (tail_ctas > sms) tail_ctas = sms;
+            if (tail_ctas < rest) tail_ctas = rest < sms ? rest : sms;
+        }
+    }
+    const int64_t rest = tiles - full;
+    const int64_t grid = tail_ctas > (full < sms ? full : sms) ? tail_ctas : (full < sms ? full : sms);
+    CN_REQUIRE(tiles < (1LL << 29) && grid < (1LL << 30) && rest * nt * 4 < (1LL << 31), CN_ERR_UNSUPPORTED, "cn_gemm_f32: too many work units");
 
     TcParams prm;
-    prm.M = M; prm.N = N; prm.K = K;
+    prm.M = M; prm.N = N;
     prm.C = C; prm.ldc = ldc;
     prm.bias = epi ? epi->bias : nullptr;
     prm.act = epi ? epi->activation : CN_ACT_LINEAR;
-    prm.maxout_level = epi ? epi->maxout_level : 1;
+    prm.maxout_level = maxout;
     prm.argmax = epi ? epi->argmax_out : nullptr;
-    prm.tiles_n = tiles_n; prm.tiles_m = tiles_m;
-    prm.splits = splits; prm.kb_per_split = kb_per_split; prm.kb_total = kb_total;
-    prm.chain_kb = TC_CHAIN_DEFAULT;
-    if (ws->force_chain >= 1) prm.chain_kb = ws->force_chain;
+    prm.tiles_n = (int)tiles_n; prm.tiles_m = (int)tiles_m;
+    prm.full_tiles = (int)full; prm.tail_ctas = (int)tail_ctas; prm.kb_total = kb_total;
+    int chain = TC_GROUP_KB;
+    if (ws->force_chain >= 1)
+        while (chain > 1 && chain > ws->force_chain) chain >>= 1;
+    prm.chain_mask = chain - 1;
+    prm.a_inv = reinterpret_cast<const float *>(planes + pl.inv_off);
+    prm.m_pad = pl.m_pad;
     prm.partials = nullptr;
     prm.status = ws->d_status;
+    prm.w_ready = ahead ? 0 : 1;
     prm.npeers = 0;
-    prm.ready = nullptr;
     prm.peer_flags = nullptr;
     prm.nranks = 0; prm.my_rank = 0; prm.epoch = 0;
-    for (int i = 0; i < CN_MAX_PEERS; ++i) prm.peerC[i] = nullptr;
     if (peers && peers->npeers > 0) {
         prm.npeers = peers->npeers;
-        for (int i = 0; i < peers->npeers; ++i) prm.peerC[i] = peers->C[i];
-        prm.ready = peers->ready;
         prm.peer_flags = peers->peer_flags;
         prm.nranks = peers->nranks; prm.my_rank = peers->my_rank; prm.epoch = peers->epoch;
     }
-    if (splits > 1) {
-        const size_t part_bytes = (size_t)tiles * splits * nt * TC_BM * TC_BN * sizeof(float);
+    if (rest > 0) {
+        const size_t part_bytes = (size_t)(tail_ctas + rest) * nt * TC_BM * TC_BN * sizeof(float);
         void *buf = nullptr;
         st = cn_gemm_scratch(ctx, CN_GEMM_SLOT_SPLITK, part_bytes, &buf);
         if (st != CN_OK) return st;
@@ -1062,13 +1308,16 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
 
     // 3. tensor maps
     CUtensorMap mw, mhi, mlo;
-    if (transB) st = make_map(enc, &mw, B, N, K, ldb, true);   // stored N x K, n contiguous
-    else        st = make_map(enc, &mw, B, K, N, ldb);
+    if (transB) st = make_w_map(enc, &mw, B, N, K, ldb, true);   // stored N x K, n contiguous
+    else        st = make_w_map(enc, &mw, B, K, N, ldb, false);
     if (st != CN_OK) return st;
-    if ((st = make_map(enc, &mhi, hi, Kpad, M, Kpad)) != CN_OK) return st;
-    if ((st = make_map(enc, &mlo, mode3x ? lo : hi, Kpad, M, Kpad)) != CN_OK) return st;
+    if ((st = make_a_map(enc, &mhi, reinterpret_cast<const uint16_t *>(planes), pl.Kp, M)) != CN_OK) return st;
+    if (mode3x) {
+        if ((st = make_a_map(enc, &mlo, reinterpret_cast<const uint16_t *>(planes + pl.lo_off), pl.Kp, M)) != CN_OK) return st;
+    } else {
+        mlo = mhi;
+    }
 
-    const int64_t grid = tiles * splits;
     cudaEvent_t ev_stop = nullptr;
     if (ws->profile) {
         while (ws->prof_events.size() < ws->prof_used + 2) {
@@ -1079,8 +1328,9 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
         CN_CUDA(cudaEventRecord(ws->prof_events[ws->prof_used], s));
         ev_stop = ws->prof_events[ws->prof_used + 1];
         ws->prof_used += 2;
+        prm.w_ready = 0;   // the event stands between the pre-pass and this launch: keep the plain order
     }
-#define CN_LAUNCH(NTV, M3, TB) launch_cfg<NTV, M3, TB>(mw, mhi, mlo, prm, grid, s)
+#define CN_LAUNCH(NTV, M3, TB) launch_cfg<NTV, M3, TB>(mw, mhi, mlo, prm, grid, ctx->device, s)
     if (nt == 1) {
         if (transB) st = mode3x ? CN_LAUNCH(1, true, true) : CN_LAUNCH(1, false, true);
         else        st = mode3x ? CN_LAUNCH(1, true, false) : CN_LAUNCH(1, false, false);
@@ -1090,18 +1340,16 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
     }
 #undef CN_LAUNCH
     if (st != CN_OK) return st;
-    if (splits > 1) {
+    if (rest > 0) {
         ReduceParams rp;
-        rp.partials = prm.partials; rp.splits = splits; rp.nt = nt;
-        rp.tiles_n = tiles_n; rp.tiles_m = tiles_m; rp.M = M; rp.N = N;
+        rp.partials = prm.partials; rp.nt = nt; rp.tail_ctas = (int)tail_ctas; rp.kb_total = kb_total;
+        rp.tail_tiles = (int)rest; rp.full_tiles = (int)full; rp.tiles_m = (int)tiles_m; rp.M = M; rp.N = N;
         rp.C = C; rp.ldc = ldc; rp.bias = prm.bias; rp.act = prm.act;
         rp.npeers = prm.npeers;
-        for (int i = 0; i < CN_MAX_PEERS; ++i) rp.peerC[i] = prm.peerC[i];
-        rp.ready = prm.ready; rp.nranks = prm.nranks; rp.my_rank = prm.my_rank; rp.epoch = prm.epoch; rp.status = prm.status;
-        const int64_t quads = tiles * nt * (TC_BM * TC_BN / 4);
-        int64_t blocks = (quads + 255) / 256, cap = (int64_t)ctx->sm_count * 8;
-        cn_splitk_reduce_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, s>>>(rp);
-        CN_CUDA(cudaGetLastError());
+        for (int i = 0; i < CN_MAX_PEERS; ++i) rp.peerC[i] = prm.npeers > i ? peers->C[i] : nullptr;
+        rp.ready = prm.npeers > 0 ? peers->ready : nullptr;
+        rp.nranks = prm.nranks; rp.my_rank = prm.my_rank; rp.epoch = prm.epoch; rp.status = prm.status;
+        CN_CUDA(cn_launch_pdl(cn_splitk_reduce_kernel, dim3((unsigned)(rest * nt * 4)), 256, 0, s, rp));
         cn_count_launch();
     }
     if (ev_stop) CN_CUDA(cudaEventRecord(ev_stop, s));
