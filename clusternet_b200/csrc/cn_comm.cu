@@ -912,7 +912,7 @@ extern "C" int cn_dotmpi_from_coded_f32(cn_context *ctx, const cn_coded *A, int6
     const int G = ctx->comm ? ctx->comm->nranks : 1, rank = ctx->comm ? ctx->comm->rank : 0;
     int64_t start, cnt;
     cn_shard_cols(n_total, rank, G, &start, &cnt);
-    if (mode != CN_GEMM_FP32_SIMT && cnt > 0 &&
+    if (mode != CN_GEMM_FP32_SIMT && cnt > 0 && !cn_gemm_small_shape(ctx, M, cnt, K) &&
         cn_gemm_tc_supported(ctx, 0, 0, M, cnt, K, A->own_fp32, M, d_Wshard, K, d_C, M)) {
         if (!ctx->gemm) ctx->gemm = cn_gemm_workspace_new();
         cn_coded_src src;
@@ -928,7 +928,7 @@ extern "C" int cn_dotmpi_from_coded_f32(cn_context *ctx, const cn_coded *A, int6
         ctx->gemm->coded_src = nullptr;
         return st;
     }
-    // shapes the tensor-core kernel does not take: decode to fp32 scratch first
+    // small products, and shapes the streaming kernel does not take: decode to fp32 scratch first
     void *buf = nullptr;
     int st = cn_gemm_scratch(ctx, CN_GEMM_SLOT_MAXOUT, (size_t)M * K * sizeof(float), &buf);
     if (st != CN_OK) return st;
@@ -966,6 +966,14 @@ extern "C" int cn_gemm_prepare_create(cn_context *ctx, int64_t M, int64_t K, int
         delete p;
         return cn_cuda_fail(e, "cn_gemm_prepare_create");
     }
+    if (K <= CN_SMALL_MAX_K) {
+        p->raw_ld = (K + 3) / 4 * 4;
+        if ((e = cudaMalloc(&p->raw, (size_t)M * p->raw_ld * sizeof(float))) != cudaSuccess) {
+            cudaFree(p->planes);
+            delete p;
+            return cn_cuda_fail(e, "cn_gemm_prepare_create");
+        }
+    }
     *out = p;
     return CN_OK;
 }
@@ -974,6 +982,7 @@ extern "C" int cn_gemm_prepare_destroy(cn_prepared *p)
 {
     if (!p) return CN_OK;
     cudaFree(p->planes);
+    cudaFree(p->raw);
     delete p;
     return CN_OK;
 }
@@ -984,6 +993,14 @@ extern "C" int cn_gemm_prepare(cn_context *ctx, cn_prepared *p, int transA, cons
     CN_REQUIRE(lda >= (transA ? p->K : p->M), CN_ERR_SHAPE, "cn_gemm_prepare: leading dimension smaller than the stored rows");
     if (!ctx->gemm) ctx->gemm = cn_gemm_workspace_new();
     int st = cn_gemm_tc_split_activations(ctx, transA, p->M, p->K, d_A, lda, p->mode, p->planes, cn_stream(stream));
+    if (st == CN_OK && p->raw) {
+        // K-major copy for small products: row m at m * raw_ld
+        if (transA)
+            CN_CUDA(cudaMemcpy2DAsync(p->raw, p->raw_ld * sizeof(float), d_A, lda * sizeof(float), p->K * sizeof(float), p->M, cudaMemcpyDeviceToDevice,
+                                      cn_stream(stream)));
+        else
+            st = cn_transpose_pitched(d_A, lda, p->raw, p->raw_ld, p->K, p->M, cn_stream(stream));
+    }
     if (st == CN_OK) p->filled = true;
     return st;
 }

@@ -198,7 +198,31 @@ int cn_gemm_dispatch(cn_context *ctx, int transA, int transB, int64_t M, int64_t
     // maxout that cannot be fused: full product into scratch, then the stand-alone reduction
     float *target = d_C;
     int64_t target_ld = ldc;
-    bool tc_ok = mode != CN_GEMM_FP32_SIMT && cn_gemm_tc_supported(ctx, transA, transB, M, N, K, d_A, lda, d_B, ldb, d_C, ldc);
+    const bool tma_ok = mode != CN_GEMM_FP32_SIMT && cn_gemm_tc_supported(ctx, transA, transB, M, N, K, d_A, lda, d_B, ldb, d_C, ldc);
+    // Small products take one launch (see cn_gemm_small.cu), unless a test or sweep set the streaming kernel's knobs.  Products of a
+    // few thousand multiplications whose weights TMA cannot read stay on the FMA kernel, which adds along k in order.
+    cn_gemm_workspace *ws = ctx->gemm;
+    const bool tuned = ws && (ws->force_nt || ws->force_splits || ws->force_chain);
+    if (mode != CN_GEMM_FP32_SIMT && L == 1 && !tuned && !(ws && (ws->coded_src || ws->profile)) && cn_gemm_small_shape(ctx, M, N, K) &&
+        (tma_ok || M * N * K >= 4096)) {
+        const cn_prepared *pr = ws ? ws->prepared : nullptr;
+        if (!pr || pr->raw) {
+            if (pr) {
+                ws->prepared = nullptr;
+                CN_REQUIRE(pr->filled && pr->M == M && pr->K == K && pr->mode == mode, CN_ERR_SHAPE,
+                           "prepared activations are %lld x %lld for mode %d, the product wants %lld x %lld for mode %d", (long long)pr->M,
+                           (long long)pr->K, pr->mode, (long long)M, (long long)K, mode);
+                d_A = pr->raw;
+                lda = pr->raw_ld;
+                transA = 1;
+            }
+            const bool push = peers && peers->npeers > 0;
+            int st = cn_gemm_small_launch(ctx, transA, transB, M, N, K, d_A, lda, d_B, ldb, d_C, ldc, epi, mode, s, push ? peers : nullptr);
+            if (push && used_peers) *used_peers = st == CN_OK;
+            return st;
+        }
+    }
+    const bool tc_ok = tma_ok;
     bool fused_maxout = tc_ok && (L == 1 || cn_gemm_tc_can_fuse_maxout(L));
     if (L > 1 && !fused_maxout) {
         void *p = nullptr;

@@ -36,7 +36,8 @@ void cn_plane_layout(int64_t M, int64_t K, int mode, cn_planes *pl);
 struct cn_prepared {
     cn_context *ctx = nullptr;
     void *planes = nullptr;
-    int64_t M = 0, K = 0;
+    float *raw = nullptr;       // K-major fp32 copy with pitch raw_ld, for products small enough for the one-launch kernel
+    int64_t M = 0, K = 0, raw_ld = 0;
     int mode = 0;
     bool filled = false;
 };
@@ -84,6 +85,11 @@ int cn_gemm_tc_split_activations(cn_context *ctx, int transA, int64_t M, int64_t
 int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda,
                       const float *B, int64_t ldb, float *C, int64_t ldc, const cn_epilogue *epi, int mode, cudaStream_t s,
                       const cn_peer_out *peers = nullptr, int transA = 0, int transB = 0);
+// Small products in one launch (cn_gemm_small.cu): whether a shape is one, and the launch.  Takes any layout and alignment.
+bool cn_gemm_small_shape(const cn_context *ctx, int64_t M, int64_t N, int64_t K);
+#define CN_SMALL_MAX_K 16384   // no shape with a longer inner dimension is small
+int cn_gemm_small_launch(cn_context *ctx, int transA, int transB, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, const float *B, int64_t ldb,
+                         float *C, int64_t ldc, const cn_epilogue *epi, int mode, cudaStream_t s, const cn_peer_out *peers);
 // cn_gemm_f32 with optional peer windows; *used_peers tells whether the launch took them (tensor-core path only).
 int cn_gemm_dispatch(cn_context *ctx, int transA, int transB, int64_t M, int64_t N, int64_t K, const float *d_A, int64_t lda,
                      const float *d_B, int64_t ldb, float *d_C, int64_t ldc, const cn_epilogue *epi, int mode, void *stream,

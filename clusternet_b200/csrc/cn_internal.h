@@ -70,6 +70,8 @@ void cn_gemm_workspace_free(cn_context *ctx);
 // Device status block of the context (word 0: code of the first bounded wait that ran out, read by cn_gemm_check_status),
 // allocated and zeroed on first use.
 int cn_status_block(cn_context *ctx, unsigned int **d_status);
+// cn_layout.cu: out (C x R, row-major, pitch ldo) = transpose of in (R x C, row-major, pitch ldi)
+int cn_transpose_pitched(const float *in, int64_t ldi, float *out, int64_t ldo, int64_t R, int64_t C, cudaStream_t s);
 // cn_comm.cu
 void cn_comm_state_free(cn_context *ctx);
 // Addresses of a symmetric buffer on every rank ([nranks] entries, own rank = local); false if `local` is not inside one.

@@ -7,9 +7,9 @@
 #define TP_TILE 32
 #define TP_ROWS 8
 
-// out (C x R, row-major) = transpose of in (R x C, row-major).  One CTA per 32x32 tile, linear tile index.
+// out (C x R, row-major, pitch ldo) = transpose of in (R x C, row-major, pitch ldi).  One CTA per 32x32 tile, linear tile index.
 __global__ void __launch_bounds__(TP_TILE *TP_ROWS)
-cn_transpose_kernel(const float *in, float *out, int64_t R, int64_t C, int64_t tiles_c)
+cn_transpose_kernel(const float *in, int64_t ldi, float *out, int64_t ldo, int64_t R, int64_t C, int64_t tiles_c)
 {
     __shared__ float tile[TP_TILE][TP_TILE + 1];
     cn_pdl_launch_dependents();
@@ -21,14 +21,14 @@ cn_transpose_kernel(const float *in, float *out, int64_t R, int64_t C, int64_t t
 #pragma unroll
     for (int j = ty; j < TP_TILE; j += TP_ROWS) {
         const int64_t r = tr * TP_TILE + j;
-        if (r < R && c < C) tile[j][tx] = in[r * C + c];
+        if (r < R && c < C) tile[j][tx] = in[r * ldi + c];
     }
     __syncthreads();
     const int64_t r2 = tr * TP_TILE + tx;
 #pragma unroll
     for (int j = ty; j < TP_TILE; j += TP_ROWS) {
         const int64_t c2 = tc * TP_TILE + j;
-        if (r2 < R && c2 < C) out[c2 * R + r2] = tile[tx][j];
+        if (r2 < R && c2 < C) out[c2 * ldo + r2] = tile[tx][j];
     }
 }
 
@@ -40,16 +40,18 @@ __global__ void cn_fill_kernel(float *A, int64_t n, float v)
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) A[i] = v;
 }
 
-static int transpose_launch(const float *in, float *out, int64_t R, int64_t C, cudaStream_t s)
+int cn_transpose_pitched(const float *in, int64_t ldi, float *out, int64_t ldo, int64_t R, int64_t C, cudaStream_t s)
 {
     if (R == 0 || C == 0) return CN_OK;
     const int64_t tiles_r = (R + TP_TILE - 1) / TP_TILE, tiles_c = (C + TP_TILE - 1) / TP_TILE;
     const int64_t tiles = tiles_r * tiles_c;
     CN_REQUIRE(tiles < (1LL << 31), CN_ERR_UNSUPPORTED, "transpose: %lld tiles exceed the grid limit", (long long)tiles);
-    CN_CUDA(cn_launch_pdl(cn_transpose_kernel, dim3((unsigned)tiles), TP_TILE * TP_ROWS, 0, s, in, out, R, C, tiles_c));
+    CN_CUDA(cn_launch_pdl(cn_transpose_kernel, dim3((unsigned)tiles), TP_TILE * TP_ROWS, 0, s, in, ldi, out, ldo, R, C, tiles_c));
     cn_count_launch();
     return CN_OK;
 }
+
+static int transpose_launch(const float *in, float *out, int64_t R, int64_t C, cudaStream_t s) { return cn_transpose_pitched(in, C, out, R, R, C, s); }
 
 // A row-major rows x cols array is the transpose of the col-major array of the same logical matrix.
 extern "C" int cn_to_col_major(cn_context *ctx, const float *d_src, float *d_dst, int64_t rows, int64_t cols, void *stream)
