@@ -90,9 +90,6 @@ class Context:
         h = ctypes.c_void_p()
         check(self.lib.cn_context_create(device, self.codebook.ctypes.data, ctypes.byref(h)))
         self.h = h
-        # one epilogue record for all products of the context (the call reads it before it returns)
-        self._epi = Epilogue(None, 0, 0, None)
-        self._epi_ref = ctypes.byref(self._epi)
 
     def close(self):
         if getattr(self, "h", None):
@@ -180,10 +177,10 @@ class Context:
         L = maxout_level if maxout_level and maxout_level > 1 else 1
         if out is None:
             out = self.empty(M, N // L)
-        epi = self._epi
-        epi.bias, epi.activation, epi.maxout_level, epi.argmax_out = _ptr(bias), int(activation), int(maxout_level), _ptr(argmax_out)
+        # a record of its own for every call: the call runs without the interpreter lock, so another thread may be in here too
+        epi = Epilogue(_ptr(bias), int(activation), int(maxout_level), _ptr(argmax_out))
         check(self.lib.cn_gemm_f32(self.h, int(transA), int(transB), M, N, K, _ptr(A), a_rows, _ptr(B), b_rows, _ptr(out), M,
-                                   self._epi_ref, int(mode), self.stream_ptr()))
+                                   ctypes.byref(epi), int(mode), self.stream_ptr()))
         return out
 
     def gemm_check(self):
@@ -267,9 +264,8 @@ class Context:
     def dotmpi(self, A, Wshard, n_total, out=None, bias=None, activation=_lib.ACT_LINEAR, mode=_lib.GEMM_3XTF32, exchange=0):
         K, M = A.shape
         out = out if out is not None else self.empty(M, n_total)
-        epi = self._epi
-        epi.bias, epi.activation, epi.maxout_level, epi.argmax_out = _ptr(bias), int(activation), 0, None
-        check(self.lib.cn_dotmpi_f32(self.h, M, K, n_total, _ptr(A), _ptr(Wshard), _ptr(out), self._epi_ref, int(mode),
+        epi = Epilogue(_ptr(bias), int(activation), 0, None)
+        check(self.lib.cn_dotmpi_f32(self.h, M, K, n_total, _ptr(A), _ptr(Wshard), _ptr(out), ctypes.byref(epi), int(mode),
                                      int(exchange), self.stream_ptr()))
         return out
 
