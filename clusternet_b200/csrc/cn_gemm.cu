@@ -3,8 +3,8 @@
 // cn_gemm_f32 takes over the cublasSgemm call of ClusterNet::dot (source/clusterNet.cpp:404-487): column-
 // major operands, alpha = 1, beta = 0, optional transposes, shape check first.  Shapes the tensor-core
 // kernel can take (see cn_gemm_tc.cu) go there; everything else — tiny matrices such as the reference's
-// 2x3 . 3x2 known-answer tests, a weight pitch that is not a multiple of 4 — runs on the fp32 FMA kernel
-// below, which accumulates along k in order and therefore reproduces plain fp32 dot products exactly.
+// 2x3 . 3x2 known-answer tests — runs on the fp32 FMA kernel below, which accumulates along k in order and
+// therefore reproduces plain fp32 dot products exactly.
 #include <stdlib.h>
 #include "cn_epilogue.cuh"
 #include "cn_gemm.h"
@@ -203,27 +203,14 @@ int cn_gemm_dispatch(cn_context *ctx, int transA, int transB, int64_t M, int64_t
     // few thousand multiplications whose weights TMA cannot read stay on the FMA kernel, which adds along k in order.
     cn_gemm_workspace *ws = ctx->gemm;
     const bool tuned = ws && (ws->force_nt || ws->force_splits || ws->force_chain);
-    if (mode != CN_GEMM_FP32_SIMT && L == 1 && !tuned && !(ws && (ws->coded_src || ws->profile)) && cn_gemm_small_shape(ctx, M, N, K) &&
-        (tma_ok || M * N * K >= 4096)) {
-        const cn_prepared *pr = ws ? ws->prepared : nullptr;
-        if (!pr || pr->raw) {
-            if (pr) {
-                ws->prepared = nullptr;
-                CN_REQUIRE(pr->filled && pr->M == M && pr->K == K && pr->mode == mode, CN_ERR_SHAPE,
-                           "prepared activations are %lld x %lld for mode %d, the product wants %lld x %lld for mode %d", (long long)pr->M,
-                           (long long)pr->K, pr->mode, (long long)M, (long long)K, mode);
-                d_A = pr->raw;
-                lda = pr->raw_ld;
-                transA = 1;
-            }
-            const bool push = peers && peers->npeers > 0;
-            int st = cn_gemm_small_launch(ctx, transA, transB, M, N, K, d_A, lda, d_B, ldb, d_C, ldc, epi, mode, s, push ? peers : nullptr);
-            if (push && used_peers) *used_peers = st == CN_OK;
-            return st;
-        }
-    }
-    const bool tc_ok = tma_ok;
-    bool fused_maxout = tc_ok && (L == 1 || cn_gemm_tc_can_fuse_maxout(L));
+    const cn_prepared *pr = ws ? ws->prepared : nullptr;
+    const bool small = mode != CN_GEMM_FP32_SIMT && (L == 1 || ldc == M) && !tuned && !(ws && (ws->coded_src || ws->profile)) && (!pr || pr->raw) &&
+                       cn_gemm_small_shape(ctx, M, N, K) && (tma_ok || M * N * K >= 4096);
+    // Weights that TMA cannot read as they are keep fp32-level accuracy in every mode: the fp32 kernel took them before.
+    const int tc_mode = tma_ok ? mode : CN_GEMM_3XTF32;
+    const bool tc_ok = tma_ok || (mode != CN_GEMM_FP32_SIMT && M * N * K >= 4096 && cn_gemm_tc_any_supported(transB, M, N, K, d_B));
+    // a small product and its maxout are two launches as well, and the maxima are those of the very product a call without maxout gives
+    const bool fused_maxout = tma_ok && (L == 1 || (!small && cn_gemm_tc_can_fuse_maxout(L)));
     if (L > 1 && !fused_maxout) {
         void *p = nullptr;
         int st = cn_gemm_scratch(ctx, CN_GEMM_SLOT_MAXOUT, (size_t)M * N * sizeof(float), &p);
@@ -233,14 +220,27 @@ int cn_gemm_dispatch(cn_context *ctx, int transA, int transB, int64_t M, int64_t
         CN_REQUIRE(ldc == M, CN_ERR_UNSUPPORTED, "cn_gemm_f32: un-fused maxout needs ldc == M");
     }
     int st;
-    if (tc_ok) {
+    if (small) {
+        if (pr) {
+            ws->prepared = nullptr;
+            CN_REQUIRE(pr->filled && pr->M == M && pr->K == K && pr->mode == mode, CN_ERR_SHAPE,
+                       "prepared activations are %lld x %lld for mode %d, the product wants %lld x %lld for mode %d", (long long)pr->M,
+                       (long long)pr->K, pr->mode, (long long)M, (long long)K, mode);
+            d_A = pr->raw;
+            lda = pr->raw_ld;
+            transA = 1;
+        }
+        const bool push = peers && peers->npeers > 0 && L == 1;
+        st = cn_gemm_small_launch(ctx, transA, transB, M, N, K, d_A, lda, d_B, ldb, target, target_ld, epi, tc_mode, s, push ? peers : nullptr);
+        if (push && used_peers) *used_peers = st == CN_OK;
+    } else if (tc_ok) {
         cn_epilogue e2;
         e2.bias = bias;
         e2.activation = act;
         e2.maxout_level = fused_maxout ? L : 1;
         e2.argmax_out = fused_maxout ? argmax : nullptr;
-        const bool push = peers && peers->npeers > 0 && L == 1;
-        st = cn_gemm_tc_launch(ctx, M, N, K, d_A, lda, d_B, ldb, target, target_ld, &e2, mode, s, push ? peers : nullptr, transA, transB);
+        const bool push = peers && peers->npeers > 0 && L == 1 && tma_ok;
+        st = cn_gemm_tc_launch(ctx, M, N, K, d_A, lda, d_B, ldb, target, target_ld, &e2, tc_mode, s, push ? peers : nullptr, transA, transB);
         if (push && used_peers) *used_peers = true;
     } else {
         st = simt_launch(ctx, transA, transB, M, N, K, d_A, lda, d_B, ldb, target, target_ld, bias, act, s);

@@ -78,6 +78,8 @@ struct cn_peer_out {
 
 bool cn_gemm_tc_supported(cn_context *ctx, int transA, int transB, int64_t M, int64_t N, int64_t K,
                           const float *A, int64_t lda, const float *B, int64_t ldb, const float *C, int64_t ldc);
+// Weights of any pitch and alignment: the same kernel in its 3x mode, no peers, no prepared or coded activations.
+bool cn_gemm_tc_any_supported(int transB, int64_t M, int64_t N, int64_t K, const float *B);
 bool cn_gemm_tc_can_fuse_maxout(int level);
 // the activation pre-pass alone, into caller-owned planes of cn_plane_layout's size
 int cn_gemm_tc_split_activations(cn_context *ctx, int transA, int64_t M, int64_t K, const float *A, int64_t lda, int mode, void *planes,

@@ -48,23 +48,46 @@
 #define TC_WK 32           // k per W block: one 128-byte swizzle row of fp32
 #define TC_AK 64           // k per activation stage: one 128-byte swizzle row of fp16
 #define TC_W_TILE_BYTES (TC_BN * TC_WK * 4)
+
+// How the weights lie in memory: k contiguous or n contiguous ("transposed"), the rows of that layout 16-byte aligned or not.
+//
+// TMA wants 16-byte aligned rows.  For any other pitch or base the rows of the stored matrix are read as four tensors: rows
+// r, r + 4, r + 8, ... lie 4 * pitch floats = 16 * pitch bytes apart, a multiple of 16 for every pitch, and all start at the same
+// offset d_r of 0 to 3 floats behind a 16-byte boundary.  Tensor r starts at that boundary and is d_r floats wider; its box is four
+// floats wider than the tile, and the converters begin to read d_r floats in.  What is read to the left of a row is not used; behind
+// its end and below the last row TMA fills with zeros, as for aligned weights.  Every weight is still read from memory once, with
+// no copy of the matrix.
+enum { W_K = 0, W_N = 1, W_K_ANY = 2, W_N_ANY = 3 };
+#define TC_CLASSES 4
+#define TC_WK_PITCH (TC_WK + 4)                                  // floats per row of a W_K_ANY box (32 rows), conflict-free for odd pitches
+#define TC_WK_CLASS_BYTES (TC_BN / TC_CLASSES * TC_WK_PITCH * 4)
+#define TC_WN_PITCH (TC_BN + 4)                                  // floats per row of a W_N_ANY box (8 rows)
+#define TC_WN_CLASS_BYTES (TC_WK / TC_CLASSES * TC_WN_PITCH * 4)
+static_assert(TC_WK_CLASS_BYTES % 128 == 0 && TC_WN_CLASS_BYTES % 128 == 0, "TMA destinations");
+__host__ __device__ constexpr bool w_any(int wk) { return wk >= W_K_ANY; }
+__host__ __device__ constexpr int w_box_bytes(int wk)
+{
+    return wk == W_K_ANY ? TC_CLASSES * TC_WK_CLASS_BYTES : wk == W_N_ANY ? TC_CLASSES * TC_WN_CLASS_BYTES : TC_W_TILE_BYTES;
+}
 #define TC_A_TILE_BYTES (TC_BM * TC_AK * 2)
 #define TC_GROUP_K CN_PLANE_GROUP_K
 #define TC_GROUP_KB (TC_GROUP_K / TC_WK)
 #define TC_DRAIN_SLEEP_NS 100   // poll interval of the drain warps while a chain accumulates
 
-template <int NT>
+template <int NT, int WK>
 struct TcCfg {
     static constexpr int THREADS = 128 + 256 * NT;    // WG0 (producers, MMA), per W tile one converter and one drain warpgroup
     // Two shared-memory rings with their own depth: raw W blocks (released by the converters as soon as they have
     // been read) and activation hi / lo tiles (released when the MMAs that read them retire).
     static constexpr int W_STAGES = NT == 1 ? 6 : 3;
     static constexpr int A_STAGES = 3;
-    static constexpr int W_STAGE_BYTES = NT * TC_W_TILE_BYTES;
+    static constexpr int W_TILE_BYTES = w_any(WK) ? TC_CLASSES * TC_WK_CLASS_BYTES : TC_W_TILE_BYTES;
+    static constexpr int W_STAGE_BYTES = NT * W_TILE_BYTES;
     static constexpr int A_STAGE_BYTES = 2 * TC_A_TILE_BYTES;
     static constexpr int W_RING = 0;
     static constexpr int A_RING = W_STAGES * W_STAGE_BYTES;
     static constexpr int RING_BYTES = A_RING + A_STAGES * A_STAGE_BYTES;
+    static_assert(A_RING % 1024 == 0, "swizzled tiles");
     static constexpr int TMEM_STAGES = 4;
     static constexpr int ACC_BUFS = NT == 1 ? 2 : 1;  // accumulators per W tile
     static constexpr int ACC_COL = 0;                 // NT * ACC_BUFS accumulators of 128 columns
@@ -110,6 +133,7 @@ struct TcParams {
     int64_t m_pad;
     float *partials;        // [slot][w][32 quads of m][128 n] float4: slot = CTA + tile - full_tiles
     unsigned int *status;
+    uint32_t w_shift;       // byte r: d_r of the weights' rows r, r + 4, ... (see W_K_ANY)
     int w_ready;            // nothing before the pre-pass still writes W: it may be loaded before the pre-pass has finished
     // fused all-gather: the peers are told that this rank's C may be overwritten; the tiles go to them in the reduction
     int npeers;
@@ -397,33 +421,40 @@ cn_act_planes_t_kernel(const float *A, int64_t lda, int64_t M, int64_t K, int64_
 }
 
 // -------------------------------------------------------------------------------------------------- main kernel
-// Four consecutive k of one row of a 128 x 32 W tile (chunk c of 8).
-// TRANSB: the weight operand is stored transposed (N x K column-major, n contiguous).  Its tiles arrive in shared
-// memory as [32 k][128 n] without swizzle and are read column-wise (conflict-free: consecutive lanes read consecutive n).
-// `base` is the address tc_row_base gives.
-template <bool TRANSB>
-__device__ __forceinline__ uint32_t tc_row_base(uint32_t tile, int row)
+// Four consecutive k of one row of a 128 x 32 W tile (chunk c of 8).  `base` is the address tc_row_base gives.
+// W_N: the tiles arrive in shared memory as [32 k][128 n] without swizzle and are read column-wise (conflict-free: consecutive
+// lanes read consecutive n).  The _ANY layouts lie in four boxes, one per class of rows.
+template <int WK>
+__device__ __forceinline__ uint32_t tc_row_base(uint32_t tile, int row, uint32_t w_shift)
 {
+    if (WK == W_N || WK == W_N_ANY) return tile + row * 4;
+    if (WK == W_K_ANY) return tile + (row & 3) * TC_WK_CLASS_BYTES + (row >> 2) * (TC_WK_PITCH * 4) + ((w_shift >> ((row & 3) * 8)) & 0xffu) * 4;
     // 16-byte chunk c of row r sits at chunk position c ^ (r & 7) under the 128-byte swizzle (tiles are 1024-byte aligned)
-    return TRANSB ? tile + row * 4 : tile + row * 128 + ((row & 7) << 4);
+    return tile + row * 128 + ((row & 7) << 4);
 }
-template <bool TRANSB>
-__device__ __forceinline__ float4 tc_read4(uint32_t base, int c)
+template <int WK>
+__device__ __forceinline__ float4 tc_read4(uint32_t base, int c, uint32_t w_shift)
 {
-    if (TRANSB)
+    if (WK == W_N)
         return make_float4(lds1(base + (4 * c) * (TC_BN * 4)), lds1(base + (4 * c + 1) * (TC_BN * 4)), lds1(base + (4 * c + 2) * (TC_BN * 4)),
                            lds1(base + (4 * c + 3) * (TC_BN * 4)));
+    if (WK == W_K_ANY) return make_float4(lds1(base + 16 * c), lds1(base + 16 * c + 4), lds1(base + 16 * c + 8), lds1(base + 16 * c + 12));
+    if (WK == W_N_ANY) {
+        const uint32_t q = base + c * (TC_WN_PITCH * 4);
+        return make_float4(lds1(q + (w_shift & 0xffu) * 4), lds1(q + TC_WN_CLASS_BYTES + ((w_shift >> 8) & 0xffu) * 4),
+                           lds1(q + 2 * TC_WN_CLASS_BYTES + ((w_shift >> 16) & 0xffu) * 4), lds1(q + 3 * TC_WN_CLASS_BYTES + (w_shift >> 24) * 4));
+    }
     return lds4(base ^ (c << 4));
 }
 
 // One k-step (16 consecutive k of column n) of one row, scaled by sc -> hl[0..7] packed high parts, hl[8..15] packed low parts.
 // Returns the running packed largest |high part|: a half equal to 0x7c00 means that a value left fp16's range.
-template <bool MODE3X, bool TRANSB>
-__device__ __forceinline__ void tc_convert_step(uint32_t base, int step, uint64_t sc2, uint32_t (&hl)[16], uint32_t &top)
+template <bool MODE3X, int WK>
+__device__ __forceinline__ void tc_convert_step(uint32_t base, uint32_t w_shift, int step, uint64_t sc2, uint32_t (&hl)[16], uint32_t &top)
 {
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
-        const float4 v = tc_read4<TRANSB>(base, step * 4 + c);
+        const float4 v = tc_read4<WK>(base, step * 4 + c, w_shift);
         tc_split2<MODE3X>(tc_mul2(tc_pack2(v.x, v.y), sc2), hl[2 * c], hl[8 + 2 * c]);
         tc_split2<MODE3X>(tc_mul2(tc_pack2(v.z, v.w), sc2), hl[2 * c + 1], hl[8 + 2 * c + 1]);
         asm("max.xorsign.abs.f16x2 %0, %0, %1;" : "+r"(top) : "r"(hl[2 * c]));
@@ -431,18 +462,23 @@ __device__ __forceinline__ void tc_convert_step(uint32_t base, int step, uint64_
     }
 }
 
-template <bool TRANSB>
-__device__ __forceinline__ uint32_t tc_row_amax(uint32_t base)
+template <int WK>
+__device__ __forceinline__ uint32_t tc_row_amax(uint32_t base, uint32_t w_shift)
 {
     uint32_t amax = 0u;
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
-        const float4 v = tc_read4<TRANSB>(base, c);
+        const float4 v = tc_read4<WK>(base, c, w_shift);
         amax = max(max(amax, __float_as_uint(v.x) & 0x7fffffffu), max(__float_as_uint(v.y) & 0x7fffffffu, __float_as_uint(v.z) & 0x7fffffffu));
         amax = max(amax, __float_as_uint(v.w) & 0x7fffffffu);
     }
     return amax;
 }
+
+// Tensor maps of the weights: one, or one per class of rows (W_K_ANY, W_N_ANY).
+struct WMaps {
+    CUtensorMap map[TC_CLASSES];
+};
 
 // Warp roles (warpgroups of 4 warps so that register budgets can be moved between them):
 //   WG0  warp 0: TMA producer for W, warp 1: MMA issuer of W tile 0 + TMEM owner, warp 2: TMA producer for the
@@ -458,12 +494,12 @@ __device__ __forceinline__ uint32_t tc_row_amax(uint32_t base)
 // cut into chains of at most 512 k, which end where the activations' scale groups end: each chain starts a fresh TMEM
 // accumulator, and when it ends the drain warps read it with tcgen05.ld, remove both scales and add it, in round-to-nearest
 // fp32, to running sums that they keep in registers (one thread = one output column n, 128 sums = 128 rows m).
-template <int NT, bool MODE3X, bool TRANSB>
-__global__ void __launch_bounds__(TcCfg<NT>::THREADS, 1)
-cn_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_ahi,
+template <int NT, bool MODE3X, int WK>
+__global__ void __launch_bounds__(TcCfg<NT, WK>::THREADS, 1)
+cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CUtensorMap tm_ahi,
                   const __grid_constant__ CUtensorMap tm_alo, const __grid_constant__ TcParams p)
 {
-    using Cfg = TcCfg<NT>;
+    using Cfg = TcCfg<NT, WK>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     constexpr int B_WFULL = 0, B_WEMPTY = B_WFULL + Cfg::W_STAGES, B_AFULL = B_WEMPTY + Cfg::W_STAGES,
@@ -529,11 +565,20 @@ cn_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
                         ok = mbar_wait(wempty_bar(s), ((it / Cfg::W_STAGES) & 1u) ^ 1u, abort_flag, p.status, 1u);
                         if (!ok) break;
                         const uint32_t stage = smem_base + Cfg::W_RING + s * Cfg::W_STAGE_BYTES;
-                        mbar_expect_tx(wfull_bar(s), (uint32_t)Cfg::W_STAGE_BYTES);
+                        mbar_expect_tx(wfull_bar(s), (uint32_t)(NT * w_box_bytes(WK)));
 #pragma unroll
                         for (int t = 0; t < NT; ++t) {
-                            if (TRANSB) tma_load_2d(stage + t * TC_W_TILE_BYTES, &tm_w, wfull_bar(s), n0 + t * TC_BN, kb * TC_WK);
-                            else        tma_load_2d(stage + t * TC_W_TILE_BYTES, &tm_w, wfull_bar(s), kb * TC_WK, n0 + t * TC_BN);
+                            const uint32_t dst = stage + t * Cfg::W_TILE_BYTES;
+                            const int32_t n = n0 + t * TC_BN;
+                            if (WK == W_K) tma_load_2d(dst, &tm_w.map[0], wfull_bar(s), kb * TC_WK, n);
+                            if (WK == W_N) tma_load_2d(dst, &tm_w.map[0], wfull_bar(s), n, kb * TC_WK);
+                            if (w_any(WK)) {
+#pragma unroll
+                                for (int r = 0; r < TC_CLASSES; ++r) {
+                                    if (WK == W_K_ANY) tma_load_2d(dst + r * TC_WK_CLASS_BYTES, &tm_w.map[r], wfull_bar(s), kb * TC_WK, n / TC_CLASSES);
+                                    else               tma_load_2d(dst + r * TC_WN_CLASS_BYTES, &tm_w.map[r], wfull_bar(s), n, kb * (TC_WK / TC_CLASSES));
+                                }
+                            }
                         }
                     }
                 }
@@ -675,12 +720,12 @@ cn_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
                 ok = __all_sync(0xffffffffu, ok);   // the tcgen05 stores below need the whole warp
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t rowp = tc_row_base<TRANSB>(smem_base + Cfg::W_RING + s * Cfg::W_STAGE_BYTES + w * TC_W_TILE_BYTES, row);
+                const uint32_t rowp = tc_row_base<WK>(smem_base + Cfg::W_RING + s * Cfg::W_STAGE_BYTES + w * Cfg::W_TILE_BYTES, row, p.w_shift);
                 const bool chain_start = kb == seg.k0 || (kb & p.chain_mask) == 0;
                 if (chain_start) set = false;
                 if (!set) {
                     // nothing but zeros of this row is in the accumulator: any scale is right for what is there
-                    const uint32_t amax = tc_row_amax<TRANSB>(rowp);
+                    const uint32_t amax = tc_row_amax<WK>(rowp, p.w_shift);
                     tc_scale<TC_W_EXP>(amax, sc, inv);
                     set = amax != 0u;
                 }
@@ -693,7 +738,7 @@ cn_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
 #pragma unroll 1
                     for (int step = 0; step < 2; ++step) {
                         uint32_t hl[16];
-                        tc_convert_step<MODE3X, TRANSB>(rowp, step, sc2, hl, top);
+                        tc_convert_step<MODE3X, WK>(rowp, p.w_shift, step, sc2, hl, top);
                         if (MODE3X) tc_st16(dst + step * 16, hl);
                         else        tc_st8(dst + step * 16, hl);
                     }
@@ -702,7 +747,7 @@ cn_gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constan
                     if (grew || !__any_sync(0xffffffffu, over)) break;
                     // rare: a row's magnitudes grew more than fourfold since its chain began: new scale, and once more
                     grew = true;
-                    if (over) tc_scale<TC_W_EXP>(tc_row_amax<TRANSB>(rowp), sc, inv);
+                    if (over) tc_scale<TC_W_EXP>(tc_row_amax<WK>(rowp, p.w_shift), sc, inv);
                     tc_wait_st();
                     __syncwarp();
                 }
@@ -980,19 +1025,42 @@ static int get_encode_fn(cn_context *ctx, EncodeTiledFn *out)
     return CN_OK;
 }
 
-// Weight map: fp32, inner extent `inner`, outer extent `outer`, row pitch in elements.  K-major: box 32 (k) x 128 rows with the
-// 128-byte swizzle; transposed (n contiguous): box 128 (n) x 32 k-rows, no swizzle.
-static int make_w_map(EncodeTiledFn enc, CUtensorMap *map, const float *base, int64_t inner, int64_t outer, int64_t pitch, bool transposed)
+// Weight map: fp32, inner extent `inner`, outer extent `outer`, row pitch in elements, box in elements.  The 128-byte swizzle for
+// 128-byte box rows that the converters read in 16-byte chunks (W_K), none otherwise.
+static int make_w_map(EncodeTiledFn enc, CUtensorMap *map, const float *base, int64_t inner, int64_t outer, int64_t pitch, int box_inner, int box_outer,
+                      bool swizzle)
 {
     cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)outer};
     cuuint64_t strides[1] = {(cuuint64_t)pitch * sizeof(float)};
-    cuuint32_t box[2] = {transposed ? (cuuint32_t)TC_BN : (cuuint32_t)TC_WK, transposed ? (cuuint32_t)TC_WK : (cuuint32_t)TC_BN};
+    cuuint32_t box[2] = {(cuuint32_t)box_inner, (cuuint32_t)box_outer};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(base), dims, strides, box, estr,
-                     CU_TENSOR_MAP_INTERLEAVE_NONE, transposed ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B,
+                     CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     CN_REQUIRE(r == CUDA_SUCCESS, CN_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d (inner %lld outer %lld pitch %lld)", (int)r,
                (long long)inner, (long long)outer, (long long)pitch);
+    return CN_OK;
+}
+
+// The maps of a stored matrix of `outer` rows of `inner` elements, and the offsets of the classes of rows.
+static int make_w_maps(EncodeTiledFn enc, WMaps *m, uint32_t *shift, const float *base, int64_t inner, int64_t outer, int64_t pitch, int wk)
+{
+    const bool n_inner = wk == W_N || wk == W_N_ANY;
+    const int box_inner = n_inner ? TC_BN : TC_WK, box_outer = n_inner ? TC_WK : TC_BN;
+    *shift = 0;
+    if (!w_any(wk)) {
+        int st = make_w_map(enc, &m->map[0], base, inner, outer, pitch, box_inner, box_outer, wk == W_K);
+        for (int r = 1; r < TC_CLASSES; ++r) m->map[r] = m->map[0];
+        return st;
+    }
+    for (int r = 0; r < TC_CLASSES; ++r) {
+        const uintptr_t row = reinterpret_cast<uintptr_t>(base + r * pitch);
+        const int64_t d = (int64_t)((row & 15u) / sizeof(float));
+        int st = make_w_map(enc, &m->map[r], reinterpret_cast<const float *>(row & ~(uintptr_t)15), inner + d, (outer - r + TC_CLASSES - 1) / TC_CLASSES,
+                            pitch * TC_CLASSES, box_inner + 4, box_outer / TC_CLASSES, false);
+        if (st != CN_OK) return st;
+        *shift |= (uint32_t)d << (8 * r);
+    }
     return CN_OK;
 }
 
@@ -1011,26 +1079,39 @@ static int make_a_map(EncodeTiledFn enc, CUtensorMap *map, const uint16_t *base,
 
 bool cn_gemm_tc_can_fuse_maxout(int L) { return L == 2 || L == 4 || L == 8 || L == 16 || L == 32; }
 
+// Rows that TMA can read as they are.
+static bool w_aligned(const float *B, int64_t ldb) { return (ldb & 3) == 0 && (reinterpret_cast<uintptr_t>(B) & 15u) == 0; }
+
+// short dimensions are zero-filled by TMA up to the tile; its coordinates are 32-bit
+static bool tc_dims(int64_t M, int64_t N, int64_t K)
+{
+    return M >= 1 && N >= 1 && K >= 1 && K < (1LL << 31) - 64 && N < (1LL << 31) - 256 && M < (1LL << 31) - 256;
+}
+
+bool cn_gemm_tc_any_supported(int transB, int64_t M, int64_t N, int64_t K, const float *B)
+{
+    if ((transB ? K : N) < TC_CLASSES) return false;   // every class of rows has at least one
+    return tc_dims(M, N, K) && (reinterpret_cast<uintptr_t>(B) & 3u) == 0;
+}
+
 bool cn_gemm_tc_supported(cn_context *, int transA, int transB, int64_t M, int64_t N, int64_t K, const float *,
                           int64_t, const float *B, int64_t ldb, const float *, int64_t)
 {
     (void)transA;   // a transposed activation operand only changes the pre-pass
     (void)transB;   // a transposed weight only changes the TMA box and the converter's read pattern
-    if (M < 1 || N < 1 || K < 1) return false;   // short dimensions are zero-filled by TMA up to the tile
-    if ((ldb & 3) != 0 || (reinterpret_cast<uintptr_t>(B) & 15u) != 0) return false;   // TMA: 16-byte pitch and base
-    if (K >= (1LL << 31) - 64 || N >= (1LL << 31) - 256 || M >= (1LL << 31) - 256) return false;   // TMA coordinates are 32-bit
-    return true;
+    return tc_dims(M, N, K) && w_aligned(B, ldb);
 }
 
-template <int NT, bool MODE3X, bool TRANSB>
-static int launch_cfg(const CUtensorMap &mw, const CUtensorMap &mhi, const CUtensorMap &mlo, const TcParams &prm, int64_t grid, int dev, cudaStream_t s)
+template <int NT, bool MODE3X, int WK>
+static int launch_cfg(const WMaps &mw, const CUtensorMap &mhi, const CUtensorMap &mlo, const TcParams &prm, int64_t grid, int dev, cudaStream_t s)
 {
+    using Cfg = TcCfg<NT, WK>;
     static bool attr_set[64] = {};   // per device: the attribute belongs to the device's copy of the function
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-        CN_CUDA(cudaFuncSetAttribute(cn_gemm_tc_kernel<NT, MODE3X, TRANSB>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcCfg<NT>::SMEM_BYTES));
+        CN_CUDA(cudaFuncSetAttribute(cn_gemm_tc_kernel<NT, MODE3X, WK>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
-    CN_CUDA(cn_launch_pdl(cn_gemm_tc_kernel<NT, MODE3X, TRANSB>, dim3((unsigned)grid), TcCfg<NT>::THREADS, TcCfg<NT>::SMEM_BYTES, s, mw, mhi, mlo, prm));
+    CN_CUDA(cn_launch_pdl(cn_gemm_tc_kernel<NT, MODE3X, WK>, dim3((unsigned)grid), Cfg::THREADS, Cfg::SMEM_BYTES, s, mw, mhi, mlo, prm));
     cn_count_launch();
     return CN_OK;
 }
@@ -1091,6 +1172,7 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
         if ((st = cn_status_block(ctx, &d_status)) != CN_OK) return st;
     }
     const bool mode3x = mode == CN_GEMM_3XTF32;
+    CN_REQUIRE(mode3x || w_aligned(B, ldb), CN_ERR_UNSUPPORTED, "cn_gemm_f32: weights of any alignment take the 3x mode");
 
     // 1. activations -> K-major hi / lo planes (made here, or ahead of the call by cn_gemm_prepare)
     cn_planes pl;
@@ -1181,9 +1263,11 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
     }
 
     // 3. tensor maps
-    CUtensorMap mw, mhi, mlo;
-    if (transB) st = make_w_map(enc, &mw, B, N, K, ldb, true);   // stored N x K, n contiguous
-    else        st = make_w_map(enc, &mw, B, K, N, ldb, false);
+    WMaps mw;
+    CUtensorMap mhi, mlo;
+    const int wk = w_aligned(B, ldb) ? (transB ? W_N : W_K) : (transB ? W_N_ANY : W_K_ANY);
+    st = transB ? make_w_maps(enc, &mw, &prm.w_shift, B, N, K, ldb, wk)    // stored N x K, n contiguous
+                : make_w_maps(enc, &mw, &prm.w_shift, B, K, N, ldb, wk);
     if (st != CN_OK) return st;
     if ((st = make_a_map(enc, &mhi, reinterpret_cast<const uint16_t *>(planes), pl.Kp, M)) != CN_OK) return st;
     if (mode3x) {
@@ -1204,14 +1288,12 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
         ws->prof_used += 2;
         prm.w_ready = 0;   // the event stands between the pre-pass and this launch: keep the plain order
     }
-#define CN_LAUNCH(NTV, M3, TB) launch_cfg<NTV, M3, TB>(mw, mhi, mlo, prm, grid, ctx->device, s)
-    if (nt == 1) {
-        if (transB) st = mode3x ? CN_LAUNCH(1, true, true) : CN_LAUNCH(1, false, true);
-        else        st = mode3x ? CN_LAUNCH(1, true, false) : CN_LAUNCH(1, false, false);
-    } else {
-        if (transB) st = mode3x ? CN_LAUNCH(2, true, true) : CN_LAUNCH(2, false, true);
-        else        st = mode3x ? CN_LAUNCH(2, true, false) : CN_LAUNCH(2, false, false);
-    }
+#define CN_LAUNCH(M3, WKV) \
+    (nt == 1 ? launch_cfg<1, M3, WKV>(mw, mhi, mlo, prm, grid, ctx->device, s) : launch_cfg<2, M3, WKV>(mw, mhi, mlo, prm, grid, ctx->device, s))
+    if (wk == W_K_ANY)      st = CN_LAUNCH(true, W_K_ANY);
+    else if (wk == W_N_ANY) st = CN_LAUNCH(true, W_N_ANY);
+    else if (mode3x)        st = wk == W_N ? CN_LAUNCH(true, W_N) : CN_LAUNCH(true, W_K);
+    else                    st = wk == W_N ? CN_LAUNCH(false, W_N) : CN_LAUNCH(false, W_K);
 #undef CN_LAUNCH
     if (st != CN_OK) return st;
     if (rest > 0) {

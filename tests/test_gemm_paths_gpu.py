@@ -1,0 +1,156 @@
+"""Edges of the product kernels' dispatch: the one-launch kernel for small products (any layout and alignment, K over a
+cluster), the operand scales of the streaming kernel, and its weights of any pitch, against an fp64 product.
+
+Bound of an element, with s = sum over k of |a_k b_k|.  3x mode: an operand keeps 22 of its 24 bits (2^-22 of each factor, 2^-22
+more for the product of the low parts), and a chain of 512 k accumulates 3 products per k-step of at least 8, each addition
+truncated to 2^-23 of a running sum that is at most s: 3 * 64 * 2^-23 s = 2.3e-5 s.  Single pass: both operands rounded to 11
+bits, 2^-10 s."""
+import numpy as np
+import pytest
+import torch
+
+from clusternet_b200 import _lib
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+REL_3X, REL_1X = 2.5e-5, 1.05e-3
+
+
+def place(x, off):
+    """Row-major numpy (rows x cols) -> column-major device matrix whose base lies `off` floats past a 16-byte boundary."""
+    rows, cols = x.shape
+    t = torch.zeros(rows * cols + 4, device="cuda")[off:off + rows * cols].view(cols, rows)
+    t.copy_(torch.from_numpy(np.ascontiguousarray(x.T)))
+    return t
+
+
+def check(C, A, B, transA, transB, rel):
+    a, b = (A.T if transA else A).astype(np.float64), (B.T if transB else B).astype(np.float64)
+    err = np.abs(C.T.cpu().numpy().astype(np.float64) - a @ b)
+    bound = rel * (np.abs(a) @ np.abs(b))
+    assert np.all(err <= bound), float((err / np.maximum(bound, 1e-300)).max())
+
+
+# one row, one column, one k-step; tile edges; odd pitches; one CTA per tile, clusters of 2, 4 and 8; several accumulation chains
+SMALL = [(1, 4096, 1), (17, 33, 15), (128, 31, 128), (129, 97, 127), (127, 1201, 129), (128, 785, 1201), (1201, 128, 1201), (203, 2049, 301),
+         (16, 8193, 100), (500, 130, 64)]
+
+
+@pytest.mark.parametrize("M,K,N", SMALL)
+@pytest.mark.parametrize("transA,transB", [(False, False), (True, False), (False, True), (True, True)])
+def test_small_products_in_every_layout(ctx, M, K, N, transA, transB):
+    rng = np.random.default_rng(M + 3 * K + 5 * N)
+    A = rng.standard_normal((K, M) if transA else (M, K)).astype(np.float32)
+    B = rng.standard_normal((N, K) if transB else (K, N)).astype(np.float32)
+    for off in (0, 1):
+        aligned = off == 0 and (N if transB else K) % 4 == 0
+        for mode, rel in ((_lib.GEMM_3XTF32, REL_3X), (_lib.GEMM_TF32, REL_1X if aligned else REL_3X)):
+            if not aligned and M * N * K < 4096:
+                continue
+            C = torch.full((N, M), float("nan"), device="cuda")
+            ctx.gemm(place(A, off), place(B, off), out=C, transA=transA, transB=transB, mode=mode)
+            ctx.gemm_check()
+            assert ctx.gemm_last_path().startswith("tcgen05")
+            check(C, A, B, transA, transB, rel)
+
+
+@pytest.mark.parametrize("transB", [False, True])
+@pytest.mark.parametrize("M,K,N", [(128, 8192, 512), (300, 5000, 2052)])
+def test_streaming_product_of_rows_whose_magnitudes_change(ctx, M, K, N, transB):
+    """Weights that grow along k past fp16's range (the scale is taken anew), start with zeros, or fall; activation rows of very
+    different size.  Every element lies within 2^15 of the largest of its 512-k segment, so no bit may be lost."""
+    rng = np.random.default_rng(N)
+    A = rng.uniform(0.25, 1.0, (M, K)) * rng.choice([-1.0, 1.0], (M, K)) * np.exp2(rng.integers(-30, 30, (M, 1)))
+    W = rng.uniform(0.5, 1.0, (K, N)) * rng.choice([-1.0, 1.0], (K, N))
+    seg = np.arange(K) // 512
+    W[:, 1::4] *= np.exp2((np.arange(K) % 512) // 40)[:, None]                   # grows 2^12-fold within every segment
+    W[:, 2::4] *= np.exp2(-3.0 * seg)[:, None]                                   # falls from segment to segment
+    W[:, 3::4] *= ((np.arange(K) % 512 > 100) & (seg % 2 == 0))[:, None]         # zeros first, then whole segments of zeros
+    A, W = A.astype(np.float32), W.astype(np.float32)
+    B = np.ascontiguousarray(W.T) if transB else W
+    C = ctx.gemm(place(A, 0), place(B, 0), transB=transB)
+    ctx.gemm_check()
+    check(C, A, B, False, transB, REL_3X)
+
+
+def test_streaming_product_keeps_non_finite_values_to_their_row_and_column(ctx):
+    rng = np.random.default_rng(5)
+    M, K, N = 128, 6000, 1028
+    A, W = rng.standard_normal((M, K)).astype(np.float32), rng.standard_normal((K, N)).astype(np.float32)
+    clean = ctx.gemm(place(A, 0), place(W, 0)).clone()
+    A2, W2 = A.copy(), W.copy()
+    A2[7, 900], A2[9, 5000] = np.nan, np.inf
+    W2[31, 3], W2[5999, 600] = np.inf, np.nan
+    C = ctx.gemm(place(A2, 0), place(W2, 0))
+    ctx.gemm_check()
+    hit = torch.zeros(N, M, dtype=torch.bool, device="cuda")
+    hit[:, [7, 9]] = True
+    hit[[3, 600], :] = True
+    assert not torch.isfinite(C[hit]).any()
+    assert torch.equal(C[~hit], clean[~hit])
+
+
+@pytest.mark.parametrize("M,K,N", [(203, 4001, 3001), (5, 2049, 1031), (128, 20003, 131), (300, 130, 20005), (128, 4002, 1026), (64, 5, 500001)])
+@pytest.mark.parametrize("transB", [False, True])
+@pytest.mark.parametrize("off", [0, 1, 2, 3])
+def test_streaming_weights_of_any_pitch_and_alignment(ctx, M, K, N, transB, off):
+    """The four classes of rows of a matrix whose rows TMA cannot read one by one; what lies in front of and behind it is NaN."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M + K + N)
+    A = torch.randn((K, M), device="cuda", generator=g)
+    inner, outer = (N, K) if transB else (K, N)
+    buf = torch.full((inner * outer + 64,), float("nan"), device="cuda")
+    W = buf[32 + off:32 + off + inner * outer].view(outer, inner)
+    W.copy_(torch.randn((outer, inner), device="cuda", generator=g))
+    bias = torch.randn(N, device="cuda", generator=g)
+    C = torch.full((N, M), float("nan"), device="cuda")
+    ctx.gemm(A, W, out=C, transB=transB, bias=bias, activation=_lib.ACT_RELU)
+    ctx.gemm_check()
+    assert ctx.gemm_last_path() == "tcgen05_3xtf32"
+    Wd, Ad = (W.T if transB else W).double(), A.double()
+    ref = torch.relu(Wd @ Ad + bias.double()[:, None])
+    bound = REL_3X * (Wd.abs() @ Ad.abs() + bias.double().abs()[:, None])
+    assert bool(((C.double() - ref).abs() <= bound).all())
+    # the single-pass mode does not make such weights less exact than they were on the fp32 kernel
+    C1 = ctx.gemm(A, W, transB=transB, bias=bias, activation=_lib.ACT_RELU, mode=_lib.GEMM_TF32)
+    if off or inner % 4:
+        assert torch.equal(C1, C)
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 1023, 262147])
+@pytest.mark.parametrize("off", [0, 1])
+def test_elementwise_tails_and_alignment(ctx, n, off):
+    """16-byte accesses on aligned buffers, single elements on the others and for the remainder."""
+    rng = np.random.default_rng(n)
+    host = [rng.standard_normal(n).astype(np.float32) for _ in range(3)]
+    dev = [torch.zeros(n + 4, device="cuda") for _ in range(4)]
+    g, w, r, out = (t[off:off + n] for t in dev)
+    sp = ctx.stream_ptr()
+    for t, h in zip((g, w), host):
+        t.copy_(torch.from_numpy(h))
+    rms = np.abs(host[2]) + np.float32(0.1)
+    r.copy_(torch.from_numpy(rms))
+    assert ctx.lib.cn_mul_activation_gradient(ctx.h, g.data_ptr(), w.data_ptr(), _lib.ACT_RELU, None, out.data_ptr(), n, sp) == 0
+    assert np.array_equal(out.cpu().numpy(), host[0] * (host[1] > 0).astype(np.float32))
+    assert ctx.lib.cn_dropout(ctx.h, w.data_ptr(), out.data_ptr(), n, 0.5, 3, 0, sp) == 0
+    kept = out.cpu().numpy()
+    assert np.all((kept == host[1]) | (kept == 0))
+    w2, aligned = torch.empty(n, device="cuda"), torch.empty(n, device="cuda")
+    w2.copy_(w)
+    assert ctx.lib.cn_dropout(ctx.h, w2.data_ptr(), aligned.data_ptr(), n, 0.5, 3, 0, sp) == 0
+    assert torch.equal(aligned, out)                                             # the mask does not depend on the alignment
+    assert ctx.lib.cn_rmsprop_update(ctx.h, r.data_ptr(), g.data_ptr(), w.data_ptr(), 0.9, 0.01, n, sp) == 0
+    want_r, want_w = oracle.rmsprop_update(rms, host[0], host[1], 0.9, 0.01)
+    assert np.abs(r.cpu().numpy() - want_r).max() <= 1e-6 * np.abs(want_r).max()
+    assert np.abs(w.cpu().numpy() - want_w).max() <= 2e-6
+    for t in dev:                                                                # nothing outside the buffers
+        assert float(t[:off].abs().sum()) == 0 and float(t[off + n:].abs().sum()) == 0
+
+
+@pytest.mark.parametrize("cols", [1, 31, 32, 33])
+def test_softmax_at_the_edge_of_the_register_rows(ctx, cols):
+    A = (np.random.default_rng(cols).standard_normal((65, cols)) * 3).astype(np.float32)
+    out = ctx.empty(65, cols)
+    assert ctx.lib.cn_softmax(ctx.h, place(A, 0).data_ptr(), out.data_ptr(), 65, cols, ctx.stream_ptr()) == 0
+    assert np.abs(ctx.to_numpy(out) - oracle.softmax_rows(A)).max() < 2e-6       # __expf against libm's exp
