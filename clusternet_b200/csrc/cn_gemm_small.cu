@@ -12,8 +12,8 @@
 //   * the CTAs of a cluster share a tile: each multiplies its part of K, sends every other CTA its slice of the partial tile
 //     through distributed shared memory, adds the slices it received in K order (reproducible), and finishes its slice: bias,
 //     activation, 512-byte runs of stores to C and, for the fused all-gather, to the peers.
-// The tensor core's accumulator truncates; chains of at most SM_CHAIN_KB blocks (512 k) get an accumulator each (four at most)
-// and are added in round-to-nearest fp32.
+// The tensor core's accumulator truncates, so a share of K is cut into as many chains as tensor memory holds accumulators for (four,
+// of at most SM_CHAIN_KB blocks) and the chains are added in round-to-nearest fp32.
 //
 // Bound by latency.  128 x 784 . 784 x 1024 + bias + ReLU: see cn_gemm_small_shape for what it measured.
 #include "cn_epilogue.cuh"
@@ -193,7 +193,7 @@ cn_gemm_small_kernel(const __grid_constant__ SmallParams p)
     const int m_rows = (int)(p.M - m0 < SM_BM ? p.M - m0 : SM_BM), n_rows = (int)(p.N - n0 < SM_BN ? p.N - n0 : SM_BN);
     const int m_need = (m_rows + 15) & ~15;   // UMMA N
     const int kb0 = (int)((int64_t)p.kb_total * rank / p.cluster), kb1 = (int)((int64_t)p.kb_total * (rank + 1) / p.cluster);
-    const int chains = (kb1 - kb0 + SM_CHAIN_KB - 1) / SM_CHAIN_KB;
+    const int chain_kb = (kb1 - kb0 + SM_MAX_CHAINS - 1) / SM_MAX_CHAINS, chains = (kb1 - kb0 + chain_kb - 1) / chain_kb;
     cn_pdl_launch_dependents();
     if (p.cluster > 1) cluster_arrive();   // every CTA of the cluster has started: waited for before the first remote store
     if (threadIdx.x == 0) {
@@ -230,18 +230,19 @@ cn_gemm_small_kernel(const __grid_constant__ SmallParams p)
         // kind::tf32 instruction descriptor: D fp32, A and B TF32 (format 2), K-major, N >> 3 at bits 17-22, M >> 4 at bits 24-28
         const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(m_need >> 3) << 17) | ((uint32_t)(SM_BN >> 4) << 24);
         const int n = kb1 - kb0;
-        for (int i = 0; i < n; ++i) {
+        uint32_t acc = tmem;
+        for (int i = 0, in_chain = 0; i < n; ++i, ++in_chain) {
             const int s = i & 1;
+            if (in_chain == chain_kb) { in_chain = 0; acc += SM_BM; }
             ok = mbar_wait(full0 + 8 * s, (uint32_t)(i >> 1) & 1u, abort_flag, p.status, 15u);
             if (!ok) break;
             tc_fence_after();
             const uint64_t d = make_kmajor_sw128_desc(ring + s * SM_STAGE_BYTES);
             const uint32_t hi = (uint32_t)(d >> 32), whi = (uint32_t)d, wlo = whi + (SM_TILE_BYTES >> 4), ahi = wlo + (SM_TILE_BYTES >> 4),
                            alo = ahi + (SM_TILE_BYTES >> 4);
-            const uint32_t acc = tmem + (uint32_t)(i / SM_CHAIN_KB) * SM_BM;
 #pragma unroll
             for (int j = 0; j < SM_BK / 8; ++j) {   // 8 TF32 per k-step: 32 bytes (descriptor units of 16 B)
-                sm_mma_ss(acc, whi + 2 * j, ahi + 2 * j, hi, idesc, (i % SM_CHAIN_KB != 0 || j > 0) ? 1u : 0u);
+                sm_mma_ss(acc, whi + 2 * j, ahi + 2 * j, hi, idesc, (in_chain != 0 || j > 0) ? 1u : 0u);
                 if (MODE3X) {
                     sm_mma_ss(acc, wlo + 2 * j, ahi + 2 * j, hi, idesc, 1u);
                     sm_mma_ss(acc, whi + 2 * j, alo + 2 * j, hi, idesc, 1u);
@@ -357,7 +358,7 @@ bool cn_gemm_small_shape(const cn_context *ctx, int64_t M, int64_t N, int64_t K)
     const int kb = (int)((K + SM_BK - 1) / SM_BK);
     const int c = small_cluster(tiles, kb, ctx->sm_count);
     const int64_t per_cta = (kb + c - 1) / c, rounds = (tiles * c + ctx->sm_count - 1) / ctx->sm_count;
-    return per_cta <= SM_CHAIN_KB * SM_MAX_CHAINS && rounds * per_cta <= 64;
+    return per_cta <= SM_CHAIN_KB * SM_MAX_CHAINS && rounds <= 2;
 }
 
 template <int WKIND, int AKIND, bool MODE3X>

@@ -845,8 +845,32 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
             const int L = p.maxout_level;
             const float bias = (p.bias && n < p.N) ? p.bias[n] : 0.0f;
             float *dst = p.C + n * p.ldc + m0;
-            const bool vec = m0 + TC_BM <= p.M && ((reinterpret_cast<uintptr_t>(dst) & 15u) == 0);
-            if (L <= 1 && n >= p.N) continue;
+            if (L <= 1) {
+                // every lane writes a column of its own: 32 bytes at a time fill whole sectors of L2
+                const uintptr_t at = reinterpret_cast<uintptr_t>(dst);
+                const bool whole = m0 + TC_BM <= p.M, vec8 = whole && (at & 31u) == 0, vec4 = whole && (at & 15u) == 0;
+#pragma unroll
+                for (int i = 0; i < TC_BM; i += 8) {
+                    float v[8];
+#pragma unroll
+                    for (int e = 0; e < 8; e += 2) tc_unpack2(sum[(i + e) / 2], v[e], v[e + 1]);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) v[e] = cn_apply_activation(p.bias ? v[e] + bias : v[e], p.act);
+                    if (n >= p.N) continue;
+                    if (vec8) {
+                        stg8(dst + i, v);
+                    } else if (vec4) {
+                        *reinterpret_cast<float4 *>(dst + i) = make_float4(v[0], v[1], v[2], v[3]);
+                        *reinterpret_cast<float4 *>(dst + i + 4) = make_float4(v[4], v[5], v[6], v[7]);
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            if (m0 + i + e < p.M) dst[i + e] = v[e];
+                    }
+                }
+                __syncwarp();   // the next tile's tensor-memory loads need the whole warp
+                continue;
+            }
 #pragma unroll
             for (int i = 0; i < TC_BM; i += 4) {
                 float v[4];
@@ -854,32 +878,22 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
                 tc_unpack2(sum[i / 2 + 1], v[2], v[3]);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) v[e] = cn_apply_activation(p.bias ? v[e] + bias : v[e], p.act);
-                if (L <= 1) {
-                    if (vec) {
-                        *reinterpret_cast<float4 *>(dst + i) = make_float4(v[0], v[1], v[2], v[3]);
-                    } else {
+                // maxout over L consecutive columns = L adjacent lanes (L is a power of two <= 32).
+                // Same comparison tree as the reference's 32-slot reduction: at offsets L/2 .. 1 slot t
+                // takes slot t+offset when strictly smaller; larger offsets only meet -FLT_MAX padding.
+                const int tl = lane & (L - 1);
 #pragma unroll
-                        for (int e = 0; e < 4; ++e)
-                            if (m0 + i + e < p.M) dst[i + e] = v[e];
+                for (int e = 0; e < 4; ++e) {
+                    float val = v[e], idx = (float)n;
+                    for (int off = L >> 1; off > 0; off >>= 1) {
+                        const float ov = __shfl_down_sync(0xffffffffu, val, off, L);
+                        const float oi = __shfl_down_sync(0xffffffffu, idx, off, L);
+                        if (tl < off && val < ov) { val = ov; idx = oi; }
                     }
-                } else {
-                    // maxout over L consecutive columns = L adjacent lanes (L is a power of two <= 32).
-                    // Same comparison tree as the reference's 32-slot reduction: at offsets L/2 .. 1 slot t
-                    // takes slot t+offset when strictly smaller; larger offsets only meet -FLT_MAX padding.
-                    const int tl = lane & (L - 1);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        float val = v[e], idx = (float)n;
-                        for (int off = L >> 1; off > 0; off >>= 1) {
-                            const float ov = __shfl_down_sync(0xffffffffu, val, off, L);
-                            const float oi = __shfl_down_sync(0xffffffffu, idx, off, L);
-                            if (tl < off && val < ov) { val = ov; idx = oi; }
-                        }
-                        if (tl == 0 && n < p.N && m0 + i + e < p.M) {
-                            const int64_t g = n / L;
-                            p.C[g * p.ldc + m0 + i + e] = val;
-                            if (p.argmax) p.argmax[g * p.ldc + m0 + i + e] = idx;
-                        }
+                    if (tl == 0 && n < p.N && m0 + i + e < p.M) {
+                        const int64_t g = n / L;
+                        p.C[g * p.ldc + m0 + i + e] = val;
+                        if (p.argmax) p.argmax[g * p.ldc + m0 + i + e] = idx;
                     }
                 }
             }
@@ -1102,6 +1116,12 @@ bool cn_gemm_tc_supported(cn_context *, int transA, int transB, int64_t M, int64
     return tc_dims(M, N, K) && w_aligned(B, ldb);
 }
 
+// K blocks per accumulation chain for weights of any pitch.  They were multiplied on the fp32 kernel before, whose error grows with
+// the square root of K: relative to an fp64 product (uniform operands) 2.1e-7 at K = 130, 5.0e-7 at 785, 1.13e-6 at 4001, 3.6e-6 at
+// 39999.  Here it grows with the chain: 2.1e-7 with one block, 3.2e-7 with 2, 5.2e-7 with 4, 9.0e-7 with 8, 1.8e-6 with 16.  The
+// longest chain that is no less exact than the fp32 kernel was:
+static int any_chain(int64_t K) { return K < 384 ? 1 : K < 1024 ? 2 : K < 3072 ? 4 : K < 12288 ? 8 : TC_GROUP_KB; }
+
 template <int NT, bool MODE3X, int WK>
 static int launch_cfg(const WMaps &mw, const CUtensorMap &mhi, const CUtensorMap &mlo, const TcParams &prm, int64_t grid, int dev, cudaStream_t s)
 {
@@ -1237,7 +1257,7 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
     prm.argmax = epi ? epi->argmax_out : nullptr;
     prm.tiles_n = (int)tiles_n; prm.tiles_m = (int)tiles_m;
     prm.full_tiles = (int)full; prm.tail_ctas = (int)tail_ctas; prm.kb_total = kb_total;
-    int chain = TC_GROUP_KB;
+    int chain = w_aligned(B, ldb) ? TC_GROUP_KB : any_chain(K);
     if (ws->force_chain >= 1)
         while (chain > 1 && chain > ws->force_chain) chain >>= 1;
     prm.chain_mask = chain - 1;

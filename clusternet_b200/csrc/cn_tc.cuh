@@ -52,6 +52,13 @@ __device__ __forceinline__ void sts1(uint32_t a, float v) { asm volatile("st.sha
 __device__ __forceinline__ void sts1u(uint32_t a, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
 __device__ __forceinline__ void sts1b(uint32_t a, uint32_t v) { asm volatile("st.shared.u8 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
 
+// 32-byte aligned global store: a whole sector.
+__device__ __forceinline__ void stg8(float *q, const float (&v)[8])
+{
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"l"(q), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
+}
+
 // Bounded wait.  Returns false when the limit ran out or another role already gave up.
 // SLEEP_NS > 0 parks the warp between polls: used by roles that wait for a long time (the drain warps sit out a
 // whole accumulation chain) so that their polling does not take issue slots from the converter and MMA warps.
