@@ -677,7 +677,7 @@ def main():
         oacc = accuracy(TOL[oname], oname)
         if rank == 0:
             w_bytes_rank = 4.0 * K1 * (N1 / world)
-            tensor_peak = peaks["bf16_tflops"] / 2.0 / (3.0 if oname == "3xtf32" else 1.0)
+            tensor_peak = peaks["bf16_tflops"] / (3.0 if oname == "3xtf32" else 1.0)   # the split products are fp16
             hbm_bound = 2.0 * M / 4.0 * peaks["hbm_gbs"] / 1e3          # 64 flop per W byte x HBM GB/s -> TFLOP/s
             l1_tf = 2.0 * M * K1 * (N1 / world) / (ol1 * 1e-3) / 1e12 if ol1 else None
             other = {"mode": oname, "value": FLOPS_STEP / (oms * 1e-3) / 1e12, "unit": "TFLOP/s", "ms_per_step": oms, "steps": osteps,
@@ -861,8 +861,7 @@ def main():
 
     value = FLOPS_STEP * args.steps / (ms_total * 1e-3) / 1e12
     e2e_value = FLOPS_STEP * args.steps / (ms_e2e * 1e-3) / 1e12
-    tf32_peak = peaks["bf16_tflops"] / 2.0
-    peak = tf32_peak / 3.0 if args.mode == "3xtf32" else tf32_peak
+    peak = peaks["bf16_tflops"] / (3.0 if args.mode == "3xtf32" else 1.0)   # the split products are fp16
     l1_flops_rank = 2.0 * M * K1 * (N1 // world if world > 1 else N1)
     achieved = l1_flops_rank / (l1_ms * 1e-3) / 1e12 if l1_ms else None
     e2e_ok = bool(e2e_match and acc_e2e["ok"])
@@ -873,7 +872,7 @@ def main():
         "config": {"workload": ("README dotMPI two-layer skinny GEMM: " if headline else "REDUCED (profiling) two-layer skinny GEMM: ") +
                                f"128x{K1} . {K1}x{N1} . {N1}x{N2}, W column-sharded",
                    "gemm_mode": args.mode, "exchange": args.exchange, "gather": ("fused peer stores" if fused else ("nccl" if world > 1 else "none")), "parallelism": f"tp{world} (columns of W)",
-                   "activation_planes": ("layer 1's TF32 hi/lo planes are made one step ahead on a second stream (cn_gemm_prepare): every step makes "
+                   "activation_planes": ("layer 1's hi/lo planes are made one step ahead on a second stream (cn_gemm_prepare): every step makes "
                                          "the planes of its successor beside its own products" if use_prep else "made inside each product call"),
                    "timed_regions": "each starts after 1.5 s of idle GPUs and its own warm-up steps (the products are power-limited)",
                    "l2": f"inputs larger than L2 ({4e-9 * (K1 * N1 + N1 * N2):.1f} GB of weights stream once per step)", "flops_per_step": FLOPS_STEP},
@@ -894,7 +893,7 @@ def main():
                      "ms_per_launch": l1_ms, "layer2_ms_per_launch": l2_ms,
                      "peak_source": f"{peaks['source']} burst: bf16_tflops {peaks['bf16_tflops']} / 2 (TF32 rate)" + (" / 3 (three TF32 products per tile)" if args.mode == "3xtf32" else ""),
                      # side note: the same against the power-capped (seconds-long) cuBLAS figure
-                     "frac_sustained": (achieved / (peaks["bf16_tflops_sustained"] / 2.0 / (3.0 if args.mode == "3xtf32" else 1.0))) if achieved else None,
+                     "frac_sustained": (achieved / (peaks["bf16_tflops_sustained"] / (3.0 if args.mode == "3xtf32" else 1.0))) if achieved else None,
                      "hbm_frac_layer1": (4.0 * K1 * (N1 / world) / (l1_ms * 1e-3) / 1e9 / peaks["hbm_gbs"]) if l1_ms else None},
     }
     if other:

@@ -159,7 +159,7 @@ int cn_arange_f32(cn_context *ctx, float *d_A, int64_t start, int64_t rows, int6
  * (lda = A->rows, ldb = B->rows, ldc = out->rows).
  * ------------------------------------------------------------------------------------------- */
 typedef enum cn_gemm_mode {
-    CN_GEMM_3XTF32 = 0,  /* fp32-accurate: hi/lo TF32 split, three tensor-core products per tile */
+    CN_GEMM_3XTF32 = 0,  /* fp32-accurate: hi/lo split of 11 bits each (TF32's), three tensor-core products per tile */
     CN_GEMM_TF32 = 1,    /* single TF32 product (10-bit mantissa operands), reported separately */
     CN_GEMM_FP32_SIMT = 2 /* plain fp32 FMA kernel; also chosen automatically for shapes the tensor path cannot take */
 } cn_gemm_mode;
