@@ -57,8 +57,14 @@ struct SmallParams {
     unsigned int epoch;
 };
 
-// fp32 -> TF32, round to nearest with ties away from zero: add half a TF32 ulp to the magnitude bits and truncate.
-__device__ __forceinline__ uint32_t sm_tf32(float x) { return (__float_as_uint(x) + 0x1000u) & 0xffffe000u; }
+// fp32 -> TF32, round to nearest with ties away from zero: add half a TF32 ulp to the magnitude bits and truncate.  That carry would
+// take the finite values from 0x7f7ff000 up to infinity and a NaN with a full mantissa (0x7fffffff, the one GPU arithmetic makes)
+// over into the sign bit, to -0: those are truncated instead, NaNs after an addition that makes them the canonical one.
+__device__ __forceinline__ uint32_t sm_tf32(float x)
+{
+    const float top = __uint_as_float(0x7f7ff000u);
+    return (fabsf(x) < top ? __float_as_uint(x) + 0x1000u : __float_as_uint(__fadd_rn(x, 0.0f))) & 0xffffe000u;
+}
 
 __device__ __forceinline__ void sts4u(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w)
 {

@@ -91,6 +91,35 @@ def test_streaming_product_keeps_non_finite_values_to_their_row_and_column(ctx):
     assert torch.equal(C[~hit], clean[~hit])
 
 
+@pytest.mark.parametrize("transA,transB", [(False, False), (True, False), (False, True), (True, True)])
+@pytest.mark.parametrize("off", [0, 1])
+def test_small_products_keep_non_finite_and_the_largest_finite_values(ctx, transA, transB, off):
+    """NaNs of any bit pattern (0x7fffffff is the one that GPU arithmetic makes) and infinities in either operand stay in their row
+    or column and make it non-finite; a value that rounds past the largest TF32 number stays finite in the 3x mode."""
+    rng = np.random.default_rng(11)
+    M, K, N = 128, 785, 300
+    A = rng.standard_normal((K, M) if transA else (M, K)).astype(np.float32)
+    B = rng.standard_normal((N, K) if transB else (K, N)).astype(np.float32)
+    a, b = (A.T if transA else A), (B.T if transB else B)          # views: op(A)(m, k), op(B)(k, n)
+    a[100] = 0.0
+    a[100, 3], b[3, :] = np.frombuffer(np.uint32(0x7f7fffff).tobytes(), np.float32)[0], 0.25
+    bad = np.frombuffer(np.array([0x7fffffff, 0xffffffff, 0x7fc00000, 0x7f800000], np.uint32).tobytes(), np.float32)
+    for i, v in enumerate(bad):
+        a.view(np.uint32)[7 + i, 50 * i] = v.view(np.uint32)
+        b.view(np.uint32)[60 * i + 1, 11 + i] = v.view(np.uint32)
+    for mode in (_lib.GEMM_3XTF32, _lib.GEMM_TF32):
+        n0 = ctx.lib.cn_kernel_launches()
+        C = ctx.gemm(place(A, off), place(B, off), transA=transA, transB=transB, mode=mode).T.cpu().numpy()
+        assert ctx.lib.cn_kernel_launches() - n0 == 1              # the one-launch kernel
+        ctx.gemm_check()
+        finite = np.isfinite(C)
+        assert not finite[7:11].any() and not finite[:, 11:15].any()
+        rest = np.ones((M, N), bool)
+        rest[7:11], rest[:, 11:15] = False, False
+        assert finite[rest].all()
+        assert np.allclose(C[100][rest[100]], a[100, 3].astype(np.float64) * 0.25, rtol=REL_1X)
+
+
 @pytest.mark.parametrize("M,K,N", [(203, 4001, 3001), (5, 2049, 1031), (128, 20003, 131), (300, 130, 20005), (128, 4002, 1026), (64, 5, 500001)])
 @pytest.mark.parametrize("transB", [False, True])
 @pytest.mark.parametrize("off", [0, 1, 2, 3])
