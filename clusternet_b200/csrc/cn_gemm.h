@@ -22,12 +22,15 @@ struct cn_coded_src {
     int nranks = 1, own_rank = 0;
 };
 
-// Planes of an M x K activation operand, in one allocation: fp16 hi [M][Kp], fp16 lo [M][Kp] (only in the 3x mode), inverse
-// scales [groups of CN_PLANE_GROUP_K k][m_pad] (see cn_gemm_tc.cu).
+// Planes of an M x K activation operand, in one allocation: per band fp16 hi [M][Kp] and, in the 3x mode, lo, `plane` elements apart;
+// inverse scales [band][group of CN_PLANE_GROUP_K k][m_pad]; bands behind the first that a block of 16 rows x 64 k has, a byte each
+// [tile of 128 rows][64 k][8] (see cn_gemm_tc.cu).
 #define CN_PLANE_GROUP_K 512
+#define CN_PLANE_BANDS 3
 struct cn_planes {
-    int64_t Kp, m_pad, groups;
-    size_t lo_off, inv_off, bytes;   // lo_off = 0: no low plane
+    int64_t Kp, plane, m_pad, groups;
+    int parts;
+    size_t inv_off, bands_off, bytes;
 };
 void cn_plane_layout(int64_t M, int64_t K, int mode, cn_planes *pl);
 

@@ -12,9 +12,20 @@
 //   * activations: row m, segment of 512 k: the largest magnitude is brought into [2^14, 2^15);
 //   * weights: column n, accumulation chain (below): the first K block that is not all zero brings its largest magnitude
 //     into [2^13, 2^14); a later block that would leave fp16's range ends the chain early and starts a new one with a new scale.
-// hi = fp16(s x) is exact to 2^-12 |s x|, lo = fp16(s x - hi) to 2^-24 |s x| or 2^-25, whichever is larger.  So every
-// element within a factor 2^-15 of the largest of its segment keeps all 22 bits of the split, and a smaller one has an absolute
-// error below 2^-38 of that largest element: 2^-14 of the last bit the largest element itself has in fp32.
+// hi = fp16(s x) is exact to 2^-12 |s x|, lo = fp16(s x - hi) to 2^-24 |s x| or 2^-25, whichever is larger.  So an element within
+// a factor 2^-15 of the largest of its segment keeps all 22 bits of the split, one 2^-19 below it 20.
+//
+// What fp16 cannot hold.  Of a smaller element more is lost, all of it from 2^-39 down; that counts where the large one meets a
+// zero.  What hi + lo leave of an element, if it is more than 2^-20 of it (2^-10 in the single pass), is multiplied as well, in
+// accumulation chains of its own with scales of their own:
+//   * activations: what is left goes to a second pair of planes, scaled anew, and what that leaves to a third: 58 more binades.  They
+//     are written, loaded and multiplied only for the blocks of 16 rows x 32 k that have something in them;
+//   * weights: a converter warp that finds such elements in its 32 rows of a block writes what is left of them, 2^38 times the scale,
+//     to an operand stage of its own, and again until nothing is left (elements 2^115 below the largest lose bits after all).
+// Random operands have a few such elements by chance (uniform ones about 1 in 2^20); their chains cost less than the runs of a
+// measurement differ, looking for them 5 to 10 %: 4096^3 432 -> 476 us, 128 x 100000 . 100000 x 40000 3450 -> 3700 us, single pass 128 x
+// 40000 . 40000 x 40000 1030 -> 1078 us.  Measured on the same boxes: three bf16 parts of 8 bits and six products, which need no scales,
+// 647, 5290 and (as TF32) 1310 us.
 //
 // Mapping.  A column-major W has its K index contiguous for a fixed column n, i.e. it is a K-major operand with
 // N "rows".  The kernel therefore computes the transposed tile D[n, m] = sum_k W[k, n] * A[m, k]:
@@ -72,9 +83,11 @@ __host__ __device__ constexpr int w_box_bytes(int wk)
 #define TC_A_TILE_BYTES (TC_BM * TC_AK * 2)
 #define TC_GROUP_K CN_PLANE_GROUP_K
 #define TC_GROUP_KB (TC_GROUP_K / TC_WK)
+#define TC_BANDS CN_PLANE_BANDS   // the planes of the activations and of what they leave, twice
+#define TC_SUB 16                 // rows m of a block of left-overs
 #define TC_DRAIN_SLEEP_NS 100   // poll interval of the drain warps while a chain accumulates
 
-template <int NT, int WK>
+template <int NT, bool MODE3X, int WK>
 struct TcCfg {
     static constexpr int THREADS = 128 + 256 * NT;    // WG0 (producers, MMA), per W tile one converter and one drain warpgroup
     // Two shared-memory rings with their own depth: raw W blocks (released by the converters as soon as they have
@@ -88,12 +101,15 @@ struct TcCfg {
     static constexpr int A_RING = W_STAGES * W_STAGE_BYTES;
     static constexpr int RING_BYTES = A_RING + A_STAGES * A_STAGE_BYTES;
     static_assert(A_RING % 1024 == 0, "swizzled tiles");
-    static constexpr int TMEM_STAGES = 4;
+    static_assert(A_STAGES >= TC_BANDS, "the bands of a stage are held together");
+    static constexpr int TMEM_STAGES = NT == 2 && MODE3X ? 3 : 4;
     static constexpr int ACC_BUFS = NT == 1 ? 2 : 1;  // accumulators per W tile
     static constexpr int ACC_COL = 0;                 // NT * ACC_BUFS accumulators of 128 columns
-    static constexpr int OP_COL = NT * ACC_BUFS * TC_BM;   // then TMEM_STAGES x NT x 2 k-steps x (8 hi + 8 lo) columns
-    static constexpr int OP_STAGE_COLS = NT * 32;
-    static_assert(OP_COL + TMEM_STAGES * OP_STAGE_COLS <= 512, "tensor memory");
+    static constexpr int OP_COL = NT * ACC_BUFS * TC_BM;   // then TMEM_STAGES x NT x 2 k-steps x (8 hi + 8 lo) columns (no lo in the single pass)
+    static constexpr int STEP_COLS = MODE3X ? 16 : 8, OP_COLS = 2 * STEP_COLS;
+    static constexpr int OP_STAGE_COLS = NT * OP_COLS;
+    static constexpr int LEFT_COL = OP_COL + TMEM_STAGES * OP_STAGE_COLS;   // what is left of a block of weights, per W tile
+    static_assert(LEFT_COL + OP_STAGE_COLS <= 512, "tensor memory");
     // Scales of the W rows, one slot per W block: the drain warps read the slot of a chain's last block.  The converters
     // run at most TMEM_STAGES blocks ahead of the MMAs, and the MMAs at most ACC_BUFS - 1 chains ahead of the drain.
     static constexpr int WS_SLOTS = NT == 1 ? 32 : 8;
@@ -101,17 +117,20 @@ struct TcCfg {
     static constexpr int WS_OFF = RING_BYTES;                              // [WS_SLOTS][NT][128] floats
     static constexpr int AS_OFF = WS_OFF + WS_SLOTS * NT * TC_BN * 4;      // [2][NT][128] floats
     static constexpr int BRK_OFF = AS_OFF + 2 * NT * TC_BM * 4;            // [TMEM_STAGES][NT] words of four bytes, one per converter warp
-    static constexpr int INFO_OFF = BRK_OFF + TMEM_STAGES * NT * 4;        // [NT][ACC_BUFS] pairs of words
+    static constexpr int LEFT_OFF = BRK_OFF + TMEM_STAGES * NT * 4;        // [NT] words: whether more is left, a byte per converter warp
+    static constexpr int BAND_OFF = LEFT_OFF + NT * 4;        // [A_STAGES] words: blocks of 16 rows with left-overs, a byte per 32 k and band
+    static_assert(TC_BANDS == 3, "four bytes");
+    static constexpr int INFO_OFF = BAND_OFF + A_STAGES * 4;               // [NT][ACC_BUFS] pairs of words
     static constexpr int BAR_OFF = (INFO_OFF + NT * ACC_BUFS * 8 + 7) & ~7;
-    static constexpr int BARS = 2 * (W_STAGES + A_STAGES + NT * TMEM_STAGES + NT * ACC_BUFS);
+    static constexpr int BARS = 2 * (W_STAGES + A_STAGES + NT * TMEM_STAGES + NT * ACC_BUFS + NT * 4);
     static constexpr int HOLD_OFF = BAR_OFF + BARS * 8;                    // tensor-memory base, abort flag
     static constexpr int SMEM_BYTES = HOLD_OFF + 16 + 1024 /*align*/;
     static_assert(SMEM_BYTES <= 232448, "shared memory");
     // register budgets after the warpgroups re-balance: multiples of 8, their sum over the warpgroups at most what the launch has
-    // (NT = 2: 5 x 96, NT = 1: 3 x 168)
+    // (NT = 2: 5 x 96, NT = 1: 3 x 168).  4096^3: 495 us with 48 and 168, 476 with 56 and 160; single pass 128 x 40000 x 40000: 1090 and 1101.
     static constexpr int REGS_WG0 = NT == 1 ? 88 : 48;
-    static constexpr int REGS_CONV = NT == 1 ? 104 : 48;
-    static constexpr int REGS_DRAIN = NT == 1 ? 232 : 168;
+    static constexpr int REGS_CONV = NT == 1 ? 104 : MODE3X ? 56 : 48;
+    static constexpr int REGS_DRAIN = NT == 1 ? 232 : MODE3X ? 160 : 168;
     static_assert(REGS_WG0 + NT * (REGS_CONV + REGS_DRAIN) <= (1 + 2 * NT) * (65536 / THREADS / 8 * 8), "registers");
 };
 
@@ -129,8 +148,11 @@ struct TcParams {
     int tail_ctas;
     int kb_total;           // K blocks of 32
     int chain_mask;         // K blocks per accumulation chain - 1 (a power of two, at most TC_GROUP_KB)
-    const float *a_inv;     // [group of 512 k][m_pad] inverse scales of the activation rows
+    const float *a_inv;     // [band][group of 512 k][m_pad] inverse scales of the activation rows
     int64_t m_pad;
+    int groups;
+    const uint8_t *a_bands; // [tile of 128 rows][64 k][block of 16 rows]: bands behind the first that have something in them, four bits per 32 k
+    int a_stages;           // ceil(K / 64)
     float *partials;        // [slot][w][32 quads of m][128 n] float4: slot = CTA + tile - full_tiles
     unsigned int *status;
     uint32_t w_shift;       // byte r: d_r of the weights' rows r, r + 4, ... (see W_K_ANY)
@@ -244,6 +266,24 @@ __device__ __forceinline__ uint64_t tc_fma2(uint64_t a, uint64_t b, uint64_t c)
     return r;
 }
 
+// Two packed fp16 values -> floats, negated.
+__device__ __forceinline__ uint64_t tc_minus_f16x2(uint32_t h)
+{
+    float h0, h1;
+    asm("{\n\t.reg .b16 a, b;\n\t"
+        "mov.b32 {a, b}, %2;\n\t"
+        "cvt.f32.f16 %0, a;\n\t"
+        "cvt.f32.f16 %1, b;\n\t}"
+        : "=f"(h0), "=f"(h1) : "r"(h));
+    return tc_pack2(-h0, -h1);
+}
+__device__ __forceinline__ uint64_t tc_add2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
 // Two scaled values -> packed fp16 high parts, and (LO) packed fp16 low parts: lo = fp16(y - hi), the difference being exact.
 // Measured on registers with two warps per scheduler: 10 issue cycles per pair, 12 with the mixed-precision subtraction
 // (sub.f32.f16) in place of the two conversions back and the packed one.
@@ -254,23 +294,35 @@ __device__ __forceinline__ void tc_split2(uint64_t y, uint32_t &hi, uint32_t &lo
     tc_unpack2(y, y0, y1);
     asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(y1), "f"(y0));
     if (LO) {
-        float h0, h1;
-        asm("{\n\t.reg .b16 a, b;\n\t"
-            "mov.b32 {a, b}, %2;\n\t"
-            "cvt.f32.f16 %0, a;\n\t"
-            "cvt.f32.f16 %1, b;\n\t}"
-            : "=f"(h0), "=f"(h1) : "r"(hi));
-        uint64_t d;
-        asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(y), "l"(tc_pack2(-h0, -h1)));
         float d0, d1;
-        tc_unpack2(d, d0, d1);
+        tc_unpack2(tc_add2(y, tc_minus_f16x2(hi)), d0, d1);
         asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(d1), "f"(d0));
     }
 }
 
+// ... and what the parts leave of the two values (exact), where it is more of an element than the product may lose; 0 otherwise.
+#define TC_LEFT_3X 9.5367431640625e-7f   // 2^-20
+#define TC_LEFT_1X 9.765625e-4f          // 2^-10
+#define TC_LEFT_SCALE 274877906944.0f    // 2^38: what is left of a scaled value is at most 2^-25
+template <bool LO>
+__device__ __forceinline__ void tc_split2_left(float y0, float y1, uint32_t &hi, uint32_t &lo, float &r0, float &r1)
+{
+    const uint64_t y = tc_pack2(y0, y1);
+    tc_split2<LO>(y, hi, lo);
+    uint64_t r = tc_add2(y, tc_minus_f16x2(hi));
+    if (LO) r = tc_add2(r, tc_minus_f16x2(lo));
+    tc_unpack2(r, r0, r1);
+    constexpr float LEFT = LO ? TC_LEFT_3X : TC_LEFT_1X;
+    r0 = fabsf(r0) > LEFT * fabsf(y0) ? r0 : 0.0f;   // false for a NaN, which the parts carry
+    r1 = fabsf(r1) > LEFT * fabsf(y1) ? r1 : 0.0f;
+}
+// A high part of at least this (fp16 bits) leaves less: half an fp16 denormal, 2^-25, is 2^-20 of 2^-5 and 2^-10 of 2^-15.
+template <bool LO> __host__ __device__ constexpr uint32_t tc_safe_f16() { return LO ? 0x2800u : 0x0400u; }
+
 // ------------------------------------------------------------------------------------------ activation pre-pass
 // A (M x K) -> planes hi, lo: [M][Kp] fp16 with k contiguous, k in [K, Kp) zero, and the inverse scales a_inv[group][m_pad].
-// One CTA per 16 rows and group of 512 k.  Bound by latency for a layer's activations and by memory otherwise: 4 bytes read
+// One CTA per 16 rows and group of 512 k.  What the planes leave of an element (see the top) goes to the next band's planes and
+// scales; `bands` tells which blocks of 16 rows x 32 k have any.  Bound by latency for a layer's activations and by memory otherwise: 4 bytes read
 // and 4 written per element.  CODED: the consumer-side half of the 8-bit exchange.  The activations arrive as gathered codes
 // (column-major like the fp32 matrix; column block r was coded by rank r with scale scales[r]) and are decoded here, inside
 // the pre-pass of the GEMM that consumes them, instead of being written out as fp32 first.  This rank's own block is taken
@@ -280,17 +332,51 @@ struct ActCoded {
     const float *scales, *tbl, *own_fp32;
     int own_rank, nranks;
 };
-#define ACT_ROWS 16
+#define ACT_ROWS TC_SUB
 #define ACT_PITCH (ACT_ROWS + 1)
 
-template <bool CODED>
+// Where the planes of an operand are (cn_plane_layout).
+struct ActPlanes {
+    uint16_t *p;            // band 0: hi, lo (3x mode only), band 1: ...
+    int64_t plane, Kp, m_pad, groups;
+    float *inv;
+    uint8_t *bands;
+    int stages;
+    __device__ __forceinline__ uint8_t *band_byte(int64_t m0, int64_t stage) const
+    {
+        return bands + ((m0 / TC_BM) * stages + stage) * (TC_BM / TC_SUB) + (m0 % TC_BM) / TC_SUB;
+    }
+};
+
+// Eight consecutive k of one row, scaled, into the planes of a band; x becomes what they leave, unscaled.  Returns whether anything is
+// left; a row with an element that is not finite leaves nothing, since its sums are not finite anyway.
+template <bool LO>
+__device__ __forceinline__ bool act_store8(const ActPlanes &pl, int band, int64_t at, float (&x)[8], float sc, float inv, bool finite)
+{
+    uint32_t h[4], l[4];
+    bool left = false;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        tc_split2_left<LO>(x[2 * e] * sc, x[2 * e + 1] * sc, h[e], l[e], x[2 * e], x[2 * e + 1]);
+        left |= x[2 * e] != 0.0f || x[2 * e + 1] != 0.0f;
+        x[2 * e] = finite ? x[2 * e] * inv : 0.0f;
+        x[2 * e + 1] = finite ? x[2 * e + 1] * inv : 0.0f;
+    }
+    uint16_t *q = pl.p + band * (LO ? 2 : 1) * pl.plane + at;
+    *reinterpret_cast<uint4 *>(q) = make_uint4(h[0], h[1], h[2], h[3]);
+    if (LO) *reinterpret_cast<uint4 *>(q + pl.plane) = make_uint4(l[0], l[1], l[2], l[3]);
+    return left && finite;
+}
+
+template <bool LO, bool CODED>
 __global__ void __launch_bounds__(256)
-cn_act_planes_kernel(const float *A, int64_t lda, int64_t M, int64_t K, int64_t Kp, uint16_t *hi, uint16_t *lo, float *a_inv, int64_t m_pad,
-                     const ActCoded cd)
+cn_act_planes_kernel(const float *A, int64_t lda, int64_t M, int64_t K, const ActPlanes pl, const ActCoded cd)
 {
     __shared__ float tile[TC_GROUP_K * ACT_PITCH];
     __shared__ uint32_t red[16][ACT_ROWS];
-    __shared__ float s_sc[ACT_ROWS];
+    __shared__ float s_sc[ACT_ROWS], s_inv[ACT_ROWS];
+    __shared__ bool s_finite[ACT_ROWS];
+    __shared__ uint32_t s_left[TC_BANDS][TC_GROUP_KB];   // something is left of these 32 k after the band
     extern __shared__ float lut[];   // CODED: nranks x 256
     const int tid = threadIdx.x;
     // wait first, then release the product: it may then rely on everything before this pass having finished, and start on W
@@ -312,7 +398,7 @@ cn_act_planes_kernel(const float *A, int64_t lda, int64_t M, int64_t K, int64_t 
         __syncthreads();
     }
     const int64_t split = CODED ? K / cd.nranks : 0;
-    const int64_t m_blocks = m_pad / ACT_ROWS;
+    const int64_t m_blocks = pl.m_pad / ACT_ROWS, Kp = pl.Kp;
     const int64_t g = blockIdx.x / m_blocks, m0 = (blockIdx.x - g * m_blocks) * ACT_ROWS, k0 = g * TC_GROUP_K;
     {
         const int ml = tid & 15, kl = tid >> 4;
@@ -338,85 +424,102 @@ cn_act_planes_kernel(const float *A, int64_t lda, int64_t M, int64_t K, int64_t 
         }
         red[kl][ml] = amax;
     }
-    __syncthreads();
-    if (tid < ACT_ROWS) {
-        uint32_t amax = 0u;
-#pragma unroll
-        for (int j = 0; j < 16; ++j) amax = max(amax, red[j][tid]);
-        float sc, inv;
-        tc_scale<TC_A_EXP>(amax, sc, inv);
-        s_sc[tid] = sc;
-        a_inv[g * m_pad + m0 + tid] = inv;
-    }
-    __syncthreads();
+    if (tid < TC_BANDS * TC_GROUP_KB) (&s_left[0][0])[tid] = 0u;
     // eight consecutive k per item; a warp covers 8 rows x 32 k (conflict-free reads, 64 contiguous bytes per row)
     const int lane = tid & 31, warp = tid >> 5;
+    for (int band = 0;; ++band) {
+        __syncthreads();
+        if (tid < ACT_ROWS) {
+            uint32_t amax = 0u;
 #pragma unroll
-    for (int it = 0; it < 4; ++it) {
-        const int ml = (it & 1) * 8 + (lane & 7), kk = ((warp + 8 * (it >> 1)) * 4 + (lane >> 3)) * 8;
-        const int64_t m = m0 + ml, k = k0 + kk;
-        if (m < M && k < Kp) {
-            const float sc = s_sc[ml];
-            uint32_t h[4], l[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float y0 = tile[(kk + 2 * e) * ACT_PITCH + ml] * sc, y1 = tile[(kk + 2 * e + 1) * ACT_PITCH + ml] * sc;
-                if (lo) tc_split2<true>(tc_pack2(y0, y1), h[e], l[e]);
-                else tc_split2<false>(tc_pack2(y0, y1), h[e], l[e]);
-            }
-            *reinterpret_cast<uint4 *>(hi + m * Kp + k) = make_uint4(h[0], h[1], h[2], h[3]);
-            if (lo) *reinterpret_cast<uint4 *>(lo + m * Kp + k) = make_uint4(l[0], l[1], l[2], l[3]);
+            for (int j = 0; j < 16; ++j) amax = max(amax, red[j][tid]);
+            tc_scale<TC_A_EXP>(amax, s_sc[tid], s_inv[tid]);
+            s_finite[tid] = amax < 0x7f800000u;
+            pl.inv[(band * pl.groups + g) * pl.m_pad + m0 + tid] = s_inv[tid];
         }
+        __syncthreads();
+        bool left = false;
+#pragma unroll
+        for (int it = 0; it < 4; ++it) {
+            const int ml = (it & 1) * 8 + (lane & 7), kk = ((warp + 8 * (it >> 1)) * 4 + (lane >> 3)) * 8, st = kk / TC_WK;
+            const int64_t m = m0 + ml, k = k0 + kk;
+            if (m < M && k < Kp && (band == 0 || s_left[band - 1][st] != 0u)) {
+                float x[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) x[e] = tile[(kk + e) * ACT_PITCH + ml];
+                if (act_store8<LO>(pl, band, m * Kp + k, x, s_sc[ml], s_inv[ml], s_finite[ml])) {
+                    left = true;
+                    s_left[band][st] = 1u;
+                }
+#pragma unroll
+                for (int e = 0; e < 8; ++e) tile[(kk + e) * ACT_PITCH + ml] = x[e];
+            }
+        }
+        if (!__syncthreads_or(left) || band == TC_BANDS - 1) break;
+        // the largest left of each row, as at the start (what the others leave is zero)
+        uint32_t amax = 0u;
+        for (int j = 0; j < TC_GROUP_K / 16; ++j) amax = max(amax, __float_as_uint(tile[(j * 16 + (tid >> 4)) * ACT_PITCH + (tid & 15)]) & 0x7fffffffu);
+        red[tid >> 4][tid & 15] = amax;
+    }
+    if (tid < TC_GROUP_K / TC_AK && k0 + tid * TC_AK < Kp) {
+        uint32_t n = 0u;
+        for (int band = 0; band < TC_BANDS - 1; ++band) n += s_left[band][2 * tid] + (s_left[band][2 * tid + 1] << 4);
+        *pl.band_byte(m0, k0 / TC_AK + tid) = (uint8_t)n;
     }
 }
 
 // Same planes for a transposed activation operand: op(A)(m, k) = A[k + m * lda] is already K-major (this is also what
-// a row-major M x K batch looks like): one warp per row and group, sixteen k per lane, 16-byte loads when the row pitch and
-// the base allow.
-__global__ void __launch_bounds__(256)
-cn_act_planes_t_kernel(const float *A, int64_t lda, int64_t M, int64_t K, int64_t Kp, uint16_t *hi, uint16_t *lo, float *a_inv, int64_t m_pad,
-                       int vec_ok)
+// a row-major M x K batch looks like): one warp per row and group, two times eight k per lane, 16-byte loads when the row pitch
+// and the base allow.
+template <bool LO>
+__global__ void __launch_bounds__(32 * ACT_ROWS)
+cn_act_planes_t_kernel(const float *A, int64_t lda, int64_t M, int64_t K, const ActPlanes pl, int vec_ok)
 {
-    const int lane = threadIdx.x & 31;
-    const int64_t m_blocks = m_pad / 8;
-    const int64_t g = blockIdx.x / m_blocks, m = (blockIdx.x - g * m_blocks) * 8 + (threadIdx.x >> 5);
+    __shared__ uint32_t s_left[TC_BANDS][TC_GROUP_KB];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int64_t m_blocks = pl.m_pad / ACT_ROWS;
+    const int64_t g = blockIdx.x / m_blocks, m0 = (blockIdx.x - g * m_blocks) * ACT_ROWS, m = m0 + (tid >> 5), k0 = g * TC_GROUP_K;
     cn_pdl_wait();
     cn_pdl_launch_dependents();   // after the wait: see cn_act_planes_kernel
-    if (m >= M) return;
+    if (tid < TC_BANDS * TC_GROUP_KB) (&s_left[0][0])[tid] = 0u;
+    __syncthreads();
     const float *src = A + m * lda;
-    float x[16];
-    uint32_t amax = 0u;
+    float x[2][8];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int64_t k = g * TC_GROUP_K + 128 * j + 4 * lane;
-        if (vec_ok && k + 3 < K) {
-            const float4 v = *reinterpret_cast<const float4 *>(src + k);
-            x[4 * j] = v.x; x[4 * j + 1] = v.y; x[4 * j + 2] = v.z; x[4 * j + 3] = v.w;
+    for (int j = 0; j < 2; ++j) {
+        const int64_t k = k0 + 256 * j + 8 * lane;
+        if (vec_ok && m < M && k + 7 < K) {
+            const float4 a = *reinterpret_cast<const float4 *>(src + k), b = *reinterpret_cast<const float4 *>(src + k + 4);
+            x[j][0] = a.x; x[j][1] = a.y; x[j][2] = a.z; x[j][3] = a.w;
+            x[j][4] = b.x; x[j][5] = b.y; x[j][6] = b.z; x[j][7] = b.w;
         } else {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) x[4 * j + e] = (k + e < K) ? src[k + e] : 0.0f;
+            for (int e = 0; e < 8; ++e) x[j][e] = (m < M && k + e < K) ? src[k + e] : 0.0f;
         }
     }
+    for (int band = 0;; ++band) {
+        uint32_t amax = 0u;
 #pragma unroll
-    for (int e = 0; e < 16; ++e) amax = max(amax, __float_as_uint(x[e]) & 0x7fffffffu);
-    amax = __reduce_max_sync(0xffffffffu, amax);
-    float sc, inv;
-    tc_scale<TC_A_EXP>(amax, sc, inv);
-    if (lane == 0) a_inv[g * m_pad + m] = inv;
+        for (int e = 0; e < 16; ++e) amax = max(amax, __float_as_uint(x[e >> 3][e & 7]) & 0x7fffffffu);
+        amax = __reduce_max_sync(0xffffffffu, amax);
+        float sc, inv;
+        tc_scale<TC_A_EXP>(amax, sc, inv);
+        if (lane == 0) pl.inv[(band * pl.groups + g) * pl.m_pad + m] = inv;
+        bool left = false;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int64_t k = g * TC_GROUP_K + 128 * j + 4 * lane;
-        if (k >= Kp) continue;   // Kp is a multiple of 64
-        uint32_t h0, h1, l0 = 0u, l1 = 0u;
-        if (lo) {
-            tc_split2<true>(tc_pack2(x[4 * j] * sc, x[4 * j + 1] * sc), h0, l0);
-            tc_split2<true>(tc_pack2(x[4 * j + 2] * sc, x[4 * j + 3] * sc), h1, l1);
-            *reinterpret_cast<uint2 *>(lo + m * Kp + k) = make_uint2(l0, l1);
-        } else {
-            tc_split2<false>(tc_pack2(x[4 * j] * sc, x[4 * j + 1] * sc), h0, l0);
-            tc_split2<false>(tc_pack2(x[4 * j + 2] * sc, x[4 * j + 3] * sc), h1, l1);
+        for (int j = 0; j < 2; ++j) {
+            const int kk = 256 * j + 8 * lane, st = kk / TC_WK;
+            if (m < M && k0 + kk < pl.Kp && (band == 0 || s_left[band - 1][st] != 0u) && act_store8<LO>(pl, band, m * pl.Kp + k0 + kk, x[j], sc, inv, amax < 0x7f800000u)) {
+                left = true;
+                s_left[band][st] = 1u;
+            }
         }
-        *reinterpret_cast<uint2 *>(hi + m * Kp + k) = make_uint2(h0, h1);
+        if (!__syncthreads_or(left) || band == TC_BANDS - 1) break;
+    }
+    if (tid < TC_GROUP_K / TC_AK && k0 + tid * TC_AK < pl.Kp) {
+        uint32_t n = 0u;
+        for (int band = 0; band < TC_BANDS - 1; ++band) n += s_left[band][2 * tid] + (s_left[band][2 * tid + 1] << 4);
+        *pl.band_byte(m0, k0 / TC_AK + tid) = (uint8_t)n;
     }
 }
 
@@ -447,10 +550,27 @@ __device__ __forceinline__ float4 tc_read4(uint32_t base, int c, uint32_t w_shif
     return lds4(base ^ (c << 4));
 }
 
+template <int WK>
+__device__ __forceinline__ void tc_write4(uint32_t base, int c, uint32_t w_shift, float4 v)
+{
+    if (WK == W_K) {
+        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(base ^ (c << 4)), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+        return;
+    }
+    const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        if (WK == W_N) sts1(base + (4 * c + e) * (TC_BN * 4), x[e]);
+        if (WK == W_K_ANY) sts1(base + 16 * c + 4 * e, x[e]);
+        if (WK == W_N_ANY) sts1(base + c * (TC_WN_PITCH * 4) + e * TC_WN_CLASS_BYTES + ((w_shift >> (8 * e)) & 0xffu) * 4, x[e]);
+    }
+}
+
 // One k-step (16 consecutive k of column n) of one row, scaled by sc -> hl[0..7] packed high parts, hl[8..15] packed low parts.
-// Returns the running packed largest |high part|: a half equal to 0x7c00 means that a value left fp16's range.
+// Keeps the running packed largest and smallest |high part|: 0x7c00 means that a value left fp16's range, less than
+// tc_safe_f16 that its parts may leave something (or that it is a zero).
 template <bool MODE3X, int WK>
-__device__ __forceinline__ void tc_convert_step(uint32_t base, uint32_t w_shift, int step, uint64_t sc2, uint32_t (&hl)[16], uint32_t &top)
+__device__ __forceinline__ void tc_convert_step(uint32_t base, uint32_t w_shift, int step, uint64_t sc2, uint32_t (&hl)[16], uint32_t &top, uint32_t &low)
 {
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
@@ -459,6 +579,8 @@ __device__ __forceinline__ void tc_convert_step(uint32_t base, uint32_t w_shift,
         tc_split2<MODE3X>(tc_mul2(tc_pack2(v.z, v.w), sc2), hl[2 * c + 1], hl[8 + 2 * c + 1]);
         asm("max.xorsign.abs.f16x2 %0, %0, %1;" : "+r"(top) : "r"(hl[2 * c]));
         asm("max.xorsign.abs.f16x2 %0, %0, %1;" : "+r"(top) : "r"(hl[2 * c + 1]));
+        asm("min.xorsign.abs.f16x2 %0, %0, %1;" : "+r"(low) : "r"(hl[2 * c]));
+        asm("min.xorsign.abs.f16x2 %0, %0, %1;" : "+r"(low) : "r"(hl[2 * c + 1]));
     }
 }
 
@@ -473,6 +595,32 @@ __device__ __forceinline__ uint32_t tc_row_amax(uint32_t base, uint32_t w_shift)
         amax = max(amax, __float_as_uint(v.w) & 0x7fffffffu);
     }
     return amax;
+}
+
+// Whether the parts of this row's 32 values leave something: the smallest nonzero magnitude tells that they do not, else every
+// value's parts are made once more.
+template <bool MODE3X, int WK>
+__device__ __forceinline__ bool tc_row_left(uint32_t base, uint32_t w_shift, float sc)
+{
+    uint32_t amin = 0xffffffffu;   // of 2 |bits| - 1, in which a zero is the largest
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        const float4 v = tc_read4<WK>(base, c, w_shift);
+        amin = min(min(amin, __float_as_uint(v.x) * 2u - 1u), min(__float_as_uint(v.y) * 2u - 1u, __float_as_uint(v.z) * 2u - 1u));
+        amin = min(amin, __float_as_uint(v.w) * 2u - 1u);
+    }
+    if (amin == 0xffffffffu || __uint_as_float((amin + 1u) >> 1) * sc >= (MODE3X ? 0.03125f : 6.103515625e-5f)) return false;
+    bool left = false;
+#pragma unroll 1
+    for (int c = 0; c < 8; ++c) {
+        const float4 v = tc_read4<WK>(base, c, w_shift);
+        uint32_t h, l;
+        float r[4];
+        tc_split2_left<MODE3X>(v.x * sc, v.y * sc, h, l, r[0], r[1]);
+        tc_split2_left<MODE3X>(v.z * sc, v.w * sc, h, l, r[2], r[3]);
+        left |= r[0] != 0.0f || r[1] != 0.0f || r[2] != 0.0f || r[3] != 0.0f;
+    }
+    return left;
 }
 
 // Tensor maps of the weights: one, or one per class of rows (W_K_ANY, W_N_ANY).
@@ -495,17 +643,17 @@ struct WMaps {
 // accumulator, and when it ends the drain warps read it with tcgen05.ld, remove both scales and add it, in round-to-nearest
 // fp32, to running sums that they keep in registers (one thread = one output column n, 128 sums = 128 rows m).
 template <int NT, bool MODE3X, int WK>
-__global__ void __launch_bounds__(TcCfg<NT, WK>::THREADS, 1)
-cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CUtensorMap tm_ahi,
-                  const __grid_constant__ CUtensorMap tm_alo, const __grid_constant__ TcParams p)
+__global__ void __launch_bounds__(TcCfg<NT, MODE3X, WK>::THREADS, 1)
+cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ TcParams p)
 {
-    using Cfg = TcCfg<NT, WK>;
+    using Cfg = TcCfg<NT, MODE3X, WK>;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     constexpr int B_WFULL = 0, B_WEMPTY = B_WFULL + Cfg::W_STAGES, B_AFULL = B_WEMPTY + Cfg::W_STAGES,
                   B_AEMPTY = B_AFULL + Cfg::A_STAGES, B_TFULL = B_AEMPTY + Cfg::A_STAGES, B_TEMPTY = B_TFULL + NT * Cfg::TMEM_STAGES,
                   B_ACCFULL = B_TEMPTY + NT * Cfg::TMEM_STAGES, B_ACCEMPTY = B_ACCFULL + NT * Cfg::ACC_BUFS;
-    static_assert(B_ACCEMPTY + NT * Cfg::ACC_BUFS == Cfg::BARS, "barrier count");
+    constexpr int B_XFULL = B_ACCEMPTY + NT * Cfg::ACC_BUFS, B_XEMPTY = B_XFULL + NT * 4;   // left-overs of the weights, per converter warp
+    static_assert(B_XEMPTY + NT * 4 == Cfg::BARS, "barrier count");
     auto bar = [&](int idx) { return smem_base + Cfg::BAR_OFF + 8u * idx; };
     auto wfull_bar = [&](int s) { return bar(B_WFULL + s); };
     auto wempty_bar = [&](int s) { return bar(B_WEMPTY + s); };
@@ -515,6 +663,8 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
     auto tempty_bar = [&](int w, int t) { return bar(B_TEMPTY + w * Cfg::TMEM_STAGES + t); };
     auto accfull_bar = [&](int w, int b) { return bar(B_ACCFULL + w * Cfg::ACC_BUFS + b); };
     auto accempty_bar = [&](int w, int b) { return bar(B_ACCEMPTY + w * Cfg::ACC_BUFS + b); };
+    auto xfull_bar = [&](int w, int q) { return bar(B_XFULL + w * 4 + q); };
+    auto xempty_bar = [&](int w, int q) { return bar(B_XEMPTY + w * 4 + q); };
     const uint32_t tmem_holder = smem_base + Cfg::HOLD_OFF, abort_flag = tmem_holder + 4;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -535,6 +685,7 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
         for (int w = 0; w < NT; ++w) {
             for (int t = 0; t < Cfg::TMEM_STAGES; ++t) { mbar_init(tfull_bar(w, t), 4); mbar_init(tempty_bar(w, t), 1); }
             for (int b = 0; b < Cfg::ACC_BUFS; ++b) { mbar_init(accfull_bar(w, b), 2); mbar_init(accempty_bar(w, b), 4); }
+            for (int q = 0; q < 4; ++q) { mbar_init(xfull_bar(w, q), 1); mbar_init(xempty_bar(w, q), 1); }
         }
         sts1u(abort_flag, 0u);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -601,14 +752,29 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
                 bool ok = true;
                 while (ok && walk.next(p, seg)) {
                     const int32_t m0 = (seg.tile % p.tiles_m) * TC_BM;
-                    for (int kb = seg.k0 & ~1; kb < seg.k1; kb += 2, ++it) {
-                        const int s = it % Cfg::A_STAGES;
-                        ok = mbar_wait(aempty_bar(s), ((it / Cfg::A_STAGES) & 1u) ^ 1u, abort_flag, p.status, 8u);
-                        if (!ok) break;
-                        const uint32_t stage = smem_base + Cfg::A_RING + s * Cfg::A_STAGE_BYTES;
-                        mbar_expect_tx(afull_bar(s), (uint32_t)((MODE3X ? 2 : 1) * TC_A_TILE_BYTES));
-                        tma_load_2d(stage, &tm_ahi, afull_bar(s), kb * TC_WK, m0);
-                        if (MODE3X) tma_load_2d(stage + TC_A_TILE_BYTES, &tm_alo, afull_bar(s), kb * TC_WK, m0);
+                    const uint2 *bands = reinterpret_cast<const uint2 *>(p.a_bands) + (int64_t)(seg.tile % p.tiles_m) * p.a_stages;
+                    uint2 b8 = __ldcg(bands + (seg.k0 >> 1));   // bands of the eight blocks of 16 rows, a byte each
+                    for (int kb = seg.k0 & ~1; kb < seg.k1 && ok; kb += 2) {
+                        const uint2 now = b8;
+                        if (kb + 2 < seg.k1) b8 = __ldcg(bands + (kb >> 1) + 1);
+                        uint32_t masks = 0u;                        // byte b - 1, and b + 1 for the second 32 k: the blocks that have something in band b
+                        if ((now.x | now.y) != 0u) {
+                            for (int j = 0; j < 16; ++j) {
+                                const uint32_t n = ((j < 8 ? now.x : now.y) >> (4 * (j & 7))) & 0xfu;
+                                for (uint32_t b = 0; b < n; ++b) masks |= 1u << (16 * (j & 1) + 8 * b + (j >> 1));
+                            }
+                        }
+                        const int bands_here = 1 + (masks != 0u) + ((masks & 0xff00ff00u) != 0u);
+                        for (int band = 0; band < bands_here; ++band, ++it) {
+                            const int s = it % Cfg::A_STAGES;
+                            ok = mbar_wait(aempty_bar(s), ((it / Cfg::A_STAGES) & 1u) ^ 1u, abort_flag, p.status, 8u);
+                            if (!ok) break;
+                            if (band == 0) sts1u(smem_base + Cfg::BAND_OFF + s * 4, masks);
+                            const uint32_t stage = smem_base + Cfg::A_RING + s * Cfg::A_STAGE_BYTES;
+                            mbar_expect_tx(afull_bar(s), (uint32_t)((MODE3X ? 2 : 1) * TC_A_TILE_BYTES));
+                            tma_load_3d(stage, &tm_a, afull_bar(s), kb * TC_WK, m0, band * (MODE3X ? 2 : 1));
+                            if (MODE3X) tma_load_3d(stage + TC_A_TILE_BYTES, &tm_a, afull_bar(s), kb * TC_WK, m0, 2 * band + 1);
+                        }
                     }
                 }
                 // the last stages' releases (commits of the MMA issuers) must have arrived before the CTA may exit; on the way out
@@ -635,44 +801,51 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
                 constexpr uint32_t idesc = make_idesc_f16(TC_BN, TC_BM);
                 uint32_t it = 0, a_it = 0;       // W blocks and activation stages so far
                 int ab = 0;                      // accumulator buffer and its phase
-                uint32_t aph = 0;
+                uint32_t aph = 0, xph = 0;       // ... of the left-overs, a bit per converter warp
                 bool open = false, ok = true;    // a chain is accumulating
-                // Ends the open chain: the drain warps learn where its scales are, and that it is complete when its MMAs retire
-                auto close_chain = [&](uint32_t last_it, int last_kb, bool last_of_run) {
+                // Ends the open chain: the drain warps learn where its scales are and which blocks of 16 rows m it has (mask, from bit
+                // 16), for left-overs of the weights how often they were scaled (from bit 9) and which quarters of the rows n have
+                // any (from bit 24), and that it is complete when its MMAs retire
+                constexpr uint32_t WHOLE = 0x0fff0000u;
+                auto close_chain = [&](uint32_t last_it, int a_scales, uint32_t what, bool last_of_run) {
                     const uint32_t q = smem_base + Cfg::INFO_OFF + (w * Cfg::ACC_BUFS + ab) * 8;
-                    sts1u(q, (last_it % Cfg::WS_SLOTS) | (last_of_run ? 0x100u : 0u));
-                    sts1u(q + 4, (uint32_t)(last_kb / TC_GROUP_KB));
+                    sts1u(q, (last_it % Cfg::WS_SLOTS) | (last_of_run ? 0x100u : 0u) | what);
+                    sts1u(q + 4, (uint32_t)a_scales);
                     mbar_arrive(accfull_bar(w, ab));
                     tc_commit(accfull_bar(w, ab));
                     if (++ab == Cfg::ACC_BUFS) { ab = 0; aph ^= 1u; }
                     open = false;
                 };
-                // operands of one W block: the activation stage where it opens one, and the converted W rows
-                auto wait_block = [&](uint32_t i, uint32_t a, bool opens_stage) {
-                    if (opens_stage && !mbar_wait(afull_bar(a % Cfg::A_STAGES), (a / Cfg::A_STAGES) & 1u, abort_flag, p.status, 2u)) return false;
-                    return mbar_wait(tfull_bar(w, i % Cfg::TMEM_STAGES), (i / Cfg::TMEM_STAGES) & 1u, abort_flag, p.status, 3u);
+                auto open_chain = [&]() {   // the drain warps must have emptied this accumulator
+                    if (!mbar_wait(accempty_bar(w, ab), aph ^ 1u, abort_flag, p.status, 7u)) return false;
+                    tc_fence_after();
+                    open = true;
+                    return true;
                 };
+                auto wait_weights = [&](uint32_t i) { return mbar_wait(tfull_bar(w, i % Cfg::TMEM_STAGES), (i / Cfg::TMEM_STAGES) & 1u, abort_flag, p.status, 3u); };
+                auto wait_stage = [&](uint32_t a) { return mbar_wait(afull_bar(a % Cfg::A_STAGES), (a / Cfg::A_STAGES) & 1u, abort_flag, p.status, 2u); };
+                // operands of one W block: the activation stage where it opens one, and the converted W rows
+                auto wait_block = [&](uint32_t i, uint32_t a, bool opens_stage) { return (!opens_stage || wait_stage(a)) && wait_weights(i); };
+                // what the converters say of a block of weights, a byte per warp: 1 = a row's scale had to change, the chain ends before
+                // it; 2 = something is left of it.  And what is left of the activations of a stage, see their producer.
+                auto block_word = [&](uint32_t i) { return lds1u(smem_base + Cfg::BRK_OFF + ((i % Cfg::TMEM_STAGES) * NT + w) * 4); };
+                auto stage_masks = [&](uint32_t a) { return lds1u(smem_base + Cfg::BAND_OFF + (a % Cfg::A_STAGES) * 4); };
                 while (ok && walk.next(p, seg)) {
                     ok = wait_block(it, a_it, true);
+                    uint32_t word = block_word(it), masks = stage_masks(a_it);
                     for (int kb = seg.k0; kb < seg.k1 && ok; ++kb, ++it) {
-                        const int t = it % Cfg::TMEM_STAGES;
+                        const int s = a_it % Cfg::A_STAGES, t = it % Cfg::TMEM_STAGES;
+                        const bool last_block = kb == seg.k1 - 1, ends_stage = (kb & 1) || last_block;
                         tc_fence_after();
-                        // a row whose scale had to change (see the converters) ends the chain before this block
-                        if (open && lds1u(smem_base + Cfg::BRK_OFF + (t * NT + w) * 4) != 0u) close_chain(it - 1, kb - 1, false);
-                        bool first = false;
-                        if (!open) {   // the drain warps must have emptied this accumulator
-                            ok = mbar_wait(accempty_bar(w, ab), aph ^ 1u, abort_flag, p.status, 7u);
-                            if (!ok) break;
-                            tc_fence_after();
-                            open = first = true;
-                        }
-                        const int s = a_it % Cfg::A_STAGES;
+                        if (open && (word & 0x01010101u) != 0u) close_chain(it - 1, (kb - 1) / TC_GROUP_KB, WHOLE, false);
+                        const bool first = !open;
+                        if (!open && !(ok = open_chain())) break;
+                        const uint32_t rare = (word & 0x02020202u) | masks;
                         const uint32_t stage = smem_base + Cfg::A_RING + s * Cfg::A_STAGE_BYTES + (uint32_t)(kb & 1) * (TC_WK * 2);
                         const uint64_t bhi = make_kmajor_sw128_desc(stage), blo = make_kmajor_sw128_desc(stage + TC_A_TILE_BYTES);
                         const uint32_t bhi_lo = (uint32_t)bhi, bhi_hi = (uint32_t)(bhi >> 32), blo_lo = (uint32_t)blo, blo_hi = (uint32_t)(blo >> 32);
                         const uint32_t acc = tmem_base + Cfg::ACC_COL + (w * Cfg::ACC_BUFS + ab) * TC_BM;
-                        const uint32_t w_hi = tmem_base + Cfg::OP_COL + t * Cfg::OP_STAGE_COLS + w * 32;
-                        const bool last_of_run = kb == seg.k1 - 1, ends_stage = (kb & 1) || last_of_run;
+                        const uint32_t w_hi = tmem_base + Cfg::OP_COL + t * Cfg::OP_STAGE_COLS + w * Cfg::OP_COLS;
                         // 16 fp16 per k-step: 8 TMEM columns of W, 32 bytes (descriptor units of 16 B) of the activations
                         tc_mma_ts(acc, w_hi, bhi_lo, bhi_hi, idesc, first ? 0u : 1u);
                         if (MODE3X) {
@@ -682,18 +855,90 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
                         // Look ahead: make sure the operands of the next block are there BEFORE the last MMAs of this one are
                         // issued.  Issue is back-pressured by the tensor pipe, so once those are in, only the commits stand
                         // between them and the next block's first MMA.
-                        if (!last_of_run) ok = wait_block(it + 1, a_it + 1, ends_stage);
-                        tc_mma_ts(acc, w_hi + 16, bhi_lo + 2, bhi_hi, idesc, 1u);
+                        uint32_t next_word = 0u, next_masks = masks;
+                        if (rare == 0u && !last_block) {
+                            ok = wait_block(it + 1, a_it + 1, ends_stage);
+                            next_word = block_word(it + 1);
+                            if (ends_stage) next_masks = stage_masks(a_it + 1);
+                        }
+                        tc_mma_ts(acc, w_hi + Cfg::STEP_COLS, bhi_lo + 2, bhi_hi, idesc, 1u);
                         if (MODE3X) {
                             tc_mma_ts(acc, w_hi + 24, bhi_lo + 2, bhi_hi, idesc, 1u);
                             tc_mma_ts(acc, w_hi + 16, blo_lo + 2, blo_hi, idesc, 1u);
                         }
-                        if (last_of_run || ((kb + 1) & p.chain_mask) == 0) close_chain(it, kb, last_of_run);
-                        if (ends_stage) {   // the activation stage may be refilled once these MMAs retire
-                            tc_commit(aempty_bar(s));
-                            ++a_it;
+                        if (rare != 0u || last_block || ((kb + 1) & p.chain_mask) == 0) close_chain(it, kb / TC_GROUP_KB, WHOLE, last_block && (word & 0x02020202u) == 0u && (masks >> (16 * (kb & 1)) & 0xffffu) == 0u);
+                        if (rare == 0u) {
+                            if (ends_stage) {   // the activation stage may be refilled once these MMAs retire
+                                tc_commit(aempty_bar(s));
+                                ++a_it;
+                            }
+                            tc_commit(tempty_bar(w, t));   // and the TMEM operand stage rewritten
+                        } else {
+                            // chains of the left-overs.  Level 0 multiplies the weights' parts with what is left of the
+                            // activations, the others what is left of the weights with both.
+                            const uint32_t here = masks >> (16 * (kb & 1)) & 0xffffu;
+                            uint32_t more = 0u, quarters = 0xfu, wt = w_hi;
+                            for (int q = 0; q < 4; ++q) more |= (word >> (8 * q + 1) & 1u) << q;
+#pragma unroll 1
+                            for (uint32_t level = 0;; ++level) {
+                                if (level > 0) {
+                                    quarters = more;
+                                    more = 0u;
+#pragma unroll 1
+                                    for (int q = 0; q < 4 && ok; ++q) {
+                                        if ((quarters >> q & 1u) == 0u) continue;
+                                        ok = mbar_wait(xfull_bar(w, q), xph >> q & 1u, abort_flag, p.status, 18u);
+                                        more |= (lds1u(smem_base + Cfg::LEFT_OFF + w * 4) >> (8 * q) & 1u) << q;
+                                    }
+                                    xph ^= quarters;
+                                    if (!ok) break;
+                                    tc_fence_after();
+                                    wt = tmem_base + Cfg::LEFT_COL + w * Cfg::OP_COLS;
+                                }
+#pragma unroll 1
+                                for (int band = level == 0 ? 1 : 0; band < TC_BANDS; ++band) {
+                                    const uint32_t mask = band == 0 ? 0xffu : here >> (8 * (band - 1)) & 0xffu;
+                                    if (mask == 0u) break;
+                                    ok = (band == 0 || wait_stage(a_it + band)) && open_chain();
+                                    if (!ok) break;
+                                    constexpr uint32_t idesc16 = make_idesc_f16(TC_BN, TC_SUB);
+                                    uint32_t at = (smem_base + Cfg::A_RING + ((a_it + band) % Cfg::A_STAGES) * Cfg::A_STAGE_BYTES + (uint32_t)(kb & 1) * (TC_WK * 2)) >> 4;
+                                    uint32_t d = tmem_base + Cfg::ACC_COL + (w * Cfg::ACC_BUFS + ab) * TC_BM;
+#pragma unroll 1
+                                    for (uint32_t rows = mask; rows != 0u; rows >>= 1, d += TC_SUB, at += TC_SUB * 128 / 16) {
+                                        if ((rows & 1u) == 0u) continue;
+#pragma unroll 1
+                                        for (uint32_t step = 0; step < 2; ++step) {
+                                            const uint32_t a = wt + Cfg::STEP_COLS * step, h = (bhi_lo & ~0x3fffu) | (at + 2 * step);
+                                            tc_mma_ts(d, a, h, bhi_hi, idesc16, step);
+                                            if (MODE3X) {
+                                                tc_mma_ts(d, a + 8, h, bhi_hi, idesc16, 1u);
+                                                tc_mma_ts(d, a, h + (TC_A_TILE_BYTES >> 4), bhi_hi, idesc16, 1u);
+                                            }
+                                        }
+                                    }
+                                    const bool last_band = band == TC_BANDS - 1 || (here >> (8 * band) & 0xffu) == 0u;
+                                    close_chain(it, band * p.groups + kb / TC_GROUP_KB, level << 9 | mask << 16 | quarters << 24, last_block && more == 0u && last_band);
+                                }
+                                if (!ok) break;
+                                if (level == 0) {
+                                    tc_commit(tempty_bar(w, t));
+                                } else {
+                                    for (int q = 0; q < 4; ++q)
+                                        if (quarters >> q & 1u) tc_commit(xempty_bar(w, q));
+                                }
+                                if (more == 0u) break;
+                            }
+                            if (ok && ends_stage)
+                                for (uint32_t n = 1u + (masks != 0u) + ((masks & 0xff00ff00u) != 0u); n > 0; --n, ++a_it) tc_commit(aempty_bar(a_it % Cfg::A_STAGES));
+                            if (ok && !last_block) {
+                                ok = wait_block(it + 1, a_it, ends_stage);
+                                next_word = block_word(it + 1);
+                                next_masks = stage_masks(a_it);
+                            }
                         }
-                        tc_commit(tempty_bar(w, t));   // and the TMEM operand stage rewritten
+                        word = next_word;
+                        masks = next_masks;
                     }
                 }
             }
@@ -705,13 +950,53 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
         const int w = (warp - 4) >> 2;                // W tile of this warpgroup
         const int q = warp & 3;                       // TMEM lane quarter this warp may touch
         const int row = q * 32 + lane;                // row of the W tile = TMEM lane
-        const uint32_t dst0 = tmem_base + ((uint32_t)(q * 32) << 16) + Cfg::OP_COL + w * 32;
+        const uint32_t dst0 = tmem_base + ((uint32_t)(q * 32) << 16) + Cfg::OP_COL + w * Cfg::OP_COLS;
         TcWalk walk(p);
         TcSeg seg;
         float sc = 1.0f, inv = 1.0f;                  // this row's scale in the open chain
         bool set = false;                             // ... is fixed: the row has had a nonzero element
         uint32_t it = 0;
         bool ok = true;
+        // What is left of this warp's rows of a block, 2^38 times the scale, replaces the raw values; its parts go to the left-overs'
+        // stage, and once more what those leave.
+        uint32_t x_it = 0;
+        auto left_overs = [&](uint32_t rowp) {
+            const uint32_t dst = tmem_base + ((uint32_t)(q * 32) << 16) + Cfg::LEFT_COL + w * Cfg::OP_COLS;
+            bool again = true;
+#pragma unroll 1
+            for (bool raw = true; again; raw = false, ++x_it) {
+                ok = mbar_wait(xempty_bar(w, q), (x_it & 1u) ^ 1u, abort_flag, p.status, 17u);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) return;
+                tc_fence_after();
+                again = false;
+#pragma unroll 1
+                for (int c = 0; c < 8; ++c) {
+                    float4 v = tc_read4<WK>(rowp, c, p.w_shift);
+                    uint32_t h[2], l[2];
+                    if (raw) {
+                        tc_split2_left<MODE3X>(v.x * sc, v.y * sc, h[0], l[0], v.x, v.y);
+                        tc_split2_left<MODE3X>(v.z * sc, v.w * sc, h[0], l[0], v.z, v.w);
+                    }
+                    tc_split2_left<MODE3X>(v.x * TC_LEFT_SCALE, v.y * TC_LEFT_SCALE, h[0], l[0], v.x, v.y);
+                    tc_split2_left<MODE3X>(v.z * TC_LEFT_SCALE, v.w * TC_LEFT_SCALE, h[1], l[1], v.z, v.w);
+                    tc_write4<WK>(rowp, c, p.w_shift, v);
+                    again |= v.x != 0.0f || v.y != 0.0f || v.z != 0.0f || v.w != 0.0f;
+                    __syncwarp();
+                    const uint32_t at = dst + (c >> 2) * Cfg::STEP_COLS + 2 * (c & 3);
+                    tc_st2(at, h[0], h[1]);
+                    if (MODE3X) tc_st2(at + 8, l[0], l[1]);
+                }
+                again = __any_sync(0xffffffffu, again);
+                if (lane == 0) sts1b(smem_base + Cfg::LEFT_OFF + w * 4 + q, again ? 1u : 0u);
+                tc_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(xfull_bar(w, q));
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the slot's next contents come through TMA
+            __syncwarp();
+        };
         while (ok && walk.next(p, seg)) {
             for (int kb = seg.k0; kb < seg.k1; ++kb, ++it) {
                 const int s = it % Cfg::W_STAGES, t = it % Cfg::TMEM_STAGES;
@@ -727,39 +1012,50 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
                     // nothing but zeros of this row is in the accumulator: any scale is right for what is there
                     const uint32_t amax = tc_row_amax<WK>(rowp, p.w_shift);
                     tc_scale<TC_W_EXP>(amax, sc, inv);
-                    set = amax != 0u;
+                    set = amax != 0u && amax < 0x7f800000u;   // (a row that is not finite any more may have any scale, too)
                 }
                 __syncwarp();
                 const uint32_t dst = dst0 + t * Cfg::OP_STAGE_COLS;
-                bool grew = false;
+                bool grew = false, left = false;
                 for (;;) {
-                    uint32_t top = 0u;
+                    uint32_t top = 0u, low = 0x7bff7bffu;
                     const uint64_t sc2 = tc_pack2(sc, sc);
 #pragma unroll 1
                     for (int step = 0; step < 2; ++step) {
                         uint32_t hl[16];
-                        tc_convert_step<MODE3X, WK>(rowp, p.w_shift, step, sc2, hl, top);
+                        tc_convert_step<MODE3X, WK>(rowp, p.w_shift, step, sc2, hl, top, low);
                         if (MODE3X) tc_st16(dst + step * 16, hl);
-                        else        tc_st8(dst + step * 16, hl);
+                        else        tc_st8(dst + step * Cfg::STEP_COLS, hl);
                     }
                     top &= 0x7fff7fffu;
+                    low &= 0x7fff7fffu;
                     const bool over = (top >> 16) >= 0x7c00u || (top & 0xffffu) >= 0x7c00u;
-                    if (grew || !__any_sync(0xffffffffu, over)) break;
-                    // rare: a row's magnitudes grew more than fourfold since its chain began: new scale, and once more
-                    grew = true;
-                    if (over) tc_scale<TC_W_EXP>(tc_row_amax<WK>(rowp, p.w_shift), sc, inv);
-                    tc_wait_st();
-                    __syncwarp();
+                    const bool small = set && ((low >> 16) < tc_safe_f16<MODE3X>() || (low & 0xffffu) < tc_safe_f16<MODE3X>());
+                    if (!__any_sync(0xffffffffu, over || small)) break;
+                    if (!grew && __any_sync(0xffffffffu, over)) {
+                        // rare: a row's magnitudes grew more than fourfold since its chain began: new scale, and once more
+                        grew = true;
+                        if (over) {
+                            const uint32_t amax = tc_row_amax<WK>(rowp, p.w_shift);
+                            tc_scale<TC_W_EXP>(amax, sc, inv);
+                            set = amax < 0x7f800000u;
+                        }
+                        tc_wait_st();
+                        __syncwarp();
+                        continue;
+                    }
+                    // zeros, or elements too small for this scale
+                    left = __any_sync(0xffffffffu, small && tc_row_left<MODE3X, WK>(rowp, p.w_shift, sc));
+                    break;
                 }
                 sts1(smem_base + Cfg::WS_OFF + (((it % Cfg::WS_SLOTS) * NT + w) * TC_BN + row) * 4, inv);
-                if (lane == 0) sts1b(smem_base + Cfg::BRK_OFF + (t * NT + w) * 4 + q, grew && !chain_start ? 1u : 0u);
+                if (lane == 0) sts1b(smem_base + Cfg::BRK_OFF + (t * NT + w) * 4 + q, (grew && !chain_start ? 1u : 0u) | (left ? 2u : 0u));
                 tc_wait_st();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) {
-                    mbar_arrive(wempty_bar(s));   // the raw block now lives in TMEM: its ring slot may be refilled
-                    mbar_arrive(tfull_bar(w, t));
-                }
+                if (lane == 0) mbar_arrive(tfull_bar(w, t));
+                if (left) left_overs(rowp);
+                if (lane == 0) mbar_arrive(wempty_bar(s));   // the raw block now lives in TMEM: its ring slot may be refilled
             }
         }
         // the last operand stages' releases must have arrived before the CTA may exit
@@ -778,13 +1074,13 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
         uint32_t chains = 0;
         bool ok = true;
         while (ok && walk.next(p, seg)) {
-            const int64_t m0 = (int64_t)(seg.tile % p.tiles_m) * TC_BM, n0 = (int64_t)(seg.tile / p.tiles_m) * (NT * TC_BN) + w * TC_BN;
+            const float *a_inv = p.a_inv + (int64_t)(seg.tile % p.tiles_m) * TC_BM + row;
             uint64_t sum[TC_BM / 2];   // pairs of rows
 #pragma unroll
             for (int i = 0; i < TC_BM / 2; ++i) sum[i] = 0ull;
             // the inverse scales of the activation rows: thread `row` fetches row m0 + row of the group it expects next
-            int have_group = seg.k0 / TC_GROUP_KB;
-            float my_inv = p.a_inv[(int64_t)have_group * p.m_pad + m0 + row];
+            int have = seg.k0 / TC_GROUP_KB;   // scales: band * groups + group
+            float my_inv = a_inv[have * p.m_pad];
             for (bool last = false; !last; ++chains) {
                 const int ab = chains % Cfg::ACC_BUFS;
                 ok = mbar_wait<TC_DRAIN_SLEEP_NS>(accfull_bar(w, ab), (chains / Cfg::ACC_BUFS) & 1u, abort_flag, p.status, 6u);
@@ -801,24 +1097,24 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t what = lds1u(smem_base + Cfg::INFO_OFF + (w * Cfg::ACC_BUFS + ab) * 8);
-                const int group = (int)lds1u(smem_base + Cfg::INFO_OFF + (w * Cfg::ACC_BUFS + ab) * 8 + 4);
+                const int scales = (int)lds1u(smem_base + Cfg::INFO_OFF + (w * Cfg::ACC_BUFS + ab) * 8 + 4);
                 last = (what & 0x100u) != 0u;
-                if (group != have_group) my_inv = p.a_inv[(int64_t)group * p.m_pad + m0 + row];
+                if (scales != have) my_inv = a_inv[scales * p.m_pad];
                 const uint32_t as = smem_base + Cfg::AS_OFF + ((chains & 1u) * NT + w) * (TC_BM * 4);
                 sts1(as + row * 4, my_inv);
-                const float wi = lds1(smem_base + Cfg::WS_OFF + (((what & 0xffu) * NT + w) * TC_BN + row) * 4);
+                float wi = lds1(smem_base + Cfg::WS_OFF + (((what & 0xffu) * NT + w) * TC_BN + row) * 4);
+                for (uint32_t level = what >> 9 & 7u; level > 0; --level) wi *= 1.0f / TC_LEFT_SCALE;
                 asm volatile("bar.sync %0, 128;" ::"r"(1 + w) : "memory");
-                have_group = group;
-                if (!last && group < (seg.k1 - 1) / TC_GROUP_KB) {   // most likely the next chain's group
-                    have_group = group + 1;
-                    my_inv = p.a_inv[(int64_t)have_group * p.m_pad + m0 + row];
+                have = scales;
+                if (!last && scales < (seg.k1 - 1) / TC_GROUP_KB) {   // most likely the next chain's group
+                    have = scales + 1;
+                    my_inv = a_inv[have * p.m_pad];
                 }
                 const uint32_t src = tmem_base + lane_addr + Cfg::ACC_COL + (w * Cfg::ACC_BUFS + ab) * TC_BM;
                 // Remove both scales and add.  (The product of the two inverse scales is finite unless the product of the segment's
                 // largest magnitudes is beyond fp32's range by 2^27.)
                 const uint64_t wi2 = tc_pack2(wi, wi);
-#pragma unroll
-                for (int cc = 0; cc < TC_BM / 16; ++cc) {
+                auto add16 = [&](int cc) {
                     uint32_t r[16];
                     tc_ld16(src + cc * 16, r);
 #pragma unroll
@@ -828,13 +1124,26 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
                         s0 = tc_fma2(tc_pack2(__uint_as_float(r[i]), __uint_as_float(r[i + 1])), tc_mul2(tc_pack2(f.x, f.y), wi2), s0);
                         s1 = tc_fma2(tc_pack2(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])), tc_mul2(tc_pack2(f.z, f.w), wi2), s1);
                     }
+                };
+                if ((what & 0x00ff0e00u) == 0x00ff0000u) {
+#pragma unroll
+                    for (int cc = 0; cc < TC_BM / TC_SUB; ++cc) add16(cc);
+                } else {
+                    // left-overs: the blocks of 16 rows m, and the quarters of the rows n, that have some
+                    uint32_t mask = (what >> (24 + q) & 1u) ? what >> 16 & 0xffu : 0u;
+#pragma unroll
+                    for (int cc = 0; cc < TC_BM / TC_SUB; ++cc) {
+                        const bool in_chain = (mask & 1u) != 0u;
+                        asm volatile("shr.u32 %0, %0, 1;" : "+r"(mask));   // one test at a time: eight predicates held together are too many
+                        if (in_chain) add16(cc);
+                    }
                 }
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(accempty_bar(w, ab));
             }
             if (!ok) break;
-            const int64_t n = n0 + row;
+            const int64_t m0 = (int64_t)(seg.tile % p.tiles_m) * TC_BM, n = (int64_t)(seg.tile / p.tiles_m) * (NT * TC_BN) + w * TC_BN + row;
             if (seg.slot >= 0) {
                 // partial tile: float4 number i of 32 for all 128 columns, then the next, so that a warp writes 512 contiguous bytes
                 ulonglong2 *P = reinterpret_cast<ulonglong2 *>(p.partials) + ((int64_t)seg.slot * NT + w) * (TC_BM * TC_BN / 4) + row;
@@ -1079,14 +1388,14 @@ static int make_w_maps(EncodeTiledFn enc, WMaps *m, uint32_t *shift, const float
     return CN_OK;
 }
 
-// Activation plane: fp16, k contiguous with pitch Kp, box 64 k x 128 rows, 128-byte swizzle.
-static int make_a_map(EncodeTiledFn enc, CUtensorMap *map, const uint16_t *base, int64_t Kp, int64_t M)
+// Activation planes: fp16, k contiguous with pitch Kp, `plane` elements apart, box 64 k x 128 rows of one, 128-byte swizzle.
+static int make_a_map(EncodeTiledFn enc, CUtensorMap *map, const uint16_t *base, int64_t Kp, int64_t M, int64_t plane, int planes)
 {
-    cuuint64_t dims[2] = {(cuuint64_t)Kp, (cuuint64_t)M};
-    cuuint64_t strides[1] = {(cuuint64_t)Kp * sizeof(uint16_t)};
-    cuuint32_t box[2] = {(cuuint32_t)TC_AK, (cuuint32_t)TC_BM};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<uint16_t *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    cuuint64_t dims[3] = {(cuuint64_t)Kp, (cuuint64_t)M, (cuuint64_t)planes};
+    cuuint64_t strides[2] = {(cuuint64_t)Kp * sizeof(uint16_t), (cuuint64_t)plane * sizeof(uint16_t)};
+    cuuint32_t box[3] = {(cuuint32_t)TC_AK, (cuuint32_t)TC_BM, 1};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<uint16_t *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     CN_REQUIRE(r == CUDA_SUCCESS, CN_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d (activation planes %lld x %lld)", (int)r, (long long)M, (long long)Kp);
     return CN_OK;
@@ -1124,60 +1433,72 @@ bool cn_gemm_tc_supported(cn_context *, int transA, int transB, int64_t M, int64
 static int any_chain(int64_t K) { return K < 384 ? 1 : K < 1024 ? 2 : K < 3072 ? 4 : K < 12288 ? 8 : TC_GROUP_KB; }
 
 template <int NT, bool MODE3X, int WK>
-static int launch_cfg(const WMaps &mw, const CUtensorMap &mhi, const CUtensorMap &mlo, const TcParams &prm, int64_t grid, int dev, cudaStream_t s)
+static int launch_cfg(const WMaps &mw, const CUtensorMap &ma, const TcParams &prm, int64_t grid, int dev, cudaStream_t s)
 {
-    using Cfg = TcCfg<NT, WK>;
+    using Cfg = TcCfg<NT, MODE3X, WK>;
     static bool attr_set[64] = {};   // per device: the attribute belongs to the device's copy of the function
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
         CN_CUDA(cudaFuncSetAttribute(cn_gemm_tc_kernel<NT, MODE3X, WK>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
-    CN_CUDA(cn_launch_pdl(cn_gemm_tc_kernel<NT, MODE3X, WK>, dim3((unsigned)grid), Cfg::THREADS, Cfg::SMEM_BYTES, s, mw, mhi, mlo, prm));
+    CN_CUDA(cn_launch_pdl(cn_gemm_tc_kernel<NT, MODE3X, WK>, dim3((unsigned)grid), Cfg::THREADS, Cfg::SMEM_BYTES, s, mw, ma, prm));
     cn_count_launch();
     return CN_OK;
 }
 
-// Geometry of the planes of an M x K operand in one allocation: hi, lo (only in the 3x mode), inverse scales.
+// Geometry of the planes of an M x K operand in one allocation.
 void cn_plane_layout(int64_t M, int64_t K, int mode, cn_planes *pl)
 {
+    pl->parts = mode == CN_GEMM_3XTF32 ? 2 : 1;
     pl->Kp = (K + TC_AK - 1) / TC_AK * TC_AK;
+    pl->plane = (M * pl->Kp + 127) / 128 * 128;
     pl->m_pad = (M + TC_BM - 1) / TC_BM * TC_BM;
     pl->groups = (K + TC_GROUP_K - 1) / TC_GROUP_K;
-    const size_t plane = ((size_t)M * pl->Kp * sizeof(uint16_t) + 255) & ~(size_t)255;
-    pl->lo_off = mode == CN_GEMM_3XTF32 ? plane : 0;
-    pl->inv_off = plane * (mode == CN_GEMM_3XTF32 ? 2 : 1);
-    pl->bytes = pl->inv_off + (size_t)pl->groups * pl->m_pad * sizeof(float);
+    pl->inv_off = (size_t)TC_BANDS * pl->parts * pl->plane * sizeof(uint16_t);
+    pl->bands_off = pl->inv_off + (size_t)TC_BANDS * pl->groups * pl->m_pad * sizeof(float);
+    pl->bytes = pl->bands_off + (size_t)(pl->m_pad / TC_SUB) * (pl->Kp / TC_AK);
 }
 
+template <bool LO>
 static int act_planes(cn_context *ctx, int transA, int64_t M, int64_t K, const float *A, int64_t lda, const cn_coded_src *cs, const cn_planes &pl,
                       uint8_t *base, cudaStream_t s)
 {
-    uint16_t *hi = reinterpret_cast<uint16_t *>(base), *lo = pl.lo_off ? reinterpret_cast<uint16_t *>(base + pl.lo_off) : nullptr;
-    float *inv = reinterpret_cast<float *>(base + pl.inv_off);
-    CN_REQUIRE(pl.groups * (pl.m_pad / 8) < (1LL << 31), CN_ERR_UNSUPPORTED, "cn_gemm_f32: activation matrix too large for the split pre-pass");
+    const int64_t ctas = pl.groups * (pl.m_pad / ACT_ROWS);
+    CN_REQUIRE(ctas < (1LL << 31), CN_ERR_UNSUPPORTED, "cn_gemm_f32: activation matrix too large for the split pre-pass");
+    const dim3 grid((unsigned)ctas);
+    ActPlanes ap;
+    ap.p = reinterpret_cast<uint16_t *>(base);
+    ap.plane = pl.plane; ap.Kp = pl.Kp; ap.m_pad = pl.m_pad; ap.groups = pl.groups;
+    ap.inv = reinterpret_cast<float *>(base + pl.inv_off);
+    ap.bands = base + pl.bands_off;
+    ap.stages = (int)(pl.Kp / TC_AK);
     if (cs) {
         ActCoded cd;
         cd.codes = cs->codes; cd.scales = cs->scales; cd.tbl = ctx->d_tbl; cd.own_fp32 = cs->own_fp32;
         cd.own_rank = cs->own_rank; cd.nranks = cs->nranks;
-        CN_CUDA(cn_launch_pdl(cn_act_planes_kernel<true>, dim3((unsigned)(pl.groups * (pl.m_pad / ACT_ROWS))), 256, (size_t)cs->nranks * 256 * sizeof(float), s,
-                              A, lda, M, K, pl.Kp, hi, lo, inv, pl.m_pad, cd));
+        CN_CUDA(cn_launch_pdl(cn_act_planes_kernel<LO, true>, grid, 256, (size_t)cs->nranks * 256 * sizeof(float), s, A, lda, M, K, ap, cd));
     } else if (transA) {
         const int vec_ok = ((lda & 3) == 0) && ((reinterpret_cast<uintptr_t>(A) & 15u) == 0);
-        CN_CUDA(cn_launch_pdl(cn_act_planes_t_kernel, dim3((unsigned)(pl.groups * (pl.m_pad / 8))), 256, 0, s, A, lda, M, K, pl.Kp, hi, lo, inv, pl.m_pad,
-                              vec_ok));
+        CN_CUDA(cn_launch_pdl(cn_act_planes_t_kernel<LO>, grid, 32 * ACT_ROWS, 0, s, A, lda, M, K, ap, vec_ok));
     } else {
-        CN_CUDA(cn_launch_pdl(cn_act_planes_kernel<false>, dim3((unsigned)(pl.groups * (pl.m_pad / ACT_ROWS))), 256, 0, s, A, lda, M, K, pl.Kp, hi, lo, inv,
-                              pl.m_pad, ActCoded()));
+        CN_CUDA(cn_launch_pdl(cn_act_planes_kernel<LO, false>, grid, 256, 0, s, A, lda, M, K, ap, ActCoded()));
     }
     cn_count_launch();
     return CN_OK;
+}
+
+static int act_planes(cn_context *ctx, int transA, int64_t M, int64_t K, const float *A, int64_t lda, const cn_coded_src *cs, const cn_planes &pl,
+                      void *planes, cudaStream_t s)
+{
+    return pl.parts == 2 ? act_planes<true>(ctx, transA, M, K, A, lda, cs, pl, (uint8_t *)planes, s)
+                         : act_planes<false>(ctx, transA, M, K, A, lda, cs, pl, (uint8_t *)planes, s);
 }
 
 int cn_gemm_tc_split_activations(cn_context *ctx, int transA, int64_t M, int64_t K, const float *A, int64_t lda, int mode, void *planes, cudaStream_t s)
 {
     cn_planes pl;
     cn_plane_layout(M, K, mode, &pl);
-    return act_planes(ctx, transA, M, K, A, lda, nullptr, pl, (uint8_t *)planes, s);
+    return act_planes(ctx, transA, M, K, A, lda, nullptr, pl, planes, s);
 }
 
 int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, const float *B,
@@ -1264,6 +1585,9 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
     prm.chain_mask = chain - 1;
     prm.a_inv = reinterpret_cast<const float *>(planes + pl.inv_off);
     prm.m_pad = pl.m_pad;
+    prm.groups = (int)pl.groups;
+    prm.a_bands = planes + pl.bands_off;
+    prm.a_stages = (int)(pl.Kp / TC_AK);
     prm.partials = nullptr;
     prm.status = ws->d_status;
     prm.w_ready = ahead ? 0 : 1;
@@ -1285,17 +1609,13 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
 
     // 3. tensor maps
     WMaps mw;
-    CUtensorMap mhi, mlo;
+    CUtensorMap ma;
     const int wk = w_aligned(B, ldb) ? (transB ? W_N : W_K) : (transB ? W_N_ANY : W_K_ANY);
     st = transB ? make_w_maps(enc, &mw, &prm.w_shift, B, N, K, ldb, wk)    // stored N x K, n contiguous
                 : make_w_maps(enc, &mw, &prm.w_shift, B, K, N, ldb, wk);
     if (st != CN_OK) return st;
-    if ((st = make_a_map(enc, &mhi, reinterpret_cast<const uint16_t *>(planes), pl.Kp, M)) != CN_OK) return st;
-    if (mode3x) {
-        if ((st = make_a_map(enc, &mlo, reinterpret_cast<const uint16_t *>(planes + pl.lo_off), pl.Kp, M)) != CN_OK) return st;
-    } else {
-        mlo = mhi;
-    }
+    st = make_a_map(enc, &ma, reinterpret_cast<const uint16_t *>(planes), pl.Kp, M, pl.plane, TC_BANDS * pl.parts);
+    if (st != CN_OK) return st;
 
     cudaEvent_t ev_stop = nullptr;
     if (ws->profile) {
@@ -1310,7 +1630,7 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
         prm.w_ready = 0;   // the event stands between the pre-pass and this launch: keep the plain order
     }
 #define CN_LAUNCH(M3, WKV) \
-    (nt == 1 ? launch_cfg<1, M3, WKV>(mw, mhi, mlo, prm, grid, ctx->device, s) : launch_cfg<2, M3, WKV>(mw, mhi, mlo, prm, grid, ctx->device, s))
+    (nt == 1 ? launch_cfg<1, M3, WKV>(mw, ma, prm, grid, ctx->device, s) : launch_cfg<2, M3, WKV>(mw, ma, prm, grid, ctx->device, s))
     if (wk == W_K_ANY)      st = CN_LAUNCH(true, W_K_ANY);
     else if (wk == W_N_ANY) st = CN_LAUNCH(true, W_N_ANY);
     else if (mode3x)        st = wk == W_N ? CN_LAUNCH(true, W_N) : CN_LAUNCH(true, W_K);

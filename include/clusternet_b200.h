@@ -159,8 +159,12 @@ int cn_arange_f32(cn_context *ctx, float *d_A, int64_t start, int64_t rows, int6
  * (lda = A->rows, ldb = B->rows, ldc = out->rows).
  * ------------------------------------------------------------------------------------------- */
 typedef enum cn_gemm_mode {
-    CN_GEMM_3XTF32 = 0,  /* fp32-accurate: hi/lo split of 11 bits each (TF32's), three tensor-core products per tile */
-    CN_GEMM_TF32 = 1,    /* single TF32 product (10-bit mantissa operands), reported separately */
+    /* fp32-accurate: operands in parts of 11 significand bits (TF32's), three tensor-core products per tile.  Every element keeps at
+     * least 20 bits, whatever stands beside it (activations within 2^97 of the largest of their row and 512 k, weights within 2^115
+     * of theirs); a sum of K products is off by about 2e-6 of its 2-norm.  An operand that is not finite makes the sums it enters
+     * not finite (an infinity may come out as a NaN). */
+    CN_GEMM_3XTF32 = 0,
+    CN_GEMM_TF32 = 1,    /* single product of operands of at least 10 bits over the same ranges, 11 as a rule; reported separately */
     CN_GEMM_FP32_SIMT = 2 /* plain fp32 FMA kernel; also chosen automatically for shapes the tensor path cannot take */
 } cn_gemm_mode;
 

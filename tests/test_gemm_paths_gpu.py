@@ -1,10 +1,10 @@
 """Edges of the product kernels' dispatch: the one-launch kernel for small products (any layout and alignment, K over a
-cluster), the operand scales of the streaming kernel, and its weights of any pitch, against an fp64 product.
+cluster), the operand parts of the streaming kernel, and its weights of any pitch, against an fp64 product.
 
-Bound of an element, with s = sum over k of |a_k b_k|.  3x mode: an operand keeps 22 of its 24 bits (2^-22 of each factor, 2^-22
-more for the product of the low parts), and a chain of 512 k accumulates 3 products per k-step of at least 8, each addition
-truncated to 2^-23 of a running sum that is at most s: 3 * 64 * 2^-23 s = 2.3e-5 s.  Single pass: both operands rounded to 11
-bits, 2^-10 s."""
+Bound of an element, with s = sum over k of |a_k b_k|.  3x mode: what the split leaves out is below 2^-21 of each product, and a
+chain of at most 512 k accumulates at most 12 products per 32 k, each addition truncated to 2^-23 of a running sum that is at most
+s: 192 * 2^-23 s = 2.3e-5 s.  Single pass: both operands rounded to 11 bits, 2^-10 s.  These bounds hold for any signs and are loose
+for random ones, so the streaming kernel is also held to a 2-norm and to sums of a single term."""
 import numpy as np
 import pytest
 import torch
@@ -55,11 +55,64 @@ def test_small_products_in_every_layout(ctx, M, K, N, transA, transB):
             check(C, A, B, transA, transB, rel)
 
 
+@pytest.mark.parametrize("mode", [_lib.GEMM_3XTF32, _lib.GEMM_TF32])
+@pytest.mark.parametrize("transA,transB", [(False, False), (True, False), (False, True)])
+@pytest.mark.parametrize("wide", ["A", "B"])
+@pytest.mark.parametrize("M,K,N,off", [(130, 4100, 1028, 0), (64, 40000, 100, 0), (130, 4100, 1028, 1), (64, 40001, 101, 0)])
+def test_streaming_product_of_single_terms(ctx, M, K, N, off, wide, transA, transB, mode):
+    """One operand has elements over many binades beside each other, the other one nonzero element per row or column, so every output
+    is one product.  3x: 2^-20 for what the parts of each operand may leave, 2^-22 for the product of the low parts, four additions
+    truncated to 2^-23; high parts alone would leave 2^-11.  Single pass: 2^-10 for what is left of the wide operand, 2^-11 for the
+    other one's rounding."""
+    rng = np.random.default_rng(K + N + transB)
+    binades = 45 if wide == "A" else 60                            # activations: 2^97 in all, weights: any
+    A = rng.uniform(1.0, 2.0, (M, K)) * rng.choice([-1.0, 1.0], (M, K))
+    W = rng.uniform(1.0, 2.0, (K, N)) * rng.choice([-1.0, 1.0], (K, N))
+    if wide == "A":
+        at = rng.integers(0, K, N)
+        W *= np.arange(K)[:, None] == at
+        A *= np.exp2(rng.integers(-binades, binades, (M, K)))
+    else:
+        at = rng.integers(0, K, M)
+        A *= np.arange(K) == at[:, None]
+        W *= np.exp2(rng.integers(-binades, binades, (K, N)))
+    A, W = A.astype(np.float32), W.astype(np.float32)
+    n0 = ctx.lib.cn_kernel_launches()
+    C = ctx.gemm(place(np.ascontiguousarray(A.T) if transA else A, 0), place(np.ascontiguousarray(W.T) if transB else W, off), transA=transA,
+                 transB=transB, mode=mode).T.cpu().numpy().astype(np.float64)
+    assert ctx.lib.cn_kernel_launches() - n0 > 1                   # planes and product at least: the streaming kernel
+    ctx.gemm_check()
+    A, W = A.astype(np.float64), W.astype(np.float64)
+    ref = A[:, at] * W[at, np.arange(N)] if wide == "A" else A[np.arange(M), at][:, None] * W[at]
+    bound = 2.7e-6 if mode == _lib.GEMM_3XTF32 or off or (N if transB else K) % 4 else 2.0 ** -10 + 2.0 ** -11 + 2.0 ** -20
+    assert float((np.abs(C - ref) / np.abs(ref)).max()) <= bound
+
+
+@pytest.mark.parametrize("mode,rel", [(_lib.GEMM_3XTF32, 8e-6), (_lib.GEMM_TF32, 1e-3)])
+@pytest.mark.parametrize("transB", [False, True])
+@pytest.mark.parametrize("outlier", [1.0, 2.0 ** 20, 2.0 ** 30, 2.0 ** 40])
+def test_streaming_product_with_large_elements_opposite_zeros(ctx, outlier, transB, mode, rel):
+    """Activations and weights of very different size in one row or column, the large ones opposite zeros: the small ones are the whole
+    result.  2-norm of every row and column; 3x: four times the 1.9e-6 of random operands of one size."""
+    rng = np.random.default_rng(3)
+    M, K, N = 128, 4096, 1024
+    A, W = rng.standard_normal((M, K)), rng.standard_normal((K, N))
+    ka, kw = np.arange(5, K, 64), np.arange(37, K, 64)
+    A[:, ka], W[ka, :] = A[:, ka] * outlier, 0.0
+    W[kw, :], A[:, kw] = W[kw, :] * outlier, 0.0
+    A, W = A.astype(np.float32), W.astype(np.float32)
+    B = np.ascontiguousarray(W.T) if transB else W
+    C = ctx.gemm(place(A, 0), place(B, 0), transB=transB, mode=mode).T.cpu().numpy().astype(np.float64)
+    ctx.gemm_check()
+    ref = A.astype(np.float64) @ W.astype(np.float64)
+    for axis in (0, 1):
+        assert float((np.linalg.norm(C - ref, axis=axis) / np.linalg.norm(ref, axis=axis)).max()) <= rel
+
+
 @pytest.mark.parametrize("transB", [False, True])
 @pytest.mark.parametrize("M,K,N", [(128, 8192, 512), (300, 5000, 2052)])
 def test_streaming_product_of_rows_whose_magnitudes_change(ctx, M, K, N, transB):
-    """Weights that grow along k past fp16's range (the scale is taken anew), start with zeros, or fall; activation rows of very
-    different size.  Every element lies within 2^15 of the largest of its 512-k segment, so no bit may be lost."""
+    """Weights that grow along k, start with zeros, or fall; activation rows of very different size."""
     rng = np.random.default_rng(N)
     A = rng.uniform(0.25, 1.0, (M, K)) * rng.choice([-1.0, 1.0], (M, K)) * np.exp2(rng.integers(-30, 30, (M, 1)))
     W = rng.uniform(0.5, 1.0, (K, N)) * rng.choice([-1.0, 1.0], (K, N))
