@@ -122,8 +122,8 @@ __device__ __forceinline__ uint32_t fast_code4(const float4 q, uint32_t pb, uint
 
 template <bool PRECISION_ON_DEVICE>
 __global__ void __launch_bounds__(CODEC_THREADS, 1)
-cn_compress_kernel(const float *__restrict__ A, float precision_arg, const float *__restrict__ d_precision,
-                   int64_t n, uint8_t *__restrict__ out, const __grid_constant__ CodecConst cc, int vector_ok)
+cn_compress_kernel(const float *A, float precision_arg, const float *d_precision,
+                   int64_t n, uint8_t *out, const __grid_constant__ CodecConst cc, int vector_ok)
 {
     __shared__ CodecTables t;
     const int tid = threadIdx.x;
@@ -488,9 +488,9 @@ enum { RING_SCALE_HOST = 0, RING_SCALE_DEVICE = 1, RING_SCALE_ABSMAX = 2 };
 // so that a tensor that fits the L2 is read from HBM once.  d_precision then receives the scale.
 template <int SCALE>
 __global__ void __launch_bounds__(RING_THREADS, 2)
-cn_compress_ring_kernel(const float *__restrict__ A, float precision_arg, float *__restrict__ d_precision,
-                        int64_t n, uint8_t *__restrict__ out, const __grid_constant__ RingConst rc, unsigned int *status,
-                        int tile_groups, int tiles_per_cta, float *__restrict__ partials, unsigned int *barrier_words,
+cn_compress_ring_kernel(const float *A, float precision_arg, float *d_precision,
+                        int64_t n, uint8_t *out, const __grid_constant__ RingConst rc, unsigned int *status,
+                        int tile_groups, int tiles_per_cta, float *partials, unsigned int *barrier_words,
                         int input_ready_before_predecessor)
 {
     extern __shared__ __align__(128) uint8_t ring_smem[];
@@ -730,8 +730,8 @@ __device__ __forceinline__ bool push_wait_flags(const unsigned int *local_flags,
 }
 
 __global__ void __launch_bounds__(RING_THREADS, 2)
-cn_absmax_compress_push_kernel(const float *__restrict__ A, int64_t n, float *__restrict__ scale_out, uint8_t *__restrict__ out,
-                               const __grid_constant__ RingConst rc, unsigned int *status, float *__restrict__ partials,
+cn_absmax_compress_push_kernel(const float *A, int64_t n, float *scale_out, uint8_t *out,
+                               const __grid_constant__ RingConst rc, unsigned int *status, float *partials,
                                unsigned int *barrier_words, const __grid_constant__ cn_codec_push cp)
 {
     __shared__ RingTables t;
@@ -867,8 +867,8 @@ cn_absmax_compress_push_kernel(const float *__restrict__ A, int64_t n, float *__
 // Used for large tensors (see decompress_impl).
 template <bool PRECISION_ON_DEVICE>
 __global__ void __launch_bounds__(CODEC_THREADS, 1)
-cn_decompress_kernel(const uint8_t *__restrict__ codes, float precision_arg, const float *__restrict__ d_precision,
-                     int64_t n, float *__restrict__ out, const __grid_constant__ DecodeConst dc, int vector_ok)
+cn_decompress_kernel(const uint8_t *codes, float precision_arg, const float *d_precision,
+                     int64_t n, float *out, const __grid_constant__ DecodeConst dc, int vector_ok)
 {
     __shared__ float lut[256];
     const int tid = threadIdx.x;
@@ -933,8 +933,8 @@ cn_decompress_kernel(const uint8_t *__restrict__ codes, float precision_arg, con
 
 template <bool PRECISION_ON_DEVICE>
 __global__ void __launch_bounds__(CODEC_THREADS, 2)
-cn_decompress16_kernel(const uint8_t *__restrict__ codes, float precision_arg, const float *__restrict__ d_precision,
-                       int64_t n, float *__restrict__ out, const __grid_constant__ DecodeConst dc)
+cn_decompress16_kernel(const uint8_t *codes, float precision_arg, const float *d_precision,
+                       int64_t n, float *out, const __grid_constant__ DecodeConst dc)
 {
     __shared__ float lut[256];
     const int tid = threadIdx.x;
@@ -983,8 +983,8 @@ __device__ __forceinline__ float absmax_term(float x) { return ABS ? fabsf(x) : 
 
 template <bool ABS>
 __global__ void __launch_bounds__(ABSMAX_THREADS)
-cn_absmax_kernel(const float *__restrict__ A, int64_t n, float *__restrict__ out, float *__restrict__ partials,
-                 unsigned int *__restrict__ ticket, int vector_ok)
+cn_absmax_kernel(const float *A, int64_t n, float *out, float *partials,
+                 unsigned int *ticket, int vector_ok)
 {
     __shared__ float warp_max[ABSMAX_THREADS / 32];
     __shared__ bool is_last;
@@ -1052,8 +1052,8 @@ cn_absmax_kernel(const float *__restrict__ A, int64_t n, float *__restrict__ out
 // hold in registers - at a few tens of MiB, where every microsecond of ramp shows, this is what keeps HBM busy.
 // Same partial-maximum + last-ticket fold as cn_absmax_kernel; work split as in cn_compress_ring_kernel.
 __global__ void __launch_bounds__(RING_THREADS, 2)
-cn_absmax_ring_kernel(const float *__restrict__ A, int64_t n, float *__restrict__ out, float *__restrict__ partials,
-                      unsigned int *__restrict__ ticket, unsigned int *status, int tile_groups, int tiles_per_cta)
+cn_absmax_ring_kernel(const float *A, int64_t n, float *out, float *partials,
+                      unsigned int *ticket, unsigned int *status, int tile_groups, int tiles_per_cta)
 {
     extern __shared__ __align__(128) uint8_t ring_smem[];
     __shared__ __align__(8) uint64_t bars[2 * RING_STAGES];

@@ -24,6 +24,35 @@ cn_bias_act_kernel(const float *A, const float *bias, int act, float *out, int64
     }
 }
 
+// Any number of rows, an element at a time: with few rows per column the blocks above would be nearly empty (16 x 40000: 34 rounds of
+// blocks with 16 of 256 threads at work).
+template <typename I>
+__global__ void __launch_bounds__(256)
+cn_bias_act_flat_kernel(const float *A, const float *bias, int act, float *out, I rows, I n)
+{
+    cn_pdl_launch_dependents();
+    cn_pdl_wait();
+    const I stride = (I)gridDim.x * 256;
+    for (I i0 = (I)blockIdx.x * 256 + threadIdx.x; i0 < n;) {
+        float v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const I i = i0 + u * stride;
+            if (i < n) {
+                v[u] = A[i];
+                if (bias) v[u] += bias[i / rows];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const I i = i0 + u * stride;
+            if (i < n) out[i] = cn_apply_activation(v[u], act);
+        }
+        if (n - i0 <= 4 * stride) break;   // (the next index may not fit the type)
+        i0 += 4 * stride;
+    }
+}
+
 // One warp per (row, output column).  The reference reduces 32 shared-memory slots (slot t = column
 // g*L + t for t < L, -FLT_MAX with index -1 otherwise) with a fixed tree: at offsets 16, 8, 4, 2, 1 slot t
 // takes slot t+offset when its own value is strictly smaller (reduceToMaxAndArgMax,
@@ -64,8 +93,16 @@ extern "C" int cn_bias_activation(cn_context *ctx, const float *d_A, const float
     if (n == 0) return CN_OK;
     CN_REQUIRE(d_A && d_out, CN_ERR_ARG, "cn_bias_activation: null buffer");
     CN_REQUIRE(activation >= CN_ACT_LINEAR && activation <= CN_ACT_DOUBLE_RELU, CN_ERR_ARG, "cn_bias_activation: unknown activation %d", activation);
-    const int64_t row_blocks = (rows + 1023) / 1024;
-    int64_t blocks = row_blocks * cols, cap = (int64_t)ctx->sm_count * 8;
+    const int64_t row_blocks = (rows + 1023) / 1024, cap = (int64_t)ctx->sm_count * 8;
+    if (rows < 1024) {
+        const int64_t want = (n + 1023) / 1024;
+        const dim3 grid((unsigned)(want < cap ? want : cap));
+        if (n < (1LL << 31)) CN_CUDA(cn_launch_pdl(cn_bias_act_flat_kernel<uint32_t>, grid, 256, 0, cn_stream(stream), d_A, d_bias, activation, d_out, (uint32_t)rows, (uint32_t)n));
+        else CN_CUDA(cn_launch_pdl(cn_bias_act_flat_kernel<int64_t>, grid, 256, 0, cn_stream(stream), d_A, d_bias, activation, d_out, rows, n));
+        cn_count_launch();
+        return CN_OK;
+    }
+    int64_t blocks = row_blocks * cols;
     CN_CUDA(cn_launch_pdl(cn_bias_act_kernel, dim3((unsigned)(blocks < cap ? blocks : cap)), 256, 0, cn_stream(stream), d_A, d_bias, activation, d_out,
                           rows, cols, row_blocks));
     cn_count_launch();

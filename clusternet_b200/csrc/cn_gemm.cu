@@ -205,7 +205,7 @@ int cn_gemm_dispatch(cn_context *ctx, int transA, int transB, int64_t M, int64_t
     const bool tuned = ws && (ws->force_nt || ws->force_splits || ws->force_chain);
     const cn_prepared *pr = ws ? ws->prepared : nullptr;
     const bool small = mode != CN_GEMM_FP32_SIMT && (L == 1 || ldc == M) && !tuned && !(ws && (ws->coded_src || ws->profile)) && (!pr || pr->raw) &&
-                       cn_gemm_small_shape(ctx, M, N, K) && (tma_ok || M * N * K >= 4096);
+                       cn_gemm_small_shape(ctx, M, N, K, tma_ok) && (tma_ok || M * N * K >= 4096);
     // Weights that TMA cannot read as they are keep fp32-level accuracy in every mode: the fp32 kernel took them before.
     const int tc_mode = tma_ok ? mode : CN_GEMM_3XTF32;
     const bool tc_ok = tma_ok || (mode != CN_GEMM_FP32_SIMT && M * N * K >= 4096 && cn_gemm_tc_any_supported(transB, M, N, K, d_B));
@@ -231,7 +231,8 @@ int cn_gemm_dispatch(cn_context *ctx, int transA, int transB, int64_t M, int64_t
             transA = 1;
         }
         const bool push = peers && peers->npeers > 0 && L == 1;
-        st = cn_gemm_small_launch(ctx, transA, transB, M, N, K, d_A, lda, d_B, ldb, target, target_ld, epi, tc_mode, s, push ? peers : nullptr);
+        st = cn_gemm_small_launch(ctx, transA, transB, M, N, K, d_A, lda, d_B, ldb, target, target_ld, epi, tc_mode, s, push ? peers : nullptr,
+                                  tma_ok);
         if (push && used_peers) *used_peers = st == CN_OK;
     } else if (tc_ok) {
         cn_epilogue e2;

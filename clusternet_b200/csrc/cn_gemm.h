@@ -91,10 +91,12 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
                       const float *B, int64_t ldb, float *C, int64_t ldc, const cn_epilogue *epi, int mode, cudaStream_t s,
                       const cn_peer_out *peers = nullptr, int transA = 0, int transB = 0);
 // Small products in one launch (cn_gemm_small.cu): whether a shape is one, and the launch.  Takes any layout and alignment.
-bool cn_gemm_small_shape(const cn_context *ctx, int64_t M, int64_t N, int64_t K);
-#define CN_SMALL_MAX_K 16384   // no shape with a longer inner dimension is small
+bool cn_gemm_small_shape(const cn_context *ctx, int64_t M, int64_t N, int64_t K, bool w_aligned);
+#define CN_SMALL_MAX_K 3072   // no product of aligned weights with a longer inner dimension is small: eight CTAs of twelve blocks of 32
+// K blocks of 32 per accumulation chain for weights whose rows TMA cannot read (cn_gemm_tc.cu)
+int cn_gemm_any_chain(int64_t K);
 int cn_gemm_small_launch(cn_context *ctx, int transA, int transB, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, const float *B, int64_t ldb,
-                         float *C, int64_t ldc, const cn_epilogue *epi, int mode, cudaStream_t s, const cn_peer_out *peers);
+                         float *C, int64_t ldc, const cn_epilogue *epi, int mode, cudaStream_t s, const cn_peer_out *peers, bool w_aligned);
 // cn_gemm_f32 with optional peer windows; *used_peers tells whether the launch took them (tensor-core path only).
 int cn_gemm_dispatch(cn_context *ctx, int transA, int transB, int64_t M, int64_t N, int64_t K, const float *d_A, int64_t lda,
                      const float *d_B, int64_t ldb, float *d_C, int64_t ldc, const cn_epilogue *epi, int mode, void *stream,

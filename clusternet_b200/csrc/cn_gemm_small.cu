@@ -12,8 +12,8 @@
 //   * the CTAs of a cluster share a tile: each multiplies its part of K, sends every other CTA its slice of the partial tile
 //     through distributed shared memory, adds the slices it received in K order (reproducible), and finishes its slice: bias,
 //     activation, 512-byte runs of stores to C and, for the fused all-gather, to the peers.
-// The tensor core's accumulator truncates, so a share of K is cut into as many chains as tensor memory holds accumulators for (four,
-// of at most SM_CHAIN_KB blocks) and the chains are added in round-to-nearest fp32.
+// The tensor core's accumulator truncates, so a share of K (at most SM_MAX_BLOCKS_ANY blocks) is cut into as many chains as tensor memory
+// holds accumulators for, four, and the chains are added in round-to-nearest fp32.
 //
 // Bound by latency.  128 x 784 . 784 x 1024 + bias + ReLU: 13.2 us a call, against 22.5 us in three launches.
 #include "cn_epilogue.cuh"
@@ -27,7 +27,8 @@
 #define SM_STAGES 2
 #define SM_TILE_BYTES (128 * 128)
 #define SM_STAGE_BYTES (4 * SM_TILE_BYTES)   // W hi, W lo, A hi, A lo
-#define SM_CHAIN_KB 16
+#define SM_MAX_BLOCKS 12
+#define SM_MAX_BLOCKS_ANY 16   // weights that TMA cannot read, of which the streaming kernel wants four rows at least
 #define SM_MAX_CHAINS 4
 #define SM_MAX_CLUSTER 8
 #define SM_RING_BYTES (SM_STAGES * SM_STAGE_BYTES)
@@ -48,6 +49,7 @@ struct SmallParams {
     int tiles_m;
     int cluster;
     int kb_total;
+    int fine_chains;      // chains end between k-steps of 8, not blocks (see cn_gemm_small_launch)
     unsigned int *status;
     int npeers;
     float *peerC[CN_MAX_PEERS];
@@ -57,11 +59,13 @@ struct SmallParams {
     unsigned int epoch;
 };
 
-// fp32 -> TF32, round to nearest with ties away from zero: add half a TF32 ulp to the magnitude bits and truncate.  That carry would
-// take the finite values from 0x7f7ff000 up to infinity and a NaN with a full mantissa (0x7fffffff, the one GPU arithmetic makes)
-// over into the sign bit, to -0: those are truncated instead, NaNs after an addition that makes them the canonical one.
+// fp32 -> TF32, round to nearest with ties away from zero: add half a TF32 ulp to the magnitude bits and truncate.  That carry takes
+// the finite values from 0x7f7ff000 up to infinity and a NaN with a full mantissa (0x7fffffff, the one GPU arithmetic makes)
+// over into the sign bit, to -0.  CAREFUL truncates those instead, NaNs after an addition that makes them the canonical one.
+template <bool CAREFUL>
 __device__ __forceinline__ uint32_t sm_tf32(float x)
 {
+    if (!CAREFUL) return (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
     const float top = __uint_as_float(0x7f7ff000u);
     return (fabsf(x) < top ? __float_as_uint(x) + 0x1000u : __float_as_uint(__fadd_rn(x, 0.0f))) & 0xffffe000u;
 }
@@ -121,8 +125,17 @@ __device__ __forceinline__ void sm_load(const float *base, int64_t ld, int rows,
     }
 }
 
+// Whether sm_tf32 has to be CAREFUL with some of the values.
+__device__ __forceinline__ bool sm_unsafe(const float (&x)[32])
+{
+    float m = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 32; i += 2) asm("max.NaN.abs.f32 %0, %1, %2, %0;" : "+f"(m) : "f"(x[i]), "f"(x[i + 1]));
+    return !(m < __uint_as_float(0x7f7ff000u));
+}
+
 // The same block -> TF32 parts in shared memory: 16-byte chunk c of row r lies at r * 128 + ((c ^ (r & 7)) << 4).
-template <int KIND, bool MODE3X>
+template <int KIND, bool MODE3X, bool CAREFUL>
 __device__ __forceinline__ void sm_store(uint32_t hi, uint32_t lo, int need_rows, int t, const float (&x)[32])
 {
     if (KIND == SM_K_SCALAR) {
@@ -131,9 +144,9 @@ __device__ __forceinline__ void sm_store(uint32_t hi, uint32_t lo, int need_rows
             const int r = i * 4 + (t >> 5), kk = t & 31;
             if (r >= need_rows) continue;
             const uint32_t at = (uint32_t)(r * 128 + (((kk >> 2) ^ (r & 7)) << 4) + (kk & 3) * 4);
-            const uint32_t h = sm_tf32(x[i]);
+            const uint32_t h = sm_tf32<CAREFUL>(x[i]);
             sts1u(hi + at, h);
-            if (MODE3X) sts1u(lo + at, sm_tf32(x[i] - __uint_as_float(h)));
+            if (MODE3X) sts1u(lo + at, sm_tf32<CAREFUL>(x[i] - __uint_as_float(h)));
         }
     } else {
 #pragma unroll
@@ -143,11 +156,11 @@ __device__ __forceinline__ void sm_store(uint32_t hi, uint32_t lo, int need_rows
             const uint32_t at = (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4));
             uint32_t h[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) h[e] = sm_tf32(x[4 * i + e]);
+            for (int e = 0; e < 4; ++e) h[e] = sm_tf32<CAREFUL>(x[4 * i + e]);
             sts4u(hi + at, h[0], h[1], h[2], h[3]);
             if (MODE3X)
-                sts4u(lo + at, sm_tf32(x[4 * i] - __uint_as_float(h[0])), sm_tf32(x[4 * i + 1] - __uint_as_float(h[1])),
-                      sm_tf32(x[4 * i + 2] - __uint_as_float(h[2])), sm_tf32(x[4 * i + 3] - __uint_as_float(h[3])));
+                sts4u(lo + at, sm_tf32<CAREFUL>(x[4 * i] - __uint_as_float(h[0])), sm_tf32<CAREFUL>(x[4 * i + 1] - __uint_as_float(h[1])),
+                      sm_tf32<CAREFUL>(x[4 * i + 2] - __uint_as_float(h[2])), sm_tf32<CAREFUL>(x[4 * i + 3] - __uint_as_float(h[3])));
         }
     }
 }
@@ -170,10 +183,12 @@ __device__ __forceinline__ bool sm_feed(const float *base, int64_t ld, int rows,
             const int i = i0 + u;
             if (i >= n || !ok) continue;
             if (i + 1 < n) sm_load<KIND>(base, ld, rows, (int64_t)(kb0 + i + 1) * SM_BK, K, t, x[u ^ 1]);
+            const bool unsafe = sm_unsafe(x[u]);
             ok = mbar_wait(empty0 + 8 * u, ((uint32_t)(i >> 1) & 1u) ^ 1u, abort_flag, status, 14u);
             if (!ok) continue;
             const uint32_t hi = ring + u * SM_STAGE_BYTES + operand_off;
-            sm_store<KIND, MODE3X>(hi, hi + SM_TILE_BYTES, need_rows, t, x[u]);
+            if (unsafe) sm_store<KIND, MODE3X, true>(hi, hi + SM_TILE_BYTES, need_rows, t, x[u]);
+            else        sm_store<KIND, MODE3X, false>(hi, hi + SM_TILE_BYTES, need_rows, t, x[u]);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
             if ((t & 31) == 0) mbar_arrive(full0 + 8 * u);
@@ -199,7 +214,10 @@ cn_gemm_small_kernel(const __grid_constant__ SmallParams p)
     const int m_rows = (int)(p.M - m0 < SM_BM ? p.M - m0 : SM_BM), n_rows = (int)(p.N - n0 < SM_BN ? p.N - n0 : SM_BN);
     const int m_need = (m_rows + 15) & ~15;   // UMMA N
     const int kb0 = (int)((int64_t)p.kb_total * rank / p.cluster), kb1 = (int)((int64_t)p.kb_total * (rank + 1) / p.cluster);
-    const int chain_kb = (kb1 - kb0 + SM_MAX_CHAINS - 1) / SM_MAX_CHAINS, chains = (kb1 - kb0 + chain_kb - 1) / chain_kb;
+    // accumulation chains, in k-steps of 8
+    const int steps = (kb1 - kb0) * (SM_BK / 8);
+    const int chain_steps = p.fine_chains ? (steps + SM_MAX_CHAINS - 1) / SM_MAX_CHAINS : (kb1 - kb0 + SM_MAX_CHAINS - 1) / SM_MAX_CHAINS * (SM_BK / 8);
+    const int chains = (steps + chain_steps - 1) / chain_steps;
     cn_pdl_launch_dependents();
     if (p.cluster > 1) cluster_arrive();   // every CTA of the cluster has started: waited for before the first remote store
     if (threadIdx.x == 0) {
@@ -237,9 +255,9 @@ cn_gemm_small_kernel(const __grid_constant__ SmallParams p)
         const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(m_need >> 3) << 17) | ((uint32_t)(SM_BN >> 4) << 24);
         const int n = kb1 - kb0;
         uint32_t acc = tmem;
-        for (int i = 0, in_chain = 0; i < n; ++i, ++in_chain) {
+        int in_chain = 0;
+        for (int i = 0; i < n; ++i) {
             const int s = i & 1;
-            if (in_chain == chain_kb) { in_chain = 0; acc += SM_BM; }
             ok = mbar_wait(full0 + 8 * s, (uint32_t)(i >> 1) & 1u, abort_flag, p.status, 15u);
             if (!ok) break;
             tc_fence_after();
@@ -248,7 +266,8 @@ cn_gemm_small_kernel(const __grid_constant__ SmallParams p)
                            alo = ahi + (SM_TILE_BYTES >> 4);
 #pragma unroll
             for (int j = 0; j < SM_BK / 8; ++j) {   // 8 TF32 per k-step: 32 bytes (descriptor units of 16 B)
-                sm_mma_ss(acc, whi + 2 * j, ahi + 2 * j, hi, idesc, (in_chain != 0 || j > 0) ? 1u : 0u);
+                if (in_chain == chain_steps) { in_chain = 0; acc += SM_BM; }
+                sm_mma_ss(acc, whi + 2 * j, ahi + 2 * j, hi, idesc, in_chain++ != 0 ? 1u : 0u);
                 if (MODE3X) {
                     sm_mma_ss(acc, wlo + 2 * j, ahi + 2 * j, hi, idesc, 1u);
                     sm_mma_ss(acc, whi + 2 * j, alo + 2 * j, hi, idesc, 1u);
@@ -356,7 +375,7 @@ static int small_cluster(int64_t tiles, int kb, int sms)
     return c;
 }
 
-bool cn_gemm_small_shape(const cn_context *ctx, int64_t M, int64_t N, int64_t K)
+bool cn_gemm_small_shape(const cn_context *ctx, int64_t M, int64_t N, int64_t K, bool w_aligned)
 {
     if (M < 1 || N < 1 || K < 1) return false;
     if (N > (1 << 21) / K) return false;   // at most 8 MB of weights
@@ -366,7 +385,12 @@ bool cn_gemm_small_shape(const cn_context *ctx, int64_t M, int64_t N, int64_t K)
     const int64_t per_cta = (kb + c - 1) / c, rounds = (tiles * c + ctx->sm_count - 1) / ctx->sm_count;
     // more than two rounds of CTAs cost more than the streaming kernel's three launches: the 4096 x 4096 weight gradient of a batch of
     // 128 (1024 tiles, seven rounds) took 108 us here; the whole backward pass went from 210 to 162 us
-    return per_cta <= SM_CHAIN_KB * SM_MAX_CHAINS && rounds <= 2;
+    // a block costs a CTA 1.5 us, the streaming kernel's launches and reduction 15 to 20: 16 x 8000 . 8000 x 64 (32 blocks) took 43 us here
+    if (per_cta > (w_aligned ? SM_MAX_BLOCKS : SM_MAX_BLOCKS_ANY) || rounds > 2) return false;
+    // weights that TMA cannot read must not become less exact than on the fp32 kernel (cn_gemm_any_chain); a TF32 block has twice the
+    // additions of an fp16 one
+    const int chain = cn_gemm_any_chain(K) / 2;
+    return w_aligned || (per_cta + SM_MAX_CHAINS - 1) / SM_MAX_CHAINS <= (chain > 1 ? chain : 1);
 }
 
 template <int WKIND, int AKIND, bool MODE3X>
@@ -410,7 +434,7 @@ static int small_pick(cn_context *ctx, const SmallParams &p, int wk, int ak, int
 }
 
 int cn_gemm_small_launch(cn_context *ctx, int transA, int transB, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, const float *B, int64_t ldb,
-                         float *C, int64_t ldc, const cn_epilogue *epi, int mode, cudaStream_t s, const cn_peer_out *peers)
+                         float *C, int64_t ldc, const cn_epilogue *epi, int mode, cudaStream_t s, const cn_peer_out *peers, bool w_aligned)
 {
     SmallParams p;
     unsigned int *d_status = nullptr;
@@ -425,6 +449,7 @@ int cn_gemm_small_launch(cn_context *ctx, int transA, int transB, int64_t M, int
     const int64_t tiles = (int64_t)p.tiles_m * ((N + SM_BN - 1) / SM_BN);
     p.kb_total = (int)((K + SM_BK - 1) / SM_BK);
     p.cluster = small_cluster(tiles, p.kb_total, ctx->sm_count);
+    p.fine_chains = !w_aligned;
     p.status = d_status;
     p.npeers = 0;
     p.ready = nullptr; p.peer_flags = nullptr;

@@ -1207,6 +1207,7 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
                     }
                 }
             }
+            __syncwarp();   // as above
         }
     }
 
@@ -1219,7 +1220,7 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
 }
 
 // ------------------------------------------------------------------------------------------ reduction of the runs
-// One CTA per 32 columns of one W tile: adds the partial tiles of all runs in K order (a fixed order, so the result does not
+// One CTA per COLS columns of one W tile: adds the partial tiles of all runs in K order (a fixed order, so the result does not
 // depend on scheduling), applies bias and activation, turns the block through shared memory so that a warp stores 512
 // contiguous bytes of a column, and stores to C and, for the fused all-gather, to every peer's C (full NVLink packets).
 struct ReduceParams {
@@ -1240,10 +1241,15 @@ struct ReduceParams {
     unsigned int *status;
 };
 
+//
+// 32 columns where there are tiles for every SM.  Few tiles are cut into many runs, and what bounds them is how many loads a CTA has in
+// flight: 8 columns, eight partial tiles at a time (16 x 40000 . 40000 x 201, 148 runs: FIXME us with 32 columns, FIXME with 8).
+template <int COLS>
 __global__ void __launch_bounds__(256)
 cn_splitk_reduce_kernel(const __grid_constant__ ReduceParams p)
 {
-    __shared__ float turn[32][TC_BM + 4];
+    constexpr int QSTEP = 256 / COLS, QUADS = 32 / QSTEP, UNROLL = 8 / QUADS;   // quads of m per thread; partial tiles in flight
+    __shared__ float turn[COLS][TC_BM + 4];
     cn_pdl_launch_dependents();
     cn_pdl_wait();
     if (p.npeers > 0) {   // peers must have announced that their copy of C may be overwritten (bounded wait)
@@ -1260,9 +1266,9 @@ cn_splitk_reduce_kernel(const __grid_constant__ ReduceParams p)
         }
         __syncthreads();
     }
-    const int chunk = blockIdx.x & 3;
-    const int tw = blockIdx.x >> 2, r = tw / p.nt, w = tw - r * p.nt, tile = p.full_tiles + r;
-    const int64_t m0 = (int64_t)(tile % p.tiles_m) * TC_BM, n0 = ((int64_t)(tile / p.tiles_m) * p.nt + w) * TC_BN + chunk * 32;
+    const int chunk = blockIdx.x % (TC_BN / COLS);
+    const int tw = blockIdx.x / (TC_BN / COLS), r = tw / p.nt, w = tw - r * p.nt, tile = p.full_tiles + r;
+    const int64_t m0 = (int64_t)(tile % p.tiles_m) * TC_BM, n0 = ((int64_t)(tile / p.tiles_m) * p.nt + w) * TC_BN + chunk * COLS;
     if (n0 >= p.N) return;
     // the CTAs whose runs hold K blocks of this tile: run c is [total c / ctas, total (c + 1) / ctas)
     const int64_t total = (int64_t)p.tail_tiles * p.kb_total, first = (int64_t)r * p.kb_total, last = first + p.kb_total - 1;
@@ -1273,41 +1279,41 @@ cn_splitk_reduce_kernel(const __grid_constant__ ReduceParams p)
         return c;
     };
     const int64_t c0 = owner(first), c1 = owner(last);
-    const int row = threadIdx.x & 31, quad = threadIdx.x >> 5;   // column of the chunk; quads of m: quad + 8 j
+    const int row = threadIdx.x % COLS, quad = threadIdx.x / COLS;   // column of the chunk; quads of m: quad + QSTEP j
     constexpr int64_t TILE4 = TC_BM * TC_BN / 4;
-    const float4 *src = reinterpret_cast<const float4 *>(p.partials) + ((c0 + r) * p.nt + w) * TILE4 + quad * TC_BN + chunk * 32 + row;
+    const float4 *src = reinterpret_cast<const float4 *>(p.partials) + ((c0 + r) * p.nt + w) * TILE4 + quad * TC_BN + chunk * COLS + row;
     const int64_t step = p.nt * TILE4;
-    float4 acc[4];
+    float4 acc[QUADS];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j = 0; j < QUADS; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
     int64_t left = c1 - c0 + 1;
-    // two partial tiles in flight at a time; the additions stay in K order, so the sum does not depend on the grouping
-    for (; left >= 2; left -= 2, src += 2 * step) {
-        float4 v[2][4];
+    // the additions stay in K order, so the sum does not depend on the grouping
+    for (; left >= UNROLL; left -= UNROLL, src += UNROLL * step) {
+        float4 v[UNROLL][QUADS];
 #pragma unroll
-        for (int u = 0; u < 2; ++u)
+        for (int u = 0; u < UNROLL; ++u)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) v[u][j] = __ldcs(src + u * step + j * 8 * TC_BN);
+            for (int j = 0; j < QUADS; ++j) v[u][j] = __ldcs(src + u * step + j * QSTEP * TC_BN);
 #pragma unroll
-        for (int u = 0; u < 2; ++u)
+        for (int u = 0; u < UNROLL; ++u)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) { acc[j].x += v[u][j].x; acc[j].y += v[u][j].y; acc[j].z += v[u][j].z; acc[j].w += v[u][j].w; }
+            for (int j = 0; j < QUADS; ++j) { acc[j].x += v[u][j].x; acc[j].y += v[u][j].y; acc[j].z += v[u][j].z; acc[j].w += v[u][j].w; }
     }
-    if (left > 0) {
+    for (; left > 0; --left, src += step) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float4 v = __ldcs(src + j * 8 * TC_BN);
+        for (int j = 0; j < QUADS; ++j) {
+            const float4 v = __ldcs(src + j * QSTEP * TC_BN);
             acc[j].x += v.x; acc[j].y += v.y; acc[j].z += v.z; acc[j].w += v.w;
         }
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) *reinterpret_cast<float4 *>(&turn[row][(quad + 8 * j) * 4]) = acc[j];
+    for (int j = 0; j < QUADS; ++j) *reinterpret_cast<float4 *>(&turn[row][(quad + QSTEP * j) * 4]) = acc[j];
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const int64_t m = m0 + lane * 4;
     const bool vec = (m + 4 <= p.M) && ((p.ldc & 3) == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15u) == 0);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < COLS / 8; ++j) {
         const int nl = (threadIdx.x >> 5) + 8 * j;
         const int64_t n = n0 + nl;
         if (n >= p.N || m >= p.M) continue;
@@ -1430,7 +1436,7 @@ bool cn_gemm_tc_supported(cn_context *, int transA, int transB, int64_t M, int64
 // the square root of K: relative to an fp64 product (uniform operands) 2.1e-7 at K = 130, 5.0e-7 at 785, 1.13e-6 at 4001, 3.6e-6 at
 // 39999.  Here it grows with the chain: 2.1e-7 with one block, 3.2e-7 with 2, 5.2e-7 with 4, 9.0e-7 with 8, 1.8e-6 with 16.  The
 // longest chain that is no less exact than the fp32 kernel was:
-static int any_chain(int64_t K) { return K < 384 ? 1 : K < 1024 ? 2 : K < 3072 ? 4 : K < 12288 ? 8 : TC_GROUP_KB; }
+int cn_gemm_any_chain(int64_t K) { return K < 384 ? 1 : K < 1024 ? 2 : K < 3072 ? 4 : K < 12288 ? 8 : TC_GROUP_KB; }
 
 template <int NT, bool MODE3X, int WK>
 static int launch_cfg(const WMaps &mw, const CUtensorMap &ma, const TcParams &prm, int64_t grid, int dev, cudaStream_t s)
@@ -1579,7 +1585,7 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
     prm.argmax = epi ? epi->argmax_out : nullptr;
     prm.tiles_n = (int)tiles_n; prm.tiles_m = (int)tiles_m;
     prm.full_tiles = (int)full; prm.tail_ctas = (int)tail_ctas; prm.kb_total = kb_total;
-    int chain = w_aligned(B, ldb) ? TC_GROUP_KB : any_chain(K);
+    int chain = w_aligned(B, ldb) ? TC_GROUP_KB : cn_gemm_any_chain(K);
     if (ws->force_chain >= 1)
         while (chain > 1 && chain > ws->force_chain) chain >>= 1;
     prm.chain_mask = chain - 1;
@@ -1646,7 +1652,8 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
         for (int i = 0; i < CN_MAX_PEERS; ++i) rp.peerC[i] = prm.npeers > i ? peers->C[i] : nullptr;
         rp.ready = prm.npeers > 0 ? peers->ready : nullptr;
         rp.nranks = prm.nranks; rp.my_rank = prm.my_rank; rp.epoch = prm.epoch; rp.status = prm.status;
-        CN_CUDA(cn_launch_pdl(cn_splitk_reduce_kernel, dim3((unsigned)(rest * nt * 4)), 256, 0, s, rp));
+        if (rest * nt * 4 <= sms) CN_CUDA(cn_launch_pdl(cn_splitk_reduce_kernel<8>, dim3((unsigned)(rest * nt * (TC_BN / 8))), 256, 0, s, rp));
+        else CN_CUDA(cn_launch_pdl(cn_splitk_reduce_kernel<32>, dim3((unsigned)(rest * nt * (TC_BN / 32))), 256, 0, s, rp));
         cn_count_launch();
     }
     if (ev_stop) CN_CUDA(cudaEventRecord(ev_stop, s));

@@ -86,8 +86,11 @@ static inline cudaStream_t cn_stream(void *s) { return reinterpret_cast<cudaStre
 #ifdef __CUDACC__
 // Programmatic dependent launch.  A kernel launched with cn_launch_pdl may become resident while its predecessor in the
 // stream still runs; it calls cn_pdl_launch_dependents() ("my successor may start too") and, before its first access to
-// global memory, cn_pdl_wait() ("my predecessor has finished and its writes are visible").  Every thread of every such kernel
-// waits, so that a kernel's end implies the end of everything before it.  Launch latency and CTA start-up then overlap the
+// global memory, cn_pdl_wait() ("my predecessor has finished and its writes are visible").  Some thread of every such kernel
+// waits before the kernel can end (in cn_gemm_tc_kernel the activations' producer and the drain warps; its producer of weights may
+// start on what was written before the pre-pass), so that a kernel's end implies the end of everything before it.  Inputs that
+// the predecessor may still be writing while such a kernel runs are no __restrict__ const pointers: those are read through a path
+// that is not coherent with writes during the kernel.  Launch latency and CTA start-up then overlap the
 // predecessor's tail: about 1 us per launch in a chain of small kernels.
 __device__ __forceinline__ void cn_pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void cn_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -222,9 +222,9 @@ struct SegParams {
 // Four elements per thread where the buffers allow 16-byte accesses (vec_ok) and the four lie in one segment.
 template <bool UPDATE>
 __global__ void __launch_bounds__(512)
-cn_decode_sum_multi_kernel(float *__restrict__ grad, const uint8_t *__restrict__ blocks, size_t block_bytes, size_t scales_off,
-                           const float *__restrict__ g_tbl, int64_t n, int nranks, int my_rank, const SegParams sp,
-                           float *__restrict__ RMS, float *__restrict__ w, float rms_mult, float lr, int vec_ok)
+cn_decode_sum_multi_kernel(float *grad, const uint8_t *blocks, size_t block_bytes, size_t scales_off,
+                           const float *g_tbl, int64_t n, int nranks, int my_rank, const SegParams sp,
+                           float *RMS, float *w, float rms_mult, float lr, int vec_ok)
 {
     extern __shared__ float lut[];   // (segment, rank) x 256
     cn_pdl_launch_dependents();

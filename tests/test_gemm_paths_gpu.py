@@ -173,7 +173,7 @@ def test_small_products_keep_non_finite_and_the_largest_finite_values(ctx, trans
         assert np.allclose(C[100][rest[100]], a[100, 3].astype(np.float64) * 0.25, rtol=REL_1X)
 
 
-@pytest.mark.parametrize("M,K,N", [(203, 4001, 3001), (5, 2049, 1031), (128, 20003, 131), (300, 130, 20005), (128, 4002, 1026), (64, 5, 500001)])
+@pytest.mark.parametrize("M,K,N", [(203, 4001, 3001), (5, 2049, 1031), (128, 20003, 131), (300, 130, 20005), (128, 4002, 1026), (64, 5, 500001), (70, 40001, 101)])
 @pytest.mark.parametrize("transB", [False, True])
 @pytest.mark.parametrize("off", [0, 1, 2, 3])
 def test_streaming_weights_of_any_pitch_and_alignment(ctx, M, K, N, transB, off):
@@ -198,6 +198,77 @@ def test_streaming_weights_of_any_pitch_and_alignment(ctx, M, K, N, transB, off)
     C1 = ctx.gemm(A, W, transB=transB, bias=bias, activation=_lib.ACT_RELU, mode=_lib.GEMM_TF32)
     if off or inner % 4:
         assert torch.equal(C1, C)
+
+
+@pytest.mark.parametrize("M,K,N", [(128, 257, 201), (128, 785, 1201), (203, 2001, 301), (500, 2001, 999), (1280, 2047, 1023), (70, 40001, 101)])
+@pytest.mark.parametrize("transB", [False, True])
+def test_weights_of_odd_pitch_are_as_exact_as_on_the_fp32_kernel(ctx, M, K, N, transB):
+    """2-norm against fp64, small and streaming kernel, beside the fp32 kernel's on the same operands, whose own error scatters by some
+    per cent of it and by the last bit of the result (6e-8)."""
+    rng = np.random.default_rng(M + K + N)
+    A, W = rng.uniform(-1, 1, (M, K)).astype(np.float32), rng.uniform(-1, 1, (K, N)).astype(np.float32)
+    dA, dW = place(A, 0), place(np.ascontiguousarray(W.T) if transB else W, 1)
+    ref = A.astype(np.float64) @ W.astype(np.float64)
+    err = [np.linalg.norm(ctx.gemm(dA, dW, transB=transB, mode=m).T.cpu().numpy() - ref) / np.linalg.norm(ref)
+           for m in (_lib.GEMM_3XTF32, _lib.GEMM_FP32_SIMT)]
+    ctx.gemm_check()
+    assert err[0] <= 1.1 * err[1] + 6e-8, err
+
+
+@pytest.mark.parametrize("level", [2, 8, 32])
+@pytest.mark.parametrize("M,K,N,full", [(128, 320, 40960, True), (130, 4100, 1024, False)])
+def test_maxout_fused_into_the_streaming_kernel(ctx, level, M, K, N, full):
+    """The shuffle tree over the drain warps' sums: two tiles per CTA, a ragged second tile of rows, bias.  Where the product without
+    maxout is not cut along K either (full), its maxima exactly."""
+    rng = np.random.default_rng(level + N)
+    A, B = rng.uniform(-1, 1, (M, K)).astype(np.float32), rng.uniform(-1, 1, (K, N)).astype(np.float32)
+    dA, dB, db = ctx.colmajor(A), ctx.colmajor(B), torch.from_numpy(rng.uniform(-1, 1, N).astype(np.float32)).cuda()
+    arg = ctx.empty(M, N // level)
+    n0 = ctx.lib.cn_kernel_launches()
+    out = ctx.gemm(dA, dB, bias=db, maxout_level=level, argmax_out=arg)
+    assert ctx.lib.cn_kernel_launches() - n0 == 2                  # planes and product: no separate reduction
+    out = ctx.to_numpy(out)
+    plain = ctx.to_numpy(ctx.gemm(dA, dB, bias=db))
+    ctx.gemm_check()
+    wv, wi = oracle.maxout(plain, level)
+    if full:
+        assert np.array_equal(out, wv) and np.array_equal(ctx.to_numpy(arg), wi)
+    else:
+        got = ctx.to_numpy(arg).astype(np.int64)
+        assert np.array_equal(got // level, np.broadcast_to(np.arange(N // level), got.shape))
+        bound = REL_3X * (np.abs(A) @ np.abs(B)).max()
+        assert np.abs(out - wv).max() <= bound
+        assert np.abs(np.take_along_axis(plain, got, 1) - out).max() <= bound
+
+
+@pytest.mark.parametrize("M,K,N", [(5, 20000, 70), (128, 8000, 300), (260, 12000, 130)])
+@pytest.mark.parametrize("nt", [1, 2])
+def test_few_tiles_in_many_runs(ctx, M, K, N, nt):
+    """The reduction with eight columns per CTA: remainders of rows, columns and partial tiles; bit for bit the same twice."""
+    from clusternet_b200 import check as status
+    rng = np.random.default_rng(M + N)
+    A, B = rng.uniform(-1, 1, (M, K)).astype(np.float32), rng.uniform(-1, 1, (K, N)).astype(np.float32)
+    bias = torch.from_numpy(rng.uniform(-1, 1, N).astype(np.float32)).cuda()
+    dA, dB = ctx.colmajor(A), ctx.colmajor(B)
+    status(ctx.lib.cn_gemm_set_tuning(ctx.h, nt, 0, 0))
+    try:
+        C, C2 = (ctx.gemm(dA, dB, bias=bias, activation=_lib.ACT_RELU) for _ in range(2))
+        ctx.gemm_check()
+    finally:
+        status(ctx.lib.cn_gemm_set_tuning(ctx.h, 0, 0, 0))
+    assert torch.equal(C, C2)
+    ref = np.maximum(A.astype(np.float64) @ B.astype(np.float64) + bias.cpu().numpy(), 0)
+    assert np.linalg.norm(ctx.to_numpy(C) - ref) <= 8e-6 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 300001), (3, 1001), (16, 40000), (1023, 7), (1024, 7), (1500, 3)])
+def test_bias_activation_of_any_shape(ctx, rows, cols):
+    rng = np.random.default_rng(rows)
+    A, b = rng.standard_normal((rows, cols)).astype(np.float32), rng.standard_normal(cols).astype(np.float32)
+    got = ctx.bias_activation(ctx.colmajor(A), torch.from_numpy(b).cuda(), _lib.ACT_RELU)
+    assert np.array_equal(ctx.to_numpy(got), np.maximum(A + b, 0))
+    got = ctx.bias_activation(ctx.colmajor(A), None, _lib.ACT_DOUBLE_RELU)
+    assert np.array_equal(ctx.to_numpy(got), np.clip(A, 0, 1))
 
 
 @pytest.mark.parametrize("n", [1, 3, 4, 5, 1023, 262147])
