@@ -912,7 +912,7 @@ extern "C" int cn_dotmpi_from_coded_f32(cn_context *ctx, const cn_coded *A, int6
     const int G = ctx->comm ? ctx->comm->nranks : 1, rank = ctx->comm ? ctx->comm->rank : 0;
     int64_t start, cnt;
     cn_shard_cols(n_total, rank, G, &start, &cnt);
-    if (mode != CN_GEMM_FP32_SIMT && cnt > 0 && !cn_gemm_small_shape(ctx, M, cnt, K, true) &&
+    if (mode != CN_GEMM_FP32_SIMT && cnt > 0 && !cn_gemm_small_shape(ctx, M, cnt, K, true, 2) &&
         cn_gemm_tc_supported(ctx, 0, 0, M, cnt, K, A->own_fp32, M, d_Wshard, K, d_C, M)) {
         if (!ctx->gemm) ctx->gemm = cn_gemm_workspace_new();
         cn_coded_src src;

@@ -170,12 +170,12 @@ extern "C" int cn_gemm_f32(cn_context *ctx, int transA, int transB, int64_t M, i
                            const float *d_A, int64_t lda, const float *d_B, int64_t ldb, float *d_C, int64_t ldc,
                            const cn_epilogue *epi, int mode, void *stream)
 {
-    return cn_gemm_dispatch(ctx, transA, transB, M, N, K, d_A, lda, d_B, ldb, d_C, ldc, epi, mode, stream, nullptr, nullptr);
+    return cn_gemm_dispatch(ctx, transA, transB, M, N, K, d_A, lda, d_B, ldb, d_C, ldc, epi, mode, stream, nullptr, nullptr, true);
 }
 
 int cn_gemm_dispatch(cn_context *ctx, int transA, int transB, int64_t M, int64_t N, int64_t K, const float *d_A, int64_t lda,
                      const float *d_B, int64_t ldb, float *d_C, int64_t ldc, const cn_epilogue *epi, int mode, void *stream,
-                     const cn_peer_out *peers, bool *used_peers)
+                     const cn_peer_out *peers, bool *used_peers, bool planes_ok)
 {
     if (used_peers) *used_peers = false;
     CN_REQUIRE(ctx, CN_ERR_ARG, "cn_gemm_f32: null context");
@@ -204,10 +204,17 @@ int cn_gemm_dispatch(cn_context *ctx, int transA, int transB, int64_t M, int64_t
     cn_gemm_workspace *ws = ctx->gemm;
     const bool tuned = ws && (ws->force_nt || ws->force_splits || ws->force_chain);
     const cn_prepared *pr = ws ? ws->prepared : nullptr;
-    const bool small = mode != CN_GEMM_FP32_SIMT && (L == 1 || ldc == M) && !tuned && !(ws && (ws->coded_src || ws->profile)) && (!pr || pr->raw) &&
-                       cn_gemm_small_shape(ctx, M, N, K, tma_ok) && (tma_ok || M * N * K >= 4096);
     // Weights that TMA cannot read as they are keep fp32-level accuracy in every mode: the fp32 kernel took them before.
     const int tc_mode = tma_ok ? mode : CN_GEMM_3XTF32;
+    // Many rows: both operands as planes (see cn_gemm_planes.cu), which also beats two rounds of CTAs of the small products' kernel (128
+    // x 4096 weights, 800 rows: 34 us against 24; 300 x 3000: 48 against 28).  Its four launches do not pay below 2^30 multiplications
+    // (520 x 784 . 784 x 1200: 38 us against 30 on the streaming kernel; 520 x 2000 . 2000 x 1000: 41 against 43).
+    const bool plain = mode != CN_GEMM_FP32_SIMT && !tuned && !(ws && (ws->coded_src || ws->profile));
+    const bool fine = plain && cn_gemm_small_shape(ctx, M, N, K, tma_ok, 2);
+    const bool planes = planes_ok && plain && L == 1 && !pr && !(peers && peers->npeers > 0) && cn_gemm_planes_shape(M, N, K, tc_mode, tma_ok) &&
+                        (fine || K >= (1LL << 30) / (M * N));
+    const bool small = plain && (L == 1 || ldc == M) && (!pr || pr->raw) && fine && (!planes || cn_gemm_small_shape(ctx, M, N, K, tma_ok, 1)) &&
+                       (tma_ok || M * N * K >= 4096);
     const bool tc_ok = tma_ok || (mode != CN_GEMM_FP32_SIMT && M * N * K >= 4096 && cn_gemm_tc_any_supported(transB, M, N, K, d_B));
     // a small product and its maxout are two launches as well, and the maxima are those of the very product a call without maxout gives
     const bool fused_maxout = tma_ok && (L == 1 || (!small && cn_gemm_tc_can_fuse_maxout(L)));
@@ -219,7 +226,7 @@ int cn_gemm_dispatch(cn_context *ctx, int transA, int transB, int64_t M, int64_t
         target_ld = M;
         CN_REQUIRE(ldc == M, CN_ERR_UNSUPPORTED, "cn_gemm_f32: un-fused maxout needs ldc == M");
     }
-    int st;
+    int st = CN_OK;
     if (small) {
         if (pr) {
             ws->prepared = nullptr;
@@ -241,7 +248,10 @@ int cn_gemm_dispatch(cn_context *ctx, int transA, int transB, int64_t M, int64_t
         e2.maxout_level = fused_maxout ? L : 1;
         e2.argmax_out = fused_maxout ? argmax : nullptr;
         const bool push = peers && peers->npeers > 0 && L == 1 && tma_ok;
-        st = cn_gemm_tc_launch(ctx, M, N, K, d_A, lda, d_B, ldb, target, target_ld, &e2, tc_mode, s, push ? peers : nullptr, transA, transB);
+        bool done = false;
+        if (planes) st = cn_gemm_planes_launch(ctx, M, N, K, d_A, lda, d_B, ldb, target, target_ld, &e2, tc_mode, s, transA, transB, tma_ok, fine,
+                                               &done);
+        if (!done && st == CN_OK) st = cn_gemm_tc_launch(ctx, M, N, K, d_A, lda, d_B, ldb, target, target_ld, &e2, tc_mode, s, push ? peers : nullptr, transA, transB);
         if (push && used_peers) *used_peers = true;
     } else {
         st = simt_launch(ctx, transA, transB, M, N, K, d_A, lda, d_B, ldb, target, target_ld, bias, act, s);

@@ -7,7 +7,8 @@ enum {
     CN_GEMM_SLOT_ASPLIT = 1,   // activations re-laid K-major as hi / lo planes with their scales
     CN_GEMM_SLOT_SPLITK = 2,   // partial tiles of the runs of K blocks of a launch
     CN_GEMM_SLOT_EXCHANGE = 3, // codes + scales of the 8-bit exchange in dotMPI
-    CN_GEMM_SLOTS = 4
+    CN_GEMM_SLOT_WSPLIT = 4,   // weights as hi / lo planes, for products with many rows
+    CN_GEMM_SLOTS = 5
 };
 
 #define CN_GEMM_MAX_TICKETS 4096
@@ -24,15 +25,18 @@ struct cn_coded_src {
 
 // Planes of an M x K activation operand, in one allocation: per band fp16 hi [M][Kp] and, in the 3x mode, lo, `plane` elements apart;
 // inverse scales [band][group of CN_PLANE_GROUP_K k][m_pad]; bands behind the first that a block of 16 rows x 64 k has, a byte each
-// [tile of 128 rows][64 k][8] (see cn_gemm_tc.cu).
+// [tile of 128 rows][64 k][8] (see cn_gemm_tc.cu); cells of left-overs [block of 16 rows][group]: how many elements of the 16 x 512
+// band 0 leaves something of, a byte each, and up to CN_CELL of them, {row << 16 | k, value}.
 #define CN_PLANE_GROUP_K 512
 #define CN_PLANE_BANDS 3
+#define CN_CELL 8
+#define CN_CELL_MANY 0xff   // more than that
 struct cn_planes {
     int64_t Kp, plane, m_pad, groups;
-    int parts;
-    size_t inv_off, bands_off, bytes;
+    int parts, bands;
+    size_t inv_off, bands_off, counts_off, cells_off, bytes;
 };
-void cn_plane_layout(int64_t M, int64_t K, int mode, cn_planes *pl);
+void cn_plane_layout(int64_t M, int64_t K, int mode, cn_planes *pl, int bands = CN_PLANE_BANDS);
 
 // The planes of an activation operand made ahead of the product that consumes them (cn_gemm_prepare): the product's own
 // pre-pass is then skipped.
@@ -44,6 +48,8 @@ struct cn_prepared {
     int mode = 0;
     bool filled = false;
 };
+
+struct cn_tc_cond;
 
 struct cn_gemm_workspace {
     void *ptr[CN_GEMM_SLOTS] = {nullptr, nullptr, nullptr, nullptr};
@@ -89,15 +95,23 @@ int cn_gemm_tc_split_activations(cn_context *ctx, int transA, int64_t M, int64_t
                                  cudaStream_t s);
 int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda,
                       const float *B, int64_t ldb, float *C, int64_t ldc, const cn_epilogue *epi, int mode, cudaStream_t s,
-                      const cn_peer_out *peers = nullptr, int transA = 0, int transB = 0);
+                      const cn_peer_out *peers = nullptr, int transA = 0, int transB = 0, const cn_tc_cond *cond = nullptr);
+// Products of planes by planes (cn_gemm_planes.cu), any layout and alignment of both operands: whether it is the faster kernel for a
+// shape, and the launch.  `fine`: the shape is one for the small products' kernel,
+// whose error must not be exceeded.  *done = false: no room for the planes of the weights, nothing was launched.
+bool cn_gemm_planes_shape(int64_t M, int64_t N, int64_t K, int mode, bool w_aligned);
+int cn_gemm_planes_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, const float *B, int64_t ldb, float *C, int64_t ldc,
+                          const cn_epilogue *epi, int mode, cudaStream_t s, int transA, int transB, bool w_aligned, bool fine, bool *done);
 // Small products in one launch (cn_gemm_small.cu): whether a shape is one, and the launch.  Takes any layout and alignment.
-bool cn_gemm_small_shape(const cn_context *ctx, int64_t M, int64_t N, int64_t K, bool w_aligned);
+bool cn_gemm_small_shape(const cn_context *ctx, int64_t M, int64_t N, int64_t K, bool w_aligned, int max_rounds);
 #define CN_SMALL_MAX_K 3072   // no product of aligned weights with a longer inner dimension is small: eight CTAs of twelve blocks of 32
 // K blocks of 32 per accumulation chain for weights whose rows TMA cannot read (cn_gemm_tc.cu)
 int cn_gemm_any_chain(int64_t K);
 int cn_gemm_small_launch(cn_context *ctx, int transA, int transB, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, const float *B, int64_t ldb,
                          float *C, int64_t ldc, const cn_epilogue *epi, int mode, cudaStream_t s, const cn_peer_out *peers, bool w_aligned);
-// cn_gemm_f32 with optional peer windows; *used_peers tells whether the launch took them (tensor-core path only).
+// cn_gemm_f32 with optional peer windows; *used_peers tells whether the launch took them (tensor-core path only).  planes_ok: the
+// kernel for many rows may be taken.  The sharded products stay with the streaming kernel, whose bits do not depend on whether
+// the activations' planes were made ahead or the output goes to peers.
 int cn_gemm_dispatch(cn_context *ctx, int transA, int transB, int64_t M, int64_t N, int64_t K, const float *d_A, int64_t lda,
                      const float *d_B, int64_t ldb, float *d_C, int64_t ldc, const cn_epilogue *epi, int mode, void *stream,
-                     const cn_peer_out *peers, bool *used_peers);
+                     const cn_peer_out *peers, bool *used_peers, bool planes_ok = false);

@@ -375,7 +375,7 @@ static int small_cluster(int64_t tiles, int kb, int sms)
     return c;
 }
 
-bool cn_gemm_small_shape(const cn_context *ctx, int64_t M, int64_t N, int64_t K, bool w_aligned)
+bool cn_gemm_small_shape(const cn_context *ctx, int64_t M, int64_t N, int64_t K, bool w_aligned, int max_rounds)
 {
     if (M < 1 || N < 1 || K < 1) return false;
     if (N > (1 << 21) / K) return false;   // at most 8 MB of weights
@@ -386,7 +386,7 @@ bool cn_gemm_small_shape(const cn_context *ctx, int64_t M, int64_t N, int64_t K,
     // more than two rounds of CTAs cost more than the streaming kernel's three launches: the 4096 x 4096 weight gradient of a batch of
     // 128 (1024 tiles, seven rounds) took 108 us here; the whole backward pass went from 210 to 162 us
     // a block costs a CTA 1.5 us, the streaming kernel's launches and reduction 15 to 20: 16 x 8000 . 8000 x 64 (32 blocks) took 43 us here
-    if (per_cta > (w_aligned ? SM_MAX_BLOCKS : SM_MAX_BLOCKS_ANY) || rounds > 2) return false;
+    if (per_cta > (w_aligned ? SM_MAX_BLOCKS : SM_MAX_BLOCKS_ANY) || rounds > max_rounds) return false;
     // weights that TMA cannot read must not become less exact than on the fp32 kernel (cn_gemm_any_chain); a TF32 block has twice the
     // additions of an fp16 one
     const int chain = cn_gemm_any_chain(K) / 2;

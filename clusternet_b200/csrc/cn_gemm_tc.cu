@@ -52,12 +52,9 @@
 #include <stdlib.h>
 #include "cn_epilogue.cuh"
 #include "cn_gemm.h"
-#include "cn_tc.cuh"
+#include "cn_gemm_tc.h"
+#include "cn_tc_split.cuh"
 
-#define TC_BM 128          // activation rows per CTA = UMMA N
-#define TC_BN 128          // W columns per tile       = UMMA M
-#define TC_WK 32           // k per W block: one 128-byte swizzle row of fp32
-#define TC_AK 64           // k per activation stage: one 128-byte swizzle row of fp16
 #define TC_W_TILE_BYTES (TC_BN * TC_WK * 4)
 
 // How the weights lie in memory: k contiguous or n contiguous ("transposed"), the rows of that layout 16-byte aligned or not.
@@ -80,12 +77,6 @@ __host__ __device__ constexpr int w_box_bytes(int wk)
 {
     return wk == W_K_ANY ? TC_CLASSES * TC_WK_CLASS_BYTES : wk == W_N_ANY ? TC_CLASSES * TC_WN_CLASS_BYTES : TC_W_TILE_BYTES;
 }
-#define TC_A_TILE_BYTES (TC_BM * TC_AK * 2)
-#define TC_GROUP_K CN_PLANE_GROUP_K
-#define TC_GROUP_KB (TC_GROUP_K / TC_WK)
-#define TC_BANDS CN_PLANE_BANDS   // the planes of the activations and of what they leave, twice
-#define TC_SUB 16                 // rows m of a block of left-overs
-#define TC_DRAIN_SLEEP_NS 100   // poll interval of the drain warps while a chain accumulates
 
 template <int NT, bool MODE3X, int WK>
 struct TcCfg {
@@ -156,6 +147,8 @@ struct TcParams {
     float *partials;        // [slot][w][32 quads of m][128 n] float4: slot = CTA + tile - full_tiles
     unsigned int *status;
     uint32_t w_shift;       // byte r: d_r of the weights' rows r, r + 4, ... (see W_K_ANY)
+    const uint8_t *cond[2]; // run only if one of these counts is CN_CELL_MANY (see cn_tc_cond); null: always
+    int64_t cond_n[2];
     int w_ready;            // nothing before the pre-pass still writes W: it may be loaded before the pre-pass has finished
     // fused all-gather: the peers are told that this rank's C may be overwritten; the tiles go to them in the reduction
     int npeers;
@@ -220,307 +213,6 @@ __device__ __forceinline__ void tc_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint
         "mov.b64 bd, {%2, %3};\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], bd, %4, p;\n\t}"
         ::"r"(d_tmem), "r"(a_tmem), "r"(b_desc_lo), "r"(b_desc_hi), "r"(idesc), "r"(accumulate) : "memory");
-}
-
-// kind::f16 instruction descriptor: D fp32 (bits 4-5 = 1), A and B fp16 (format 0 at bits 7-9 and 10-12),
-// both operands K-major (bits 15, 16 = 0), N >> 3 at bits 17-22, M >> 4 at bits 24-28.
-__host__ __device__ constexpr uint32_t make_idesc_f16(int m, int n)
-{
-    return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
-
-// ------------------------------------------------------------------------------------------------------- split
-// Power of two that brings a magnitude with these bits into [2^EXP, 2^(EXP+1)), and its inverse; both are normal numbers.
-// Zero and non-finite magnitudes keep the scale 1 (a non-finite element makes every sum it enters non-finite anyway).
-template <int EXP>
-__device__ __forceinline__ void tc_scale(uint32_t amax_bits, float &sc, float &inv)
-{
-    const int e = (int)(amax_bits >> 23);
-    int b = 254 + EXP - e;
-    if (b > 253) b = 253;
-    if (amax_bits == 0u || e == 255) b = 127;
-    sc = __uint_as_float((uint32_t)b << 23);
-    inv = __uint_as_float((uint32_t)(254 - b) << 23);
-}
-#define TC_A_EXP 14
-#define TC_W_EXP 13
-
-// Two floats in one 64-bit register pair, as the packed fp32 instructions take them.
-__device__ __forceinline__ uint64_t tc_pack2(float a, float b)
-{
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void tc_unpack2(uint64_t r, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r)); }
-__device__ __forceinline__ uint64_t tc_mul2(uint64_t a, uint64_t b)
-{
-    uint64_t r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ uint64_t tc_fma2(uint64_t a, uint64_t b, uint64_t c)
-{
-    uint64_t r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-
-// Two packed fp16 values -> floats, negated.
-__device__ __forceinline__ uint64_t tc_minus_f16x2(uint32_t h)
-{
-    float h0, h1;
-    asm("{\n\t.reg .b16 a, b;\n\t"
-        "mov.b32 {a, b}, %2;\n\t"
-        "cvt.f32.f16 %0, a;\n\t"
-        "cvt.f32.f16 %1, b;\n\t}"
-        : "=f"(h0), "=f"(h1) : "r"(h));
-    return tc_pack2(-h0, -h1);
-}
-__device__ __forceinline__ uint64_t tc_add2(uint64_t a, uint64_t b)
-{
-    uint64_t r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-
-// Two scaled values -> packed fp16 high parts, and (LO) packed fp16 low parts: lo = fp16(y - hi), the difference being exact.
-// Measured on registers with two warps per scheduler: 10 issue cycles per pair, 12 with the mixed-precision subtraction
-// (sub.f32.f16) in place of the two conversions back and the packed one.
-template <bool LO>
-__device__ __forceinline__ void tc_split2(uint64_t y, uint32_t &hi, uint32_t &lo)
-{
-    float y0, y1;
-    tc_unpack2(y, y0, y1);
-    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(y1), "f"(y0));
-    if (LO) {
-        float d0, d1;
-        tc_unpack2(tc_add2(y, tc_minus_f16x2(hi)), d0, d1);
-        asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(d1), "f"(d0));
-    }
-}
-
-// ... and what the parts leave of the two values (exact), where it is more of an element than the product may lose; 0 otherwise.
-#define TC_LEFT_3X 9.5367431640625e-7f   // 2^-20
-#define TC_LEFT_1X 9.765625e-4f          // 2^-10
-#define TC_LEFT_SCALE 274877906944.0f    // 2^38: what is left of a scaled value is at most 2^-25
-template <bool LO>
-__device__ __forceinline__ void tc_split2_left(float y0, float y1, uint32_t &hi, uint32_t &lo, float &r0, float &r1)
-{
-    const uint64_t y = tc_pack2(y0, y1);
-    tc_split2<LO>(y, hi, lo);
-    uint64_t r = tc_add2(y, tc_minus_f16x2(hi));
-    if (LO) r = tc_add2(r, tc_minus_f16x2(lo));
-    tc_unpack2(r, r0, r1);
-    constexpr float LEFT = LO ? TC_LEFT_3X : TC_LEFT_1X;
-    r0 = fabsf(r0) > LEFT * fabsf(y0) ? r0 : 0.0f;   // false for a NaN, which the parts carry
-    r1 = fabsf(r1) > LEFT * fabsf(y1) ? r1 : 0.0f;
-}
-// A high part of at least this (fp16 bits) leaves less: half an fp16 denormal, 2^-25, is 2^-20 of 2^-5 and 2^-10 of 2^-15.
-template <bool LO> __host__ __device__ constexpr uint32_t tc_safe_f16() { return LO ? 0x2800u : 0x0400u; }
-
-// ------------------------------------------------------------------------------------------ activation pre-pass
-// A (M x K) -> planes hi, lo: [M][Kp] fp16 with k contiguous, k in [K, Kp) zero, and the inverse scales a_inv[group][m_pad].
-// One CTA per 16 rows and group of 512 k.  What the planes leave of an element (see the top) goes to the next band's planes and
-// scales; `bands` tells which blocks of 16 rows x 32 k have any.  Bound by latency for a layer's activations and by memory otherwise: 4 bytes read
-// and 4 written per element.  CODED: the consumer-side half of the 8-bit exchange.  The activations arrive as gathered codes
-// (column-major like the fp32 matrix; column block r was coded by rank r with scale scales[r]) and are decoded here, inside
-// the pre-pass of the GEMM that consumes them, instead of being written out as fp32 first.  This rank's own block is taken
-// from its exact fp32 values.  Decode table as kDecompression_8bit builds it (source/clusterKernels.cu:1141-1152).
-struct ActCoded {
-    const uint8_t *codes;
-    const float *scales, *tbl, *own_fp32;
-    int own_rank, nranks;
-};
-#define ACT_ROWS TC_SUB
-#define ACT_PITCH (ACT_ROWS + 1)
-
-// Where the planes of an operand are (cn_plane_layout).
-struct ActPlanes {
-    uint16_t *p;            // band 0: hi, lo (3x mode only), band 1: ...
-    int64_t plane, Kp, m_pad, groups;
-    float *inv;
-    uint8_t *bands;
-    int stages;
-    __device__ __forceinline__ uint8_t *band_byte(int64_t m0, int64_t stage) const
-    {
-        return bands + ((m0 / TC_BM) * stages + stage) * (TC_BM / TC_SUB) + (m0 % TC_BM) / TC_SUB;
-    }
-};
-
-// Eight consecutive k of one row, scaled, into the planes of a band; x becomes what they leave, unscaled.  Returns whether anything is
-// left; a row with an element that is not finite leaves nothing, since its sums are not finite anyway.
-template <bool LO>
-__device__ __forceinline__ bool act_store8(const ActPlanes &pl, int band, int64_t at, float (&x)[8], float sc, float inv, bool finite)
-{
-    uint32_t h[4], l[4];
-    bool left = false;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        tc_split2_left<LO>(x[2 * e] * sc, x[2 * e + 1] * sc, h[e], l[e], x[2 * e], x[2 * e + 1]);
-        left |= x[2 * e] != 0.0f || x[2 * e + 1] != 0.0f;
-        x[2 * e] = finite ? x[2 * e] * inv : 0.0f;
-        x[2 * e + 1] = finite ? x[2 * e + 1] * inv : 0.0f;
-    }
-    uint16_t *q = pl.p + band * (LO ? 2 : 1) * pl.plane + at;
-    *reinterpret_cast<uint4 *>(q) = make_uint4(h[0], h[1], h[2], h[3]);
-    if (LO) *reinterpret_cast<uint4 *>(q + pl.plane) = make_uint4(l[0], l[1], l[2], l[3]);
-    return left && finite;
-}
-
-template <bool LO, bool CODED>
-__global__ void __launch_bounds__(256)
-cn_act_planes_kernel(const float *A, int64_t lda, int64_t M, int64_t K, const ActPlanes pl, const ActCoded cd)
-{
-    __shared__ float tile[TC_GROUP_K * ACT_PITCH];
-    __shared__ uint32_t red[16][ACT_ROWS];
-    __shared__ float s_sc[ACT_ROWS], s_inv[ACT_ROWS];
-    __shared__ bool s_finite[ACT_ROWS];
-    __shared__ uint32_t s_left[TC_BANDS][TC_GROUP_KB];   // something is left of these 32 k after the band
-    extern __shared__ float lut[];   // CODED: nranks x 256
-    const int tid = threadIdx.x;
-    // wait first, then release the product: it may then rely on everything before this pass having finished, and start on W
-    cn_pdl_wait();
-    cn_pdl_launch_dependents();
-    if (CODED) {
-        for (int e = tid; e < cd.nranks * 256; e += 256) {
-            const int r = e >> 8, c = e & 255, i = c & 127;
-            const float p = cd.scales[r];
-            float v;
-            if (i < CN_CODEBOOK_N) {
-                v = __fmul_rn(cd.tbl[i], p);
-                if (c >= 128) v = -v;
-            } else {
-                v = (c == 255) ? -p : p;
-            }
-            lut[e] = v;
-        }
-        __syncthreads();
-    }
-    const int64_t split = CODED ? K / cd.nranks : 0;
-    const int64_t m_blocks = pl.m_pad / ACT_ROWS, Kp = pl.Kp;
-    const int64_t g = blockIdx.x / m_blocks, m0 = (blockIdx.x - g * m_blocks) * ACT_ROWS, k0 = g * TC_GROUP_K;
-    {
-        const int ml = tid & 15, kl = tid >> 4;
-        const int64_t m = m0 + ml;
-        uint32_t amax = 0u;
-#pragma unroll 8
-        for (int j = 0; j < TC_GROUP_K / 16; ++j) {
-            const int kk = j * 16 + kl;
-            const int64_t k = k0 + kk;
-            float x = 0.0f;
-            if (m < M && k < K) {
-                if (CODED) {
-                    int r = split > 0 ? (int)(k / split) : cd.nranks - 1;
-                    if (r > cd.nranks - 1) r = cd.nranks - 1;
-                    if (r == cd.own_rank && cd.own_fp32) x = cd.own_fp32[m + (k - split * cd.own_rank) * M];
-                    else x = lut[(r << 8) + cd.codes[m + k * M]];
-                } else {
-                    x = A[m + k * lda];
-                }
-            }
-            tile[kk * ACT_PITCH + ml] = x;
-            amax = max(amax, __float_as_uint(x) & 0x7fffffffu);
-        }
-        red[kl][ml] = amax;
-    }
-    if (tid < TC_BANDS * TC_GROUP_KB) (&s_left[0][0])[tid] = 0u;
-    // eight consecutive k per item; a warp covers 8 rows x 32 k (conflict-free reads, 64 contiguous bytes per row)
-    const int lane = tid & 31, warp = tid >> 5;
-    for (int band = 0;; ++band) {
-        __syncthreads();
-        if (tid < ACT_ROWS) {
-            uint32_t amax = 0u;
-#pragma unroll
-            for (int j = 0; j < 16; ++j) amax = max(amax, red[j][tid]);
-            tc_scale<TC_A_EXP>(amax, s_sc[tid], s_inv[tid]);
-            s_finite[tid] = amax < 0x7f800000u;
-            pl.inv[(band * pl.groups + g) * pl.m_pad + m0 + tid] = s_inv[tid];
-        }
-        __syncthreads();
-        bool left = false;
-#pragma unroll
-        for (int it = 0; it < 4; ++it) {
-            const int ml = (it & 1) * 8 + (lane & 7), kk = ((warp + 8 * (it >> 1)) * 4 + (lane >> 3)) * 8, st = kk / TC_WK;
-            const int64_t m = m0 + ml, k = k0 + kk;
-            if (m < M && k < Kp && (band == 0 || s_left[band - 1][st] != 0u)) {
-                float x[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) x[e] = tile[(kk + e) * ACT_PITCH + ml];
-                if (act_store8<LO>(pl, band, m * Kp + k, x, s_sc[ml], s_inv[ml], s_finite[ml])) {
-                    left = true;
-                    s_left[band][st] = 1u;
-                }
-#pragma unroll
-                for (int e = 0; e < 8; ++e) tile[(kk + e) * ACT_PITCH + ml] = x[e];
-            }
-        }
-        if (!__syncthreads_or(left) || band == TC_BANDS - 1) break;
-        // the largest left of each row, as at the start (what the others leave is zero)
-        uint32_t amax = 0u;
-        for (int j = 0; j < TC_GROUP_K / 16; ++j) amax = max(amax, __float_as_uint(tile[(j * 16 + (tid >> 4)) * ACT_PITCH + (tid & 15)]) & 0x7fffffffu);
-        red[tid >> 4][tid & 15] = amax;
-    }
-    if (tid < TC_GROUP_K / TC_AK && k0 + tid * TC_AK < Kp) {
-        uint32_t n = 0u;
-        for (int band = 0; band < TC_BANDS - 1; ++band) n += s_left[band][2 * tid] + (s_left[band][2 * tid + 1] << 4);
-        *pl.band_byte(m0, k0 / TC_AK + tid) = (uint8_t)n;
-    }
-}
-
-// Same planes for a transposed activation operand: op(A)(m, k) = A[k + m * lda] is already K-major (this is also what
-// a row-major M x K batch looks like): one warp per row and group, two times eight k per lane, 16-byte loads when the row pitch
-// and the base allow.
-template <bool LO>
-__global__ void __launch_bounds__(32 * ACT_ROWS)
-cn_act_planes_t_kernel(const float *A, int64_t lda, int64_t M, int64_t K, const ActPlanes pl, int vec_ok)
-{
-    __shared__ uint32_t s_left[TC_BANDS][TC_GROUP_KB];
-    const int tid = threadIdx.x, lane = tid & 31;
-    const int64_t m_blocks = pl.m_pad / ACT_ROWS;
-    const int64_t g = blockIdx.x / m_blocks, m0 = (blockIdx.x - g * m_blocks) * ACT_ROWS, m = m0 + (tid >> 5), k0 = g * TC_GROUP_K;
-    cn_pdl_wait();
-    cn_pdl_launch_dependents();   // after the wait: see cn_act_planes_kernel
-    if (tid < TC_BANDS * TC_GROUP_KB) (&s_left[0][0])[tid] = 0u;
-    __syncthreads();
-    const float *src = A + m * lda;
-    float x[2][8];
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-        const int64_t k = k0 + 256 * j + 8 * lane;
-        if (vec_ok && m < M && k + 7 < K) {
-            const float4 a = *reinterpret_cast<const float4 *>(src + k), b = *reinterpret_cast<const float4 *>(src + k + 4);
-            x[j][0] = a.x; x[j][1] = a.y; x[j][2] = a.z; x[j][3] = a.w;
-            x[j][4] = b.x; x[j][5] = b.y; x[j][6] = b.z; x[j][7] = b.w;
-        } else {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) x[j][e] = (m < M && k + e < K) ? src[k + e] : 0.0f;
-        }
-    }
-    for (int band = 0;; ++band) {
-        uint32_t amax = 0u;
-#pragma unroll
-        for (int e = 0; e < 16; ++e) amax = max(amax, __float_as_uint(x[e >> 3][e & 7]) & 0x7fffffffu);
-        amax = __reduce_max_sync(0xffffffffu, amax);
-        float sc, inv;
-        tc_scale<TC_A_EXP>(amax, sc, inv);
-        if (lane == 0) pl.inv[(band * pl.groups + g) * pl.m_pad + m] = inv;
-        bool left = false;
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int kk = 256 * j + 8 * lane, st = kk / TC_WK;
-            if (m < M && k0 + kk < pl.Kp && (band == 0 || s_left[band - 1][st] != 0u) && act_store8<LO>(pl, band, m * pl.Kp + k0 + kk, x[j], sc, inv, amax < 0x7f800000u)) {
-                left = true;
-                s_left[band][st] = 1u;
-            }
-        }
-        if (!__syncthreads_or(left) || band == TC_BANDS - 1) break;
-    }
-    if (tid < TC_GROUP_K / TC_AK && k0 + tid * TC_AK < pl.Kp) {
-        uint32_t n = 0u;
-        for (int band = 0; band < TC_BANDS - 1; ++band) n += s_left[band][2 * tid] + (s_left[band][2 * tid + 1] << 4);
-        *pl.band_byte(m0, k0 / TC_AK + tid) = (uint8_t)n;
-    }
 }
 
 // -------------------------------------------------------------------------------------------------- main kernel
@@ -669,6 +361,10 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     cn_pdl_launch_dependents();
+    if (p.cond[0]) {
+        cn_pdl_wait();
+        if (!__syncthreads_or(tc_many(p.cond[0], p.cond_n[0]) || tc_many(p.cond[1], p.cond_n[1]))) return;
+    }
 
     // Fused all-gather: everything queued earlier on this GPU's stream has finished, so this rank's copy of C may now be
     // overwritten by its peers: tell them (slot 0 of their flag block).
@@ -1223,24 +919,6 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
 // One CTA per COLS columns of one W tile: adds the partial tiles of all runs in K order (a fixed order, so the result does not
 // depend on scheduling), applies bias and activation, turns the block through shared memory so that a warp stores 512
 // contiguous bytes of a column, and stores to C and, for the fused all-gather, to every peer's C (full NVLink packets).
-struct ReduceParams {
-    const float *partials;
-    int nt, tail_ctas, kb_total;
-    int tail_tiles;              // tiles cut into runs, [full_tiles, full_tiles + tail_tiles)
-    int full_tiles, tiles_m;
-    int64_t M, N;
-    float *C;
-    int64_t ldc;
-    const float *bias;
-    int act;
-    int npeers;
-    float *peerC[CN_MAX_PEERS];
-    const unsigned int *ready;
-    int nranks, my_rank;
-    unsigned int epoch;
-    unsigned int *status;
-};
-
 //
 // 32 columns where there are tiles for every SM.  Few tiles are cut into many runs, and what bounds them is how many loads a CTA has in
 // flight: 8 columns, eight partial tiles at a time (16 x 40000 . 40000 x 201, 148 runs: FIXME us with 32 columns, FIXME with 8).
@@ -1267,9 +945,9 @@ cn_splitk_reduce_kernel(const __grid_constant__ ReduceParams p)
         __syncthreads();
     }
     const int chunk = blockIdx.x % (TC_BN / COLS);
-    const int tw = blockIdx.x / (TC_BN / COLS), r = tw / p.nt, w = tw - r * p.nt, tile = p.full_tiles + r;
-    const int64_t m0 = (int64_t)(tile % p.tiles_m) * TC_BM, n0 = ((int64_t)(tile / p.tiles_m) * p.nt + w) * TC_BN + chunk * COLS;
-    if (n0 >= p.N) return;
+    const int tw = blockIdx.x / (TC_BN / COLS), rm = tw / p.nt, w = tw - rm * p.nt, r = rm / p.mt, mh = rm - r * p.mt, tile = p.full_tiles + r;
+    const int64_t m0 = ((int64_t)(tile % p.tiles_m) * p.mt + mh) * p.rows, n0 = ((int64_t)(tile / p.tiles_m) * p.nt + w) * TC_BN + chunk * COLS;
+    if (n0 >= p.N || m0 >= p.M) return;
     // the CTAs whose runs hold K blocks of this tile: run c is [total c / ctas, total (c + 1) / ctas)
     const int64_t total = (int64_t)p.tail_tiles * p.kb_total, first = (int64_t)r * p.kb_total, last = first + p.kb_total - 1;
     auto owner = [&](int64_t x) {
@@ -1281,8 +959,8 @@ cn_splitk_reduce_kernel(const __grid_constant__ ReduceParams p)
     const int64_t c0 = owner(first), c1 = owner(last);
     const int row = threadIdx.x % COLS, quad = threadIdx.x / COLS;   // column of the chunk; quads of m: quad + QSTEP j
     constexpr int64_t TILE4 = TC_BM * TC_BN / 4;
-    const float4 *src = reinterpret_cast<const float4 *>(p.partials) + ((c0 + r) * p.nt + w) * TILE4 + quad * TC_BN + chunk * COLS + row;
-    const int64_t step = p.nt * TILE4;
+    const float4 *src = reinterpret_cast<const float4 *>(p.partials) + (((c0 + r) * p.mt + mh) * p.nt + w) * TILE4 + quad * TC_BN + chunk * COLS + row;
+    const int64_t step = p.mt * p.nt * TILE4;
     float4 acc[QUADS];
 #pragma unroll
     for (int j = 0; j < QUADS; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1316,7 +994,7 @@ cn_splitk_reduce_kernel(const __grid_constant__ ReduceParams p)
     for (int j = 0; j < COLS / 8; ++j) {
         const int nl = (threadIdx.x >> 5) + 8 * j;
         const int64_t n = n0 + nl;
-        if (n >= p.N || m >= p.M) continue;
+        if (n >= p.N || m >= p.M || lane * 4 >= p.rows) continue;
         const float b = p.bias ? p.bias[n] : 0.0f;
         const float4 a = *reinterpret_cast<const float4 *>(&turn[nl][lane * 4]);
         float v[4] = {a.x, a.y, a.z, a.w};
@@ -1337,11 +1015,16 @@ cn_splitk_reduce_kernel(const __grid_constant__ ReduceParams p)
 }
 
 // ------------------------------------------------------------------------------------------------------ host
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                                  const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+int cn_splitk_reduce_launch(cn_context *ctx, const ReduceParams &rp, cudaStream_t s)
+{
+    const int64_t blocks = (int64_t)rp.tail_tiles * rp.nt * rp.mt;
+    if (blocks * 4 <= ctx->sm_count) CN_CUDA(cn_launch_pdl(cn_splitk_reduce_kernel<8>, dim3((unsigned)(blocks * (TC_BN / 8))), 256, 0, s, rp));
+    else CN_CUDA(cn_launch_pdl(cn_splitk_reduce_kernel<32>, dim3((unsigned)(blocks * (TC_BN / 32))), 256, 0, s, rp));
+    cn_count_launch();
+    return CN_OK;
+}
 
-static int get_encode_fn(cn_context *ctx, EncodeTiledFn *out)
+int cn_get_encode_fn(cn_context *ctx, EncodeTiledFn *out)
 {
     if (!ctx->gemm) ctx->gemm = cn_gemm_workspace_new();
     if (!ctx->gemm->encode_fn) {
@@ -1394,19 +1077,6 @@ static int make_w_maps(EncodeTiledFn enc, WMaps *m, uint32_t *shift, const float
     return CN_OK;
 }
 
-// Activation planes: fp16, k contiguous with pitch Kp, `plane` elements apart, box 64 k x 128 rows of one, 128-byte swizzle.
-static int make_a_map(EncodeTiledFn enc, CUtensorMap *map, const uint16_t *base, int64_t Kp, int64_t M, int64_t plane, int planes)
-{
-    cuuint64_t dims[3] = {(cuuint64_t)Kp, (cuuint64_t)M, (cuuint64_t)planes};
-    cuuint64_t strides[2] = {(cuuint64_t)Kp * sizeof(uint16_t), (cuuint64_t)plane * sizeof(uint16_t)};
-    cuuint32_t box[3] = {(cuuint32_t)TC_AK, (cuuint32_t)TC_BM, 1};
-    cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<uint16_t *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    CN_REQUIRE(r == CUDA_SUCCESS, CN_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d (activation planes %lld x %lld)", (int)r, (long long)M, (long long)Kp);
-    return CN_OK;
-}
-
 bool cn_gemm_tc_can_fuse_maxout(int L) { return L == 2 || L == 4 || L == 8 || L == 16 || L == 32; }
 
 // Rows that TMA can read as they are.
@@ -1452,67 +1122,12 @@ static int launch_cfg(const WMaps &mw, const CUtensorMap &ma, const TcParams &pr
     return CN_OK;
 }
 
-// Geometry of the planes of an M x K operand in one allocation.
-void cn_plane_layout(int64_t M, int64_t K, int mode, cn_planes *pl)
-{
-    pl->parts = mode == CN_GEMM_3XTF32 ? 2 : 1;
-    pl->Kp = (K + TC_AK - 1) / TC_AK * TC_AK;
-    pl->plane = (M * pl->Kp + 127) / 128 * 128;
-    pl->m_pad = (M + TC_BM - 1) / TC_BM * TC_BM;
-    pl->groups = (K + TC_GROUP_K - 1) / TC_GROUP_K;
-    pl->inv_off = (size_t)TC_BANDS * pl->parts * pl->plane * sizeof(uint16_t);
-    pl->bands_off = pl->inv_off + (size_t)TC_BANDS * pl->groups * pl->m_pad * sizeof(float);
-    pl->bytes = pl->bands_off + (size_t)(pl->m_pad / TC_SUB) * (pl->Kp / TC_AK);
-}
-
-template <bool LO>
-static int act_planes(cn_context *ctx, int transA, int64_t M, int64_t K, const float *A, int64_t lda, const cn_coded_src *cs, const cn_planes &pl,
-                      uint8_t *base, cudaStream_t s)
-{
-    const int64_t ctas = pl.groups * (pl.m_pad / ACT_ROWS);
-    CN_REQUIRE(ctas < (1LL << 31), CN_ERR_UNSUPPORTED, "cn_gemm_f32: activation matrix too large for the split pre-pass");
-    const dim3 grid((unsigned)ctas);
-    ActPlanes ap;
-    ap.p = reinterpret_cast<uint16_t *>(base);
-    ap.plane = pl.plane; ap.Kp = pl.Kp; ap.m_pad = pl.m_pad; ap.groups = pl.groups;
-    ap.inv = reinterpret_cast<float *>(base + pl.inv_off);
-    ap.bands = base + pl.bands_off;
-    ap.stages = (int)(pl.Kp / TC_AK);
-    if (cs) {
-        ActCoded cd;
-        cd.codes = cs->codes; cd.scales = cs->scales; cd.tbl = ctx->d_tbl; cd.own_fp32 = cs->own_fp32;
-        cd.own_rank = cs->own_rank; cd.nranks = cs->nranks;
-        CN_CUDA(cn_launch_pdl(cn_act_planes_kernel<LO, true>, grid, 256, (size_t)cs->nranks * 256 * sizeof(float), s, A, lda, M, K, ap, cd));
-    } else if (transA) {
-        const int vec_ok = ((lda & 3) == 0) && ((reinterpret_cast<uintptr_t>(A) & 15u) == 0);
-        CN_CUDA(cn_launch_pdl(cn_act_planes_t_kernel<LO>, grid, 32 * ACT_ROWS, 0, s, A, lda, M, K, ap, vec_ok));
-    } else {
-        CN_CUDA(cn_launch_pdl(cn_act_planes_kernel<LO, false>, grid, 256, 0, s, A, lda, M, K, ap, ActCoded()));
-    }
-    cn_count_launch();
-    return CN_OK;
-}
-
-static int act_planes(cn_context *ctx, int transA, int64_t M, int64_t K, const float *A, int64_t lda, const cn_coded_src *cs, const cn_planes &pl,
-                      void *planes, cudaStream_t s)
-{
-    return pl.parts == 2 ? act_planes<true>(ctx, transA, M, K, A, lda, cs, pl, (uint8_t *)planes, s)
-                         : act_planes<false>(ctx, transA, M, K, A, lda, cs, pl, (uint8_t *)planes, s);
-}
-
-int cn_gemm_tc_split_activations(cn_context *ctx, int transA, int64_t M, int64_t K, const float *A, int64_t lda, int mode, void *planes, cudaStream_t s)
-{
-    cn_planes pl;
-    cn_plane_layout(M, K, mode, &pl);
-    return act_planes(ctx, transA, M, K, A, lda, nullptr, pl, planes, s);
-}
-
 int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, const float *B,
                       int64_t ldb, float *C, int64_t ldc, const cn_epilogue *epi, int mode, cudaStream_t s, const cn_peer_out *peers,
-                      int transA, int transB)
+                      int transA, int transB, const cn_tc_cond *cond)
 {
     EncodeTiledFn enc = nullptr;
-    int st = get_encode_fn(ctx, &enc);
+    int st = cn_get_encode_fn(ctx, &enc);
     if (st != CN_OK) return st;
     cn_gemm_workspace *ws = ctx->gemm;
     {
@@ -1527,7 +1142,9 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
     cn_plane_layout(M, K, mode, &pl);
     uint8_t *planes = nullptr;
     const bool ahead = ws->prepared != nullptr;
-    if (ahead) {
+    if (cond) {
+        planes = (uint8_t *)cond->planes;
+    } else if (ahead) {
         const cn_prepared *pr = ws->prepared;
         ws->prepared = nullptr;
         CN_REQUIRE(pr->filled && pr->M == M && pr->K == K && pr->mode == mode, CN_ERR_SHAPE,
@@ -1541,7 +1158,7 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
         const cn_coded_src *cs = ws->coded_src;
         ws->coded_src = nullptr;
         CN_REQUIRE(!cs || (!transA && lda == M), CN_ERR_UNSUPPORTED, "coded activations must be untransposed with ld = rows");
-        if ((st = act_planes(ctx, transA, M, K, A, lda, cs, pl, planes, s)) != CN_OK) return st;
+        if ((st = cn_make_planes(ctx, transA != 0, M, K, A, lda, cs, pl, planes, s)) != CN_OK) return st;
     }
 
     // 2. work decomposition
@@ -1552,7 +1169,7 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
     const int kb_total = (int)((K + TC_WK - 1) / TC_WK);
     const int64_t sms = ctx->sm_count;
     int64_t full = 0, tail_ctas = 0;
-    if (maxout > 1) {
+    if (maxout > 1 || cond) {
         full = tiles;   // the reduction kernel has no maxout; such layers are small
     } else if (ws->force_splits >= 1) {
         const int64_t splits = ws->force_splits <= kb_total ? ws->force_splits : kb_total;
@@ -1596,7 +1213,8 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
     prm.a_stages = (int)(pl.Kp / TC_AK);
     prm.partials = nullptr;
     prm.status = ws->d_status;
-    prm.w_ready = ahead ? 0 : 1;
+    prm.w_ready = ahead || cond ? 0 : 1;
+    for (int i = 0; i < 2; ++i) { prm.cond[i] = cond ? cond->counts[i] : nullptr; prm.cond_n[i] = cond ? cond->n[i] : 0; }
     prm.npeers = 0;
     prm.peer_flags = nullptr;
     prm.nranks = 0; prm.my_rank = 0; prm.epoch = 0;
@@ -1620,7 +1238,7 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
     st = transB ? make_w_maps(enc, &mw, &prm.w_shift, B, N, K, ldb, wk)    // stored N x K, n contiguous
                 : make_w_maps(enc, &mw, &prm.w_shift, B, K, N, ldb, wk);
     if (st != CN_OK) return st;
-    st = make_a_map(enc, &ma, reinterpret_cast<const uint16_t *>(planes), pl.Kp, M, pl.plane, TC_BANDS * pl.parts);
+    st = cn_make_planes_map(enc, &ma, reinterpret_cast<const uint16_t *>(planes), pl.Kp, M, pl.plane, TC_BANDS * pl.parts, TC_BM);
     if (st != CN_OK) return st;
 
     cudaEvent_t ev_stop = nullptr;
@@ -1645,16 +1263,14 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
     if (st != CN_OK) return st;
     if (rest > 0) {
         ReduceParams rp;
-        rp.partials = prm.partials; rp.nt = nt; rp.tail_ctas = (int)tail_ctas; rp.kb_total = kb_total;
+        rp.partials = prm.partials; rp.nt = nt; rp.mt = 1; rp.rows = TC_BM; rp.tail_ctas = (int)tail_ctas; rp.kb_total = kb_total;
         rp.tail_tiles = (int)rest; rp.full_tiles = (int)full; rp.tiles_m = (int)tiles_m; rp.M = M; rp.N = N;
         rp.C = C; rp.ldc = ldc; rp.bias = prm.bias; rp.act = prm.act;
         rp.npeers = prm.npeers;
         for (int i = 0; i < CN_MAX_PEERS; ++i) rp.peerC[i] = prm.npeers > i ? peers->C[i] : nullptr;
         rp.ready = prm.npeers > 0 ? peers->ready : nullptr;
         rp.nranks = prm.nranks; rp.my_rank = prm.my_rank; rp.epoch = prm.epoch; rp.status = prm.status;
-        if (rest * nt * 4 <= sms) CN_CUDA(cn_launch_pdl(cn_splitk_reduce_kernel<8>, dim3((unsigned)(rest * nt * (TC_BN / 8))), 256, 0, s, rp));
-        else CN_CUDA(cn_launch_pdl(cn_splitk_reduce_kernel<32>, dim3((unsigned)(rest * nt * (TC_BN / 32))), 256, 0, s, rp));
-        cn_count_launch();
+        if ((st = cn_splitk_reduce_launch(ctx, rp, s)) != CN_OK) return st;
     }
     if (ev_stop) CN_CUDA(cudaEventRecord(ev_stop, s));
     ctx->gemm_last_path = mode3x ? "tcgen05_3xtf32" : "tcgen05_tf32";

@@ -1,0 +1,126 @@
+// Operands of the tensor-core products as fp16 parts: constants and the arithmetic of the split (see cn_gemm_tc.cu), shared by the
+// streaming kernel, the kernel that multiplies planes (cn_gemm_planes.cu) and the pre-pass that makes planes.
+#pragma once
+#include "cn_gemm.h"
+#include "cn_tc.cuh"
+
+#define TC_BM 128          // activation rows per CTA = UMMA N
+#define TC_BN 128          // W columns per tile       = UMMA M
+#define TC_WK 32           // k per W block: one 128-byte swizzle row of fp32
+#define TC_AK 64           // k per stage of planes: one 128-byte swizzle row of fp16
+#define TC_A_TILE_BYTES (TC_BM * TC_AK * 2)
+#define TC_GROUP_K CN_PLANE_GROUP_K
+#define TC_GROUP_KB (TC_GROUP_K / TC_WK)
+#define TC_BANDS CN_PLANE_BANDS   // the planes of the activations and of what they leave, twice
+#define TC_SUB 16                 // rows m of a block of left-overs
+#define TC_DRAIN_SLEEP_NS 100   // poll interval of the drain warps while a chain accumulates
+
+// kind::f16 instruction descriptor: D fp32 (bits 4-5 = 1), A and B fp16 (format 0 at bits 7-9 and 10-12),
+// both operands K-major (bits 15, 16 = 0), N >> 3 at bits 17-22, M >> 4 at bits 24-28.
+__host__ __device__ constexpr uint32_t make_idesc_f16(int m, int n)
+{
+    return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
+
+// ------------------------------------------------------------------------------------------------------- split
+// Power of two that brings a magnitude with these bits into [2^EXP, 2^(EXP+1)), and its inverse; both are normal numbers.
+// Zero and non-finite magnitudes keep the scale 1 (a non-finite element makes every sum it enters non-finite anyway).
+template <int EXP>
+__device__ __forceinline__ void tc_scale(uint32_t amax_bits, float &sc, float &inv)
+{
+    const int e = (int)(amax_bits >> 23);
+    int b = 254 + EXP - e;
+    if (b > 253) b = 253;
+    if (amax_bits == 0u || e == 255) b = 127;
+    sc = __uint_as_float((uint32_t)b << 23);
+    inv = __uint_as_float((uint32_t)(254 - b) << 23);
+}
+#define TC_A_EXP 14
+#define TC_W_EXP 13
+
+// Two floats in one 64-bit register pair, as the packed fp32 instructions take them.
+__device__ __forceinline__ uint64_t tc_pack2(float a, float b)
+{
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void tc_unpack2(uint64_t r, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r)); }
+__device__ __forceinline__ uint64_t tc_mul2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t tc_fma2(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// Two packed fp16 values -> floats, negated.
+__device__ __forceinline__ uint64_t tc_minus_f16x2(uint32_t h)
+{
+    float h0, h1;
+    asm("{\n\t.reg .b16 a, b;\n\t"
+        "mov.b32 {a, b}, %2;\n\t"
+        "cvt.f32.f16 %0, a;\n\t"
+        "cvt.f32.f16 %1, b;\n\t}"
+        : "=f"(h0), "=f"(h1) : "r"(h));
+    return tc_pack2(-h0, -h1);
+}
+__device__ __forceinline__ uint64_t tc_add2(uint64_t a, uint64_t b)
+{
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// Two scaled values -> packed fp16 high parts, and (LO) packed fp16 low parts: lo = fp16(y - hi), the difference being exact.
+// Measured on registers with two warps per scheduler: 10 issue cycles per pair, 12 with the mixed-precision subtraction
+// (sub.f32.f16) in place of the two conversions back and the packed one.
+template <bool LO>
+__device__ __forceinline__ void tc_split2(uint64_t y, uint32_t &hi, uint32_t &lo)
+{
+    float y0, y1;
+    tc_unpack2(y, y0, y1);
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(hi) : "f"(y1), "f"(y0));
+    if (LO) {
+        float d0, d1;
+        tc_unpack2(tc_add2(y, tc_minus_f16x2(hi)), d0, d1);
+        asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(lo) : "f"(d1), "f"(d0));
+    }
+}
+
+// ... and what the parts leave of the two values (exact), where it is more of an element than the product may lose; 0 otherwise.
+#define TC_LEFT_3X 9.5367431640625e-7f   // 2^-20
+#define TC_LEFT_1X 9.765625e-4f          // 2^-10
+#define TC_LEFT_SCALE 274877906944.0f    // 2^38: what is left of a scaled value is at most 2^-25
+template <bool LO>
+__device__ __forceinline__ void tc_split2_left(float y0, float y1, uint32_t &hi, uint32_t &lo, float &r0, float &r1)
+{
+    const uint64_t y = tc_pack2(y0, y1);
+    tc_split2<LO>(y, hi, lo);
+    uint64_t r = tc_add2(y, tc_minus_f16x2(hi));
+    if (LO) r = tc_add2(r, tc_minus_f16x2(lo));
+    tc_unpack2(r, r0, r1);
+    constexpr float LEFT = LO ? TC_LEFT_3X : TC_LEFT_1X;
+    r0 = fabsf(r0) > LEFT * fabsf(y0) ? r0 : 0.0f;   // false for a NaN, which the parts carry
+    r1 = fabsf(r1) > LEFT * fabsf(y1) ? r1 : 0.0f;
+}
+// A high part of at least this (fp16 bits) leaves less: half an fp16 denormal, 2^-25, is 2^-20 of 2^-5 and 2^-10 of 2^-15.
+template <bool LO> __host__ __device__ constexpr uint32_t tc_safe_f16() { return LO ? 0x2800u : 0x0400u; }
+
+// Whether one of the counts of left-overs is CN_CELL_MANY (all threads of the CTA).
+__device__ __forceinline__ bool tc_many(const uint8_t *counts, int64_t n)
+{
+    bool many = false;
+    const int64_t n16 = n >> 4;
+    for (int64_t i = threadIdx.x; i < n16; i += blockDim.x) {
+        const uint4 v = __ldcg(reinterpret_cast<const uint4 *>(counts) + i);
+        many |= (__vcmpeq4(v.x, 0xffffffffu) | __vcmpeq4(v.y, 0xffffffffu) | __vcmpeq4(v.z, 0xffffffffu) | __vcmpeq4(v.w, 0xffffffffu)) != 0u;
+    }
+    for (int64_t i = (n16 << 4) + threadIdx.x; i < n; i += blockDim.x) many |= __ldcg(counts + i) == CN_CELL_MANY;
+    return many;
+}

@@ -1,0 +1,176 @@
+"""The product of planes by planes (many rows): edges of its tiles, stages and chains, every layout and alignment of both operands, the
+lists of elements that two fp16 parts cannot hold, and the way back to the streaming kernel where a list overflows.
+
+Bounds as for the streaming kernel (test_gemm_paths_gpu.py): per element 2.5e-5 of sum |a_k b_k| in the 3x mode and 1.05e-3 in the
+single pass; a single term 2^-20 for what the parts of each operand may leave, 2^-22 for the product of the low parts and four
+additions truncated to 2^-23 (2.7e-6), in the single pass 2^-10 + 2^-11 + 2^-20."""
+import numpy as np
+import pytest
+import torch
+
+from clusternet_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+REL_3X, REL_1X = 2.5e-5, 1.05e-3
+ACT = {_lib.ACT_LINEAR: lambda x: x, _lib.ACT_RELU: lambda x: x.clamp(min=0), _lib.ACT_LOGISTIC: torch.sigmoid,
+       _lib.ACT_DOUBLE_RELU: lambda x: x.clamp(0, 1)}
+
+
+def place(x, off=0):
+    """torch (rows x cols) -> column-major device matrix whose base lies `off` floats past a 16-byte boundary, between NaNs."""
+    rows, cols = x.shape
+    buf = torch.full((rows * cols + 64,), float("nan"), device="cuda")
+    t = buf[32 + off:32 + off + rows * cols].view(cols, rows)
+    t.copy_(x.t())
+    return t
+
+
+def product(ctx, A, W, transA=False, transB=False, offA=0, offW=0, planes=True, **kw):
+    """gemm of A (M x K) and W (K x N), stored as the flags say; `planes`: one pre-pass for both operands, product, maybe a reduction,
+    and the streaming kernel that ends at once."""
+    a, w = place(A.t() if transA else A, offA), place(W.t() if transB else W, offW)
+    C = torch.full((W.shape[1], A.shape[0]), float("nan"), device="cuda")
+    n0 = ctx.lib.cn_kernel_launches()
+    ctx.gemm(a, w, out=C, transA=transA, transB=transB, **kw)
+    launches = ctx.lib.cn_kernel_launches() - n0
+    ctx.gemm_check()
+    assert launches >= 3 if planes else launches <= 3
+    return C.t().double()
+
+
+def within(C, A, W, rel, bias=None, act=_lib.ACT_LINEAR):
+    A, W = A.double(), W.double()
+    ref, bound = A @ W, rel * (A.abs() @ W.abs())
+    if bias is not None:
+        ref, bound = ref + bias.double(), bound + rel * bias.double().abs()
+    return bool(((C - ACT[act](ref)).abs() <= bound + 1e-7 * (act != _lib.ACT_LINEAR)).all())
+
+
+# tiles of 256 columns by 32 .. 256 rows; 64 k per stage, chains of 512 k; one pair, a full round and runs along K; odd pitches
+SHAPES = [(513, 40, 4200), (514, 64, 4500), (640, 65, 5000), (769, 448, 4100), (1025, 513, 2049), (800, 1100, 1537), (520, 8192, 256), (2080, 3000, 770),
+          (1536, 1040, 9500)]
+
+
+@pytest.mark.parametrize("M,K,N", SHAPES)
+@pytest.mark.parametrize("transA,transB", [(False, False), (True, False), (False, True), (True, True)])
+def test_edges_in_every_layout(ctx, M, K, N, transA, transB):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(M + K + N)
+    A, W, bias = (torch.randn(s, device="cuda", generator=g) for s in ((M, K), (K, N), (N,)))
+    acts = sorted(ACT)
+    for i, off in enumerate((0, 1, 3)):
+        aligned = off == 0 and (N if transB else K) % 4 == 0
+        if not aligned and K < 384:
+            continue
+        act = acts[(i + M) % 4]
+        C = product(ctx, A, W, transA, transB, off, off, bias=bias, activation=act)
+        assert within(C, A, W, REL_3X, bias, act)
+        if i == 0:
+            assert within(product(ctx, A, W, transA, transB, mode=_lib.GEMM_TF32), A, W, REL_1X if aligned else REL_3X)
+            # bit for bit the same again
+            assert torch.equal(C, product(ctx, A, W, transA, transB, off, off, bias=bias, activation=act))
+
+
+@pytest.mark.parametrize("mode", [_lib.GEMM_3XTF32, _lib.GEMM_TF32])
+@pytest.mark.parametrize("transA,transB", [(False, False), (True, True)])
+@pytest.mark.parametrize("spread", ["few", "cell", "many"])
+def test_elements_the_parts_cannot_hold(ctx, spread, transA, transB, mode):
+    """Elements far below the largest of their 512 k, as the only ones that count: their row meets one nonzero weight per column (and
+    the other way round), and small ones of both operands meet.  few: scattered; cell: as many as a list holds in 16 x 512; many: more."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(7)
+    M, K, N = 600, 1536, 1100
+    gen = lambda *s: (torch.rand(s, device="cuda", generator=g) + 1) * torch.where(torch.rand(s, device="cuda", generator=g) < 0.5, -1.0, 1.0)
+    A, W = torch.zeros(M, K, device="cuda"), torch.zeros(K, N, device="cuda")
+    A[:, ::512], W[::512] = gen(M, 3) * 2.0 ** 30, 0.0          # the large activations opposite zeros
+    W[1::512], A[:, 1::512] = gen(3, N) * 2.0 ** 30, 0.0        # and the large weights
+    step = {"few": 64, "cell": 2, "many": 1}[spread]            # every 64th row: one in 16 x 512; every second: eight
+    k = torch.tensor([2, 514, 1030], device="cuda")
+    for s, e in enumerate((-12, -25, -45)):
+        A[s::step, k[s]] = (gen(M, 1) * 2.0 ** e).expand(M, 1)[s::step, 0]
+        W[k[s], s::step] = (gen(1, N) * 2.0 ** (e + 3))[0, s::step]
+    C = product(ctx, A, W, transA, transB, mode=mode)
+    ref = A.double() @ W.double()
+    some = ref != 0
+    rel = 2.7e-6 if mode == _lib.GEMM_3XTF32 else 2.0 ** -10 + 2.0 ** -11 + 2.0 ** -20
+    assert int(some.sum()) > 500
+    assert float(((C - ref)[some] / ref[some]).abs().max()) <= 3 * rel   # three terms at most
+    assert bool((C[~some] == 0).all())
+
+
+@pytest.mark.parametrize("spread", [0.0, 12.0])
+@pytest.mark.parametrize("transB", [False, True])
+def test_no_less_exact_than_the_streaming_kernel(ctx, spread, transB):
+    """2-norm of the error of both kernels on the same operands: normal, and log-normal over many binades (all by the streaming kernel)."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(3)
+    A, W = (torch.randn(s, device="cuda", generator=g) * torch.exp2(spread * torch.randn(s, device="cuda", generator=g)) for s in ((700, 4096), (4096, 1024)))
+    ref = A.double() @ W.double()
+    many = product(ctx, A, W, transB=transB)
+    ctx.lib.cn_gemm_set_tuning(ctx.h, 2, 0, 0)                      # the streaming kernel, as it cuts the product
+    try:
+        one = product(ctx, A, W, transB=transB, planes=False)
+    finally:
+        ctx.lib.cn_gemm_set_tuning(ctx.h, 0, 0, 0)
+    err = [float((c - ref).norm() / ref.norm()) for c in (many, one)]
+    assert err[0] <= 1.1 * err[1], err
+
+
+def test_non_finite_values_stay_in_their_row_and_column(ctx):
+    g = torch.Generator(device="cuda")
+    g.manual_seed(5)
+    A, W = torch.randn(600, 2000, device="cuda", generator=g), torch.randn(2000, 1028, device="cuda", generator=g)
+    clean = product(ctx, A, W)
+    A[7, 900], A[9, 1999], W[31, 3], W[1200, 600] = float("nan"), float("inf"), float("-inf"), float("nan")
+    C = product(ctx, A, W)
+    hit = torch.zeros(600, 1028, dtype=torch.bool, device="cuda")
+    hit[[7, 9]] = True
+    hit[:, [3, 600]] = True
+    assert not torch.isfinite(C[hit]).any()
+    assert torch.equal(C[~hit], clean[~hit])
+
+
+def test_recorded_in_a_graph(ctx):
+    """Replayed on other data, beyond what the lists hold."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(9)
+    A, W = torch.randn(1024, 640, device="cuda", generator=g), torch.randn(768, 1024, device="cuda", generator=g)   # (cols, rows)
+    C = torch.empty(768, 640, device="cuda")
+    ctx.gemm(A, W, out=C)
+    want = C.clone()
+    graph = torch.cuda.CUDAGraph()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side), torch.cuda.graph(graph, stream=side):
+        ctx.gemm(A, W, out=C)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(C, want)
+    A.mul_(torch.exp2(torch.randint(-30, 30, A.shape, device="cuda", generator=g).float()))
+    graph.replay()
+    torch.cuda.synchronize()
+    ref, bound = W.double() @ A.double(), REL_3X * (W.double().abs() @ A.double().abs())
+    assert bool(((C.double() - ref).abs() <= bound).all())
+
+
+def test_recorded_without_room_for_the_planes(ctx):
+    """A workspace that would have to grow while a graph is recorded: the streaming kernel, whose workspace is there, does the product."""
+    from clusternet_b200 import Context
+    g = torch.Generator(device="cuda")
+    g.manual_seed(9)
+    A, W, C = torch.randn(2048, 640, device="cuda", generator=g), torch.randn(1024, 2048, device="cuda", generator=g), torch.empty(1024, 640, device="cuda")
+    other = Context(0)
+    other.lib.cn_gemm_set_tuning(other.h, 2, 0, 0)
+    other.gemm(A, W, out=C)
+    other.lib.cn_gemm_set_tuning(other.h, 0, 0, 0)
+    want = C.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        other.gemm(A, W, out=C)
+    C.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(C, want)
+    del graph
+    other.gemm_check()
+    other.close()
