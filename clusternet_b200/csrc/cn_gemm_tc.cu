@@ -853,16 +853,13 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
             if (L <= 1) {
                 // every lane writes a column of its own: 32 bytes at a time fill whole sectors of L2, 16 half of one.  Product of
                 // 4096^3 alone: 475 us with 16-byte stores, 455 us with these.
+                // Rows beyond M are left out, and the logistic function, whose code is long, has a copy of the loop to itself: a pass
+                // through the other one is 128 additions and 16 stores, not a walk over 128 branches around it (16 x 248 . 248 x 35720 with
+                // logistic units: 36 us, 20 now; linear ones of 128 rows 27, 22).
                 const uintptr_t at = reinterpret_cast<uintptr_t>(dst);
                 const bool whole = m0 + TC_BM <= p.M, vec8 = whole && (at & 31u) == 0, vec4 = whole && (at & 15u) == 0;
-#pragma unroll
-                for (int i = 0; i < TC_BM; i += 8) {
-                    float v[8];
-#pragma unroll
-                    for (int e = 0; e < 8; e += 2) tc_unpack2(sum[(i + e) / 2], v[e], v[e + 1]);
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) v[e] = cn_apply_activation(p.bias ? v[e] + bias : v[e], p.act);
-                    if (n >= p.N) continue;
+                auto store8 = [&](int i, const float (&v)[8]) {
+                    if (n >= p.N) return;
                     if (vec8) {
                         stg8(dst + i, v);
                     } else if (vec4) {
@@ -872,6 +869,38 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
 #pragma unroll
                         for (int e = 0; e < 8; ++e)
                             if (m0 + i + e < p.M) dst[i + e] = v[e];
+                    }
+                };
+                if (p.act == CN_ACT_LOGISTIC) {
+#pragma unroll
+                    for (int i = 0; i < TC_BM; i += 8) {
+                        if (m0 + i >= p.M) break;
+                        float v[8];
+#pragma unroll
+                        for (int e = 0; e < 8; e += 2) tc_unpack2(sum[(i + e) / 2], v[e], v[e + 1]);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) v[e] = cn_apply_activation(p.bias ? v[e] + bias : v[e], CN_ACT_LOGISTIC);
+                        store8(i, v);
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < TC_BM; i += 8) {
+                        if (m0 + i >= p.M) break;
+                        float v[8];
+#pragma unroll
+                        for (int e = 0; e < 8; e += 2) tc_unpack2(sum[(i + e) / 2], v[e], v[e + 1]);
+                        if (p.bias) {
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) v[e] += bias;
+                        }
+                        if (p.act != CN_ACT_LINEAR) {
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) {
+                                v[e] = v[e] > 0.0f ? v[e] : 0.0f;
+                                if (p.act == CN_ACT_DOUBLE_RELU) v[e] = v[e] < 1.0f ? v[e] : 1.0f;
+                            }
+                        }
+                        store8(i, v);
                     }
                 }
                 __syncwarp();   // the next tile's tensor-memory loads need the whole warp
