@@ -238,8 +238,7 @@ int cn_gemm_dispatch(cn_context *ctx, int transA, int transB, int64_t M, int64_t
             transA = 1;
         }
         const bool push = peers && peers->npeers > 0 && L == 1;
-        st = cn_gemm_small_launch(ctx, transA, transB, M, N, K, d_A, lda, d_B, ldb, target, target_ld, epi, tc_mode, s, push ? peers : nullptr,
-                                  tma_ok);
+        st = cn_gemm_small_launch(ctx, transA, transB, M, N, K, d_A, lda, d_B, ldb, target, target_ld, epi, tc_mode, s, push ? peers : nullptr);
         if (push && used_peers) *used_peers = st == CN_OK;
     } else if (tc_ok) {
         cn_epilogue e2;

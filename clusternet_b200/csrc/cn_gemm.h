@@ -108,7 +108,7 @@ bool cn_gemm_small_shape(const cn_context *ctx, int64_t M, int64_t N, int64_t K,
 // K blocks of 32 per accumulation chain for weights whose rows TMA cannot read (cn_gemm_tc.cu)
 int cn_gemm_any_chain(int64_t K);
 int cn_gemm_small_launch(cn_context *ctx, int transA, int transB, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, const float *B, int64_t ldb,
-                         float *C, int64_t ldc, const cn_epilogue *epi, int mode, cudaStream_t s, const cn_peer_out *peers, bool w_aligned);
+                         float *C, int64_t ldc, const cn_epilogue *epi, int mode, cudaStream_t s, const cn_peer_out *peers);
 // cn_gemm_f32 with optional peer windows; *used_peers tells whether the launch took them (tensor-core path only).  planes_ok: the
 // kernel for many rows may be taken.  The sharded products stay with the streaming kernel, whose bits do not depend on whether
 // the activations' planes were made ahead or the output goes to peers.

@@ -4,43 +4,61 @@
 // right price for weights that have to come from HBM.  A layer of a small network (128 x 784 . 784 x 1024, the weight gradients
 // and back-propagated errors of a 784-1200-1200-10 network) is over in a few microseconds; there the launches, the passes
 // over memory between them and the idle SMs of a product with eight tiles are the cost.  Here
-//   * a CTA takes a tile of 128 columns n by up to 128 rows m and a share of K.  Four warps load and split 128 x 32 blocks of
-//     the weights, four those of the activations, straight from global memory in whatever layout they have (either operand
-//     transposed or not, any alignment), with the next block's loads in flight while the current one is split;
+//   * a CTA takes a tile of 128 rows m by NT = 32, 64 or 128 columns n and a share of K.  Eight warps each load and split blocks of 32 k of
+//     the activations and the weights, straight from global memory in whatever layout they have (either operand transposed or not, any
+//     alignment), three blocks of loads in flight;
 //   * the operands are TF32 hi / lo parts in shared memory (K-major, 128-byte swizzle), three tcgen05.mma kind::tf32 products per
 //     k-step as CN_GEMM_3XTF32 promises, one for CN_GEMM_TF32; one thread issues them;
-//   * the CTAs of a cluster share a tile: each multiplies its part of K, sends every other CTA its slice of the partial tile
-//     through distributed shared memory, adds the slices it received in K order (reproducible), and finishes its slice: bias,
-//     activation, 512-byte runs of stores to C and, for the fused all-gather, to the peers.
-// The tensor core's accumulator truncates, so a share of K (at most SM_MAX_BLOCKS_ANY blocks) is cut into as many chains as tensor memory
-// holds accumulators for, four, and the chains are added in round-to-nearest fp32.
+//   * the accumulator tile has the rows m in tensor memory's lanes, so that a warp holds 32 consecutive rows of a column: it sends
+//     and stores whole lines of 128 bytes without turning anything;
+//   * the CTAs of a cluster share a tile: each multiplies its part of K, sends every other CTA its columns of the partial tile
+//     through distributed shared memory, adds the parts it received in K order (reproducible), and finishes its columns: bias,
+//     activation, stores to C and, for the fused all-gather, to the peers.
+// The tensor core's accumulator truncates, so a share of K is cut into as many chains as tensor memory holds accumulators for, and the
+// chains are added in round-to-nearest fp32.  The products with a low part have accumulators of their own, which costs no instruction (one
+// MMA multiplies the activations' high parts with both parts of the weights, whose rows lie behind one another): an addition
+// truncates what it adds to a large sum.
 //
-// Bound by latency.  128 x 784 . 784 x 1024 + bias + ReLU: 13.2 us a call, against 22.5 us in three launches.
+// Bound by latency and, per block of K, by the instructions that load and split it and the MMAs' trips to shared memory (0.7 us).  In a
+// series, with tiles of 128 columns n in the lanes, partial tiles of 64 KB through the cluster and output by way of shared memory before:
+// 128 x 784 . 784 x 1024 14.3 -> 10.9 us, 128 x 1200 . 1200 x 10 13.5 -> 7.4, weight gradient 1200 x 128 . 128 x 1200 16.3 -> 9.0.
 #include "cn_epilogue.cuh"
 #include "cn_gemm.h"
 #include "cn_tc.cuh"
 
-#define SM_BN 128
 #define SM_BM 128
 #define SM_BK 32
-#define SM_THREADS 288          // warps 0-3: weights, 4-7: activations, 8: MMA issuer
+#define SM_FEED 256             // threads that load and split an operand: warps 0-7 the activations, 8-15 the weights; all of them the epilogue
+#define SM_EPI (2 * SM_FEED)
+#define SM_THREADS (SM_EPI + 32)   // warp 16: MMA issuer
 #define SM_STAGES 2
-#define SM_TILE_BYTES (128 * 128)
-#define SM_STAGE_BYTES (4 * SM_TILE_BYTES)   // W hi, W lo, A hi, A lo
+#define SM_AHEAD 3              // blocks of loads in flight
+#define SM_A_TILE (SM_BM * 128)
 #define SM_MAX_BLOCKS 12
 #define SM_MAX_BLOCKS_ANY 16   // weights that TMA cannot read, of which the streaming kernel wants four rows at least
-#define SM_MAX_CHAINS 4
 #define SM_MAX_CLUSTER 8
-#define SM_RING_BYTES (SM_STAGES * SM_STAGE_BYTES)
-#define SM_TURN_BYTES (SM_BN * SM_BM * 4)
-#define SM_SMEM_BYTES(cluster) (1024 + SM_RING_BYTES + ((cluster) > 1 ? SM_TURN_BYTES : 0))
 
-// How an operand lies in memory: k contiguous with 16-byte rows, k contiguous otherwise, or the tile's rows contiguous.
-enum { SM_K_VEC = 0, SM_K_SCALAR = 1, SM_ROWS = 2 };
+template <int NT, bool MODE3X>
+struct SmCfg {
+    static constexpr int W_TILE = NT * 128;
+    static constexpr int STAGE_BYTES = 2 * (SM_A_TILE + W_TILE);   // A hi, A lo, W hi, W lo
+    static constexpr int RING_BYTES = SM_STAGES * STAGE_BYTES;
+    static constexpr int PART_BYTES = SM_BM * NT * 4;              // what the cluster's CTAs send: [sender][column][128 m]
+    // An accumulator has NT columns for the products of the high parts and, in the 3x mode, NT for those with a low part
+    static constexpr int ACC_COLS = MODE3X ? 2 * NT : NT;
+    static constexpr int MAX_CHAINS = 512 / ACC_COLS < 8 ? 512 / ACC_COLS : 8;
+    static constexpr int smem(int cluster) { return 1024 + RING_BYTES + (cluster > 1 ? PART_BYTES : 0); }
+};
+
+// An operand: element (row, k) at p[row * sr + k * sk].
+struct SmOperand {
+    const float *p;
+    int64_t sr, sk;
+    int vec;                // 16-byte aligned along the contiguous one of the two
+};
 
 struct SmallParams {
-    const float *W, *A;
-    int64_t ldw, lda;
+    SmOperand A, W;
     int64_t M, N, K;
     float *C;
     int64_t ldc;
@@ -49,7 +67,6 @@ struct SmallParams {
     int tiles_m;
     int cluster;
     int kb_total;
-    int fine_chains;      // chains end between k-steps of 8, not blocks (see cn_gemm_small_launch)
     unsigned int *status;
     int npeers;
     float *peerC[CN_MAX_PEERS];
@@ -87,154 +104,237 @@ __device__ __forceinline__ void sm_mma_ss(uint32_t d_tmem, uint32_t a_lo, uint32
         ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate) : "memory");
 }
 
-// One 128 x 32 block of an operand, spread over 128 threads: 32 values per thread.
-// `rows`: rows of the tile that exist; everything else reads as zero.
-template <int KIND>
-__device__ __forceinline__ void sm_load(const float *base, int64_t ld, int rows, int64_t k0, int64_t K, int t, float (&x)[32])
-{
-    if (KIND == SM_K_VEC) {   // eight lanes per row (128 bytes), sixteen rows per pass
-        const int c = t & 7;
-        const int64_t k = k0 + 4 * c;
+// The share of one thread of a block of ROWS x 32 k: up to four 16-byte chunks (a chunk is four consecutive k of a row).
+// QUADS false: chunks of rows 32 apart; with k contiguous, eight lanes read a row's 128 bytes, 16 at a time where the rows are aligned;
+// else (rows contiguous but not aligned) a chunk's four elements are read one by one.
+// QUADS true (rows contiguous and aligned): four rows by four k, read 16 bytes at a time along the rows and turned in registers.
+// Lanes: two quads of rows, eight chunks, two quads again, so that eight lanes that store together meet in no bank.
+template <int ROWS, bool QUADS>
+struct SmShare {
+    static constexpr int CHUNKS = QUADS ? 4 : ROWS * 8 / SM_FEED;
+    const float *src;       // the first element of chunk 0 (QUADS: of row 4 q)
+    int64_t sr, sk;
+    int row0, c0, rows;
+    bool vec;
+    // t: 0 .. SM_FEED - 1
+    __device__ __forceinline__ SmShare(const SmOperand &o, int64_t first_row, int rows_here, int t)
+    {
+        vec = o.vec;
+        rows = rows_here;
+        sr = o.sr;
+        sk = o.sk;
+        if (QUADS) {
+            row0 = 4 * ((t & 1) | (t >> 3 & 2) | (t >> 5 << 2));
+            c0 = t >> 1 & 7;
+        } else if (o.sk == 1) {
+            row0 = t >> 3;
+            c0 = t & 7;
+        } else {   // a warp reads 32 rows
+            row0 = t & 31;
+            c0 = t >> 5;
+        }
+        src = o.p + (first_row + row0) * o.sr + 4 * c0 * o.sk;
+    }
+    __device__ __forceinline__ bool mine() const { return !QUADS || row0 < ROWS; }
+    __device__ __forceinline__ void load(int64_t k0, int64_t K, float4 (&x)[CHUNKS]) const
+    {
+        const float *q = src + k0 * sk;
+        const int left = (int)(K - k0 < SM_BK ? K - k0 : SM_BK) - 4 * c0;   // k of this chunk that exist
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int r = i * 16 + (t >> 3);
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (r < rows) {
-                const float *p = base + (int64_t)r * ld + k;
-                if (k + 3 < K) {
-                    v = *reinterpret_cast<const float4 *>(p);
-                } else {
-                    if (k < K) v.x = p[0];
-                    if (k + 1 < K) v.y = p[1];
-                    if (k + 2 < K) v.z = p[2];
+        for (int i = 0; i < CHUNKS; ++i) x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (QUADS) {
+            if (left >= 4 && row0 + 3 < rows) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) x[e] = *reinterpret_cast<const float4 *>(q + e * sk);
+            } else if (mine()) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    if (e >= left) continue;
+                    if (row0 < rows) x[e].x = q[e * sk];
+                    if (row0 + 1 < rows) x[e].y = q[e * sk + 1];
+                    if (row0 + 2 < rows) x[e].z = q[e * sk + 2];
+                    if (row0 + 3 < rows) x[e].w = q[e * sk + 3];
                 }
             }
-            x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
+        } else if (vec && left >= 4 && sk == 1) {
+#pragma unroll
+            for (int i = 0; i < CHUNKS; ++i)
+                if (row0 + 32 * i < rows) x[i] = *reinterpret_cast<const float4 *>(q + 32 * i * sr);
+        } else {
+#pragma unroll
+            for (int i = 0; i < CHUNKS; ++i) {
+                if (row0 + 32 * i >= rows) continue;
+                if (left > 0) x[i].x = q[32 * i * sr];
+                if (left > 1) x[i].y = q[32 * i * sr + sk];
+                if (left > 2) x[i].z = q[32 * i * sr + 2 * sk];
+                if (left > 3) x[i].w = q[32 * i * sr + 3 * sk];
+            }
         }
-    } else if (KIND == SM_K_SCALAR) {   // one row (128 bytes) per warp and pass
-        const int64_t k = k0 + (t & 31);
-        const float *p = base + (int64_t)(t >> 5) * ld + k;
-        const bool in_k = k < K;
-#pragma unroll
-        for (int i = 0; i < 32; ++i) x[i] = (in_k && i * 4 + (t >> 5) < rows) ? p[(int64_t)(i * 4) * ld] : 0.0f;
-    } else {   // one row per thread, consecutive threads on consecutive rows
-        const float *p = base + t + k0 * ld;
-        const bool in_r = t < rows;
-#pragma unroll
-        for (int i = 0; i < 32; ++i) x[i] = (in_r && k0 + i < K) ? p[(int64_t)i * ld] : 0.0f;
     }
-}
-
-// Whether sm_tf32 has to be CAREFUL with some of the values.
-__device__ __forceinline__ bool sm_unsafe(const float (&x)[32])
-{
-    float m = 0.0f;
+    // TF32 parts into shared memory: 16-byte chunk c of row r lies at r * 128 + ((c ^ (r & 7)) << 4).
+    template <bool MODE3X, bool CAREFUL>
+    __device__ __forceinline__ void put(uint32_t hi, uint32_t lo, const float4 (&x)[CHUNKS]) const
+    {
 #pragma unroll
-    for (int i = 0; i < 32; i += 2) asm("max.NaN.abs.f32 %0, %1, %2, %0;" : "+f"(m) : "f"(x[i]), "f"(x[i + 1]));
-    return !(m < __uint_as_float(0x7f7ff000u));
-}
-
-// The same block -> TF32 parts in shared memory: 16-byte chunk c of row r lies at r * 128 + ((c ^ (r & 7)) << 4).
-template <int KIND, bool MODE3X, bool CAREFUL>
-__device__ __forceinline__ void sm_store(uint32_t hi, uint32_t lo, int need_rows, int t, const float (&x)[32])
-{
-    if (KIND == SM_K_SCALAR) {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-            const int r = i * 4 + (t >> 5), kk = t & 31;
-            if (r >= need_rows) continue;
-            const uint32_t at = (uint32_t)(r * 128 + (((kk >> 2) ^ (r & 7)) << 4) + (kk & 3) * 4);
-            const uint32_t h = sm_tf32<CAREFUL>(x[i]);
-            sts1u(hi + at, h);
-            if (MODE3X) sts1u(lo + at, sm_tf32<CAREFUL>(x[i] - __uint_as_float(h)));
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int r = KIND == SM_K_VEC ? i * 16 + (t >> 3) : t, c = KIND == SM_K_VEC ? (t & 7) : i;
-            if (r >= need_rows) continue;
-            const uint32_t at = (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4));
+        for (int i = 0; i < CHUNKS; ++i) {
+            const int r = row0 + (QUADS ? i : 32 * i);
+            const uint32_t at = (uint32_t)(r * 128 + ((c0 ^ (r & 7)) << 4));
+            auto of = [](const float4 &v, int e) { return e == 0 ? v.x : e == 1 ? v.y : e == 2 ? v.z : v.w; };
+            float y[4];
             uint32_t h[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) h[e] = sm_tf32<CAREFUL>(x[4 * i + e]);
+            for (int e = 0; e < 4; ++e) {
+                y[e] = QUADS ? of(x[QUADS ? e : 0], i) : of(x[i], e);
+                h[e] = sm_tf32<CAREFUL>(y[e]);
+            }
             sts4u(hi + at, h[0], h[1], h[2], h[3]);
             if (MODE3X)
-                sts4u(lo + at, sm_tf32<CAREFUL>(x[4 * i] - __uint_as_float(h[0])), sm_tf32<CAREFUL>(x[4 * i + 1] - __uint_as_float(h[1])),
-                      sm_tf32<CAREFUL>(x[4 * i + 2] - __uint_as_float(h[2])), sm_tf32<CAREFUL>(x[4 * i + 3] - __uint_as_float(h[3])));
+                sts4u(lo + at, sm_tf32<CAREFUL>(y[0] - __uint_as_float(h[0])), sm_tf32<CAREFUL>(y[1] - __uint_as_float(h[1])),
+                      sm_tf32<CAREFUL>(y[2] - __uint_as_float(h[2])), sm_tf32<CAREFUL>(y[3] - __uint_as_float(h[3])));
         }
     }
-}
+    template <bool MODE3X>
+    __device__ __forceinline__ void store(uint32_t hi, uint32_t lo, const float4 (&x)[CHUNKS]) const
+    {
+        if (!mine()) return;
+        float m = 0.0f;   // whether sm_tf32 has to be careful with some of the values
+#pragma unroll
+        for (int i = 0; i < CHUNKS; ++i) {
+            asm("max.NaN.abs.f32 %0, %1, %2, %0;" : "+f"(m) : "f"(x[i].x), "f"(x[i].y));
+            asm("max.NaN.abs.f32 %0, %1, %2, %0;" : "+f"(m) : "f"(x[i].z), "f"(x[i].w));
+        }
+        if (m < __uint_as_float(0x7f7ff000u)) put<MODE3X, false>(hi, lo, x);
+        else put<MODE3X, true>(hi, lo, x);
+    }
+};
+
+// Blocks kb0 .. kb0 + n - 1 of one operand's tile into the ring.  begin() issues the first loads, run() does the rest.
+template <class Share, bool MODE3X>
+struct SmFeed {
+    const Share share;
+    float4 x[SM_AHEAD][Share::CHUNKS];
+    __device__ __forceinline__ SmFeed(const SmOperand &o, int64_t first_row, int rows, int t) : share(o, first_row, rows, t) {}
+    __device__ __forceinline__ void begin(int kb0, int n, int64_t K)
+    {
+#pragma unroll
+        for (int u = 0; u < SM_AHEAD; ++u)
+            if (u < n) share.load((int64_t)(kb0 + u) * SM_BK, K, x[u]);
+    }
+    __device__ __forceinline__ bool run(int kb0, int n, int64_t K, uint32_t ring, int stage_bytes, uint32_t hi_off, uint32_t lo_off, uint32_t full0, uint32_t empty0,
+                                        uint32_t abort_flag, unsigned int *status)
+    {
+        bool ok = true;
+        for (int i0 = 0; i0 < n && ok; i0 += SM_AHEAD) {
+#pragma unroll
+            for (int u = 0; u < SM_AHEAD; ++u) {
+                const int i = i0 + u, s = i & 1;
+                if (i >= n || !ok) continue;
+                ok = mbar_wait(empty0 + 8 * s, ((uint32_t)(i >> 1) & 1u) ^ 1u, abort_flag, status, 14u);
+                if (!ok) continue;
+                const uint32_t stage = ring + s * stage_bytes;
+                share.template store<MODE3X>(stage + hi_off, stage + lo_off, x[u]);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if ((threadIdx.x & 31) == 0) mbar_arrive(full0 + 8 * s);
+                if (i + SM_AHEAD < n) share.load((int64_t)(kb0 + i + SM_AHEAD) * SM_BK, K, x[u]);
+            }
+        }
+        return ok;
+    }
+};
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
-// The loading side of one operand: blocks kb0 .. kb1 - 1 of its tile into the ring.
-template <int KIND, bool MODE3X>
-__device__ __forceinline__ bool sm_feed(const float *base, int64_t ld, int rows, int need_rows, int64_t K, int kb0, int kb1, int t, uint32_t ring,
-                                        uint32_t operand_off, uint32_t full0, uint32_t empty0, uint32_t abort_flag, unsigned int *status)
+__device__ __forceinline__ void sm_ld8(uint32_t taddr, uint32_t *r)
 {
-    float x[2][32];
-    const int n = kb1 - kb0;
-    bool ok = true;
-    sm_load<KIND>(base, ld, rows, (int64_t)kb0 * SM_BK, K, t, x[0]);
-    for (int i0 = 0; i0 < n && ok; i0 += 2) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+}
+// Eight columns of the accumulators of all chains, in K order, the products with a low part last.  Up to four accumulators are loaded
+// before the wait.
+template <int NT, bool MODE3X>
+__device__ __forceinline__ void sm_sum8(uint32_t taddr, int chains, float (&v)[8])
+{
+    using Cfg = SmCfg<NT, MODE3X>;
+    constexpr int PARTS = MODE3X ? 2 : 1, GROUP = Cfg::MAX_CHAINS < 4 ? Cfg::MAX_CHAINS : 4;
+    float low[8];
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-            const int i = i0 + u;
-            if (i >= n || !ok) continue;
-            if (i + 1 < n) sm_load<KIND>(base, ld, rows, (int64_t)(kb0 + i + 1) * SM_BK, K, t, x[u ^ 1]);
-            const bool unsafe = sm_unsafe(x[u]);
-            ok = mbar_wait(empty0 + 8 * u, ((uint32_t)(i >> 1) & 1u) ^ 1u, abort_flag, status, 14u);
-            if (!ok) continue;
-            const uint32_t hi = ring + u * SM_STAGE_BYTES + operand_off;
-            if (unsafe) sm_store<KIND, MODE3X, true>(hi, hi + SM_TILE_BYTES, need_rows, t, x[u]);
-            else        sm_store<KIND, MODE3X, false>(hi, hi + SM_TILE_BYTES, need_rows, t, x[u]);
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if ((t & 31) == 0) mbar_arrive(full0 + 8 * u);
+    for (int c = 0; c < 8; ++c) v[c] = low[c] = 0.0f;
+#pragma unroll 1
+    for (int ch0 = 0; ch0 < chains; ch0 += GROUP) {
+        uint32_t r[GROUP][PARTS][8];
+#pragma unroll
+        for (int ch = 0; ch < GROUP; ++ch) {
+            if (ch0 + ch >= chains) break;
+#pragma unroll
+            for (int part = 0; part < PARTS; ++part) sm_ld8(taddr + (ch0 + ch) * Cfg::ACC_COLS + part * NT, r[ch][part]);
+        }
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int ch = 0; ch < GROUP; ++ch) {
+            if (ch0 + ch >= chains) break;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+#pragma unroll
+                for (int part = 0; part < PARTS; ++part) asm volatile("" : "+r"(r[ch][part][c]));   // no use moves before the wait
+                v[c] += __uint_as_float(r[ch][0][c]);
+                if (MODE3X) low[c] += __uint_as_float(r[ch][PARTS - 1][c]);
+            }
         }
     }
-    return ok;
+    if (MODE3X) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) v[c] += low[c];
+    }
 }
 
-template <int WKIND, int AKIND, bool MODE3X>
+// Peers must have announced that their copy of C may be overwritten (bounded wait).
+__device__ __forceinline__ void sm_wait_peers(const SmallParams &p)
+{
+    const long long t0 = clock64();
+    for (int r = 0; r < p.nranks; ++r) {
+        if (r == p.my_rank) continue;
+        const volatile unsigned int *f = p.ready + r;
+        while ((int)(*f - p.epoch) < 0) {
+            if (clock64() - t0 > TC_WAIT_LIMIT) { atomicMax(p.status, 9u); break; }
+            __nanosleep(100);
+        }
+    }
+}
+
+template <int NT, bool MODE3X, bool A_QUADS, bool W_QUADS>
 __global__ void __launch_bounds__(SM_THREADS, 1)
 cn_gemm_small_kernel(const __grid_constant__ SmallParams p)
 {
+    using Cfg = SmCfg<NT, MODE3X>;
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t bars[2 * SM_STAGES + 1];
     __shared__ uint32_t s_words[2];   // tensor-memory base, abort flag
-    const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    __shared__ float s_bias[NT];
+    const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u, part = ring + Cfg::RING_BYTES;
     const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[SM_STAGES]), acc_bar = smem_u32(&bars[2 * SM_STAGES]);
     const uint32_t abort_flag = smem_u32(&s_words[1]);
-    const uint32_t turn = p.cluster > 1 ? ring + SM_RING_BYTES : ring;   // partial-tile slices; with one CTA per tile the idle ring serves
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = blockIdx.x % p.cluster, tile = blockIdx.x / p.cluster;
-    const int64_t m0 = (int64_t)(tile % p.tiles_m) * SM_BM, n0 = (int64_t)(tile / p.tiles_m) * SM_BN;
-    const int m_rows = (int)(p.M - m0 < SM_BM ? p.M - m0 : SM_BM), n_rows = (int)(p.N - n0 < SM_BN ? p.N - n0 : SM_BN);
-    const int m_need = (m_rows + 15) & ~15;   // UMMA N
-    const int kb0 = (int)((int64_t)p.kb_total * rank / p.cluster), kb1 = (int)((int64_t)p.kb_total * (rank + 1) / p.cluster);
-    // accumulation chains, in k-steps of 8
-    const int steps = (kb1 - kb0) * (SM_BK / 8);
-    const int chain_steps = p.fine_chains ? (steps + SM_MAX_CHAINS - 1) / SM_MAX_CHAINS : (kb1 - kb0 + SM_MAX_CHAINS - 1) / SM_MAX_CHAINS * (SM_BK / 8);
-    const int chains = (steps + chain_steps - 1) / chain_steps;
+    const int64_t m0 = (int64_t)(tile % p.tiles_m) * SM_BM, n0 = (int64_t)(tile / p.tiles_m) * NT;
+    const int m_rows = (int)(p.M - m0 < SM_BM ? p.M - m0 : SM_BM), n_rows = (int)(p.N - n0 < NT ? p.N - n0 : NT);
+    const int kb0 = p.kb_total * rank / p.cluster, n_blocks = p.kb_total * (rank + 1) / p.cluster - kb0;
+    const int per_chain = (n_blocks + Cfg::MAX_CHAINS - 1) / Cfg::MAX_CHAINS, chains = (n_blocks + per_chain - 1) / per_chain;
     cn_pdl_launch_dependents();
     if (p.cluster > 1) cluster_arrive();   // every CTA of the cluster has started: waited for before the first remote store
     if (threadIdx.x == 0) {
-        for (int s = 0; s < SM_STAGES; ++s) { mbar_init(full0 + 8 * s, 8); mbar_init(empty0 + 8 * s, 1); }
+        for (int s = 0; s < SM_STAGES; ++s) { mbar_init(full0 + 8 * s, SM_EPI / 32); mbar_init(empty0 + 8 * s, 1); }
         mbar_init(acc_bar, 1);
         s_words[1] = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    const uint32_t cols = chains == 1 ? 128u : chains == 2 ? 256u : 512u;
-    if (warp == 8) {
+    uint32_t cols = 32;
+    while (cols < (uint32_t)(chains * Cfg::ACC_COLS)) cols <<= 1;
+    if (warp == 16) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_words[0])), "r"(cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = s_words[0];
     cn_pdl_wait();
     if (p.npeers > 0 && blockIdx.x == 0 && threadIdx.x < p.nranks && (int)threadIdx.x != p.my_rank) {
         // fused all-gather: this rank's copy of C may be overwritten by its peers (slot 0 of their flag block)
@@ -242,132 +342,190 @@ cn_gemm_small_kernel(const __grid_constant__ SmallParams p)
         volatile unsigned int *f = p.peer_flags[threadIdx.x] + p.my_rank;
         *f = p.epoch;
     }
+    // the first loads are on their way while the CTA sets itself up
     bool ok = true;
-    if (warp < 4) {
-        const float *base = WKIND == SM_ROWS ? p.W + n0 : p.W + n0 * p.ldw;
-        ok = sm_feed<WKIND, MODE3X>(base, p.ldw, n_rows, SM_BN, p.K, kb0, kb1, threadIdx.x, ring, 0, full0, empty0, abort_flag, p.status);
-    } else if (warp < 8) {
-        const float *base = AKIND == SM_ROWS ? p.A + m0 : p.A + m0 * p.lda;
-        ok = sm_feed<AKIND, MODE3X>(base, p.lda, m_rows, m_need, p.K, kb0, kb1, threadIdx.x - 128, ring, 2 * SM_TILE_BYTES, full0, empty0, abort_flag,
-                                    p.status);
-    } else if (lane == 0) {
+    uint32_t tmem = 0u;
+    auto set_up = [&]() {
+        if (threadIdx.x < NT) s_bias[threadIdx.x] = p.bias && (int)threadIdx.x < n_rows ? p.bias[n0 + threadIdx.x] : 0.0f;
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+        tmem = s_words[0];
+    };
+    if (warp < 8) {
+        SmFeed<SmShare<SM_BM, A_QUADS>, MODE3X> feed(p.A, m0, m_rows, threadIdx.x);
+        feed.begin(kb0, n_blocks, p.K);
+        set_up();
+        ok = feed.run(kb0, n_blocks, p.K, ring, Cfg::STAGE_BYTES, 0, SM_A_TILE, full0, empty0, abort_flag, p.status);
+    } else if (warp < 16) {
+        SmFeed<SmShare<NT, W_QUADS>, MODE3X> feed(p.W, n0, n_rows, threadIdx.x - SM_FEED);
+        feed.begin(kb0, n_blocks, p.K);
+        set_up();
+        ok = feed.run(kb0, n_blocks, p.K, ring, Cfg::STAGE_BYTES, 2 * SM_A_TILE, 2 * SM_A_TILE + Cfg::W_TILE, full0, empty0, abort_flag, p.status);
+    } else {
+        set_up();
+    }
+    if (warp == 16 && lane == 0) {
         // kind::tf32 instruction descriptor: D fp32, A and B TF32 (format 2), K-major, N >> 3 at bits 17-22, M >> 4 at bits 24-28
-        const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(m_need >> 3) << 17) | ((uint32_t)(SM_BN >> 4) << 24);
-        const int n = kb1 - kb0;
-        uint32_t acc = tmem;
+        const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(SM_BM >> 4) << 24);
+        const uint32_t idesc2 = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(Cfg::ACC_COLS >> 3) << 17) | ((uint32_t)(SM_BM >> 4) << 24);
         int in_chain = 0;
-        for (int i = 0; i < n; ++i) {
+        uint32_t acc = tmem;
+        for (int i = 0; i < n_blocks; ++i) {
             const int s = i & 1;
             ok = mbar_wait(full0 + 8 * s, (uint32_t)(i >> 1) & 1u, abort_flag, p.status, 15u);
             if (!ok) break;
             tc_fence_after();
-            const uint64_t d = make_kmajor_sw128_desc(ring + s * SM_STAGE_BYTES);
-            const uint32_t hi = (uint32_t)(d >> 32), whi = (uint32_t)d, wlo = whi + (SM_TILE_BYTES >> 4), ahi = wlo + (SM_TILE_BYTES >> 4),
-                           alo = ahi + (SM_TILE_BYTES >> 4);
+            const uint64_t d = make_kmajor_sw128_desc(ring + s * Cfg::STAGE_BYTES);
+            const uint32_t hi = (uint32_t)(d >> 32), ahi = (uint32_t)d, alo = ahi + (SM_A_TILE >> 4), w = alo + (SM_A_TILE >> 4);
+            if (in_chain == per_chain) { in_chain = 0; acc += Cfg::ACC_COLS; }
+            const bool first = in_chain++ == 0;
 #pragma unroll
             for (int j = 0; j < SM_BK / 8; ++j) {   // 8 TF32 per k-step: 32 bytes (descriptor units of 16 B)
-                if (in_chain == chain_steps) { in_chain = 0; acc += SM_BM; }
-                sm_mma_ss(acc, whi + 2 * j, ahi + 2 * j, hi, idesc, in_chain++ != 0 ? 1u : 0u);
-                if (MODE3X) {
-                    sm_mma_ss(acc, wlo + 2 * j, ahi + 2 * j, hi, idesc, 1u);
-                    sm_mma_ss(acc, whi + 2 * j, alo + 2 * j, hi, idesc, 1u);
-                }
+                // the weights' low rows lie behind the high ones: one instruction multiplies both with the activations' high parts
+                sm_mma_ss(acc, ahi + 2 * j, w + 2 * j, hi, idesc2, first && j == 0 ? 0u : 1u);
+                if (MODE3X) sm_mma_ss(acc + NT, alo + 2 * j, w + 2 * j, hi, idesc, 1u);
             }
             tc_commit(empty0 + 8 * s);
         }
         if (ok) tc_commit(acc_bar);
     }
     __syncwarp();
-    const int R = SM_BN / p.cluster;   // columns n this CTA finishes
-    if (warp < 8) {
+    const int r_log = 31 - __clz(NT / p.cluster), R = 1 << r_log;   // columns n this CTA finishes
+    if (p.cluster > 1) {
+        cluster_wait();
+    } else if (p.npeers > 0) {
+        if (threadIdx.x == 0) sm_wait_peers(p);
+        __syncthreads();
+    }
+    if (warp < 16) {
         ok = ok && mbar_wait(acc_bar, 0u, abort_flag, p.status, 16u);
         ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
-    }
-    if (p.cluster > 1) cluster_wait();
-    else __syncthreads();              // the ring is about to be overwritten: every warp has seen the last MMA retire
-    if (warp < 8 && ok) {
-        // warps w and w + 4 share a lane quarter and take 64 rows m each
-        const int n_l = (warp & 3) * 32 + lane, col0 = (warp >> 2) * 64;
-        const int dst = n_l / R, i = n_l - dst * R;
-        uint32_t slice = turn + (uint32_t)((rank * R + i) * SM_BM) * 4;
-        if (p.cluster > 1) asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(slice) : "r"(slice), "r"(dst));
-        const uint32_t src = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+        if (ok) {
+            // four warps share a lane quarter and take a quarter of the columns each
+            const int ml = (warp & 3) * 32 + lane, col0 = (warp >> 2) * (NT / 4);
+            const int64_t m = m0 + ml;
+            const uint32_t src = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+            const bool plain = p.act == CN_ACT_LINEAR && p.npeers == 0;
+#pragma unroll 1
+            for (int col = col0; col < col0 + NT / 4 && col < n_rows; col += 8) {
+                float v[8];
+                sm_sum8<NT, MODE3X>(src + col, chains, v);
+                if (p.cluster > 1) {
 #pragma unroll
-        for (int cc = 0; cc < 4; ++cc) {
-            const int col = col0 + cc * 16;
-            if (col >= m_need) break;
-            uint32_t r[16];
-            tc_ld16(src + col, r);
-            for (int ch = 1; ch < chains; ++ch) {
-                uint32_t q[16];
-                tc_ld16(src + ch * SM_BM + col, q);
+                    for (int e = 0; e < 8; ++e) {
+                        const int dst = (col + e) >> r_log, i = (col + e) & (R - 1);
+                        uint32_t at = part + (uint32_t)((rank * R + i) * SM_BM + ml) * 4;
+                        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(at), "r"(dst));
+                        asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(at), "f"(v[e]) : "memory");
+                    }
+                } else if (m < p.M) {
+                    float *q = p.C + (n0 + col) * p.ldc + m;
+                    const int cols_here = n_rows - col < 8 ? n_rows - col : 8;
+                    if (p.bias) {
 #pragma unroll
-                for (int e = 0; e < 16; ++e) r[e] = __float_as_uint(__uint_as_float(r[e]) + __uint_as_float(q[e]));
-            }
+                        for (int e = 0; e < 8; ++e) v[e] += s_bias[col + e];
+                    }
+                    if (plain) {
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {   // 16-byte chunk col/4 + c of the row, chunks permuted by the row against bank conflicts
-                const uint32_t at = slice + ((uint32_t)((col / 4 + c) ^ (i & 7)) << 4);
-                if (p.cluster > 1)
-                    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(r[4 * c]), "r"(r[4 * c + 1]), "r"(r[4 * c + 2]), "r"(r[4 * c + 3]) : "memory");
-                else
-                    sts4u(at, r[4 * c], r[4 * c + 1], r[4 * c + 2], r[4 * c + 3]);
+                        for (int e = 0; e < 8; ++e, q += p.ldc)
+                            if (e < cols_here) *q = v[e];
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e, q += p.ldc) {
+                            if (e >= cols_here) continue;
+                            const float a = cn_apply_activation(v[e], p.act);
+                            *q = a;
+                            for (int d = 0; d < p.npeers; ++d) p.peerC[d][(n0 + col + e) * p.ldc + m] = a;
+                        }
+                    }
+                }
             }
         }
     }
+    __syncwarp();
     tc_fence_before();
     if (p.cluster > 1) { cluster_arrive(); cluster_wait(); }
     else __syncthreads();
-    if (warp == 8) {
+    if (warp == 16) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
         return;
     }
-    if (p.npeers > 0) {   // peers must have announced that their copy of C may be overwritten (bounded wait)
-        if (threadIdx.x == 0) {
-            const long long t0 = clock64();
-            for (int r = 0; r < p.nranks; ++r) {
-                if (r == p.my_rank) continue;
-                const volatile unsigned int *f = p.ready + r;
-                while ((int)(*f - p.epoch) < 0) {
-                    if (clock64() - t0 > TC_WAIT_LIMIT) { atomicMax(p.status, 9u); break; }
-                    __nanosleep(100);
-                }
-            }
-        }
-        asm volatile("bar.sync 1, 256;" ::: "memory");
+    if (p.cluster == 1) return;
+    if (p.npeers > 0) {
+        if (threadIdx.x == 0) sm_wait_peers(p);
+        asm volatile("bar.sync 1, %0;" ::"n"(SM_EPI) : "memory");
     }
-    // this CTA's slice: column n0 + rank * R + i, four rows m per lane
-    const int64_t m = m0 + lane * 4;
-    const bool vec = (m + 4 <= p.M) && ((p.ldc & 3) == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15u) == 0);
-    for (int i = warp; i < R; i += 8) {
-        const int64_t n = n0 + rank * R + i;
-        if (n >= p.N || m >= p.M) continue;
-        const uint32_t at = turn + (uint32_t)(i * SM_BM) * 4 + ((uint32_t)(lane ^ (i & 7)) << 4);
-        float4 a = lds4(at);
-        for (int s = 1; s < p.cluster; ++s) {
-            const float4 b = lds4(at + (uint32_t)(s * R * SM_BM) * 4);
-            a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
-        }
-        const float b = p.bias ? p.bias[n] : 0.0f;
-        float v[4] = {a.x, a.y, a.z, a.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) v[e] = cn_apply_activation(p.bias ? v[e] + b : v[e], p.act);
-        const int64_t off = n * p.ldc + m;
-        for (int d = 0; d <= p.npeers; ++d) {
-            float *q = (d == 0 ? p.C : p.peerC[d - 1]) + off;
-            if (vec) {
-                *reinterpret_cast<float4 *>(q) = make_float4(v[0], v[1], v[2], v[3]);
-            } else {
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (m + e < p.M) q[e] = v[e];
-            }
-        }
+    // this CTA's columns: n0 + rank * R + i, a row m per lane
+#pragma unroll 1
+    for (int x = threadIdx.x; x < R * SM_BM; x += SM_EPI) {
+        const int i = x / SM_BM, ml = x % SM_BM, col = rank * R + i;
+        const int64_t m = m0 + ml;
+        if (col >= n_rows || m >= p.M) continue;
+        const uint32_t at = part + (uint32_t)x * 4;
+        float v = lds1(at);
+        for (int s = 1; s < p.cluster; ++s) v += lds1(at + (uint32_t)(s * R * SM_BM) * 4);
+        v = cn_apply_activation(p.bias ? v + s_bias[col] : v, p.act);
+        const int64_t off = (n0 + col) * p.ldc + m;
+        p.C[off] = v;
+        for (int d = 0; d < p.npeers; ++d) p.peerC[d][off] = v;
     }
 }
 
-// CTAs per tile: a power of two, as many as there are SMs for, each with at least two K blocks.
+// Clusters of c CTAs that the device holds at once (c = 1, 2, 4, 8): the SMs of a cluster have to lie in one GPC.
+static int max_clusters(const cn_context *ctx, int c)
+{
+    static int known[64][4] = {};
+    const int log = c == 8 ? 3 : c == 4 ? 2 : c == 2 ? 1 : 0, dev = ctx->device;
+    if (c == 1) return ctx->sm_count;
+    if (dev >= 0 && dev < 64 && known[dev][log] > 0) return known[dev][log];
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(ctx->sm_count / c * c));
+    cfg.blockDim = dim3(SM_THREADS);
+    cfg.dynamicSmemBytes = SmCfg<64, true>::smem(c);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)c;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(cn_gemm_small_kernel<64, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SmCfg<64, true>::smem(2)) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, cn_gemm_small_kernel<64, true, false, false>, &cfg) != cudaSuccess || n < 1) {
+        cudaGetLastError();
+        n = 1;
+    }
+    if (dev >= 0 && dev < 64) known[dev][log] = n;
+    return n;
+}
+
+// Columns per tile and CTAs per tile: the least of a rough model in ns, in which the blocks of K that a CTA takes (700 each) weigh most, then
+// what comes once per CTA, the exchange in the cluster, and the output.  Measured with 128 rows (columns / CTAs, us): 784 x 1024 weights 128 / 8
+// 10.8, 64 / 4 11.0, 32 / 4 11.4, 32 / 1 24; 1200 x 10 32 / 8 7.3, 128 / 8 8.8.  Clusters that wait for room cost a whole round more (784 x
+// 1024, 64 / 8: 16.6).
+struct SmallPlan {
+    int nt, cluster;
+    int64_t ctas;
+};
+static SmallPlan small_plan(const cn_context *ctx, int64_t M, int64_t N, int kb)
+{
+    SmallPlan best = {};
+    int64_t best_cost = INT64_MAX;
+    const int64_t tiles_m = (M + SM_BM - 1) / SM_BM;
+    for (int nt = 32; nt <= 128; nt *= 2)
+        for (int c = 1; c <= SM_MAX_CLUSTER; c *= 2) {
+            if (c > 1 && kb < 2 * c) break;
+            const int64_t tiles = tiles_m * ((N + nt - 1) / nt), rounds = (tiles + max_clusters(ctx, c) - 1) / max_clusters(ctx, c), blocks = (kb + c - 1) / c;
+            const int64_t cost = rounds * (4000 + blocks * 700 + (c == 1 ? nt * 15 : 1500 + nt * 12));
+            if (cost < best_cost) { best_cost = cost; best.nt = nt; best.cluster = c; best.ctas = tiles * c; }
+        }
+    return best;
+}
+
+// CTAs per tile of 128 x 128 that there are SMs for, each with at least two K blocks; the measure of which products are small.
 static int small_cluster(int64_t tiles, int kb, int sms)
 {
     int c = 1;
@@ -379,7 +537,7 @@ bool cn_gemm_small_shape(const cn_context *ctx, int64_t M, int64_t N, int64_t K,
 {
     if (M < 1 || N < 1 || K < 1) return false;
     if (N > (1 << 21) / K) return false;   // at most 8 MB of weights
-    const int64_t tiles = ((M + SM_BM - 1) / SM_BM) * ((N + SM_BN - 1) / SM_BN);
+    const int64_t tiles = ((M + SM_BM - 1) / SM_BM) * ((N + 127) / 128);
     const int kb = (int)((K + SM_BK - 1) / SM_BK);
     const int c = small_cluster(tiles, kb, ctx->sm_count);
     const int64_t per_cta = (kb + c - 1) / c, rounds = (tiles * c + ctx->sm_count - 1) / ctx->sm_count;
@@ -390,22 +548,22 @@ bool cn_gemm_small_shape(const cn_context *ctx, int64_t M, int64_t N, int64_t K,
     // weights that TMA cannot read must not become less exact than on the fp32 kernel (cn_gemm_any_chain); a TF32 block has twice the
     // additions of an fp16 one
     const int chain = cn_gemm_any_chain(K) / 2;
-    return w_aligned || (per_cta + SM_MAX_CHAINS - 1) / SM_MAX_CHAINS <= (chain > 1 ? chain : 1);
+    return w_aligned || (per_cta + 3) / 4 <= (chain > 1 ? chain : 1);
 }
 
-template <int WKIND, int AKIND, bool MODE3X>
+template <int NT, bool MODE3X, bool A_QUADS, bool W_QUADS>
 static int small_launch(cn_context *ctx, const SmallParams &p, int64_t ctas, cudaStream_t s)
 {
     static bool attr_set[64] = {};
     const int dev = ctx->device;
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-        CN_CUDA(cudaFuncSetAttribute(cn_gemm_small_kernel<WKIND, AKIND, MODE3X>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM_SMEM_BYTES(2)));
+        CN_CUDA(cudaFuncSetAttribute(cn_gemm_small_kernel<NT, MODE3X, A_QUADS, W_QUADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SmCfg<NT, MODE3X>::smem(2)));
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ctas);
     cfg.blockDim = dim3(SM_THREADS);
-    cfg.dynamicSmemBytes = SM_SMEM_BYTES(p.cluster);
+    cfg.dynamicSmemBytes = SmCfg<NT, MODE3X>::smem(p.cluster);
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -416,40 +574,44 @@ static int small_launch(cn_context *ctx, const SmallParams &p, int64_t ctas, cud
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = p.cluster > 1 ? 2 : 1;
-    CN_CUDA(cudaLaunchKernelEx(&cfg, cn_gemm_small_kernel<WKIND, AKIND, MODE3X>, p));
+    CN_CUDA(cudaLaunchKernelEx(&cfg, cn_gemm_small_kernel<NT, MODE3X, A_QUADS, W_QUADS>, p));
     cn_count_launch();
     return CN_OK;
 }
 
-template <bool MODE3X>
-static int small_pick(cn_context *ctx, const SmallParams &p, int wk, int ak, int64_t ctas, cudaStream_t s)
+template <int NT, bool MODE3X>
+static int small_pick(cn_context *ctx, const SmallParams &p, int64_t ctas, cudaStream_t s)
 {
-#define CN_SMALL(W) \
-    return ak == SM_K_VEC ? small_launch<W, SM_K_VEC, MODE3X>(ctx, p, ctas, s) : ak == SM_K_SCALAR ? small_launch<W, SM_K_SCALAR, MODE3X>(ctx, p, ctas, s) \
-                                                                                                    : small_launch<W, SM_ROWS, MODE3X>(ctx, p, ctas, s)
-    if (wk == SM_K_VEC) CN_SMALL(SM_K_VEC);
-    if (wk == SM_K_SCALAR) CN_SMALL(SM_K_SCALAR);
-    CN_SMALL(SM_ROWS);
-#undef CN_SMALL
+    const bool aq = p.A.sk != 1 && p.A.vec, wq = p.W.sk != 1 && p.W.vec;
+    return aq ? (wq ? small_launch<NT, MODE3X, true, true>(ctx, p, ctas, s) : small_launch<NT, MODE3X, true, false>(ctx, p, ctas, s))
+              : (wq ? small_launch<NT, MODE3X, false, true>(ctx, p, ctas, s) : small_launch<NT, MODE3X, false, false>(ctx, p, ctas, s));
 }
 
 int cn_gemm_small_launch(cn_context *ctx, int transA, int transB, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, const float *B, int64_t ldb,
-                         float *C, int64_t ldc, const cn_epilogue *epi, int mode, cudaStream_t s, const cn_peer_out *peers, bool w_aligned)
+                         float *C, int64_t ldc, const cn_epilogue *epi, int mode, cudaStream_t s, const cn_peer_out *peers)
 {
     SmallParams p;
     unsigned int *d_status = nullptr;
     int st = cn_status_block(ctx, &d_status);
     if (st != CN_OK) return st;
-    p.W = B; p.A = A; p.ldw = ldb; p.lda = lda;
+    auto operand = [](const float *q, bool k_contiguous, int64_t ld) {
+        SmOperand o;
+        o.p = q;
+        o.sr = k_contiguous ? ld : 1;
+        o.sk = k_contiguous ? 1 : ld;
+        o.vec = (ld & 3) == 0 && ((uintptr_t)q & 15u) == 0;
+        return o;
+    };
+    p.A = operand(A, transA != 0, lda);
+    p.W = operand(B, transB == 0, ldb);
     p.M = M; p.N = N; p.K = K;
     p.C = C; p.ldc = ldc;
     p.bias = epi ? epi->bias : nullptr;
     p.act = epi ? epi->activation : CN_ACT_LINEAR;
     p.tiles_m = (int)((M + SM_BM - 1) / SM_BM);
-    const int64_t tiles = (int64_t)p.tiles_m * ((N + SM_BN - 1) / SM_BN);
     p.kb_total = (int)((K + SM_BK - 1) / SM_BK);
-    p.cluster = small_cluster(tiles, p.kb_total, ctx->sm_count);
-    p.fine_chains = !w_aligned;
+    const SmallPlan plan = small_plan(ctx, M, N, p.kb_total);
+    p.cluster = plan.cluster;
     p.status = d_status;
     p.npeers = 0;
     p.ready = nullptr; p.peer_flags = nullptr;
@@ -461,11 +623,10 @@ int cn_gemm_small_launch(cn_context *ctx, int transA, int transB, int64_t M, int
         p.ready = peers->ready; p.peer_flags = peers->peer_flags;
         p.nranks = peers->nranks; p.my_rank = peers->my_rank; p.epoch = peers->epoch;
     }
-    auto kind = [](bool k_contiguous, int64_t ld, const float *q) {
-        return !k_contiguous ? SM_ROWS : ((ld & 3) == 0 && ((uintptr_t)q & 15u) == 0) ? SM_K_VEC : SM_K_SCALAR;
-    };
-    const int wk = kind(!transB, ldb, B), ak = kind(transA != 0, lda, A);
-    st = mode == CN_GEMM_3XTF32 ? small_pick<true>(ctx, p, wk, ak, tiles * p.cluster, s) : small_pick<false>(ctx, p, wk, ak, tiles * p.cluster, s);
-    if (st == CN_OK) ctx->gemm_last_path = mode == CN_GEMM_3XTF32 ? "tcgen05_3xtf32" : "tcgen05_tf32";
+    const bool m3 = mode == CN_GEMM_3XTF32;
+    if (plan.nt == 32)      st = m3 ? small_pick<32, true>(ctx, p, plan.ctas, s) : small_pick<32, false>(ctx, p, plan.ctas, s);
+    else if (plan.nt == 64) st = m3 ? small_pick<64, true>(ctx, p, plan.ctas, s) : small_pick<64, false>(ctx, p, plan.ctas, s);
+    else                    st = m3 ? small_pick<128, true>(ctx, p, plan.ctas, s) : small_pick<128, false>(ctx, p, plan.ctas, s);
+    if (st == CN_OK) ctx->gemm_last_path = m3 ? "tcgen05_3xtf32" : "tcgen05_tf32";
     return st;
 }

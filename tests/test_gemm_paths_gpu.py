@@ -55,6 +55,28 @@ def test_small_products_in_every_layout(ctx, M, K, N, transA, transB):
             check(C, A, B, transA, transB, rel)
 
 
+# tiles of 32, 64 and 128 columns, by one CTA and by clusters of 2, 4 and 8; more blocks than accumulators
+@pytest.mark.parametrize("M,K,N", [(48, 80, 1091), (128, 1200, 10), (1200, 128, 10), (784, 128, 1200), (32, 500, 500), (1200, 120, 1201), (512, 500, 1000), (128, 785, 1100),
+                                   (200, 380, 2100), (64, 3000, 600)])
+@pytest.mark.parametrize("act", [_lib.ACT_LINEAR, _lib.ACT_RELU, _lib.ACT_LOGISTIC])
+def test_small_products_of_every_tile(ctx, M, K, N, act):
+    """Bias and activation in both ends of the kernel, the same bits twice; 2-norm of the 3x mode's linear product against the error of
+    fp32 sums (random rounding of two TF32 parts, 2^-23, and of 8 sequential additions per chain: 4e-7)."""
+    rng = np.random.default_rng(M + K + N)
+    A, B, b = rng.uniform(-1, 1, (M, K)).astype(np.float32), rng.uniform(-1, 1, (K, N)).astype(np.float32), rng.uniform(-1, 1, N).astype(np.float32)
+    n0 = ctx.lib.cn_kernel_launches()
+    C, C2 = (ctx.gemm(place(A, 0), place(B, 0), bias=torch.from_numpy(b).cuda(), activation=act) for _ in range(2))
+    assert ctx.lib.cn_kernel_launches() - n0 == 2
+    ctx.gemm_check()
+    assert torch.equal(C, C2)
+    ref, bound = A.astype(np.float64) @ B + b, REL_3X * (np.abs(A).astype(np.float64) @ np.abs(B) + np.abs(b))
+    got = C.T.cpu().numpy().astype(np.float64)
+    if act == _lib.ACT_LINEAR:
+        assert np.linalg.norm(got - ref) <= 4e-7 * np.linalg.norm(ref)
+    want = {_lib.ACT_LINEAR: ref, _lib.ACT_RELU: np.maximum(ref, 0), _lib.ACT_LOGISTIC: 1 / (1 + np.exp(-ref))}[act]
+    assert np.all(np.abs(got - want) <= bound + 1e-7)
+
+
 @pytest.mark.parametrize("mode", [_lib.GEMM_3XTF32, _lib.GEMM_TF32])
 @pytest.mark.parametrize("transA,transB", [(False, False), (True, False), (False, True)])
 @pytest.mark.parametrize("wide", ["A", "B"])
