@@ -29,6 +29,7 @@
 // calls the launch latency, the CTA start-up and the table build of call i+1 then overlap the tail of call i.
 #include <math.h>
 #include <string.h>
+#include <vector>
 #include "cn_internal.h"
 
 #define CODEC_THREADS 1024
@@ -476,27 +477,20 @@ __device__ __forceinline__ void cdc_grid_barrier(unsigned int *arrive, unsigned 
     __syncthreads();
 }
 
-enum { RING_SCALE_HOST = 0, RING_SCALE_DEVICE = 1, RING_SCALE_ABSMAX = 2 };
+enum { RING_SCALE_HOST = 0, RING_SCALE_DEVICE = 1 };
 
 // Work split: every CTA codes the same number of tiles (tiles_per_cta) of the same size (tile_groups 16-byte groups,
 // at most RING_TILE / 4), chosen on the host so that grid * tiles_per_cta tiles cover the tensor with less than one
 // group of slack per tile; tile j goes to CTA j % grid.  The last tiles may be short or missing.
-//
-// SCALE = RING_SCALE_ABSMAX is the fused form of "scale = absmax(A); codes = compress(A, scale)" (cooperative launch):
-// pass 1 reduces |A| over the CTA's own tiles with plain loads that leave the lines in L2, a grid barrier publishes the
-// per-CTA maxima, every CTA folds them, and pass 2 codes the CTA's tiles in reverse order - most recently read first -
-// so that a tensor that fits the L2 is read from HBM once.  d_precision then receives the scale.
 template <int SCALE>
 __global__ void __launch_bounds__(RING_THREADS, 2)
-cn_compress_ring_kernel(const float *A, float precision_arg, float *d_precision,
+cn_compress_ring_kernel(const float *A, float precision_arg, const float *d_precision,
                         int64_t n, uint8_t *out, const __grid_constant__ RingConst rc, unsigned int *status,
-                        int tile_groups, int tiles_per_cta, float *partials, unsigned int *barrier_words,
-                        int input_ready_before_predecessor)
+                        int tile_groups, int tiles_per_cta, int input_ready_before_predecessor)
 {
     extern __shared__ __align__(128) uint8_t ring_smem[];
     __shared__ RingTables t;
     __shared__ __align__(8) uint64_t bars[2 * RING_STAGES];
-    __shared__ float s_red[RING_THREADS / 32];
     const int tid = threadIdx.x;
     const uint32_t ring_base = (cdc_smem_u32(ring_smem) + 127u) & ~127u;
     const uint8_t *ring_gen = ring_smem + (ring_base - cdc_smem_u32(ring_smem));
@@ -523,8 +517,8 @@ cn_compress_ring_kernel(const float *A, float precision_arg, float *d_precision,
             my_tiles = (int)(mine < tiles_per_cta ? mine : tiles_per_cta);
         }
     }
-    // the i-th tile this CTA codes (pass 2 of the fused form walks its tiles backwards) and its size in 16-byte groups
-    auto tile_of = [&](int i) { return (int64_t)blockIdx.x + (int64_t)(SCALE == RING_SCALE_ABSMAX ? my_tiles - 1 - i : i) * gridDim.x; };
+    // the i-th tile this CTA codes and its size in 16-byte groups
+    auto tile_of = [&](int i) { return (int64_t)blockIdx.x + (int64_t)i * gridDim.x; };
     auto tile_count = [&](int64_t j) {
         const int64_t left = groups_total - j * tile_groups;
         return (int)(left < tile_groups ? left : tile_groups);
@@ -546,54 +540,9 @@ cn_compress_ring_kernel(const float *A, float precision_arg, float *d_precision,
     // ---- everything below may touch global memory: the predecessor in the stream must have finished
     cn_pdl_wait();
     float p = precision_arg;
-    if (SCALE == RING_SCALE_ABSMAX) {
-        // pass 1: maximum of |A| over this CTA's tiles (and, in CTA 0, the last n % 4 elements)
-        float m = -1.0f;   // seed of the reference's reduction (source/basicOps.cu:1079)
-        const float4 *A4 = reinterpret_cast<const float4 *>(A);
-        for (int k = 0; k < my_tiles; ++k) {
-            const int64_t j = (int64_t)blockIdx.x + (int64_t)k * gridDim.x;
-            const int groups = tile_count(j);
-            const float4 *src = A4 + j * tile_groups;
-            float4 q[RING_GROUPS_PER_THREAD];
-#pragma unroll
-            for (int u = 0; u < RING_GROUPS_PER_THREAD; ++u)
-                q[u] = (tid + u * RING_THREADS < groups) ? src[tid + u * RING_THREADS] : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int u = 0; u < RING_GROUPS_PER_THREAD; ++u)
-                if (tid + u * RING_THREADS < groups)
-                    m = fmaxf(m, fmaxf(fmaxf(fabsf(q[u].x), fabsf(q[u].y)), fmaxf(fabsf(q[u].z), fabsf(q[u].w))));
-        }
-        if (blockIdx.x == 0 && tid < (int)(n - (groups_total << 2))) m = fmaxf(m, fabsf(A[(groups_total << 2) + tid]));
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if ((tid & 31) == 0) s_red[tid >> 5] = m;
-        __syncthreads();
-        if (tid < 32) {
-            m = tid < RING_THREADS / 32 ? s_red[tid] : -1.0f;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-            if (tid == 0) partials[blockIdx.x] = m;
-        }
-        cdc_grid_barrier(barrier_words, barrier_words + 1, status);
-    }
     // fill the ring before anything else: the first loads are in flight while the tables are built
     if (tid == 0 && !(SCALE == RING_SCALE_DEVICE && input_ready_before_predecessor)) fill_ring();
     if (SCALE == RING_SCALE_DEVICE) p = *d_precision;
-    if (SCALE == RING_SCALE_ABSMAX) {
-        // every CTA folds the per-CTA maxima (the same values in the same order everywhere)
-        float m = -1.0f;
-        for (int i = tid; i < (int)gridDim.x; i += RING_THREADS) m = fmaxf(m, __ldcg(partials + i));
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        __syncthreads();   // s_red was read above
-        if ((tid & 31) == 0) s_red[tid >> 5] = m;
-        __syncthreads();
-        m = s_red[0];
-#pragma unroll
-        for (int w = 1; w < RING_THREADS / 32; ++w) m = fmaxf(m, s_red[w]);
-        p = m;
-        if (blockIdx.x == 0 && tid == 0) *d_precision = p;
-    }
     const uint32_t pb = __float_as_uint(p);
     const float ap = fabsf(p);
     // 2^-100 <= |p| <= 2^100 keeps every boundary T*|p| a normal number; NaN fails both tests
@@ -700,6 +649,132 @@ cn_compress_ring_kernel(const float *A, float precision_arg, float *d_precision,
     if (blockIdx.x == 0 && tid < (int)(n - n4)) {
         const float x = A[n4 + tid];
         out[n4 + tid] = (uint8_t)(fast ? ring_code(__float_as_uint(x), pb, kadd, span, lut_addr) : ring_generic(x, p, t));
+    }
+}
+
+// ---- scale and codes in one launch
+//
+// scale = absmax(A); codes = compress(A, scale) for tensors that the threads of one CTA per SM can hold in registers: 64 elements per thread,
+// 4 Mi on 148 SMs.  Every element is read once, coded after the maxima have gone round, and written once.  Bound by latency: launch,
+// one trip to memory, the exchange of the maxima, the stores.
+//   * A few CTAs are one cluster, which passes the maxima through distributed shared memory; more are a cooperative launch with a grid
+//     barrier.
+//   * The decision table is that of the quotient |x / scale| (thresholds of the codebook, no scale in it): it is made once, when the context
+//     is, and fetched while the first loads are under way.  Elements are divided as the reference divides them, which costs less than a
+//     table for this scale, made between the barrier and the coding.
+//   * Any alignment: up to three elements before the first 16-byte boundary of A and after the last are coded one by one, and codes that do
+//     not lie on a 4-byte boundary then are stored as words of the lane's own and its neighbour's bytes.  (Segments of a packed
+//     gradient buffer, whose lengths are odd.)
+// Scale and codes of one tensor in a series, us, before (two passes, a table per scale) and now: 131072 elements 10.3, 7.8; 940800 11.4,
+// 10.3; 2.4 M 14.4, 12.4; 4 Mi 16.4, 16.4.  Scales, codes and decoded values of three tensors of odd length in a row: 44, 33 (the
+// second and third took two launches of 9 and 7 us).
+#define CODE_THREADS 512         // at 64 registers, half an SM: the next kernel's CTAs find room beside
+#define CODE_QUADS 8
+#define CODE_CLUSTER 8
+#define CODE_CLUSTER_QUADS 2
+
+struct CodeTable {          // of quotients, see RingTables
+    uint32_t lut[LUT_MAX];
+    uint32_t kadd;
+    int32_t span;
+    int nb;
+};
+
+__device__ __forceinline__ uint32_t code_one(float x, float p, uint32_t kadd, int32_t span, uint32_t lut_addr)
+{
+    const float a = __fdiv_rn(x, p);
+    const uint32_t c = (ring_lookup(__float_as_uint(a), kadd, span, lut_addr) & 0xffu) | (__float_as_uint(a) >> 24 & 0x80u);
+    return a != a ? 1u : c;   // NaN: the reference's search ends on index 1, sign clear (code 254 of a zero has the sign bit anyway)
+}
+
+template <bool CLUSTER, int QUADS>
+__global__ void __launch_bounds__(CODE_THREADS, QUADS <= CODE_QUADS ? 2 : 1)
+cn_absmax_code_kernel(const float *A, int64_t n, float *scale, uint8_t *codes, const CodeTable *table, float *partials, unsigned int *barrier_words,
+                      unsigned int *status)
+{
+    __shared__ __align__(16) uint32_t lut[LUT_MAX];
+    __shared__ float s_red[CODE_THREADS / 32], s_peer[CODE_CLUSTER];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    cn_pdl_launch_dependents();
+    if (CLUSTER) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // all CTAs run before one writes into another
+    const uint32_t kadd = table->kadd;
+    const int32_t span = table->span;
+    const int nb = table->nb;
+    cn_pdl_wait();
+    const int to16 = (int)((0 - (reinterpret_cast<uintptr_t>(A) >> 2)) & 3), head = to16 < n ? to16 : (int)n;
+    const int quads = (int)((n - head) >> 2), tail = (int)(n - head) & 3;
+    const float4 *A4 = reinterpret_cast<const float4 *>(A + head);
+    const int stride = gridDim.x * CODE_THREADS, q0 = blockIdx.x * CODE_THREADS + tid;
+    float4 v[QUADS];
+#pragma unroll
+    for (int u = 0; u < QUADS; ++u)
+        v[u] = q0 + u * stride < quads ? A4[q0 + u * stride] : make_float4(0.f, 0.f, 0.f, 0.f);
+    // the first CTA's first warps take the elements outside the quads
+    const bool single = blockIdx.x == 0 && (tid < head || (tid >= 32 && tid - 32 < tail));
+    const int64_t at1 = tid < 32 ? tid : head + 4 * (int64_t)quads + tid - 32;
+    const float x1 = single ? A[at1] : 0.0f;
+    for (int i = tid; i < nb; i += CODE_THREADS) lut[i] = table->lut[i];
+    float m = -1.0f;   // seed of the reference's reduction (source/basicOps.cu:1079)
+#pragma unroll
+    for (int u = 0; u < QUADS; ++u)
+        if (q0 + u * stride < quads) m = fmaxf(m, fmaxf(fmaxf(fabsf(v[u].x), fabsf(v[u].y)), fmaxf(fabsf(v[u].z), fabsf(v[u].w))));
+    if (single) m = fmaxf(m, fabsf(x1));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane == 0) s_red[warp] = m;
+    __syncthreads();
+    m = s_red[lane % (CODE_THREADS / 32)];
+#pragma unroll
+    for (int o = CODE_THREADS / 64; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (CLUSTER) {
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (tid < (int)gridDim.x) {
+            uint32_t at = cdc_smem_u32(&s_peer[blockIdx.x]);
+            asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(at), "r"(tid));
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(m) : "memory");
+        }
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        m = s_peer[0];
+        for (int i = 1; i < (int)gridDim.x; ++i) m = fmaxf(m, s_peer[i]);
+    } else {
+        if (tid == 0) partials[blockIdx.x] = m;
+        cdc_grid_barrier(barrier_words, barrier_words + 1, status);
+        m = -1.0f;
+        for (int i = lane; i < (int)gridDim.x; i += 32) m = fmaxf(m, __ldcg(partials + i));
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    }
+    const float p = m;
+    if (blockIdx.x == 0 && tid == 0) *scale = p;
+    const uint32_t lut_addr = cdc_smem_u32(lut);
+    if (single) codes[at1] = (uint8_t)code_one(x1, p, kadd, span, lut_addr);
+    // `off` bytes of a quad's codes lie before the next 4-byte boundary: the word there takes the other bytes of this lane's codes and the
+    // first of the next lane's
+    uint8_t *out = codes + head;
+    const int off = (int)((0 - reinterpret_cast<uintptr_t>(out)) & 3u);
+#pragma unroll
+    for (int u = 0; u < QUADS; ++u) {
+        const int q = q0 + u * stride;
+        if (q - lane >= quads) break;   // the same for the whole warp
+        const bool mine = q < quads;
+        const uint32_t c = pack4(code_one(v[u].x, p, kadd, span, lut_addr), code_one(v[u].y, p, kadd, span, lut_addr),
+                                 code_one(v[u].z, p, kadd, span, lut_addr), code_one(v[u].w, p, kadd, span, lut_addr));
+        if (off == 0) {
+            if (mine) reinterpret_cast<uint32_t *>(out)[q] = c;
+            continue;
+        }
+        const uint32_t next = __shfl_down_sync(0xffffffffu, c, 1);
+        if (!mine) continue;
+        uint8_t *at = out + 4 * (int64_t)q;
+        if (lane == 0)
+            for (int b = 0; b < off; ++b) at[b] = (uint8_t)(c >> (8 * b));
+        if (lane < 31 && q < quads - 1) {
+            *reinterpret_cast<uint32_t *>(at + off) = __funnelshift_r(c, next, 8 * off);
+        } else {
+            for (int b = off; b < 4; ++b) at[b] = (uint8_t)(c >> (8 * b));
+        }
     }
 }
 
@@ -868,7 +943,7 @@ cn_absmax_compress_push_kernel(const float *A, int64_t n, float *scale_out, uint
 template <bool PRECISION_ON_DEVICE>
 __global__ void __launch_bounds__(CODEC_THREADS, 1)
 cn_decompress_kernel(const uint8_t *codes, float precision_arg, const float *d_precision,
-                     int64_t n, float *out, const __grid_constant__ DecodeConst dc, int vector_ok)
+                     int64_t n, float *out, const __grid_constant__ DecodeConst dc, int vector_ok, int head)
 {
     __shared__ float lut[256];
     const int tid = threadIdx.x;
@@ -888,6 +963,10 @@ cn_decompress_kernel(const uint8_t *codes, float precision_arg, const float *d_p
     }
     if (!PRECISION_ON_DEVICE) cn_pdl_wait();
     __syncthreads();
+    if (blockIdx.x == 0 && tid < head) out[tid] = lut[codes[tid]];
+    codes += head;
+    out += head;
+    n -= head;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     float4 *out4 = reinterpret_cast<float4 *>(out);
 #define CN_DEC4(w) make_float4(lut[(w) & 0xffu], lut[((w) >> 8) & 0xffu], lut[((w) >> 16) & 0xffu], lut[(w) >> 24])
@@ -1215,37 +1294,24 @@ static bool host_boundaries(cn_context *ctx, float precision, uint32_t X[128])
     return ok;
 }
 
-// scale_mode: RING_SCALE_HOST (precision), RING_SCALE_DEVICE (d_precision read) or RING_SCALE_ABSMAX (d_precision written)
-static int compress_impl(cn_context *ctx, const float *d_A, float precision, float *d_precision, int scale_mode, int64_t n,
+// scale_mode: RING_SCALE_HOST (precision) or RING_SCALE_DEVICE (d_precision read)
+static int compress_impl(cn_context *ctx, const float *d_A, float precision, const float *d_precision, int scale_mode, int64_t n,
                          uint8_t *d_codes, void *stream, int after_own_absmax = 0)
 {
     CN_REQUIRE(ctx, CN_ERR_ARG, "cn_compress_8bit: null context");
     CN_REQUIRE(n >= 0, CN_ERR_ARG, "cn_compress_8bit: negative size");
     cudaStream_t s = cn_stream(stream);
     const bool ring_ok = ((uintptr_t)d_A % 16 == 0) && ((uintptr_t)d_codes % 4 == 0) && n >= 4;
-    // The single cooperative launch pays off while the pair of launches is bound by launch latency; from a few million
-    // elements on, two pipelined launches are faster (measured on a B200: 13.7 vs 21.6 us at 2.4 M elements, 39.2 vs 33.6 us at
-    // 16.8 M: the second pass is bound by the integer pipe, not by HBM, so reading it from L2 gains nothing).
-    if (scale_mode == RING_SCALE_ABSMAX && (!ring_ok || n > CN_FUSED_ABSMAX_MAX_N)) {
-        // also for buffers the ring kernel does not take (unaligned, tiny, empty): the two-call form
-        int st = cn_absmax_f32(ctx, d_A, n, d_precision, stream);
-        if (st != CN_OK || n == 0) return st;
-        return compress_impl(ctx, d_A, 0.f, d_precision, RING_SCALE_DEVICE, n, d_codes, stream, 1);
-    }
     if (n == 0) return CN_OK;
     CN_REQUIRE(d_A && d_codes, CN_ERR_ARG, "cn_compress_8bit: null buffer");
     if (ring_ok) {
         static bool attr_set[64] = {};   // per device: the attribute belongs to the device's copy of the function
-        static int occupancy[64] = {};
         const size_t smem = (size_t)RING_STAGES * RING_TILE * 4 + 128;
         const int dev = ctx->device;
         if (dev < 0 || dev >= 64 || !attr_set[dev]) {
             CN_CUDA(cudaFuncSetAttribute(cn_compress_ring_kernel<RING_SCALE_HOST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             CN_CUDA(cudaFuncSetAttribute(cn_compress_ring_kernel<RING_SCALE_DEVICE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            CN_CUDA(cudaFuncSetAttribute(cn_compress_ring_kernel<RING_SCALE_ABSMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            int occ = 0;
-            CN_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, cn_compress_ring_kernel<RING_SCALE_ABSMAX>, RING_THREADS, smem));
-            if (dev >= 0 && dev < 64) { attr_set[dev] = true; occupancy[dev] = occ; }
+            if (dev >= 0 && dev < 64) attr_set[dev] = true;
         }
         unsigned int *d_status = nullptr;
         int st = cn_status_block(ctx, &d_status);
@@ -1257,13 +1323,7 @@ static int compress_impl(cn_context *ctx, const float *d_A, float precision, flo
         // every CTA gets the same number of equally sized tiles (at most RING_TILE elements each)
         const int64_t groups = n >> 2, max_groups = RING_TILE / 4;
         const int64_t min_tiles = (groups + max_groups - 1) / max_groups;
-        int ctas_per_sm = 2;
-        if (scale_mode == RING_SCALE_ABSMAX) {   // cooperative launch: all CTAs must be resident at once
-            const int occ = (dev >= 0 && dev < 64) ? occupancy[dev] : 1;
-            CN_REQUIRE(occ >= 1, CN_ERR_UNSUPPORTED, "cn_absmax_compress_8bit: the kernel does not fit this device");
-            if (occ < ctas_per_sm) ctas_per_sm = occ;
-        }
-        const int64_t max_grid = (int64_t)ctas_per_sm * ctx->sm_count;
+        const int64_t max_grid = 2LL * ctx->sm_count;
         int grid = (int)(min_tiles < max_grid ? min_tiles : max_grid);
         if (grid > CN_MAX_PARTIALS) grid = CN_MAX_PARTIALS;
         const int64_t tpc64 = (min_tiles + grid - 1) / grid;
@@ -1273,26 +1333,12 @@ static int compress_impl(cn_context *ctx, const float *d_A, float precision, flo
         // whole tiles save the per-thread bounds tests: take them when the busiest CTA gets at most 2 % more work than with
         // the exactly balanced size
         if ((int64_t)tiles_per_cta * max_groups * 100 <= (int64_t)tiles_per_cta * tile_groups * 102) tile_groups = (int)max_groups;
-        unsigned int *barrier_words = ctx->d_ticket + 4;   // words 4, 5 of the ticket block: arrival count, generation
-        if (scale_mode == RING_SCALE_ABSMAX) {
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3((unsigned)grid);
-            cfg.blockDim = dim3(RING_THREADS);
-            cfg.dynamicSmemBytes = smem;
-            cfg.stream = s;
-            cudaLaunchAttribute attr[1];
-            attr[0].id = cudaLaunchAttributeCooperative;
-            attr[0].val.cooperative = 1;
-            cfg.attrs = attr;
-            cfg.numAttrs = 1;
-            CN_CUDA(cudaLaunchKernelEx(&cfg, cn_compress_ring_kernel<RING_SCALE_ABSMAX>, d_A, 0.f, d_precision, n, d_codes, rc, d_status, tile_groups,
-                                       tiles_per_cta, ctx->d_partials, barrier_words, 0));
-        } else if (scale_mode == RING_SCALE_DEVICE) {
+        if (scale_mode == RING_SCALE_DEVICE) {
             CN_CUDA(cn_launch_pdl(cn_compress_ring_kernel<RING_SCALE_DEVICE>, grid, RING_THREADS, smem, s, d_A, 0.f, d_precision, n, d_codes, rc, d_status,
-                               tile_groups, tiles_per_cta, (float *)nullptr, (unsigned int *)nullptr, after_own_absmax));
+                               tile_groups, tiles_per_cta, after_own_absmax));
         } else {
-            CN_CUDA(cn_launch_pdl(cn_compress_ring_kernel<RING_SCALE_HOST>, grid, RING_THREADS, smem, s, d_A, precision, (float *)nullptr, n, d_codes, rc,
-                               d_status, tile_groups, tiles_per_cta, (float *)nullptr, (unsigned int *)nullptr, 0));
+            CN_CUDA(cn_launch_pdl(cn_compress_ring_kernel<RING_SCALE_HOST>, grid, RING_THREADS, smem, s, d_A, precision, (const float *)nullptr, n, d_codes, rc,
+                               d_status, tile_groups, tiles_per_cta, 0));
         }
         cn_count_launch();
         return CN_OK;
@@ -1366,11 +1412,89 @@ extern "C" int cn_compress_8bit_dp(cn_context *ctx, const float *d_A, const floa
     return compress_impl(ctx, d_A, 0.f, const_cast<float *>(d_precision), RING_SCALE_DEVICE, n, d_codes, stream);
 }
 
+// The table of quotients of a codebook, on the host; false where two thresholds share a bucket (see ring_build_tables, whose steps it
+// takes with the thresholds themselves in place of a scale's boundaries).
+static bool host_code_table(const uint32_t thr[128], const uint8_t lc[128], CodeTable *t)
+{
+    for (int j = 0; j < CN_NUM_THR; ++j)
+        if (thr[j] >= 0x7f800000u) return false;
+    const uint32_t xtop = thr[CN_NUM_THR - 1], delta = ((xtop + 0xffffu) & 0xffff0000u) - xtop, hi = xtop + delta;
+    const int base = (int)((thr[0] + delta) >> 16) - 1, nb = (int)(hi >> 16) - base + 1;
+    if (base < 1 || nb < 3 || nb > LUT_MAX) return false;
+    t->kadd = delta - ((uint32_t)base << 16);
+    t->span = (int32_t)(hi - ((uint32_t)base << 16));
+    t->nb = nb;
+    int first = 0;   // first threshold whose shifted bucket is >= this one
+    for (int b = 0; b < nb; ++b) {
+        const uint32_t bucket = (uint32_t)(b + base);
+        while (first < CN_NUM_THR && (thr[first] + delta) >> 16 < bucket) ++first;
+        if (first < CN_NUM_THR && (thr[first] + delta) >> 16 == bucket) {
+            if (first + 1 < CN_NUM_THR && (thr[first + 1] + delta) >> 16 == bucket) return false;
+            t->lut[b] = (thr[first] + delta) << 16 | (uint32_t)lc[first + 1] << 8 | lc[first];
+        } else {
+            t->lut[b] = (uint32_t)lc[first] << 8 | lc[first];
+        }
+    }
+    return true;
+}
+
+cudaError_t cn_codec_make_table(cn_context *ctx)
+{
+    std::vector<CodeTable> t(1);
+    if (!host_code_table(ctx->h_thr, ctx->h_level_codes, &t[0])) return cudaSuccess;   // two launches then
+    cudaError_t e = cudaMalloc(&ctx->d_code_table, sizeof(CodeTable));
+    if (e == cudaSuccess) e = cudaMemcpy(ctx->d_code_table, &t[0], sizeof(CodeTable), cudaMemcpyHostToDevice);
+    return e;
+}
+
+static int absmax_code(cn_context *ctx, const float *d_A, int64_t n, float *d_scale, uint8_t *d_codes, void *stream)
+{
+    unsigned int *d_status = nullptr;
+    const int st = cn_status_block(ctx, &d_status);
+    if (st != CN_OK) return st;
+    // one cluster while its threads have few elements each; else a quad per thread, up to one CTA per SM, which holds 64 elements per thread
+    // of the largest (4 Mi: two CTAs per SM of 32 take 20 us)
+    const int64_t per_cta = CODE_THREADS * 4;
+    const bool cluster = n <= per_cta * CODE_CLUSTER * CODE_CLUSTER_QUADS;
+    int64_t grid = (n + per_cta - 1) / per_cta;
+    if (cluster) grid = grid <= 1 ? 1 : grid <= 2 ? 2 : grid <= 4 ? 4 : CODE_CLUSTER;
+    else if (grid > ctx->sm_count) grid = ctx->sm_count;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(CODE_THREADS);
+    cfg.stream = cn_stream(stream);
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    if (cluster) {
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = (unsigned)grid;
+        attr[1].val.clusterDim.y = 1;
+        attr[1].val.clusterDim.z = 1;
+    } else {
+        attr[1].id = cudaLaunchAttributeCooperative;
+        attr[1].val.cooperative = 1;
+    }
+    cfg.numAttrs = 2;
+    cfg.attrs = attr;
+    const CodeTable *table = (const CodeTable *)ctx->d_code_table;
+    unsigned int *barrier_words = ctx->d_ticket + 4;   // words 4, 5 of the ticket block: arrival count, generation
+    if (cluster) CN_CUDA(cudaLaunchKernelEx(&cfg, cn_absmax_code_kernel<true, CODE_QUADS>, d_A, n, d_scale, d_codes, table, ctx->d_partials, barrier_words, d_status));
+    else if (n <= per_cta * CODE_QUADS * ctx->sm_count - 4) CN_CUDA(cudaLaunchKernelEx(&cfg, cn_absmax_code_kernel<false, CODE_QUADS>, d_A, n, d_scale, d_codes, table, ctx->d_partials, barrier_words, d_status));
+    else CN_CUDA(cudaLaunchKernelEx(&cfg, cn_absmax_code_kernel<false, 2 * CODE_QUADS>, d_A, n, d_scale, d_codes, table, ctx->d_partials, barrier_words, d_status));
+    cn_count_launch();
+    return CN_OK;
+}
+
 extern "C" int cn_absmax_compress_8bit(cn_context *ctx, const float *d_A, int64_t n, float *d_scale_out, uint8_t *d_codes, void *stream)
 {
     CN_REQUIRE(ctx && d_scale_out, CN_ERR_ARG, "cn_absmax_compress_8bit: null argument");
     CN_REQUIRE(n >= 0 && (n == 0 || (d_A && d_codes)), CN_ERR_ARG, "cn_absmax_compress_8bit: bad input");
-    return compress_impl(ctx, d_A, 0.f, d_scale_out, RING_SCALE_ABSMAX, n, d_codes, stream);
+    if (n > 0 && ctx->d_code_table && n <= CN_FUSED_ABSMAX_MAX_N && n <= 2LL * ctx->sm_count * CODE_THREADS * CODE_QUADS * 4 && ((uintptr_t)d_A & 3u) == 0)
+        return absmax_code(ctx, d_A, n, d_scale_out, d_codes, stream);
+    int st = cn_absmax_f32(ctx, d_A, n, d_scale_out, stream);
+    if (st != CN_OK || n == 0) return st;
+    return compress_impl(ctx, d_A, 0.f, d_scale_out, RING_SCALE_DEVICE, n, d_codes, stream, 1);
 }
 
 static int decompress_impl(cn_context *ctx, const uint8_t *d_codes, float precision, const float *d_precision, int64_t n,
@@ -1380,11 +1504,13 @@ static int decompress_impl(cn_context *ctx, const uint8_t *d_codes, float precis
     CN_REQUIRE(n >= 0, CN_ERR_ARG, "cn_decompress_8bit: negative size");
     if (n == 0) return CN_OK;
     CN_REQUIRE(d_out && d_codes, CN_ERR_ARG, "cn_decompress_8bit: null buffer");
-    int vector_ok = ((uintptr_t)d_out % 16 == 0) && ((uintptr_t)d_codes % 4 == 0);
+    // up to three elements one by one bring the output to a 16-byte boundary: a segment of a packed buffer then has its codes on a 4-byte one
+    const int to16 = (int)((0 - ((uintptr_t)d_out >> 2)) & 3), head = to16 < n ? to16 : (int)n;
+    int vector_ok = ((uintptr_t)d_out & 3u) == 0 && ((uintptr_t)(d_codes + head) & 3u) == 0;
     // Sixteen codes per load for large tensors (2^28 codes: 218 vs 236 us).  Up to tens of MiB the four-codes kernel stays:
     // in a series of calls its one 1024-thread CTA per SM leaves room for the next launch to become resident early
     // (programmatic dependent launch), which is worth more there (4096 x 4096: 15.8 vs 16.9 us).
-    if (vector_ok && (uintptr_t)d_codes % 16 == 0 && n >= (1LL << 26)) vector_ok = 2;
+    if (vector_ok && head == 0 && (uintptr_t)d_codes % 16 == 0 && n >= (1LL << 26)) vector_ok = 2;
     int grid = codec_grid(ctx, n, CODEC_THREADS, vector_ok == 2 ? 16 : 4, 1);   // one resident CTA per SM
     DecodeConst dc;
     for (int i = 0; i < 128; ++i) dc.tbl[i] = ctx->h_tbl[i];
@@ -1397,9 +1523,9 @@ static int decompress_impl(cn_context *ctx, const uint8_t *d_codes, float precis
         return CN_OK;
     }
     if (d_precision)
-        CN_CUDA(cn_launch_pdl(cn_decompress_kernel<true>, grid, CODEC_THREADS, 0, cn_stream(stream), d_codes, 0.f, d_precision, n, d_out, dc, vector_ok));
+        CN_CUDA(cn_launch_pdl(cn_decompress_kernel<true>, grid, CODEC_THREADS, 0, cn_stream(stream), d_codes, 0.f, d_precision, n, d_out, dc, vector_ok, vector_ok ? head : 0));
     else
-        CN_CUDA(cn_launch_pdl(cn_decompress_kernel<false>, grid, CODEC_THREADS, 0, cn_stream(stream), d_codes, precision, (const float *)nullptr, n, d_out, dc, vector_ok));
+        CN_CUDA(cn_launch_pdl(cn_decompress_kernel<false>, grid, CODEC_THREADS, 0, cn_stream(stream), d_codes, precision, (const float *)nullptr, n, d_out, dc, vector_ok, vector_ok ? head : 0));
     cn_count_launch();
     return CN_OK;
 }

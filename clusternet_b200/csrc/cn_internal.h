@@ -46,6 +46,7 @@ struct cn_context {
     float *d_tbl = nullptr;            // 128 floats: codebook[0..125], +inf, +inf
     uint32_t *d_thr = nullptr;         // 128 words: 127 thresholds (fp32 bit patterns of |x/precision|) + 0xffffffff pad
     uint8_t *d_level_codes = nullptr;  // 128 bytes
+    void *d_code_table = nullptr;      // decision table of quotients (cn_codec.cu), null where the codebook has none
     float h_tbl[128];
     uint32_t h_thr[128];
     uint8_t h_level_codes[128];
@@ -65,6 +66,8 @@ struct cn_context {
     std::map<std::string, cn_timer_slot> timers;
 };
 
+// cn_codec.cu: the context's decision table of quotients, from h_thr and h_level_codes
+cudaError_t cn_codec_make_table(cn_context *ctx);
 // cn_gemm.cu
 void cn_gemm_workspace_free(cn_context *ctx);
 // Device status block of the context (word 0: code of the first bounded wait that ran out, read by cn_gemm_check_status),

@@ -87,8 +87,7 @@ def test_compress_config2_full_size(ctx):
 @pytest.mark.parametrize("n", [0, 1, 3, 4, 5, 2047, 8192, 100003, 1 << 20, (4 << 20) - 1, 4096 * 4096 + 2])
 def test_fused_absmax_compress_equals_the_two_calls(ctx, n):
     """cn_absmax_compress_8bit (one cooperative launch: reduce, grid barrier, code) gives the scale and the codes of
-    cn_absmax_f32 followed by cn_compress_8bit_dp, on consecutive calls and for a buffer that is not 16-byte aligned
-    (two-call fallback)."""
+    cn_absmax_f32 followed by cn_compress_8bit_dp, on consecutive calls and for a buffer that is not 16-byte aligned."""
     rng = np.random.default_rng(n + 1)
     for rep in range(3):
         x = torch.from_numpy((rng.standard_normal(n + 1) * rng.uniform(1e-3, 30)).astype(np.float32)).cuda()
@@ -103,6 +102,50 @@ def test_fused_absmax_compress_equals_the_two_calls(ctx, n):
     if n:
         p = float(pm.item())
         assert np.array_equal(got.cpu().numpy(), oracle.compress(ctx.codebook, a.cpu().numpy(), p))
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 6, 33, 127, 4097, 8191, 32770, 65539, 65536 + 7, 148 * 4096 + 5, 942785, 1442401, 4 << 20])
+@pytest.mark.parametrize("xo,co", [(0, 0), (1, 1), (2, 2), (3, 3), (1, 0), (0, 3), (2, 1), (3, 2)])
+def test_scale_and_codes_in_one_launch_at_any_alignment(ctx, n, xo, co):
+    """One launch for every size and alignment up to 4 Mi elements, codes bit for bit the oracle's, nothing written beside them; one CTA,
+    clusters, the whole chip; and the codes decoded to an output of the input's alignment."""
+    rng = np.random.default_rng(n + xo)
+    h = (rng.standard_normal(n) * rng.choice([1e-3, 1.0, 40.0])).astype(np.float32)
+    h[rng.integers(0, n, max(1, n // 50))] = 0.0
+    h[rng.integers(0, n, max(1, n // 50))] *= np.float32(1e-9)
+    if n > 100:
+        h[[5, 50]] = np.nan, -0.0
+    h[0] = 50.0
+    buf = torch.full((n + 8,), 1e30, device="cuda")
+    x = buf[xo:xo + n]
+    x.copy_(torch.from_numpy(h))
+    codes, scale = torch.full((n + 8,), 77, dtype=torch.uint8, device="cuda"), torch.empty(1, device="cuda")
+    n0 = ctx.lib.cn_kernel_launches()
+    ctx.absmax_compress(x, scale=scale, out=codes[co:co + n])
+    assert ctx.lib.cn_kernel_launches() - n0 == 1
+    ctx.gemm_check()
+    p = float(np.nanmax(np.abs(h)))
+    assert scale.item() == p
+    want = oracle.compress(ctx.codebook, h, p)
+    assert np.array_equal(codes[co:co + n].cpu().numpy(), want)
+    assert bool((codes[:co] == 77).all()) and bool((codes[co + n:] == 77).all())
+    back = torch.full((n + 8,), 3.0, device="cuda")
+    ctx.decompress(codes[co:co + n], scale, out=back[xo:xo + n])
+    assert np.array_equal(back[xo:xo + n].cpu().numpy(), oracle.decompress(ctx.codebook, want, p))
+    assert bool((back[:xo] == 3).all()) and bool((back[xo + n:] == 3).all())
+
+
+@pytest.mark.parametrize("value", [0.0, 1e-42, 1e-38, 3e38, float("inf"), float("nan")])
+@pytest.mark.parametrize("n", [1000, 200001])
+def test_scale_and_codes_in_one_launch_of_extreme_tensors(ctx, n, value):
+    """Scales that are zero, denormal, huge or infinite, and no scale at all: the division decides, as in the two calls."""
+    x = torch.zeros(n, device="cuda")
+    x[::3] = value
+    x[1::7] = -value
+    got, scale = ctx.absmax_compress(x)
+    pm = ctx.absmax(x)
+    assert scale.item() == pm.item()
+    assert torch.equal(got, ctx.compress(x, pm))
 
 
 def test_fused_absmax_compress_replays_from_a_cuda_graph(ctx):
