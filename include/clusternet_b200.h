@@ -115,8 +115,8 @@ int cn_compress_8bit_dp(cn_context *ctx, const float *d_A, const float *d_precis
 
 /* scale = max |A|, then compression_8bit(A, scale) - the pair of calls the reference makes when the scale is not known
  * beforehand (source/test.cu:1964-1968,2108-2109: max(abs(A)) followed by compression_8bit).  Up to 4 Mi elements it is ONE
- * cooperative kernel launch: pass 1 reduces, a bounded grid-wide barrier publishes the maximum, pass 2 codes the tensor
- * out of L2; larger tensors, for which launch latency no longer matters, take two pipelined launches.
+ * kernel launch, which holds the tensor in registers while the maxima go round (in a cluster, or through a bounded grid-wide
+ * barrier of a cooperative launch); larger tensors, for which launch latency no longer matters, take two pipelined launches.
  * d_scale_out (device) receives the scale; the codes equal
  * cn_absmax_f32 + cn_compress_8bit_dp bit for bit.  Uses context scratch: calls on one context must be serialised on
  * one stream.  A barrier wait that runs out (it cannot unless the GPU is shared with a kernel that blocks half of it)
