@@ -950,7 +950,7 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
 // contiguous bytes of a column, and stores to C and, for the fused all-gather, to every peer's C (full NVLink packets).
 //
 // 32 columns where there are tiles for every SM.  Few tiles are cut into many runs, and what bounds them is how many loads a CTA has in
-// flight: 8 columns, eight partial tiles at a time (16 x 40000 . 40000 x 201, 148 runs: FIXME us with 32 columns, FIXME with 8).
+// flight: 8 columns, eight partial tiles at a time.
 template <int COLS>
 __global__ void __launch_bounds__(256)
 cn_splitk_reduce_kernel(const __grid_constant__ ReduceParams p)
