@@ -200,7 +200,7 @@ def codec_bench(ctx, torch, peaks):
             ctx.compress(xs[i], scale, out=codes[i])
 
         def fused(i):
-            # the same through cn_absmax_compress_8bit: one cooperative launch up to 4 Mi elements, above that absmax and a
+            # the same through cn_absmax_compress_8bit: one launch up to 4 Mi elements, above that absmax and a
             # compressor that loads its first tiles while absmax drains
             ctx.absmax_compress(xs[i], scale=scale, out=codes[i])
         for name, fn, bytes_per in (("compress", lambda i: ctx.compress(xs[i], p, out=codes[i]), 5),
