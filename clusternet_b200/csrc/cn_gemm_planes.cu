@@ -553,16 +553,6 @@ __device__ __forceinline__ uint32_t pl_in_first(uint32_t a)
     asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(a));
     return r;
 }
-__device__ __forceinline__ uint32_t pl_try_cluster(uint32_t bar, uint32_t parity)
-{
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-    return done;
-}
 
 // Calls f(row, k, value), by whole warps and in a fixed order, for the left-overs of `blocks` blocks of 16 rows from block b0 on with
 // k in [64 k0, 64 k1).
@@ -684,8 +674,8 @@ cn_gemm_planes_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
                     const bool first = st == k0 || (st & (p.chain - 1)) == 0;
                     if (first) {   // both CTAs' drain warps must have emptied this accumulator
                         const uint32_t parity = ((chains >> 1) & 1u) ^ 1u;
-                        ok = pl_try_cluster(accempty_bar(ab), parity) != 0u || (mbar_wait(accempty_bar(ab), parity, abort_flag, p.status, 21u) &&
-                                                                                 pl_try_cluster(accempty_bar(ab), parity) != 0u);
+                        ok = mbar_try_cluster(accempty_bar(ab), parity) != 0u || (mbar_wait(accempty_bar(ab), parity, abort_flag, p.status, 21u) &&
+                                                                                 mbar_try_cluster(accempty_bar(ab), parity) != 0u);
                         if (!ok) break;
                     }
                     ok = mbar_wait(full_bar(s), (it / Cfg::STAGES) & 1u, abort_flag, p.status, 22u);

@@ -11,17 +11,27 @@
 //     k-step as CN_GEMM_3XTF32 promises, one for CN_GEMM_TF32; one thread issues them;
 //   * the accumulator tile has the rows m in tensor memory's lanes, so that a warp holds 32 consecutive rows of a column: it sends
 //     and stores whole lines of 128 bytes without turning anything;
-//   * the CTAs of a cluster share a tile: each multiplies its part of K, sends every other CTA its columns of the partial tile
-//     through distributed shared memory, adds the parts it received in K order (reproducible), and finishes its columns: bias,
-//     activation, stores to C and, for the fused all-gather, to the peers.
+//   * the CTAs of a cluster (up to eight, any number) share a tile: each multiplies its part of K, sends every other CTA its columns of the
+//     partial tile through distributed shared memory, adds the parts it received in K order (reproducible), and finishes its columns:
+//     bias, activation, stores to C and, for the fused all-gather, to the peers.
 // The tensor core's accumulator truncates, so a share of K is cut into as many chains as tensor memory holds accumulators for, and the
 // chains are added in round-to-nearest fp32.  The products with a low part have accumulators of their own, which costs no instruction (one
 // MMA multiplies the activations' high parts with both parts of the weights, whose rows lie behind one another): an addition
 // truncates what it adds to a large sum.
 //
-// Bound by latency and, per block of K, by the instructions that load and split it and the MMAs' trips to shared memory (0.7 us).  In a
-// series, with tiles of 128 columns n in the lanes, partial tiles of 64 KB through the cluster and output by way of shared memory before:
-// 128 x 784 . 784 x 1024 14.3 -> 10.9 us, 128 x 1200 . 1200 x 10 13.5 -> 7.4, weight gradient 1200 x 128 . 128 x 1200 16.3 -> 9.0.
+// Bound by latency and, per block of K, by shared memory: the feeding warps write, and the MMAs read, 64 to 144 KB of it, 0.6 us at 128
+// bytes per clock for tiles of 128 columns.  In a series, with tiles of 128 columns n in the lanes, partial tiles of 64 KB through the cluster
+// and output by way of shared memory before: 128 x 784 . 784 x 1024 14.3 -> 10.9 us, 128 x 1200 . 1200 x 10 13.5 -> 7.4, weight gradient
+// 1200 x 128 . 128 x 1200 16.3 -> 9.0.
+//
+// The exchange.  Distributed shared memory takes about 20 bytes per clock from a CTA.  Sent as single floats between two barriers of the
+// cluster, and added and stored a float at a time, a tile of 128 columns took 11 300 of the kernel's 19 000 clocks (by clock64 in a copy of it:
+// 3500 until a CTA had sent, 4100 until all had, 3700 to finish).  Now a lane sends four columns of its row at once, st.async counts the
+// bytes at the receiver's mbarrier (no release has to wait for every store's acknowledgement), a CTA's own share stays where it is, and the
+// sums of four columns are one pass over the senders with a single copy of the activation's code, which a launch has to fetch once: 128 x
+// 784 . 784 x 1024 11.1 -> 9.3 us, 128 x 1200 . 1200 x 1200 12.6 -> 10.5, 1200 x 10 8.2 -> 7.1.  Setting the CTA up before the predecessor has
+// ended, and clusters of 3, 5, 6 and 7 where more of them fit, are in these figures.
+#include <limits.h>
 #include "cn_epilogue.cuh"
 #include "cn_gemm.h"
 #include "cn_tc.cuh"
@@ -43,11 +53,14 @@ struct SmCfg {
     static constexpr int W_TILE = NT * 128;
     static constexpr int STAGE_BYTES = 2 * (SM_A_TILE + W_TILE);   // A hi, A lo, W hi, W lo
     static constexpr int RING_BYTES = SM_STAGES * STAGE_BYTES;
-    static constexpr int PART_BYTES = SM_BM * NT * 4;              // what the cluster's CTAs send: [sender][column][128 m]
+    // what the cluster's CTAs send: [sender][four columns][128 m] float4
+    static constexpr int part_bytes(int cluster) { return cluster > 1 ? cluster * ((NT / 4 + cluster - 1) / cluster) * SM_BM * 16 : 0; }
     // An accumulator has NT columns for the products of the high parts and, in the 3x mode, NT for those with a low part
     static constexpr int ACC_COLS = MODE3X ? 2 * NT : NT;
     static constexpr int MAX_CHAINS = 512 / ACC_COLS < 8 ? 512 / ACC_COLS : 8;
-    static constexpr int smem(int cluster) { return 1024 + RING_BYTES + (cluster > 1 ? PART_BYTES : 0); }
+    static constexpr int smem(int cluster) { return 1024 + RING_BYTES + part_bytes(cluster); }
+    static constexpr int SMEM_MAX = 1024 + RING_BYTES + (NT / 4 + SM_MAX_CLUSTER - 1) * SM_BM * 16;
+    static_assert(SMEM_MAX <= 232448 - 1024, "shared memory");
 };
 
 // An operand: element (row, k) at p[row * sr + k * sk].
@@ -66,6 +79,7 @@ struct SmallParams {
     int act;
     int tiles_m;
     int cluster;
+    int per, per_inv;       // of a tile's columns, in fours, those that a CTA of the cluster finishes; 65536 / per, rounded up
     int kb_total;
     unsigned int *status;
     int npeers;
@@ -90,6 +104,11 @@ __device__ __forceinline__ uint32_t sm_tf32(float x)
 __device__ __forceinline__ void sts4u(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w)
 {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+
+__device__ __forceinline__ void sts4f(uint32_t a, const float *v)
+{
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
 }
 
 // D[tmem] (+)= A[smem] * B[smem], both K-major TF32 tiles.
@@ -243,6 +262,8 @@ struct SmFeed {
     }
 };
 
+// Arrival for its order alone: what the CTAs send each other is counted by mbarriers.
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
@@ -309,11 +330,12 @@ cn_gemm_small_kernel(const __grid_constant__ SmallParams p)
 {
     using Cfg = SmCfg<NT, MODE3X>;
     extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t bars[2 * SM_STAGES + 1];
+    __shared__ __align__(8) uint64_t bars[2 * SM_STAGES + 2];
     __shared__ uint32_t s_words[2];   // tensor-memory base, abort flag
     __shared__ float s_bias[NT];
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u, part = ring + Cfg::RING_BYTES;
     const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[SM_STAGES]), acc_bar = smem_u32(&bars[2 * SM_STAGES]);
+    const uint32_t part_bar = acc_bar + 8;   // this CTA's columns of all partial tiles have arrived
     const uint32_t abort_flag = smem_u32(&s_words[1]);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int rank = blockIdx.x % p.cluster, tile = blockIdx.x / p.cluster;
@@ -321,20 +343,29 @@ cn_gemm_small_kernel(const __grid_constant__ SmallParams p)
     const int m_rows = (int)(p.M - m0 < SM_BM ? p.M - m0 : SM_BM), n_rows = (int)(p.N - n0 < NT ? p.N - n0 : NT);
     const int kb0 = p.kb_total * rank / p.cluster, n_blocks = p.kb_total * (rank + 1) / p.cluster - kb0;
     const int per_chain = (n_blocks + Cfg::MAX_CHAINS - 1) / Cfg::MAX_CHAINS, chains = (n_blocks + per_chain - 1) / per_chain;
+    // the columns of the tile in fours: this CTA finishes `per` of them, from `mine` on; those from `fours` on do not exist
+    const int per = p.per, mine = rank * per, fours = (n_rows + 3) >> 2, n_mine = fours - mine < per ? fours - mine : per;
     cn_pdl_launch_dependents();
-    if (p.cluster > 1) cluster_arrive();   // every CTA of the cluster has started: waited for before the first remote store
     if (threadIdx.x == 0) {
         for (int s = 0; s < SM_STAGES; ++s) { mbar_init(full0 + 8 * s, SM_EPI / 32); mbar_init(empty0 + 8 * s, 1); }
         mbar_init(acc_bar, 1);
+        mbar_init(part_bar, 1);
+        if (n_mine > 0) mbar_expect_tx(part_bar, (uint32_t)((p.cluster - 1) * n_mine * SM_BM * 16));
         s_words[1] = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    __syncwarp();
+    if (p.cluster > 1) cluster_arrive();   // every CTA of the cluster has started and its barriers are there: waited for before the first remote store
     uint32_t cols = 32;
     while (cols < (uint32_t)(chains * Cfg::ACC_COLS)) cols <<= 1;
     if (warp == 16) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_words[0])), "r"(cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = s_words[0];
     cn_pdl_wait();
     if (p.npeers > 0 && blockIdx.x == 0 && threadIdx.x < p.nranks && (int)threadIdx.x != p.my_rank) {
         // fused all-gather: this rank's copy of C may be overwritten by its peers (slot 0 of their flag block)
@@ -342,28 +373,16 @@ cn_gemm_small_kernel(const __grid_constant__ SmallParams p)
         volatile unsigned int *f = p.peer_flags[threadIdx.x] + p.my_rank;
         *f = p.epoch;
     }
-    // the first loads are on their way while the CTA sets itself up
     bool ok = true;
-    uint32_t tmem = 0u;
-    auto set_up = [&]() {
-        if (threadIdx.x < NT) s_bias[threadIdx.x] = p.bias && (int)threadIdx.x < n_rows ? p.bias[n0 + threadIdx.x] : 0.0f;
-        tc_fence_before();
-        __syncthreads();
-        tc_fence_after();
-        tmem = s_words[0];
-    };
     if (warp < 8) {
         SmFeed<SmShare<SM_BM, A_QUADS>, MODE3X> feed(p.A, m0, m_rows, threadIdx.x);
         feed.begin(kb0, n_blocks, p.K);
-        set_up();
+        if ((int)threadIdx.x < n_rows && p.bias) s_bias[threadIdx.x] = p.bias[n0 + threadIdx.x];
         ok = feed.run(kb0, n_blocks, p.K, ring, Cfg::STAGE_BYTES, 0, SM_A_TILE, full0, empty0, abort_flag, p.status);
     } else if (warp < 16) {
         SmFeed<SmShare<NT, W_QUADS>, MODE3X> feed(p.W, n0, n_rows, threadIdx.x - SM_FEED);
         feed.begin(kb0, n_blocks, p.K);
-        set_up();
         ok = feed.run(kb0, n_blocks, p.K, ring, Cfg::STAGE_BYTES, 2 * SM_A_TILE, 2 * SM_A_TILE + Cfg::W_TILE, full0, empty0, abort_flag, p.status);
-    } else {
-        set_up();
     }
     if (warp == 16 && lane == 0) {
         // kind::tf32 instruction descriptor: D fp32, A and B TF32 (format 2), K-major, N >> 3 at bits 17-22, M >> 4 at bits 24-28
@@ -391,7 +410,6 @@ cn_gemm_small_kernel(const __grid_constant__ SmallParams p)
         if (ok) tc_commit(acc_bar);
     }
     __syncwarp();
-    const int r_log = 31 - __clz(NT / p.cluster), R = 1 << r_log;   // columns n this CTA finishes
     if (p.cluster > 1) {
         cluster_wait();
     } else if (p.npeers > 0) {
@@ -399,6 +417,7 @@ cn_gemm_small_kernel(const __grid_constant__ SmallParams p)
         __syncthreads();
     }
     if (warp < 16) {
+        if (p.bias) asm volatile("bar.sync 1, %0;" ::"n"(SM_EPI) : "memory");   // s_bias
         ok = ok && mbar_wait(acc_bar, 0u, abort_flag, p.status, 16u);
         ok = __all_sync(0xffffffffu, ok);
         tc_fence_after();
@@ -414,11 +433,19 @@ cn_gemm_small_kernel(const __grid_constant__ SmallParams p)
                 sm_sum8<NT, MODE3X>(src + col, chains, v);
                 if (p.cluster > 1) {
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        const int dst = (col + e) >> r_log, i = (col + e) & (R - 1);
-                        uint32_t at = part + (uint32_t)((rank * R + i) * SM_BM + ml) * 4;
-                        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(at), "r"(dst));
-                        asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(at), "f"(v[e]) : "memory");
+                    for (int e = 0; e < 8; e += 4) {   // four columns of a row: 512 contiguous bytes per warp
+                        const int four = (col + e) >> 2, dst = four * p.per_inv >> 16;
+                        if (four >= fours) break;
+                        const uint32_t at = part + (uint32_t)((rank * per + four - dst * per) * SM_BM + ml) * 16;
+                        if (dst == rank) {
+                            sts4f(at, v + e);
+                            continue;
+                        }
+                        uint32_t to, bar;
+                        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(at), "r"(dst));
+                        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(part_bar), "r"(dst));
+                        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
+                                     ::"r"(to), "f"(v[e]), "f"(v[e + 1]), "f"(v[e + 2]), "f"(v[e + 3]), "r"(bar) : "memory");
                     }
                 } else if (m < p.M) {
                     float *q = p.C + (n0 + col) * p.ldc + m;
@@ -446,41 +473,60 @@ cn_gemm_small_kernel(const __grid_constant__ SmallParams p)
     }
     __syncwarp();
     tc_fence_before();
-    if (p.cluster > 1) { cluster_arrive(); cluster_wait(); }
-    else __syncthreads();
+    __syncthreads();
     if (warp == 16) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols) : "memory");
-        return;
     }
     if (p.cluster == 1) return;
-    if (p.npeers > 0) {
-        if (threadIdx.x == 0) sm_wait_peers(p);
-        asm volatile("bar.sync 1, %0;" ::"n"(SM_EPI) : "memory");
-    }
-    // this CTA's columns: n0 + rank * R + i, a row m per lane
+    cluster_arrive_relaxed();   // this CTA has sent what it sends
+    if (warp < 16) {
+        if (p.npeers > 0) {
+            if (threadIdx.x == 0) sm_wait_peers(p);
+            asm volatile("bar.sync 1, %0;" ::"n"(SM_EPI) : "memory");
+        }
+        if (ok && n_mine > 0) ok = mbar_wait(part_bar, 0u, abort_flag, p.status, 24u) && mbar_try_cluster(part_bar, 0u) != 0u;
+        // this CTA's columns, four at a time, a row m per lane
 #pragma unroll 1
-    for (int x = threadIdx.x; x < R * SM_BM; x += SM_EPI) {
-        const int i = x / SM_BM, ml = x % SM_BM, col = rank * R + i;
-        const int64_t m = m0 + ml;
-        if (col >= n_rows || m >= p.M) continue;
-        const uint32_t at = part + (uint32_t)x * 4;
-        float v = lds1(at);
-        for (int s = 1; s < p.cluster; ++s) v += lds1(at + (uint32_t)(s * R * SM_BM) * 4);
-        v = cn_apply_activation(p.bias ? v + s_bias[col] : v, p.act);
-        const int64_t off = (n0 + col) * p.ldc + m;
-        p.C[off] = v;
-        for (int d = 0; d < p.npeers; ++d) p.peerC[d][off] = v;
+        for (int x = threadIdx.x; x < n_mine * SM_BM && ok; x += SM_EPI) {
+            const int ml = x % SM_BM, col = 4 * (mine + x / SM_BM);
+            const int64_t m = m0 + ml;
+            if (m >= p.M) continue;
+            uint32_t at = part + (uint32_t)x * 16;
+            float4 v = lds4(at);
+#pragma unroll 1
+            for (int s = 1; s < p.cluster; ++s) {
+                const float4 w = lds4(at += (uint32_t)(per * SM_BM * 16));
+                v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
+            }
+            // one copy of the activations' code: it is fetched once per launch
+            int64_t off = (n0 + col) * p.ldc + m;
+#pragma unroll 1
+            for (int e = col; e < col + 4 && e < n_rows; ++e, off += p.ldc) {
+                const float y = cn_apply_activation(p.bias ? v.x + s_bias[e] : v.x, p.act);
+                v.x = v.y; v.y = v.z; v.z = v.w;
+                p.C[off] = y;
+                for (int d = 0; d < p.npeers; ++d) p.peerC[d][off] = y;
+            }
+        }
     }
+    // no CTA leaves before the others have sent; after a wait that ran out, what is under way gets a bounded chance to land
+    __syncwarp();
+    if (!ok) {
+        const long long t0 = clock64();
+        while (clock64() - t0 < 20000000LL) {}
+    }
+    __syncwarp();
+    cluster_wait();
 }
 
-// Clusters of c CTAs that the device holds at once (c = 1, 2, 4, 8): the SMs of a cluster have to lie in one GPC.
+// Clusters of c CTAs that the device holds at once: the SMs of a cluster have to lie in one GPC.
 static int max_clusters(const cn_context *ctx, int c)
 {
-    static int known[64][4] = {};
-    const int log = c == 8 ? 3 : c == 4 ? 2 : c == 2 ? 1 : 0, dev = ctx->device;
+    static int known[64][SM_MAX_CLUSTER + 1] = {};
+    const int dev = ctx->device;
     if (c == 1) return ctx->sm_count;
-    if (dev >= 0 && dev < 64 && known[dev][log] > 0) return known[dev][log];
+    if (dev >= 0 && dev < 64 && known[dev][c] > 0) return known[dev][c];
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(ctx->sm_count / c * c));
     cfg.blockDim = dim3(SM_THREADS);
@@ -493,42 +539,57 @@ static int max_clusters(const cn_context *ctx, int c)
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaFuncSetAttribute(cn_gemm_small_kernel<64, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SmCfg<64, true>::smem(2)) != cudaSuccess ||
+    if (cudaFuncSetAttribute(cn_gemm_small_kernel<64, true, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SmCfg<64, true>::SMEM_MAX) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&n, cn_gemm_small_kernel<64, true, false, false>, &cfg) != cudaSuccess || n < 1) {
         cudaGetLastError();
         n = 1;
     }
-    if (dev >= 0 && dev < 64) known[dev][log] = n;
+    if (dev >= 0 && dev < 64) known[dev][c] = n;
     return n;
 }
 
 // Columns per tile and CTAs per tile: the least of a rough model in ns, in which the blocks of K that a CTA takes (700 each) weigh most, then
-// what comes once per CTA, the exchange in the cluster, and the output.  Measured with 128 rows (columns / CTAs, us): 784 x 1024 weights 128 / 8
-// 10.8, 64 / 4 11.0, 32 / 4 11.4, 32 / 1 24; 1200 x 10 32 / 8 7.3, 128 / 8 8.8.  Clusters that wait for room cost a whole round more (784 x
-// 1024, 64 / 8: 16.6).
+// what comes once per CTA, the exchange in the cluster, and the output.  Measured with 128 rows (columns / CTAs, us): 784 x 1024 weights 64 / 5
+// 9.3, 64 / 6 9.3, 128 / 8 9.3, 64 / 4 9.9, 32 / 4 10.7, 64 / 2 14.4; 400 x 400 32 / 5 6.1, 32 / 6 6.3, 32 / 4 6.7, 128 / 8 9; 1200 x 10 32 / 8 7.0, 128 / 8
+// 7.8.  Clusters that wait for room (the GPCs hold 15 of eight or seven CTAs, 22 of six, 26 of five, 33 of four) cost a whole round more
+// (1200 x 1200, 128 / 8 10.5, 64 / 8 18.0).
 //
 // In the 3x mode blocks_per_chain bounds the accumulation chains: tiles of 128 columns leave room for two accumulators, of 64 for four, of 32
 // for eight, and a cluster of fewer CTAs makes them longer.  768 x 3873 . 3873 x 335 by four CTAs of 128 columns, 16 blocks per chain,
 // was off by 1.17e-6, the fp32 kernel by 1.12e-6; see small_chain.
+// Clusters of three, five, six or seven CTAs only with chains no longer than those of the best plan without them, on average over the blocks
+// (372 x 436 . 436 x 1512 by three CTAs in place of four was off by 2.5e-7 instead of 1.8e-7).
 struct SmallPlan {
     int nt, cluster;
     int64_t ctas;
+    double chain;   // blocks in the chain of a block, on average
 };
 static SmallPlan small_plan(const cn_context *ctx, int64_t M, int64_t N, int kb, int mode, int blocks_per_chain)
 {
-    SmallPlan best = {};
-    int64_t best_cost = INT64_MAX;
-    const int64_t tiles_m = (M + SM_BM - 1) / SM_BM;
-    for (int nt = 32; nt <= 128; nt *= 2)
-        for (int c = 1; c <= SM_MAX_CLUSTER; c *= 2) {
+    // 32-bit numbers: the shapes that come here have at most two rounds of CTAs, and this runs on every call
+    const int tiles_m = (int)((M + SM_BM - 1) / SM_BM), n32 = (int)((N + 31) / 32);
+    auto least = [&](bool any_cluster, double max_chain) {
+        SmallPlan best = {};
+        int best_cost = INT_MAX;
+        for (int c = 1; c <= SM_MAX_CLUSTER; c += any_cluster ? 1 : c) {
             if (c > 1 && kb < 2 * c) break;
-            const int chains = nt == 128 ? SmCfg<128, true>::MAX_CHAINS : nt == 64 ? SmCfg<64, true>::MAX_CHAINS : SmCfg<32, true>::MAX_CHAINS;
-            if (mode == CN_GEMM_3XTF32 && ((kb + c - 1) / c + chains - 1) / chains > blocks_per_chain) continue;
-            const int64_t tiles = tiles_m * ((N + nt - 1) / nt), rounds = (tiles + max_clusters(ctx, c) - 1) / max_clusters(ctx, c), blocks = (kb + c - 1) / c;
-            const int64_t cost = rounds * (4000 + blocks * 700 + (c == 1 ? nt * 15 : 1500 + nt * 12));
-            if (cost < best_cost) { best_cost = cost; best.nt = nt; best.cluster = c; best.ctas = tiles * c; }
+            const int more = kb % c, least_blocks = kb / c, blocks = least_blocks + (more > 0), places = max_clusters(ctx, c);
+            for (int nt = 32; nt <= 128; nt *= 2) {
+                const int chains = nt == 128 ? SmCfg<128, true>::MAX_CHAINS : nt == 64 ? SmCfg<64, true>::MAX_CHAINS : SmCfg<32, true>::MAX_CHAINS;
+                auto squares = [&](int b) { const int l = (b + chains - 1) / chains; return b / l * l * l + (b % l) * (b % l); };   // of a CTA's chains
+                const double chain = (double)(more * squares(blocks) + (c - more) * squares(least_blocks)) / kb;
+                if (mode == CN_GEMM_3XTF32 && ((blocks + chains - 1) / chains > blocks_per_chain || chain > max_chain)) continue;
+                const int tiles = tiles_m * ((n32 + nt / 32 - 1) / (nt / 32)), rounds = (tiles + places - 1) / places;
+                const int cost = rounds * (4000 + blocks * 700 + (c == 1 ? nt * 15 : 1500 + nt * 12));
+                if (cost < best_cost) {
+                    best_cost = cost;
+                    best.nt = nt; best.cluster = c; best.chain = chain; best.ctas = (int64_t)tiles * c;
+                }
+            }
         }
-    return best;
+        return best;
+    };
+    return least(true, least(false, blocks_per_chain).chain);
 }
 
 // CTAs per tile of 128 x 128 that there are SMs for, each with at least two K blocks; the measure of which products are small, and of how
@@ -578,7 +639,7 @@ static int small_launch(cn_context *ctx, const SmallParams &p, int64_t ctas, cud
     static bool attr_set[64] = {};
     const int dev = ctx->device;
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-        CN_CUDA(cudaFuncSetAttribute(cn_gemm_small_kernel<NT, MODE3X, A_QUADS, W_QUADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SmCfg<NT, MODE3X>::smem(2)));
+        CN_CUDA(cudaFuncSetAttribute(cn_gemm_small_kernel<NT, MODE3X, A_QUADS, W_QUADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, SmCfg<NT, MODE3X>::SMEM_MAX));
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
     cudaLaunchConfig_t cfg = {};
@@ -633,6 +694,8 @@ int cn_gemm_small_launch(cn_context *ctx, int transA, int transB, int64_t M, int
     p.kb_total = (int)((K + SM_BK - 1) / SM_BK);
     const SmallPlan plan = small_plan(ctx, M, N, p.kb_total, mode, small_chain(ctx, M, N, p.kb_total, p.W.vec != 0));
     p.cluster = plan.cluster;
+    p.per = (plan.nt / 4 + plan.cluster - 1) / plan.cluster;
+    p.per_inv = (65536 + p.per - 1) / p.per;
     p.status = d_status;
     p.npeers = 0;
     p.ready = nullptr; p.peer_flags = nullptr;

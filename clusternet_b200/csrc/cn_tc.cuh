@@ -29,6 +29,17 @@ __device__ __forceinline__ uint32_t mbar_try(uint32_t bar, uint32_t parity)
         : "=r"(done) : "r"(bar), "r"(parity) : "memory");
     return done;
 }
+// ... with what other CTAs of the cluster wrote before they arrived, or what their st.async brought.
+__device__ __forceinline__ uint32_t mbar_try_cluster(uint32_t bar, uint32_t parity)
+{
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+    return done;
+}
 // Shared-memory accesses by 32-bit address (half the registers of generic pointers).
 __device__ __forceinline__ float4 lds4(uint32_t a)
 {

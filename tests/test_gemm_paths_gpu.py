@@ -77,6 +77,28 @@ def test_small_products_of_every_tile(ctx, M, K, N, act):
     assert np.all(np.abs(got - want) <= bound + 1e-7)
 
 
+# clusters of 3, 5, 6 and 7 CTAs (tiles of 32, 64 and 128 columns), whose last CTAs finish fewer columns than the others, or none; last
+# tiles of a few columns, the last four of them not whole
+@pytest.mark.parametrize("M,K,N", [(149, 206, 352), (128, 614, 234), (253, 277, 1373), (100, 784, 1030), (137, 811, 615), (18, 1047, 507), (282, 580, 1467),
+                                   (328, 1561, 472), (300, 600, 601), (128, 460, 33)])
+@pytest.mark.parametrize("act", [_lib.ACT_LINEAR, _lib.ACT_RELU, _lib.ACT_LOGISTIC])
+def test_small_products_over_clusters_of_any_size(ctx, M, K, N, act):
+    rng = np.random.default_rng(M + K + N)
+    A, B = rng.standard_normal((M, K)).astype(np.float32), rng.standard_normal((K, N)).astype(np.float32)
+    bias = torch.from_numpy(rng.standard_normal(N).astype(np.float32)).cuda()
+    buf = torch.full((N + 1, M), 7.0, device="cuda")
+    C = buf[:N]
+    ctx.gemm(place(A, 0), place(B, 0), out=C, bias=bias, activation=act)
+    ctx.gemm_check()
+    assert ctx.gemm_last_kernel() == "small"
+    assert bool((buf[N] == 7.0).all())   # nothing behind the last column
+    z = A.astype(np.float64) @ B.astype(np.float64) + bias.cpu().numpy().astype(np.float64)
+    want = z if act == _lib.ACT_LINEAR else np.maximum(z, 0.0) if act == _lib.ACT_RELU else 1.0 / (1.0 + np.exp(-z))
+    # the units' slopes are at most 1; the bias and the unit are rounded once each
+    bound = REL_3X * (np.abs(A.astype(np.float64)) @ np.abs(B.astype(np.float64))) + 2.0 ** -22 * (np.abs(z) + 1.0)
+    assert np.all(np.abs(C.T.cpu().numpy() - want) <= bound)
+
+
 @pytest.mark.parametrize("mode", [_lib.GEMM_3XTF32, _lib.GEMM_TF32])
 @pytest.mark.parametrize("transA,transB", [(False, False), (True, False), (False, True)])
 @pytest.mark.parametrize("wide", ["A", "B"])
