@@ -54,6 +54,7 @@ _SIGNATURES = {
     "cn_compress_8bit": (c_int, [c_void_p, c_void_p, c_float, c_int64, c_void_p, c_void_p]),
     "cn_compress_8bit_dp": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p]),
     "cn_absmax_compress_8bit": (c_int, [c_void_p, c_void_p, c_int64, c_void_p, c_void_p, c_void_p]),
+    "cn_codec_set_patience": (c_int, [c_void_p, c_int64]),
     "cn_decompress_8bit": (c_int, [c_void_p, c_void_p, c_float, c_int64, c_void_p, c_void_p]),
     "cn_decompress_8bit_dp": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p]),
     "cn_to_col_major": (c_int, [c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_void_p]),

@@ -28,6 +28,7 @@
 // predecessor to finish (griddepcontrol.wait) - before its first access to global memory.  In a series of codec
 // calls the launch latency, the CTA start-up and the table build of call i+1 then overlap the tail of call i.
 #include <math.h>
+#include <limits.h>
 #include <string.h>
 #include <vector>
 #include "cn_internal.h"
@@ -657,19 +658,19 @@ cn_compress_ring_kernel(const float *A, float precision_arg, const float *d_prec
 // scale = absmax(A); codes = compress(A, scale) for tensors that the threads of one CTA per SM can hold in registers: 64 elements per thread,
 // 4 Mi on 148 SMs.  Every element is read once, coded after the maxima have gone round, and written once.  Bound by latency: launch,
 // one trip to memory, the exchange of the maxima, the stores.
-//   * A few CTAs are one cluster, which passes the maxima through distributed shared memory; more are a cooperative launch with a grid
-//     barrier.
+//   * A few CTAs are one cluster, which passes the maxima through distributed shared memory; more pass them through device memory (see
+//     code_exchange).
 //   * The decision table is that of the quotient |x / scale| (thresholds of the codebook, no scale in it): it is made once, when the context
-//     is, and fetched while the first loads are under way.  Elements are divided as the reference divides them, which costs less than a
-//     table for this scale, made between the barrier and the coding.
+//     is, and fetched before the predecessor has ended.  Elements are divided as the reference divides them, which costs less than a
+//     table for this scale, made between the exchange and the coding.
 //   * Any alignment: up to three elements before the first 16-byte boundary of A and after the last are coded one by one, and codes that do
 //     not lie on a 4-byte boundary then are stored as words of the lane's own and its neighbour's bytes.  (Segments of a packed
 //     gradient buffer, whose lengths are odd.)
-// Scale and codes of one tensor in a series, us, before (two passes, a table per scale) and now: 32768 elements (one cluster) 10.3, 4.4;
-// 131072 (grid barrier) 10.3, 8.2; 940800 11.4, 10.3; 2.4 M 14.4, 12.3; 4 Mi 16.4, 16.4.  With the decoder behind each: 12.3, 8.9; 14.1,
-// 9.5; 14.4, 14.3; 17.6, 16.4; 21.1, 20.5: its CTAs take a whole SM's registers, so that they wait for this kernel's to end, and the gain of a
-// tensor that fills the chip is lost again.  Scales, codes and decoded values of three tensors of odd length in a row: 44, 33 (the second and
-// third took two launches of 9 and 7 us).
+// Scale and codes of one tensor in a series, us: by two passes with a table per scale; by a cooperative launch with a barrier of atomics
+// and fences, behind which every warp read all maxima; now: 32768 elements (one cluster) 10.3, 4.0, 4.0; 131072 10.3, 8.3, 4.5; 940800 11.4,
+// 11.1, 6.7; 2.4 M 14.4, 12.5, 8.3; 4 Mi 16.4, 16.5, 10.6.  With the decoder behind each, the last two: 131072 10.3, 8.1; 940800 14.4, 9.6; 2.4 M
+// 16.5, 13.2; 4 Mi 20.6, 15.0.  Scales, codes and decoded values of three tensors of odd length in a row: 33.0, 25.4, of which 23.5 are the
+// host's six launches.
 #define CODE_THREADS 512         // at 64 registers, half an SM: the next tensor's CTAs of this kernel find room beside
 #define CODE_QUADS 8
 #define CODE_CLUSTER 8
@@ -689,33 +690,156 @@ __device__ __forceinline__ uint32_t code_one(float x, float p, uint32_t kadd, in
     return a != a ? 1u : c;   // NaN: the reference's search ends on index 1, sign clear (code 254 of a zero has the sign bit anyway)
 }
 
+// Largest of the CTAs' maxima.  A CTA stores its maximum with the launch's number in one 64-bit word, so that nothing has to be ordered; the
+// first CTA reads the words until all carry that number and stores the largest eight times, 128 bytes apart, for the others to read.  3 500
+// clocks; with the last to arrive in the first one's place, known by a counter, 5 500, with fences around that counter in place of the number
+// 8 000; where every CTA read every word, a few lines that all SMs read at once bounded the exchange, 9 000.  The number lives in device
+// memory, so that a recorded launch can be replayed; it is advanced when all CTAs have read it.
+//
+// Nothing says that all CTAs run at once: other streams' kernels may hold the SMs (a cooperative launch says so, and waits until it has
+// them all).  So no CTA waits for long.  One that runs out of patience leaves its elements to the CTA that finishes the launch, which codes them
+// behind its own, and its place to those that have not started.  The first CTA finishes the launch; where it leaves, the last to arrive does,
+// which waits until the first has done either.  Who leaves stores a word, then looks once more for what it waited for; who finishes stores the
+// scale, then looks for such words (and the last to arrive its maximum, then for the first one's): one of the two sees the other, and
+// where both do, both code the same bytes.
+struct CodeWords {
+    unsigned long long all[CN_CODE_COPIES][16];       // launch, largest maximum
+    unsigned long long part[CN_CODE_MAX_CTAS];        // by CTA: launch, its maximum
+    unsigned int left[CN_CODE_MAX_CTAS];              // by CTA: the last launch in which it left its elements
+    unsigned int launches, tickets[2];                // tickets of launches of odd and even numbers: a launch clears the next one's
+};
+static_assert(sizeof(CodeWords) <= CN_CODE_WORDS_BYTES, "allocation");
+enum { CODE_LEAVE = 0, CODE_OWN = 1, CODE_FINISH = 2 };   // what a CTA does next: nothing; its own elements; these and those that were left
+
+__device__ __forceinline__ unsigned long long code_load(const unsigned long long *at)
+{
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(at) : "memory");
+    return v;
+}
+__device__ __forceinline__ bool code_get(const unsigned long long *at, unsigned int number, float &m)
+{
+    const unsigned long long v = code_load(at);
+    if ((unsigned int)(v >> 32) != number) return false;
+    m = __uint_as_float((unsigned int)v);
+    return true;
+}
+__device__ __forceinline__ void code_put(unsigned long long *at, unsigned int number, float m)
+{
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(at), "l"((unsigned long long)number << 32 | __float_as_uint(m)) : "memory");
+}
+__device__ __forceinline__ bool code_has_left(const CodeWords *w, int cta, unsigned int number)
+{
+    return *reinterpret_cast<const volatile unsigned int *>(&w->left[cta]) == number;
+}
+__device__ __forceinline__ void code_leave(CodeWords *w, unsigned int number)
+{
+    *reinterpret_cast<volatile unsigned int *>(&w->left[blockIdx.x]) = number;
+    __threadfence();
+}
+// One warp: the words that `todo` has bits for, lane + 32 u, until they are there or the clocks have passed; at least one look.
+__device__ __forceinline__ void code_gather(float &m, uint32_t &todo, unsigned int number, const CodeWords *w, long long clocks)
+{
+    constexpr int PER_LANE = CN_CODE_MAX_CTAS / 32;
+    const long long t0 = clock64();
+    do {
+        unsigned long long v[PER_LANE];
+#pragma unroll
+        for (int u = 0; u < PER_LANE; ++u) {   // a lane's loads are under way together
+            v[u] = 0ull;
+            if (todo >> u & 1u) v[u] = code_load(&w->part[(threadIdx.x & 31) + 32 * u]);
+        }
+#pragma unroll
+        for (int u = 0; u < PER_LANE; ++u)
+            if ((todo >> u & 1u) && (unsigned int)(v[u] >> 32) == number) {
+                m = fmaxf(m, __uint_as_float((unsigned int)v[u]));
+                todo &= ~(1u << u);
+            }
+    } while (__any_sync(0xffffffffu, todo != 0u && clock64() - t0 <= clocks));
+}
+// One warp; m becomes the scale in lane 0 unless the CTA leaves.
+__device__ __forceinline__ int code_exchange(float &m, unsigned int number, CodeWords *w, long long patience, unsigned int *status)
+{
+    const int lane = threadIdx.x & 31;
+    unsigned int ticket = 0u;   // compared when it is needed: it takes as long to come as the first look at the others' words
+    if (lane == 0) {
+        code_put(&w->part[blockIdx.x], number, m);
+        ticket = atomicAdd(&w->tickets[number & 1u], 1u);
+    }
+    uint32_t todo = 0u;
+    for (int u = 0; lane + 32 * u < (int)gridDim.x; ++u) todo |= 1u << u;
+    int next = CODE_FINISH;
+    if (blockIdx.x == 0) {
+        code_gather(m, todo, number, w, patience);
+        if (__any_sync(0xffffffffu, todo != 0u)) {
+            if (__any_sync(0xffffffffu, ticket == gridDim.x - 1)) {   // all words have been stored
+                code_gather(m, todo, number, w, RING_WAIT_LIMIT);
+            } else {
+                if (lane == 0) code_leave(w, number);
+                __syncwarp();
+                code_gather(m, todo, number, w, 0);
+                if (__any_sync(0xffffffffu, todo != 0u)) return CODE_LEAVE;
+            }
+        }
+    } else {
+        if (lane == 0) {
+            const unsigned long long *all = w->all[blockIdx.x % CN_CODE_COPIES];
+            const long long t0 = clock64();
+            bool here = code_get(all, number, m);
+            const bool last = !here && ticket == gridDim.x - 1;
+            if (last) __threadfence();
+            while (!here && !(last && code_has_left(w, 0, number)) && clock64() - t0 <= (last ? RING_WAIT_LIMIT : patience)) here = code_get(all, number, m);
+            next = here ? CODE_OWN : last && code_has_left(w, 0, number) ? CODE_FINISH : CODE_LEAVE;
+            if (next == CODE_LEAVE) {
+                if (last) atomicMax(status, 13u);
+                code_leave(w, number);
+                if (code_get(all, number, m)) next = CODE_OWN;
+            }
+        }
+        next = __shfl_sync(0xffffffffu, next, 0);
+        if (next != CODE_FINISH) return next;
+        code_gather(m, todo, number, w, RING_WAIT_LIMIT);
+    }
+    if (todo != 0u) atomicMax(status, 13u);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (lane < CN_CODE_COPIES) code_put(w->all[lane], number, m);
+    if (lane == 0) {
+        *reinterpret_cast<volatile unsigned int *>(&w->tickets[(number + 1u) & 1u]) = 0u;
+        *reinterpret_cast<volatile unsigned int *>(&w->launches) = number;
+    }
+    return CODE_FINISH;
+}
+
 template <bool CLUSTER, int QUADS>
 __global__ void __launch_bounds__(CODE_THREADS, QUADS <= CODE_QUADS ? 2 : 1)
-cn_absmax_code_kernel(const float *A, int64_t n, float *scale, uint8_t *codes, const CodeTable *table, float *partials, unsigned int *barrier_words,
-                      unsigned int *status)
+cn_absmax_code_kernel(const float *A, int64_t n, float *scale, uint8_t *codes, const CodeTable *table, CodeWords *words, long long patience, unsigned int *status)
 {
     __shared__ __align__(16) uint32_t lut[LUT_MAX];
-    __shared__ float s_red[CODE_THREADS / 32], s_peer[CODE_CLUSTER];
+    __shared__ float s_red[CODE_THREADS / 32], s_peer[CODE_CLUSTER], s_max;
+    __shared__ int s_next, s_left;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     cn_pdl_launch_dependents();
     if (CLUSTER) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // all CTAs run before one writes into another
     const uint32_t kadd = table->kadd;
     const int32_t span = table->span;
     const int nb = table->nb;
+    for (int i = tid; i < nb; i += CODE_THREADS) lut[i] = table->lut[i];   // made with the context: nothing before this launch writes it
     cn_pdl_wait();
+    const unsigned int number = CLUSTER ? 0u : *reinterpret_cast<volatile unsigned int *>(&words->launches) + 1u;
     const int to16 = (int)((0 - (reinterpret_cast<uintptr_t>(A) >> 2)) & 3), head = to16 < n ? to16 : (int)n;
     const int quads = (int)((n - head) >> 2), tail = (int)(n - head) & 3;
     const float4 *A4 = reinterpret_cast<const float4 *>(A + head);
-    const int stride = gridDim.x * CODE_THREADS, q0 = blockIdx.x * CODE_THREADS + tid;
+    const int stride = gridDim.x * CODE_THREADS;
+    int cta = blockIdx.x, q0 = cta * CODE_THREADS + tid;
     float4 v[QUADS];
 #pragma unroll
     for (int u = 0; u < QUADS; ++u)
         v[u] = q0 + u * stride < quads ? A4[q0 + u * stride] : make_float4(0.f, 0.f, 0.f, 0.f);
     // the first CTA's first warps take the elements outside the quads
-    const bool single = blockIdx.x == 0 && (tid < head || (tid >= 32 && tid - 32 < tail));
+    bool single = cta == 0 && (tid < head || (tid >= 32 && tid - 32 < tail));
     const int64_t at1 = tid < 32 ? tid : head + 4 * (int64_t)quads + tid - 32;
-    const float x1 = single ? A[at1] : 0.0f;
-    for (int i = tid; i < nb; i += CODE_THREADS) lut[i] = table->lut[i];
+    float x1 = single ? A[at1] : 0.0f;
     float m = -1.0f;   // seed of the reference's reduction (source/basicOps.cu:1079)
 #pragma unroll
     for (int u = 0; u < QUADS; ++u)
@@ -741,42 +865,68 @@ cn_absmax_code_kernel(const float *A, int64_t n, float *scale, uint8_t *codes, c
         m = s_peer[0];
         for (int i = 1; i < (int)gridDim.x; ++i) m = fmaxf(m, s_peer[i]);
     } else {
-        if (tid == 0) partials[blockIdx.x] = m;
-        cdc_grid_barrier(barrier_words, barrier_words + 1, status);
-        m = -1.0f;
-        for (int i = lane; i < (int)gridDim.x; i += 32) m = fmaxf(m, __ldcg(partials + i));
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if (warp == 0) {
+            const int next = code_exchange(m, number, words, patience, status);
+            if (lane == 0) { s_max = m; s_next = next; }
+        }
+        __syncthreads();
+        m = s_max;
+        if (s_next == CODE_LEAVE) return;
     }
     const float p = m;
-    if (blockIdx.x == 0 && tid == 0) *scale = p;
+    const bool finish = CLUSTER ? blockIdx.x == 0 : s_next == CODE_FINISH;
+    if (finish && tid == 0) *scale = p;
     const uint32_t lut_addr = cdc_smem_u32(lut);
-    if (single) codes[at1] = (uint8_t)code_one(x1, p, kadd, span, lut_addr);
     // `off` bytes of a quad's codes lie before the next 4-byte boundary: the word there takes the other bytes of this lane's codes and the
     // first of the next lane's
     uint8_t *out = codes + head;
     const int off = (int)((0 - reinterpret_cast<uintptr_t>(out)) & 3u);
+    bool left = false, looked = CLUSTER;
+    for (;;) {
+        if (single) codes[at1] = (uint8_t)code_one(x1, p, kadd, span, lut_addr);
 #pragma unroll
-    for (int u = 0; u < QUADS; ++u) {
-        const int q = q0 + u * stride;
-        if (q - lane >= quads) break;   // the same for the whole warp
-        const bool mine = q < quads;
-        const uint32_t c = pack4(code_one(v[u].x, p, kadd, span, lut_addr), code_one(v[u].y, p, kadd, span, lut_addr),
-                                 code_one(v[u].z, p, kadd, span, lut_addr), code_one(v[u].w, p, kadd, span, lut_addr));
-        if (off == 0) {
-            if (mine) reinterpret_cast<uint32_t *>(out)[q] = c;
-            continue;
+        for (int u = 0; u < QUADS; ++u) {
+            const int q = q0 + u * stride;
+            if (q - lane >= quads) break;   // the same for the whole warp
+            const bool mine = q < quads;
+            const uint32_t c = pack4(code_one(v[u].x, p, kadd, span, lut_addr), code_one(v[u].y, p, kadd, span, lut_addr),
+                                     code_one(v[u].z, p, kadd, span, lut_addr), code_one(v[u].w, p, kadd, span, lut_addr));
+            if (off == 0) {
+                if (mine) reinterpret_cast<uint32_t *>(out)[q] = c;
+                continue;
+            }
+            const uint32_t next = __shfl_down_sync(0xffffffffu, c, 1);
+            if (!mine) continue;
+            uint8_t *at = out + 4 * (int64_t)q;
+            if (lane == 0)
+                for (int b = 0; b < off; ++b) at[b] = (uint8_t)(c >> (8 * b));
+            if (lane < 31 && q < quads - 1) {
+                *reinterpret_cast<uint32_t *>(at + off) = __funnelshift_r(c, next, 8 * off);
+            } else {
+                for (int b = off; b < 4; ++b) at[b] = (uint8_t)(c >> (8 * b));
+            }
         }
-        const uint32_t next = __shfl_down_sync(0xffffffffu, c, 1);
-        if (!mine) continue;
-        uint8_t *at = out + 4 * (int64_t)q;
-        if (lane == 0)
-            for (int b = 0; b < off; ++b) at[b] = (uint8_t)(c >> (8 * b));
-        if (lane < 31 && q < quads - 1) {
-            *reinterpret_cast<uint32_t *>(at + off) = __funnelshift_r(c, next, 8 * off);
-        } else {
-            for (int b = off; b < 4; ++b) at[b] = (uint8_t)(c >> (8 * b));
+        if (CLUSTER || !finish) return;
+        if (!looked) {
+            // whether CTA number `tid` has left its elements
+            if (warp == 0) __threadfence();   // the scale is stored before the words are looked at
+            __syncthreads();
+            left = tid < (int)gridDim.x && tid != (int)blockIdx.x && code_has_left(words, tid, number);
+            looked = true;
         }
+        if (tid == 0) s_left = INT_MAX;
+        if (!__syncthreads_or(left)) return;
+        if (left) atomicMin(&s_left, tid);
+        __syncthreads();
+        cta = s_left;
+        if (tid == cta) left = false;
+        __syncthreads();
+        q0 = cta * CODE_THREADS + tid;
+#pragma unroll
+        for (int u = 0; u < QUADS; ++u)
+            v[u] = q0 + u * stride < quads ? A4[q0 + u * stride] : make_float4(0.f, 0.f, 0.f, 0.f);
+        single = cta == 0 && (tid < head || (tid >= 32 && tid - 32 < tail));
+        if (single) x1 = A[at1];
     }
 }
 
@@ -950,22 +1100,23 @@ cn_decompress_kernel(const uint8_t *codes, float precision_arg, const float *d_p
     __shared__ float lut[256];
     const int tid = threadIdx.x;
     cn_pdl_launch_dependents();
-    if (PRECISION_ON_DEVICE) cn_pdl_wait();   // the scale is in global memory; a host scale lets the table precede the wait
-    const float p = PRECISION_ON_DEVICE ? *d_precision : precision_arg;
-    if (tid < 256) {
-        float v = 0.0f;
-        const int i = tid & 127;
-        if (i < CN_CODEBOOK_N) {
-            v = __fmul_rn(dc.tbl[i], p);
-            if (tid >= 128) v = -v;
-        } else {
-            v = (tid == 255) ? -p : p;   // 126, 127, 254 -> +precision; 255 -> -precision
+    auto make_table = [&](float p) {
+        if (tid < 256) {
+            float v = 0.0f;
+            const int i = tid & 127;
+            if (i < CN_CODEBOOK_N) {
+                v = __fmul_rn(dc.tbl[i], p);
+                if (tid >= 128) v = -v;
+            } else {
+                v = (tid == 255) ? -p : p;   // 126, 127, 254 -> +precision; 255 -> -precision
+            }
+            lut[tid] = v;
         }
-        lut[tid] = v;
-    }
-    if (!PRECISION_ON_DEVICE) cn_pdl_wait();
-    __syncthreads();
-    if (blockIdx.x == 0 && tid < head) out[tid] = lut[codes[tid]];
+    };
+    if (!PRECISION_ON_DEVICE) make_table(precision_arg);   // a host scale lets the table precede the wait
+    cn_pdl_wait();
+    const uint8_t *first = codes;
+    float *first_out = out;
     codes += head;
     out += head;
     n -= head;
@@ -975,39 +1126,34 @@ cn_decompress_kernel(const uint8_t *codes, float precision_arg, const float *d_p
     const int64_t nvec = vector_ok ? (n >> 2) : 0;
     int64_t v = (int64_t)blockIdx.x * blockDim.x + tid;
     const uint32_t *in4 = reinterpret_cast<const uint32_t *>(codes);
+    // the first codes are on their way while the table is made
+    uint32_t cur[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+        if (v + u * stride < nvec) cur[u] = __ldcs(in4 + v + u * stride);
+    if (PRECISION_ON_DEVICE) make_table(*d_precision);
+    __syncthreads();
+    if (blockIdx.x == 0 && tid < head) first_out[tid] = lut[first[tid]];
     if (v + 3 * stride < nvec) {
         const int64_t step = 4 * stride;
-        uint32_t cur[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) cur[u] = __ldcs(in4 + v + u * stride);
         while (true) {
             const int64_t vn = v + step;
             const bool more = vn + 3 * stride < nvec;
             uint32_t nxt[4];
-            if (more) {
 #pragma unroll
-                for (int u = 0; u < 4; ++u) nxt[u] = __ldcs(in4 + vn + u * stride);
-            }
+            for (int u = 0; u < 4; ++u)
+                if (vn + u * stride < nvec) nxt[u] = __ldcs(in4 + vn + u * stride);
 #pragma unroll
             for (int u = 0; u < 4; ++u) __stcs(out4 + v + u * stride, CN_DEC4(cur[u]));
             v = vn;
-            if (!more) break;
 #pragma unroll
             for (int u = 0; u < 4; ++u) cur[u] = nxt[u];
+            if (!more) break;
         }
     }
-    if (v < nvec) {   // last, partial group: all its loads are issued before any is used
-        uint32_t q[3];
-        bool has[3];
 #pragma unroll
-        for (int u = 0; u < 3; ++u) {
-            has[u] = v + u * stride < nvec;
-            if (has[u]) q[u] = __ldcs(in4 + v + u * stride);
-        }
-#pragma unroll
-        for (int u = 0; u < 3; ++u)
-            if (has[u]) __stcs(out4 + v + u * stride, CN_DEC4(q[u]));
-    }
+    for (int u = 0; u < 3; ++u)   // last, partial group
+        if (v + u * stride < nvec) __stcs(out4 + v + u * stride, CN_DEC4(cur[u]));
 #undef CN_DEC4
     for (int64_t i = (nvec << 2) + (int64_t)blockIdx.x * blockDim.x + tid; i < n; i += stride) out[i] = lut[codes[i]];
 }
@@ -1449,6 +1595,13 @@ cudaError_t cn_codec_make_table(cn_context *ctx)
     return e;
 }
 
+extern "C" int cn_codec_set_patience(cn_context *ctx, int64_t clocks)
+{
+    CN_REQUIRE(ctx && clocks >= 0, CN_ERR_ARG, "cn_codec_set_patience: bad argument");
+    ctx->code_patience = clocks;
+    return CN_OK;
+}
+
 static int absmax_code(cn_context *ctx, const float *d_A, int64_t n, float *d_scale, uint8_t *d_codes, void *stream)
 {
     unsigned int *d_status = nullptr;
@@ -1461,6 +1614,7 @@ static int absmax_code(cn_context *ctx, const float *d_A, int64_t n, float *d_sc
     int64_t grid = (n + per_cta - 1) / per_cta;
     if (cluster) grid = grid <= 1 ? 1 : grid <= 2 ? 2 : grid <= 4 ? 4 : CODE_CLUSTER;
     else if (grid > ctx->sm_count) grid = ctx->sm_count;
+    CN_REQUIRE(grid <= CN_CODE_MAX_CTAS, CN_ERR_UNSUPPORTED, "cn_absmax_compress_8bit: more SMs than words");
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(CODE_THREADS);
@@ -1473,17 +1627,15 @@ static int absmax_code(cn_context *ctx, const float *d_A, int64_t n, float *d_sc
         attr[1].val.clusterDim.x = (unsigned)grid;
         attr[1].val.clusterDim.y = 1;
         attr[1].val.clusterDim.z = 1;
-    } else {
-        attr[1].id = cudaLaunchAttributeCooperative;
-        attr[1].val.cooperative = 1;
     }
-    cfg.numAttrs = 2;
+    cfg.numAttrs = cluster ? 2 : 1;
     cfg.attrs = attr;
     const CodeTable *table = (const CodeTable *)ctx->d_code_table;
-    unsigned int *barrier_words = ctx->d_ticket + 4;   // words 4, 5 of the ticket block: arrival count, generation
-    if (cluster) CN_CUDA(cudaLaunchKernelEx(&cfg, cn_absmax_code_kernel<true, CODE_CLUSTER_QUADS>, d_A, n, d_scale, d_codes, table, ctx->d_partials, barrier_words, d_status));
-    else if (n <= per_cta * CODE_QUADS * ctx->sm_count - 4) CN_CUDA(cudaLaunchKernelEx(&cfg, cn_absmax_code_kernel<false, CODE_QUADS>, d_A, n, d_scale, d_codes, table, ctx->d_partials, barrier_words, d_status));
-    else CN_CUDA(cudaLaunchKernelEx(&cfg, cn_absmax_code_kernel<false, 2 * CODE_QUADS>, d_A, n, d_scale, d_codes, table, ctx->d_partials, barrier_words, d_status));
+    CodeWords *words = (CodeWords *)ctx->d_code_words;
+    const long long patience = ctx->code_patience;
+    if (cluster) CN_CUDA(cudaLaunchKernelEx(&cfg, cn_absmax_code_kernel<true, CODE_CLUSTER_QUADS>, d_A, n, d_scale, d_codes, table, words, patience, d_status));
+    else if (n <= per_cta * CODE_QUADS * ctx->sm_count - 4) CN_CUDA(cudaLaunchKernelEx(&cfg, cn_absmax_code_kernel<false, CODE_QUADS>, d_A, n, d_scale, d_codes, table, words, patience, d_status));
+    else CN_CUDA(cudaLaunchKernelEx(&cfg, cn_absmax_code_kernel<false, 2 * CODE_QUADS>, d_A, n, d_scale, d_codes, table, words, patience, d_status));
     cn_count_launch();
     return CN_OK;
 }

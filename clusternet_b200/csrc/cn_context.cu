@@ -496,6 +496,8 @@ extern "C" int cn_context_create(int device, const float *codebook, cn_context *
         (e = cudaMemcpy(c->d_thr, c->h_thr, 128 * sizeof(uint32_t), cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaMemcpy(c->d_level_codes, c->h_level_codes, 128, cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaMemset(c->d_ticket, 0, 64)) != cudaSuccess ||
+        (e = cudaMalloc(&c->d_code_words, CN_CODE_WORDS_BYTES)) != cudaSuccess ||
+        (e = cudaMemset(c->d_code_words, 0, CN_CODE_WORDS_BYTES)) != cudaSuccess ||
         (e = cudaMalloc(&c->d_status, 64)) != cudaSuccess ||
         (e = cudaMemset(c->d_status, 0, 64)) != cudaSuccess ||
         (e = cn_codec_make_table(c)) != cudaSuccess) {
@@ -523,6 +525,7 @@ extern "C" int cn_context_destroy(cn_context *c)
     cudaFree(c->d_status);
     cudaFree(c->d_partials);
     cudaFree(c->d_ticket);
+    cudaFree(c->d_code_words);
     delete c;
     return CN_OK;
 }

@@ -11,6 +11,9 @@
 #define CN_NUM_THR 127      // decision thresholds of the compressor
 #define CN_NUM_LEVELS 128   // levels they separate: 254, 0..125, 127
 #define CN_MAX_PARTIALS 4096
+#define CN_CODE_MAX_CTAS 256
+#define CN_CODE_COPIES 8
+#define CN_CODE_WORDS_BYTES 8192
 
 void cn_set_error(const char *fmt, ...);
 // every kernel launch of the library is counted (cn_kernel_launches), so that callers can tell library work from fallbacks
@@ -57,7 +60,9 @@ struct cn_context {
     uint32_t codec_cache_X[128];
     // reduction scratch: per-CTA partial maxima + a ticket counter that the last CTA resets
     float *d_partials = nullptr;
-    unsigned int *d_ticket = nullptr;   // 64 bytes: word 0 = absmax ticket, words 4 and 5 = grid barrier of the fused compressor (arrivals, generation)
+    unsigned int *d_ticket = nullptr;   // 64 bytes: word 0 = absmax ticket, words 4 and 5 = grid barrier of the compressor that pushes (arrivals, generation)
+    void *d_code_words = nullptr;       // what the CTAs of the compressor that finds its scale exchange (CodeWords in cn_codec.cu)
+    int64_t code_patience = 400000;     // clocks for which its CTAs wait for the scale, see code_exchange: 0.2 ms
     // GEMM
     cn_gemm_workspace *gemm = nullptr;
     const char *gemm_last_path = "";

@@ -148,6 +148,25 @@ def test_scale_and_codes_in_one_launch_of_extreme_tensors(ctx, n, value):
     assert torch.equal(got, ctx.compress(x, pm))
 
 
+@pytest.mark.parametrize("n,off", [(32770, 0), (65539, 3), (148 * 2048 + 1, 1), (942785, 2), (148 * 512 * 32 + 5, 0), (4 << 20, 1)])
+@pytest.mark.parametrize("clocks", [0, 3000])
+def test_scale_and_codes_where_ctas_do_not_wait(ctx, n, off, clocks):
+    """CTAs that leave their elements to the last one (all others, or those that come first), the first CTA and its elements outside the
+    quads among them: the same scale and codes, call after call, nothing written beside them."""
+    try:
+        cn.check(ctx.lib.cn_codec_set_patience(ctx.h, clocks))
+        for rep in range(4):
+            x = (torch.randn(n + 8, device="cuda") * 10.0 ** -rep)[off:off + n]   # a scale of the call before would be too large
+            codes, scale = torch.full((n + 8,), 77, dtype=torch.uint8, device="cuda"), torch.empty(1, device="cuda")
+            ctx.absmax_compress(x, scale=scale, out=codes[off:off + n])
+            assert scale.item() == x.abs().max().item()
+            want = oracle.compress(ctx.codebook, x.cpu().numpy(), scale.item())
+            assert np.array_equal(codes[off:off + n].cpu().numpy(), want)
+            assert bool((codes[:off] == 77).all()) and bool((codes[off + n:] == 77).all())
+    finally:
+        cn.check(ctx.lib.cn_codec_set_patience(ctx.h, 400000))
+
+
 def test_fused_absmax_compress_replays_from_a_cuda_graph(ctx):
     """The one-launch form keeps its grid barrier's state on the device only, so a recorded launch can be replayed: every
     replay must wait for ITS maxima.  The data shrink from replay to replay - a barrier that let a CTA through early would
