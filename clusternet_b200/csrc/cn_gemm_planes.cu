@@ -22,7 +22,8 @@
 //
 // Bound by the tensor cores (their pipe is busy in 80 % of the cycles at 2048 x 4096 . 4096 x 4096): 4096^3, 3x mode, 245 us of the product's 340 at 1.68 PFLOP/s of fp16, against 476 us on the streaming
 // kernel (2048 rows 187 / 263, 1024 rows 120 / 142; single pass 184 / 392); the pre-pass moves 256 MB in 60 us, the reduction of the cut
-// tail takes 13, the launch that ends at once 3.  Short K is bound by the drain warps and the stores: 4096 x 128 . 128 x 4096 48 / 53 us.
+// tail takes 13, the launch that ends at once 3.  Short K is bound by the drain warps and the stores: 4096 x 128 . 128 x 4096 44 us with 32-byte
+// stores from registers, 39 by TMA (see the epilogue); 1320 x 144 . 144 x 1872 with ReLU 27 -> 23.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include "cn_epilogue.cuh"
@@ -429,17 +430,24 @@ cn_act_planes_kernel(const __grid_constant__ ActJob job0, const __grid_constant_
 #define PL_REGS_DRAIN 224
 static_assert(PL_REGS_WG0 + 2 * PL_REGS_DRAIN <= 3 * (65536 / PL_THREADS / 8 * 8), "registers");
 
-template <bool MODE3X>
+// SHORT: tiles of up to PL_SHORT_K k.  A third of the stages makes room for what the drain warps have on its way to C: with two blocks each
+// they waited for most of a tile's stores (6900 clocks of 10 400 per tile at 4096 x 128 . 128 x 4096).
+// In the single pass, whose tiles take a third of the MMAs, three times as long ones.  Not with logistic units, which bound the drain warps.
+#define PL_SHORT_K 256
+#define PL_DIRECT_STAGES 12   // of 64 k: up to here logistic units go to C from registers
+template <bool MODE3X, bool SHORT>
 struct PlCfg {
     static constexpr int PARTS = MODE3X ? 2 : 1;
-    static constexpr int STAGES = MODE3X ? 3 : 6;
+    static constexpr int STAGES = (MODE3X ? 3 : 6) * (SHORT ? 2 : 3) / 3;
+    static constexpr int BATCH = SHORT ? 3 : 1, OUT = 2 * BATCH;    // blocks of output that a drain warp hands over together; that it has room for
     static constexpr int STAGE_BYTES = 2 * PARTS * PL_TILE_BYTES;   // W parts, then activation parts
-    static constexpr int AS_OFF = STAGES * STAGE_BYTES;             // [2 chains][256] inverse scales of the activation rows
+    static constexpr int TURN_OFF = STAGES * STAGE_BYTES;           // [drain warp][OUT] blocks of 16 rows m x 32 columns n
+    static constexpr int TURN_BYTES = OUT * 2048;
+    static constexpr int AS_OFF = TURN_OFF + 8 * TURN_BYTES;        // [2 chains][256] inverse scales of the activation rows
     static constexpr int BAR_OFF = AS_OFF + 2 * 256 * 4;
     static constexpr int BARS = 2 * STAGES + 4;
-    static constexpr int HOLD_OFF = BAR_OFF + BARS * 8;
-    static constexpr int TURN_OFF = (HOLD_OFF + 16 + 127) & ~127;   // a block of 32 columns n x 32 rows m per drain warp
-    static constexpr int SMEM_BYTES = TURN_OFF + 8 * 4096 + 768;    // the base is 256-byte aligned, the stages want 1024
+    static constexpr int HOLD_OFF = BAR_OFF + BARS * 8;             // tensor-memory base, abort flag, whether the streaming kernel does it
+    static constexpr int SMEM_BYTES = HOLD_OFF + 16 + 768;          // the base is 256-byte aligned, the stages want 1024
     static_assert(SMEM_BYTES <= 232448, "shared memory");
 };
 
@@ -449,6 +457,7 @@ struct PlParams {
     int64_t ldc;
     const float *bias;
     int act;
+    int tma_out;            // C has 16-byte aligned columns: tm_c
     int tiles_m;
     int half;               // rows m per CTA and per drain warpgroup: a tile has twice as many; a multiple of 16, at most 128
     int full_tiles, tiles;  // tiles [0, full_tiles) by one pair each, the others cut into runs over tail_pairs pairs
@@ -532,6 +541,11 @@ __device__ __forceinline__ void pl_load(uint32_t dst, const CUtensorMap *map, ui
         "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
         ::"r"(dst), "l"((uint64_t)map), "r"(bar), "r"(x), "r"(y), "r"(z) : "memory");
 }
+// A block of 16 rows m by 32 columns n from shared memory to C; what lies outside C is left out.
+__device__ __forceinline__ void pl_store(const CUtensorMap *map, uint32_t src, int32_t m, int32_t n)
+{
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"((uint64_t)map), "r"(src), "r"(m), "r"(n) : "memory");
+}
 // 16 columns of tensor memory, and the wait for them (which the registers pass through, so that no use moves before it).
 __device__ __forceinline__ void pl_ld16(uint32_t taddr, uint32_t (&r)[16])
 {
@@ -584,6 +598,7 @@ __device__ __forceinline__ void pl_cells(const uint8_t *counts, const uint2 *cel
 __device__ __forceinline__ uint32_t pl_first(const uint8_t *counts, int groups, int64_t b0, int blocks, int k0, int k1)
 {
     const int g0 = k0 / (TC_GROUP_K / TC_AK), ng = (k1 - 1) / (TC_GROUP_K / TC_AK) + 1 - g0, i = threadIdx.x & 31;
+    if (ng == 1) return i < blocks ? __ldcg(counts + (b0 + i) * groups + g0) : 0u;   // without the divisions, on every short tile's way
     return i < blocks * ng ? __ldcg(counts + (b0 + i / ng) * groups + g0 + i % ng) : 0u;
 }
 __device__ __forceinline__ bool pl_any(uint32_t any, const uint8_t *counts, int groups, int64_t b0, int blocks, int k0, int k1)
@@ -593,18 +608,18 @@ __device__ __forceinline__ bool pl_any(uint32_t any, const uint8_t *counts, int 
     return __any_sync(0xffffffffu, any != 0u);
 }
 
-template <bool MODE3X>
+template <bool MODE3X, bool SHORT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PL_THREADS, 1)
-cn_gemm_planes_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ PlParams p)
+cn_gemm_planes_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_c, const __grid_constant__ PlParams p)
 {
-    using Cfg = PlCfg<MODE3X>;
+    using Cfg = PlCfg<MODE3X, SHORT>;
     extern __shared__ __align__(256) uint8_t smem_raw[];
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     auto full_bar = [&](int s) { return smem_base + Cfg::BAR_OFF + 8u * s; };                             // first CTA: both CTAs' tiles have landed
     auto empty_bar = [&](int s) { return smem_base + Cfg::BAR_OFF + 8u * (Cfg::STAGES + s); };            // each CTA: the stage has been multiplied
     auto accfull_bar = [&](int b) { return smem_base + Cfg::BAR_OFF + 8u * (2 * Cfg::STAGES + b); };      // each CTA
     auto accempty_bar = [&](int b) { return smem_base + Cfg::BAR_OFF + 8u * (2 * Cfg::STAGES + 2 + b); }; // first CTA: both CTAs have drained it
-    const uint32_t tmem_holder = smem_base + Cfg::HOLD_OFF, abort_flag = tmem_holder + 4;
+    const uint32_t tmem_holder = smem_base + Cfg::HOLD_OFF, abort_flag = tmem_holder + 4, skip_flag = tmem_holder + 8;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = blockIdx.x & 1u;
     cn_pdl_launch_dependents();
@@ -613,19 +628,28 @@ cn_gemm_planes_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
         for (int b = 0; b < 2; ++b) { mbar_init(accfull_bar(b), 1); mbar_init(accempty_bar(b), 16); }
         sts1u(abort_flag, 0u);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        tma_prefetch_map(&tm_w);
+        tma_prefetch_map(&tm_a);
+        if (p.tma_out) tma_prefetch_map(&tm_c);
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_holder), "r"(512u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
-    cn_pdl_wait();
-    const bool skip = __ldcg(p.many + (CN_STATUS_OVERFLOW - CN_STATUS_MANY)) != 0u;
     tc_fence_before();
     __syncthreads();
-    if (blockIdx.x == 0 && threadIdx.x == 0) *p.many = skip ? 1u : 0u;
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cn_pdl_wait();
+    // one thread looks at the word: the reads of every warp of all CTAs meet in one line
+    if (threadIdx.x == 0) {
+        const bool over = __ldcg(p.many + (CN_STATUS_OVERFLOW - CN_STATUS_MANY)) != 0u;
+        if (blockIdx.x == 0) *p.many = over ? 1u : 0u;
+        sts1u(skip_flag, over ? 1u : 0u);
+    }
+    __syncthreads();
     tc_fence_after();
+    const bool skip = lds1u(skip_flag) != 0u;
     const uint32_t tmem_base = lds1u(tmem_holder);
 
     if (skip) {
@@ -718,7 +742,7 @@ cn_gemm_planes_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
         const uint32_t src0 = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(wg * half);
         PlWalk walk(p);
         int tile, k0, k1, slot;
-        uint32_t chains = 0;
+        uint32_t chains = 0, out_it = 0;
         bool ok = true, more = walk.next(p, tile, k0, k1, slot);
         // of a run, fetched while the one before it is stored: the first group's inverse scales, and whether it has left-overs
         int64_t n, m0, ma, nw, wb, ab0;
@@ -843,12 +867,64 @@ cn_gemm_planes_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
                     if (i * 4 < half) P[i * TC_BN] = make_ulonglong2(sum[2 * i], sum[2 * i + 1]);
                 continue;
             }
-            // Every lane holds a column of its own and may store 32 bytes at a time, which fill whole sectors of L2 and leave shared memory
-            // to the tensor cores.  4096 x 128 . 128 x 4096: 48 us, 54 by
-            // way of shared memory
-            if (mt + half <= p.M && (p.ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(p.C) & 31u) == 0) {
-                float *q = p.C + (nw0 + lane) * p.ldc + mt;
-                if (p.act == CN_ACT_LOGISTIC) {   // its code is long: a copy of the loop to itself
+            // Every lane holds a column of its own.  Blocks of 16 rows x 32 columns go through buffers of shared memory, 16-byte chunks
+            // permuted as the tensor map says, which keeps eight lanes that store together apart, and from there to C by TMA while the warp
+            // fills another one or has gone on to the next tile.  Short code: a launch fetches it once, and 128 values with a bias and a choice of
+            // units each took 15000 clocks of the first tile.  32-byte stores from registers, each lane into a column of
+            // its own, took 8400 clocks per tile, in which nothing was drained.
+            const uint32_t turn = smem_base + Cfg::TURN_OFF + (uint32_t)((warp - 4) * Cfg::TURN_BYTES);
+            if (p.bias) {
+                const uint64_t bias2 = tc_pack2(bias, bias);
+#pragma unroll
+                for (int i = 0; i < 64; ++i) sum[i] = tc_add2(sum[i], bias2);
+            }
+            if (p.tma_out) {
+                const int blocks = nw0 < p.N && mt < p.M ? ((int)(p.M - mt < half ? p.M - mt : half) + 15) >> 4 : 0;
+                const uint32_t turned = (uint32_t)(lane >> 1 & 3) * 16u;
+                // room for the next BATCH blocks, when the batch before the last has left it
+                auto take = [&]() {
+                    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                    __syncwarp();
+                    return turn + (out_it++ & 1u) * (Cfg::BATCH * 2048u);
+                };
+                auto put = [&](uint32_t buf, int i, auto unit) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        float v[4];
+                        tc_unpack2(sum[8 * i + 2 * c], v[0], v[1]);
+                        tc_unpack2(sum[8 * i + 2 * c + 1], v[2], v[3]);
+                        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(buf + (uint32_t)lane * 64u + ((uint32_t)c * 16u ^ turned)), "f"(unit(v[0])), "f"(unit(v[1])), "f"(unit(v[2])), "f"(unit(v[3])) : "memory");
+                    }
+                };
+                // blocks first to last - 1 to C
+                auto give = [&](uint32_t buf, int first, int last) {
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) {
+#pragma unroll 1
+                        for (int i = first; i < last; ++i, buf += 2048u) pl_store(&tm_c, buf, (int32_t)mt + 16 * i, (int32_t)nw0);
+                        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                    }
+                };
+                auto straight = [&](auto unit) {
+#pragma unroll
+                    for (int i = 0; i < 8; i += Cfg::BATCH) {
+                        if (i >= blocks) break;
+                        const uint32_t buf = take();
+#pragma unroll
+                        for (int b = 0; b < Cfg::BATCH; ++b)
+                            if (i + b < 8) put(buf + 2048u * b, i + b, unit);
+                        give(buf, i, blocks < i + Cfg::BATCH ? blocks : i + Cfg::BATCH);
+                    }
+                };
+                if (p.act == CN_ACT_LINEAR) {
+                    straight([](float x) { return x; });
+                } else if (p.act == CN_ACT_RELU) {
+                    straight([](float x) { return fmaxf(x, 0.0f); });   // 0 for a NaN, as x > 0 ? x : 0
+                } else if (p.act == CN_ACT_LOGISTIC && p.stages <= PL_DIRECT_STAGES && mt + half <= p.M && (p.ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(p.C) & 31u) == 0) {
+                    // short tiles are bound by the function itself: straight code, and no trip through shared memory (704 x 592 . 592 x 9176, single pass, 55 us, 63
+                    // by the way below)
+                    float *q = p.C + (nw0 + lane) * p.ldc + mt;
 #pragma unroll
                     for (int i = 0; i < 128; i += 8) {
                         if (i >= half) break;
@@ -856,38 +932,42 @@ cn_gemm_planes_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
 #pragma unroll
                         for (int e = 0; e < 8; e += 2) tc_unpack2(sum[(i + e) / 2], v[e], v[e + 1]);
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) v[e] = cn_apply_activation(p.bias ? v[e] + bias : v[e], CN_ACT_LOGISTIC);
+                        for (int e = 0; e < 8; ++e) v[e] = cn_apply_activation(v[e], CN_ACT_LOGISTIC);
                         if (nw0 + lane < p.N) stg8(q + i, v);
                     }
-                    __syncwarp();   // the next tile's tensor-memory loads need the whole warp
-                    continue;
-                }
+                } else {
+                    // one copy of the units' longer code (1736 x 2000 . 2000 x 4800 with logistic units: 160 us with straight code, 137)
+#pragma unroll 1
+                    for (int b = 0; b < blocks; ++b) {
+                        const uint32_t buf = take();
 #pragma unroll
-                for (int i = 0; i < 128; i += 8) {
-                    if (i >= half) break;
-                    float v[8];
+                        for (int i = 0; i < 8; ++i)
+                            if (b == i) put(buf, i, [](float x) { return x; });
+                        float v[16];
+                        const uint32_t at = buf + (uint32_t)lane * 64u;
 #pragma unroll
-                    for (int e = 0; e < 8; e += 2) tc_unpack2(sum[(i + e) / 2], v[e], v[e + 1]);
-                    if (p.bias) {
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) v[e] += bias;
-                    }
-                    if (p.act != CN_ACT_LINEAR) {
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) {
-                            v[e] = v[e] > 0.0f ? v[e] : 0.0f;
-                            if (p.act == CN_ACT_DOUBLE_RELU) v[e] = v[e] < 1.0f ? v[e] : 1.0f;
+                        for (int e = 0; e < 16; e += 4) {
+                            const float4 q = lds4(at + 4u * e);
+                            v[e] = q.x; v[e + 1] = q.y; v[e + 2] = q.z; v[e + 3] = q.w;
                         }
+                        if (p.act == CN_ACT_LOGISTIC) {
+#pragma unroll
+                            for (int e = 0; e < 16; ++e) v[e] = cn_apply_activation(v[e], CN_ACT_LOGISTIC);
+                        } else {
+#pragma unroll
+                            for (int e = 0; e < 16; ++e) v[e] = cn_apply_activation(v[e], CN_ACT_DOUBLE_RELU);
+                        }
+#pragma unroll
+                        for (int e = 0; e < 16; e += 4)
+                            asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at + 4u * e), "f"(v[e]), "f"(v[e + 1]), "f"(v[e + 2]), "f"(v[e + 3]) : "memory");
+                        give(buf, b, b + 1);
                     }
-                    if (nw0 + lane < p.N) stg8(q + i, v);
                 }
                 __syncwarp();   // the next tile's tensor-memory loads need the whole warp
                 continue;
             }
-            // Blocks of 32 columns x 32 rows are turned in shared memory (16-byte chunks permuted
-            // by the column against bank conflicts), so that a warp stores whole lines.
-            const uint32_t turn = smem_base + Cfg::TURN_OFF + (uint32_t)(warp - 4) * 4096u;
-            const bool vec = (p.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15u) == 0;
+            // Columns of C that do not start on 16 bytes: blocks of 32 columns x 32 rows are turned in shared memory (16-byte chunks permuted
+            // by the column against bank conflicts), so that a warp stores a column's rows together.
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
                 if (b * 32 >= half || mt + b * 32 >= p.M) break;
@@ -896,10 +976,6 @@ cn_gemm_planes_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
                     float v[4];
                     tc_unpack2(sum[b * 16 + 2 * c], v[0], v[1]);
                     tc_unpack2(sum[b * 16 + 2 * c + 1], v[2], v[3]);
-                    if (p.bias) {
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) v[e] += bias;
-                    }
                     asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(turn + lane * 128 + ((uint32_t)(c ^ (lane & 7)) << 4)), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
                 }
                 if (p.act != CN_ACT_LINEAR) {
@@ -912,36 +988,17 @@ cn_gemm_planes_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
                     }
                 }
                 __syncwarp();
-                const int c = lane & 7, col0 = lane >> 3;
                 const int rows = half - b * 32 < 32 ? half - b * 32 : 32;   // 16 or 32 of the block belong to this warpgroup
-                if (vec) {
-                    const int64_t m = mt + b * 32 + 4 * c;
-                    float *q = p.C + (nw0 + col0) * p.ldc + m;
-                    const int64_t step = 4 * p.ldc;
-                    const int cols = (int)(p.N - nw0 < 32 ? p.N - nw0 : 32) - col0, left = 4 * c < rows ? (int)(p.M - m < 4 ? p.M - m : 4) : 0;
-#pragma unroll
-                    for (int i = 0; i < 8; ++i, q += step) {
-                        const float4 v = lds4(turn + (i * 4 + col0) * 128 + ((uint32_t)(c ^ ((i * 4 + col0) & 7)) << 4));
-                        if (i * 4 >= cols) continue;
-                        if (left == 4) {
-                            *reinterpret_cast<float4 *>(q) = v;
-                        } else {
-                            if (left > 0) q[0] = v.x;
-                            if (left > 1) q[1] = v.y;
-                            if (left > 2) q[2] = v.z;
-                        }
-                    }
-                } else {
-                    const int64_t m = mt + b * 32 + lane;
-                    float *q = p.C + nw0 * p.ldc + m;
-                    const int cols = lane < rows && m < p.M ? (int)(p.N - nw0 < 32 ? p.N - nw0 : 32) : 0;
+                const int64_t m = mt + b * 32 + lane;
+                float *q = p.C + nw0 * p.ldc + m;
+                const int cols = lane < rows && m < p.M ? (int)(p.N - nw0 < 32 ? p.N - nw0 : 32) : 0;
 #pragma unroll 4
-                    for (int col = 0; col < cols; ++col, q += p.ldc) *q = lds1(turn + col * 128 + ((uint32_t)((lane >> 2) ^ (col & 7)) << 4) + (lane & 3) * 4);
-                }
+                for (int col = 0; col < cols; ++col, q += p.ldc) *q = lds1(turn + col * 128 + ((uint32_t)((lane >> 2) ^ (col & 7)) << 4) + (lane & 3) * 4);
                 __syncwarp();
             }
             __syncwarp();   // the next tile's tensor-memory loads need the whole warp
         }
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
     __syncwarp();
     tc_fence_before();
@@ -1114,16 +1171,30 @@ static int planes_chain(int64_t K, int mode, bool w_aligned, bool fine)
 }
 
 
-template <bool MODE3X>
-static int planes_launch_cfg(cn_context *ctx, const CUtensorMap &mw, const CUtensorMap &ma, const PlParams &prm, int64_t pairs, cudaStream_t s)
+// C (M x N, column-major) in blocks of 16 rows by 32 columns, 64 bytes of a column per line of shared memory.
+static int pl_make_out_map(EncodeTiledFn enc, CUtensorMap *map, float *C, int64_t M, int64_t N, int64_t ldc)
 {
+    cuuint64_t dims[2] = {(cuuint64_t)M, (cuuint64_t)N};
+    cuuint64_t strides[1] = {(cuuint64_t)ldc * sizeof(float)};
+    cuuint32_t box[2] = {16, 32};
+    cuuint32_t estr[2] = {1, 1};
+    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, C, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+                     CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    CN_REQUIRE(r == CUDA_SUCCESS, CN_ERR_CUDA, "cuTensorMapEncodeTiled failed with %d (output %lld x %lld)", (int)r, (long long)M, (long long)N);
+    return CN_OK;
+}
+
+template <bool MODE3X, bool SHORT>
+static int planes_launch_cfg(cn_context *ctx, const CUtensorMap &mw, const CUtensorMap &ma, const CUtensorMap &mc, const PlParams &prm, int64_t pairs, cudaStream_t s)
+{
+    constexpr int smem = PlCfg<MODE3X, SHORT>::SMEM_BYTES;
     static bool attr_set[64] = {};   // per device: the attribute belongs to the device's copy of the function
     const int dev = ctx->device;
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-        CN_CUDA(cudaFuncSetAttribute(cn_gemm_planes_kernel<MODE3X>, cudaFuncAttributeMaxDynamicSharedMemorySize, PlCfg<MODE3X>::SMEM_BYTES));
+        CN_CUDA(cudaFuncSetAttribute(cn_gemm_planes_kernel<MODE3X, SHORT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
-    CN_CUDA(cn_launch_pdl(cn_gemm_planes_kernel<MODE3X>, dim3((unsigned)(2 * pairs)), PL_THREADS, PlCfg<MODE3X>::SMEM_BYTES, s, mw, ma, prm));
+    CN_CUDA(cn_launch_pdl(cn_gemm_planes_kernel<MODE3X, SHORT>, dim3((unsigned)(2 * pairs)), PL_THREADS, smem, s, mw, ma, mc, prm));
     cn_count_launch();
     return CN_OK;
 }
@@ -1195,10 +1266,14 @@ int cn_gemm_planes_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, cons
     prm.partials = (float *)parts;
     prm.status = d_status;
 
-    CUtensorMap mw, ma;
+    CUtensorMap mw, ma, mc = {};
     if ((st = cn_make_planes_map(enc, &mw, reinterpret_cast<const uint16_t *>(bw), pw.Kp, N, pw.plane, pw.parts, 128)) != CN_OK) return st;
     if ((st = cn_make_planes_map(enc, &ma, reinterpret_cast<const uint16_t *>(ba), pa.Kp, M, pa.plane, pa.parts, half)) != CN_OK) return st;
-    st = mode == CN_GEMM_3XTF32 ? planes_launch_cfg<true>(ctx, mw, ma, prm, pairs, s) : planes_launch_cfg<false>(ctx, mw, ma, prm, pairs, s);
+    prm.tma_out = (ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 15u) == 0;
+    if (prm.tma_out && (st = pl_make_out_map(enc, &mc, C, M, N, ldc)) != CN_OK) return st;
+    const bool shorter = K <= (mode == CN_GEMM_3XTF32 ? 1 : 3) * PL_SHORT_K && prm.tma_out && prm.act != CN_ACT_LOGISTIC;
+    if (mode == CN_GEMM_3XTF32) st = shorter ? planes_launch_cfg<true, true>(ctx, mw, ma, mc, prm, pairs, s) : planes_launch_cfg<true, false>(ctx, mw, ma, mc, prm, pairs, s);
+    else                        st = shorter ? planes_launch_cfg<false, true>(ctx, mw, ma, mc, prm, pairs, s) : planes_launch_cfg<false, false>(ctx, mw, ma, mc, prm, pairs, s);
     if (st != CN_OK) return st;
     if (rest > 0) {
         ReduceParams rp = {};

@@ -363,7 +363,8 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
     if (p.cond) {
         cn_pdl_wait();
         if (blockIdx.x == 0 && threadIdx.x == 0) p.cond[CN_STATUS_OVERFLOW - CN_STATUS_MANY] = 0u;   // for the next product
-        if (__ldcg(p.cond) == 0u) return;
+        // one thread looks at the word: the reads of every warp of all CTAs meet in one line
+        if (!__syncthreads_or(threadIdx.x == 0 && __ldcg(p.cond) != 0u)) return;
     }
 
     // Fused all-gather: everything queued earlier on this GPU's stream has finished, so this rank's copy of C may now be
@@ -977,7 +978,7 @@ cn_splitk_reduce_kernel(const __grid_constant__ ReduceParams p)
         }
         __syncthreads();
     }
-    if (p.cond && __ldcg(p.cond) == 0u) return;
+    if (p.cond && !__syncthreads_or(threadIdx.x == 0 && __ldcg(p.cond) != 0u)) return;
     const int chunk = blockIdx.x % (TC_BN / COLS);
     const int tw = blockIdx.x / (TC_BN / COLS), rm = tw / p.nt, w = tw - rm * p.nt, r = rm / p.mt, mh = rm - r * p.mt, tile = p.full_tiles + r;
     const int64_t m0 = ((int64_t)(tile % p.tiles_m) * p.mt + mh) * p.rows, n0 = ((int64_t)(tile / p.tiles_m) * p.nt + w) * TC_BN + chunk * COLS;

@@ -106,6 +106,9 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map
         ::"r"(dst), "l"((uint64_t)map), "r"(bar), "r"(x), "r"(y), "r"(z) : "memory");
 }
 
+// A tensor map in a kernel's parameters, fetched before the first load that names it.
+__device__ __forceinline__ void tma_prefetch_map(const CUtensorMap *map) { asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)map) : "memory"); }
+
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
