@@ -274,7 +274,8 @@ int cn_gemm_dispatch(cn_context *ctx, int transA, int transB, int64_t M, int64_t
             done = true;
             st = small_product(nullptr);
         }
-        if (!done && st == CN_OK) st = cn_gemm_tc_launch(ctx, M, N, K, d_A, lda, d_B, ldb, target, target_ld, &e2, tc_mode, s, push ? peers : nullptr, transA, transB);
+        if (!done && st == CN_OK) st = cn_gemm_tc_launch(ctx, M, N, K, d_A, lda, d_B, ldb, target, target_ld, &e2, tc_mode, s, push ? peers : nullptr, transA, transB,
+                                                                nullptr, planes_ok && plain && !planes && !pr && !push);
         if (push && used_peers) *used_peers = true;
     } else {
         st = simt_launch(ctx, transA, transB, M, N, K, d_A, lda, d_B, ldb, target, target_ld, bias, act, s);

@@ -101,7 +101,7 @@ int cn_gemm_tc_split_activations(cn_context *ctx, int transA, int64_t M, int64_t
                                  cudaStream_t s);
 int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda,
                       const float *B, int64_t ldb, float *C, int64_t ldc, const cn_epilogue *epi, int mode, cudaStream_t s,
-                      const cn_peer_out *peers = nullptr, int transA = 0, int transB = 0, const cn_tc_cond *cond = nullptr);
+                      const cn_peer_out *peers = nullptr, int transA = 0, int transB = 0, const cn_tc_cond *cond = nullptr, bool clusters = false);
 // Products of planes by planes (cn_gemm_planes.cu), any layout and alignment of both operands: whether it is the faster kernel for a
 // shape, and the launch.  `fine`: the shape is one for the small products' kernel,
 // whose error must not be exceeded, and which is the one to record in a graph.  *done = false: no room for the planes of the weights, or that;

@@ -262,11 +262,6 @@ struct SmFeed {
     }
 };
 
-// Arrival for its order alone: what the CTAs send each other is counted by mbarriers.
-__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-
 __device__ __forceinline__ void sm_ld8(uint32_t taddr, uint32_t *r)
 {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -441,11 +436,7 @@ cn_gemm_small_kernel(const __grid_constant__ SmallParams p)
                             sts4f(at, v + e);
                             continue;
                         }
-                        uint32_t to, bar;
-                        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(at), "r"(dst));
-                        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(part_bar), "r"(dst));
-                        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
-                                     ::"r"(to), "f"(v[e]), "f"(v[e + 1]), "f"(v[e + 2]), "f"(v[e + 3]), "r"(bar) : "memory");
+                        st_async2(in_cta(at, dst), in_cta(part_bar, dst), tc_pair(v[e], v[e + 1]), tc_pair(v[e + 2], v[e + 3]));
                     }
                 } else if (m < p.M) {
                     float *q = p.C + (n0 + col) * p.ldc + m;

@@ -56,6 +56,7 @@
 #include "cn_tc_split.cuh"
 
 #define TC_W_TILE_BYTES (TC_BN * TC_WK * 4)
+#define CN_TC_MAX_CLUSTER 8
 
 // How the weights lie in memory: k contiguous or n contiguous ("transposed"), the rows of that layout 16-byte aligned or not.
 //
@@ -113,7 +114,7 @@ struct TcCfg {
     static_assert(TC_BANDS == 3, "four bytes");
     static constexpr int INFO_OFF = BAND_OFF + A_STAGES * 4;               // [NT][ACC_BUFS] pairs of words
     static constexpr int BAR_OFF = (INFO_OFF + NT * ACC_BUFS * 8 + 7) & ~7;
-    static constexpr int BARS = 2 * (W_STAGES + A_STAGES + NT * TMEM_STAGES + NT * ACC_BUFS + NT * 4);
+    static constexpr int BARS = 2 * (W_STAGES + A_STAGES + NT * TMEM_STAGES + NT * ACC_BUFS + NT * 4) + 1;
     static constexpr int HOLD_OFF = BAR_OFF + BARS * 8;                    // tensor-memory base, abort flag
     static constexpr int SMEM_BYTES = HOLD_OFF + 16 + 1024 /*align*/;
     static_assert(SMEM_BYTES <= 232448, "shared memory");
@@ -138,6 +139,7 @@ struct TcParams {
     int full_tiles;         // tiles [0, full_tiles): all of K by one CTA; the others are cut into runs over tail_ctas CTAs
     int tail_ctas;
     int kb_total;           // K blocks of 32
+    int cluster;            // CTAs that share a tile's K and add its parts themselves; 1: runs leave partial tiles
     int chain_mask;         // K blocks per accumulation chain - 1 (a power of two, at most TC_GROUP_KB)
     const float *a_inv;     // [band][group of 512 k][m_pad] inverse scales of the activation rows
     int64_t m_pad;
@@ -161,6 +163,20 @@ struct TcParams {
 struct TcSeg {
     int tile, k0, k1;
     int slot;       // where the partial tile goes; -1: the run is the whole tile and is finished in place
+};
+
+// A cluster's CTAs share the rows m of their tile in units of 16: CTA number `rank` finishes `mine` of them, from unit rank * per on.
+struct TcShare {
+    int rank, units, per, mine;
+    __device__ __forceinline__ explicit TcShare(const TcParams &p)
+    {
+        const int tile = (int)blockIdx.x / p.cluster;
+        const int64_t rows = p.M - (int64_t)(tile % p.tiles_m) * TC_BM;
+        rank = (int)blockIdx.x - tile * p.cluster;
+        units = rows < TC_BM ? (int)(rows + 15) >> 4 : TC_BM / 16;
+        per = (units + p.cluster - 1) / p.cluster;
+        mine = units - rank * per < per ? units - rank * per : per;
+    }
 };
 
 // The runs of CTA `cta`, in order.  All roles of a CTA walk the same list.
@@ -333,7 +349,8 @@ struct WMaps {
 // cut into chains of at most 512 k, which end where the activations' scale groups end: each chain starts a fresh TMEM
 // accumulator, and when it ends the drain warps read it with tcgen05.ld, remove both scales and add it, in round-to-nearest
 // fp32, to running sums that they keep in registers (one thread = one output column n, 128 sums = 128 rows m).
-template <int NT, bool MODE3X, int WK>
+// SHARED: the CTAs of a cluster share a tile's K and add its parts themselves (an instance of its own: as a branch it cost the others 0.6 us).
+template <int NT, bool MODE3X, int WK, bool SHARED>
 __global__ void __launch_bounds__(TcCfg<NT, MODE3X, WK>::THREADS, 1)
 cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ TcParams p)
 {
@@ -344,7 +361,8 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
                   B_AEMPTY = B_AFULL + Cfg::A_STAGES, B_TFULL = B_AEMPTY + Cfg::A_STAGES, B_TEMPTY = B_TFULL + NT * Cfg::TMEM_STAGES,
                   B_ACCFULL = B_TEMPTY + NT * Cfg::TMEM_STAGES, B_ACCEMPTY = B_ACCFULL + NT * Cfg::ACC_BUFS;
     constexpr int B_XFULL = B_ACCEMPTY + NT * Cfg::ACC_BUFS, B_XEMPTY = B_XFULL + NT * 4;   // left-overs of the weights, per converter warp
-    static_assert(B_XEMPTY + NT * 4 == Cfg::BARS, "barrier count");
+    constexpr int B_PART = B_XEMPTY + NT * 4;   // this CTA's rows of the partial tiles of its cluster have arrived
+    static_assert(B_PART + 1 == Cfg::BARS, "barrier count");
     auto bar = [&](int idx) { return smem_base + Cfg::BAR_OFF + 8u * idx; };
     auto wfull_bar = [&](int s) { return bar(B_WFULL + s); };
     auto wempty_bar = [&](int s) { return bar(B_WEMPTY + s); };
@@ -383,6 +401,11 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
             for (int t = 0; t < Cfg::TMEM_STAGES; ++t) { mbar_init(tfull_bar(w, t), 4); mbar_init(tempty_bar(w, t), 1); }
             for (int b = 0; b < Cfg::ACC_BUFS; ++b) { mbar_init(accfull_bar(w, b), 2); mbar_init(accempty_bar(w, b), 4); }
             for (int q = 0; q < 4; ++q) { mbar_init(xfull_bar(w, q), 1); mbar_init(xempty_bar(w, q), 1); }
+        }
+        if (SHARED) mbar_init(bar(B_PART), 1);
+        if (SHARED) {
+            const TcShare s(p);
+            if (s.mine > 0) mbar_expect_tx(bar(B_PART), (uint32_t)((p.cluster - 1) * s.mine * (16 * 4) * (NT * TC_BN)));
         }
         sts1u(abort_flag, 0u);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -444,6 +467,7 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
             if (lane == 0) {
                 TcWalk walk(p);
                 TcSeg seg;
+                tma_prefetch_map(&tm_a);
                 cn_pdl_wait();
                 uint32_t it = 0;
                 bool ok = true;
@@ -845,6 +869,61 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
             }
             if (!ok) break;
             const int64_t m0 = (int64_t)(seg.tile % p.tiles_m) * TC_BM, n = (int64_t)(seg.tile / p.tiles_m) * (NT * TC_BN) + w * TC_BN + row;
+            if (SHARED) {
+                // The rings are idle in every CTA of the cluster: each unit of 16 rows goes to the CTA that finishes it, [sender][quad of m][column n]
+                // float4, which adds the parts in K order.  A lane's own share stays where it is, and it reads what it wrote itself.
+                cluster_arrive();
+                cluster_wait();
+                chains = ~0u;   // done
+                const TcShare share(p);
+                const int per = share.per, rank = share.rank, mine = share.mine;
+                constexpr uint32_t QUAD = NT * TC_BN * 16;
+                const uint32_t column = (uint32_t)(w * TC_BN + row) * 16u;
+                int to = 0, at_unit = 0;
+#pragma unroll
+                for (int u = 0; u < TC_BM / 16; ++u) {
+                    if (u >= share.units) break;
+                    const uint32_t at = smem_base + (uint32_t)((rank * per + at_unit) * 4) * QUAD + column;
+                    if (to == rank) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) sts2l(at + j * QUAD, sum[8 * u + 2 * j], sum[8 * u + 2 * j + 1]);
+                    } else {
+                        const uint32_t there = in_cta(at, to), counted = in_cta(bar(B_PART), to);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) st_async2(there + j * QUAD, counted, sum[8 * u + 2 * j], sum[8 * u + 2 * j + 1]);
+                    }
+                    if (++at_unit == per) { at_unit = 0; ++to; }
+                }
+                if (mine <= 0) break;
+                ok = mbar_wait(bar(B_PART), 0u, abort_flag, p.status, 24u) && mbar_try_cluster(bar(B_PART), 0u) != 0u;
+                if (!ok) break;
+                if (n >= p.N) break;
+                const float bias = p.bias ? p.bias[n] : 0.0f;
+                const bool vec = (p.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(p.C) & 15u) == 0;
+                int64_t m = m0 + 16 * (rank * per);
+                float *q = p.C + n * p.ldc + m;
+#pragma unroll 1
+                for (int i = 0; i < 4 * mine && m < p.M; ++i, m += 4, q += 4) {
+                    float4 part[CN_TC_MAX_CLUSTER];
+#pragma unroll
+                    for (int s = 0; s < CN_TC_MAX_CLUSTER; ++s)
+                        if (s < p.cluster) part[s] = lds4(smem_base + (uint32_t)(s * per * 4 + i) * QUAD + column);
+                    float v[4] = {part[0].x, part[0].y, part[0].z, part[0].w};
+#pragma unroll
+                    for (int s = 1; s < CN_TC_MAX_CLUSTER; ++s)
+                        if (s < p.cluster) { v[0] += part[s].x; v[1] += part[s].y; v[2] += part[s].z; v[3] += part[s].w; }
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) v[e] = cn_apply_activation(p.bias ? v[e] + bias : v[e], p.act);
+                    if (vec && m + 4 <= p.M) {
+                        *reinterpret_cast<float4 *>(q) = make_float4(v[0], v[1], v[2], v[3]);
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            if (m + e < p.M) q[e] = v[e];
+                    }
+                }
+                break;
+            }
             if (seg.slot >= 0) {
                 // partial tile: float4 number i of 32 for all 128 columns, then the next, so that a warp writes 512 contiguous bytes
                 ulonglong2 *P = reinterpret_cast<ulonglong2 *>(p.partials) + ((int64_t)seg.slot * NT + w) * (TC_BM * TC_BN / 4) + row;
@@ -939,10 +1018,27 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
             }
             __syncwarp();   // as above
         }
+        __syncwarp();
+        if (SHARED && chains != ~0u) { cluster_arrive(); cluster_wait(); }   // gave up before
+    }
+    if (SHARED && warp < 4 + 4 * NT) {   // this CTA's loads and products are over, once all warps say so
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
     }
 
     tc_fence_before();
     __syncthreads();
+    if (SHARED) {
+        // no CTA leaves before the others have sent; after a wait that ran out, what is under way gets a bounded chance to land
+        if (lds1u(abort_flag) != 0u) {
+            const long long t0 = clock64();
+            while (clock64() - t0 < 20000000LL) {}
+        }
+        __syncwarp();
+        cluster_arrive_relaxed();
+        cluster_wait();
+    }
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
@@ -1143,21 +1239,108 @@ bool cn_gemm_tc_supported(cn_context *, int transA, int transB, int64_t M, int64
 // longest chain that is no less exact than the fp32 kernel was:
 int cn_gemm_any_chain(int64_t K) { return K < 384 ? 1 : K < 1024 ? 2 : K < 3072 ? 4 : K < 12288 ? 8 : TC_GROUP_KB; }
 
-template <int NT, bool MODE3X, int WK>
+template <class Kernel>
+static cudaError_t tc_launch_clusters(Kernel kernel, unsigned grid, int cluster, int block, size_t smem, cudaStream_t s, const WMaps &mw, const CUtensorMap &ma,
+                                      const TcParams &prm)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)cluster;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, kernel, mw, ma, prm);
+}
+
+// Clusters of c CTAs of an SM each that the device holds at once: their SMs have to lie in one GPC.
+static int tc_max_clusters(const cn_context *ctx, int c)
+{
+    using Cfg = TcCfg<2, true, W_K>;
+    static int known[64][CN_TC_MAX_CLUSTER + 1] = {};
+    const int dev = ctx->device;
+    if (dev >= 0 && dev < 64 && known[dev][c] > 0) return known[dev][c];
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(ctx->sm_count / c * c));
+    cfg.blockDim = dim3(Cfg::THREADS);
+    cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)c;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaFuncSetAttribute(cn_gemm_tc_kernel<2, true, W_K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, cn_gemm_tc_kernel<2, true, W_K, true>, &cfg) != cudaSuccess || n < 1) {
+        cudaGetLastError();
+        n = 1;
+    }
+    if (dev >= 0 && dev < 64) known[dev][c] = n;
+    return n;
+}
+
+template <int NT, bool MODE3X, int WK, bool SHARED>
 static int launch_cfg(const WMaps &mw, const CUtensorMap &ma, const TcParams &prm, int64_t grid, int dev, cudaStream_t s)
 {
     using Cfg = TcCfg<NT, MODE3X, WK>;
     static bool attr_set[64] = {};   // per device: the attribute belongs to the device's copy of the function
     if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-        CN_CUDA(cudaFuncSetAttribute(cn_gemm_tc_kernel<NT, MODE3X, WK>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
+        CN_CUDA(cudaFuncSetAttribute(cn_gemm_tc_kernel<NT, MODE3X, WK, SHARED>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_BYTES));
         if (dev >= 0 && dev < 64) attr_set[dev] = true;
     }
-    CN_CUDA(cn_launch_pdl(cn_gemm_tc_kernel<NT, MODE3X, WK>, dim3((unsigned)grid), Cfg::THREADS, Cfg::SMEM_BYTES, s, mw, ma, prm));
+    if (SHARED) CN_CUDA(tc_launch_clusters(cn_gemm_tc_kernel<NT, MODE3X, WK, SHARED>, (unsigned)grid, prm.cluster, Cfg::THREADS, Cfg::SMEM_BYTES, s, mw, ma, prm));
+    else CN_CUDA(cn_launch_pdl(cn_gemm_tc_kernel<NT, MODE3X, WK, SHARED>, dim3((unsigned)grid), Cfg::THREADS, Cfg::SMEM_BYTES, s, mw, ma, prm));
     cn_count_launch();
     return CN_OK;
 }
 
-size_t cn_tc_cut::partial_bytes() const { return rest() > 0 ? (size_t)(tail_ctas + rest()) * nt * TC_BM * TC_BN * sizeof(float) : 0; }
+size_t cn_tc_cut::partial_bytes() const { return rest() > 0 && cluster == 1 ? (size_t)(tail_ctas + rest()) * nt * TC_BM * TC_BN * sizeof(float) : 0; }
+
+// Clusters in place of runs that leave partial tiles, for products of one tile of rows.  A run's partial tiles go to memory and a reduction reads
+// them, a launch later: 17 us, 8 more where all SMs leave some, and 0.9 per K block of a CTA for the whole product, by a fit to what
+// follows.  A cluster's CTAs exchange the parts through distributed shared memory (20 bytes per clock from a CTA), in one launch less: 15 us
+// and 0.66 per block with one tile of 128 columns per CTA, 20 and 0.74 with two; but K is cut into as many parts as CTAs find room in the GPCs
+// for every tile, not one per SM.  us, runs / clusters: 24 x 560 . 560 x 5192 23.8 / 14.5; 100 x 1500 . 1500 x 2500 30.6 / 19.6; 48 x 1568 . 1568 x 11448 39.4
+// / 28.7; 128 x 3000 . 3000 x 3000 31.1 / 28.1; 128 x 4096 . 4096 x 4096 36.5 / 38.0; 128 x 10000 . 10000 x 1000 39.7 / 40.1, x 100000 131 / 299.  With
+// two tiles of rows a few gain (256 x 4096 . 4096 x 4096 55.5 / 49.7), others lose (150 x 2344 . 2344 x 2208 33 / 38).
+//
+// Runs are short, and so are their accumulation chains; clusters' chains are cut as short, so that no product is less exact: relative to fp64,
+// runs of 28 blocks 1.6e-6, of 14 1.3e-6, of 6 7e-7; chains of 8 blocks 9.8e-7, of 4 5.4e-7.  That costs long runs more than the launch
+// (152 x 9384 . 9384 x 3152 85 / 103): at most 24 blocks.
+static void tc_share_tiles(const cn_context *ctx, int64_t N, cn_tc_cut *cut)
+{
+    if (cut->rest() == 0 || cut->tiles_m > 1) return;
+    const double run = (double)cut->rest() * cut->kb_total / cut->tail_ctas;
+    const double runs = 17.0 + 8.0 * (double)cut->tail_ctas / ctx->sm_count + 0.9 * (cut->full > 0 ? (double)cut->tiles * cut->kb_total / ctx->sm_count : run);
+    double best = 0.95 * runs;
+    for (int nt = 1; nt <= (N > TC_BN ? 2 : 1); ++nt) {
+        const int64_t tiles = (N + nt * TC_BN - 1) / (nt * TC_BN) * cut->tiles_m;
+        for (int c = 2; c <= CN_TC_MAX_CLUSTER && cut->kb_total >= 2 * c; ++c) {
+            const int per = (TC_BM / 16 + c - 1) / c;
+            // room for the parts in the rings' shared memory
+            if (c * per * 16 * nt * TC_BN * (int)sizeof(float) > (nt == 1 ? TcCfg<1, true, W_K>::RING_BYTES : TcCfg<2, true, W_K>::RING_BYTES)) continue;
+            const double t = (nt == 1 ? 15.0 : 20.0) + (nt == 1 ? 0.66 : 0.74) * (double)((cut->kb_total + c - 1) / c);
+            if (t >= best || (cut->kb_total + c - 1) / c > 24 || tiles > tc_max_clusters(ctx, c)) continue;
+            best = t;
+            cut->nt = nt;
+            cut->cluster = c;
+        }
+    }
+    if (cut->cluster == 1) return;
+    cut->tiles = (N + cut->nt * TC_BN - 1) / (cut->nt * TC_BN) * cut->tiles_m;
+    cut->full = 0;
+    cut->tail_ctas = cut->tiles * cut->cluster;
+    cut->max_chain = run >= 12.0 ? 8 : run >= 6.0 ? 4 : 2;
+}
 
 cn_tc_cut cn_tc_decompose(const cn_context *ctx, int64_t M, int64_t N, int64_t K, int kind, bool push)
 {
@@ -1171,6 +1354,8 @@ cn_tc_cut cn_tc_decompose(const cn_context *ctx, int64_t M, int64_t N, int64_t K
     c.kb_total = (int)((K + TC_WK - 1) / TC_WK);
     const int64_t sms = ctx->sm_count;
     c.full = c.tail_ctas = 0;
+    c.cluster = 1;
+    c.max_chain = TC_GROUP_KB;
     if (kind == CN_TC_WHOLE) {
         c.full = c.tiles;   // the reduction kernel has no maxout; such layers are small
     } else if (ws && ws->force_splits >= 1) {
@@ -1192,12 +1377,13 @@ cn_tc_cut cn_tc_decompose(const cn_context *ctx, int64_t M, int64_t N, int64_t K
             if (c.tail_ctas < c.rest()) c.tail_ctas = c.rest() < sms ? c.rest() : sms;
         }
     }
+    if (kind == CN_TC_CLUSTERS && !push) tc_share_tiles(ctx, N, &c);
     return c;
 }
 
 int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, const float *B,
                       int64_t ldb, float *C, int64_t ldc, const cn_epilogue *epi, int mode, cudaStream_t s, const cn_peer_out *peers,
-                      int transA, int transB, const cn_tc_cond *cond)
+                      int transA, int transB, const cn_tc_cond *cond, bool clusters)
 {
     EncodeTiledFn enc = nullptr;
     int st = cn_get_encode_fn(ctx, &enc);
@@ -1236,7 +1422,7 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
 
     // 2. work decomposition
     const int maxout = epi ? epi->maxout_level : 1;
-    const cn_tc_cut cut = cn_tc_decompose(ctx, M, N, K, maxout > 1 ? CN_TC_WHOLE : cond ? CN_TC_BEHIND : CN_TC_ALONE, peers && peers->npeers > 0);
+    const cn_tc_cut cut = cn_tc_decompose(ctx, M, N, K, maxout > 1 ? CN_TC_WHOLE : cond ? CN_TC_BEHIND : clusters ? CN_TC_CLUSTERS : CN_TC_ALONE, peers && peers->npeers > 0);
     const int nt = cut.nt, kb_total = cut.kb_total;
     const int64_t tiles_m = cut.tiles_m, tiles_n = cut.tiles / tiles_m, tiles = cut.tiles, full = cut.full, tail_ctas = cut.tail_ctas, rest = cut.rest();
     const int64_t sms = ctx->sm_count;
@@ -1252,7 +1438,10 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
     prm.argmax = epi ? epi->argmax_out : nullptr;
     prm.tiles_n = (int)tiles_n; prm.tiles_m = (int)tiles_m;
     prm.full_tiles = (int)full; prm.tail_ctas = (int)tail_ctas; prm.kb_total = kb_total;
+    prm.cluster = cut.cluster;
     int chain = w_aligned(B, ldb) ? TC_GROUP_KB : cn_gemm_any_chain(K);
+    while (chain > cut.max_chain) chain >>= 1;
+    if (cut.cluster > 1 && !w_aligned(B, ldb) && chain > 2) chain >>= 1;   // else 49 x 1597 . 1597 x 4326 is off by 4.0e-7, 3.5e-7 by runs
     if (ws->force_chain >= 1)
         while (chain > 1 && chain > ws->force_chain) chain >>= 1;
     prm.chain_mask = chain - 1;
@@ -1273,7 +1462,7 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
         prm.peer_flags = peers->peer_flags;
         prm.nranks = peers->nranks; prm.my_rank = peers->my_rank; prm.epoch = peers->epoch;
     }
-    if (rest > 0) {
+    if (cut.partial_bytes() > 0) {
         void *buf = nullptr;
         st = cn_gemm_scratch(ctx, CN_GEMM_SLOT_SPLITK, cut.partial_bytes(), &buf);
         if (st != CN_OK) return st;
@@ -1294,14 +1483,15 @@ int cn_gemm_tc_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const fl
     if (!cond && (st = cn_gemm_profile_start(ctx, s, &ev_stop)) != CN_OK) return st;
     if (ev_stop) prm.w_ready = 0;   // the event stands between the pre-pass and this launch: keep the plain order
 #define CN_LAUNCH(M3, WKV) \
-    (nt == 1 ? launch_cfg<1, M3, WKV>(mw, ma, prm, grid, ctx->device, s) : launch_cfg<2, M3, WKV>(mw, ma, prm, grid, ctx->device, s))
+    (cut.cluster > 1 ? (nt == 1 ? launch_cfg<1, M3, WKV, true>(mw, ma, prm, grid, ctx->device, s) : launch_cfg<2, M3, WKV, true>(mw, ma, prm, grid, ctx->device, s)) \
+                     : (nt == 1 ? launch_cfg<1, M3, WKV, false>(mw, ma, prm, grid, ctx->device, s) : launch_cfg<2, M3, WKV, false>(mw, ma, prm, grid, ctx->device, s)))
     if (wk == W_K_ANY)      st = CN_LAUNCH(true, W_K_ANY);
     else if (wk == W_N_ANY) st = CN_LAUNCH(true, W_N_ANY);
     else if (mode3x)        st = wk == W_N ? CN_LAUNCH(true, W_N) : CN_LAUNCH(true, W_K);
     else                    st = wk == W_N ? CN_LAUNCH(false, W_N) : CN_LAUNCH(false, W_K);
 #undef CN_LAUNCH
     if (st != CN_OK) return st;
-    if (rest > 0) {
+    if (rest > 0 && cut.cluster == 1) {
         ReduceParams rp;
         rp.partials = prm.partials; rp.nt = nt; rp.mt = 1; rp.rows = TC_BM; rp.tail_ctas = (int)tail_ctas; rp.kb_total = kb_total;
         rp.tail_tiles = (int)rest; rp.full_tiles = (int)full; rp.tiles_m = (int)tiles_m; rp.cond = prm.cond; rp.M = M; rp.N = N;

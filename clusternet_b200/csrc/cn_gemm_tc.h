@@ -36,14 +36,17 @@ struct ReduceParams {
 };
 int cn_splitk_reduce_launch(cn_context *ctx, const ReduceParams &rp, cudaStream_t s);
 
-// The streaming kernel's decomposition of a product: nt tiles of 128 columns n per CTA, whole tiles, then tiles cut into runs.
+// The streaming kernel's decomposition of a product: nt tiles of 128 columns n per CTA, whole tiles, then tiles cut into runs; or, cluster > 1,
+// every tile's K shared by the CTAs of a cluster.
 struct cn_tc_cut {
-    int nt, kb_total;
+    int nt, kb_total, cluster;
+    int max_chain;   // K blocks per accumulation chain, at most
     int64_t tiles_m, tiles, full, tail_ctas;
     int64_t rest() const { return tiles - full; }
     size_t partial_bytes() const;   // of CN_GEMM_SLOT_SPLITK
 };
-enum { CN_TC_ALONE, CN_TC_WHOLE, CN_TC_BEHIND };   // CN_TC_WHOLE: whole tiles only; CN_TC_BEHIND: the launch behind the planes kernel
+// CN_TC_WHOLE: whole tiles only; CN_TC_BEHIND: the launch behind the planes kernel; CN_TC_CLUSTERS: clusters, where they are faster
+enum { CN_TC_ALONE, CN_TC_WHOLE, CN_TC_BEHIND, CN_TC_CLUSTERS };
 cn_tc_cut cn_tc_decompose(const cn_context *ctx, int64_t M, int64_t N, int64_t K, int kind, bool push);
 
 // The streaming kernel behind the one that multiplies planes: it runs where the word at `many` (CN_STATUS_MANY) is not zero, on these

@@ -40,6 +40,23 @@ __device__ __forceinline__ uint32_t mbar_try_cluster(uint32_t bar, uint32_t pari
         : "=r"(done) : "r"(bar), "r"(parity) : "memory");
     return done;
 }
+// Arrival for its order alone: what the CTAs send each other is counted by mbarriers.
+__device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// The same place in the shared memory of CTA `rank` of the cluster, and 16 bytes to such a place, counted at a barrier there.
+__device__ __forceinline__ uint32_t in_cta(uint32_t a, uint32_t rank)
+{
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void st_async2(uint32_t to, uint32_t bar, uint64_t a, uint64_t b)
+{
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(to), "l"(a), "l"(b), "r"(bar) : "memory");
+}
+__device__ __forceinline__ uint64_t tc_pair(float a, float b) { return (uint64_t)__float_as_uint(b) << 32 | __float_as_uint(a); }
+__device__ __forceinline__ void sts2l(uint32_t a, uint64_t x, uint64_t y) { asm volatile("st.shared.v2.b64 [%0], {%1, %2};" ::"r"(a), "l"(x), "l"(y) : "memory"); }
 // Shared-memory accesses by 32-bit address (half the registers of generic pointers).
 __device__ __forceinline__ float4 lds4(uint32_t a)
 {

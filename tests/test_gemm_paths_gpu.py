@@ -394,3 +394,37 @@ def test_softmax_at_the_edge_of_the_register_rows(ctx, cols):
     out = ctx.empty(65, cols)
     assert ctx.lib.cn_softmax(ctx.h, place(A, 0).data_ptr(), out.data_ptr(), 65, cols, ctx.stream_ptr()) == 0
     assert np.abs(ctx.to_numpy(out) - oracle.softmax_rows(A)).max() < 2e-6       # __expf against libm's exp
+
+
+# tiles whose K a cluster of CTAs shares (one tile of rows, short K, weights beyond the small products'): one and two tiles of columns per CTA,
+# clusters of 2 to 8, rows that give some CTAs nothing to finish, last tiles of few columns; weights of either layout and of odd pitch
+SHARED = [(24, 560, 5192), (100, 1500, 2500), (128, 1024, 3000), (17, 640, 9001), (128, 2000, 8000), (1, 992, 6000), (72, 912, 3624), (120, 777, 4099), (97, 528, 7258)]
+
+
+@pytest.mark.parametrize("M,K,N", SHARED)
+@pytest.mark.parametrize("transA,transB", [(False, False), (True, True)])
+@pytest.mark.parametrize("act,mode", [(_lib.ACT_LINEAR, _lib.GEMM_3XTF32), (_lib.ACT_LOGISTIC, _lib.GEMM_3XTF32), (_lib.ACT_RELU, _lib.GEMM_TF32)])
+def test_tiles_shared_by_clusters(ctx, M, K, N, transA, transB, act, mode):
+    """Elements of very different size among them: what the parts leave is in chains of its own."""
+    g = torch.Generator(device="cuda").manual_seed(M + K + N)
+    A, W = torch.randn(M, K, device="cuda", generator=g), torch.randn(K, N, device="cuda", generator=g)
+    A[0, ::7] *= 2.0 ** -30
+    W[::5, N - 1] *= 2.0 ** -30
+    bias = torch.randn(N, device="cuda", generator=g)
+    buf = torch.full((N + 1, M), 7.0, device="cuda")
+    a, w = (A if transA else A.t()).contiguous(), (W if transB else W.t()).contiguous()
+    n0 = ctx.lib.cn_kernel_launches()
+    for rep in range(2):
+        ctx.gemm(a, w, out=buf[:N], transA=transA, transB=transB, bias=bias, activation=act, mode=mode)
+        if rep == 0:
+            first = buf.clone()
+    assert ctx.lib.cn_kernel_launches() - n0 == 4   # planes and product: no reduction
+    ctx.gemm_check()
+    assert ctx.gemm_last_kernel() == "streaming"
+    assert torch.equal(first, buf) and bool((buf[N] == 7.0).all())
+    z = A.double() @ W.double() + bias.double()
+    want = {_lib.ACT_LINEAR: z, _lib.ACT_LOGISTIC: torch.sigmoid(z), _lib.ACT_RELU: z.clamp(min=0)}[act]
+    aligned = (N if transB else K) % 4 == 0
+    rel = REL_1X if mode == _lib.GEMM_TF32 and aligned else REL_3X
+    bound = rel * (A.double().abs() @ W.double().abs()) + 2.0 ** -22 * (z.abs() + 1.0)
+    assert bool(((buf[:N].t().double() - want).abs() <= bound).all())
