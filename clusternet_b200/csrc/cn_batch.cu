@@ -26,6 +26,10 @@
 #include <string.h>
 #include "cn_internal.h"
 
+#define CN_BATCH_SLOTS 16                  // swaps whose ends are known
+#define CN_BATCH_SMALL_BYTES (4 << 20)
+#define CN_BATCH_SLOT_BYTES (16 << 10)
+
 struct cn_batch {
     cn_context *ctx = nullptr;
     const float *h_X = nullptr, *h_y = nullptr;   // caller's row-major data set (not owned)
@@ -39,12 +43,18 @@ struct cn_batch {
     bool direct = false;         // the data set itself is pinned: copy from it, no staging memcpy
     float *p_X = nullptr, *p_y = nullptr;     // pinned staging
     float *dn_y = nullptr;                    // device, next batch's labels, row-major
+    // Few labels: kept in pinned slots, from which the swap's kernel reads them over PCIe.  A slot is written again when the swap
+    // that read it, CN_BATCH_SLOTS before, has finished.
+    float *slot_y = nullptr;
+    int64_t swaps = 0;
     // options (cn_batch_create_ex)
     int flags = 0;
-    // Row-major X buffers form a ring: one (plain: transposed into dc_X at the swap), two (the current batch stays valid
+    // Row-major X buffers form a ring: one (plain: transposed into dc_X at the swap), two (small batches, or the current batch stays valid
     // while the next one is copied) or three (CN_BATCH_LOOKAHEAD: two copies in flight).  `fill` is where the next copy
     // goes, `ready` what the next swap takes, `in_flight` how many copies lie between them.
     int nb = 1, depth = 1;
+    bool turns = false;                       // buffers are read by the swap's kernel only: free once it has run
+    cudaEvent_t read[3] = {};                 // ... the swap that read buffer i last
     float *xb[3] = {nullptr, nullptr, nullptr};
     bool xb_sym = false;                      // xb[] came from cn_sym_alloc
     float *peer_xb[3][8] = {};                // peer addresses of xb[i]
@@ -62,7 +72,8 @@ struct cn_batch {
     cudaEvent_t e_prof[5] = {};
     float *dc_X = nullptr, *dc_y = nullptr;   // device, current batch, column-major
     cudaStream_t s_X = nullptr, s_y = nullptr;
-    cudaEvent_t e_y = nullptr, e_consumed = nullptr;
+    cudaEvent_t e_y = nullptr;
+    cudaEvent_t e_swap[CN_BATCH_SLOTS] = {}, e_consumed = nullptr;   // after the last swaps' kernels; after the last one's
 };
 
 // Sharded upload: this rank's block of the batch, already in its own buffer, goes to the same place in every peer's
@@ -101,6 +112,8 @@ extern "C" int cn_batch_destroy(cn_batch *b)
     if (!b) return CN_OK;
     if (b->s_X) cudaStreamSynchronize(b->s_X);
     if (b->s_y) cudaStreamSynchronize(b->s_y);
+    if (b->slot_y && b->e_consumed) cudaEventSynchronize(b->e_consumed);   // the last swap reads its slot
+    cudaFreeHost(b->slot_y);
     cudaFreeHost(b->p_X); cudaFreeHost(b->p_y);
     for (int i = 0; i < 3; ++i) {
         if (!b->xb[i]) continue;
@@ -111,7 +124,7 @@ extern "C" int cn_batch_destroy(cn_batch *b)
     if (b->s_y) cudaStreamDestroy(b->s_y);
     for (cudaEvent_t e : b->e_Xb) if (e) cudaEventDestroy(e);
     if (b->e_y) cudaEventDestroy(b->e_y);
-    if (b->e_consumed) cudaEventDestroy(b->e_consumed);
+    for (cudaEvent_t e : b->e_swap) if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : b->e_prof) if (e) cudaEventDestroy(e);
     delete b;
     return CN_OK;
@@ -147,9 +160,12 @@ extern "C" int cn_batch_create_ex(cn_context *ctx, const float *h_X, const float
     b->G = G;
     b->rank = cn_comm_rank(ctx);
     b->total_batches = (rows + batch_size - 1) / batch_size;
-    b->nb = (flags & CN_BATCH_LOOKAHEAD) ? 3 : (flags & CN_BATCH_KEEP_ROW_MAJOR) ? 2 : 1;
     b->depth = (flags & CN_BATCH_LOOKAHEAD) ? 2 : 1;
     const size_t bx = (size_t)batch_size * cols_X * sizeof(float), by = (size_t)batch_size * cols_y * sizeof(float);
+    // Small batches that are only turned have two row-major buffers as well, so that the next copy runs beside the swap's kernel; of large ones,
+    // whose copies take long beside that kernel, a second buffer would only take room.
+    b->turns = !(flags & CN_BATCH_KEEP_ROW_MAJOR);
+    b->nb = (flags & CN_BATCH_LOOKAHEAD) ? 3 : (flags & CN_BATCH_KEEP_ROW_MAJOR) || bx <= CN_BATCH_SMALL_BYTES ? 2 : 1;
     cudaError_t e;
     // The copy streams get the highest priority: their work is a few copies and, with the sharded upload, two one-warp flag
     // kernels, which must not queue behind the thousands of CTAs of a product that runs on the compute stream meanwhile.
@@ -163,9 +179,14 @@ extern "C" int cn_batch_create_ex(cn_context *ctx, const float *h_X, const float
         cudaGetLastError();
         b->direct = px && py;
     }
-    if ((!b->direct && (e = cudaHostAlloc(&b->p_X, bx, cudaHostAllocPortable)) != cudaSuccess) ||
-        (!b->direct && (e = cudaHostAlloc(&b->p_y, by, cudaHostAllocPortable)) != cudaSuccess) ||
-        (e = cudaMalloc(&b->dn_y, by)) != cudaSuccess ||
+    // A copy of a few labels is three calls (wait, copy, event) and the swap's wait for it, more than the kernel that turns the batch takes
+    // to read them over PCIe, now that the next copy does not wait for that kernel.  Larger ones stay with the copy engine.  128 x 784 images with
+    // a label each, us per batch: 19.1; with the second buffer, one kernel for both and the labels in slots 15.1 (with one buffer 23).
+    const bool few = by <= CN_BATCH_SLOT_BYTES;
+    if ((few && (e = cudaHostAlloc(&b->slot_y, by * CN_BATCH_SLOTS, cudaHostAllocPortable | cudaHostAllocMapped)) != cudaSuccess) ||
+        (!b->direct && (e = cudaHostAlloc(&b->p_X, bx, cudaHostAllocPortable)) != cudaSuccess) ||
+        (!few && !b->direct && (e = cudaHostAlloc(&b->p_y, by, cudaHostAllocPortable)) != cudaSuccess) ||
+        (!few && (e = cudaMalloc(&b->dn_y, by)) != cudaSuccess) ||
         (!(flags & CN_BATCH_NO_COL_MAJOR) && (e = cudaMalloc(&b->dc_X, bx)) != cudaSuccess) ||
         (e = cudaMalloc(&b->dc_y, by)) != cudaSuccess ||
         (e = cudaStreamCreateWithPriority(&b->s_X, cudaStreamNonBlocking, prio_high)) != cudaSuccess ||
@@ -174,10 +195,16 @@ extern "C" int cn_batch_create_ex(cn_context *ctx, const float *h_X, const float
         (e = cudaEventCreateWithFlags(&b->e_Xb[1], cudaEventDisableTiming)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&b->e_Xb[2], cudaEventDisableTiming)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&b->e_y, cudaEventDisableTiming)) != cudaSuccess ||
-        (e = cudaEventCreateWithFlags(&b->e_consumed, cudaEventDisableTiming)) != cudaSuccess) {
+        (e = cudaEventCreateWithFlags(&b->e_swap[0], cudaEventDisableTiming)) != cudaSuccess) {
         cn_batch_destroy(b);
         return cn_cuda_fail(e, "cn_batch_create");
     }
+    for (int i = 1; i < CN_BATCH_SLOTS; ++i)
+        if ((e = cudaEventCreateWithFlags(&b->e_swap[i], cudaEventDisableTiming)) != cudaSuccess) {
+            cn_batch_destroy(b);
+            return cn_cuda_fail(e, "cn_batch_create");
+        }
+    b->e_consumed = b->e_swap[0];
     for (int i = 0; i < b->nb; ++i) {
         int st2;
         if (flags & CN_BATCH_SHARDED_UPLOAD) {
@@ -325,8 +352,8 @@ static int start_x_copy(cn_batch *b)
         b->staged_from = buf;
     }
     // do not overwrite a buffer while the work that read it may still run: its last reader is the batch before the current
-    // one (or, with one buffer, the last swap's transpose), and e_consumed, recorded at the last swap, follows both
-    CN_CUDA(cudaStreamWaitEvent(b->s_X, b->e_consumed, 0));
+    // one, and e_consumed, recorded at the last swap, follows that; or a swap's kernel
+    if (!b->turns || b->read[buf]) CN_CUDA(cudaStreamWaitEvent(b->s_X, b->turns ? b->read[buf] : b->e_consumed, 0));
     if (b->flags & CN_BATCH_SHARDED_UPLOAD) {
         // (1) every peer's buffer of this index must be free, and each rank says so only after its own e_consumed (waited
         //     for above); (2) own block over this rank's PCIe link; (3) the block into every peer's buffer over NVLink;
@@ -375,14 +402,25 @@ extern "C" int cn_batch_copy_next_async(cn_batch *b)
     // labels: always one batch ahead
     const int64_t idx = b->next_batch, r = rows_of_batch(b, idx);
     const float *src_y = b->h_y + (size_t)idx * b->batch * b->cols_y;
-    if (!b->direct) {
-        CN_CUDA(cudaEventSynchronize(b->e_y));   // the staging buffer is free once the last copy out of it has finished
-        memcpy(b->p_y, src_y, (size_t)r * b->cols_y * sizeof(float));
-        src_y = b->p_y;
+    const size_t bytes_y = (size_t)r * b->cols_y * sizeof(float);
+    if (b->slot_y) {
+        const int slot = (int)(b->swaps % CN_BATCH_SLOTS);
+        cudaStreamCaptureMode capture = cudaStreamCaptureModeRelaxed;   // another stream may be recording a graph
+        CN_CUDA(cudaThreadExchangeStreamCaptureMode(&capture));
+        const cudaError_t e = cudaEventSynchronize(b->e_swap[slot]);   // the swap before the last fifteen: finished long ago but where the host is far ahead
+        CN_CUDA(cudaThreadExchangeStreamCaptureMode(&capture));
+        CN_CUDA(e);
+        memcpy(b->slot_y + (size_t)slot * b->batch * b->cols_y, src_y, bytes_y);
+    } else {
+        if (!b->direct) {
+            CN_CUDA(cudaEventSynchronize(b->e_y));   // the staging buffer is free once the last copy out of it has finished
+            memcpy(b->p_y, src_y, bytes_y);
+            src_y = b->p_y;
+        }
+        CN_CUDA(cudaStreamWaitEvent(b->s_y, b->e_consumed, 0));
+        CN_CUDA(cudaMemcpyAsync(b->dn_y, src_y, bytes_y, cudaMemcpyHostToDevice, b->s_y));
+        CN_CUDA(cudaEventRecord(b->e_y, b->s_y));
     }
-    CN_CUDA(cudaStreamWaitEvent(b->s_y, b->e_consumed, 0));
-    CN_CUDA(cudaMemcpyAsync(b->dn_y, src_y, (size_t)r * b->cols_y * sizeof(float), cudaMemcpyHostToDevice, b->s_y));
-    CN_CUDA(cudaEventRecord(b->e_y, b->s_y));
     // X: one copy in flight, or two with CN_BATCH_LOOKAHEAD (the first call then starts two)
     while (b->in_flight < b->depth) {
         int st = start_x_copy(b);
@@ -402,14 +440,16 @@ extern "C" int cn_batch_swap(cn_batch *b, void *stream, float **d_X, float **d_y
                "cn_batch_swap: the copied batch (%lld) is not the next one (%lld)", (long long)b->idx_in[buf], (long long)b->next_batch);
     cudaStream_t s = cn_stream(stream);
     CN_CUDA(cudaStreamWaitEvent(s, b->e_Xb[buf], 0));
-    CN_CUDA(cudaStreamWaitEvent(s, b->e_y, 0));
-    int st = CN_OK;
-    if (!(b->flags & CN_BATCH_NO_COL_MAJOR)) st = cn_to_col_major(b->ctx, b->xb[buf], b->dc_X, b->next_rows, b->cols_X, stream);
-    if (st == CN_OK) st = cn_to_col_major(b->ctx, b->dn_y, b->dc_y, b->next_rows, b->cols_y, stream);
+    const int slot = (int)(b->swaps % CN_BATCH_SLOTS);
+    if (!b->slot_y) CN_CUDA(cudaStreamWaitEvent(s, b->e_y, 0));
+    const float *y = b->slot_y ? b->slot_y + (size_t)slot * b->batch * b->cols_y : b->dn_y;
+    const int st = cn_transpose_batch(b->xb[buf], b->dc_X, y, b->dc_y, b->next_rows, b->cols_X, b->cols_y, s);
     if (st != CN_OK) return st;
     // everything queued on the compute stream so far - the transposes above and the caller's work on the batch that was
     // current until now - precedes this event; the next copy waits for it before it overwrites a buffer
+    b->e_consumed = b->read[buf] = b->e_swap[slot];
     CN_CUDA(cudaEventRecord(b->e_consumed, s));
+    b->swaps += 1;
     b->cur_rows = b->next_rows;
     if (b->flags & CN_BATCH_KEEP_ROW_MAJOR) b->cur_rm = b->xb[buf];   // stays valid until the next swap
     b->ready = (buf + 1) % b->nb;

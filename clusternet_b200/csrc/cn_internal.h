@@ -81,6 +81,8 @@ void cn_gemm_workspace_free(cn_context *ctx);
 // in cn_gemm.h).
 int cn_status_block(cn_context *ctx, unsigned int **d_status);
 // cn_layout.cu: out (C x R, row-major, pitch ldo) = transpose of in (R x C, row-major, pitch ldi)
+// ... outX (null: not wanted) = transpose of X (R x C), outy = transpose of y (R x CY), in one launch; y may lie in pinned host memory
+int cn_transpose_batch(const float *X, float *outX, const float *y, float *outy, int64_t R, int64_t C, int64_t CY, cudaStream_t s);
 int cn_transpose_pitched(const float *in, int64_t ldi, float *out, int64_t ldo, int64_t R, int64_t C, cudaStream_t s);
 // cn_comm.cu
 void cn_comm_state_free(cn_context *ctx);

@@ -7,14 +7,9 @@
 #define TP_TILE 32
 #define TP_ROWS 8
 
-// out (C x R, row-major, pitch ldo) = transpose of in (R x C, row-major, pitch ldi).  One CTA per 32x32 tile, linear tile index.
-__global__ void __launch_bounds__(TP_TILE *TP_ROWS)
-cn_transpose_kernel(const float *in, int64_t ldi, float *out, int64_t ldo, int64_t R, int64_t C, int64_t tiles_c)
+__device__ __forceinline__ void transpose_tile(const float *in, int64_t ldi, float *out, int64_t ldo, int64_t R, int64_t C, int64_t tiles_c, int64_t tile_id)
 {
     __shared__ float tile[TP_TILE][TP_TILE + 1];
-    cn_pdl_launch_dependents();
-    cn_pdl_wait();
-    const int64_t tile_id = blockIdx.x;
     const int64_t tr = tile_id / tiles_c, tc = tile_id % tiles_c;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const int64_t c = tc * TP_TILE + tx;
@@ -29,6 +24,32 @@ cn_transpose_kernel(const float *in, int64_t ldi, float *out, int64_t ldo, int64
     for (int j = ty; j < TP_TILE; j += TP_ROWS) {
         const int64_t c2 = tc * TP_TILE + j;
         if (r2 < R && c2 < C) out[c2 * ldo + r2] = tile[tx][j];
+    }
+}
+
+// out (C x R, row-major, pitch ldo) = transpose of in (R x C, row-major, pitch ldi).  One CTA per 32x32 tile, linear tile index.
+__global__ void __launch_bounds__(TP_TILE *TP_ROWS)
+cn_transpose_kernel(const float *in, int64_t ldi, float *out, int64_t ldo, int64_t R, int64_t C, int64_t tiles_c)
+{
+    cn_pdl_launch_dependents();
+    cn_pdl_wait();
+    transpose_tile(in, ldi, out, ldo, R, C, tiles_c, blockIdx.x);
+}
+
+// A batch and its labels (R rows of CY, which may lie in pinned host memory) in one launch: the first CTAs take the labels, a few of the
+// rows' elements per thread in the order they lie in, since what bounds them is the trip over PCIe, beside which the batch is transposed.
+__global__ void __launch_bounds__(TP_TILE *TP_ROWS)
+cn_transpose_batch_kernel(const float *X, float *outX, const float *y, float *outy, int64_t R, int64_t C, int64_t CY, int64_t tiles_c, int y_ctas)
+{
+    cn_pdl_launch_dependents();
+    cn_pdl_wait();
+    if ((int)blockIdx.x >= y_ctas) {
+        transpose_tile(X, C, outX, R, R, C, tiles_c, (int64_t)blockIdx.x - y_ctas);
+        return;
+    }
+    for (int64_t i = (int64_t)blockIdx.x * (TP_TILE * TP_ROWS) + threadIdx.x; i < R * CY; i += (int64_t)y_ctas * (TP_TILE * TP_ROWS)) {
+        const int64_t r = i / CY;
+        outy[(i - r * CY) * R + r] = y[i];
     }
 }
 
@@ -47,6 +68,17 @@ int cn_transpose_pitched(const float *in, int64_t ldi, float *out, int64_t ldo, 
     const int64_t tiles = tiles_r * tiles_c;
     CN_REQUIRE(tiles < (1LL << 31), CN_ERR_UNSUPPORTED, "transpose: %lld tiles exceed the grid limit", (long long)tiles);
     CN_CUDA(cn_launch_pdl(cn_transpose_kernel, dim3((unsigned)tiles), TP_TILE * TP_ROWS, 0, s, in, ldi, out, ldo, R, C, tiles_c));
+    cn_count_launch();
+    return CN_OK;
+}
+
+int cn_transpose_batch(const float *X, float *outX, const float *y, float *outy, int64_t R, int64_t C, int64_t CY, cudaStream_t s)
+{
+    const int64_t tiles_c = (C + TP_TILE - 1) / TP_TILE, tiles = outX ? (R + TP_TILE - 1) / TP_TILE * tiles_c : 0;
+    const int64_t want = (R * CY + TP_TILE * TP_ROWS - 1) / (TP_TILE * TP_ROWS), y_ctas = want < 64 ? want : 64;
+    CN_REQUIRE(tiles + y_ctas < (1LL << 31), CN_ERR_UNSUPPORTED, "transpose: %lld tiles exceed the grid limit", (long long)tiles);
+    if (tiles + y_ctas == 0) return CN_OK;
+    CN_CUDA(cn_launch_pdl(cn_transpose_batch_kernel, dim3((unsigned)(tiles + y_ctas)), TP_TILE * TP_ROWS, 0, s, X, outX, y, outy, R, C, CY, tiles_c, (int)y_ctas));
     cn_count_launch();
     return CN_OK;
 }

@@ -214,6 +214,36 @@ def test_packed_gradient_exchange_is_a_no_op_on_one_rank(ctx):
     assert ctx.lib.cn_grad_sync_8bit_multi(ctx.h, g.data_ptr(), seg, 1, 0.0, ctx.stream_ptr()) == _lib.CN_ERR_ARG
 
 
+@pytest.mark.parametrize("B,cols,cols_y", [(32, 8, 1), (48, 33, 3), (32, 8, 128), (32, 8, 129), (1, 5, 2)])
+@pytest.mark.parametrize("pinned", [False, True])
+def test_batches_far_ahead_of_the_gpu(ctx, B, cols, cols_y, pinned):
+    """Many batches without a wait for the GPU, which is busy at first: labels in slots that come round (up to 16 KB a batch) and beyond, and
+    a last batch that is short."""
+    rows = 40 * B + B // 2
+    X, y = torch.arange(rows * cols, dtype=torch.float32).view(rows, cols), torch.arange(rows * cols_y, dtype=torch.float32).view(rows, cols_y) + 0.5
+    hX, hy = (X.pin_memory(), y.pin_memory()) if pinned else (X, y)
+    h = ctypes.c_void_p()
+    cn.check(ctx.lib.cn_batch_create(ctx.h, hX.data_ptr(), hy.data_ptr(), rows, cols, cols_y, B, 0, ctypes.byref(h)))
+    px, py, n = ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_int64()
+
+    def view(p, c):
+        class Raw:
+            __cuda_array_interface__ = {"shape": (c, n.value), "typestr": "<f4", "data": (p.value, False), "version": 2, "strides": None}
+        return torch.as_tensor(Raw(), device="cuda")
+    total = ctx.lib.cn_batch_total_batches(h)
+    got = []
+    torch.cuda._sleep(50_000_000)
+    for step in range(2 * total):
+        cn.check(ctx.lib.cn_batch_copy_next_async(h))
+        cn.check(ctx.lib.cn_batch_swap(h, ctx.stream_ptr(), ctypes.byref(px), ctypes.byref(py), ctypes.byref(n)))
+        got.append((view(px, cols).clone(), view(py, cols_y).clone()))
+    torch.cuda.synchronize()
+    for step, (gx, gy) in enumerate(got):
+        i = (step + 1) % total * B
+        assert torch.equal(gx.t().cpu(), X[i:i + B]) and torch.equal(gy.t().cpu(), y[i:i + B])
+    ctx.lib.cn_batch_destroy(h)
+
+
 def test_batch_size_larger_than_data_is_rejected(ctx):
     x = torch.zeros(10, 4)
     h = ctypes.c_void_p()
