@@ -273,6 +273,11 @@ cn_compress_kernel(const float *A, float precision_arg, const float *d_precision
 #define RING_STAGES 3                       // per CTA: 6 tiles = 192 KB in flight per SM
 #define RING_GROUPS_PER_THREAD (RING_TILE / 4 / RING_THREADS)
 #define CN_FUSED_ABSMAX_MAX_N (4LL << 20)   // above this size cn_absmax_compress_8bit issues two launches
+// Behind an absmax of the ring kind the tensor is coded from its end where L2 (126 MB) does not hold all of it beside the codes and the decoded
+// values: scale, codes and decoded values of 16 Mi elements 47 -> 43 us, 24 Mi 71 -> 65, 32 Mi 90 -> 84, 64 Mi 172 -> 165.  Smaller ones gain
+// nothing; larger ones are read past L2 by the other absmax (evict-first; 128 Mi 320, 337 with both changed).
+#define CN_BACKWARDS_MIN_N (16LL << 20)
+#define CN_ABSMAX_RING_MAX_N (1LL << 27)
 #define RING_WAIT_LIMIT (4000000000LL)      // clock cycles (~2 s)
 
 __device__ __forceinline__ uint32_t cdc_smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -483,7 +488,7 @@ enum { RING_SCALE_HOST = 0, RING_SCALE_DEVICE = 1 };
 // Work split: every CTA codes the same number of tiles (tiles_per_cta) of the same size (tile_groups 16-byte groups,
 // at most RING_TILE / 4), chosen on the host so that grid * tiles_per_cta tiles cover the tensor with less than one
 // group of slack per tile; tile j goes to CTA j % grid.  The last tiles may be short or missing.
-template <int SCALE>
+template <int SCALE, bool BACKWARDS>
 __global__ void __launch_bounds__(RING_THREADS, 2)
 cn_compress_ring_kernel(const float *A, float precision_arg, const float *d_precision,
                         int64_t n, uint8_t *out, const __grid_constant__ RingConst rc, unsigned int *status,
@@ -511,15 +516,20 @@ cn_compress_ring_kernel(const float *A, float precision_arg, const float *d_prec
     const int64_t groups_total = n >> 2;                    // 16-byte groups of the tensor
     // tiles of this CTA that hold data: tile (blockIdx.x + k * gridDim.x), k = 0 .. my_tiles - 1
     int my_tiles = 0;
+    const int64_t tiles_total = (groups_total + tile_groups - 1) / tile_groups;
     {
-        const int64_t tiles_total = (groups_total + tile_groups - 1) / tile_groups;
         if ((int64_t)blockIdx.x < tiles_total) {
             const int64_t mine = (tiles_total - blockIdx.x + gridDim.x - 1) / gridDim.x;
             my_tiles = (int)(mine < tiles_per_cta ? mine : tiles_per_cta);
         }
     }
     // the i-th tile this CTA codes and its size in 16-byte groups
-    auto tile_of = [&](int i) { return (int64_t)blockIdx.x + (int64_t)i * gridDim.x; };
+    // BACKWARDS: behind its own absmax, from the end of the tensor, which is still in L2; the codes written last are then those that a decoder
+    // behind it reads first.
+    auto tile_of = [&](int i) {
+        const int64_t t = (int64_t)blockIdx.x + (int64_t)i * gridDim.x;
+        return BACKWARDS ? tiles_total - 1 - t : t;
+    };
     auto tile_count = [&](int64_t j) {
         const int64_t left = groups_total - j * tile_groups;
         return (int)(left < tile_groups ? left : tile_groups);
@@ -1457,8 +1467,9 @@ static int compress_impl(cn_context *ctx, const float *d_A, float precision, con
         const size_t smem = (size_t)RING_STAGES * RING_TILE * 4 + 128;
         const int dev = ctx->device;
         if (dev < 0 || dev >= 64 || !attr_set[dev]) {
-            CN_CUDA(cudaFuncSetAttribute(cn_compress_ring_kernel<RING_SCALE_HOST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-            CN_CUDA(cudaFuncSetAttribute(cn_compress_ring_kernel<RING_SCALE_DEVICE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            CN_CUDA(cudaFuncSetAttribute(cn_compress_ring_kernel<RING_SCALE_HOST, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            CN_CUDA(cudaFuncSetAttribute(cn_compress_ring_kernel<RING_SCALE_DEVICE, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            CN_CUDA(cudaFuncSetAttribute(cn_compress_ring_kernel<RING_SCALE_DEVICE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             if (dev >= 0 && dev < 64) attr_set[dev] = true;
         }
         unsigned int *d_status = nullptr;
@@ -1482,10 +1493,11 @@ static int compress_impl(cn_context *ctx, const float *d_A, float precision, con
         // the exactly balanced size
         if ((int64_t)tiles_per_cta * max_groups * 100 <= (int64_t)tiles_per_cta * tile_groups * 102) tile_groups = (int)max_groups;
         if (scale_mode == RING_SCALE_DEVICE) {
-            CN_CUDA(cn_launch_pdl(cn_compress_ring_kernel<RING_SCALE_DEVICE>, grid, RING_THREADS, smem, s, d_A, 0.f, d_precision, n, d_codes, rc, d_status,
+            const bool backwards = after_own_absmax && n >= CN_BACKWARDS_MIN_N && n < CN_ABSMAX_RING_MAX_N;
+            CN_CUDA(cn_launch_pdl(backwards ? cn_compress_ring_kernel<RING_SCALE_DEVICE, true> : cn_compress_ring_kernel<RING_SCALE_DEVICE, false>, grid, RING_THREADS, smem, s, d_A, 0.f, d_precision, n, d_codes, rc, d_status,
                                tile_groups, tiles_per_cta, after_own_absmax));
         } else {
-            CN_CUDA(cn_launch_pdl(cn_compress_ring_kernel<RING_SCALE_HOST>, grid, RING_THREADS, smem, s, d_A, precision, (const float *)nullptr, n, d_codes, rc,
+            CN_CUDA(cn_launch_pdl(cn_compress_ring_kernel<RING_SCALE_HOST, false>, grid, RING_THREADS, smem, s, d_A, precision, (const float *)nullptr, n, d_codes, rc,
                                d_status, tile_groups, tiles_per_cta, 0));
         }
         cn_count_launch();
@@ -1700,7 +1712,7 @@ extern "C" int cn_absmax_f32(cn_context *ctx, const float *d_A, int64_t n, float
     CN_REQUIRE(ctx && d_out, CN_ERR_ARG, "cn_absmax_f32: null argument");
     CN_REQUIRE(n >= 0 && (n == 0 || d_A), CN_ERR_ARG, "cn_absmax_f32: bad input");
     int vector_ok = ((uintptr_t)d_A % 16 == 0);
-    if (vector_ok && n >= (1LL << 16) && n < (1LL << 27)) {
+    if (vector_ok && n >= (1LL << 16) && n < CN_ABSMAX_RING_MAX_N) {
         // mid-sized tensors: the ring kernel (see there); small ones are launch-bound, large ones stream best below
         static bool attr_set[64] = {};
         const size_t smem = (size_t)RING_STAGES * RING_TILE * 4 + 128;

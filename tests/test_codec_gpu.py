@@ -322,3 +322,16 @@ def test_against_reference_kernels_on_this_gpu(ctx):
     assert torch.equal(out, ref_out)
     tmp = torch.empty_like(d)
     assert L.ref_absmax(fp(d.data_ptr()), fp(tmp.data_ptr()), n) == float(ctx.absmax(d).item())
+
+
+@pytest.mark.parametrize("n", [(16 << 20) - 1, 16 << 20, (16 << 20) + 5, 20_000_003, (1 << 25) + 4096 * 7 + 2])
+def test_scale_and_codes_from_the_end_of_a_tensor(ctx, n):
+    """Tensors that L2 does not hold are coded from their end: the codes of the two calls, the last tile short or not, nothing behind them."""
+    x = torch.randn(n, device="cuda")
+    x[-1], x[0], x[n // 2] = 9.0, -8.5, float("nan")
+    codes, scale = torch.full((n + 64,), 77, dtype=torch.uint8, device="cuda"), torch.empty(1, device="cuda")
+    ctx.absmax_compress(x, scale=scale, out=codes[:n])
+    ctx.gemm_check()
+    assert scale.item() == 9.0
+    assert torch.equal(codes[:n], ctx.compress(x, 9.0)) and bool((codes[n:] == 77).all())
+    assert np.array_equal(codes[n - 100000:n].cpu().numpy(), oracle.compress(ctx.codebook, x[n - 100000:].cpu().numpy(), 9.0))
