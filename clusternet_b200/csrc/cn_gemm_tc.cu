@@ -490,8 +490,8 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
                             const int s = it % Cfg::A_STAGES;
                             ok = mbar_wait(aempty_bar(s), ((it / Cfg::A_STAGES) & 1u) ^ 1u, abort_flag, p.status, 8u);
                             if (!ok) break;
-                            if (band == 0) sts1u(smem_base + Cfg::BAND_OFF + s * 4, masks);
                             const uint32_t stage = smem_base + Cfg::A_RING + s * Cfg::A_STAGE_BYTES;
+                            if (band == 0) sts1u(smem_base + Cfg::BAND_OFF + s * 4, masks);
                             mbar_expect_tx(afull_bar(s), (uint32_t)((MODE3X ? 2 : 1) * TC_A_TILE_BYTES));
                             tma_load_3d(stage, &tm_a, afull_bar(s), kb * TC_WK, m0, band * (MODE3X ? 2 : 1));
                             if (MODE3X) tma_load_3d(stage + TC_A_TILE_BYTES, &tm_a, afull_bar(s), kb * TC_WK, m0, 2 * band + 1);
@@ -1059,6 +1059,19 @@ cn_splitk_reduce_kernel(const __grid_constant__ ReduceParams p)
     constexpr int QSTEP = 256 / COLS, QUADS = 32 / QSTEP, UNROLL = 8 / QUADS;   // quads of m per thread; partial tiles in flight
     __shared__ float turn[COLS][TC_BM + 4];
     cn_pdl_launch_dependents();
+    // where this CTA's partial tiles are, worked out (divisions of 64 bits) while the product still runs
+    const int chunk = blockIdx.x % (TC_BN / COLS);
+    const int tw = blockIdx.x / (TC_BN / COLS), rm = tw / p.nt, w = tw - rm * p.nt, r = rm / p.mt, mh = rm - r * p.mt, tile = p.full_tiles + r;
+    const int64_t m0 = ((int64_t)(tile % p.tiles_m) * p.mt + mh) * p.rows, n0 = ((int64_t)(tile / p.tiles_m) * p.nt + w) * TC_BN + chunk * COLS;
+    // the CTAs whose runs hold K blocks of this tile: run c is [total c / ctas, total (c + 1) / ctas)
+    const int64_t total = (int64_t)p.tail_tiles * p.kb_total, first = (int64_t)r * p.kb_total, last = first + p.kb_total - 1;
+    auto owner = [&](int64_t x) {
+        int64_t c = x * p.tail_ctas / total;
+        while (total * (c + 1) / p.tail_ctas <= x) ++c;
+        while (total * c / p.tail_ctas > x) --c;
+        return c;
+    };
+    const int64_t c0 = owner(first), c1 = owner(last);
     cn_pdl_wait();
     if (p.npeers > 0) {   // peers must have announced that their copy of C may be overwritten (bounded wait)
         if (threadIdx.x == 0) {
@@ -1075,19 +1088,7 @@ cn_splitk_reduce_kernel(const __grid_constant__ ReduceParams p)
         __syncthreads();
     }
     if (p.cond && !__syncthreads_or(threadIdx.x == 0 && __ldcg(p.cond) != 0u)) return;
-    const int chunk = blockIdx.x % (TC_BN / COLS);
-    const int tw = blockIdx.x / (TC_BN / COLS), rm = tw / p.nt, w = tw - rm * p.nt, r = rm / p.mt, mh = rm - r * p.mt, tile = p.full_tiles + r;
-    const int64_t m0 = ((int64_t)(tile % p.tiles_m) * p.mt + mh) * p.rows, n0 = ((int64_t)(tile / p.tiles_m) * p.nt + w) * TC_BN + chunk * COLS;
     if (n0 >= p.N || m0 >= p.M) return;
-    // the CTAs whose runs hold K blocks of this tile: run c is [total c / ctas, total (c + 1) / ctas)
-    const int64_t total = (int64_t)p.tail_tiles * p.kb_total, first = (int64_t)r * p.kb_total, last = first + p.kb_total - 1;
-    auto owner = [&](int64_t x) {
-        int64_t c = x * p.tail_ctas / total;
-        while (total * (c + 1) / p.tail_ctas <= x) ++c;
-        while (total * c / p.tail_ctas > x) --c;
-        return c;
-    };
-    const int64_t c0 = owner(first), c1 = owner(last);
     const int row = threadIdx.x % COLS, quad = threadIdx.x / COLS;   // column of the chunk; quads of m: quad + QSTEP j
     constexpr int64_t TILE4 = TC_BM * TC_BN / 4;
     const float4 *src = reinterpret_cast<const float4 *>(p.partials) + (((c0 + r) * p.mt + mh) * p.nt + w) * TILE4 + quad * TC_BN + chunk * COLS + row;
@@ -1096,24 +1097,19 @@ cn_splitk_reduce_kernel(const __grid_constant__ ReduceParams p)
 #pragma unroll
     for (int j = 0; j < QUADS; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
     int64_t left = c1 - c0 + 1;
-    // the additions stay in K order, so the sum does not depend on the grouping
-    for (; left >= UNROLL; left -= UNROLL, src += UNROLL * step) {
+    // the additions stay in K order, so the sum does not depend on the grouping; what is left of a group is loaded together, too
+    for (; left > 0; left -= UNROLL, src += UNROLL * step) {
         float4 v[UNROLL][QUADS];
 #pragma unroll
         for (int u = 0; u < UNROLL; ++u)
 #pragma unroll
-            for (int j = 0; j < QUADS; ++j) v[u][j] = __ldcs(src + u * step + j * QSTEP * TC_BN);
+            for (int j = 0; j < QUADS; ++j)
+                if (u < left) v[u][j] = __ldcs(src + u * step + j * QSTEP * TC_BN);
 #pragma unroll
         for (int u = 0; u < UNROLL; ++u)
 #pragma unroll
-            for (int j = 0; j < QUADS; ++j) { acc[j].x += v[u][j].x; acc[j].y += v[u][j].y; acc[j].z += v[u][j].z; acc[j].w += v[u][j].w; }
-    }
-    for (; left > 0; --left, src += step) {
-#pragma unroll
-        for (int j = 0; j < QUADS; ++j) {
-            const float4 v = __ldcs(src + j * QSTEP * TC_BN);
-            acc[j].x += v.x; acc[j].y += v.y; acc[j].z += v.z; acc[j].w += v.w;
-        }
+            for (int j = 0; j < QUADS; ++j)
+                if (u < left) { acc[j].x += v[u][j].x; acc[j].y += v[u][j].y; acc[j].z += v[u][j].z; acc[j].w += v[u][j].w; }
     }
 #pragma unroll
     for (int j = 0; j < QUADS; ++j) *reinterpret_cast<float4 *>(&turn[row][(quad + QSTEP * j) * 4]) = acc[j];
