@@ -1138,21 +1138,32 @@ cn_decompress_kernel(const uint8_t *codes, float precision_arg, const float *d_p
     const uint32_t *in4 = reinterpret_cast<const uint32_t *>(codes);
     // the first codes are on their way while the table is made
     uint32_t cur[4];
+    const bool whole = v + 3 * stride < nvec;
+    if (whole) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u)
-        if (v + u * stride < nvec) cur[u] = __ldcs(in4 + v + u * stride);
+        for (int u = 0; u < 4; ++u) cur[u] = __ldcs(in4 + v + u * stride);
+    } else {
+#pragma unroll
+        for (int u = 0; u < 3; ++u)
+            if (v + u * stride < nvec) cur[u] = __ldcs(in4 + v + u * stride);
+    }
     if (PRECISION_ON_DEVICE) make_table(*d_precision);
     __syncthreads();
     if (blockIdx.x == 0 && tid < head) first_out[tid] = lut[first[tid]];
-    if (v + 3 * stride < nvec) {
+    if (whole) {
         const int64_t step = 4 * stride;
         while (true) {
             const int64_t vn = v + step;
             const bool more = vn + 3 * stride < nvec;
             uint32_t nxt[4];
+            if (more) {
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-                if (vn + u * stride < nvec) nxt[u] = __ldcs(in4 + vn + u * stride);
+                for (int u = 0; u < 4; ++u) nxt[u] = __ldcs(in4 + vn + u * stride);
+            } else {
+#pragma unroll
+                for (int u = 0; u < 3; ++u)
+                    if (vn + u * stride < nvec) nxt[u] = __ldcs(in4 + vn + u * stride);
+            }
 #pragma unroll
             for (int u = 0; u < 4; ++u) __stcs(out4 + v + u * stride, CN_DEC4(cur[u]));
             v = vn;

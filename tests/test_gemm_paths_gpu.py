@@ -396,6 +396,22 @@ def test_softmax_at_the_edge_of_the_register_rows(ctx, cols):
     assert np.abs(ctx.to_numpy(out) - oracle.softmax_rows(A)).max() < 2e-6       # __expf against libm's exp
 
 
+@pytest.mark.parametrize("cols", [1, 2, 10, 31, 32])
+@pytest.mark.parametrize("rows", [1, 5, 4095])
+def test_softmax_of_few_rows_gives_the_bits_of_many(ctx, rows, cols):
+    """A warp per row against a thread per row, with infinities and NaN among the values, in place and with the error."""
+    g = torch.Generator(device="cuda").manual_seed(rows + cols)
+    big = torch.randn((cols, 4096 + rows), device="cuda", generator=g) * 5
+    big[0, 0], big[-1, 0], big[0, min(2, rows - 1)], big[-1, min(3, rows - 1)] = float("inf"), float("nan"), float("-inf"), -1e38
+    labels = torch.randint(0, cols, (4096 + rows,), device="cuda", generator=g).float()
+    few, want, want_err, err = big[:, :rows].contiguous(), torch.empty_like(big), torch.empty_like(big), torch.empty((cols, rows), device="cuda")
+    lib, h, s = ctx.lib, ctx.h, ctx.stream_ptr()
+    assert lib.cn_softmax_error(h, big.data_ptr(), labels.data_ptr(), want.data_ptr(), want_err.data_ptr(), 4096 + rows, cols, s) == 0
+    assert lib.cn_softmax_error(h, few.data_ptr(), labels.data_ptr(), few.data_ptr(), err.data_ptr(), rows, cols, s) == 0
+    assert torch.equal(few.view(torch.int32), want[:, :rows].contiguous().view(torch.int32))
+    assert torch.equal(err.view(torch.int32), want_err[:, :rows].contiguous().view(torch.int32))
+
+
 # tiles whose K a cluster of CTAs shares (one tile of rows, short K, weights beyond the small products'): one and two tiles of columns per CTA,
 # clusters of 2 to 8, rows that give some CTAs nothing to finish, last tiles of few columns; weights of either layout and of odd pitch
 SHARED = [(24, 560, 5192), (100, 1500, 2500), (128, 1024, 3000), (17, 640, 9001), (128, 2000, 8000), (1, 992, 6000), (72, 912, 3624), (120, 777, 4099), (97, 528, 7258)]
