@@ -1125,6 +1125,8 @@ cn_decompress_kernel(const uint8_t *codes, float precision_arg, const float *d_p
     };
     if (!PRECISION_ON_DEVICE) make_table(precision_arg);   // a host scale lets the table precede the wait
     cn_pdl_wait();
+    float scale = precision_arg;
+    if (PRECISION_ON_DEVICE) asm volatile("ld.global.f32 %0, [%1];" : "=f"(scale) : "l"(d_precision) : "memory");   // asked for before the codes
     const uint8_t *first = codes;
     float *first_out = out;
     codes += head;
@@ -1147,7 +1149,7 @@ cn_decompress_kernel(const uint8_t *codes, float precision_arg, const float *d_p
         for (int u = 0; u < 3; ++u)
             if (v + u * stride < nvec) cur[u] = __ldcs(in4 + v + u * stride);
     }
-    if (PRECISION_ON_DEVICE) make_table(*d_precision);
+    if (PRECISION_ON_DEVICE) make_table(scale);
     __syncthreads();
     if (blockIdx.x == 0 && tid < head) first_out[tid] = lut[first[tid]];
     if (whole) {
