@@ -32,7 +32,7 @@ def check(C, A, B, transA, transB, rel):
     assert np.all(err <= bound), float((err / np.maximum(bound, 1e-300)).max())
 
 
-# one row, one column, one k-step; tile edges; odd pitches; one CTA per tile, clusters of 2, 4 and 8; several accumulation chains
+# one row, one column, one k-step; tile edges; odd pitches; one CTA per tile, clusters; several accumulation chains
 SMALL = [(1, 4096, 1), (17, 33, 15), (128, 31, 128), (129, 97, 127), (127, 1201, 129), (128, 785, 1201), (1201, 128, 1201), (203, 2049, 301),
          (16, 8193, 100), (500, 130, 64)]
 
@@ -55,7 +55,7 @@ def test_small_products_in_every_layout(ctx, M, K, N, transA, transB):
             check(C, A, B, transA, transB, rel)
 
 
-# tiles of 32, 64 and 128 columns, by one CTA and by clusters of 2, 4 and 8; more blocks than accumulators
+# tiles of 32, 64 and 128 columns, by one CTA and by clusters; more blocks than accumulators
 @pytest.mark.parametrize("M,K,N", [(48, 80, 1091), (128, 1200, 10), (1200, 128, 10), (784, 128, 1200), (32, 500, 500), (1200, 120, 1201), (512, 500, 1000), (128, 785, 1100),
                                    (200, 380, 2100), (64, 3000, 600)])
 @pytest.mark.parametrize("act", [_lib.ACT_LINEAR, _lib.ACT_RELU, _lib.ACT_LOGISTIC])
