@@ -490,8 +490,8 @@ int cn_batch_set_skip_last(cn_batch *b, int skip_last_batch);
 /* Stage + asynchronous copy of the next batch (allocate_next_batch_async). */
 int cn_batch_copy_next_async(cn_batch *b);
 /* Make the next batch current (replace_current_batch_with_next): waits (on the device, through an
- * event) for the copies, transposes into the current-batch buffers on `stream`, advances the counter
- * with wrap-around.  Returns the device pointers and the row count of the batch (the last batch of an
+ * event) for the copies and for the swap before, on whatever stream that was, transposes into the
+ * current-batch buffers on `stream`, advances the counter with wrap-around.  Returns the device pointers and the row count of the batch (the last batch of an
  * epoch may be short). */
 int cn_batch_swap(cn_batch *b, void *stream, float **d_X, float **d_y, int64_t *batch_rows);
 

@@ -244,6 +244,59 @@ def test_batches_far_ahead_of_the_gpu(ctx, B, cols, cols_y, pinned):
     ctx.lib.cn_batch_destroy(h)
 
 
+class Batches:
+    """A batch allocator over numbers that say which batch they belong to, the data set in pinned memory."""
+
+    def __init__(self, ctx, B, cols, cols_y, batches, flags=0):
+        self.lib, self.B, self.cols, self.cols_y, rows = ctx.lib, B, cols, cols_y, batches * B
+        self.X = torch.arange(rows * cols, dtype=torch.float32).view(rows, cols).pin_memory()
+        self.y = (torch.arange(rows * cols_y, dtype=torch.float32).view(rows, cols_y) + 0.5).pin_memory()
+        self.h, self.px, self.py, self.n = ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_int64()
+        cn.check(ctx.lib.cn_batch_create_ex(ctx.h, self.X.data_ptr(), self.y.data_ptr(), rows, cols, cols_y, B, 0, flags, ctypes.byref(self.h)))
+
+    def next(self, stream):
+        cn.check(self.lib.cn_batch_copy_next_async(self.h))
+        cn.check(self.lib.cn_batch_swap(self.h, ctypes.c_void_p(stream.cuda_stream), ctypes.byref(self.px), ctypes.byref(self.py), ctypes.byref(self.n)))
+
+    def view(self, p, cols):
+        n = self.n.value
+
+        class Raw:
+            __cuda_array_interface__ = {"shape": (cols, n), "typestr": "<f4", "data": (p.value, False), "version": 2, "strides": None}
+        return torch.as_tensor(Raw(), device="cuda")
+
+    def current(self):
+        """Column-major: (cols, rows).  None for X where it is not turned."""
+        return (self.view(self.px, self.cols) if self.px.value else None), self.view(self.py, self.cols_y)
+
+    def is_batch(self, i, X, y):
+        at = slice(i * self.B, (i + 1) * self.B)
+        return (X is None or torch.equal(X.t().cpu(), self.X[at])) and torch.equal(y.t().cpu(), self.y[at])
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *a):
+        torch.cuda.synchronize()
+        self.lib.cn_batch_destroy(self.h)
+
+
+@pytest.mark.parametrize("flags", [0, _lib.BATCH_KEEP_ROW_MAJOR, _lib.BATCH_LOOKAHEAD])
+@pytest.mark.parametrize("B,cols,cols_y", [(32, 40, 1), (32, 40, 200), (1100, 1000, 2)])
+def test_swaps_on_two_streams_keep_their_order(ctx, flags, B, cols, cols_y):
+    """The first stream is busy when its swap is queued; the next batch's swap goes to another stream, and that batch is then the current one.
+    Labels in slots and beyond, one and two buffers."""
+    first, second = torch.cuda.Stream(), torch.cuda.Stream()
+    with Batches(ctx, B, cols, cols_y, 6, flags) as b:
+        for i in (1, 3):
+            with torch.cuda.stream(first):
+                torch.cuda._sleep(200_000_000)
+            b.next(first)
+            b.next(second)
+            torch.cuda.synchronize()
+            assert b.is_batch(i + 1, *b.current())
+
+
 def test_batch_size_larger_than_data_is_rejected(ctx):
     x = torch.zeros(10, 4)
     h = ctypes.c_void_p()
