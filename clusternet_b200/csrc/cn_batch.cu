@@ -26,7 +26,9 @@
 #include <string.h>
 #include "cn_internal.h"
 
-#define CN_BATCH_SLOTS 16                  // swaps whose ends are known
+#define CN_BATCH_SWAPS 16                  // swaps whose ends are known, and slots of labels that are given back together
+#define CN_BATCH_GROUPS 16                 // of such slots, at most: as many as have room in
+#define CN_BATCH_RING_BYTES (1 << 20)
 #define CN_BATCH_SMALL_BYTES (4 << 20)
 #define CN_BATCH_SLOT_BYTES (16 << 10)
 
@@ -43,9 +45,12 @@ struct cn_batch {
     bool direct = false;         // the data set itself is pinned: copy from it, no staging memcpy
     float *p_X = nullptr, *p_y = nullptr;     // pinned staging
     float *dn_y = nullptr;                    // device, next batch's labels, row-major
-    // Few labels: kept in pinned slots, from which the swap's kernel reads them over PCIe.  A slot is written again when the swap
-    // that read it, CN_BATCH_SLOTS before, has finished.
+    // Few labels: kept in pinned slots, from which the swap's kernel reads them over PCIe.  Sixteen slots are written again when the swap
+    // that read the last of them has finished; until then a pinned data set's labels go by the copy engine.
     float *slot_y = nullptr;
+    int groups = 0;                           // of CN_BATCH_SWAPS slots
+    bool group_free = false;                  // the group that the next batch's slot is in
+    bool in_slot = false;                     // where the next batch's labels are
     int64_t swaps = 0;
     // options (cn_batch_create_ex)
     int flags = 0;
@@ -73,7 +78,8 @@ struct cn_batch {
     float *dc_X = nullptr, *dc_y = nullptr;   // device, current batch, column-major
     cudaStream_t s_X = nullptr, s_y = nullptr;
     cudaEvent_t e_y = nullptr;
-    cudaEvent_t e_swap[CN_BATCH_SLOTS] = {}, e_consumed = nullptr;   // after the last swaps' kernels; after the last one's
+    cudaEvent_t e_swap[CN_BATCH_SWAPS] = {}, e_consumed = nullptr;   // after the last swaps' kernels; after the last one's
+    cudaEvent_t e_group[CN_BATCH_GROUPS] = {};                       // after the swap that read a group's last slot, in place of one of e_swap
 };
 
 // Sharded upload: this rank's block of the batch, already in its own buffer, goes to the same place in every peer's
@@ -125,6 +131,7 @@ extern "C" int cn_batch_destroy(cn_batch *b)
     for (cudaEvent_t e : b->e_Xb) if (e) cudaEventDestroy(e);
     if (b->e_y) cudaEventDestroy(b->e_y);
     for (cudaEvent_t e : b->e_swap) if (e) cudaEventDestroy(e);
+    for (cudaEvent_t e : b->e_group) if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : b->e_prof) if (e) cudaEventDestroy(e);
     delete b;
     return CN_OK;
@@ -183,10 +190,13 @@ extern "C" int cn_batch_create_ex(cn_context *ctx, const float *h_X, const float
     // to read them over PCIe, now that the next copy does not wait for that kernel.  Larger ones stay with the copy engine.  128 x 784 images with
     // a label each, us per batch: 19.1; with the second buffer, one kernel for both and the labels in slots 15.1 (with one buffer 23).
     const bool few = by <= CN_BATCH_SLOT_BYTES;
-    if ((few && (e = cudaHostAlloc(&b->slot_y, by * CN_BATCH_SLOTS, cudaHostAllocPortable | cudaHostAllocMapped)) != cudaSuccess) ||
+    // With up to 4 KB of labels per batch the host may be 240 batches ahead before labels take the copy engine, with 16 KB 48.  (With a hundred
+    // batches queued in a row and only sixteen slots, 128 x 784 images took 16 to 25 us; with the host waiting for a slot, 13.3 to 15.4.)
+    b->groups = !few ? 0 : by * CN_BATCH_SWAPS * CN_BATCH_GROUPS <= CN_BATCH_RING_BYTES ? CN_BATCH_GROUPS : (int)(CN_BATCH_RING_BYTES / (by * CN_BATCH_SWAPS));
+    if ((few && (e = cudaHostAlloc(&b->slot_y, by * CN_BATCH_SWAPS * b->groups, cudaHostAllocPortable | cudaHostAllocMapped)) != cudaSuccess) ||
         (!b->direct && (e = cudaHostAlloc(&b->p_X, bx, cudaHostAllocPortable)) != cudaSuccess) ||
         (!few && !b->direct && (e = cudaHostAlloc(&b->p_y, by, cudaHostAllocPortable)) != cudaSuccess) ||
-        (!few && (e = cudaMalloc(&b->dn_y, by)) != cudaSuccess) ||
+        ((!few || b->direct) && (e = cudaMalloc(&b->dn_y, by)) != cudaSuccess) ||
         (!(flags & CN_BATCH_NO_COL_MAJOR) && (e = cudaMalloc(&b->dc_X, bx)) != cudaSuccess) ||
         (e = cudaMalloc(&b->dc_y, by)) != cudaSuccess ||
         (e = cudaStreamCreateWithPriority(&b->s_X, cudaStreamNonBlocking, prio_high)) != cudaSuccess ||
@@ -199,8 +209,8 @@ extern "C" int cn_batch_create_ex(cn_context *ctx, const float *h_X, const float
         cn_batch_destroy(b);
         return cn_cuda_fail(e, "cn_batch_create");
     }
-    for (int i = 1; i < CN_BATCH_SLOTS; ++i)
-        if ((e = cudaEventCreateWithFlags(&b->e_swap[i], cudaEventDisableTiming)) != cudaSuccess) {
+    for (int i = 1; i < CN_BATCH_SWAPS + b->groups; ++i)
+        if ((e = cudaEventCreateWithFlags(i < CN_BATCH_SWAPS ? &b->e_swap[i] : &b->e_group[i - CN_BATCH_SWAPS], cudaEventDisableTiming)) != cudaSuccess) {
             cn_batch_destroy(b);
             return cn_cuda_fail(e, "cn_batch_create");
         }
@@ -403,15 +413,20 @@ extern "C" int cn_batch_copy_next_async(cn_batch *b)
     const int64_t idx = b->next_batch, r = rows_of_batch(b, idx);
     const float *src_y = b->h_y + (size_t)idx * b->batch * b->cols_y;
     const size_t bytes_y = (size_t)r * b->cols_y * sizeof(float);
-    if (b->slot_y) {
-        const int slot = (int)(b->swaps % CN_BATCH_SLOTS);
+    if (b->slot_y && !b->group_free) {
+        // Given back long ago but where the host is far ahead.  Staged batches wait for the GPU in any case; with a pinned data set nothing here does.
+        const cudaEvent_t last = b->e_group[b->swaps / CN_BATCH_SWAPS % b->groups];
         cudaStreamCaptureMode capture = cudaStreamCaptureModeRelaxed;   // another stream may be recording a graph
         CN_CUDA(cudaThreadExchangeStreamCaptureMode(&capture));
-        const cudaError_t e = cudaEventSynchronize(b->e_swap[slot]);   // the swap before the last fifteen: finished long ago but where the host is far ahead
+        const cudaError_t e = b->direct ? cudaEventQuery(last) : cudaEventSynchronize(last);
         CN_CUDA(cudaThreadExchangeStreamCaptureMode(&capture));
-        CN_CUDA(e);
-        memcpy(b->slot_y + (size_t)slot * b->batch * b->cols_y, src_y, bytes_y);
-    } else {
+        b->group_free = e != cudaErrorNotReady;
+        if (b->group_free) CN_CUDA(e);
+        else cudaGetLastError();
+    }
+    b->in_slot = b->group_free;
+    if (b->in_slot) memcpy(b->slot_y + (size_t)(b->swaps % (b->groups * CN_BATCH_SWAPS)) * b->batch * b->cols_y, src_y, bytes_y);
+    if (!b->in_slot) {
         if (!b->direct) {
             CN_CUDA(cudaEventSynchronize(b->e_y));   // the staging buffer is free once the last copy out of it has finished
             memcpy(b->p_y, src_y, bytes_y);
@@ -443,16 +458,18 @@ extern "C" int cn_batch_swap(cn_batch *b, void *stream, float **d_X, float **d_y
     // also where the stream is the same)
     CN_CUDA(cudaStreamWaitEvent(s, b->e_consumed, 0));
     CN_CUDA(cudaStreamWaitEvent(s, b->e_Xb[buf], 0));
-    const int slot = (int)(b->swaps % CN_BATCH_SLOTS);
-    if (!b->slot_y) CN_CUDA(cudaStreamWaitEvent(s, b->e_y, 0));
-    const float *y = b->slot_y ? b->slot_y + (size_t)slot * b->batch * b->cols_y : b->dn_y;
+    if (!b->in_slot) CN_CUDA(cudaStreamWaitEvent(s, b->e_y, 0));
+    const float *y = b->in_slot ? b->slot_y + (size_t)(b->swaps % (b->groups * CN_BATCH_SWAPS)) * b->batch * b->cols_y : b->dn_y;
     const int st = cn_transpose_batch(b->xb[buf], b->dc_X, y, b->dc_y, b->next_rows, b->cols_X, b->cols_y, s);
     if (st != CN_OK) return st;
     // everything queued on the compute stream so far - the transposes above and the caller's work on the batch that was
     // current until now - precedes this event; the next copy waits for it before it overwrites a buffer
-    b->e_consumed = b->read[buf] = b->e_swap[slot];
+    const int in_group = (int)(b->swaps % CN_BATCH_SWAPS);
+    const bool last = b->slot_y && in_group == CN_BATCH_SWAPS - 1;
+    b->e_consumed = b->read[buf] = last ? b->e_group[b->swaps / CN_BATCH_SWAPS % b->groups] : b->e_swap[in_group];
     CN_CUDA(cudaEventRecord(b->e_consumed, s));
     b->swaps += 1;
+    if (last) b->group_free = false;   // the next group's turn
     b->cur_rows = b->next_rows;
     if (b->flags & CN_BATCH_KEEP_ROW_MAJOR) b->cur_rm = b->xb[buf];   // stays valid until the next swap
     b->ready = (buf + 1) % b->nb;

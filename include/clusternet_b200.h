@@ -487,7 +487,8 @@ int64_t cn_batch_total_batches(const cn_batch *b);
 int cn_batch_current(const cn_batch *b, float **d_X, float **d_y, int64_t *batch_rows);
 /* BatchAllocator::SKIP_LAST_BATCH is a public field that callers flip after init (source/batchAllocator.h:37). */
 int cn_batch_set_skip_last(cn_batch *b, int skip_last_batch);
-/* Stage + asynchronous copy of the next batch (allocate_next_batch_async). */
+/* Stage + asynchronous copy of the next batch (allocate_next_batch_async).  With X and y in pinned memory nothing waits on the host;
+ * otherwise the call waits until the staging memory has been read. */
 int cn_batch_copy_next_async(cn_batch *b);
 /* Make the next batch current (replace_current_batch_with_next): waits (on the device, through an
  * event) for the copies and for the swap before, on whatever stream that was, transposes into the

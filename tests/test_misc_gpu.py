@@ -297,6 +297,32 @@ def test_swaps_on_two_streams_keep_their_order(ctx, flags, B, cols, cols_y):
             assert b.is_batch(i + 1, *b.current())
 
 
+@pytest.mark.parametrize("flags", [0, _lib.BATCH_LOOKAHEAD | _lib.BATCH_NO_COL_MAJOR])
+@pytest.mark.parametrize("B,cols,cols_y", [(32, 40, 1), (32, 40, 128)])
+def test_a_pinned_data_set_never_makes_the_host_wait(ctx, flags, B, cols, cols_y):
+    """Batches queued behind work that is still running when the eightieth is queued, 16 KB of labels each (sixty-four slots) or fewer; then
+    more, with the GPU idle, so that labels come from slots again, until these have come round (256 of them)."""
+    s, steps = torch.cuda.Stream(), 340
+    with Batches(ctx, B, cols, cols_y, 50, flags) as b, torch.cuda.stream(s):
+        keep_X, keep_y = torch.empty((steps, cols, B), device="cuda"), torch.empty((steps, cols_y, B), device="cuda")
+        torch.cuda.synchronize()
+        torch.cuda._sleep(2_000_000_000)
+        held = torch.cuda.Event()
+        held.record()
+        for i in range(steps):
+            if i == 80:
+                assert not held.query()
+                torch.cuda.synchronize()
+            b.next(s)
+            X, y = b.current()
+            if X is not None:
+                keep_X[i].copy_(X)
+            keep_y[i].copy_(y)
+        torch.cuda.synchronize()
+        for i in range(steps):
+            assert b.is_batch((i + 1) % 50, keep_X[i] if b.px.value else None, keep_y[i])
+
+
 def test_batch_size_larger_than_data_is_rejected(ctx):
     x = torch.zeros(10, 4)
     h = ctypes.c_void_p()
