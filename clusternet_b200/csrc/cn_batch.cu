@@ -30,7 +30,6 @@
 #define CN_BATCH_GROUPS 16                 // of such slots, at most: as many as have room in
 #define CN_BATCH_RING_BYTES (1 << 20)
 #define CN_BATCH_SMALL_BYTES (4 << 20)
-#define CN_BATCH_SLOT_BYTES (16 << 10)
 
 struct cn_batch {
     cn_context *ctx = nullptr;

@@ -14,6 +14,7 @@
 #define CN_CODE_MAX_CTAS 256
 #define CN_CODE_COPIES 8
 #define CN_CODE_WORDS_BYTES 8192
+#define CN_BATCH_SLOT_BYTES (16 << 10)   // labels of a batch that are read from pinned memory, at most
 
 void cn_set_error(const char *fmt, ...);
 // every kernel launch of the library is counted (cn_kernel_launches), so that callers can tell library work from fallbacks

@@ -6,6 +6,7 @@
 
 #define TP_TILE 32
 #define TP_ROWS 8
+#define TP_FEW_COLS 16
 
 __device__ __forceinline__ void transpose_tile(const float *in, int64_t ldi, float *out, int64_t ldo, int64_t R, int64_t C, int64_t tiles_c, int64_t tile_id)
 {
@@ -36,15 +37,18 @@ cn_transpose_kernel(const float *in, int64_t ldi, float *out, int64_t ldo, int64
     transpose_tile(in, ldi, out, ldo, R, C, tiles_c, blockIdx.x);
 }
 
-// A batch and its labels (R rows of CY, which may lie in pinned host memory) in one launch: the first CTAs take the labels, a few of the
-// rows' elements per thread in the order they lie in, since what bounds them is the trip over PCIe, beside which the batch is transposed.
+// A batch and its labels (R rows of CY) in one launch, the labels by the first CTAs.  Few labels may lie in pinned host memory: single elements in
+// the order they lie in, since what bounds them is the trip over PCIe, beside which the batch is transposed (128 x 30: 8.2 us for the whole swap, 12.3 by
+// tiles).  The same for up to 16 columns of labels in device memory, whose stores still lie together (65536 x 4 11.1 us, 13.2 by tiles; x 16 13.1 and 14.3; x 32
+// 21.4 and 14.2); wider labels by tiles as the batch is (512 x 2000 8.1, by single elements and 64 CTAs 36.8).
 __global__ void __launch_bounds__(TP_TILE *TP_ROWS)
-cn_transpose_batch_kernel(const float *X, float *outX, const float *y, float *outy, int64_t R, int64_t C, int64_t CY, int64_t tiles_c, int y_ctas)
+cn_transpose_batch_kernel(const float *X, float *outX, const float *y, float *outy, int64_t R, int64_t C, int64_t CY, int64_t tiles_c, int64_t y_tiles_c, int y_ctas)
 {
     cn_pdl_launch_dependents();
     cn_pdl_wait();
-    if ((int)blockIdx.x >= y_ctas) {
-        transpose_tile(X, C, outX, R, R, C, tiles_c, (int64_t)blockIdx.x - y_ctas);
+    const bool labels = (int)blockIdx.x < y_ctas;
+    if (!labels || y_tiles_c > 0) {
+        transpose_tile(labels ? y : X, labels ? CY : C, labels ? outy : outX, R, R, labels ? CY : C, labels ? y_tiles_c : tiles_c, (int64_t)blockIdx.x - (labels ? 0 : y_ctas));
         return;
     }
     for (int64_t i = (int64_t)blockIdx.x * (TP_TILE * TP_ROWS) + threadIdx.x; i < R * CY; i += (int64_t)y_ctas * (TP_TILE * TP_ROWS)) {
@@ -75,10 +79,11 @@ int cn_transpose_pitched(const float *in, int64_t ldi, float *out, int64_t ldo, 
 int cn_transpose_batch(const float *X, float *outX, const float *y, float *outy, int64_t R, int64_t C, int64_t CY, cudaStream_t s)
 {
     const int64_t tiles_c = (C + TP_TILE - 1) / TP_TILE, tiles = outX ? (R + TP_TILE - 1) / TP_TILE * tiles_c : 0;
-    const int64_t want = (R * CY + TP_TILE * TP_ROWS - 1) / (TP_TILE * TP_ROWS), y_ctas = want < 64 ? want : 64;
+    const int64_t y_tiles_c = CY > TP_FEW_COLS && R * CY * (int64_t)sizeof(float) > CN_BATCH_SLOT_BYTES ? (CY + TP_TILE - 1) / TP_TILE : 0;
+    const int64_t want = (R * CY + TP_TILE * TP_ROWS - 1) / (TP_TILE * TP_ROWS), y_ctas = y_tiles_c > 0 ? (R + TP_TILE - 1) / TP_TILE * y_tiles_c : want < 592 ? want : 592;
     CN_REQUIRE(tiles + y_ctas < (1LL << 31), CN_ERR_UNSUPPORTED, "transpose: %lld tiles exceed the grid limit", (long long)tiles);
     if (tiles + y_ctas == 0) return CN_OK;
-    CN_CUDA(cn_launch_pdl(cn_transpose_batch_kernel, dim3((unsigned)(tiles + y_ctas)), TP_TILE * TP_ROWS, 0, s, X, outX, y, outy, R, C, CY, tiles_c, (int)y_ctas));
+    CN_CUDA(cn_launch_pdl(cn_transpose_batch_kernel, dim3((unsigned)(tiles + y_ctas)), TP_TILE * TP_ROWS, 0, s, X, outX, y, outy, R, C, CY, tiles_c, y_tiles_c, (int)y_ctas));
     cn_count_launch();
     return CN_OK;
 }

@@ -323,6 +323,17 @@ def test_a_pinned_data_set_never_makes_the_host_wait(ctx, flags, B, cols, cols_y
             assert b.is_batch((i + 1) % 50, keep_X[i] if b.px.value else None, keep_y[i])
 
 
+@pytest.mark.parametrize("flags", [0, _lib.BATCH_NO_COL_MAJOR])
+@pytest.mark.parametrize("B,cols,cols_y", [(241, 40, 16), (241, 40, 17), (31, 3, 133), (33, 65, 257), (2000, 5, 3), (40000, 2, 5), (1, 9, 5001), (700, 130, 700)])
+def test_batches_with_many_labels(ctx, flags, B, cols, cols_y):
+    """More labels than slots hold, element by element (up to 16 columns, also more than the CTAs take at once) and by tiles, whole and not."""
+    with Batches(ctx, B, cols, cols_y, 3, flags) as b:
+        for i in (1, 2, 0):
+            b.next(torch.cuda.current_stream())
+            torch.cuda.synchronize()
+            assert b.is_batch(i, *b.current())
+
+
 def test_batch_size_larger_than_data_is_rejected(ctx):
     x = torch.zeros(10, 4)
     h = ctypes.c_void_p()
