@@ -719,6 +719,8 @@ struct CodeWords {
     unsigned int launches, tickets[2];                // tickets of launches of odd and even numbers: a launch clears the next one's
 };
 static_assert(sizeof(CodeWords) <= CN_CODE_WORDS_BYTES, "allocation");
+// The last to arrive waits RING_WAIT_LIMIT for the first CTA to have done either: patience stays far below that.
+#define CODE_MAX_PATIENCE (RING_WAIT_LIMIT / 8)
 enum { CODE_LEAVE = 0, CODE_OWN = 1, CODE_FINISH = 2 };   // what a CTA does next: nothing; its own elements; these and those that were left
 
 __device__ __forceinline__ unsigned long long code_load(const unsigned long long *at)
@@ -1622,7 +1624,7 @@ cudaError_t cn_codec_make_table(cn_context *ctx)
 
 extern "C" int cn_codec_set_patience(cn_context *ctx, int64_t clocks)
 {
-    CN_REQUIRE(ctx && clocks >= 0, CN_ERR_ARG, "cn_codec_set_patience: bad argument");
+    CN_REQUIRE(ctx && clocks >= 0 && clocks <= CODE_MAX_PATIENCE, CN_ERR_ARG, "cn_codec_set_patience: bad argument");
     ctx->code_patience = clocks;
     return CN_OK;
 }

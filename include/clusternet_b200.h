@@ -119,11 +119,13 @@ int cn_compress_8bit_dp(cn_context *ctx, const float *d_A, const float *d_precis
  * tensors, for which launch latency no longer matters, take two pipelined launches.
  * d_scale_out (device) receives the scale; the codes equal
  * cn_absmax_f32 + cn_compress_8bit_dp bit for bit.  Uses context scratch: calls on one context must be serialised on
- * one stream. */
+ * one stream.  A CTA that waits two seconds in vain (it cannot unless another that has begun stands still that long) makes
+ * cn_gemm_check_status report CN_ERR_TIMEOUT. */
 int cn_absmax_compress_8bit(cn_context *ctx, const float *d_A, int64_t n, float *d_scale_out, uint8_t *d_codes, void *stream);
 
-/* Test knob of that launch, per context: the clocks for which a CTA waits for the scale before it leaves its elements to the CTA that is
- * last to have its maximum (0: at once).  The results do not depend on it.  No counterpart in the reference. */
+/* Test knob of that launch, per context: the clocks (0 to 500 million; 0: not at all) for which a CTA waits for the scale before it leaves its
+ * elements to the first CTA, which finds the scale, or, where that one has left as well, to the last to have its maximum.  The results do
+ * not depend on it.  No counterpart in the reference. */
 int cn_codec_set_patience(cn_context *ctx, int64_t clocks);
 
 /* decompression_8bit: replaces ::decompression_8bit (source/basicOps.cu:1172-1176) and

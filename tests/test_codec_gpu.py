@@ -8,6 +8,7 @@ import pytest
 import torch
 
 import clusternet_b200 as cn
+from clusternet_b200 import _lib
 from oracle import oracle
 
 pytestmark = pytest.mark.gpu
@@ -165,6 +166,14 @@ def test_scale_and_codes_where_ctas_do_not_wait(ctx, n, off, clocks):
             assert bool((codes[:off] == 77).all()) and bool((codes[off + n:] == 77).all())
     finally:
         cn.check(ctx.lib.cn_codec_set_patience(ctx.h, 400000))
+
+
+def test_patience_is_bounded(ctx):
+    """Far below the two seconds for which the last CTA waits for the first."""
+    for clocks in (-1, 500_000_001, 1 << 40, (1 << 63) - 1):
+        assert ctx.lib.cn_codec_set_patience(ctx.h, clocks) == _lib.CN_ERR_ARG
+    for clocks in (500_000_000, 400000):
+        cn.check(ctx.lib.cn_codec_set_patience(ctx.h, clocks))
 
 
 def test_fused_absmax_compress_replays_from_a_cuda_graph(ctx):
