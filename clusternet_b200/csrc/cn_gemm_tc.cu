@@ -1050,9 +1050,11 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
 // depend on scheduling), applies bias and activation, turns the block through shared memory so that a warp stores 512
 // contiguous bytes of a column, and stores to C and, for the fused all-gather, to every peer's C (full NVLink packets).
 //
-// Tiles that are cut into many runs are bound by how many loads are in flight: 8 columns per CTA, eight partial tiles at a time, from three
-// CTAs per tile on; else 32.  us of the whole product, 32 columns / 8: 203 x 4001 . 4001 x 3001 (six CTAs per tile) 50.5 / 44.7, 500 x 3000 . 3000 x
-// 3000 (three) 59.5 / 56.1; 300 x 6000 . 6000 x 6000 (two) 117.6 / 120.1, 1000 x 4096 . 4096 x 2048 (two pairs) 71 / 73.6.
+// Few tiles, and tiles that are cut into many runs, are bound by how many loads are in flight: 8 columns per CTA, eight partial tiles at a time,
+// where 32 would leave SMs without a CTA, and from three CTAs per tile on; else 32.  us of the whole product, 32 columns / 8: 203 x 4001 . 4001 x 3001
+// (six CTAs per tile) 50.5 / 44.7, 500 x 3000 . 3000 x 3000 (three) 59.5 / 56.1; 2304 x 512 . 512 x 2304 (seven tiles of 256 x 256 by 18 pairs) 43.4 /
+// 40.1, 4850 x 512 . 512 x 1024 (two by five) 48.2 / 44.5; 300 x 6000 . 6000 x 6000 (72 by two CTAs each) 117.6 / 120.1, 1000 x 4096 . 4096 x 2048 (32 by two
+// pairs each) 71 / 73.6.
 template <int COLS>
 __global__ void __launch_bounds__(256)
 cn_splitk_reduce_kernel(const __grid_constant__ ReduceParams p)
@@ -1146,7 +1148,7 @@ cn_splitk_reduce_kernel(const __grid_constant__ ReduceParams p)
 int cn_splitk_reduce_launch(cn_context *ctx, const ReduceParams &rp, cudaStream_t s)
 {
     const int64_t blocks = (int64_t)rp.tail_tiles * rp.nt * rp.mt;
-    if (rp.tail_ctas >= 3LL * rp.tail_tiles) CN_CUDA(cn_launch_pdl(cn_splitk_reduce_kernel<8>, dim3((unsigned)(blocks * (TC_BN / 8))), 256, 0, s, rp));
+    if (rp.tail_ctas >= 3LL * rp.tail_tiles || blocks * 4 <= ctx->sm_count) CN_CUDA(cn_launch_pdl(cn_splitk_reduce_kernel<8>, dim3((unsigned)(blocks * (TC_BN / 8))), 256, 0, s, rp));
     else CN_CUDA(cn_launch_pdl(cn_splitk_reduce_kernel<32>, dim3((unsigned)(blocks * (TC_BN / 32))), 256, 0, s, rp));
     cn_count_launch();
     return CN_OK;
