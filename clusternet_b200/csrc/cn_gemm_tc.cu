@@ -1309,20 +1309,22 @@ size_t cn_tc_cut::partial_bytes() const { return rest() > 0 && cluster == 1 ? (s
 // follows.  A cluster's CTAs exchange the parts through distributed shared memory (20 bytes per clock from a CTA), in one launch less: 15 us
 // and 0.66 per block with one tile of 128 columns per CTA, 20 and 0.74 with two; but K is cut into as many parts as CTAs find room in the GPCs
 // for every tile, not one per SM.  us, runs / clusters: 24 x 560 . 560 x 5192 23.8 / 14.5; 100 x 1500 . 1500 x 2500 30.6 / 19.6; 48 x 1568 . 1568 x 11448 39.4
-// / 28.7; 128 x 3000 . 3000 x 3000 31.1 / 28.1; 128 x 4096 . 4096 x 4096 36.5 / 38.0; 128 x 10000 . 10000 x 1000 39.7 / 40.1, x 100000 131 / 299.  With
-// two tiles of rows a few gain (256 x 4096 . 4096 x 4096 55.5 / 49.7), others lose (150 x 2344 . 2344 x 2208 33 / 38).
+// / 28.7; 128 x 2348 . 2348 x 8289 40.4 / 38.5; 128 x 100000 . 100000 x 1000 131 / 299.  With two tiles of rows a few gain (256 x 4096 . 4096 x 4096 55.5 /
+// 49.7), others lose (150 x 2344 . 2344 x 2208 33 / 38).  The fit is older than the reduction's CTAs of eight columns: of 548 products drawn where
+// this rule takes clusters, which take 0.80 of the runs' time on average, 27 are more than 3 % faster by runs today (104 x 5014 . 5014 x 3526 42.1 /
+// 48.6 the worst of them); a fit with the rows in it gained nothing over drawn products.
 //
 // Runs are short, and so are their accumulation chains; clusters' chains are cut as short, so that no product is less exact: relative to fp64,
 // runs of 28 blocks 1.6e-6, of 14 1.3e-6, of 6 7e-7; chains of 8 blocks 9.8e-7, of 4 5.4e-7.  That costs long runs more than the launch
-// (152 x 9384 . 9384 x 3152 85 / 103): at most 24 blocks.
+// (25 blocks per CTA, 128 x 6400 . 6400 x 448 23.2 / 30.0; 32, 128 x 4064 . 4064 x 6702 47.6 / 51.1): at most 24 blocks.
 static void tc_share_tiles(const cn_context *ctx, int64_t N, cn_tc_cut *cut)
 {
-    if (cut->rest() == 0 || cut->tiles_m > 1) return;
+    if (cut->rest() == 0 || cut->full > 0 || cut->tiles_m > 1) return;   // with whole tiles besides, no two CTAs per tile find room
     const double run = (double)cut->rest() * cut->kb_total / cut->tail_ctas;
-    const double runs = 17.0 + 8.0 * (double)cut->tail_ctas / ctx->sm_count + 0.9 * (cut->full > 0 ? (double)cut->tiles * cut->kb_total / ctx->sm_count : run);
+    const double runs = 17.0 + 8.0 * (double)cut->tail_ctas / ctx->sm_count + 0.9 * run;
     double best = 0.95 * runs;
     for (int nt = 1; nt <= (N > TC_BN ? 2 : 1); ++nt) {
-        const int64_t tiles = (N + nt * TC_BN - 1) / (nt * TC_BN) * cut->tiles_m;
+        const int64_t tiles = (N + nt * TC_BN - 1) / (nt * TC_BN);
         for (int c = 2; c <= CN_TC_MAX_CLUSTER && cut->kb_total >= 2 * c; ++c) {
             const int per = (TC_BM / 16 + c - 1) / c;
             // room for the parts in the rings' shared memory
@@ -1335,8 +1337,7 @@ static void tc_share_tiles(const cn_context *ctx, int64_t N, cn_tc_cut *cut)
         }
     }
     if (cut->cluster == 1) return;
-    cut->tiles = (N + cut->nt * TC_BN - 1) / (cut->nt * TC_BN) * cut->tiles_m;
-    cut->full = 0;
+    cut->tiles = (N + cut->nt * TC_BN - 1) / (cut->nt * TC_BN);
     cut->tail_ctas = cut->tiles * cut->cluster;
     cut->max_chain = run >= 12.0 ? 8 : run >= 6.0 ? 4 : 2;
 }
