@@ -187,7 +187,7 @@ extern "C" int cn_batch_create_ex(cn_context *ctx, const float *h_X, const float
     }
     // A copy of a few labels is three calls (wait, copy, event) and the swap's wait for it, more than the kernel that turns the batch takes
     // to read them over PCIe, now that the next copy does not wait for that kernel.  Larger ones stay with the copy engine.  128 x 784 images with
-    // a label each, us per batch: 19.1; with the second buffer, one kernel for both and the labels in slots 15.1 (with one buffer 23).
+    // a label each, us per batch: 18.5; with the second buffer, one kernel for both and the labels in slots 13.8 (with one buffer 23).
     const bool few = by <= CN_BATCH_SLOT_BYTES;
     // With up to 4 KB of labels per batch the host may be 240 batches ahead before labels take the copy engine, with 16 KB 48.  (With a hundred
     // batches queued in a row and only sixteen slots, 128 x 784 images took 16 to 25 us; with the host waiting for a slot, 13.3 to 15.4.)

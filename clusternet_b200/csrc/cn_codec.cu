@@ -1140,7 +1140,7 @@ cn_decompress_kernel(const uint8_t *codes, float precision_arg, const float *d_p
     const int64_t nvec = vector_ok ? (n >> 2) : 0;
     int64_t v = (int64_t)blockIdx.x * blockDim.x + tid;
     const uint32_t *in4 = reinterpret_cast<const uint32_t *>(codes);
-    // the first codes are on their way while the table is made
+    // the first codes are on their way while the table of a scale on the device is made (behind a host scale, whose table is there, this gains nothing)
     uint32_t cur[4];
     const bool whole = v + 3 * stride < nvec;
     if (whole) {

@@ -20,9 +20,10 @@
 // unwritten.  Lists that overflow, against the streaming kernel alone, us: 520 x 40000 . 40000 x 256 154 / 123 (1296 with whole tiles), 640 x
 // 100000 . 100000 x 256 309 / 275 (3148); with whole tiles 520 x 4096 . 4096 x 4096 204 / 132, 1024 rows 212 / 183, 4096^3 650 / 584.
 //
-// Bound by the tensor cores (their pipe is busy in 80 % of the cycles at 2048 x 4096 . 4096 x 4096): 4096^3, 3x mode, 245 us of the product's 340 at 1.68 PFLOP/s of fp16, against 476 us on the streaming
-// kernel (2048 rows 187 / 263, 1024 rows 120 / 142; single pass 184 / 392); the pre-pass moves 256 MB in 60 us, the reduction of the cut
-// tail takes 13, the launch that ends at once 3.  Short K is bound by the drain warps and the stores: 4096 x 128 . 128 x 4096 44 us with 32-byte
+// Bound by the tensor cores (their pipe is busy in 80 % of the cycles at 2048 x 4096 . 4096 x 4096): 4096^3, 3x mode, 336 us from an idle GPU, against 476 us on the streaming
+// kernel (2048 rows 187 / 263, 1024 rows 120 / 142; single pass 184 / 392): 52 for the pre-pass, which moves 256 MB, 274 for this kernel (1.50 PFLOP/s of
+// fp16), 8 for the reduction of the cut tail, 2 for the launch that ends at once.  In a series of seconds the power cap takes the clock to 1.4 GHz, and
+// they take 51, 340, 10 and 6: 407.  Short K is bound by the drain warps and the stores: 4096 x 128 . 128 x 4096 44 us with 32-byte
 // stores from registers, 39 by TMA (see the epilogue); 1320 x 144 . 144 x 1872 with ReLU 27 -> 23.
 #include <cuda.h>
 #include <cuda_fp16.h>

@@ -152,14 +152,16 @@ def test_scale_and_codes_in_one_launch_of_extreme_tensors(ctx, n, value):
 @pytest.mark.parametrize("n,off", [(32770, 0), (65539, 3), (148 * 2048 + 1, 1), (942785, 2), (148 * 512 * 32 + 5, 0), (4 << 20, 1)])
 @pytest.mark.parametrize("clocks", [0, 3000])
 def test_scale_and_codes_where_ctas_do_not_wait(ctx, n, off, clocks):
-    """CTAs that leave their elements to the last one (all others, or those that come first), the first CTA and its elements outside the
-    quads among them: the same scale and codes, call after call, nothing written beside them."""
+    """CTAs that leave their elements to the first one, or to the last to arrive where the first has left (all others, or those that come first),
+    the first CTA and its elements outside the quads among them: the same scale and codes, call after call, nothing written beside them, and no
+    wait that ran out."""
     try:
         cn.check(ctx.lib.cn_codec_set_patience(ctx.h, clocks))
         for rep in range(4):
             x = (torch.randn(n + 8, device="cuda") * 10.0 ** -rep)[off:off + n]   # a scale of the call before would be too large
             codes, scale = torch.full((n + 8,), 77, dtype=torch.uint8, device="cuda"), torch.empty(1, device="cuda")
             ctx.absmax_compress(x, scale=scale, out=codes[off:off + n])
+            ctx.gemm_check()
             assert scale.item() == x.abs().max().item()
             want = oracle.compress(ctx.codebook, x.cpu().numpy(), scale.item())
             assert np.array_equal(codes[off:off + n].cpu().numpy(), want)
@@ -177,9 +179,9 @@ def test_patience_is_bounded(ctx):
 
 
 def test_fused_absmax_compress_replays_from_a_cuda_graph(ctx):
-    """The one-launch form keeps its grid barrier's state on the device only, so a recorded launch can be replayed: every
-    replay must wait for ITS maxima.  The data shrink from replay to replay - a barrier that let a CTA through early would
-    fold a stale, larger maximum of the replay before into the scale."""
+    """The one-launch form keeps the launch's number on the device only, so a recorded launch can be replayed: every replay must
+    wait for ITS maxima.  The data shrink from replay to replay - a number that did not advance would hand out the larger maxima
+    of the replay before."""
     n = 1_000_003 + 1                                     # the one-launch form (at most 4 Mi elements), with a ragged end
     rng = np.random.default_rng(99)
     base = torch.from_numpy((rng.standard_normal(n) * 5).astype(np.float32)).cuda()
@@ -196,6 +198,7 @@ def test_fused_absmax_compress_replays_from_a_cuda_graph(ctx):
         a.copy_(base * f)
         g.replay()
         torch.cuda.synchronize()
+        ctx.gemm_check()
         pm = ctx.absmax(a)
         want = ctx.compress(a, pm)
         torch.cuda.synchronize()
@@ -344,3 +347,18 @@ def test_scale_and_codes_from_the_end_of_a_tensor(ctx, n):
     assert scale.item() == 9.0
     assert torch.equal(codes[:n], ctx.compress(x, 9.0)) and bool((codes[n:] == 77).all())
     assert np.array_equal(codes[n - 100000:n].cpu().numpy(), oracle.compress(ctx.codebook, x[n - 100000:].cpu().numpy(), 9.0))
+
+
+@pytest.mark.parametrize("n", [(16 << 20) - 3, (16 << 20) + 1, 20_000_001])
+@pytest.mark.parametrize("xo,co", [(1, 0), (0, 1), (3, 3)])
+def test_scale_and_codes_of_large_tensors_off_16_bytes(ctx, n, xo, co):
+    """Beyond what one launch takes, tensor or codes not aligned: the kernels that need no alignment, in the usual order."""
+    x = torch.randn(n + 8, device="cuda")[xo:xo + n]
+    x[-1], x[0], x[n // 2] = 9.0, -8.5, float("nan")
+    codes, scale = torch.full((n + 64,), 77, dtype=torch.uint8, device="cuda"), torch.empty(1, device="cuda")
+    ctx.absmax_compress(x, scale=scale, out=codes[co:co + n])
+    ctx.gemm_check()
+    assert scale.item() == 9.0
+    assert torch.equal(codes[co:co + n], ctx.compress(x, 9.0)) and bool((codes[:co] == 77).all()) and bool((codes[co + n:] == 77).all())
+    for at in (slice(0, 50000), slice(n - 50000, n)):
+        assert np.array_equal(codes[co:co + n][at].cpu().numpy(), oracle.compress(ctx.codebook, x[at].cpu().numpy(), 9.0))
