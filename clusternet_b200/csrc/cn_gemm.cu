@@ -222,10 +222,13 @@ int cn_gemm_dispatch(cn_context *ctx, int transA, int transB, int64_t M, int64_t
     // (520 x 784 . 784 x 1200: 38 us against 30 on the streaming kernel; 520 x 2000 . 2000 x 1000: 41 against 43).
     const bool plain = mode != CN_GEMM_FP32_SIMT && !tuned && !(ws && ws->coded_src);
     const bool fine = plain && cn_gemm_small_shape(ctx, M, N, K, tma_ok, 2);
-    const bool planes = planes_ok && plain && L == 1 && !pr && !(peers && peers->npeers > 0) && cn_gemm_planes_shape(ctx, M, N, K, tc_mode, tma_ok, fine) &&
-                        (fine || K >= (1LL << 30) / (M * N));
-    const bool small = plain && (L == 1 || ldc == M) && (!pr || pr->raw) && fine && (!planes || cn_gemm_small_shape(ctx, M, N, K, tma_ok, 1)) &&
-                       (tma_ok || M * N * K >= 4096);
+    const bool own = planes_ok && plain && L == 1 && !pr && !(peers && peers->npeers > 0);
+    const bool one_round = fine && cn_gemm_small_shape(ctx, M, N, K, tma_ok, 1);
+    // A weight gradient that takes more than one round of the small products' kernel, and has a short inner dimension, takes one launch as well.
+    const bool gradient = transA && !transB && !bias && act == CN_ACT_LINEAR && tc_mode == CN_GEMM_3XTF32;
+    const bool outer = own && gradient && !one_round && cn_gemm_outer_shape(M, N, K) && M * N * K >= 4096;
+    const bool planes = own && !outer && cn_gemm_planes_shape(ctx, M, N, K, tc_mode, tma_ok, fine) && (fine || K >= (1LL << 30) / (M * N));
+    const bool small = plain && !outer && (L == 1 || ldc == M) && (!pr || pr->raw) && fine && (!planes || one_round) && (tma_ok || M * N * K >= 4096);
     const bool tc_ok = tma_ok || (mode != CN_GEMM_FP32_SIMT && M * N * K >= 4096 && cn_gemm_tc_any_supported(transB, M, N, K, d_B));
     // a small product and its maxout are two launches as well, and the maxima are those of the very product a call without maxout gives
     // (with up to 512 rows; from there on that call may take the kernel for many rows, whose last bits differ)
@@ -246,7 +249,12 @@ int cn_gemm_dispatch(cn_context *ctx, int transA, int transB, int64_t M, int64_t
         if (stop && r == CN_OK) CN_CUDA(cudaEventRecord(stop, s));
         return r;
     };
-    if (small) {
+    if (outer) {
+        cudaEvent_t stop = nullptr;
+        st = cn_gemm_profile_start(ctx, s, &stop);
+        if (st == CN_OK) st = cn_gemm_outer_launch(ctx, M, N, K, d_A, lda, d_B, ldb, target, target_ld, s, fine);
+        if (stop && st == CN_OK) CN_CUDA(cudaEventRecord(stop, s));
+    } else if (small) {
         if (pr) {
             ws->prepared = nullptr;
             CN_REQUIRE(pr->filled && pr->M == M && pr->K == K && pr->mode == mode, CN_ERR_SHAPE,

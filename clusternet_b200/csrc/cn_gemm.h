@@ -116,6 +116,11 @@ bool cn_gemm_small_shape(const cn_context *ctx, int64_t M, int64_t N, int64_t K,
 int cn_gemm_any_chain(int64_t K);
 int cn_gemm_small_launch(cn_context *ctx, int transA, int transB, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, const float *B, int64_t ldb,
                          float *C, int64_t ldc, const cn_epilogue *epi, int mode, cudaStream_t s, const cn_peer_out *peers);
+// Weight gradients with a short inner dimension in one launch (cn_gemm_outer.cu): A (K x M) transposed, B (K x N), any alignment.  `fine`: the shape
+// is one for the small products' kernel, whose error must not be exceeded.
+bool cn_gemm_outer_shape(int64_t M, int64_t N, int64_t K);
+int cn_gemm_outer_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const float *A, int64_t lda, const float *B, int64_t ldb, float *C, int64_t ldc,
+                         cudaStream_t s, bool fine);
 // cn_gemm_f32 with optional peer windows; *used_peers tells whether the launch took them (tensor-core path only).  planes_ok: the
 // kernel for many rows may be taken.  The products with a column-sharded weight (cn_dotmpi_f32 and its forms) do not take it: their bits may
 // not depend on whether the activations' planes were made ahead, the activations are codes, or the output goes to peers, and those

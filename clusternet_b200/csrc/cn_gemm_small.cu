@@ -34,10 +34,8 @@
 #include <limits.h>
 #include "cn_epilogue.cuh"
 #include "cn_gemm.h"
-#include "cn_tc.cuh"
+#include "cn_tc_feed.cuh"
 
-#define SM_BM 128
-#define SM_BK 32
 #define SM_FEED 256             // threads that load and split an operand: warps 0-7 the activations, 8-15 the weights; all of them the epilogue
 #define SM_EPI (2 * SM_FEED)
 #define SM_THREADS (SM_EPI + 32)   // warp 16: MMA issuer
@@ -63,13 +61,6 @@ struct SmCfg {
     static_assert(SMEM_MAX <= 232448 - 1024, "shared memory");
 };
 
-// An operand: element (row, k) at p[row * sr + k * sk].
-struct SmOperand {
-    const float *p;
-    int64_t sr, sk;
-    int vec;                // 16-byte aligned along the contiguous one of the two
-};
-
 struct SmallParams {
     SmOperand A, W;
     int64_t M, N, K;
@@ -89,39 +80,6 @@ struct SmallParams {
     int nranks, my_rank;
     unsigned int epoch;
 };
-
-// fp32 -> TF32, round to nearest with ties away from zero: add half a TF32 ulp to the magnitude bits and truncate.  That carry takes
-// the finite values from 0x7f7ff000 up to infinity and a NaN with a full mantissa (0x7fffffff, the one GPU arithmetic makes)
-// over into the sign bit, to -0.  CAREFUL truncates those instead, NaNs after an addition that makes them the canonical one.
-template <bool CAREFUL>
-__device__ __forceinline__ uint32_t sm_tf32(float x)
-{
-    if (!CAREFUL) return (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-    const float top = __uint_as_float(0x7f7ff000u);
-    return (fabsf(x) < top ? __float_as_uint(x) + 0x1000u : __float_as_uint(__fadd_rn(x, 0.0f))) & 0xffffe000u;
-}
-
-__device__ __forceinline__ void sts4u(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w)
-{
-    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
-}
-
-__device__ __forceinline__ void sts4f(uint32_t a, const float *v)
-{
-    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
-}
-
-// D[tmem] (+)= A[smem] * B[smem], both K-major TF32 tiles.
-__device__ __forceinline__ void sm_mma_ss(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc, uint32_t accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b64 ad, bd;\n\t"
-        "setp.ne.b32 p, %5, 0;\n\t"
-        "mov.b64 ad, {%1, %3};\n\t"
-        "mov.b64 bd, {%2, %3};\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], ad, bd, %4, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate) : "memory");
-}
 
 // The share of one thread of a block of ROWS x 32 k: up to four 16-byte chunks (a chunk is four consecutive k of a row).
 // QUADS false: chunks of rows 32 apart; with k contiguous, eight lanes read a row's 128 bytes, 16 at a time where the rows are aligned;
@@ -669,16 +627,8 @@ int cn_gemm_small_launch(cn_context *ctx, int transA, int transB, int64_t M, int
     unsigned int *d_status = nullptr;
     int st = cn_status_block(ctx, &d_status);
     if (st != CN_OK) return st;
-    auto operand = [](const float *q, bool k_contiguous, int64_t ld) {
-        SmOperand o;
-        o.p = q;
-        o.sr = k_contiguous ? ld : 1;
-        o.sk = k_contiguous ? 1 : ld;
-        o.vec = (ld & 3) == 0 && ((uintptr_t)q & 15u) == 0;
-        return o;
-    };
-    p.A = operand(A, transA != 0, lda);
-    p.W = operand(B, transB == 0, ldb);
+    p.A = sm_operand(A, transA != 0, lda);
+    p.W = sm_operand(B, transB == 0, ldb);
     p.M = M; p.N = N; p.K = K;
     p.C = C; p.ldc = ldc;
     p.bias = epi ? epi->bias : nullptr;

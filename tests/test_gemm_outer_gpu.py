@@ -1,0 +1,93 @@
+"""Weight gradients of few rows (act^T . err with up to 128 k) in one launch: edges of strips, blocks of columns and blocks of k, strips that
+change in the middle of a CTA's work, any pitch and alignment.
+
+Bound per element, of sum |a_k b_k|: TF32 parts leave 2^-22 of an element, the products of two low parts are left out (2^-22), and every product has
+at most 32 additions truncated to 2^-23 (hi) or of the small sums (lo): 4.3e-6 + 4e-6, well inside the streaming kernel's 2.5e-5."""
+import numpy as np
+import pytest
+import torch
+
+from clusternet_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+REL = 2.5e-5
+
+
+def place(x, off):
+    """torch (cols x rows: column-major rows x cols), its base `off` floats past a 16-byte boundary, between NaNs."""
+    buf = torch.full((x.numel() + 64,), float("nan"), device="cuda")
+    t = buf[32 + off:32 + off + x.numel()].view(x.shape)
+    t.copy_(x)
+    return t
+
+
+# k: seventeen, a block of 32 k less one, whole ones, odd ones, all four; rows: eight, a strip and one more; columns: of one unit, of 16 units and one more;
+# 4884 x 2576: 39 strips shared by all CTAs, some of whose strips end after one block; 9000 rows: 71 strips
+SHAPES = [(8, 17, 150000), (129, 31, 33000), (2000, 32, 1700), (2001, 33, 1601), (1540, 64, 3500), (1000, 65, 4001), (1600, 96, 2000), (1537, 97, 2050), (2000, 128, 2000), (2049, 127, 1999),
+          (4096, 128, 4096), (4884, 64, 2576), (4884, 127, 2577), (9000, 100, 520), (20000, 128, 17), (300, 128, 9001)]
+
+
+@pytest.mark.parametrize("M,K,N", SHAPES)
+@pytest.mark.parametrize("off", [(0, 0, 0), (1, 0, 1), (0, 3, 2)])
+def test_weight_gradients_of_few_rows(ctx, M, K, N, off):
+    g = torch.Generator(device="cuda").manual_seed(M + K + N)
+    act, err = torch.randn(M, K, device="cuda", generator=g).clamp_(min=0), torch.randn(N, K, device="cuda", generator=g)
+    err *= torch.exp(3 * torch.randn(N, K, device="cuda", generator=g))   # of very different size within a column
+    buf = torch.full((N * M + 64,), 7.0, device="cuda")
+    C = buf[32 + off[2]:32 + off[2] + N * M].view(N, M)
+    a, w = place(act, off[0]), place(err, off[1])
+    n0 = ctx.lib.cn_kernel_launches()
+    ctx.gemm(a, w, out=C, transA=True)
+    assert ctx.lib.cn_kernel_launches() - n0 == 1
+    ctx.gemm_check()
+    assert ctx.gemm_last_kernel() == "outer"
+    assert bool((buf[:32 + off[2]] == 7.0).all()) and bool((buf[32 + off[2] + N * M:] == 7.0).all())   # nothing beside C
+    ref, mag = err.double() @ act.double().t(), err.double().abs() @ act.double().t()
+    assert bool(((C.double() - ref).abs() <= REL * mag).all())
+    first = C.clone()
+    ctx.gemm(a, w, out=C, transA=True)
+    assert torch.equal(first, C)   # bit for bit the same again
+
+
+@pytest.mark.parametrize("off", [0, 1])
+def test_non_finite_and_the_largest_finite_values_stay_in_their_row_and_column(ctx, off):
+    """NaNs of any bit pattern and infinities of either operand; a value that rounds past the largest TF32 number stays finite."""
+    rng = np.random.default_rng(3)
+    M, K, N = 2500, 100, 1300
+    a, b = rng.standard_normal((M, K)).astype(np.float32), rng.standard_normal((N, K)).astype(np.float32)
+    a[1000] = 0.0
+    a[1000, 3], b[:, 3] = np.frombuffer(np.uint32(0x7f7fffff).tobytes(), np.float32)[0], 0.25
+    for i, v in enumerate((0x7fffffff, 0xffffffff, 0x7fc00000, 0x7f800000)):
+        a.view(np.uint32)[7 + i, 20 * i] = v
+        b.view(np.uint32)[60 * i + 1, 11 + i] = v
+    C = ctx.gemm(place(torch.from_numpy(a), off), place(torch.from_numpy(b), off), transA=True).cpu().numpy()
+    ctx.gemm_check()
+    assert ctx.gemm_last_kernel() == "outer"
+    finite = np.isfinite(C)
+    rows, cols = [1 + 60 * i for i in range(4)], [7 + i for i in range(4)]
+    assert not finite[rows].any() and not finite[:, cols].any()
+    rest = np.ones((N, M), bool)
+    rest[rows], rest[:, cols] = False, False
+    assert finite[rest].all()
+    ok = [i for i in range(N) if i not in rows]
+    assert np.abs(C[ok, 1000] / (np.float64(a[1000, 3]) * 0.25) - 1.0).max() <= REL
+
+
+# what stays with the kernels it had: a bias, a unit, the single pass, other layouts, a longer K, one round of small products, few rows, a K of one addition
+@pytest.mark.parametrize("M,K,N,kw", [(2000, 128, 2000, dict(bias=True)), (2000, 128, 2000, dict(activation=_lib.ACT_RELU)), (2000, 128, 2000, dict(mode=_lib.GEMM_TF32)),
+                                      (2000, 128, 2000, dict(transA=False)), (2000, 128, 2000, dict(transB=True)), (2000, 129, 2000, {}), (784, 128, 1200, {}), (7, 128, 150000, {}), (4000, 16, 2000, {})])
+def test_what_is_no_such_weight_gradient(ctx, M, K, N, kw):
+    g = torch.Generator(device="cuda").manual_seed(1)
+    kw = dict(transA=True, transB=False, **{k: v for k, v in kw.items() if k not in ("transA", "transB")}) | {k: v for k, v in kw.items() if k in ("transA", "transB")}
+    if kw.pop("bias", False):
+        kw["bias"] = torch.randn(N, device="cuda", generator=g)
+    A, W = torch.randn((M, K) if kw["transA"] else (K, M), device="cuda", generator=g), torch.randn((K, N) if kw["transB"] else (N, K), device="cuda", generator=g)
+    C = ctx.gemm(A, W, **kw)
+    ctx.gemm_check()
+    assert ctx.gemm_last_kernel() != "outer"
+    ref = (W.double().t() if kw["transB"] else W.double()) @ (A.double().t() if kw["transA"] else A.double())
+    if "bias" in kw:
+        ref += kw["bias"].double()[:, None]
+    if "activation" in kw:
+        ref = ref.clamp(min=0)
+    assert float((C.double() - ref).norm() / ref.norm()) <= (1e-3 if kw.get("mode") else 1e-6)
