@@ -101,6 +101,17 @@ __device__ __forceinline__ bool act_store8(const ActPlanes &pl, int band, int64_
     return (low >> 16) < tc_safe_f16<LO>() || (low & 0xffffu) < tc_safe_f16<LO>();
 }
 
+// Where act_store8 finds a small high part: whether it may be more than a zero's.  The smallest nonzero magnitude tells.  Half of the elements behind a
+// rectifier, or behind dropout, are zeros, which leave nothing, but sent nearly every CTA through its block once more (a quarter of the pass over a batch's errors).
+template <bool LO>
+__device__ __forceinline__ bool act_small8(const float (&x)[8], float sc)
+{
+    uint32_t amin = 0xffffffffu;   // of 2 |bits| - 1, in which a zero is the largest
+#pragma unroll
+    for (int e = 0; e < 8; ++e) amin = min(amin, __float_as_uint(x[e]) * 2u - 1u);
+    return amin != 0xffffffffu && __uint_as_float((amin + 1u) >> 1) * sc < (LO ? 0.03125f : 6.103515625e-5f);
+}
+
 // The cell of a CTA's 16 rows x 512 k: the elements that band 0 leaves something of, in the order of their keys (row << 16 | k), if
 // they are few.  begin, add by any threads, end, with barriers between.
 struct ActCell {
@@ -253,7 +264,7 @@ __device__ __forceinline__ void act_rows(const float *A, int64_t lda, int64_t M,
                 float x[8];
 #pragma unroll
                 for (int e = 0; e < 8; ++e) x[e] = tile[act_at(kk + e, ml)];
-                maybe |= act_store8<LO>(pl, band, m * Kp + k, x, s_sc[ml]) && s_finite[ml];
+                maybe |= act_store8<LO>(pl, band, m * Kp + k, x, s_sc[ml]) && s_finite[ml] && act_small8<LO>(x, s_sc[ml]);
             }
         }
         // zeros, or elements too small for the scale: what is left takes the elements' place
@@ -370,7 +381,7 @@ __device__ __forceinline__ void act_rows_t(const float *A, int64_t lda, int64_t 
             for (int j = 0; j < 2; ++j) {
                 const int kk = 256 * j + 8 * lane;
                 if (m < M && k0 + kk < pl.Kp && (band == 0 || s_left[band - 1][kk / TC_WK] != 0u))
-                    maybe |= act_store8<LO>(pl, band, m * pl.Kp + k0 + kk, x[r][j], sc[r]) && finite[r];
+                    maybe |= act_store8<LO>(pl, band, m * pl.Kp + k0 + kk, x[r][j], sc[r]) && finite[r] && act_small8<LO>(x[r][j], sc[r]);
             }
         }
         bool left = false;
