@@ -337,7 +337,7 @@ cn_gemm_small_kernel(const __grid_constant__ SmallParams p)
         feed.begin(kb0, n_blocks, p.K);
         ok = feed.run(kb0, n_blocks, p.K, ring, Cfg::STAGE_BYTES, 2 * SM_A_TILE, 2 * SM_A_TILE + Cfg::W_TILE, full0, empty0, abort_flag, p.status);
     }
-    if (warp == 16 && lane == 0) {
+    if (warp == 16) {   // the whole warp waits, which takes half as long as by one lane; one issues
         // kind::tf32 instruction descriptor: D fp32, A and B TF32 (format 2), K-major, N >> 3 at bits 17-22, M >> 4 at bits 24-28
         const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(SM_BM >> 4) << 24);
         const uint32_t idesc2 = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(Cfg::ACC_COLS >> 3) << 17) | ((uint32_t)(SM_BM >> 4) << 24);
@@ -352,15 +352,18 @@ cn_gemm_small_kernel(const __grid_constant__ SmallParams p)
             const uint32_t hi = (uint32_t)(d >> 32), ahi = (uint32_t)d, alo = ahi + (SM_A_TILE >> 4), w = alo + (SM_A_TILE >> 4);
             if (in_chain == per_chain) { in_chain = 0; acc += Cfg::ACC_COLS; }
             const bool first = in_chain++ == 0;
+            if (lane == 0) {
 #pragma unroll
-            for (int j = 0; j < SM_BK / 8; ++j) {   // 8 TF32 per k-step: 32 bytes (descriptor units of 16 B)
-                // the weights' low rows lie behind the high ones: one instruction multiplies both with the activations' high parts
-                sm_mma_ss(acc, ahi + 2 * j, w + 2 * j, hi, idesc2, first && j == 0 ? 0u : 1u);
-                if (MODE3X) sm_mma_ss(acc + NT, alo + 2 * j, w + 2 * j, hi, idesc, 1u);
+                for (int j = 0; j < SM_BK / 8; ++j) {   // 8 TF32 per k-step: 32 bytes (descriptor units of 16 B)
+                    // the weights' low rows lie behind the high ones: one instruction multiplies both with the activations' high parts
+                    sm_mma_ss(acc, ahi + 2 * j, w + 2 * j, hi, idesc2, first && j == 0 ? 0u : 1u);
+                    if (MODE3X) sm_mma_ss(acc + NT, alo + 2 * j, w + 2 * j, hi, idesc, 1u);
+                }
+                tc_commit(empty0 + 8 * s);
             }
-            tc_commit(empty0 + 8 * s);
+            __syncwarp();
         }
-        if (ok) tc_commit(acc_bar);
+        if (ok && lane == 0) tc_commit(acc_bar);
     }
     __syncwarp();
     if (p.cluster > 1) {
@@ -379,7 +382,6 @@ cn_gemm_small_kernel(const __grid_constant__ SmallParams p)
             const int ml = (warp & 3) * 32 + lane, col0 = (warp >> 2) * (NT / 4);
             const int64_t m = m0 + ml;
             const uint32_t src = tmem + ((uint32_t)((warp & 3) * 32) << 16);
-            const bool plain = p.act == CN_ACT_LINEAR && p.npeers == 0;
 #pragma unroll 1
             for (int col = col0; col < col0 + NT / 4 && col < n_rows; col += 8) {
                 float v[8];
@@ -403,17 +405,27 @@ cn_gemm_small_kernel(const __grid_constant__ SmallParams p)
 #pragma unroll
                         for (int e = 0; e < 8; ++e) v[e] += s_bias[col + e];
                     }
-                    if (plain) {
+                    if (p.act == CN_ACT_RELU) {
 #pragma unroll
-                        for (int e = 0; e < 8; ++e, q += p.ldc)
-                            if (e < cols_here) *q = v[e];
-                    } else {
+                        for (int e = 0; e < 8; ++e) v[e] = v[e] > 0.0f ? v[e] : 0.0f;
+                    } else if (p.act != CN_ACT_LINEAR) {
+                        // one copy of the units' longer code: eight of them, with the switch around each, took 2500 clocks per pass, rectifiers too
+#pragma unroll 1
+                        for (int e = 0; e < 8; ++e) {
+                            const float y = cn_apply_activation(v[0], p.act);
 #pragma unroll
-                        for (int e = 0; e < 8; ++e, q += p.ldc) {
+                            for (int i = 0; i < 7; ++i) v[i] = v[i + 1];
+                            v[7] = y;
+                        }
+                    }
+#pragma unroll
+                    for (int e = 0; e < 8; ++e, q += p.ldc)
+                        if (e < cols_here) *q = v[e];
+                    if (p.npeers > 0) {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
                             if (e >= cols_here) continue;
-                            const float a = cn_apply_activation(v[e], p.act);
-                            *q = a;
-                            for (int d = 0; d < p.npeers; ++d) p.peerC[d][(n0 + col + e) * p.ldc + m] = a;
+                            for (int d = 0; d < p.npeers; ++d) p.peerC[d][(n0 + col + e) * p.ldc + m] = v[e];
                         }
                     }
                 }
