@@ -220,36 +220,43 @@ struct SmFeed {
     }
 };
 
-__device__ __forceinline__ void sm_ld8(uint32_t taddr, uint32_t *r)
+template <int COLS>
+__device__ __forceinline__ void sm_ld(uint32_t taddr, uint32_t (&r)[COLS])
 {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+    if constexpr (COLS == 8)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
+    else
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+              "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+            : "r"(taddr) : "memory");
 }
-// Eight columns of the accumulators of all chains, in K order, the products with a low part last.  Up to four accumulators are loaded
-// before the wait.
-template <int NT, bool MODE3X>
-__device__ __forceinline__ void sm_sum8(uint32_t taddr, int chains, float (&v)[8])
+// Columns of the accumulators of all chains, in K order, the products with a low part last.
+template <int NT, bool MODE3X, int COLS>
+__device__ __forceinline__ void sm_sum(uint32_t taddr, int chains, float (&v)[COLS])
 {
     using Cfg = SmCfg<NT, MODE3X>;
-    constexpr int PARTS = MODE3X ? 2 : 1, GROUP = Cfg::MAX_CHAINS < 4 ? Cfg::MAX_CHAINS : 4;
-    float low[8];
+    constexpr int PARTS = MODE3X ? 2 : 1, GROUP = COLS == 8 ? 4 : 1;   // accumulators that are loaded before the wait
+    float low[COLS];
 #pragma unroll
-    for (int c = 0; c < 8; ++c) v[c] = low[c] = 0.0f;
+    for (int c = 0; c < COLS; ++c) v[c] = low[c] = 0.0f;
 #pragma unroll 1
     for (int ch0 = 0; ch0 < chains; ch0 += GROUP) {
-        uint32_t r[GROUP][PARTS][8];
+        uint32_t r[GROUP][PARTS][COLS];
 #pragma unroll
         for (int ch = 0; ch < GROUP; ++ch) {
             if (ch0 + ch >= chains) break;
 #pragma unroll
-            for (int part = 0; part < PARTS; ++part) sm_ld8(taddr + (ch0 + ch) * Cfg::ACC_COLS + part * NT, r[ch][part]);
+            for (int part = 0; part < PARTS; ++part) sm_ld<COLS>(taddr + (ch0 + ch) * Cfg::ACC_COLS + part * NT, r[ch][part]);
         }
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
         for (int ch = 0; ch < GROUP; ++ch) {
             if (ch0 + ch >= chains) break;
 #pragma unroll
-            for (int c = 0; c < 8; ++c) {
+            for (int c = 0; c < COLS; ++c) {
 #pragma unroll
                 for (int part = 0; part < PARTS; ++part) asm volatile("" : "+r"(r[ch][part][c]));   // no use moves before the wait
                 v[c] += __uint_as_float(r[ch][0][c]);
@@ -259,7 +266,7 @@ __device__ __forceinline__ void sm_sum8(uint32_t taddr, int chains, float (&v)[8
     }
     if (MODE3X) {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) v[c] += low[c];
+        for (int c = 0; c < COLS; ++c) v[c] += low[c];
     }
 }
 
@@ -382,13 +389,14 @@ cn_gemm_small_kernel(const __grid_constant__ SmallParams p)
             const int ml = (warp & 3) * 32 + lane, col0 = (warp >> 2) * (NT / 4);
             const int64_t m = m0 + ml;
             const uint32_t src = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+            constexpr int COLS = NT == 32 ? 8 : 16;   // per pass
 #pragma unroll 1
-            for (int col = col0; col < col0 + NT / 4 && col < n_rows; col += 8) {
-                float v[8];
-                sm_sum8<NT, MODE3X>(src + col, chains, v);
+            for (int col = col0; col < col0 + NT / 4 && col < n_rows; col += COLS) {
+                float v[COLS];
+                sm_sum<NT, MODE3X, COLS>(src + col, chains, v);
                 if (p.cluster > 1) {
 #pragma unroll
-                    for (int e = 0; e < 8; e += 4) {   // four columns of a row: 512 contiguous bytes per warp
+                    for (int e = 0; e < COLS; e += 4) {   // four columns of a row: 512 contiguous bytes per warp
                         const int four = (col + e) >> 2, dst = four * p.per_inv >> 16;
                         if (four >= fours) break;
                         const uint32_t at = part + (uint32_t)((rank * per + four - dst * per) * SM_BM + ml) * 16;
@@ -400,30 +408,30 @@ cn_gemm_small_kernel(const __grid_constant__ SmallParams p)
                     }
                 } else if (m < p.M) {
                     float *q = p.C + (n0 + col) * p.ldc + m;
-                    const int cols_here = n_rows - col < 8 ? n_rows - col : 8;
+                    const int cols_here = n_rows - col < COLS ? n_rows - col : COLS;
                     if (p.bias) {
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) v[e] += s_bias[col + e];
+                        for (int e = 0; e < COLS; ++e) v[e] += s_bias[col + e];
                     }
                     if (p.act == CN_ACT_RELU) {
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) v[e] = v[e] > 0.0f ? v[e] : 0.0f;
+                        for (int e = 0; e < COLS; ++e) v[e] = v[e] > 0.0f ? v[e] : 0.0f;
                     } else if (p.act != CN_ACT_LINEAR) {
                         // one copy of the units' longer code: eight of them, with the switch around each, took 2500 clocks per pass, rectifiers too
 #pragma unroll 1
-                        for (int e = 0; e < 8; ++e) {
+                        for (int e = 0; e < COLS; ++e) {
                             const float y = cn_apply_activation(v[0], p.act);
 #pragma unroll
-                            for (int i = 0; i < 7; ++i) v[i] = v[i + 1];
-                            v[7] = y;
+                            for (int i = 0; i < COLS - 1; ++i) v[i] = v[i + 1];
+                            v[COLS - 1] = y;
                         }
                     }
 #pragma unroll
-                    for (int e = 0; e < 8; ++e, q += p.ldc)
+                    for (int e = 0; e < COLS; ++e, q += p.ldc)
                         if (e < cols_here) *q = v[e];
                     if (p.npeers > 0) {
 #pragma unroll
-                        for (int e = 0; e < 8; ++e) {
+                        for (int e = 0; e < COLS; ++e) {
                             if (e >= cols_here) continue;
                             for (int d = 0; d < p.npeers; ++d) p.peerC[d][(n0 + col + e) * p.ldc + m] = v[e];
                         }
