@@ -668,7 +668,8 @@ cn_gemm_planes_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
         // the streaming kernel does it
     } else if (warp < 4) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PL_REGS_WG0));
-        if (warp == 0 && lane == 0) {
+        // Whole warps wait, which takes half as long as by one lane; one lane issues.
+        if (warp == 0) {
             // ------------------------------------------------------------ TMA producer of this CTA's halves
             PlWalk walk(p);
             int tile, k0, k1, slot;
@@ -680,13 +681,16 @@ cn_gemm_planes_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
                     const int s = it % Cfg::STAGES;
                     ok = mbar_wait(empty_bar(s), ((it / Cfg::STAGES) & 1u) ^ 1u, abort_flag, p.status, 19u);
                     if (!ok) break;
-                    if (rank == 0) mbar_expect_tx(full_bar(s), (uint32_t)(2 * Cfg::PARTS * (PL_TILE_BYTES + p.half * TC_AK * 2)));
-                    const uint32_t bar = pl_in_first(full_bar(s)), dst = smem_base + s * Cfg::STAGE_BYTES;
+                    if (lane == 0) {
+                        if (rank == 0) mbar_expect_tx(full_bar(s), (uint32_t)(2 * Cfg::PARTS * (PL_TILE_BYTES + p.half * TC_AK * 2)));
+                        const uint32_t bar = pl_in_first(full_bar(s)), dst = smem_base + s * Cfg::STAGE_BYTES;
 #pragma unroll
-                    for (int part = 0; part < Cfg::PARTS; ++part) {
-                        pl_load(dst + part * PL_TILE_BYTES, &tm_w, bar, st * TC_AK, n0, part);
-                        pl_load(dst + (Cfg::PARTS + part) * PL_TILE_BYTES, &tm_a, bar, st * TC_AK, m0, part);
+                        for (int part = 0; part < Cfg::PARTS; ++part) {
+                            pl_load(dst + part * PL_TILE_BYTES, &tm_w, bar, st * TC_AK, n0, part);
+                            pl_load(dst + (Cfg::PARTS + part) * PL_TILE_BYTES, &tm_a, bar, st * TC_AK, m0, part);
+                        }
                     }
+                    __syncwarp();
                 }
             }
             // the last stages must have been multiplied before the CTA may exit; after a wait that ran out, copies in flight get a
@@ -697,7 +701,7 @@ cn_gemm_planes_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
                 const long long t0 = clock64();
                 while (clock64() - t0 < 20000000LL) {}
             }
-        } else if (warp == 1 && lane == 0 && rank == 0) {
+        } else if (warp == 1 && rank == 0) {
             // ------------------------------------------------------------ MMA issuer of the pair
             PlWalk walk(p);
             int tile, k0, k1, slot;
@@ -721,28 +725,30 @@ cn_gemm_planes_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
                     const uint64_t d = make_kmajor_sw128_desc(smem_base + s * Cfg::STAGE_BYTES);
                     const uint32_t hi = (uint32_t)(d >> 32), whi = (uint32_t)d, wlo = whi + (PL_TILE_BYTES >> 4), ahi = whi + (Cfg::PARTS * PL_TILE_BYTES >> 4),
                                    alo = ahi + (PL_TILE_BYTES >> 4);
-                    // 16 fp16 per k-step: 32 bytes (descriptor units of 16 B).  In the first stage of a chain the products with a low part
-                    // come first: an addition truncates what it adds to a large sum, and there is none yet.
-                    if (MODE3X && first) {
+                    const bool last = st == k1 - 1 || ((st + 1) & (p.chain - 1)) == 0;
+                    if (lane == 0) {
+                        // 16 fp16 per k-step: 32 bytes (descriptor units of 16 B).  In the first stage of a chain the products with a low part
+                        // come first: an addition truncates what it adds to a large sum, and there is none yet.
+                        if (MODE3X && first) {
+#pragma unroll
+                            for (int j = 0; j < TC_AK / 16; ++j) {
+                                pl_mma_ss(acc, wlo + 2 * j, ahi + 2 * j, hi, idesc, j == 0 ? 0u : 1u);
+                                pl_mma_ss(acc, whi + 2 * j, alo + 2 * j, hi, idesc, 1u);
+                            }
+                        }
 #pragma unroll
                         for (int j = 0; j < TC_AK / 16; ++j) {
-                            pl_mma_ss(acc, wlo + 2 * j, ahi + 2 * j, hi, idesc, j == 0 ? 0u : 1u);
-                            pl_mma_ss(acc, whi + 2 * j, alo + 2 * j, hi, idesc, 1u);
+                            pl_mma_ss(acc, whi + 2 * j, ahi + 2 * j, hi, idesc, !MODE3X && first && j == 0 ? 0u : 1u);
+                            if (MODE3X && !first) {
+                                pl_mma_ss(acc, wlo + 2 * j, ahi + 2 * j, hi, idesc, 1u);
+                                pl_mma_ss(acc, whi + 2 * j, alo + 2 * j, hi, idesc, 1u);
+                            }
                         }
+                        pl_commit(empty_bar(s));
+                        if (last) pl_commit(accfull_bar(ab));
                     }
-#pragma unroll
-                    for (int j = 0; j < TC_AK / 16; ++j) {
-                        pl_mma_ss(acc, whi + 2 * j, ahi + 2 * j, hi, idesc, !MODE3X && first && j == 0 ? 0u : 1u);
-                        if (MODE3X && !first) {
-                            pl_mma_ss(acc, wlo + 2 * j, ahi + 2 * j, hi, idesc, 1u);
-                            pl_mma_ss(acc, whi + 2 * j, alo + 2 * j, hi, idesc, 1u);
-                        }
-                    }
-                    pl_commit(empty_bar(s));
-                    if (st == k1 - 1 || ((st + 1) & (p.chain - 1)) == 0) {
-                        pl_commit(accfull_bar(ab));
-                        ++chains;
-                    }
+                    __syncwarp();
+                    if (last) ++chains;
                 }
             }
         }
