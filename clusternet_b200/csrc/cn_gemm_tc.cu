@@ -1099,7 +1099,7 @@ cn_splitk_reduce_kernel(const __grid_constant__ ReduceParams p)
     float4 acc[QUADS];
 #pragma unroll
     for (int j = 0; j < QUADS; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-    int64_t left = c1 - c0 + 1;
+    int64_t left = m0 + quad * 4 < p.M ? c1 - c0 + 1 : 0;   // rows that do not exist are not read
     // the additions stay in K order, so the sum does not depend on the grouping; what is left of a group is loaded together, too
     for (; left > 0; left -= UNROLL, src += UNROLL * step) {
         float4 v[UNROLL][QUADS];
