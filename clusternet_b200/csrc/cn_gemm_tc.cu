@@ -925,10 +925,14 @@ cn_gemm_tc_kernel(const __grid_constant__ WMaps tm_w, const __grid_constant__ CU
                 break;
             }
             if (seg.slot >= 0) {
-                // partial tile: float4 number i of 32 for all 128 columns, then the next, so that a warp writes 512 contiguous bytes
+                // Partial tile: float4 number i of 32 for all 128 columns, then the next, so that a warp writes 512 contiguous bytes.  Rows that
+                // do not exist are neither written nor read: 20 x 9000 . 9000 x 4000 48.4 -> 43.8 us (46.7 where only the reduction leaves
+                // them), 203 x 4001 . 4001 x 3001 47.2 -> 46.0.  Leaving them out of the multiplication and the sums, too, cost full tiles 2 %.
+                const int64_t rows = p.M - m0;
                 ulonglong2 *P = reinterpret_cast<ulonglong2 *>(p.partials) + ((int64_t)seg.slot * NT + w) * (TC_BM * TC_BN / 4) + row;
 #pragma unroll
-                for (int i = 0; i < TC_BM / 4; ++i) P[i * TC_BN] = make_ulonglong2(sum[2 * i], sum[2 * i + 1]);
+                for (int i = 0; i < TC_BM / 4; ++i)
+                    if (i * 4 < rows) P[i * TC_BN] = make_ulonglong2(sum[2 * i], sum[2 * i + 1]);
                 continue;
             }
             const int L = p.maxout_level;
@@ -1099,7 +1103,7 @@ cn_splitk_reduce_kernel(const __grid_constant__ ReduceParams p)
     float4 acc[QUADS];
 #pragma unroll
     for (int j = 0; j < QUADS; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-    int64_t left = m0 + quad * 4 < p.M ? c1 - c0 + 1 : 0;   // rows that do not exist are not read
+    int64_t left = m0 + quad * 4 < p.M ? c1 - c0 + 1 : 0;   // rows that do not exist have not been written
     // the additions stay in K order, so the sum does not depend on the grouping; what is left of a group is loaded together, too
     for (; left > 0; left -= UNROLL, src += UNROLL * step) {
         float4 v[UNROLL][QUADS];

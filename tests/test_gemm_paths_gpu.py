@@ -323,6 +323,24 @@ def test_few_tiles_in_many_runs(ctx, M, K, N, nt):
     assert np.linalg.norm(ctx.to_numpy(C) - ref) <= 8e-6 * np.linalg.norm(ref)
 
 
+@pytest.mark.parametrize("M", [1, 3, 4, 5, 31, 127, 129, 133, 255, 257])
+@pytest.mark.parametrize("nt,splits", [(1, 3), (2, 9)])
+def test_rows_that_partial_tiles_do_not_have(ctx, M, nt, splits):
+    """Neither written nor read: what an earlier product of whole tiles left there, NaN, must not show."""
+    from clusternet_b200 import check as status
+    rng = np.random.default_rng(M)
+    A, B = rng.uniform(-1, 1, (M, 3000)).astype(np.float32), rng.uniform(-1, 1, (3000, 270)).astype(np.float32)
+    status(ctx.lib.cn_gemm_set_tuning(ctx.h, nt, splits, 0))
+    try:
+        dB = place(B, 0)
+        ctx.gemm(torch.full((3000, (M + 127) // 128 * 128), float("nan"), device="cuda"), dB)
+        C = ctx.gemm(place(A, 0), dB)
+        ctx.gemm_check()
+    finally:
+        status(ctx.lib.cn_gemm_set_tuning(ctx.h, 0, 0, 0))
+    check(C, A, B, False, False, REL_3X)
+
+
 @pytest.mark.parametrize("mode,rel", [(_lib.GEMM_3XTF32, REL_3X), (_lib.GEMM_TF32, REL_1X)])
 @pytest.mark.parametrize("half", [0, 1])
 @pytest.mark.parametrize("M,N,splits", [(128, 256, 7), (200, 1000, 13), (16, 100, 37)])
