@@ -324,12 +324,12 @@ def test_few_tiles_in_many_runs(ctx, M, K, N, nt):
 
 
 @pytest.mark.parametrize("M", [1, 3, 4, 5, 31, 127, 129, 133, 255, 257])
-@pytest.mark.parametrize("nt,splits", [(1, 3), (2, 9)])
-def test_rows_that_partial_tiles_do_not_have(ctx, M, nt, splits):
-    """Neither written nor read: what an earlier product of whole tiles left there, NaN, must not show."""
+@pytest.mark.parametrize("N,nt,splits", [(270, 1, 3), (270, 2, 9), (5000, 1, 2)])
+def test_rows_that_partial_tiles_do_not_have(ctx, M, N, nt, splits):
+    """Neither written nor read, with 8 or 32 columns per CTA of the reduction: what an earlier product of whole tiles left there, NaN, must not show."""
     from clusternet_b200 import check as status
     rng = np.random.default_rng(M)
-    A, B = rng.uniform(-1, 1, (M, 3000)).astype(np.float32), rng.uniform(-1, 1, (3000, 270)).astype(np.float32)
+    A, B = rng.uniform(-1, 1, (M, 3000)).astype(np.float32), rng.uniform(-1, 1, (3000, N)).astype(np.float32)
     status(ctx.lib.cn_gemm_set_tuning(ctx.h, nt, splits, 0))
     try:
         dB = place(B, 0)
