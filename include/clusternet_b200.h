@@ -194,7 +194,7 @@ int cn_gemm_f32(cn_context *ctx, int transA, int transB, int64_t M, int64_t N, i
  * ("tcgen05_3xtf32", "tcgen05_tf32", "simt_fp32"); for tests and reports. */
 const char *cn_gemm_last_path(const cn_context *ctx);
 /* Which kernel that call took: "small" (one launch), "streaming", "planes" (many rows; the streaming kernel stands behind it for operands
- * whose elements two fp16 parts cannot hold), "fma"; for tests and reports. */
+ * whose elements two fp16 parts cannot hold), "outer" (weight gradients of few rows, one launch), "fma"; for tests and reports. */
 const char *cn_gemm_last_kernel(const cn_context *ctx);
 /* The tensor-core kernel bounds every wait of its internal pipeline; a wait that runs out makes the kernel
  * return early and set a device status word.  This call drains `stream`, reads the word and returns
