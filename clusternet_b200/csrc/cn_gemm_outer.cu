@@ -451,9 +451,9 @@ cn_gemm_outer_kernel(const __grid_constant__ OuterParams p)
             if (p.passes > 1 && ok) read(false);
             if (!ok) break;
             if (m < p.M) {
-                // a base that all lanes have in common, and 32 bits of this lane's
-                char *to = reinterpret_cast<char *>(p.C + (int64_t)col0 * p.ldc);
-                const uint32_t at = (uint32_t)m * 4u;
+                // a base that all lanes have in common, and 32 bits of this lane's: its row within the strip (a matrix may have 2^30 rows and more)
+                char *to = reinterpret_cast<char *>(p.C + ((int64_t)col0 * p.ldc + (int64_t)strip * SM_BM));
+                const uint32_t at = (uint32_t)(q * 32 + lane) * 4u;
                 const int64_t column = p.ldc * 4;
                 if (here >= 16) {
 #pragma unroll

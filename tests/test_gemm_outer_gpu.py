@@ -49,6 +49,26 @@ def test_weight_gradients_of_few_rows(ctx, M, K, N, off):
     assert torch.equal(first, C)   # bit for bit the same again
 
 
+def test_more_rows_than_a_32_bit_offset_in_bytes_reaches(ctx):
+    """Rows from 2^30 on, and those that an offset which wraps would write in their place."""
+    M, K, N = (1 << 30) + 300, 20, 1
+    if torch.cuda.mem_get_info()[0] < 100e9:
+        pytest.skip("needs 92 GB")
+    act = torch.empty(M, K, device="cuda").normal_(generator=torch.Generator(device="cuda").manual_seed(5))
+    err = torch.randn(N, K, device="cuda", generator=torch.Generator(device="cuda").manual_seed(6))
+    C = torch.full((N, M), 7.0, device="cuda")
+    try:
+        ctx.gemm(act, err, out=C, transA=True)
+        ctx.gemm_check()
+        assert ctx.gemm_last_kernel() == "outer"
+        for r in (0, 1 << 20, (1 << 30) - 400, M - 400):
+            a = act[r:r + 400].double()
+            assert bool(((C[:, r:r + 400].double() - err.double() @ a.t()).abs() <= REL * (err.double().abs() @ a.abs().t())).all())
+    finally:
+        del act, err, C
+        torch.cuda.empty_cache()
+
+
 @pytest.mark.parametrize("off", [0, 1])
 def test_non_finite_and_the_largest_finite_values_stay_in_their_row_and_column(ctx, off):
     """NaNs of any bit pattern and infinities of either operand; a value that rounds past the largest TF32 number stays finite."""
