@@ -111,3 +111,17 @@ def test_what_is_no_such_weight_gradient(ctx, M, K, N, kw):
     if "activation" in kw:
         ref = ref.clamp(min=0)
     assert float((C.double() - ref).norm() / ref.norm()) <= (1e-3 if kw.get("mode") else 1e-6)
+
+
+@pytest.mark.parametrize("M,K,N", [(300001, 17, 3), (200000, 33, 1), (90000, 126, 2)])
+def test_few_columns_of_odd_pitch_stay_exact(ctx, M, K, N):
+    """Products of two odd numbers of twelve bits: 24 bits, of which the last comes from the parts that eleven bits leave of either."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    act = torch.zeros(M, K, device="cuda")
+    act[torch.arange(M, device="cuda"), torch.randint(0, K, (M,), device="cuda", generator=g)] = \
+        2.0 * torch.randint(1024, 2048, (M,), device="cuda", generator=g).float() + 1.0
+    err = 2.0 * torch.randint(1024, 2048, (N, K), device="cuda", generator=g).float() + 1.0
+    C = ctx.gemm(act, err, transA=True)
+    ctx.gemm_check()
+    assert ctx.gemm_last_kernel() == "fma"
+    assert torch.equal(C.double(), err.double() @ act.double().t())
