@@ -250,19 +250,18 @@ __global__ void __launch_bounds__(OUT_THREADS, 1)
 cn_gemm_outer_kernel(const __grid_constant__ OuterParams p)
 {
     extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t bars[OUT_STAGES + 5];
+    __shared__ __align__(8) uint64_t bars[OUT_STAGES + 6];
     __shared__ uint32_t s_words[2];   // tensor-memory base, abort flag
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u, stage_bytes = (uint32_t)p.kb * OUT_CHUNK_BYTES;
     // the weights of a stage are there; the products of an accumulator have retired (and the stage that they read is free); an accumulator has
-    // been read; a strip is there
-    const uint32_t full0 = smem_u32(&bars[0]), done0 = full0 + 8 * OUT_STAGES, read0 = done0 + 16, strip_bar = read0 + 16;
+    // been read; a strip is there, strips by turns
+    const uint32_t full0 = smem_u32(&bars[0]), done0 = full0 + 8 * OUT_STAGES, read0 = done0 + 16, strip0 = read0 + 16;
     const uint32_t abort_flag = smem_u32(&s_words[1]);
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // the same for the whole warp, which the compiler is told
     cn_pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (int s = 0; s < OUT_STAGES; ++s) mbar_init(full0 + 8 * s, OUT_WORK / 32);
-        for (int b = 0; b < 2; ++b) { mbar_init(done0 + 8 * b, 1); mbar_init(read0 + 8 * b, OUT_WORK / 32); }
-        mbar_init(strip_bar, OUT_WORK / 32);
+        for (int b = 0; b < 2; ++b) { mbar_init(done0 + 8 * b, 1); mbar_init(read0 + 8 * b, OUT_WORK / 32); mbar_init(strip0 + 8 * b, OUT_WORK / 32); }
         s_words[1] = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -283,13 +282,16 @@ cn_gemm_outer_kernel(const __grid_constant__ OuterParams p)
         constexpr uint32_t idesc = tf32 | ((uint32_t)(OUT_N >> 3) << 17), idesc2 = tf32 | ((uint32_t)(OUT_ACC_COLS >> 3) << 17);
         const uint64_t d0 = make_kmajor_sw128_desc(ring);
         const uint32_t hi = (uint32_t)(d0 >> 32), b = warp & 1u, acc = tmem + OUT_ACC_COL + b * OUT_ACC_COLS;
+        const int first_strip = walk.strip;
         int have = -1;
-        uint32_t strip_phase = 1u, accs = 0u;
+        uint32_t accs = 0u;
         for (uint32_t i = 0; ok && walk.next(p, strip, n0, cols); ++i) {
-            if (strip != have) {   // either warp waits for every strip: a wait for the second phase from now would not wait at all
-                strip_phase ^= 1u;
+            // Either warp waits for every strip, on two barriers in turn: a wait for the phase after the next one would not wait at all, and a
+            // strip of a single block may be multiplied, and the next one made, before the warp that has no block there has looked.  That
+            // warp has the next strip's first block, so that it is never more than one phase late.
+            if (strip != have) {
                 have = strip;
-                ok = __all_sync(0xffffffffu, mbar_wait(strip_bar, strip_phase, abort_flag, p.status, 25u));
+                ok = __all_sync(0xffffffffu, mbar_wait(strip0 + 8 * (strip & 1), (uint32_t)(strip - first_strip) >> 1 & 1u, abort_flag, p.status, 25u));
                 if (!ok) break;
             }
             const uint32_t s = i % OUT_STAGES;
@@ -382,7 +384,7 @@ cn_gemm_outer_kernel(const __grid_constant__ OuterParams p)
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(strip_bar);
+            if (lane == 0) mbar_arrive(strip0 + 8 * (strip & 1));
             asm volatile("bar.sync 1, %0;" ::"n"(OUT_WORK) : "memory");   // the stage may be written
         };
         auto put = [&](uint32_t s) {

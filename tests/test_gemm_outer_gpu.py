@@ -22,9 +22,9 @@ def place(x, off):
 
 
 # k: seventeen, a block of 32 k less one, whole ones, odd ones, all four; rows: eight, a strip and one more; columns: of one unit, of 16 units and one more;
-# 4884 x 2576: 39 strips shared by all CTAs, some of whose strips end after one block; 9000 rows: 71 strips
+# 60000 x 40, 100000 x 9: several strips of one block for every CTA, of two for 70; 4884 x 2576: 39 strips shared by all CTAs, some of whose strips end after one block; 9000 rows: 71 strips
 SHAPES = [(8, 17, 150000), (129, 31, 33000), (2000, 32, 1700), (2001, 33, 1601), (1540, 64, 3500), (1000, 65, 4001), (1600, 96, 2000), (1537, 97, 2050), (2000, 128, 2000), (2049, 127, 1999),
-          (4096, 128, 4096), (4884, 64, 2576), (4884, 127, 2577), (9000, 100, 520), (20000, 128, 17), (300, 128, 9001)]
+          (60000, 64, 40), (100000, 96, 9), (60000, 20, 70), (4096, 128, 4096), (4884, 64, 2576), (4884, 127, 2577), (9000, 100, 520), (20000, 128, 17), (300, 128, 9001)]
 
 
 @pytest.mark.parametrize("M,K,N", SHAPES)
