@@ -250,18 +250,19 @@ __global__ void __launch_bounds__(OUT_THREADS, 1)
 cn_gemm_outer_kernel(const __grid_constant__ OuterParams p)
 {
     extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t bars[OUT_STAGES + 6];
+    __shared__ __align__(8) uint64_t bars[OUT_STAGES + 7];
     __shared__ uint32_t s_words[2];   // tensor-memory base, abort flag
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u, stage_bytes = (uint32_t)p.kb * OUT_CHUNK_BYTES;
     // the weights of a stage are there; the products of an accumulator have retired (and the stage that they read is free); an accumulator has
-    // been read; a strip is there, strips by turns
-    const uint32_t full0 = smem_u32(&bars[0]), done0 = full0 + 8 * OUT_STAGES, read0 = done0 + 16, strip0 = read0 + 16;
+    // been read; a strip is there, strips by turns; the stage by way of which it was made is free again
+    const uint32_t full0 = smem_u32(&bars[0]), done0 = full0 + 8 * OUT_STAGES, read0 = done0 + 16, strip0 = read0 + 16, turned_bar = strip0 + 16;
     const uint32_t abort_flag = smem_u32(&s_words[1]);
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // the same for the whole warp, which the compiler is told
     cn_pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (int s = 0; s < OUT_STAGES; ++s) mbar_init(full0 + 8 * s, OUT_WORK / 32);
         for (int b = 0; b < 2; ++b) { mbar_init(done0 + 8 * b, 1); mbar_init(read0 + 8 * b, OUT_WORK / 32); mbar_init(strip0 + 8 * b, OUT_WORK / 32); }
+        mbar_init(turned_bar, OUT_WORK / 32);
         s_words[1] = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -359,7 +360,8 @@ cn_gemm_outer_kernel(const __grid_constant__ OuterParams p)
         float x[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) x[e] = 0.0f;
-        // by way of a stage that is free
+        // by way of a stage that is free.  The last wait is for all warps of the CTA, but bounded: one of them may have given up before.
+        const int first_strip = walk.strip;
         auto make_strip = [&](int strip, uint32_t stage) {
             const int row0 = strip * SM_BM + q * 32, rows = p.M - row0 < 32 ? p.M - row0 : 32;   // none, where negative
             if (g < p.kb) {
@@ -384,8 +386,8 @@ cn_gemm_outer_kernel(const __grid_constant__ OuterParams p)
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(strip0 + 8 * (strip & 1));
-            asm volatile("bar.sync 1, %0;" ::"n"(OUT_WORK) : "memory");   // the stage may be written
+            if (lane == 0) { mbar_arrive(strip0 + 8 * (strip & 1)); mbar_arrive(turned_bar); }
+            ok = __all_sync(0xffffffffu, mbar_wait(turned_bar, (uint32_t)(strip - first_strip) & 1u, abort_flag, p.status, 27u));   // the stage may be written
         };
         auto put = [&](uint32_t s) {
             share.store(p, ring + s * stage_bytes, x);
@@ -401,7 +403,7 @@ cn_gemm_outer_kernel(const __grid_constant__ OuterParams p)
         make_strip(strip, ring);
         uint32_t accs = 0u, s = 0u;   // s: the stage of the block that is read, and of the one three blocks on
 #pragma unroll 1
-        for (; s < OUT_STAGES && amore; ++s) {
+        for (; s < OUT_STAGES && amore && ok; ++s) {
             put(s);
             amore = ahead.next(p, astrip, an0, acols);
             if (amore) share.load(p, an0, acols, x);
@@ -468,6 +470,7 @@ cn_gemm_outer_kernel(const __grid_constant__ OuterParams p)
             }
             // all products that read this strip have retired: the next one takes its place, by way of the stage that they have left
             if (change) make_strip(next_strip, ring + s * stage_bytes);
+            if (!ok) break;
             strip = next_strip;
             // Half of the warps store first, the others split first: stores are bound by the way to L2, which takes 32 bytes per clock from an SM.
             if (amore) {
