@@ -292,15 +292,14 @@ cn_gemm_outer_kernel(const __grid_constant__ OuterParams p)
             // warp has the next strip's first block, so that it is never more than one phase late.
             if (strip != have) {
                 have = strip;
-                ok = __all_sync(0xffffffffu, mbar_wait(strip0 + 8 * (strip & 1), (uint32_t)(strip - first_strip) >> 1 & 1u, abort_flag, p.status, 25u));
+                ok = mbar_wait_warp(strip0 + 8 * (strip & 1), (uint32_t)(strip - first_strip) >> 1 & 1u, abort_flag, p.status, 25u);
                 if (!ok) break;
             }
             const uint32_t s = i % OUT_STAGES;
             for (int pass = 0; pass < p.passes && ok; ++pass, ++accs) {
                 if ((accs & 1u) != b) continue;
-                ok = mbar_wait(full0 + 8 * s, i / OUT_STAGES & 1u, abort_flag, p.status, 15u) &&
-                     mbar_wait(read0 + 8 * b, (accs >> 1 & 1u) ^ 1u, abort_flag, p.status, 26u);
-                ok = __all_sync(0xffffffffu, ok);
+                ok = mbar_wait_warp(full0 + 8 * s, i / OUT_STAGES & 1u, abort_flag, p.status, 15u) &&
+                     mbar_wait_warp(read0 + 8 * b, (accs >> 1 & 1u) ^ 1u, abort_flag, p.status, 26u);
                 if (!ok) break;
                 tc_fence_after();
                 if (lane == 0) {
@@ -387,7 +386,7 @@ cn_gemm_outer_kernel(const __grid_constant__ OuterParams p)
             tc_fence_before();
             __syncwarp();
             if (lane == 0) { mbar_arrive(strip0 + 8 * (strip & 1)); mbar_arrive(turned_bar); }
-            ok = __all_sync(0xffffffffu, mbar_wait(turned_bar, (uint32_t)(strip - first_strip) & 1u, abort_flag, p.status, 27u));   // the stage may be written
+            ok = mbar_wait_warp(turned_bar, (uint32_t)(strip - first_strip) & 1u, abort_flag, p.status, 27u);   // the stage may be written
         };
         auto put = [&](uint32_t s) {
             share.store(p, ring + s * stage_bytes, x);
@@ -418,8 +417,7 @@ cn_gemm_outer_kernel(const __grid_constant__ OuterParams p)
             // the sums of the next accumulator, over all products of a part of K
             auto read = [&](bool first) {
                 const uint32_t b = accs & 1u, src = lanes + OUT_ACC_COL + b * OUT_ACC_COLS + g * 16;
-                ok = mbar_wait(done0 + 8 * b, accs >> 1 & 1u, abort_flag, p.status, 16u);
-                ok = __all_sync(0xffffffffu, ok);
+                ok = mbar_wait_warp(done0 + 8 * b, accs >> 1 & 1u, abort_flag, p.status, 16u);
                 if (!ok) return;
                 ++accs;
                 tc_fence_after();

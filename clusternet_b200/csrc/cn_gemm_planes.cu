@@ -688,7 +688,7 @@ cn_gemm_planes_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
                 const int32_t n0 = (tile / p.tiles_m) * 256 + (int)rank * 128, m0 = (tile % p.tiles_m) * 2 * p.half + (int)rank * p.half;
                 for (int st = k0; st < k1; ++st, ++it) {
                     const int s = it % Cfg::STAGES;
-                    ok = mbar_wait(empty_bar(s), ((it / Cfg::STAGES) & 1u) ^ 1u, abort_flag, p.status, 19u);
+                    ok = mbar_wait_warp(empty_bar(s), ((it / Cfg::STAGES) & 1u) ^ 1u, abort_flag, p.status, 19u);
                     if (!ok) break;
                     if (lane == 0) {
                         if (rank == 0) mbar_expect_tx(full_bar(s), (uint32_t)(2 * Cfg::PARTS * (PL_TILE_BYTES + p.half * TC_AK * 2)));
@@ -705,7 +705,7 @@ cn_gemm_planes_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
             // the last stages must have been multiplied before the CTA may exit; after a wait that ran out, copies in flight get a
             // bounded chance to land
             for (uint32_t i = it > Cfg::STAGES ? it - Cfg::STAGES : 0; i < it && ok; ++i)
-                ok = mbar_wait(empty_bar(i % Cfg::STAGES), (i / Cfg::STAGES) & 1u, abort_flag, p.status, 20u);
+                ok = mbar_wait_warp(empty_bar(i % Cfg::STAGES), (i / Cfg::STAGES) & 1u, abort_flag, p.status, 20u);
             if (!ok) {
                 const long long t0 = clock64();
                 while (clock64() - t0 < 20000000LL) {}
@@ -725,9 +725,10 @@ cn_gemm_planes_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
                         const uint32_t parity = ((chains >> 1) & 1u) ^ 1u;
                         ok = mbar_try_cluster(accempty_bar(ab), parity) != 0u || (mbar_wait(accempty_bar(ab), parity, abort_flag, p.status, 21u) &&
                                                                                  mbar_try_cluster(accempty_bar(ab), parity) != 0u);
+                        ok = __all_sync(0xffffffffu, ok);
                         if (!ok) break;
                     }
-                    ok = mbar_wait(full_bar(s), (it / Cfg::STAGES) & 1u, abort_flag, p.status, 22u);
+                    ok = mbar_wait_warp(full_bar(s), (it / Cfg::STAGES) & 1u, abort_flag, p.status, 22u);
                     if (!ok) break;
                     tc_fence_after();
                     const uint32_t acc = tmem_base + ab * 256u;

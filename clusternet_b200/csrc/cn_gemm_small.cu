@@ -206,7 +206,7 @@ struct SmFeed {
             for (int u = 0; u < SM_AHEAD; ++u) {
                 const int i = i0 + u, s = i & 1;
                 if (i >= n || !ok) continue;
-                ok = mbar_wait(empty0 + 8 * s, ((uint32_t)(i >> 1) & 1u) ^ 1u, abort_flag, status, 14u);
+                ok = mbar_wait_warp(empty0 + 8 * s, ((uint32_t)(i >> 1) & 1u) ^ 1u, abort_flag, status, 14u);
                 if (!ok) continue;
                 const uint32_t stage = ring + s * stage_bytes;
                 share.template store<MODE3X>(stage + hi_off, stage + lo_off, x[u]);
@@ -352,7 +352,7 @@ cn_gemm_small_kernel(const __grid_constant__ SmallParams p)
         uint32_t acc = tmem;
         for (int i = 0; i < n_blocks; ++i) {
             const int s = i & 1;
-            ok = mbar_wait(full0 + 8 * s, (uint32_t)(i >> 1) & 1u, abort_flag, p.status, 15u);
+            ok = mbar_wait_warp(full0 + 8 * s, (uint32_t)(i >> 1) & 1u, abort_flag, p.status, 15u);
             if (!ok) break;
             tc_fence_after();
             const uint64_t d = make_kmajor_sw128_desc(ring + s * Cfg::STAGE_BYTES);
@@ -381,8 +381,7 @@ cn_gemm_small_kernel(const __grid_constant__ SmallParams p)
     }
     if (warp < 16) {
         if (p.bias) asm volatile("bar.sync 1, %0;" ::"n"(SM_EPI) : "memory");   // s_bias
-        ok = ok && mbar_wait(acc_bar, 0u, abort_flag, p.status, 16u);
-        ok = __all_sync(0xffffffffu, ok);
+        ok = ok && mbar_wait_warp(acc_bar, 0u, abort_flag, p.status, 16u);   // a warp's lanes agree on ok
         tc_fence_after();
         if (ok) {
             // four warps share a lane quarter and take a quarter of the columns each

@@ -109,6 +109,29 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
     }
 }
 
+// ... by a whole warp, whose lanes go on together or not at all: polls of different lanes may end differently when the limit runs out or another
+// role gives up, and lanes that part there wait for each other without a limit at the warp's or the CTA's next barrier.
+template <int SLEEP_NS = 0>
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, uint32_t abort_flag, unsigned int *status, unsigned int code)
+{
+    if (__all_sync(0xffffffffu, mbar_try(bar, parity) != 0u)) return true;
+    const long long t0 = clock64();
+    for (uint32_t it = 1;; ++it) {
+        if (SLEEP_NS > 0) __nanosleep(SLEEP_NS);
+        if (__all_sync(0xffffffffu, mbar_try(bar, parity) != 0u)) return true;
+        if ((it & 63u) == 0u) {
+            const bool late = clock64() - t0 > TC_WAIT_LIMIT;
+            if (__any_sync(0xffffffffu, late || lds1u(abort_flag) != 0u)) {
+                if (late) {
+                    sts1u(abort_flag, 1u);
+                    atomicMax(status, code);
+                }
+                return false;
+            }
+        }
+    }
+}
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, uint32_t bar, int32_t x, int32_t y)
 {
     asm volatile(
