@@ -10,7 +10,9 @@
 //   * two warps issue the MMAs, blocks in turn, each into an accumulator of its own: 64 columns for the products of the high parts and 64 for
 //     those with a low part (the activations' high parts are multiplied with both parts of the weights at once);
 //   * rows m lie in the lanes, so that a warp stores 128 bytes of a column straight from registers whatever C's pitch and alignment.
-// TF32 parts need no scales, have fp32's range, and leave nothing over: no lists, no second kernel behind this one.
+// TF32 parts need no scales of rows and columns and leave nothing over: no lists, no second kernel behind this one.  A low part as it is would have no
+// bits left below 2^-113, where it meets TF32's smallest step, 2^-136 (operands of 1e-36 3.4e-6 off, of 1e-38 3.3e-4).  So all low parts are held
+// times 2^OUT_LOW, which the sums of their products lose again: operands keep their 22 bits down to 2^-124, and from there on steps of 2^-146.
 //
 // us in a series, before / now: 4096 x 128 . 128 x 4096 40 / 25, 2000 x 128 . 128 x 2000 22.5 / 12.5, 6000 x
 // 32 . 32 x 6000 63 / 37 (planes); 2001 x 77 . 77 x 3003 58 / 16.3, 1504 x 64 . 64 x 3500 43 / 9.5 (streaming); 3734 x 104 . 104 x 575 16.2 / 9.4 (two rounds of small
@@ -37,6 +39,7 @@
 #define OUT_ACC_COL 256         // two accumulators behind the strip
 #define OUT_ACC_COLS 128
 #define OUT_CHUNK_BYTES (2 * OUT_N * 128)   // hi and lo parts of 64 columns x 32 k
+#define OUT_LOW 10              // with 11, a sum could exceed fp32's range where the products that it stands for do not
 #define OUT_STAGES 3
 #define OUT_SMEM (1024 + OUT_STAGES * OUT_MAX_BLOCKS * OUT_CHUNK_BYTES)
 
@@ -50,6 +53,7 @@ struct OuterParams {
     int kb;                 // blocks of 32 k
     int passes;             // parts of K that are multiplied into an accumulator each
     int two_chains;         // the products of the high parts of the two halves of such a part are added apart
+    float low;              // what an accumulator's second half still has to be multiplied by
     int sh;                 // log2 of 16-byte chunks of k, rounded up to a power of two
     int strips, units;      // of 128 rows m; of 16 columns n per strip
     int per_strip;          // CTAs that share a strip's units; 0: all strips' units, behind one another, are shared by all CTAs
@@ -121,14 +125,48 @@ __device__ __forceinline__ void out_st4(uint32_t taddr, const uint32_t (&v)[4])
 }
 __device__ __forceinline__ uint32_t out_at(int r, int c) { return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); }   // 16-byte chunk c of row r
 
+// D[tmem] = A[tmem] * B[smem] + D[tmem] * 2^-OUT_LOW
+__device__ __forceinline__ void out_mma_ts_lowered(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 bd;\n\t"
+        "setp.eq.b32 p, 0, 0;\n\t"
+        "mov.b64 bd, {%2, %3};\n\t"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], bd, %4, p, %5;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(desc_hi), "r"(idesc), "n"(OUT_LOW) : "memory");
+}
+
+// The parts of two elements, the low ones times 2^OUT_LOW.
+template <bool CAREFUL>
+__device__ __forceinline__ void out_split2(float x, float y, uint32_t (&h)[2], uint32_t (&l)[2])
+{
+    h[0] = sm_tf32<CAREFUL>(x);
+    h[1] = sm_tf32<CAREFUL>(y);
+    float lx, ly;   // what is left of both by one subtraction and one multiplication, exactly
+    asm("{\n\t.reg .b64 a, b, m;\n\t"
+        "mov.b64 a, {%2, %3};\n\t"
+        "mov.b64 b, {%4, %5};\n\t"
+        "mov.b64 m, {%6, %6};\n\t"
+        "fma.rn.f32x2 a, b, m, a;\n\t"
+        "mov.b64 m, {%7, %7};\n\t"
+        "mul.rn.f32x2 a, a, m;\n\t"
+        "mov.b64 {%0, %1}, a;\n\t}"
+        : "=f"(lx), "=f"(ly)
+        : "f"(x), "f"(y), "f"(__uint_as_float(h[0])), "f"(__uint_as_float(h[1])), "f"(-1.0f), "f"((float)(1 << OUT_LOW)));
+    l[0] = sm_tf32<CAREFUL>(lx);
+    l[1] = sm_tf32<CAREFUL>(ly);
+}
+
 // Four elements as parts.
 template <bool CAREFUL>
 __device__ __forceinline__ void out_split4(const float *y, uint32_t (&h)[4], uint32_t (&l)[4])
 {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        h[e] = sm_tf32<CAREFUL>(y[e]);
-        l[e] = sm_tf32<CAREFUL>(y[e] - __uint_as_float(h[e]));
+    for (int e = 0; e < 4; e += 2) {
+        uint32_t hh[2], ll[2];
+        out_split2<CAREFUL>(y[e], y[e + 1], hh, ll);
+        h[e] = hh[0]; h[e + 1] = hh[1];
+        l[e] = ll[0]; l[e + 1] = ll[1];
     }
 }
 
@@ -190,7 +228,7 @@ struct OutShare {
         stage += (uint32_t)(k >> 5) * OUT_CHUNK_BYTES + (VEC ? 0 : (k & 3) * 4);
         const int n = items(p);
 #pragma unroll
-        for (int i = 0; i < (VEC ? 4 : 16); ++i) {
+        for (int i = 0; i < (VEC ? 4 : 16); i += VEC ? 1 : 2) {
             if (i >= n) break;
             const uint32_t q = stage + out_at(row + i * rows_on(p), k >> 2 & 7);
             if (VEC) {
@@ -198,10 +236,14 @@ struct OutShare {
                 out_split4<CAREFUL>(x + (VEC ? 4 * i : 0), h, l);
                 sts4u(q, h[0], h[1], h[2], h[3]);
                 sts4u(q + lo, l[0], l[1], l[2], l[3]);
-            } else {
-                const uint32_t h = sm_tf32<CAREFUL>(x[i]);
-                sts1u(q, h);
-                sts1u(q + lo, sm_tf32<CAREFUL>(x[i] - __uint_as_float(h)));
+            } else {   // columns come in twos: four, eight or sixteen
+                const uint32_t r = stage + out_at(row + (i + 1) * rows_on(p), k >> 2 & 7);
+                uint32_t h[2], l[2];
+                out_split2<CAREFUL>(x[i], x[i + 1], h, l);
+                sts1u(q, h[0]);
+                sts1u(q + lo, l[0]);
+                sts1u(r, h[1]);
+                sts1u(r + lo, l[1]);
             }
         }
     }
@@ -305,7 +347,7 @@ cn_gemm_outer_kernel(const __grid_constant__ OuterParams p)
                 if (lane == 0) {
                     // Blocks [k0, k1) of 32 k.  Up to kt the products of the high parts go to the accumulator's first half and those with a low part
                     // to the second; the remaining blocks' products with a low part go to the second, too, and then, on top of all of
-                    // those, the products of their high parts.
+                    // those, which lose their factor, the products of their high parts.
                     const int k0 = p.kb * pass / p.passes, k1 = p.kb * (pass + 1) / p.passes, kt = p.two_chains ? (k0 + k1) >> 1 : k1;
                     const uint32_t w0 = (uint32_t)d0 + s * (stage_bytes >> 4);
                     uint32_t more = 0u;
@@ -329,20 +371,24 @@ cn_gemm_outer_kernel(const __grid_constant__ OuterParams p)
                                 out_mma_ts(acc + OUT_N, a + OUT_ACC_COL / 2 + 8 * j, w + 2 * j, hi, idesc, 1u);
                             }
                         }
+                        const int j0 = odd ? SM_BK / 16 : 0;   // where the second half begins in block kt
 #pragma unroll 1
-                        for (int n = kt; n < 2 * k1 - kt; ++n) {
-                            const int kb = n < k1 ? n : n - k1 + kt;
+                        for (int kb = kt; kb < k1; ++kb) {
                             const uint32_t w = w0 + kb * (OUT_CHUNK_BYTES >> 4), a = tmem + kb * SM_BK;
 #pragma unroll
                             for (int j = 0; j < SM_BK / 8; ++j) {
-                                if (j < SM_BK / 16 && odd && kb == kt) continue;
-                                if (n < k1) {
-                                    out_mma_ts(acc + OUT_N, a + 8 * j, w + (OUT_N * 128 >> 4) + 2 * j, hi, idesc, 1u);
-                                    out_mma_ts(acc + OUT_N, a + OUT_ACC_COL / 2 + 8 * j, w + 2 * j, hi, idesc, 1u);
-                                } else {
-                                    out_mma_ts(acc + OUT_N, a + 8 * j, w + 2 * j, hi, idesc, 1u);
-                                }
+                                if (kb == kt && j < j0) continue;
+                                out_mma_ts(acc + OUT_N, a + 8 * j, w + (OUT_N * 128 >> 4) + 2 * j, hi, idesc, 1u);
+                                out_mma_ts(acc + OUT_N, a + OUT_ACC_COL / 2 + 8 * j, w + 2 * j, hi, idesc, 1u);
                             }
+                        }
+                        out_mma_ts_lowered(acc + OUT_N, tmem + kt * SM_BK + 8 * j0, w0 + kt * (OUT_CHUNK_BYTES >> 4) + 2 * j0, hi, idesc);
+#pragma unroll 1
+                        for (int kb = kt; kb < k1; ++kb) {
+                            const uint32_t w = w0 + kb * (OUT_CHUNK_BYTES >> 4), a = tmem + kb * SM_BK;
+#pragma unroll
+                            for (int j = 0; j < SM_BK / 8; ++j)
+                                if (kb > kt || j > j0) out_mma_ts(acc + OUT_N, a + 8 * j, w + 2 * j, hi, idesc, 1u);
                         }
                     }
                     tc_commit(done0 + 8 * b);
@@ -429,7 +475,7 @@ cn_gemm_outer_kernel(const __grid_constant__ OuterParams p)
 #pragma unroll
                     for (int e = 0; e < 16; ++e) {
                         asm volatile("" : "+r"(r[0][e]), "+r"(r[1][e]));   // no use moves before the wait
-                        v[e] = __uint_as_float(r[0][e]) + __uint_as_float(r[1][e]);
+                        v[e] = fmaf(__uint_as_float(r[1][e]), p.low, __uint_as_float(r[0][e]));
                     }
                 } else {   // eight columns at a time: there are no registers for more, and one that spills costs more than all of this
 #pragma unroll
@@ -441,7 +487,7 @@ cn_gemm_outer_kernel(const __grid_constant__ OuterParams p)
 #pragma unroll
                         for (int e = 0; e < 8; ++e) {
                             asm volatile("" : "+r"(r[0][e]), "+r"(r[1][e]));
-                            v[h + e] += __uint_as_float(r[0][e]) + __uint_as_float(r[1][e]);
+                            v[h + e] += fmaf(__uint_as_float(r[1][e]), p.low, __uint_as_float(r[0][e]));
                         }
                     }
                 }
@@ -539,6 +585,7 @@ int cn_gemm_outer_launch(cn_context *ctx, int64_t M, int64_t N, int64_t K, const
     // sixteen additions, below that 2.1e-7 / 1.5e-7 by two; the streaming kernel's chains of 32 k where the weights have an odd pitch, 2.1e-7 / 1.6e-7
     // by two; the small products' kernel, and planes in its place, 1.3e-7 / 1.2e-7 by two of four additions each, for half of K at a time.
     p.two_chains = fine || !w_vec || K <= 96;
+    p.low = p.two_chains ? 1.0f : 1.0f / (1 << OUT_LOW);
     p.passes = fine && p.kb > 2 ? 2 : 1;
     p.sh = p.kb == 1 ? 3 : p.kb == 2 ? 4 : 5;
     p.strips = (int)((M + SM_BM - 1) / SM_BM);

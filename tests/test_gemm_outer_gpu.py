@@ -125,3 +125,38 @@ def test_few_columns_of_odd_pitch_stay_exact(ctx, M, K, N):
     ctx.gemm_check()
     assert ctx.gemm_last_kernel() == "fma"
     assert torch.equal(C.double(), err.double() @ act.double().t())
+
+
+# one part of K each with one and two chains, two parts with two chains; aligned and not
+@pytest.mark.parametrize("M,K,N", [(4096, 128, 4096), (2001, 77, 3003), (1600, 96, 2000), (4096, 96, 4096), (4000, 20, 3000)])
+@pytest.mark.parametrize("x", [-30, -34, -36, -37])
+@pytest.mark.parametrize("which", [0, 1])
+def test_operands_whose_low_parts_are_near_the_smallest_numbers(ctx, M, K, N, x, which):
+    """Steps of 2^-146 leave 2^-148 on average, 2.8e-45: of variates of 1e-37 less than the 4.9e-8 that 22 bits leave.  Sums as ever: up to sixteen additions
+    that truncate to 2^-23 of a sum which grows from nothing, a quarter of 16 * 2^-23 in the norm."""
+    g = torch.Generator(device="cuda").manual_seed(K)
+    scale = [1e36, 1e36]
+    scale[which] = 10.0 ** x
+    act, err = ((torch.randn(n, K, device="cuda", generator=g).double() * s).float() for n, s in ((M, scale[0]), (N, scale[1])))
+    C = ctx.gemm(act, err, transA=True)
+    ctx.gemm_check()
+    assert ctx.gemm_last_kernel() == "outer"
+    ref = err.double() @ act.double().t()
+    assert float((C.double() - ref).norm() / ref.norm()) <= 4.8e-7 + 2 * 4.9e-8
+
+
+@pytest.mark.parametrize("M,K,N", [(4096, 128, 4096), (2001, 77, 3003), (1600, 96, 2000)])
+def test_the_largest_values_do_not_overflow(ctx, M, K, N):
+    """Low parts are held times 2^10: three quarters of a product at most, of the lowest value of the type, too."""
+    g = torch.Generator(device="cuda").manual_seed(K)
+    act, err = torch.randn(M, K, device="cuda", generator=g), torch.rand(N, K, device="cuda", generator=g)
+    act[:, K // 2] = torch.finfo(torch.float32).min
+    act[::2, 1], err[1::2, 1] = torch.finfo(torch.float32).max, 0.0
+    err[::2, 1] = 0.5 * err[::2, K // 2]
+    C = ctx.gemm(act, err, transA=True)
+    ctx.gemm_check()
+    assert ctx.gemm_last_kernel() == "outer"
+    ref, mag = err.double() @ act.double().t(), err.double().abs() @ act.double().abs().t()
+    fits = mag < 3.4e38
+    assert float(fits.float().mean()) > 0.5
+    assert bool(((C.double() - ref).abs() <= REL * mag)[fits].all())
