@@ -222,19 +222,21 @@ int cn_gemm_dispatch(cn_context *ctx, int transA, int transB, int64_t M, int64_t
     // (520 x 784 . 784 x 1200: 38 us against 30 on the streaming kernel; 520 x 2000 . 2000 x 1000: 41 against 43).
     const bool plain = mode != CN_GEMM_FP32_SIMT && !tuned && !(ws && ws->coded_src);
     const bool fine = plain && cn_gemm_small_shape(ctx, M, N, K, tma_ok, 2);
-    const bool own = planes_ok && plain && L == 1 && !pr && !(peers && peers->npeers > 0);
+    const bool alone = planes_ok && plain && !pr && !(peers && peers->npeers > 0), own = alone && L == 1;
     const bool one_round = fine && cn_gemm_small_shape(ctx, M, N, K, tma_ok, 1);
     const bool tc_ok = tma_ok || (mode != CN_GEMM_FP32_SIMT && M * N * K >= 4096 && cn_gemm_tc_any_supported(transB, M, N, K, d_B));
     // A weight gradient that takes more than one round of the small products' kernel, and has a short inner dimension, takes one launch as well.
     // Fewer than four columns of odd pitch stay on the FMA kernel, which adds products of all 24 bits along k in order: integers that
     // it adds exactly would lose the product of their two low parts here.
     const bool gradient = transA && !transB && !bias && act == CN_ACT_LINEAR && tc_mode == CN_GEMM_3XTF32;
-    const bool outer = own && gradient && !one_round && cn_gemm_outer_shape(M, N, K) && tc_ok;
+    // With a maxout behind it, where it else were a small product.
+    const bool outer = alone && (L == 1 || (fine && ldc == M)) && gradient && !one_round && cn_gemm_outer_shape(M, N, K) && tc_ok;
     const bool planes = own && !outer && cn_gemm_planes_shape(ctx, M, N, K, tc_mode, tma_ok, fine) && (fine || K >= (1LL << 30) / (M * N));
     const bool small = plain && !outer && (L == 1 || ldc == M) && (!pr || pr->raw) && fine && (!planes || one_round) && (tma_ok || M * N * K >= 4096);
-    // a small product and its maxout are two launches as well, and the maxima are those of the very product a call without maxout gives
-    // (with up to 512 rows; from there on that call may take the kernel for many rows, whose last bits differ)
-    const bool fused_maxout = tma_ok && (L == 1 || (!small && cn_gemm_tc_can_fuse_maxout(L)));
+    // A small product, or a weight gradient in its place, and its maxout are two launches as well, and the maxima are those of the very product a
+    // call without maxout gives (small products with up to 512 rows; from there on that call may take the kernel for many rows, whose
+    // last bits differ).
+    const bool fused_maxout = tma_ok && (L == 1 || (!small && !outer && cn_gemm_tc_can_fuse_maxout(L)));
     if (L > 1 && !fused_maxout) {
         void *p = nullptr;
         int st = cn_gemm_scratch(ctx, CN_GEMM_SLOT_MAXOUT, (size_t)M * N * sizeof(float), &p);

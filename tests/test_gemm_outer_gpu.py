@@ -160,3 +160,17 @@ def test_the_largest_values_do_not_overflow(ctx, M, K, N):
     fits = mag < 3.4e38
     assert float(fits.float().mean()) > 0.5
     assert bool(((C.double() - ref).abs() <= REL * mag)[fits].all())
+
+
+@pytest.mark.parametrize("M,K,N,level", [(300, 128, 9000, 4), (500, 33, 9000, 2), (2000, 128, 1200, 3), (401, 77, 7000, 7)])
+def test_maxima_are_those_of_the_same_product(ctx, M, K, N, level):
+    """Where a weight gradient stands in for a small product, it does so with a maxout behind it, too."""
+    g = torch.Generator(device="cuda").manual_seed(K)
+    act, err = torch.randn(M, K, device="cuda", generator=g), torch.randn(N, K, device="cuda", generator=g)
+    plain = ctx.gemm(act, err, transA=True)
+    assert ctx.gemm_last_kernel() == "outer"
+    want, want_arg = ctx.maxout(plain, level)
+    arg = torch.empty_like(want_arg)
+    out = ctx.gemm(act, err, transA=True, maxout_level=level, argmax_out=arg)
+    ctx.gemm_check()
+    assert torch.equal(out, want) and torch.equal(arg, want_arg)
