@@ -390,8 +390,14 @@ __device__ __forceinline__ void act_rows_t(const float *A, int64_t lda, int64_t 
             for (int j = 0; j < 2; ++j) {
                 const int kk = 256 * j + 8 * lane;
                 if (m < M && k0 + kk < pl.Kp && (band == 0 || s_left[band - 1][kk / TC_WK] != 0u))
-                    maybe |= act_store8<LO>(pl, band, m * pl.Kp + k0 + kk, x[r][j], sc[r]) && finite[r] && act_small8<LO>(x[r][j], sc[r]);
+                    maybe |= act_store8<LO>(pl, band, m * pl.Kp + k0 + kk, x[r][j], sc[r]) && finite[r];
             }
+        }
+        // Behind all stores, whose registers it would else be short of (64 a thread).
+        if (maybe) {
+            maybe = false;
+#pragma unroll
+            for (int rj = 0; rj < 2 * ACT_ROWS_PER_WARP; ++rj) maybe |= finite[rj >> 1] && act_small8<LO>(x[rj >> 1][rj & 1], sc[rj >> 1]);
         }
         bool left = false;
         if (__syncthreads_or(maybe)) {
