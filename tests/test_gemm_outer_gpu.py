@@ -174,3 +174,34 @@ def test_maxima_are_those_of_the_same_product(ctx, M, K, N, level):
     out = ctx.gemm(act, err, transA=True, maxout_level=level, argmax_out=arg)
     ctx.gemm_check()
     assert torch.equal(out, want) and torch.equal(arg, want_arg)
+
+
+# as many additions to one sum as the kernels have that take such a product's neighbours, whose errors these are: two parts of K with two chains each,
+# two chains (two, three and four blocks, halves of one in the middle), and one
+@pytest.mark.parametrize("M,K,N,bound", [(2000, 128, 2000, 1.3e-7), (1600, 96, 2000, 1.3e-7), (4096, 96, 4096, 2.1e-7), (4001, 77, 4003, 2.1e-7), (6000, 64, 3500, 2.1e-7),
+                                         (4001, 127, 4003, 2.1e-7), (4096, 128, 4096, 3.9e-7), (300, 128, 30000, 3.9e-7)])
+def test_chains_are_as_short_as_those_of_the_kernels_beside(ctx, M, K, N, bound):
+    g = torch.Generator(device="cuda").manual_seed(K)
+    act, err = torch.rand(M, K, device="cuda", generator=g) * 2 - 1, torch.rand(N, K, device="cuda", generator=g) * 2 - 1
+    C = ctx.gemm(act, err, transA=True)
+    ctx.gemm_check()
+    assert ctx.gemm_last_kernel() == "outer"
+    ref = err.double() @ act.double().t()
+    assert float((C.double() - ref).norm() / ref.norm()) <= bound
+
+
+@pytest.mark.parametrize("M,K,N", [(2000, 128, 2000), (2049, 77, 1999), (4096, 96, 4096), (129, 31, 33000)])
+@pytest.mark.parametrize("more", [(4, 4, 4), (5, 0, 3), (0, 1, 0)])
+def test_columns_with_room_between_them(ctx, M, K, N, more):
+    """Pitches beyond K and M; what lies between the columns is neither used nor written."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    act, err = (torch.full((n, K + d), float("nan"), device="cuda") for n, d in ((M, more[0]), (N, more[1])))
+    act[:, :K], err[:, :K] = torch.randn(M, K, device="cuda", generator=g), torch.randn(N, K, device="cuda", generator=g)
+    C = torch.full((N, M + more[2]), 7.0, device="cuda")
+    assert ctx.lib.cn_gemm_f32(ctx.h, 1, 0, M, N, K, act.data_ptr(), K + more[0], err.data_ptr(), K + more[1], C.data_ptr(), M + more[2], None,
+                               _lib.GEMM_3XTF32, ctx.stream_ptr()) == 0
+    ctx.gemm_check()
+    assert ctx.gemm_last_kernel() == "outer"
+    a, w = act[:, :K].double(), err[:, :K].double()
+    assert bool(((C[:, :M].double() - w @ a.t()).abs() <= REL * (w.abs() @ a.abs().t())).all())
+    assert bool((C[:, M:] == 7.0).all())
