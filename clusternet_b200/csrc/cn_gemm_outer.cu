@@ -106,19 +106,6 @@ __device__ __forceinline__ void out_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uin
         ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate) : "memory");
 }
 
-__device__ __forceinline__ void out_ld16(uint32_t taddr, uint32_t (&r)[16])
-{
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void out_ld8(uint32_t taddr, uint32_t (&r)[8])
-{
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
-}
 __device__ __forceinline__ void out_st4(uint32_t taddr, const uint32_t (&v)[4])
 {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
@@ -469,9 +456,9 @@ cn_gemm_outer_kernel(const __grid_constant__ OuterParams p)
                 tc_fence_after();
                 if (first) {
                     uint32_t r[2][16];
-                    out_ld16(src, r[0]);
-                    out_ld16(src + OUT_N, r[1]);
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    tc_ld_ahead(src, r[0]);
+                    tc_ld_ahead(src + OUT_N, r[1]);
+                    tc_wait_ld();
 #pragma unroll
                     for (int e = 0; e < 16; ++e) {
                         asm volatile("" : "+r"(r[0][e]), "+r"(r[1][e]));   // no use moves before the wait
@@ -481,9 +468,9 @@ cn_gemm_outer_kernel(const __grid_constant__ OuterParams p)
 #pragma unroll
                     for (int h = 0; h < 16; h += 8) {
                         uint32_t r[2][8];
-                        out_ld8(src + h, r[0]);
-                        out_ld8(src + OUT_N + h, r[1]);
-                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                        tc_ld_ahead(src + h, r[0]);
+                        tc_ld_ahead(src + OUT_N + h, r[1]);
+                        tc_wait_ld();
 #pragma unroll
                         for (int e = 0; e < 8; ++e) {
                             asm volatile("" : "+r"(r[0][e]), "+r"(r[1][e]));
@@ -516,7 +503,7 @@ cn_gemm_outer_kernel(const __grid_constant__ OuterParams p)
             if (change) make_strip(next_strip, ring + s * stage_bytes);
             if (!ok) break;
             strip = next_strip;
-            // Half of the warps store first, the others split first: stores are bound by the way to L2, which takes 32 bytes per clock from an SM.
+            // Every warp stores first and splits then; stores are bound by the way to L2, which takes 32 bytes per clock from an SM.
             if (amore) {
                 put(s);
                 amore = ahead.next(p, astrip, an0, acols);
@@ -544,8 +531,8 @@ cn_gemm_outer_kernel(const __grid_constant__ OuterParams p)
 // slower from K = 64 on (784 x 128 . 128 x 1200 8.0 / 6.8 us), but its shares of K are chains of their own, 1.2e-7 off where this one, as fast as
 // that, is off by 3.3e-7.  With fewer than eight rows most lanes have no work (up to 1.5 of the streaming kernel's time with one).  Up to 16 k are one addition
 // as planes and two here (6.6e-8 / 8.3e-8).
-// Other products with so short a K would gain as much, in any layout, with bias and units and in the single pass (133 drawn ones 0.51 of the time): which
-// kernels those take, down to K = 40, is what their tests are about, so they stay where they are.
+// Other products with so short a K (other layouts, bias, units, the single pass) keep their kernels, though a trial form of this one took 0.51 of their
+// time over 133 drawn ones: their layouts, epilogues and single pass are not written here.
 bool cn_gemm_outer_shape(int64_t M, int64_t N, int64_t K)
 {
     return M >= 8 && K > 16 && K <= OUT_MAX_K && M < (1LL << 31) - 256 && N < (1LL << 31) - 256;

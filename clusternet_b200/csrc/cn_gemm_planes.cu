@@ -573,15 +573,7 @@ __device__ __forceinline__ void pl_store(const CUtensorMap *map, uint32_t src, i
 {
     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"((uint64_t)map), "r"(src), "r"(m), "r"(n) : "memory");
 }
-// 16 columns of tensor memory, and the wait for them (which the registers pass through, so that no use moves before it).
-__device__ __forceinline__ void pl_ld16(uint32_t taddr, uint32_t (&r)[16])
-{
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr) : "memory");
-}
+// The wait for 16 columns of tensor memory, which the registers pass through, so that no use moves before it.
 __device__ __forceinline__ void pl_wait_ld16(uint32_t (&r)[16])
 {
     asm volatile("tcgen05.wait::ld.sync.aligned;"
@@ -832,12 +824,12 @@ cn_gemm_planes_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_con
                 const uint64_t wi2 = tc_pack2(wi, wi);
                 const uint32_t src = src0 + ab * 256u;
                 uint32_t r[2][16];   // the next 16 columns are on their way while these are added
-                pl_ld16(src, r[0]);
+                tc_ld_ahead(src, r[0]);
 #pragma unroll
                 for (int cc = 0; cc < 8; ++cc) {
                     if (cc * 16 >= half) break;
                     pl_wait_ld16(r[cc & 1]);
-                    if (cc < 7 && cc * 16 + 16 < half) pl_ld16(src + cc * 16 + 16, r[(cc + 1) & 1]);
+                    if (cc < 7 && cc * 16 + 16 < half) tc_ld_ahead(src + cc * 16 + 16, r[(cc + 1) & 1]);
 #pragma unroll
                     for (int i = 0; i < 16; i += 4) {
                         const float4 f = lds4(as + (cc * 16 + i) * 4);

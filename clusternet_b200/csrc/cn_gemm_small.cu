@@ -61,6 +61,22 @@ struct SmCfg {
     static_assert(SMEM_MAX <= 232448 - 1024, "shared memory");
 };
 
+// An operand: element (row, k) at p[row * sr + k * sk].
+struct SmOperand {
+    const float *p;
+    int64_t sr, sk;
+    int vec;                // 16-byte aligned along the contiguous one of the two
+};
+static inline SmOperand sm_operand(const float *p, bool k_contiguous, int64_t ld)
+{
+    SmOperand o;
+    o.p = p;
+    o.sr = k_contiguous ? ld : 1;
+    o.sk = k_contiguous ? 1 : ld;
+    o.vec = (ld & 3) == 0 && ((uintptr_t)p & 15u) == 0;
+    return o;
+}
+
 struct SmallParams {
     SmOperand A, W;
     int64_t M, N, K;
@@ -80,6 +96,18 @@ struct SmallParams {
     int nranks, my_rank;
     unsigned int epoch;
 };
+
+// D[tmem] (+)= A[smem] * B[smem], both K-major TF32 tiles.
+__device__ __forceinline__ void sm_mma_ss(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc, uint32_t accumulate)
+{
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 ad, bd;\n\t"
+        "setp.ne.b32 p, %5, 0;\n\t"
+        "mov.b64 ad, {%1, %3};\n\t"
+        "mov.b64 bd, {%2, %3};\n\t"
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], ad, bd, %4, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate) : "memory");
+}
 
 // The share of one thread of a block of ROWS x 32 k: up to four 16-byte chunks (a chunk is four consecutive k of a row).
 // QUADS false: chunks of rows 32 apart; with k contiguous, eight lanes read a row's 128 bytes, 16 at a time where the rows are aligned;
@@ -220,19 +248,6 @@ struct SmFeed {
     }
 };
 
-template <int COLS>
-__device__ __forceinline__ void sm_ld(uint32_t taddr, uint32_t (&r)[COLS])
-{
-    if constexpr (COLS == 8)
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(taddr) : "memory");
-    else
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-              "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-            : "r"(taddr) : "memory");
-}
 // Columns of the accumulators of all chains, in K order, the products with a low part last.
 template <int NT, bool MODE3X, int COLS>
 __device__ __forceinline__ void sm_sum(uint32_t taddr, int chains, float (&v)[COLS])
@@ -249,9 +264,9 @@ __device__ __forceinline__ void sm_sum(uint32_t taddr, int chains, float (&v)[CO
         for (int ch = 0; ch < GROUP; ++ch) {
             if (ch0 + ch >= chains) break;
 #pragma unroll
-            for (int part = 0; part < PARTS; ++part) sm_ld<COLS>(taddr + (ch0 + ch) * Cfg::ACC_COLS + part * NT, r[ch][part]);
+            for (int part = 0; part < PARTS; ++part) tc_ld_ahead(taddr + (ch0 + ch) * Cfg::ACC_COLS + part * NT, r[ch][part]);
         }
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        tc_wait_ld();
 #pragma unroll
         for (int ch = 0; ch < GROUP; ++ch) {
             if (ch0 + ch >= chains) break;

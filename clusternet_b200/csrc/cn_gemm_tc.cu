@@ -1317,9 +1317,9 @@ size_t cn_tc_cut::partial_bytes() const { return rest() > 0 && cluster == 1 ? (s
 // and 0.66 per block with one tile of 128 columns per CTA, 20 and 0.74 with two; but K is cut into as many parts as CTAs find room in the GPCs
 // for every tile, not one per SM.  us, runs / clusters: 24 x 560 . 560 x 5192 23.8 / 14.5; 100 x 1500 . 1500 x 2500 30.6 / 19.6; 48 x 1568 . 1568 x 11448 39.4
 // / 28.7; 128 x 2348 . 2348 x 8289 40.4 / 38.5; 128 x 100000 . 100000 x 1000 131 / 299.  With two tiles of rows a few gain (256 x 4096 . 4096 x 4096 55.5 /
-// 49.7), others lose (150 x 2344 . 2344 x 2208 33 / 38).  The fit is older than the reduction's CTAs of eight columns: of 548 products drawn where
-// this rule takes clusters, which take 0.80 of the runs' time on average, 27 are more than 3 % faster by runs today (104 x 5014 . 5014 x 3526 42.1 /
-// 48.6 the worst of them); a fit with the rows in it gained nothing over drawn products.
+// 49.7), others lose (150 x 2344 . 2344 x 2208 33 / 38).  The fit is older than the reduction's CTAs of eight columns and than
+// runs that leave out rows which do not exist: of 238 products drawn where this rule takes clusters, which take 0.94 of the runs' time on average,
+// 70 are more than 3 % faster by runs today, 54 of them among the 102 of up to 32 rows (32 x 3888 . 3888 x 3000 23.7 / 30.3 the worst of them).
 //
 // Runs are short, and so are their accumulation chains; clusters' chains are cut as short, so that no product is less exact: relative to fp64,
 // runs of 28 blocks 1.6e-6, of 14 1.3e-6, of 6 7e-7; chains of 8 blocks 9.8e-7, of 4 5.4e-7.  That costs long runs more than the launch
