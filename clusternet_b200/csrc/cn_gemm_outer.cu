@@ -10,12 +10,12 @@
 //   * two warps issue the MMAs, blocks in turn, each into an accumulator of its own: 64 columns for the products of the high parts and 64 for
 //     those with a low part (the activations' high parts are multiplied with both parts of the weights at once);
 //   * rows m lie in the lanes, so that a warp stores 128 bytes of a column straight from registers whatever C's pitch and alignment.
-// TF32 parts need no scales of rows and columns and leave nothing over: no lists, no second kernel behind this one.  A low part as it is would have no
-// bits left below 2^-113, where it meets TF32's smallest step, 2^-136 (operands of 1e-36 3.4e-6 off, of 1e-38 3.3e-4).  So all low parts are held
+// TF32 parts need no scales of rows and columns and leave nothing over: no lists, no second kernel behind this one.  A low part as it is would lose
+// bits below 2^-113, where it meets TF32's smallest step, 2^-136 (operands of 1e-36 3.4e-6 off, of 1e-38 3.3e-4).  So all low parts are held
 // times 2^OUT_LOW, which the sums of their products lose again: operands keep their 22 bits down to 2^-124, and from there on steps of 2^-146.
 //
-// us in a series, before / now: 4096 x 128 . 128 x 4096 40 / 25, 2000 x 128 . 128 x 2000 22.5 / 12.5, 6000 x
-// 32 . 32 x 6000 63 / 37 (planes); 2001 x 77 . 77 x 3003 58 / 16.3, 1504 x 64 . 64 x 3500 43 / 9.5 (streaming); 3734 x 104 . 104 x 575 16.2 / 9.4 (two rounds of small
+// us in a series, before / now: 4096 x 128 . 128 x 4096 40 / 25, 2000 x 128 . 128 x 2000 22.0 / 11.9, 6000 x
+// 32 . 32 x 6000 63 / 39 (planes); 2001 x 77 . 77 x 3003 58 / 15.8, 1504 x 64 . 64 x 3500 42 / 9.5 (streaming); 3734 x 104 . 104 x 575 15.8 / 10.3 (two rounds of small
 // products).  Drawn over batches of 17 to 128 and layers of 300 to 6000: 0.41 of the time of planes, 0.34 of the streaming kernel, 0.68 of small products in two
 // rounds, 0.86 at most.
 // Bound, per block of 64 columns and K = 128, by the MMAs (1540 clocks at their rate, 2400 with what the two warps need to issue them beside
